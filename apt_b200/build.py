@@ -1,4 +1,5 @@
-"""Builds apt_b200/libapt_b200.so from apt_b200/csrc/*.cu with nvcc for sm_100a.
+"""Builds apt_b200/libapt_b200.so from apt_b200/csrc/*.cu with nvcc for sm_100a, and apt_b200/_native.so,
+the operators' host side in C++ (apt_b200/native/*.cpp), against PyTorch's headers.
 
 Run as ``python apt_b200/build.py`` (add ``--force`` to rebuild, ``-v`` for
 ptxas register/shared-memory reports). Run as a file, it does not import the
@@ -13,7 +14,10 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libapt_b200.so")
-SOURCES = ["core.cu", "sample.cu", "relabel.cu", "bucket.cu", "gather.cu", "spmm.cu", "virt.cu", "hotness.cu", "p2p.cu", "util.cu"]
+NATIVE = os.path.join(PKG_DIR, "native")
+NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
+SOURCES = ["core.cu", "sample.cu", "relabel.cu", "bucket.cu", "gather.cu", "spmm.cu", "spmm_f32.cu", "spmm_bf16.cu",
+           "spmm_f16.cu", "gat.cu", "virt.cu", "hotness.cu", "p2p.cu", "util.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",
@@ -29,27 +33,61 @@ def _nvcc():
     return exe
 
 
-def _stale():
-    if not os.path.exists(LIB_PATH):
+def _older(target, folder):
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    t = os.path.getmtime(target)
+    deps = [os.path.join(folder, f) for f in os.listdir(folder)]
     deps.append(os.path.join(PKG_DIR, "..", "include", "apt_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _native_command(out):
+    """g++ on native/*.cpp; PyTorch is found without importing it, its libraries are loaded by the time the
+    module is, and libapt_b200.so is the one beside it."""
+    import importlib.util
+    import sysconfig
+
+    torch_dir = list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+    cuda_home = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    src = sorted(os.path.join(NATIVE, f) for f in os.listdir(NATIVE) if f.endswith(".cpp"))
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w", "-DTORCH_EXTENSION_NAME=_native",
+            *[a for d in inc for a in ("-isystem", d)], *src, "-o", out,
+            "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+            "-Wl,-rpath," + os.path.join(torch_dir, "lib"), "-Wl,-rpath,$ORIGIN", LIB_PATH]
+
+
+def _build_native(verbose=False):
+    tmp_path = NATIVE_PATH + ".tmp"
+    subprocess.run(_native_command(tmp_path), check=True)
+    os.replace(tmp_path, NATIVE_PATH)
+
+
 def build(force=False, verbose=False):
-    """Compile every kernel file to an object and link the shared library."""
-    if not force and not _stale():
-        return LIB_PATH
+    """Compile every kernel file to an object and link the shared library, then the host side over it."""
+    if force or _older(LIB_PATH, CSRC):
+        _build_kernels(force, verbose)
+    if force or _older(NATIVE_PATH, NATIVE):
+        _build_native(verbose)
+    return LIB_PATH
+
+
+def _build_kernels(force=False, verbose=False):
     nvcc = _nvcc()
     obj_dir = os.path.join(PKG_DIR, "build")
     os.makedirs(obj_dir, exist_ok=True)
     procs = []
     objs = []
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
+    headers += [os.path.join(PKG_DIR, "..", "include", "apt_b200.h"), os.path.abspath(__file__)]
     for src in SOURCES:
         obj = os.path.join(obj_dir, src.replace(".cu", ".o"))
         objs.append(obj)
+        deps = headers + [os.path.join(CSRC, src)]
+        if not force and os.path.exists(obj) and all(os.path.getmtime(d) <= os.path.getmtime(obj) for d in deps):
+            continue
         cmd = [nvcc, *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
@@ -66,10 +104,10 @@ def build(force=False, verbose=False):
         raise RuntimeError("nvcc failed; see messages above")
     # linked beside its final place and moved there in one step: a reader never sees a half-written library
     tmp_path = LIB_PATH + ".tmp"
-    link = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", tmp_path, *objs]
+    link = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-Xlinker", "-soname=libapt_b200.so", "-o", tmp_path,
+            *objs]
     subprocess.run(link, check=True)
     os.replace(tmp_path, LIB_PATH)
-    return LIB_PATH
 
 
 if __name__ == "__main__":

@@ -1,0 +1,6 @@
+// Row kernels of the SpMM for __half rows.
+#include "spmm_rows.cuh"
+
+namespace apt {
+APT_DEFINE_SPMM_ROWS(__half)
+}  // namespace apt

@@ -1,0 +1,6 @@
+// Row kernels of the SpMM for float rows.
+#include "spmm_rows.cuh"
+
+namespace apt {
+APT_DEFINE_SPMM_ROWS(float)
+}  // namespace apt

@@ -1,0 +1,498 @@
+// The row kernel of the SpMM and what it shares with the kernels that prepare a block for it.
+//
+// Every output row belongs to a group of lanes of one warp, which walks the row's edges, keeps the
+// sums in fp32 registers and writes the row once: no float atomics, no zero-fill of the output.
+//
+//   lane split   `lpe` lanes cover one input row (VPL slices of up to 16 bytes each), `ep` edges of the
+//                row are read side by side, and their partial sums meet in a shuffle butterfly at the
+//                end. Narrow rows need the second factor: with 4 lanes to a 64-byte row and one edge at a
+//                time a row of 100 edges is 100 / 4 rounds of load latency.
+//   in flight    the loads of U edges (U * VPL slices a lane) are issued before any of them is added;
+//                the next row's bounds and source indexes are fetched while this row's slices are
+//                on their way, so that a short row costs one round of latency and not three. Full rounds carry
+//                no predicate: a round is bound by its instruction count once the rows come out of L2 (lanes
+//                beyond the row read its last slice again and are not written).
+//   long rows    the reverse direction of a block gathers at its hubs: longer rows (`long_edges`) are cut into
+//                items of about sqrt(edges) edges, at least kItemEdges, that whole warps take before the rows. Each
+//                leaves its partial sums in scratch and the item that finishes last adds them in order. One
+//                block of 1024 threads per long row, the form before this, kept 26 of 148 SMs busy for
+//                62 us behind the row kernel.
+//
+// Where a row's edges are (`mode`):
+//   kFixed    every row has `fixed` consecutive edges: what a fanout sampler produces. No table.
+//   kRanges   grouped by row, any length: range[] (k_edge_ranges)
+//   kOrder    anything else: a counting sort by row leaves (source row, edge) pairs in order[]
+//   kDevice   the probe kernel's verdict is read from device memory (apt_spmm_sum, which may not wait)
+//
+// What it measured is at rows_min_blocks.
+#pragma once
+
+#include "rows.cuh"
+
+namespace apt {
+
+constexpr int kMaxSegments = 64;
+enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kGatSrc = 4 };
+enum { kDevice = -1, kFixed = 0, kRanges = 1, kOrder = 2 };
+
+// Rows of more edges are left to whole warps. A group narrower than a warp hands over earlier: its own pace is
+// one round of latency per U edges.
+constexpr int kLongRow = 128, kLongRowNarrow = 32;
+constexpr int kItemEdges = 64;
+constexpr int kLongRun = 64;     // runs of at least this many edges make the probe ask for the counting sort
+
+struct SegTable {
+  // first edge, first input row and first output row of every segment
+  const int64_t* coo_off;
+  const int64_t* in_off;
+  const int64_t* out_off;
+  int nseg;
+};
+
+// The probe's answer in one word, so that a single store delivers it to the host: rows (31 bits), mode (2), sequence (31).
+// Rows that do not fit (or are negative) answer mode 3.
+__host__ __device__ inline int64_t probe_pack(int64_t rows, int mode, int64_t sequence) {
+  return (sequence << 33) | ((int64_t)mode << 31) | rows;
+}
+__host__ __device__ inline int64_t probe_rows(int64_t w) { return w & 0x7fffffff; }
+__host__ __device__ inline int probe_mode(int64_t w) { return (int)(w >> 31) & 3; }
+__host__ __device__ inline int64_t probe_sequence(int64_t w) { return (int64_t)((uint64_t)w >> 33); }
+
+struct SpmmWs {
+  // zero when a call starts that groups edges or asks the device for the mode
+  int64_t* result;      // [1] the probe's answer (probe_pack)
+  uint32_t* probe;      // [2] what the blocks of the probe found, blocks done
+  int32_t* num_items;   // [1]
+  int32_t* num_slots;   // [1] slots of order[] given out
+  int32_t* num_parts;   // [1] rows of part[] given out
+  int32_t* cnt;         // [rows] edges per row
+  int32_t* part_done;   // [max_parts] items of a row that have finished, at the row's first part
+  size_t zero_bytes;
+  // written before they are read
+  int2* range;          // [rows] first and last slot (edge) of every row
+  uint32_t* rank;       // [edges] position inside its row
+  uint2* order;         // [edges] (source row, edge id), grouped by output row
+  int4* items;          // [max_items] row, first, last slot, part (-1: the row's only item)
+  float* part;          // [part_floats] partial sums
+  int64_t max_items, max_parts, part_floats;
+};
+
+__device__ __forceinline__ int seg_of(const int64_t* coo, int nseg, int64_t e) {
+  int k = 0;
+  while (k + 1 < nseg && coo[k + 1] <= e) ++k;
+  return k;
+}
+
+__host__ __device__ inline int item_edges(int deg) {
+  int per = kItemEdges;
+  while ((int64_t)per * per < deg) per += 32;
+  return per;
+}
+
+// How rows are divided among lanes: slices of `ve` elements, `vpl` of them a lane.
+struct RowSplit {
+  int ve, vpl;
+  int lpe, ep;       // lanes to an edge, edges side by side: powers of two, lpe * ep <= 32
+  int long_edges;    // longer rows are whole warps' work (kOrder)
+};
+inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t num_rows) {
+  RowSplit r;
+  const int64_t nvec = feat_dim / ve;
+  r.ve = ve;
+  // one slice a lane while 32 lanes cover the row; two, then four, beyond (wider rows are walked in column blocks)
+  r.vpl = nvec <= 32 ? 1 : nvec <= 64 ? 2 : 4;
+  r.lpe = pow2_ge(ceil_div(nvec, r.vpl));
+  // edges side by side: never more than half the mean row, whose second half would idle those lanes
+  r.ep = pow2_le(num_edges / (num_rows * 2), 32 / r.lpe);
+  r.long_edges = r.lpe * r.ep == 32 ? kLongRow : kLongRowNarrow;
+  return r;
+}
+
+template <typename T>
+struct RowArgs {
+  const int64_t* row;
+  const T* in;
+  const T* edata;          // kGatSrc: float2[E][heads] (attention, score gradient)
+  int64_t edata_dim, feat_dim;
+  SegTable st;
+  int64_t num_rows, num_edges;
+  SpmmWs ws;
+  T* out;
+  T* out2;                 // kGatSrc: [rows][heads] sums of the score gradients
+  int mode, fixed;
+  RowSplit split;
+  int part_stride;         // floats per part
+};
+
+// One slice of one edge's contribution, in two steps so that the loads of several edges are issued
+// before any of them is used.
+template <typename T, int VE, int OP>
+struct EdgeSlice {
+  Raw<T, VE> x;                                           // input slice (kCopyE: the edge's own)
+  Raw<T, (OP == kUMulE || OP == kUAddE) ? VE : 2 / sizeof(T) + 1> w;   // per-column edge values
+  float s, s2;                                            // per-head edge value (kGatSrc: and gradient)
+};
+
+template <typename T, int VE, int OP>
+__device__ __forceinline__ void slice_load(EdgeSlice<T, VE, OP>& v, const RowArgs<T>& a, uint32_t src, uint32_t e,
+                                           int64_t col, int per, int head) {
+  if constexpr (OP == kCopyE) {
+    v.x = load_raw<T, VE>(a.edata + (int64_t)e * a.feat_dim + col);
+  } else {
+    v.x = load_raw<T, VE>(a.in + (int64_t)src * a.feat_dim + col);
+  }
+  if constexpr (OP == kUMulE || OP == kUAddE) {
+    if (per == 1) {
+      v.w = load_raw<T, VE>(a.edata + (int64_t)e * a.feat_dim + col);
+    } else if (head >= 0) {
+      v.s = Elem<T>::to_f(a.edata[(int64_t)e * a.edata_dim + head]);
+    } else {
+      Pack<T, VE> w;
+#pragma unroll
+      for (int t = 0; t < VE; ++t) w.v[t] = a.edata[(int64_t)e * a.edata_dim + (col + t) / per];
+#pragma unroll
+      for (int k = 0; k < (int)(sizeof(v.w.w) / 4); ++k)
+        v.w.w[k] = sizeof(T) * VE < 4 ? (unsigned int)*(const unsigned short*)&w : ((const unsigned int*)&w)[k];
+    }
+  }
+  if constexpr (OP == kGatSrc) {
+    const float2 p = __ldg((const float2*)a.edata + (int64_t)e * a.edata_dim + head);
+    v.s = p.x;
+    v.s2 = p.y;
+  }
+}
+
+template <typename T, int VE, int OP>
+__device__ __forceinline__ void slice_add(float* acc, float& acc2, const EdgeSlice<T, VE, OP>& v, int per, int head) {
+#pragma unroll
+  for (int t = 0; t < VE; ++t) {
+    const float x = v.x.get(t);
+    if constexpr (OP == kUMulE || OP == kUAddE) {
+      const float w = (per != 1 && head >= 0) ? v.s : v.w.get(t);
+      acc[t] += OP == kUMulE ? x * w : x + w;
+    } else if constexpr (OP == kGatSrc) {
+      acc[t] += v.s * x;
+    } else {
+      acc[t] += x;
+    }
+  }
+  if constexpr (OP == kGatSrc) acc2 += v.s2;
+}
+
+// The sums of the edges read side by side meet, and the lanes of the first of them write the row's column block.
+template <typename T, int VE, int VPL, int OP>
+__device__ __forceinline__ void rows_write(const RowArgs<T>& a, float (&acc)[VPL][VE], float (&acc2)[VPL], const int (&col)[VPL],
+                                           const int (&head)[VPL], int d, int c0, int nvec, int per, int lpe, int lpr, int vl,
+                                           int epi, unsigned gmask) {
+#pragma unroll 1
+  for (int o = lpe; o < lpr; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+#pragma unroll
+      for (int t = 0; t < VE; ++t) acc[i][t] += __shfl_xor_sync(gmask, acc[i][t], o);
+      if constexpr (OP == kGatSrc) acc2[i] += __shfl_xor_sync(gmask, acc2[i], o);
+    }
+  if (epi != 0) return;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    if (c0 + vl + i * lpe >= nvec) continue;
+    Pack<T, VE> o;
+#pragma unroll
+    for (int t = 0; t < VE; ++t) o.v[t] = Elem<T>::from_f(acc[i][t]);
+    store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], o);
+    if constexpr (OP == kGatSrc)
+      if (col[i] % per == 0) a.out2[(int64_t)d * a.edata_dim + head[i]] = Elem<T>::from_f(acc2[i]);
+  }
+}
+
+// Blocks an SM is to hold. The gather is bound by loads in flight, and the 64 (80) registers a thread of four (three)
+// blocks hold the slices of plain sums without spilling; edge values and 8 elements a slice need more.
+// 67 584 x 15 edges, fp32 x 256 (1.04 GB gathered, mostly out of L2): 152 us at one or two blocks, 114 at three, 109 at
+// four; bf16 x 256: 89 / 65 / 63 us; the reverse direction 186 / 149 / 158 and 104 / 82 / 90 us.
+constexpr int rows_min_blocks(int op, int elems) {
+  if (op == kCopyU || op == kCopyE) return elems <= 4 ? 4 : elems <= 8 ? 3 : 2;
+  return elems <= 2 ? 3 : elems <= 8 ? 2 : 1;
+}
+
+// WIDE: a warp to an edge (lpe 32, ep 1), which leaves the geometry to the compiler and its registers to more warps.
+template <typename T, int VE, int VPL, int OP, bool WIDE>
+__global__ void __launch_bounds__(256, rows_min_blocks(OP, VE * VPL))
+k_spmm_rows(const RowArgs<T> a) {
+  constexpr int U = VPL >= 2 ? 2 : 4;
+  __shared__ int64_t coo[kMaxSegments + 1], ioff[kMaxSegments + 1];
+  int mode = a.mode, fixed = a.fixed;
+  if (mode == kDevice) {
+    const int64_t w = *a.ws.result;
+    mode = probe_mode(w);
+    fixed = mode == kFixed ? (int)(a.num_edges / a.num_rows) : 0;
+  }
+  if (mode != kOrder) {
+    for (int t = threadIdx.x; t <= a.st.nseg; t += blockDim.x) {
+      coo[t] = a.st.coo_off[t];
+      ioff[t] = OP == kCopyE ? 0 : a.st.in_off[t];
+    }
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31;
+  const int lpe = WIDE ? 32 : a.split.lpe, vl = lane & (lpe - 1);
+  const int nvec = (int)(a.feat_dim / VE);
+  const int per = (int)(a.feat_dim / a.edata_dim);
+  // rows and edges fit 31 bits, and so does everything that counts them
+  const int num_rows = (int)a.num_rows;
+  const int warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int num_items = mode == kOrder ? min(*a.ws.num_items, (int)a.ws.max_items) : 0;
+  bool items = warp < num_items;                     // whole warps first take items ...
+  // ... then groups of lanes take rows: lpr lanes, ep edges side by side
+  int g_ep = items ? 32 / lpe : a.split.ep, g_lpr = lpe * g_ep, g_sub = lane & (g_lpr - 1), g_epi = g_sub / lpe;
+  unsigned g_mask = g_lpr == 32 ? 0xffffffffu : (((1u << g_lpr) - 1u) << (lane - g_sub));
+#define EP (WIDE ? 1 : g_ep)
+#define LPR (WIDE ? 32 : g_lpr)
+#define SUB (WIDE ? lane : g_sub)
+#define EPI (WIDE ? 0 : g_epi)
+#define GMASK (WIDE ? 0xffffffffu : g_mask)
+
+  auto resolve = [&](int k, uint32_t& src, uint32_t& e) {
+    if (mode == kOrder) {
+      const uint2 o = a.ws.order[k];
+      src = o.x;
+      e = o.y;
+    } else {
+      e = (uint32_t)k;
+      src = OP == kCopyE ? 0u : (uint32_t)(ioff[a.st.nseg > 1 ? seg_of(coo, a.st.nseg, k) : 0] + a.row[k]);
+    }
+  };
+  auto bounds = [&](int d, int& b, int& e) {
+    if (mode == kFixed) {
+      b = d * fixed;
+      e = b + fixed;
+    } else {
+      const int2 r = a.ws.range[d];
+      b = r.x;
+      e = r.y;
+    }
+  };
+
+  int it = warp, d = 0, G = 0;
+  int b = 0, e = 0, nb = 0, ne = 0, part = -1;
+  uint32_t src = 0, eid = 0, nsrc = 0, neid = 0;
+  auto start_item = [&]() {
+    const int4 m = a.ws.items[it];
+    d = m.x;
+    b = m.y;
+    e = m.z;
+    part = m.w;
+    if (b + lane < e) resolve(b + lane, src, eid);
+  };
+  auto start_rows = [&]() {
+    items = false;
+    g_ep = a.split.ep, g_lpr = lpe * g_ep, g_sub = lane & (g_lpr - 1), g_epi = g_sub / lpe;
+    g_mask = g_lpr == 32 ? 0xffffffffu : (((1u << g_lpr) - 1u) << (lane - g_sub));
+    G = warps * (32 / LPR);
+    d = warp * (32 / LPR) + lane / LPR;
+    part = -1;
+    if (d < num_rows) {
+      bounds(d, b, e);
+      if (b + SUB < e) resolve(b + SUB, src, eid);
+    }
+    if (d + G < num_rows) bounds(d + G, nb, ne);
+  };
+  if (items) start_item(); else start_rows();
+
+  while (items || d < num_rows) {
+    int nnb = 0, nne = 0;
+    if (!items) {
+      // the next row's indexes and the bounds of the one after it are on their way while this one is summed
+      if (d + G < num_rows && nb + SUB < ne) resolve(nb + SUB, nsrc, neid);
+      if (d + 2 * G < num_rows) bounds(d + 2 * G, nnb, nne);
+    }
+    const bool skip = !items && mode == kOrder && e - b > a.split.long_edges;
+#pragma unroll 1
+    for (int c0 = 0; c0 < nvec && !skip; c0 += lpe * VPL) {
+      float acc[VPL][VE], acc2[VPL];
+      int head[VPL], col[VPL];
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        acc2[i] = 0.f;
+#pragma unroll
+        for (int t = 0; t < VE; ++t) acc[i][t] = 0.f;
+        col[i] = min(c0 + vl + i * lpe, nvec - 1) * VE;
+        head[i] = (OP == kGatSrc || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
+      }
+      uint32_t my_src = src, my_e = eid;
+#pragma unroll 1
+      for (int k0 = b; k0 < e; k0 += LPR) {
+        if (k0 != b && k0 + SUB < e) resolve(k0 + SUB, my_src, my_e);
+        const int cnt = min(LPR, e - k0);
+        int j = EPI;
+        const int full = cnt & ~(EP * U - 1);
+#pragma unroll 1
+        for (; j < full; j += EP * U) {
+          EdgeSlice<T, VE, OP> v[U][VPL];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint32_t s = OP == kCopyE ? 0u : __shfl_sync(GMASK, my_src, j + u * EP, LPR);
+            const uint32_t x = OP == kCopyU ? 0u : __shfl_sync(GMASK, my_e, j + u * EP, LPR);
+#pragma unroll
+            for (int i = 0; i < VPL; ++i) slice_load<T, VE, OP>(v[u][i], a, s, x, col[i], per, head[i]);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < VPL; ++i) slice_add<T, VE, OP>(acc[i], acc2[i], v[u][i], per, head[i]);
+        }
+        if (full < cnt) {
+          EdgeSlice<T, VE, OP> v[U][VPL];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint32_t s = OP == kCopyE ? 0u : __shfl_sync(GMASK, my_src, (j + u * EP) & (LPR - 1), LPR);
+            const uint32_t x = OP == kCopyU ? 0u : __shfl_sync(GMASK, my_e, (j + u * EP) & (LPR - 1), LPR);
+            if (j + u * EP < cnt) {
+#pragma unroll
+              for (int i = 0; i < VPL; ++i) slice_load<T, VE, OP>(v[u][i], a, s, x, col[i], per, head[i]);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (j + u * EP < cnt) {
+#pragma unroll
+              for (int i = 0; i < VPL; ++i) slice_add<T, VE, OP>(acc[i], acc2[i], v[u][i], per, head[i]);
+            }
+        }
+      }
+      int last = 1;
+      if (part >= 0) {
+        // several items to the row: leave the sums, and let the item that finishes last add them up in item order.
+        // Only the last column block counts the item as finished.
+        float* p = a.ws.part + (int64_t)part * a.part_stride;
+#pragma unroll 1
+        for (int o = lpe; o < LPR; o <<= 1)
+#pragma unroll
+          for (int i = 0; i < VPL; ++i) {
+#pragma unroll
+            for (int t = 0; t < VE; ++t) acc[i][t] += __shfl_xor_sync(GMASK, acc[i][t], o);
+            if constexpr (OP == kGatSrc) acc2[i] += __shfl_xor_sync(GMASK, acc2[i], o);
+          }
+        if (EPI == 0) {
+#pragma unroll
+          for (int i = 0; i < VPL; ++i) {
+            if (c0 + vl + i * lpe >= nvec) continue;
+#pragma unroll
+            for (int t = 0; t < VE; ++t) __stcg(p + col[i] + t, acc[i][t]);
+            if constexpr (OP == kGatSrc)
+              if (col[i] % per == 0) __stcg(p + a.feat_dim + head[i], acc2[i]);
+          }
+        }
+        if (c0 + lpe * VPL < nvec) continue;
+        last = 0;
+        const int2 r = a.ws.range[d];
+        const int size = item_edges(r.y - r.x), parts = (r.y - r.x + size - 1) / size;
+        const int first = part - (b - r.x) / size;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) last = atomicAdd(a.ws.part_done + first, 1) == parts - 1;
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (!last) break;
+        __threadfence();
+#pragma unroll 1
+        for (int cc = 0; cc < nvec; cc += lpe * VPL) {
+#pragma unroll
+          for (int i = 0; i < VPL; ++i) {
+            col[i] = min(cc + vl + i * lpe, nvec - 1) * VE;
+            head[i] = OP == kGatSrc ? col[i] / per : -1;
+            acc2[i] = 0.f;
+#pragma unroll
+            for (int t = 0; t < VE; ++t) acc[i][t] = 0.f;
+#pragma unroll 1
+            for (int q = EPI; q < parts; q += EP) {
+              const float* src_part = a.ws.part + (int64_t)(first + q) * a.part_stride;
+#pragma unroll
+              for (int t = 0; t < VE; ++t) acc[i][t] += __ldcg(src_part + col[i] + t);
+              if constexpr (OP == kGatSrc) acc2[i] += __ldcg(src_part + a.feat_dim + head[i]);
+            }
+          }
+          c0 = cc;
+          if (cc + lpe * VPL < nvec) {
+            rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, d, c0, nvec, per, lpe, LPR, vl, EPI, GMASK);
+          }
+        }
+      }
+      rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, d, c0, nvec, per, lpe, LPR, vl, EPI, GMASK);
+    }
+    if (items) {
+      it += warps;
+      if (it < num_items) start_item(); else start_rows();
+    } else {
+      d += G;
+      b = nb, e = ne, src = nsrc, eid = neid;
+      nb = nnb, ne = nne;
+    }
+  }
+#undef EP
+#undef LPR
+#undef SUB
+#undef EPI
+#undef GMASK
+}
+
+// ---- launch -----------------------------------------------------------------------
+template <typename T, int VE, int VPL, int OP, bool WIDE>
+static int launch_rows_kernel(const RowArgs<T>& a, cudaStream_t s) {
+  static int occupancy[64] = {};
+  int dev = 0;
+  APT_CUDA(cudaGetDevice(&dev));
+  int per_sm = dev >= 0 && dev < 64 ? occupancy[dev] : 0;
+  if (per_sm == 0) {
+    APT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm_rows<T, VE, VPL, OP, WIDE>, 256, 0));
+    if (per_sm < 1) per_sm = 1;
+    if (dev >= 0 && dev < 64) occupancy[dev] = per_sm;
+  }
+  const int64_t want = ceil_div(a.num_rows, 256 / (a.split.lpe * a.split.ep));
+  const int64_t wave = (int64_t)kNumSMs * per_sm;
+  APT_LAUNCH((k_spmm_rows<T, VE, VPL, OP, WIDE>), (int)(want < wave ? want : wave), 256, 0, s, a);
+  return APT_OK;
+}
+
+template <typename T, int VE, int OP>
+static int launch_rows_vpl(const RowArgs<T>& a, cudaStream_t s) {
+  // rows of two and four slices a lane are wide ones
+  switch (a.split.vpl) {
+    case 1:
+      return a.split.lpe == 32 ? launch_rows_kernel<T, VE, 1, OP, true>(a, s) : launch_rows_kernel<T, VE, 1, OP, false>(a, s);
+    case 2: return launch_rows_kernel<T, VE, 2, OP, true>(a, s);
+    default: return launch_rows_kernel<T, VE, 4, OP, true>(a, s);
+  }
+}
+
+template <typename T, int OP>
+static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
+  switch (a.split.ve * (int)sizeof(T)) {
+    case 16: return launch_rows_vpl<T, 16 / sizeof(T), OP>(a, s);
+    case 8: return launch_rows_vpl<T, 8 / sizeof(T), OP>(a, s);
+    case 4: return launch_rows_vpl<T, 4 / sizeof(T), OP>(a, s);
+    default: return launch_rows_vpl<T, 1, OP>(a, s);
+  }
+}
+
+// One translation unit per element type (spmm_f32.cu, spmm_bf16.cu, spmm_f16.cu) holds these.
+template <typename T>
+int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
+
+#define APT_DEFINE_SPMM_ROWS(T)                                                                          \
+  template <>                                                                                            \
+  int launch_spmm_rows<T>(int op, const RowArgs<T>& a, cudaStream_t s) {      \
+    switch (op) {                                                                                        \
+      case kCopyU: return launch_rows_ve<T, kCopyU>(a, s);                                \
+      case kCopyE: return launch_rows_ve<T, kCopyE>(a, s);                                \
+      case kUMulE: return launch_rows_ve<T, kUMulE>(a, s);                                \
+      case kUAddE: return launch_rows_ve<T, kUAddE>(a, s);                                \
+      default: return launch_rows_ve<T, kGatSrc>(a, s);                                   \
+    }                                                                                                    \
+  }
+
+// ---- shared by spmm.cu and gat.cu -----------------------------------------------------
+size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws);
+// Groups the edges by output row into ws.order / ws.range / ws.items (three launches behind one memset).
+int launch_group(const int64_t* row, const int64_t* col, int64_t num_edges, SegTable st, int64_t num_rows,
+                 const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s);
+
+}  // namespace apt

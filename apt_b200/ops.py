@@ -16,7 +16,7 @@ from typing import List, Optional, Tuple
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 from ._lib import check, lib
 
 _DTYPE_CODE = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
@@ -796,33 +796,7 @@ def alltoall(input: torch.Tensor, output: torch.Tensor, send_offset: torch.Tenso
 
 # ---------------------------------------------------------------- SpMM / SDDMM
 def _spmm(op, coo_row, coo_col, inp, edata, coo_offset, input_offset, output_offset):
-    ref = inp if inp is not None else edata
-    if ref.dtype not in _DTYPE_CODE:
-        raise RuntimeError(f"spmm: unsupported dtype {ref.dtype}")
-    coo_row = _need_cuda(coo_row, "coo_row")
-    coo_col = _need_cuda(coo_col, "coo_col")
-    coo_offset = _need_cuda(coo_offset, "coo_offset")
-    output_offset = _need_cuda(output_offset, "output_offset")
-    if input_offset is not None:
-        input_offset = _need_cuda(input_offset, "input_offset")
-    ref = _need_cuda(ref, "input", dtype=None)
-    if inp is not None:
-        inp = ref
-    if edata is not None:
-        edata = _need_cuda(edata, "edata", dtype=ref.dtype)
-    out_num = int(output_offset[-1].item())  # host read, as in src/spmm.cc:13
-    num_edges = coo_row.numel()
-    feat_dim = inp.shape[1] if inp is not None else edata.numel() // max(num_edges, 1)
-    # edata may be [E, D], [E, H] or [E, H, 1]: one value per column or per head
-    edim = edata.numel() // num_edges if edata is not None and num_edges else feat_dim
-    out = torch.empty((out_num, feat_dim), dtype=ref.dtype, device=ref.device)
-    nbytes = lib.apt_spmm_workspace_bytes(out_num, num_edges)
-    ws = STATE.workspace("spmm", nbytes)
-    check(lib.apt_spmm_sum(op, _DTYPE_CODE[ref.dtype], _ptr(coo_row), _ptr(coo_col), coo_row.numel(),
-                           _ptr(inp), _ptr(edata), int(edim), int(feat_dim), _ptr(coo_offset),
-                           _ptr(input_offset), _ptr(output_offset), coo_offset.numel() - 1, out_num,
-                           _ptr(out), _ptr(ws), ws.numel(), _stream()))
-    return out
+    return _native.spmm(op, coo_row, coo_col, inp, edata, coo_offset, input_offset, output_offset)
 
 
 def spmm_copy_u_sum(coo_row, coo_col, input, coo_offset, input_offset, output_offset):
@@ -842,31 +816,14 @@ def spmm_u_mul_e_sum(coo_row, coo_col, input, edata, coo_offset, input_offset, o
     return _spmm(3 if ref_quirk_add else 2, coo_row, coo_col, input, edata, coo_offset, input_offset, output_offset)
 
 
-def _sddmm(op, coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset):
-    if lhs.dtype not in _DTYPE_CODE or rhs.dtype != lhs.dtype:
-        raise RuntimeError(f"sddmm: unsupported dtypes {lhs.dtype}/{rhs.dtype}")
-    coo_row = _need_cuda(coo_row, "coo_row")
-    coo_col = _need_cuda(coo_col, "coo_col")
-    lhs = _need_cuda(lhs, "lhs", dtype=None)
-    rhs = _need_cuda(rhs, "rhs", dtype=None)
-    coo_offset = _need_cuda(coo_offset, "coo_offset")
-    lhs_offset = _need_cuda(lhs_offset, "lhs_offset")
-    rhs_offset = _need_cuda(rhs_offset, "rhs_offset")
-    out = torch.empty((coo_row.numel(), lhs.shape[1]), dtype=lhs.dtype, device=lhs.device)
-    check(lib.apt_sddmm(op, _DTYPE_CODE[lhs.dtype], _ptr(coo_row), _ptr(coo_col), coo_row.numel(), _ptr(lhs),
-                        _ptr(rhs), lhs.shape[1], _ptr(coo_offset), _ptr(lhs_offset), _ptr(rhs_offset),
-                        coo_offset.numel() - 1, _ptr(out), _stream()))
-    return out
-
-
 def sddmm_u_add_v(coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset):
     """UAddV, src/sddmm.cc:9-19."""
-    return _sddmm(0, coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset)
+    return _native.sddmm(0, coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset)
 
 
 def sddmm_u_mul_v(coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset):
     """UMulV, src/sddmm.cc:21-31."""
-    return _sddmm(1, coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset)
+    return _native.sddmm(1, coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset)
 
 
 def gat_edge_softmax_sum(coo_row, coo_col, ft, el, er, num_dst: int, negative_slope: float = 0.2,
@@ -905,9 +862,9 @@ def _spmm_single(op, in_index, out_index, inp, edata, edim, feat_dim, num_in, nu
     off = torch.tensor([0, E, 0, num_in, 0, num_out], dtype=torch.int64).to(ref.device, non_blocking=True)
     out = torch.empty((num_out, feat_dim), dtype=ref.dtype, device=ref.device)
     ws = STATE.workspace("spmm", lib.apt_spmm_workspace_bytes(num_out, E))
-    check(lib.apt_spmm_sum(op, _DTYPE_CODE[ref.dtype], _ptr(in_index), _ptr(out_index), E, _ptr(inp), _ptr(edata),
-                           int(edim), int(feat_dim), _ptr(off[0:2]), _ptr(off[2:4]), _ptr(off[4:6]), 1, int(num_out),
-                           _ptr(out), _ptr(ws), ws.numel(), _stream()))
+    check(lib.apt_spmm_sum_known(op, _DTYPE_CODE[ref.dtype], _ptr(in_index), _ptr(out_index), E, _ptr(inp), _ptr(edata),
+                                 int(edim), int(feat_dim), _ptr(off[0:2]), _ptr(off[2:4]), _ptr(off[4:6]), 1,
+                                 int(num_out), 2, 0, _ptr(out), _ptr(ws), ws.numel(), _stream()))
     return out
 
 

@@ -327,6 +327,29 @@ int apt_spmm_sum(int op, int dtype, const int64_t* coo_row,
                  int64_t num_out_rows, void* out, void* workspace,
                  size_t workspace_bytes, void* stream);
 
+/* The same operator for callers that read the number of output rows on the host
+ * anyway (the reference does, src/spmm.cc:13): apt_spmm_probe looks the block over
+ * with one kernel, waits for it and returns
+ *   out[0] = output_offset[num_segments], the number of output rows,
+ *   out[1] = where a row's edges are: 0 every row has out[2] consecutive edges,
+ *            1 grouped by output row with any lengths, 2 anything else,
+ *   out[2] = edges per row (mode 0).
+ * apt_spmm_sum_known then launches only what that block needs: one kernel for
+ * mode 0, which takes no workspace (it may be NULL). Passing mode -1 makes it
+ * apt_spmm_sum. A probe inside a stream capture is refused. */
+int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges,
+                   const int64_t* coo_offset, const int64_t* output_offset,
+                   int num_segments, int64_t* out_rows_mode_fixed /* host[3] */,
+                   void* stream);
+int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row,
+                       const int64_t* coo_col, int64_t num_edges,
+                       const void* input, const void* edata, int64_t edata_dim,
+                       int64_t feat_dim, const int64_t* coo_offset,
+                       const int64_t* input_offset, const int64_t* output_offset,
+                       int num_segments, int64_t num_out_rows, int mode,
+                       int fixed, void* out, void* workspace,
+                       size_t workspace_bytes, void* stream);
+
 /* op: 0 u_add_v, 1 u_mul_v; out has num_edges rows of feat_dim columns. */
 int apt_sddmm(int op, int dtype, const int64_t* coo_row,
               const int64_t* coo_col, int64_t num_edges, const void* lhs,
