@@ -1,514 +1,495 @@
-// Fused GAT edge pipeline over one sampled block: forward and the edge part of the backward.
+// Fused GAT edge pipeline over one sampled block whose edges are grouped by destination. For every destination d
+// with its edges e (src_e -> d) and every head h
+//   s_e = leaky_relu(el[src_e, h] + er[d, h]),  a_e = softmax of s over d's edges,
+//   out[d, h, :] = sum_e a_e ft[src_e, h, :]
+// (python/npc/model/gatconv.py:113-124), and in the backward, with g = grad_out[d, h, :],
+//   dot_e = <g, ft[src_e, h, :]>,  t = sum_e a_e dot_e,
+//   grad_s_e = a_e (dot_e - t) (el + er > 0 ? 1 : slope),  grad_er[d, h] = sum_e grad_s_e,
+//   grad_ft[s, h, :] = sum over the edges out of s of a_e g,  grad_el[s, h] = sum of grad_s_e.
+//
+// The work per edge and head is a few scalars, the work per edge and column is a gather of rows; they want opposite
+// kernels and are kept apart, with fp32 weights per edge and head between them (16 MB for a million edges of four
+// heads, which stay in L2):
+//
+//   k_gat_ranges    where each destination's edges are
+//   k_gat_weights   one thread per destination and head: scores and softmax. Full occupancy hides the two dependent
+//                   loads of a score; any number of edges and heads.
+//   row kernel      the weighted sum is the SpMM's row kernel (kUMulW), any head width
+//   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination. The four partial dots of a
+//                   lane are reduced together: each step halves the values a lane keeps, log2(lph) + 1 shuffles
+//                   for four edges instead of 4 log2(lph).
+//   k_gat_scores    backward: t, grad_s and grad_er, one thread per destination and head
+//   row kernel      both sums over the source side in one walk (kGatSrc) behind one counting sort by source
+//
+// One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
+// and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
+// kernels take 18 + 88 us. Backward of that block: 18 (saved after a forward) + 101 + 28, then 45 us of sort and 158 us
+// for both source-side sums, where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
+
+#include <algorithm>
 
 #include "spmm_rows.cuh"
 
 namespace apt {
 
-struct GatWs {
-  int32_t* range;   // [num_dst + 1] first edge of every destination
-  int32_t* flags;   // [1] 1 when the edges are not grouped by destination
-};
+__device__ __forceinline__ float leaky(float x, float slope) { return x > 0.f ? x : x * slope; }
 
-static bool gat_layout(int64_t num_dst, char* base, size_t bytes, GatWs* ws) {
-  SpmmWs w;
-  if (bytes < spmm_layout(num_dst, 0, base, &w)) return false;
-  ws->range = (int32_t*)w.range;
-  ws->flags = w.num_items;
-  return true;
+// Sum over groups of n lanes (a power of two).
+__device__ __forceinline__ float group_sum(float v, int n) {
+  for (int o = n >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
+// First and last edge of every destination; *none when the edges are not grouped (nothing then belongs to anybody).
 __global__ void __launch_bounds__(256)
-k_edge_ranges_single(const int64_t* __restrict__ col, int64_t E, int64_t num_out_rows, GatWs ws) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* __restrict__ range, int32_t* none, int32_t* status) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   bool bad = false;
-  for (; e < E; e += stride) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
     const int64_t d = col[e];
     const int64_t prev = e > 0 ? col[e - 1] : (int64_t)-1;
-    if (d < prev || d < 0 || d >= num_out_rows) {
+    if (d < prev || d < 0 || d >= num_dst) {
       bad = true;
       continue;
     }
-    for (int64_t t = prev + 1; t <= d; ++t) ws.range[t] = (int32_t)e;
-    if (e == E - 1)
-      for (int64_t t = d + 1; t <= num_out_rows; ++t) ws.range[t] = (int32_t)E;
-  }
-  if (bad) atomicOr(ws.flags, 1);
-}
-
-// ---- fused GAT edge pipeline ---------------------------------------------------------
-// For every destination row d with its edges e (src_e -> d) and every head h:
-//   s_e = leaky_relu(el[src_e, h] + er[d, h]);  a_e = softmax over the edges of d;
-//   out[d, h, :] = sum_e a_e * ft[src_e, h, :]
-// which is u_add_v -> leaky_relu -> edge_softmax -> u_mul_e + sum in one pass
-// over a grouped block (python/npc/model/gatconv.py:113-124). One lane group per
-// destination row as in k_spmm_rows; scores are recomputed per lane (a block has
-// at most a few dozen edges per row), sums stay in fp32 registers.
-template <typename T, int VE>
-__global__ void __launch_bounds__(256)
-k_gat_rows(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el,
-           const T* __restrict__ er, int num_heads, int64_t head_dim, float slope,
-           int64_t num_dst, GatWs ws, T* __restrict__ out, T* __restrict__ attn,
-           int group, int32_t* status) {
-  const bool unsorted = *ws.flags != 0;
-  if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, APT_FLAG_NOT_GROUPED);
-  const int sub = threadIdx.x % group;
-  const int64_t rows_per_block = blockDim.x / group;
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  const int64_t nvec = feat_dim / VE;
-  int64_t d = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / group;
-  const int64_t stride = (int64_t)gridDim.x * rows_per_block;
-  for (; d < num_dst; d += stride) {
-    const int64_t e0 = unsorted ? 0 : ws.range[d];
-    const int64_t e1 = unsorted ? 0 : ws.range[d + 1];
-    for (int64_t c = sub; c < nvec; c += group) {
-      const int h = (int)((c * VE) / head_dim);
-      const float r = Elem<T>::to_f(er[d * num_heads + h]);
-      float m = -INFINITY;
-      for (int64_t e = e0; e < e1; ++e) {
-        float s = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-        s = s > 0.f ? s : s * slope;
-        m = fmaxf(m, s);
-      }
-      float denom = 0.f;
-      for (int64_t e = e0; e < e1; ++e) {
-        float s = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-        s = s > 0.f ? s : s * slope;
-        denom += expf(s - m);
-      }
-      const float inv = denom > 0.f ? 1.f / denom : 0.f;
-      float acc[VE];
-#pragma unroll
-      for (int t = 0; t < VE; ++t) acc[t] = 0.f;
-      const bool writes_attn = attn != nullptr && (c * VE) % head_dim == 0;
-      for (int64_t e = e0; e < e1; ++e) {
-        const int64_t src = row[e];
-        float s = Elem<T>::to_f(el[src * num_heads + h]) + r;
-        s = s > 0.f ? s : s * slope;
-        const float a = expf(s - m) * inv;
-        if (writes_attn) attn[e * num_heads + h] = Elem<T>::from_f(a);
-        const Pack<T, VE> p = load_pack<T, VE>(ft + src * feat_dim + c * VE);
-#pragma unroll
-        for (int t = 0; t < VE; ++t) acc[t] += a * Elem<T>::to_f(p.v[t]);
-      }
-      Pack<T, VE> o;
-#pragma unroll
-      for (int t = 0; t < VE; ++t) o.v[t] = Elem<T>::from_f(acc[t]);
-      store_pack<T, VE>(out + d * feat_dim + c * VE, o);
+    if (d != prev) {
+      if (prev >= 0) range[prev].y = (int)e;
+      for (int64_t t = prev + 1; t < d; ++t) range[t] = make_int2(0, 0);
+      range[d].x = (int)e;
     }
+    if (e == E - 1) {
+      range[d].y = (int)E;
+      for (int64_t t = d + 1; t < num_dst; ++t) range[t] = make_int2(0, 0);
+    }
+  }
+  if (bad) {
+    atomicOr(none, 1);
+    atomicOr(status, APT_FLAG_NOT_GROUPED);
   }
 }
 
-// Fast path of the same operator for wide rows (one warp per destination row), up to
-// kGatHeads heads and up to 32 edges per row (fixed-fanout blocks): lane j computes the scores
-// of edge j for all heads once (one exp per edge and head instead of two per edge and lane),
-// the softmax statistics are warp reductions, the attention values and source ids wait in
-// shared memory, and the weighted sum then walks the edges with one shared-memory read each.
-// Rows with more than 32 edges take the recomputing walk of k_gat_rows.
-constexpr int kGatHeads = 8;
-
-template <typename T, int VE>
-__global__ void __launch_bounds__(256)
-k_gat_rows_warp(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el,
-                const T* __restrict__ er, int num_heads, int64_t head_dim, float slope,
-                int64_t num_dst, GatWs ws, T* __restrict__ out, T* __restrict__ attn, int32_t* status) {
-  __shared__ float a_sh[8][32][kGatHeads];
-  __shared__ int64_t src_sh[8][32];
-  const bool unsorted = *ws.flags != 0;
-  if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, APT_FLAG_NOT_GROUPED);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  const int64_t nvec = feat_dim / VE;
-  int64_t d = (int64_t)blockIdx.x * 8 + warp;
-  const int64_t stride = (int64_t)gridDim.x * 8;
-  for (; d < num_dst; d += stride) {
-    const int64_t e0 = unsorted ? 0 : ws.range[d];
-    const int64_t e1 = unsorted ? 0 : ws.range[d + 1];
-    const int deg = (int)(e1 - e0);
-    if (deg <= 32) {
-      const bool has = lane < deg;
-      const int64_t src = has ? row[e0 + lane] : 0;
-      src_sh[warp][lane] = src;
-#pragma unroll
-      for (int h = 0; h < kGatHeads; ++h) {
-        if (h < num_heads) {
-          float sc = -INFINITY;
-          if (has) {
-            sc = Elem<T>::to_f(el[src * num_heads + h]) + Elem<T>::to_f(er[d * num_heads + h]);
-            sc = sc > 0.f ? sc : sc * slope;
-          }
-          float m = sc;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-          const float p = has ? expf(sc - m) : 0.f;
-          float sum = p;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-          const float a = sum > 0.f ? p / sum : 0.f;
-          a_sh[warp][lane][h] = a;
-          if (has && attn) attn[(e0 + lane) * num_heads + h] = Elem<T>::from_f(a);
-        }
-      }
-      __syncwarp();
-      for (int64_t c = lane; c < nvec; c += 32) {
-        const int h = (int)((c * VE) / head_dim);
-        float acc[VE];
-#pragma unroll
-        for (int t = 0; t < VE; ++t) acc[t] = 0.f;
-#pragma unroll 4
-        for (int j = 0; j < deg; ++j) {
-          const float a = a_sh[warp][j][h];
-          const Pack<T, VE> p = load_pack<T, VE>(ft + src_sh[warp][j] * feat_dim + c * VE);
-#pragma unroll
-          for (int t = 0; t < VE; ++t) acc[t] += a * Elem<T>::to_f(p.v[t]);
-        }
-        Pack<T, VE> o;
-#pragma unroll
-        for (int t = 0; t < VE; ++t) o.v[t] = Elem<T>::from_f(acc[t]);
-        store_pack<T, VE>(out + d * feat_dim + c * VE, o);
-      }
-      __syncwarp();
-      continue;
-    }
-    for (int64_t c = lane; c < nvec; c += 32) {
-      const int h = (int)((c * VE) / head_dim);
-      const float r = Elem<T>::to_f(er[d * num_heads + h]);
-      float m = -INFINITY;
-      for (int64_t e = e0; e < e1; ++e) {
-        float sc = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-        sc = sc > 0.f ? sc : sc * slope;
-        m = fmaxf(m, sc);
-      }
-      float denom = 0.f;
-      for (int64_t e = e0; e < e1; ++e) {
-        float sc = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-        sc = sc > 0.f ? sc : sc * slope;
-        denom += expf(sc - m);
-      }
-      const float inv = denom > 0.f ? 1.f / denom : 0.f;
-      float acc[VE];
-#pragma unroll
-      for (int t = 0; t < VE; ++t) acc[t] = 0.f;
-      const bool writes_attn = attn != nullptr && (c * VE) % head_dim == 0;
-      for (int64_t e = e0; e < e1; ++e) {
-        const int64_t src = row[e];
-        float sc = Elem<T>::to_f(el[src * num_heads + h]) + r;
-        sc = sc > 0.f ? sc : sc * slope;
-        const float a = expf(sc - m) * inv;
-        if (writes_attn) attn[e * num_heads + h] = Elem<T>::from_f(a);
-        const Pack<T, VE> p = load_pack<T, VE>(ft + src * feat_dim + c * VE);
-#pragma unroll
-        for (int t = 0; t < VE; ++t) acc[t] += a * Elem<T>::to_f(p.v[t]);
-      }
-      Pack<T, VE> o;
-#pragma unroll
-      for (int t = 0; t < VE; ++t) o.v[t] = Elem<T>::from_f(acc[t]);
-      store_pack<T, VE>(out + d * feat_dim + c * VE, o);
-    }
-  }
-}
-
+// Attention weights. K edges' loads are in flight; a destination of at most K edges keeps its scores in registers.
 template <typename T>
-static int launch_gat(bool vec, const int64_t* row, const void* ft, const void* el, const void* er,
-                      int num_heads, int64_t head_dim, float slope, int64_t num_dst, GatWs ws, void* out,
-                      void* attn, int32_t* status, cudaStream_t s) {
-  constexpr int VE = 16 / sizeof(T);
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  ProfScope prof("gat_rows", s);
-  if (vec && feat_dim / VE > 16 && num_heads <= kGatHeads) {
-    const int grid = wave_grid(ceil_div(num_dst, 8), 8);
-    APT_LAUNCH((k_gat_rows_warp<T, VE>), grid, 256, 0, s, row, (const T*)ft, (const T*)el, (const T*)er, num_heads,
-               head_dim, slope, num_dst, ws, (T*)out, (T*)attn, status);
-  } else if (vec) {
-    const int group = pow2_ge(feat_dim / VE);
-    const int grid = wave_grid(ceil_div(num_dst, 256 / group), 8);
-    APT_LAUNCH((k_gat_rows<T, VE>), grid, 256, 0, s, row, (const T*)ft, (const T*)el, (const T*)er, num_heads,
-               head_dim, slope, num_dst, ws, (T*)out, (T*)attn, group, status);
-  } else {
-    const int group = pow2_ge(feat_dim);
-    const int grid = wave_grid(ceil_div(num_dst, 256 / group), 8);
-    APT_LAUNCH((k_gat_rows<T, 1>), grid, 256, 0, s, row, (const T*)ft, (const T*)el, (const T*)er, num_heads,
-               head_dim, slope, num_dst, ws, (T*)out, (T*)attn, group, status);
+__global__ void __launch_bounds__(256)
+k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
+              int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ weight,
+              T* __restrict__ attn) {
+  constexpr int K = 16;
+  if (*none != 0) return;
+  const int64_t total = num_dst * num_heads, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
+    const int2 r = range[d];
+    const float bias = Elem<T>::to_f(er[i]);
+    const int deg = r.y - r.x;
+    float s[K], m = -INFINITY, sum = 0.f;
+    auto score = [&](int e) { return leaky(Elem<T>::to_f(el[row[e] * num_heads + h]) + bias, slope); };
+    if (deg <= K) {
+      uint32_t src[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) src[k] = k < deg ? (uint32_t)row[r.x + k] : 0u;
+#pragma unroll
+      for (int k = 0; k < K; ++k) s[k] = k < deg ? Elem<T>::to_f(el[(int64_t)src[k] * num_heads + h]) : 0.f;
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (k < deg) {
+          s[k] = leaky(s[k] + bias, slope);
+          m = fmaxf(m, s[k]);
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (k < deg) {
+          s[k] = expf(s[k] - m);
+          sum += s[k];
+        }
+    } else {
+      for (int e = r.x; e < r.y; ++e) m = fmaxf(m, score(e));
+      for (int e = r.x; e < r.y; ++e) sum += expf(score(e) - m);
+    }
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    auto put = [&](int e, float w) {
+      const int64_t o = (int64_t)e * num_heads + h;
+      weight[o] = w;
+      if (attn) attn[o] = Elem<T>::from_f(w);
+    };
+    if (deg <= K) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (k < deg) put(r.x + k, s[k] * inv);
+    } else {
+      for (int e = r.x; e < r.y; ++e) put(e, expf(score(e) - m) * inv);
+    }
   }
-  return APT_OK;
 }
 
-// ---- backward of the fused GAT edge pipeline: the edge part ---------------------------
-// Per destination row d and head h (s_e, a_e as in k_gat_rows, g = grad_out[d, h, :]):
-//   dot_e = <g, ft[src_e, h, :]>;  t = sum_e a_e dot_e;
-//   grad_s_e = a_e (dot_e - t) * (s_e > 0 ? 1 : slope);  grad_er[d, h] = sum_e grad_s_e
-// attn[e, h] = a_e and grad_score[e, h] = grad_s_e go out per edge; the sums over the
-// source side (grad_ft = sum a_e g, grad_el = sum grad_s_e) are SpMM calls in the
-// reverse direction. The lanes of one head (lanes_per_head of them, a power of two
-// inside the lane group) each hold a slice of g and of the ft row and meet in a
-// butterfly of shuffles for the dot product.
+// Dots of the destination's gradient with its edges' rows. lph lanes to a head's slices, hpp heads side by side, ep
+// edges side by side; heads and slices beyond that are walked in blocks.
 template <typename T, int VE>
-__global__ void __launch_bounds__(256)
-k_gat_bwd_rows(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el,
-               const T* __restrict__ er, const T* __restrict__ grad_out, int num_heads, int64_t head_dim,
-               float slope, int64_t num_dst, GatWs ws, T* __restrict__ attn, T* __restrict__ grad_score,
-               T* __restrict__ grad_er, int group, int lanes_per_head, int32_t* status,
-               int64_t skip_up_to /* rows with at most this many edges belong to k_gat_bwd_warp */) {
-  const bool unsorted = *ws.flags != 0;
-  if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, APT_FLAG_NOT_GROUPED);
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % group;
-  const unsigned gmask = group == 32 ? 0xffffffffu : (((1u << group) - 1u) << (lane - sub));
-  const int64_t rows_per_block = blockDim.x / group;
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  const int64_t nvec = feat_dim / VE;
-  int64_t d = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / group;
-  const int64_t stride = (int64_t)gridDim.x * rows_per_block;
-  for (; d < num_dst; d += stride) {
-    const int64_t e0 = unsorted ? 0 : ws.range[d];
-    const int64_t e1 = unsorted ? 0 : ws.range[d + 1];
-    if (e1 - e0 <= skip_up_to) continue;
-    for (int64_t c0 = 0; c0 < nvec; c0 += group) {
-      const int64_t c = c0 + sub;
-      const bool live = c < nvec;
-      const int h = live ? (int)((c * VE) / head_dim) : 0;
-      const bool leader = live && (c * VE) % head_dim == 0;
-      const float r = Elem<T>::to_f(er[d * num_heads + h]);
-      float m = -INFINITY;
-      for (int64_t e = e0; e < e1; ++e) {
-        float s = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-        s = s > 0.f ? s : s * slope;
-        m = fmaxf(m, s);
-      }
-      float denom = 0.f;
-      for (int64_t e = e0; e < e1; ++e) {
-        float s = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-        s = s > 0.f ? s : s * slope;
-        denom += expf(s - m);
-      }
-      const float inv = denom > 0.f ? 1.f / denom : 0.f;
-      float g[VE];
+__global__ void __launch_bounds__(256, 3)
+k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ grad_out, int num_heads, int head_dim,
+           int64_t num_dst_, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ dots, int lph,
+           int hpp) {
+  if (*none != 0) return;
+  const int lane = threadIdx.x & 31, G = gridDim.x * 8, num_dst = (int)num_dst_;
+  const int lpe = lph * hpp, ep = 32 / lpe;
+  const int epi = lane / lpe, rh = (lane & (lpe - 1)) / lph, p = lane & (lph - 1);
+  const int nvh = head_dim / VE;
+  const uint32_t row_bytes = (uint32_t)((int64_t)num_heads * head_dim * sizeof(T));
+  int d = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (d >= num_dst) return;
+  int2 r = range[d], nr = make_int2(0, 0);
+  // lanes past the last edge hold its source too, so that a round may load past the end
+  uint32_t src = r.x < r.y ? (uint32_t)row[min(r.x + lane, r.y - 1)] : 0u, nsrc = 0;
+  if (d + G < num_dst) nr = range[d + G];
+  for (; d < num_dst; d += G) {
+    int2 nnr = make_int2(0, 0);
+    if (nr.x < nr.y) nsrc = (uint32_t)row[min(nr.x + lane, nr.y - 1)];
+    if (d + 2 * G < num_dst) nnr = range[d + 2 * G];
+    for (int h0 = 0; h0 < num_heads; h0 += hpp) {
+      const int h = h0 + rh;
+      const bool rows = h < num_heads;
+      // lanes without a slice read one that exists and contribute zero
+      const int64_t col = (int64_t)(rows ? h : h0) * head_dim;
+      const T* const grad = grad_out + (int64_t)d * num_heads * head_dim + col;
+      Raw<T, VE> g;
+      int at = 0;
+      auto block = [&](int c0) {
+        at = min(c0 + p, nvh - 1) * VE;
+        g = load_raw<T, VE>(grad + at);
+        if (c0 + p >= nvh) {
 #pragma unroll
-      for (int t = 0; t < VE; ++t) g[t] = 0.f;
-      if (live) {
-        const Pack<T, VE> p = load_pack<T, VE>(grad_out + d * feat_dim + c * VE);
+          for (int q = 0; q < (int)(sizeof(g.w) / 4); ++q) g.w[q] = 0u;
+        }
+      };
+      block(0);
+#pragma unroll 1
+      for (int base = r.x; base < r.y; base += 32) {
+        const int cnt = min(32, r.y - base);
+        uint32_t my_src = src;
+        if (base != r.x) my_src = (uint32_t)row[min(base + lane, r.y - 1)];
+#pragma unroll 1
+        for (int j0 = 0; j0 < cnt; j0 += ep * 4) {
+          float dt[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+          for (int c0 = 0; c0 < nvh; c0 += lph) {
+            if (nvh > lph) block(c0);
+            const T* const lane_ft = ft + col + at;
+            Raw<T, VE> v[4];
 #pragma unroll
-        for (int t = 0; t < VE; ++t) g[t] = Elem<T>::to_f(p.v[t]);
-      }
-      // first walk: t = sum_e a_e dot_e; second walk: the per-edge results
-      float tsum = 0.f, ger = 0.f;
-      for (int pass = 0; pass < 2; ++pass) {
-        for (int64_t e = e0; e < e1; ++e) {
-          const int64_t src = row[e];
-          const float raw = Elem<T>::to_f(el[src * num_heads + h]) + r;
-          const float s = raw > 0.f ? raw : raw * slope;
-          const float a = expf(s - m) * inv;
-          float dot = 0.f;
-          if (live) {
-            const Pack<T, VE> p = load_pack<T, VE>(ft + src * feat_dim + c * VE);
+            for (int u = 0; u < 4; ++u)
+              v[u] = load_raw<T, VE>(at_row(lane_ft, __shfl_sync(0xffffffffu, my_src, (j0 + u * ep + epi) & 31), row_bytes));
 #pragma unroll
-            for (int t = 0; t < VE; ++t) dot += g[t] * Elem<T>::to_f(p.v[t]);
+            for (int u = 0; u < 4; ++u) {
+              Acc<VE> acc;
+              acc.zero();
+              acc.fma(g, v[u]);
+              F2 pair = acc.p[0];
+#pragma unroll
+              for (int q = 1; q < Acc<VE>::P; ++q) pair = f2_add(pair, acc.p[q]);
+              float lo, hi;
+              f2_unpack(pair, lo, hi);
+              dt[u] += VE > 1 ? lo + hi : lo;
+            }
           }
-          for (int o = lanes_per_head >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(gmask, dot, o, group);
-          if (pass == 0) {
-            tsum += a * dot;
+          float* const out = dots + (int64_t)(base + j0 + epi) * num_heads + h;
+          const int left = cnt - j0 - epi;       // edges of the chunk from this lane's first one on
+          if (lph >= 4) {
+            // this lane ends up with the dot of one of the four edges
+            const bool hi = p & (lph >> 1), lo = p & (lph >> 2);
+            const float b0 = (hi ? dt[2] : dt[0]) + __shfl_xor_sync(0xffffffffu, hi ? dt[0] : dt[2], lph >> 1);
+            const float b1 = (hi ? dt[3] : dt[1]) + __shfl_xor_sync(0xffffffffu, hi ? dt[1] : dt[3], lph >> 1);
+            const float v = group_sum((lo ? b1 : b0) + __shfl_xor_sync(0xffffffffu, lo ? b0 : b1, lph >> 2), lph >> 2);
+            const int u = ((hi ? 2 : 0) + (lo ? 1 : 0)) * ep;
+            if (rows && u < left && (p & ((lph >> 2) - 1)) == 0) out[(int64_t)u * num_heads] = v;
           } else {
-            const float gs = a * (dot - tsum) * (raw > 0.f ? 1.f : slope);
-            ger += gs;
-            if (leader) {
-              attn[e * num_heads + h] = Elem<T>::from_f(a);
-              grad_score[e * num_heads + h] = Elem<T>::from_f(gs);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              if (lph == 2) dt[u] += __shfl_xor_sync(0xffffffffu, dt[u], 1);
+              if (rows && p == 0 && u * ep < left) out[(int64_t)u * ep * num_heads] = dt[u];
             }
           }
         }
       }
-      if (leader) grad_er[d * num_heads + h] = Elem<T>::from_f(ger);
     }
+    r = nr, src = nsrc, nr = nnr;
   }
 }
 
-// Wide rows with at most 32 edges (fixed-fanout blocks), one warp per destination: lane j
-// scores edge j for all heads once, the lanes then walk the edges ONCE over ft (each lane its
-// slice of grad_out and of the row, the lanes of a head meeting in a shuffle butterfly) and
-// leave <grad_out, ft> per edge and head in shared memory, and lane j finishes edge j.
-template <typename T, int VE>
-__global__ void __launch_bounds__(256)
-k_gat_bwd_warp(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el,
-               const T* __restrict__ er, const T* __restrict__ grad_out, int num_heads, int64_t head_dim,
-               float slope, int64_t num_dst, GatWs ws, T* __restrict__ attn, T* __restrict__ grad_score,
-               T* __restrict__ grad_er, int lanes_per_head, int32_t* status) {
-  __shared__ float a_sh[8][32][kGatHeads], fac_sh[8][32][kGatHeads], dot_sh[8][32][kGatHeads];
-  __shared__ int64_t src_sh[8][32];
-  const bool unsorted = *ws.flags != 0;
-  if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, APT_FLAG_NOT_GROUPED);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  const int64_t nvec = feat_dim / VE;
-  int64_t d = (int64_t)blockIdx.x * 8 + warp;
-  const int64_t stride = (int64_t)gridDim.x * 8;
-  for (; d < num_dst; d += stride) {
-    const int64_t e0 = unsorted ? 0 : ws.range[d];
-    const int64_t e1 = unsorted ? 0 : ws.range[d + 1];
-    const int deg = (int)(e1 - e0);
-    if (deg > 32) continue;            // left to k_gat_bwd_rows
-    const bool has = lane < deg;
-    const int64_t src = has ? row[e0 + lane] : 0;
-    src_sh[warp][lane] = src;
-#pragma unroll
-    for (int h = 0; h < kGatHeads; ++h) {
-      if (h < num_heads) {
-        float raw = 0.f, sc = -INFINITY;
-        if (has) {
-          raw = Elem<T>::to_f(el[src * num_heads + h]) + Elem<T>::to_f(er[d * num_heads + h]);
-          sc = raw > 0.f ? raw : raw * slope;
-        }
-        float m = sc;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const float p = has ? expf(sc - m) : 0.f;
-        float sum = p;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        a_sh[warp][lane][h] = sum > 0.f ? p / sum : 0.f;
-        fac_sh[warp][lane][h] = raw > 0.f ? 1.f : slope;
-      }
-    }
-    __syncwarp();
-    for (int64_t c0 = 0; c0 < nvec; c0 += 32) {
-      const int64_t c = c0 + lane;
-      const bool live = c < nvec;
-      const int h = live ? (int)((c * VE) / head_dim) : 0;
-      const bool leader = live && (c * VE) % head_dim == 0;
-      float g[VE];
-#pragma unroll
-      for (int t = 0; t < VE; ++t) g[t] = 0.f;
-      if (live) {
-        const Pack<T, VE> p = load_pack<T, VE>(grad_out + d * feat_dim + c * VE);
-#pragma unroll
-        for (int t = 0; t < VE; ++t) g[t] = Elem<T>::to_f(p.v[t]);
-      }
-      for (int j = 0; j < deg; ++j) {
-        float dot = 0.f;
-        if (live) {
-          const Pack<T, VE> p = load_pack<T, VE>(ft + src_sh[warp][j] * feat_dim + c * VE);
-#pragma unroll
-          for (int t = 0; t < VE; ++t) dot += g[t] * Elem<T>::to_f(p.v[t]);
-        }
-        for (int o = lanes_per_head >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (leader) dot_sh[warp][j][h] = dot;
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int h = 0; h < kGatHeads; ++h) {
-      if (h < num_heads) {
-        const float a = has ? a_sh[warp][lane][h] : 0.f;
-        const float dot = has ? dot_sh[warp][lane][h] : 0.f;
-        float t = a * dot;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        const float gs = has ? a * (dot - t) * fac_sh[warp][lane][h] : 0.f;
-        if (has) {
-          attn[(e0 + lane) * num_heads + h] = Elem<T>::from_f(a);
-          grad_score[(e0 + lane) * num_heads + h] = Elem<T>::from_f(gs);
-        }
-        float ger = gs;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ger += __shfl_xor_sync(0xffffffffu, ger, o);
-        if (lane == 0) grad_er[d * num_heads + h] = Elem<T>::from_f(ger);
-      }
-    }
-    __syncwarp();
-  }
-}
-
-// Any head width: one thread per (destination, head), everything in turn.
+// Score gradients. Writes (weight, gradient) pairs for the source side, or both in T for callers of the edge part alone.
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_gat_bwd_generic(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el,
-                  const T* __restrict__ er, const T* __restrict__ grad_out, int num_heads, int64_t head_dim,
-                  float slope, int64_t num_dst, GatWs ws, T* __restrict__ attn, T* __restrict__ grad_score,
-                  T* __restrict__ grad_er, int32_t* status) {
-  const bool unsorted = *ws.flags != 0;
-  if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, APT_FLAG_NOT_GROUPED);
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  const int64_t total = num_dst * num_heads;
+k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
+             int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
+             const float* __restrict__ weight, const float* __restrict__ dots, float2* __restrict__ pair, T* __restrict__ attn,
+             T* __restrict__ grad_score, T* __restrict__ grad_er) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  auto put = [&](int64_t o, float w, float gs) {
+    if (pair) {
+      pair[o] = make_float2(w, gs);
+    } else {
+      attn[o] = Elem<T>::from_f(w);
+      grad_score[o] = Elem<T>::from_f(gs);
+    }
+  };
+  const bool empty = *none != 0;
+  if (empty)
+    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += stride) put(o, 0.f, 0.f);
+  const int64_t total = num_dst * num_heads;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int64_t d = i / num_heads;
-    const int h = (int)(i - d * num_heads);
-    const int64_t e0 = unsorted ? 0 : ws.range[d];
-    const int64_t e1 = unsorted ? 0 : ws.range[d + 1];
-    const float r = Elem<T>::to_f(er[d * num_heads + h]);
-    float m = -INFINITY;
-    for (int64_t e = e0; e < e1; ++e) {
-      float s = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-      s = s > 0.f ? s : s * slope;
-      m = fmaxf(m, s);
+    const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
+    const int2 r = empty ? make_int2(0, 0) : range[d];
+    const float bias = Elem<T>::to_f(er[i]);
+    float t = 0.f, ger = 0.f;
+    // two short walks rather than one that keeps everything in registers: the second finds its values in L1 and L2
+#pragma unroll 8
+    for (int e = r.x; e < r.y; ++e) {
+      const int64_t o = (int64_t)e * num_heads + h;
+      t += weight[o] * dots[o];
     }
-    float denom = 0.f;
-    for (int64_t e = e0; e < e1; ++e) {
-      float s = Elem<T>::to_f(el[row[e] * num_heads + h]) + r;
-      s = s > 0.f ? s : s * slope;
-      denom += expf(s - m);
+#pragma unroll 4
+    for (int e = r.x; e < r.y; ++e) {
+      const int64_t o = (int64_t)e * num_heads + h;
+      const float w = weight[o];
+      const float gs = w * (dots[o] - t) * (Elem<T>::to_f(el[row[e] * num_heads + h]) + bias > 0.f ? 1.f : slope);
+      ger += gs;
+      put(o, w, gs);
     }
-    const float inv = denom > 0.f ? 1.f / denom : 0.f;
-    const T* g = grad_out + d * feat_dim + (int64_t)h * head_dim;
-    float tsum = 0.f, ger = 0.f;
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int64_t e = e0; e < e1; ++e) {
-        const int64_t src = row[e];
-        const float raw = Elem<T>::to_f(el[src * num_heads + h]) + r;
-        const float s = raw > 0.f ? raw : raw * slope;
-        const float a = expf(s - m) * inv;
-        const T* f = ft + src * feat_dim + (int64_t)h * head_dim;
-        float dot = 0.f;
-        for (int64_t k = 0; k < head_dim; ++k) dot += Elem<T>::to_f(g[k]) * Elem<T>::to_f(f[k]);
-        if (pass == 0) {
-          tsum += a * dot;
-        } else {
-          const float gs = a * (dot - tsum) * (raw > 0.f ? 1.f : slope);
-          ger += gs;
-          attn[e * num_heads + h] = Elem<T>::from_f(a);
-          grad_score[e * num_heads + h] = Elem<T>::from_f(gs);
-        }
-      }
-    }
-    grad_er[d * num_heads + h] = Elem<T>::from_f(ger);
+    grad_er[i] = Elem<T>::from_f(ger);
   }
 }
 
-template <typename T>
-static int launch_gat_bwd(bool vec, const int64_t* row, const void* ft, const void* el, const void* er,
-                          const void* grad_out, int num_heads, int64_t head_dim, float slope, int64_t num_dst,
-                          GatWs ws, void* attn, void* grad_score, void* grad_er, int32_t* status, cudaStream_t s) {
-  constexpr int VE = 16 / sizeof(T);
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  ProfScope prof("gat_bwd_rows", s);
-  const int64_t lph = head_dim / VE;                   // lanes per head when rows are read as 16-byte vectors
-  const bool pow2 = lph >= 1 && lph <= 32 && (lph & (lph - 1)) == 0;
-  if (vec && pow2) {
-    const int group = pow2_ge(feat_dim / VE);
-    if (group % lph == 0) {
-      int64_t skip = -1;
-      if (group == 32 && num_heads <= kGatHeads) {
-        // rows of up to 32 edges: one warp per row; the kernel after it takes the longer rows
-        const int grid_w = wave_grid(ceil_div(num_dst, 8), 8);
-        APT_LAUNCH((k_gat_bwd_warp<T, VE>), grid_w, 256, 0, s, row, (const T*)ft, (const T*)el, (const T*)er,
-                   (const T*)grad_out, num_heads, head_dim, slope, num_dst, ws, (T*)attn, (T*)grad_score,
-                   (T*)grad_er, (int)lph, status);
-        skip = 32;
-      }
-      const int grid = wave_grid(ceil_div(num_dst, 256 / group), 8);
-      APT_LAUNCH((k_gat_bwd_rows<T, VE>), grid, 256, 0, s, row, (const T*)ft, (const T*)el, (const T*)er,
-                 (const T*)grad_out, num_heads, head_dim, slope, num_dst, ws, (T*)attn, (T*)grad_score, (T*)grad_er,
-                 group, (int)lph, status, skip);
-      return APT_OK;
-    }
+// ---- host side ----------------------------------------------------------------------
+static size_t elem_size(int dtype) { return dtype == APT_F32 ? 4 : 2; }
+
+// What the forward leaves for the backward: the ranges and the weights.
+struct GatEdges {
+  int32_t* none;    // [1]
+  int2* range;      // [num_dst]
+  float* weight;    // [E][heads]
+};
+static size_t gat_edges_layout(int64_t num_dst, int64_t E, int H, char* base, GatEdges* g) {
+  const size_t o_range = 256;
+  const size_t o_weight = o_range + align_up((size_t)(num_dst > 0 ? num_dst : 1) * 8, 256);
+  if (g) {
+    g->none = (int32_t*)base;
+    g->range = (int2*)(base + o_range);
+    g->weight = (float*)(base + o_weight);
   }
-  const int grid = wave_grid(ceil_div(num_dst * num_heads, 256), 8);
-  APT_LAUNCH((k_gat_bwd_generic<T>), grid, 256, 0, s, row, (const T*)ft, (const T*)el, (const T*)er,
-             (const T*)grad_out, num_heads, head_dim, slope, num_dst, ws, (T*)attn, (T*)grad_score, (T*)grad_er, status);
+  return o_weight + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
+}
+
+struct GatBwdWs {
+  SpmmWs sort;
+  float* dots;      // [E][heads]
+  float2* pair;     // [E][heads]
+};
+static size_t gat_bwd_layout(int64_t num_src, int64_t E, int H, char* base, GatBwdWs* ws) {
+  const size_t o_dots = spmm_layout(num_src, E, base, ws ? &ws->sort : nullptr);
+  const size_t o_pair = o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
+  if (ws) {
+    ws->dots = (float*)(base + o_dots);
+    ws->pair = (float2*)(base + o_pair);
+  }
+  return o_pair + align_up((size_t)(E > 0 ? E : 1) * H * 8, 256);
+}
+
+struct GatProblem {
+  const int64_t* row;
+  const int64_t* col;
+  int64_t E;
+  const void *ft, *el, *er, *grad_out;
+  int H;
+  int64_t Dh;
+  float slope;
+  int64_t num_dst;
+  int32_t* status;
+};
+
+static int gat_check(const char* who, int dtype, int64_t num_edges, int num_heads, int64_t head_dim, int64_t num_dst) {
+  APT_CHECK_ARG(dtype >= APT_F32 && dtype <= APT_F16, "%s: dtype %d", who, dtype);
+  APT_CHECK_ARG(num_edges >= 0 && num_heads >= 1 && head_dim >= 1 && num_dst >= 0, "%s: bad sizes", who);
+  APT_CHECK_ARG(num_edges < (int64_t)0x7fffffff && num_dst < (int64_t)0x7fffffff && head_dim < (1 << 28), "%s: sizes beyond 31 bits", who);
   return APT_OK;
 }
 
+// Ranges and attention weights.
+template <typename T>
+static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaStream_t s) {
+  APT_CUDA(cudaMemsetAsync(g.none, 0, 4, s));
+  {
+    ProfScope prof("spmm_ranges", s);
+    APT_LAUNCH(k_gat_ranges, wave_grid(ceil_div(q.E, 256), 8), 256, 0, s, q.col, q.E, q.num_dst, g.range, g.none, q.status);
+  }
+  ProfScope prof("gat_rows", s);
+  APT_LAUNCH(k_gat_weights<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
+             q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn);
+  return APT_OK;
+}
+
+template <typename T>
+static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* attn, cudaStream_t s) {
+  const int rc = gat_weights<T>(q, g, attn, s);
+  if (rc != APT_OK) return rc;
+  const int64_t dim = q.H * q.Dh;
+  // a slice stays inside a head, so that one weight serves it
+  const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)out, sizeof(T));
+  SpmmWs ws{};
+  ws.range = g.range;
+  const RowArgs<T> a{q.row, (const T*)q.ft, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, ws,
+                     (T*)out, nullptr, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none};
+  ProfScope prof("gat_rows", s);
+  return launch_spmm_rows<T>(kUMulW, a, s);
+}
+
+template <typename T, int VE>
+static int launch_dots(const GatProblem& q, const GatEdges& g, float* dots, cudaStream_t s) {
+  static int occupancy[64] = {};
+  int per_sm = 0;
+  const int rc = blocks_per_sm(k_gat_dots<T, VE>, 256, occupancy, &per_sm);
+  if (rc != APT_OK) return rc;
+  const int lph = pow2_ge(q.Dh / VE), hpp = pow2_ge(q.H, 32 / lph);
+  const int64_t want = ceil_div(q.num_dst, 8), wave = (int64_t)kNumSMs * per_sm;
+  APT_LAUNCH((k_gat_dots<T, VE>), (int)(want < wave ? want : wave), 256, 0, s, q.row, (const T*)q.ft, (const T*)q.grad_out, q.H,
+             (int)q.Dh, q.num_dst, g.range, g.none, dots, lph, hpp);
+  return APT_OK;
+}
+
+// The edge part of the backward: weights are there already.
+template <typename T>
+static int gat_edge_backward(const GatProblem& q, const GatEdges& g, float* dots, float2* pair, void* attn, void* grad_score,
+                             void* grad_er, cudaStream_t s) {
+  ProfScope prof("gat_bwd_rows", s);
+  int rc;
+  switch (slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T)) {
+    case 16: rc = launch_dots<T, 16 / sizeof(T)>(q, g, dots, s); break;
+    case 8: rc = launch_dots<T, 8 / sizeof(T)>(q, g, dots, s); break;
+    case 4: rc = launch_dots<T, 4 / sizeof(T)>(q, g, dots, s); break;
+    default: rc = launch_dots<T, 1>(q, g, dots, s); break;
+  }
+  if (rc != APT_OK) return rc;
+  APT_LAUNCH(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
+             q.slope, q.num_dst, q.E, g.range, g.none, g.weight, dots, pair, (T*)attn, (T*)grad_score, (T*)grad_er);
+  return APT_OK;
+}
+
+template <typename T>
+static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, char* workspace, int64_t num_src, void* grad_ft,
+                        void* grad_el, void* grad_er, cudaStream_t s) {
+  int rc = gat_edge_backward<T>(q, g, ws.dots, ws.pair, nullptr, nullptr, grad_er, s);
+  if (rc != APT_OK) return rc;
+  const int64_t dim = q.H * q.Dh;
+  const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
+  const RowSplit split = row_split(dim, ve, q.E, num_src);
+  const SegTable st{nullptr, nullptr, nullptr, 1};
+  APT_CUDA(cudaMemsetAsync(workspace, 0, ws.sort.zero_bytes, s));
+  rc = launch_group(q.col, q.row, q.E, st, num_src, ws.sort, kOrder, split.long_edges, (int)dim + q.H, s);
+  if (rc != APT_OK) return rc;
+  const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)ws.pair, q.H, dim, st, num_src, q.E, ws.sort,
+                     (T*)grad_ft, (T*)grad_el, kOrder, 0, split, (int)dim + q.H, nullptr};
+  ProfScope prof("spmm_rows", s);
+  return launch_spmm_rows<T>(kGatSrc, a, s);
+}
+
+// Stream-ordered memory for the duration of a call, for the two entry points without a buffer for weights.
+struct StreamBuffer {
+  void* p = nullptr;
+  cudaStream_t s;
+  explicit StreamBuffer(cudaStream_t stream) : s(stream) {}
+  int take(size_t bytes) {
+    APT_CUDA(cudaMallocAsync(&p, bytes, s));
+    return APT_OK;
+  }
+  ~StreamBuffer() {
+    if (p) cudaFreeAsync(p, s);
+  }
+};
+
 }  // namespace apt
+
+extern "C" size_t apt_gat_edges_bytes(int64_t num_dst, int64_t num_edges, int num_heads) {
+  if (num_dst < 0 || num_edges < 0 || num_heads < 1) return 0;
+  return apt::gat_edges_layout(num_dst, num_edges, num_heads, nullptr, nullptr);
+}
+
+extern "C" int apt_gat_forward(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges, const void* ft,
+                               const void* el, const void* er, int num_heads, int64_t head_dim, float negative_slope,
+                               int64_t num_dst, void* out, void* out_attn, void* edges, size_t edges_bytes,
+                               int32_t* status_word, void* stream) {
+  using namespace apt;
+  const int rc = gat_check("apt_gat_forward", dtype, num_edges, num_heads, head_dim, num_dst);
+  if (rc != APT_OK || num_dst == 0) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  APT_CHECK_ARG(out && status_word, "apt_gat_forward: null output");
+  if (num_edges == 0) {
+    APT_CUDA(cudaMemsetAsync(out, 0, (size_t)num_dst * num_heads * head_dim * elem_size(dtype), s));
+    return APT_OK;
+  }
+  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && edges, "apt_gat_forward: null pointer");
+  APT_CHECK_ARG(((uintptr_t)edges & 255) == 0, "apt_gat_forward: the edge buffer must be 256-byte aligned");
+  GatEdges g;
+  const size_t need = gat_edges_layout(num_dst, num_edges, num_heads, (char*)edges, &g);
+  if (edges_bytes < need) {
+    set_error("apt_gat_forward: edge buffer %zu < %zu bytes", edges_bytes, need);
+    return APT_ERR_CAPACITY;
+  }
+  const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, nullptr, num_heads, head_dim, negative_slope, num_dst, status_word};
+  switch (dtype) {
+    case APT_F32: return gat_forward<float>(q, g, out, out_attn, s);
+    case APT_BF16: return gat_forward<__nv_bfloat16>(q, g, out, out_attn, s);
+    default: return gat_forward<__half>(q, g, out, out_attn, s);
+  }
+}
+
+extern "C" size_t apt_gat_backward_workspace_bytes(int64_t num_src, int64_t num_edges, int num_heads) {
+  if (num_src < 0 || num_edges < 0 || num_heads < 1) return 0;
+  return apt::gat_bwd_layout(num_src, num_edges, num_heads, nullptr, nullptr);
+}
+
+extern "C" int apt_gat_backward(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges,
+                                const void* ft, const void* el, const void* er, const void* grad_out, int num_heads,
+                                int64_t head_dim, float negative_slope, int64_t num_src, int64_t num_dst, void* grad_ft,
+                                void* grad_el, void* grad_er, void* edges, size_t edges_bytes, int edges_valid,
+                                void* workspace, size_t workspace_bytes, int32_t* status_word, void* stream) {
+  using namespace apt;
+  int rc = gat_check("apt_gat_backward", dtype, num_edges, num_heads, head_dim, num_dst);
+  if (rc != APT_OK) return rc;
+  APT_CHECK_ARG(num_src >= 0 && num_src < (int64_t)0x7fffffff, "apt_gat_backward: bad num_src");
+  cudaStream_t s = (cudaStream_t)stream;
+  const size_t esz = elem_size(dtype);
+  const int64_t dim = (int64_t)num_heads * head_dim;
+  APT_CHECK_ARG((num_src == 0 || (grad_ft && grad_el)) && (num_dst == 0 || grad_er) && status_word, "apt_gat_backward: null output");
+  if (num_edges == 0 || num_src == 0 || num_dst == 0) {
+    if (num_src > 0) {
+      APT_CUDA(cudaMemsetAsync(grad_ft, 0, (size_t)num_src * dim * esz, s));
+      APT_CUDA(cudaMemsetAsync(grad_el, 0, (size_t)num_src * num_heads * esz, s));
+    }
+    if (num_dst > 0) APT_CUDA(cudaMemsetAsync(grad_er, 0, (size_t)num_dst * num_heads * esz, s));
+    return APT_OK;
+  }
+  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && grad_out && edges && workspace, "apt_gat_backward: null pointer");
+  APT_CHECK_ARG((((uintptr_t)workspace | (uintptr_t)edges) & 255) == 0, "apt_gat_backward: buffers must be 256-byte aligned");
+  GatEdges g;
+  GatBwdWs ws;
+  const size_t need_e = gat_edges_layout(num_dst, num_edges, num_heads, (char*)edges, &g);
+  const size_t need_w = gat_bwd_layout(num_src, num_edges, num_heads, (char*)workspace, &ws);
+  if (edges_bytes < need_e || workspace_bytes < need_w) {
+    set_error("apt_gat_backward: buffers of %zu and %zu bytes, %zu and %zu needed", edges_bytes, workspace_bytes, need_e, need_w);
+    return APT_ERR_CAPACITY;
+  }
+  const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, grad_out, num_heads, head_dim, negative_slope, num_dst, status_word};
+#define APT_RUN(T)                                                                                          \
+  do {                                                                                                      \
+    if (!edges_valid && (rc = gat_weights<T>(q, g, nullptr, s)) != APT_OK) return rc;                       \
+    return gat_backward<T>(q, g, ws, (char*)workspace, num_src, grad_ft, grad_el, grad_er, s);              \
+  } while (0)
+  switch (dtype) {
+    case APT_F32: APT_RUN(float);
+    case APT_BF16: APT_RUN(__nv_bfloat16);
+    default: APT_RUN(__half);
+  }
+#undef APT_RUN
+}
 
 extern "C" int apt_gat_edge_softmax_sum(int dtype, const int64_t* coo_row, const int64_t* coo_col,
                                         int64_t num_edges, const void* ft, const void* el, const void* er,
@@ -516,44 +497,16 @@ extern "C" int apt_gat_edge_softmax_sum(int dtype, const int64_t* coo_row, const
                                         int64_t num_dst, void* out, void* out_attn, void* workspace,
                                         size_t workspace_bytes, int32_t* status_word, void* stream) {
   using namespace apt;
-  APT_CHECK_ARG(dtype >= APT_F32 && dtype <= APT_F16, "apt_gat_edge_softmax_sum: dtype %d", dtype);
-  APT_CHECK_ARG(num_edges >= 0 && num_heads >= 1 && head_dim >= 1 && num_dst >= 0,
-                "apt_gat_edge_softmax_sum: bad sizes");
-  if (num_dst == 0) return APT_OK;
-  const size_t esz = (size_t)(dtype == APT_F32 ? 4 : 2);
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
-  cudaStream_t s = (cudaStream_t)stream;
-  APT_CHECK_ARG(out && status_word, "apt_gat_edge_softmax_sum: null output");
-  if (num_edges == 0) {
-    APT_CUDA(cudaMemsetAsync(out, 0, (size_t)num_dst * feat_dim * esz, s));
-    return APT_OK;
+  const int rc = gat_check("apt_gat_edge_softmax_sum", dtype, num_edges, num_heads, head_dim, num_dst);
+  if (rc != APT_OK || num_dst == 0) return rc;
+  StreamBuffer edges((cudaStream_t)stream);
+  const size_t bytes = gat_edges_layout(num_dst, num_edges, num_heads, nullptr, nullptr);
+  if (num_edges > 0) {
+    const int taken = edges.take(bytes);
+    if (taken != APT_OK) return taken;
   }
-  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && workspace, "apt_gat_edge_softmax_sum: null pointer");
-  APT_CHECK_ARG(((uintptr_t)workspace & 255) == 0, "apt_gat_edge_softmax_sum: workspace must be 256-byte aligned");
-  GatWs ws;
-  if (!gat_layout(num_dst, (char*)workspace, workspace_bytes, &ws)) {
-    set_error("apt_gat_edge_softmax_sum: workspace of %zu bytes is too small", workspace_bytes);
-    return APT_ERR_CAPACITY;
-  }
-  APT_CUDA(cudaMemsetAsync(ws.flags, 0, 4, s));
-  {
-    ProfScope prof("spmm_ranges", s);
-    const int grid = wave_grid(ceil_div(num_edges, 256), 8);
-    APT_LAUNCH(k_edge_ranges_single, grid, 256, 0, s, coo_col, num_edges, num_dst, ws);
-  }
-  const int ve = 16 / (int)esz;
-  const bool vec = (((uint64_t)(feat_dim * esz) | (uintptr_t)ft | (uintptr_t)out) & 15) == 0 && head_dim % ve == 0;
-  switch (dtype) {
-    case APT_F32:
-      return launch_gat<float>(vec, coo_row, ft, el, er, num_heads, head_dim, negative_slope, num_dst, ws, out,
-                               out_attn, status_word, s);
-    case APT_BF16:
-      return launch_gat<__nv_bfloat16>(vec, coo_row, ft, el, er, num_heads, head_dim, negative_slope, num_dst, ws,
-                                       out, out_attn, status_word, s);
-    default:
-      return launch_gat<__half>(vec, coo_row, ft, el, er, num_heads, head_dim, negative_slope, num_dst, ws, out,
-                                out_attn, status_word, s);
-  }
+  return apt_gat_forward(dtype, coo_row, coo_col, num_edges, ft, el, er, num_heads, head_dim, negative_slope, num_dst, out,
+                         out_attn, edges.p, bytes, status_word, stream);
 }
 
 extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges,
@@ -562,45 +515,33 @@ extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const in
                                      void* out_attn, void* out_grad_score, void* out_grad_er, void* workspace,
                                      size_t workspace_bytes, int32_t* status_word, void* stream) {
   using namespace apt;
-  APT_CHECK_ARG(dtype >= APT_F32 && dtype <= APT_F16, "apt_gat_edge_backward: dtype %d", dtype);
-  APT_CHECK_ARG(num_edges >= 0 && num_heads >= 1 && head_dim >= 1 && num_dst >= 0, "apt_gat_edge_backward: bad sizes");
-  if (num_dst == 0) return APT_OK;
-  const size_t esz = (size_t)(dtype == APT_F32 ? 4 : 2);
-  const int64_t feat_dim = (int64_t)num_heads * head_dim;
+  int rc = gat_check("apt_gat_edge_backward", dtype, num_edges, num_heads, head_dim, num_dst);
+  if (rc != APT_OK || num_dst == 0) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   APT_CHECK_ARG(out_grad_er && status_word, "apt_gat_edge_backward: null output");
   if (num_edges == 0) {
-    APT_CUDA(cudaMemsetAsync(out_grad_er, 0, (size_t)num_dst * num_heads * esz, s));
+    APT_CUDA(cudaMemsetAsync(out_grad_er, 0, (size_t)num_dst * num_heads * elem_size(dtype), s));
     return APT_OK;
   }
-  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && grad_out && out_attn && out_grad_score && workspace,
+  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && grad_out && out_attn && out_grad_score,
                 "apt_gat_edge_backward: null pointer");
-  APT_CHECK_ARG(((uintptr_t)workspace & 255) == 0, "apt_gat_edge_backward: workspace must be 256-byte aligned");
-  GatWs ws;
-  if (!gat_layout(num_dst, (char*)workspace, workspace_bytes, &ws)) {
-    set_error("apt_gat_edge_backward: workspace of %zu bytes is too small", workspace_bytes);
-    return APT_ERR_CAPACITY;
-  }
-  APT_CUDA(cudaMemsetAsync(ws.flags, 0, 4, s));
-  // edges that name no valid destination keep zeros
-  APT_CUDA(cudaMemsetAsync(out_attn, 0, (size_t)num_edges * num_heads * esz, s));
-  APT_CUDA(cudaMemsetAsync(out_grad_score, 0, (size_t)num_edges * num_heads * esz, s));
-  {
-    ProfScope prof("spmm_ranges", s);
-    const int grid = wave_grid(ceil_div(num_edges, 256), 8);
-    APT_LAUNCH(k_edge_ranges_single, grid, 256, 0, s, coo_col, num_edges, num_dst, ws);
-  }
-  const int ve = 16 / (int)esz;
-  const bool vec = (((uint64_t)(feat_dim * esz) | (uintptr_t)ft | (uintptr_t)grad_out) & 15) == 0 && head_dim % ve == 0;
+  StreamBuffer buffer(s);
+  const size_t edges_bytes = gat_edges_layout(num_dst, num_edges, num_heads, nullptr, nullptr);
+  rc = buffer.take(edges_bytes + (size_t)num_edges * num_heads * 4);
+  if (rc != APT_OK) return rc;
+  GatEdges g;
+  gat_edges_layout(num_dst, num_edges, num_heads, (char*)buffer.p, &g);
+  float* dots = (float*)((char*)buffer.p + edges_bytes);
+  const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, grad_out, num_heads, head_dim, negative_slope, num_dst, status_word};
+#define APT_RUN(T)                                                                                         \
+  do {                                                                                                     \
+    if ((rc = gat_weights<T>(q, g, nullptr, s)) != APT_OK) return rc;                                      \
+    return gat_edge_backward<T>(q, g, dots, nullptr, out_attn, out_grad_score, out_grad_er, s);            \
+  } while (0)
   switch (dtype) {
-    case APT_F32:
-      return launch_gat_bwd<float>(vec, coo_row, ft, el, er, grad_out, num_heads, head_dim, negative_slope, num_dst,
-                                   ws, out_attn, out_grad_score, out_grad_er, status_word, s);
-    case APT_BF16:
-      return launch_gat_bwd<__nv_bfloat16>(vec, coo_row, ft, el, er, grad_out, num_heads, head_dim, negative_slope,
-                                           num_dst, ws, out_attn, out_grad_score, out_grad_er, status_word, s);
-    default:
-      return launch_gat_bwd<__half>(vec, coo_row, ft, el, er, grad_out, num_heads, head_dim, negative_slope,
-                                    num_dst, ws, out_attn, out_grad_score, out_grad_er, status_word, s);
+    case APT_F32: APT_RUN(float);
+    case APT_BF16: APT_RUN(__nv_bfloat16);
+    default: APT_RUN(__half);
   }
+#undef APT_RUN
 }

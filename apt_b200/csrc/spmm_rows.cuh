@@ -32,7 +32,8 @@
 namespace apt {
 
 constexpr int kMaxSegments = 64;
-enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kGatSrc = 4 };
+// kUMulW: one fp32 weight per head. kGatSrc: the same with a second fp32 value per head that is summed beside the row.
+enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kUMulW = 4, kGatSrc = 5 };
 enum { kDevice = -1, kFixed = 0, kRanges = 1, kOrder = 2 };
 
 // Rows of more edges are left to whole warps. A group narrower than a warp hands over earlier: its own pace is
@@ -42,7 +43,7 @@ constexpr int kItemEdges = 64;
 constexpr int kLongRun = 64;     // runs of at least this many edges make the probe ask for the counting sort
 
 struct SegTable {
-  // first edge, first input row and first output row of every segment
+  // first edge, first input row and first output row of every segment; null where a kernel has no use for them
   const int64_t* coo_off;
   const int64_t* in_off;
   const int64_t* out_off;
@@ -112,7 +113,7 @@ template <typename T>
 struct RowArgs {
   const int64_t* row;
   const T* in;
-  const T* edata;          // kGatSrc: float2[E][heads] (attention, score gradient)
+  const T* edata;          // kUMulW: float[E][heads]; kGatSrc: float2[E][heads]
   int64_t edata_dim, feat_dim;
   SegTable st;
   int64_t num_rows, num_edges;
@@ -122,6 +123,7 @@ struct RowArgs {
   int mode, fixed;
   RowSplit split;
   int part_stride;         // floats per part
+  const int32_t* none;     // when given and not zero: no row has edges (kRanges)
 };
 
 // One slice of one edge's contribution, in two steps so that the loads of several edges are issued
@@ -133,73 +135,78 @@ struct EdgeSlice {
   float s, s2;                                            // per-head edge value (kGatSrc: and gradient)
 };
 
+// `lane_in` and `lane_edata` point at the lane's column of row 0, `off` bytes before this slice.
 template <typename T, int VE, int OP>
-__device__ __forceinline__ void slice_load(EdgeSlice<T, VE, OP>& v, const RowArgs<T>& a, uint32_t src, uint32_t e,
-                                           int64_t col, int per, int head) {
-  if constexpr (OP == kCopyE) {
-    v.x = load_raw<T, VE>(a.edata + (int64_t)e * a.feat_dim + col);
-  } else {
-    v.x = load_raw<T, VE>(a.in + (int64_t)src * a.feat_dim + col);
-  }
+__device__ __forceinline__ void slice_load(EdgeSlice<T, VE, OP>& v, const RowArgs<T>& a, const T* lane_in, uint32_t off,
+                                           const T* lane_edata, uint32_t row_bytes, uint32_t edata_bytes, uint32_t src, uint32_t e,
+                                           int col, int per, int head) {
+  v.x = load_raw<T, VE>(OP == kCopyE ? at_row(lane_edata, e, edata_bytes)
+                                     : (const T*)((const char*)at_row(lane_in, src, row_bytes) + off));
   if constexpr (OP == kUMulE || OP == kUAddE) {
     if (per == 1) {
-      v.w = load_raw<T, VE>(a.edata + (int64_t)e * a.feat_dim + col);
+      v.w = load_raw<T, VE>(at_row(lane_edata, e, edata_bytes));
     } else if (head >= 0) {
-      v.s = Elem<T>::to_f(a.edata[(int64_t)e * a.edata_dim + head]);
+      v.s = Elem<T>::to_f(*at_row(lane_edata, e, edata_bytes));
     } else {
+      const T* const p = at_row(a.edata, e, edata_bytes);
       Pack<T, VE> w;
 #pragma unroll
-      for (int t = 0; t < VE; ++t) w.v[t] = a.edata[(int64_t)e * a.edata_dim + (col + t) / per];
+      for (int t = 0; t < VE; ++t) w.v[t] = p[(col + t) / per];
 #pragma unroll
       for (int k = 0; k < (int)(sizeof(v.w.w) / 4); ++k)
         v.w.w[k] = sizeof(T) * VE < 4 ? (unsigned int)*(const unsigned short*)&w : ((const unsigned int*)&w)[k];
     }
   }
+  if constexpr (OP == kUMulW) v.s = __ldg((const float*)at_row(lane_edata, e, edata_bytes));
   if constexpr (OP == kGatSrc) {
-    const float2 p = __ldg((const float2*)a.edata + (int64_t)e * a.edata_dim + head);
+    const float2 p = __ldg((const float2*)at_row(lane_edata, e, edata_bytes));
     v.s = p.x;
     v.s2 = p.y;
   }
 }
 
 template <typename T, int VE, int OP>
-__device__ __forceinline__ void slice_add(float* acc, float& acc2, const EdgeSlice<T, VE, OP>& v, int per, int head) {
-#pragma unroll
-  for (int t = 0; t < VE; ++t) {
-    const float x = v.x.get(t);
-    if constexpr (OP == kUMulE || OP == kUAddE) {
-      const float w = (per != 1 && head >= 0) ? v.s : v.w.get(t);
-      acc[t] += OP == kUMulE ? x * w : x + w;
-    } else if constexpr (OP == kGatSrc) {
-      acc[t] += v.s * x;
+__device__ __forceinline__ void slice_add(Acc<VE>& acc, float& acc2, const EdgeSlice<T, VE, OP>& v, int per, int head) {
+  if constexpr (OP == kUMulE) {
+    if (per != 1 && head >= 0) {
+      acc.fma(v.x, v.s);
     } else {
-      acc[t] += x;
+      acc.fma(v.x, v.w);
     }
+  } else if constexpr (OP == kUAddE) {
+    acc.add(v.x);
+    if (per != 1 && head >= 0) {
+      const F2 ss = f2_pack(v.s, v.s);
+#pragma unroll
+      for (int q = 0; q < Acc<VE>::P; ++q) acc.p[q] = f2_add(acc.p[q], ss);
+    } else {
+      acc.add(v.w);
+    }
+  } else if constexpr (OP == kUMulW || OP == kGatSrc) {
+    acc.fma(v.x, v.s);
+    if constexpr (OP == kGatSrc) acc2 += v.s2;
+  } else {
+    acc.add(v.x);
   }
-  if constexpr (OP == kGatSrc) acc2 += v.s2;
 }
 
 // The sums of the edges read side by side meet, and the lanes of the first of them write the row's column block.
 template <typename T, int VE, int VPL, int OP>
-__device__ __forceinline__ void rows_write(const RowArgs<T>& a, float (&acc)[VPL][VE], float (&acc2)[VPL], const int (&col)[VPL],
+__device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], float (&acc2)[VPL], const int (&col)[VPL],
                                            const int (&head)[VPL], int d, int c0, int nvec, int per, int lpe, int lpr, int vl,
                                            int epi, unsigned gmask) {
 #pragma unroll 1
   for (int o = lpe; o < lpr; o <<= 1)
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-#pragma unroll
-      for (int t = 0; t < VE; ++t) acc[i][t] += __shfl_xor_sync(gmask, acc[i][t], o);
+      acc[i].join(gmask, o);
       if constexpr (OP == kGatSrc) acc2[i] += __shfl_xor_sync(gmask, acc2[i], o);
     }
   if (epi != 0) return;
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     if (c0 + vl + i * lpe >= nvec) continue;
-    Pack<T, VE> o;
-#pragma unroll
-    for (int t = 0; t < VE; ++t) o.v[t] = Elem<T>::from_f(acc[i][t]);
-    store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], o);
+    store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
     if constexpr (OP == kGatSrc)
       if (col[i] % per == 0) a.out2[(int64_t)d * a.edata_dim + head[i]] = Elem<T>::from_f(acc2[i]);
   }
@@ -210,17 +217,18 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, float (&acc)[VPL
 // 67 584 x 15 edges, fp32 x 256 (1.04 GB gathered, mostly out of L2): 152 us at one or two blocks, 114 at three, 109 at
 // four; bf16 x 256: 89 / 65 / 63 us; the reverse direction 186 / 149 / 158 and 104 / 82 / 90 us.
 constexpr int rows_min_blocks(int op, int elems) {
-  if (op == kCopyU || op == kCopyE) return elems <= 4 ? 4 : elems <= 8 ? 3 : 2;
+  if (op == kCopyU || op == kCopyE || op == kUMulW) return elems <= 4 ? 4 : elems <= 8 ? 3 : 2;
+  if (op == kGatSrc) return elems <= 8 ? 2 : 1;   // three blocks spill: 158 -> 188 us on the attention backward (bf16, 4 x 64)
   return elems <= 2 ? 3 : elems <= 8 ? 2 : 1;
 }
 
 // WIDE: a warp to an edge (lpe 32, ep 1), which leaves the geometry to the compiler and its registers to more warps.
 template <typename T, int VE, int VPL, int OP, bool WIDE>
 __global__ void __launch_bounds__(256, rows_min_blocks(OP, VE * VPL))
-k_spmm_rows(const RowArgs<T> a) {
+k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   constexpr int U = VPL >= 2 ? 2 : 4;
   __shared__ int64_t coo[kMaxSegments + 1], ioff[kMaxSegments + 1];
-  int mode = a.mode, fixed = a.fixed;
+  int mode = OP == kGatSrc ? kOrder : a.mode, fixed = a.fixed;
   if (mode == kDevice) {
     const int64_t w = *a.ws.result;
     mode = probe_mode(w);
@@ -228,8 +236,9 @@ k_spmm_rows(const RowArgs<T> a) {
   }
   if (mode != kOrder) {
     for (int t = threadIdx.x; t <= a.st.nseg; t += blockDim.x) {
-      coo[t] = a.st.coo_off[t];
-      ioff[t] = OP == kCopyE ? 0 : a.st.in_off[t];
+      // no table: one segment whose rows start at 0
+      coo[t] = a.st.coo_off ? a.st.coo_off[t] : 0;
+      ioff[t] = a.st.in_off ? a.st.in_off[t] : 0;
     }
     __syncthreads();
   }
@@ -237,6 +246,9 @@ k_spmm_rows(const RowArgs<T> a) {
   const int lpe = WIDE ? 32 : a.split.lpe, vl = lane & (lpe - 1);
   const int nvec = (int)(a.feat_dim / VE);
   const int per = (int)(a.feat_dim / a.edata_dim);
+  const uint32_t row_bytes = (uint32_t)(a.feat_dim * sizeof(T));
+  const uint32_t ed_bytes = (uint32_t)(a.edata_dim * (OP == kGatSrc ? sizeof(float2) : OP == kUMulW ? sizeof(float) : sizeof(T)));
+  const bool none = a.none && *a.none != 0;
   // rows and edges fit 31 bits, and so does everything that counts them
   const int num_rows = (int)a.num_rows;
   const int warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -266,7 +278,7 @@ k_spmm_rows(const RowArgs<T> a) {
       b = d * fixed;
       e = b + fixed;
     } else {
-      const int2 r = a.ws.range[d];
+      const int2 r = none ? make_int2(0, 0) : a.ws.range[d];
       b = r.x;
       e = r.y;
     }
@@ -308,16 +320,21 @@ k_spmm_rows(const RowArgs<T> a) {
     const bool skip = !items && mode == kOrder && e - b > a.split.long_edges;
 #pragma unroll 1
     for (int c0 = 0; c0 < nvec && !skip; c0 += lpe * VPL) {
-      float acc[VPL][VE], acc2[VPL];
+      Acc<VE> acc[VPL];
+      float acc2[VPL];
       int head[VPL], col[VPL];
+      const T* lane_ed[VPL];
+      uint32_t off[VPL];      // bytes from the lane's first slice; lanes past the row's last slice read their first one again
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
         acc2[i] = 0.f;
-#pragma unroll
-        for (int t = 0; t < VE; ++t) acc[i][t] = 0.f;
-        col[i] = min(c0 + vl + i * lpe, nvec - 1) * VE;
-        head[i] = (OP == kGatSrc || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
+        acc[i].zero();
+        col[i] = (c0 + vl + i * lpe < nvec ? c0 + vl + i * lpe : i == 0 ? nvec - 1 : c0 + vl < nvec ? c0 + vl : nvec - 1) * VE;
+        head[i] = (OP == kGatSrc || OP == kUMulW || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
+        off[i] = (uint32_t)((col[i] - col[0]) * (int)sizeof(T));
+        lane_ed[i] = OP == kGatSrc ? (const T*)((const float2*)a.edata + head[i]) : OP == kUMulW ? (const T*)((const float*)a.edata + head[i]) : a.edata + (head[i] >= 0 ? head[i] : col[i]);
       }
+      const T* const lane_in = a.in + col[0];
       uint32_t my_src = src, my_e = eid;
 #pragma unroll 1
       for (int k0 = b; k0 < e; k0 += LPR) {
@@ -333,7 +350,7 @@ k_spmm_rows(const RowArgs<T> a) {
             const uint32_t s = OP == kCopyE ? 0u : __shfl_sync(GMASK, my_src, j + u * EP, LPR);
             const uint32_t x = OP == kCopyU ? 0u : __shfl_sync(GMASK, my_e, j + u * EP, LPR);
 #pragma unroll
-            for (int i = 0; i < VPL; ++i) slice_load<T, VE, OP>(v[u][i], a, s, x, col[i], per, head[i]);
+            for (int i = 0; i < VPL; ++i) slice_load<T, VE, OP>(v[u][i], a, lane_in, off[i], lane_ed[i], row_bytes, ed_bytes, s, x, col[i], per, head[i]);
           }
 #pragma unroll
           for (int u = 0; u < U; ++u)
@@ -348,7 +365,7 @@ k_spmm_rows(const RowArgs<T> a) {
             const uint32_t x = OP == kCopyU ? 0u : __shfl_sync(GMASK, my_e, (j + u * EP) & (LPR - 1), LPR);
             if (j + u * EP < cnt) {
 #pragma unroll
-              for (int i = 0; i < VPL; ++i) slice_load<T, VE, OP>(v[u][i], a, s, x, col[i], per, head[i]);
+              for (int i = 0; i < VPL; ++i) slice_load<T, VE, OP>(v[u][i], a, lane_in, off[i], lane_ed[i], row_bytes, ed_bytes, s, x, col[i], per, head[i]);
             }
           }
 #pragma unroll
@@ -368,8 +385,7 @@ k_spmm_rows(const RowArgs<T> a) {
         for (int o = lpe; o < LPR; o <<= 1)
 #pragma unroll
           for (int i = 0; i < VPL; ++i) {
-#pragma unroll
-            for (int t = 0; t < VE; ++t) acc[i][t] += __shfl_xor_sync(GMASK, acc[i][t], o);
+            acc[i].join(GMASK, o);
             if constexpr (OP == kGatSrc) acc2[i] += __shfl_xor_sync(GMASK, acc2[i], o);
           }
         if (EPI == 0) {
@@ -377,7 +393,7 @@ k_spmm_rows(const RowArgs<T> a) {
           for (int i = 0; i < VPL; ++i) {
             if (c0 + vl + i * lpe >= nvec) continue;
 #pragma unroll
-            for (int t = 0; t < VE; ++t) __stcg(p + col[i] + t, acc[i][t]);
+            for (int t = 0; t < VE; ++t) __stcg(p + col[i] + t, acc[i].get(t));
             if constexpr (OP == kGatSrc)
               if (col[i] % per == 0) __stcg(p + a.feat_dim + head[i], acc2[i]);
           }
@@ -400,13 +416,13 @@ k_spmm_rows(const RowArgs<T> a) {
             col[i] = min(cc + vl + i * lpe, nvec - 1) * VE;
             head[i] = OP == kGatSrc ? col[i] / per : -1;
             acc2[i] = 0.f;
-#pragma unroll
-            for (int t = 0; t < VE; ++t) acc[i][t] = 0.f;
+            acc[i].zero();
 #pragma unroll 1
             for (int q = EPI; q < parts; q += EP) {
               const float* src_part = a.ws.part + (int64_t)(first + q) * a.part_stride;
 #pragma unroll
-              for (int t = 0; t < VE; ++t) acc[i][t] += __ldcg(src_part + col[i] + t);
+              for (int t = 0; t < VE; t += 2)
+                acc[i].p[t / 2] = f2_add(acc[i].p[t / 2], f2_pack(__ldcg(src_part + col[i] + t), VE > 1 ? __ldcg(src_part + col[i] + (VE > 1 ? t + 1 : t)) : 0.f));
               if constexpr (OP == kGatSrc) acc2[i] += __ldcg(src_part + a.feat_dim + head[i]);
             }
           }
@@ -438,14 +454,9 @@ k_spmm_rows(const RowArgs<T> a) {
 template <typename T, int VE, int VPL, int OP, bool WIDE>
 static int launch_rows_kernel(const RowArgs<T>& a, cudaStream_t s) {
   static int occupancy[64] = {};
-  int dev = 0;
-  APT_CUDA(cudaGetDevice(&dev));
-  int per_sm = dev >= 0 && dev < 64 ? occupancy[dev] : 0;
-  if (per_sm == 0) {
-    APT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm_rows<T, VE, VPL, OP, WIDE>, 256, 0));
-    if (per_sm < 1) per_sm = 1;
-    if (dev >= 0 && dev < 64) occupancy[dev] = per_sm;
-  }
+  int per_sm = 0;
+  const int rc = blocks_per_sm(k_spmm_rows<T, VE, VPL, OP, WIDE>, 256, occupancy, &per_sm);
+  if (rc != APT_OK) return rc;
   const int64_t want = ceil_div(a.num_rows, 256 / (a.split.lpe * a.split.ep));
   const int64_t wave = (int64_t)kNumSMs * per_sm;
   APT_LAUNCH((k_spmm_rows<T, VE, VPL, OP, WIDE>), (int)(want < wave ? want : wave), 256, 0, s, a);
@@ -485,6 +496,7 @@ int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
       case kCopyE: return launch_rows_ve<T, kCopyE>(a, s);                                \
       case kUMulE: return launch_rows_ve<T, kUMulE>(a, s);                                \
       case kUAddE: return launch_rows_ve<T, kUAddE>(a, s);                                \
+      case kUMulW: return launch_rows_ve<T, kUMulW>(a, s);                                \
       default: return launch_rows_ve<T, kGatSrc>(a, s);                                   \
     }                                                                                                    \
   }

@@ -7,6 +7,7 @@
 // or threads never share it.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <optional>
@@ -19,12 +20,14 @@ using OptTensor = std::optional<Tensor>;
 
 namespace {
 
-struct AptFailure {
+// A std::exception: the autograd engine's threads carry nothing else over to the caller.
+struct AptFailure : std::runtime_error {
+  AptFailure(int code, const char* text) : std::runtime_error(text), status(code) {}
   int status;
 };
 
 void check(int status) {
-  if (status != APT_OK) throw AptFailure{status};
+  if (status != APT_OK) throw AptFailure(status, apt_last_error());
 }
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
@@ -56,6 +59,9 @@ Tensor ids(const Tensor& t, const char* name) { return cuda(t, name, at::kLong, 
 const int64_t* ptr(const Tensor& t) { return t.numel() ? t.const_data_ptr<int64_t>() : nullptr; }
 const void* data(const Tensor& t) { return t.numel() ? t.const_data_ptr() : nullptr; }
 void* mut(const Tensor& t) { return t.numel() ? t.mutable_data_ptr() : nullptr; }
+
+// The status flags are the last word of the state's word block.
+int32_t* status_word(const Tensor& words) { return (int32_t*)(words.mutable_data_ptr<int64_t>() + words.numel() - 1); }
 
 Tensor scratch(const Tensor& like, size_t bytes) { return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)); }
 
@@ -108,6 +114,76 @@ Tensor sddmm(int op, const Tensor& coo_row, const Tensor& coo_col, const Tensor&
   return out;
 }
 
+// ---------------------------------------------------------------------------------------- attention block
+struct GatShape {
+  int code;
+  int64_t edges, num_src, num_dst, heads, head_dim;
+};
+
+GatShape gat_shape(const char* who, const Tensor& row, const Tensor& ft, const Tensor& el, const Tensor& er, int64_t num_dst) {
+  const int code = dtype_code(ft.scalar_type());
+  if (code < 0 || el.scalar_type() != ft.scalar_type() || er.scalar_type() != ft.scalar_type())
+    fail(std::string(who) + ": unsupported dtypes " + dtype_name(ft) + "/" + dtype_name(el) + "/" + dtype_name(er));
+  const int64_t num_src = ft.size(0);
+  const int64_t heads = num_src ? el.numel() / std::max<int64_t>(num_src, 1) : er.numel() / std::max<int64_t>(num_dst, 1);
+  return {code, row.numel(), num_src, num_dst, heads, ft.numel() / std::max<int64_t>(num_src * heads, 1)};
+}
+
+// Results of the forward: sums, attention (when asked for) and the edge buffer that a backward of the same block can use.
+std::tuple<Tensor, Tensor, Tensor> gat_forward(const Tensor& coo_row, const Tensor& coo_col, const Tensor& ft_in, const Tensor& el_in,
+                                               const Tensor& er_in, int64_t num_dst, double slope, bool want_attention,
+                                               const Tensor& words) {
+  const Tensor row = ids(coo_row, "coo_row"), col = ids(coo_col, "coo_col");
+  const Tensor ft = cuda(ft_in, "ft"), el = cuda(el_in, "el"), er = cuda(er_in, "er");
+  const GatShape g = gat_shape("gat_edge_softmax_sum", row, ft, el, er, num_dst);
+  Tensor out = at::empty({num_dst, g.heads, g.head_dim}, ft.options()), attn;
+  if (want_attention) attn = at::empty({g.edges, g.heads, 1}, ft.options());
+  const size_t bytes = apt_gat_edges_bytes(num_dst, g.edges, (int)g.heads);
+  const Tensor edges = scratch(ft, bytes);
+  check(apt_gat_forward(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), (int)g.heads, g.head_dim, (float)slope,
+                        num_dst, mut(out), want_attention ? mut(attn) : nullptr, edges.mutable_data_ptr(), bytes,
+                        status_word(words), stream()));
+  return {out, attn, edges};
+}
+
+std::tuple<Tensor, Tensor, Tensor> gat_backward(const Tensor& coo_row, const Tensor& coo_col, const Tensor& ft_in,
+                                                const Tensor& el_in, const Tensor& er_in, const Tensor& grad_in, double slope,
+                                                const Tensor& words, const OptTensor& edges_of_forward) {
+  const Tensor row = ids(coo_row, "coo_row"), col = ids(coo_col, "coo_col");
+  const Tensor ft = cuda(ft_in, "ft"), el = cuda(el_in, "el"), er = cuda(er_in, "er"), grad = cuda(grad_in, "grad_out");
+  if (grad.scalar_type() != ft.scalar_type()) fail("gat_edge_softmax_sum_backward: unsupported or mixed dtypes");
+  const GatShape g = gat_shape("gat_edge_softmax_sum_backward", row, ft, el, er, grad.size(0));
+  Tensor grad_ft = at::empty(ft.sizes(), ft.options()), grad_el = at::empty(el.sizes(), el.options()),
+         grad_er = at::empty(er.sizes(), er.options());
+  const size_t edges_bytes = apt_gat_edges_bytes(g.num_dst, g.edges, (int)g.heads);
+  const Tensor edges = edges_of_forward ? *edges_of_forward : scratch(ft, edges_bytes);
+  const size_t bytes = apt_gat_backward_workspace_bytes(g.num_src, g.edges, (int)g.heads);
+  const Tensor ws = scratch(ft, bytes);
+  check(apt_gat_backward(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), data(grad), (int)g.heads, g.head_dim,
+                         (float)slope, g.num_src, g.num_dst, mut(grad_ft), mut(grad_el), mut(grad_er), edges.mutable_data_ptr(),
+                         edges_bytes, edges_of_forward ? 1 : 0, ws.mutable_data_ptr(), bytes, status_word(words), stream()));
+  return {grad_ft, grad_el, grad_er};
+}
+
+// The forward's ranges and weights are saved with its inputs: the backward of a training step starts from them.
+struct GatFunction : public torch::autograd::Function<GatFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& row, const Tensor& col, const Tensor& ft,
+                        const Tensor& el, const Tensor& er, int64_t num_dst, double slope, const Tensor& words) {
+    auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, false, words);
+    ctx->save_for_backward({row, col, ft, el, er});
+    ctx->saved_data["slope"] = slope;
+    ctx->saved_data["words"] = words;
+    ctx->saved_data["edges"] = edges;
+    return out;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto v = ctx->get_saved_variables();
+    auto [g_ft, g_el, g_er] = gat_backward(v[0], v[1], v[2], v[3], v[4], grads[0], ctx->saved_data["slope"].toDouble(),
+                                           ctx->saved_data["words"].toTensor(), ctx->saved_data["edges"].toTensor());
+    return {Tensor(), Tensor(), g_ft, g_el, g_er, Tensor(), Tensor(), Tensor()};
+  }
+};
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -118,10 +194,23 @@ PYBIND11_MODULE(_native, m) {
     } catch (const AptFailure& e) {
       // _lib.AptError(status, text), what the ctypes path raises
       py::object cls = py::module_::import("apt_b200._lib").attr("AptError");
-      py::object err = cls(e.status, py::bytes(apt_last_error()).attr("decode")("utf-8", "replace"));
+      py::object err = cls(e.status, py::bytes(e.what()).attr("decode")("utf-8", "replace"));
       PyErr_SetObject(cls.ptr(), err.ptr());
     }
   });
   m.def("spmm", &spmm);
   m.def("sddmm", &sddmm);
+  m.def("gat_forward", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
+                          int64_t num_dst, double slope, bool want_attention, const Tensor& words) {
+    auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, want_attention, words);
+    return std::make_tuple(out, attn);
+  });
+  m.def("gat_backward", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
+                           const Tensor& grad, double slope, const Tensor& words) {
+    return gat_backward(row, col, ft, el, er, grad, slope, words, std::nullopt);
+  });
+  m.def("gat_apply", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
+                        int64_t num_dst, double slope, const Tensor& words) {
+    return GatFunction::apply(row, col, ft, el, er, num_dst, slope, words);
+  });
 }

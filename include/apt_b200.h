@@ -394,6 +394,34 @@ int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const int64_t* coo_
                           void* workspace, size_t workspace_bytes,
                           int32_t* status_word, void* stream);
 
+/* Forward and whole backward for a training step. `edges` is a caller's buffer of
+ * apt_gat_edges_bytes(num_dst, num_edges, num_heads) bytes in which the forward leaves
+ * each destination's range of edges and the fp32 attention weights; handed to the
+ * backward with edges_valid = 1 (same block, el, er and slope) it saves working them
+ * out again, with edges_valid = 0 it is scratch there. The backward gives grad_ft
+ * [num_src, num_heads*head_dim], grad_el [num_src, num_heads] and grad_er [num_dst,
+ * num_heads]: the edges are grouped by source once and one walk sums both source-side
+ * gradients. workspace: apt_gat_backward_workspace_bytes(...) bytes.
+ * apt_gat_edge_softmax_sum and apt_gat_edge_backward above take the room for weights
+ * from the stream's memory pool (cudaMallocAsync) and use no workspace. */
+size_t apt_gat_edges_bytes(int64_t num_dst, int64_t num_edges, int num_heads);
+int apt_gat_forward(int dtype, const int64_t* coo_row, const int64_t* coo_col,
+                    int64_t num_edges, const void* ft, const void* el,
+                    const void* er, int num_heads, int64_t head_dim,
+                    float negative_slope, int64_t num_dst, void* out,
+                    void* out_attn, void* edges, size_t edges_bytes,
+                    int32_t* status_word, void* stream);
+size_t apt_gat_backward_workspace_bytes(int64_t num_src, int64_t num_edges,
+                                        int num_heads);
+int apt_gat_backward(int dtype, const int64_t* coo_row, const int64_t* coo_col,
+                     int64_t num_edges, const void* ft, const void* el,
+                     const void* er, const void* grad_out, int num_heads,
+                     int64_t head_dim, float negative_slope, int64_t num_src,
+                     int64_t num_dst, void* grad_ft, void* grad_el, void* grad_er,
+                     void* edges, size_t edges_bytes, int edges_valid,
+                     void* workspace, size_t workspace_bytes,
+                     int32_t* status_word, void* stream);
+
 /* ------------------------------------------- SNP virtual nodes (SAGE / GCN)
  * The id arithmetic of the SNP strategy with virtual nodes: neighbour i of
  * local destination i / fanout, owned by rank o, becomes the virtual node

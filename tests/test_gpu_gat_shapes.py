@@ -1,0 +1,95 @@
+"""The attention block at the edges of its kernels (destinations of more edges than a thread keeps in registers or a
+warp reads at once, more heads than lanes, head widths of every slice size and beyond one block of lanes, ragged and
+empty destinations), the edge-part entry points of the C ABI and the backward that starts from what the forward saved,
+against the fp64 oracle. Bounds as in test_gpu_gat.py: the sums of at most a few hundred fp32 terms within 1e-5 of the
+largest value, 16-bit results within 1e-2."""
+import numpy as np
+import pytest
+import torch
+
+import apt_b200
+from apt_b200 import _lib, ops
+from apt_b200._lib import check, lib
+from oracle import oracle as orc
+from tests.gpu_util import dev, host
+
+pytestmark = pytest.mark.gpu
+I64 = np.int64
+TOL = {torch.float32: 1e-5, torch.bfloat16: 1e-2, torch.float16: 1e-2}
+CODE = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
+
+
+def _round(x, dtype):
+    return torch.from_numpy(x).to(dtype).float().numpy() if dtype != torch.float32 else x
+
+
+def _inputs(lengths, H, Dh, dtype, seed):
+    rng = np.random.default_rng(seed)
+    S, E, n_src = len(lengths), int(sum(lengths)), 40
+    col = np.repeat(np.arange(S), lengths).astype(I64)
+    row = rng.integers(0, n_src, E).astype(I64)
+    make = lambda *shape: _round(rng.standard_normal(shape).astype(np.float32), dtype)
+    return row, col, make(n_src, H, Dh), make(n_src, H), make(S, H), make(S, H, Dh)
+
+
+def _near(got, want, dtype, name):
+    err = np.abs(host(got).astype(np.float64).reshape(want.shape) - want).max() / max(np.abs(want).max(), 1.0)
+    assert err <= TOL[dtype], f"{name}: {err:.2e}"
+
+
+RAGGED = [0, 1, 15, 16, 17, 0, 31, 32, 33, 64, 65, 130, 2, 0]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,Dh", [(1, 1), (4, 64), (3, 5), (8, 47), (9, 8), (33, 4), (1, 300), (2, 1030)])
+@pytest.mark.parametrize("lengths", [[7] * 9, RAGGED], ids=["fixed", "ragged"])
+def test_forward_and_backward(dtype, H, Dh, lengths):
+    row, col, ft, el, er, go = _inputs(lengths, H, Dh, dtype, H * 100 + Dh)
+    S = len(lengths)
+    args = dev(row), dev(col), dev(ft, dtype), dev(el, dtype), dev(er, dtype)
+    out, attn = ops.gat_edge_softmax_sum(*args, S, 0.2, return_attention=True)
+    want, want_a = orc.gat_edge_softmax_sum(row, col, ft, el, er, S, 0.2)
+    _near(out, want, dtype, "out")
+    _near(attn, want_a, dtype, "attention")
+    g_want = orc.gat_edge_softmax_sum_backward(row, col, ft, el, er, go, S, 0.2)[:3]
+    for got, w, name in zip(ops.gat_edge_softmax_sum_backward(*args, dev(go, dtype), 0.2), g_want, ("ft", "el", "er")):
+        _near(got, w, dtype, "grad_" + name)
+    # through autograd the backward starts from the ranges and weights the forward left
+    leaves = [t.requires_grad_() for t in args[2:]]
+    y = apt_b200.GATEdgeSoftmaxSum.apply(args[0], args[1], *leaves, S, 0.2)
+    for got, w, name in zip(torch.autograd.grad(y, leaves, dev(go, dtype)), g_want, ("ft", "el", "er")):
+        _near(got, w, dtype, "autograd grad_" + name)
+    ops.check_status()
+
+
+def test_edge_part_entry_points():
+    dtype, H, Dh = torch.float32, 4, 16
+    row, col, ft, el, er, go = _inputs(RAGGED, H, Dh, dtype, 1)
+    S, E = len(RAGGED), len(row)
+    t = [dev(x) for x in (row, col, ft, el, er, go)]
+    p = [x.data_ptr() for x in t]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, attn, gs, ger = (torch.full(shape, 9.0, device="cuda") for shape in ((S, H, Dh), (E, H), (E, H), (S, H)))
+    nbytes = lib.apt_spmm_workspace_bytes(S, 0)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    check(lib.apt_gat_edge_softmax_sum(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], H, Dh, 0.2, S, out.data_ptr(), None,
+                                       ws.data_ptr(), nbytes, status.data_ptr(), None))
+    check(lib.apt_gat_edge_backward(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], p[5], H, Dh, 0.2, S, attn.data_ptr(),
+                                    gs.data_ptr(), ger.data_ptr(), ws.data_ptr(), nbytes, status.data_ptr(), None))
+    torch.cuda.synchronize()
+    want, _ = orc.gat_edge_softmax_sum(row, col, ft, el, er, S, 0.2)
+    _, _, w_er, w_attn, w_gs = orc.gat_edge_softmax_sum_backward(row, col, ft, el, er, go, S, 0.2)
+    for got, w, name in ((out, want, "out"), (attn, w_attn, "attention"), (gs, w_gs, "score gradient"), (ger, w_er, "grad_er")):
+        _near(got, np.asarray(w).reshape(got.shape), dtype, name)
+    assert int(status[0]) == 0
+
+
+def test_ungrouped_backward_is_zero_and_flagged():
+    col = np.array([1, 0, 1, 1], dtype=I64)
+    row = np.array([0, 1, 2, 0], dtype=I64)
+    ft, one = torch.ones((3, 2, 8), device="cuda"), torch.ones((3, 2), device="cuda")
+    grads = ops.gat_edge_softmax_sum_backward(dev(row), dev(col), ft, one, one[:2], torch.ones((2, 2, 8), device="cuda"))
+    torch.cuda.synchronize()
+    assert not any(host(g).any() for g in grads)
+    with pytest.raises(RuntimeError, match="not grouped"):
+        ops.check_status()
