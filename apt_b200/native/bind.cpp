@@ -114,6 +114,37 @@ Tensor sddmm(int op, const Tensor& coo_row, const Tensor& coo_col, const Tensor&
   return out;
 }
 
+// ------------------------------------------------------------------------------------------ row movers
+// Rows of the device cache or of the page-locked host table (`column` is the host table's column offset in elements).
+Tensor gather(const Tensor& node_id, const Tensor& pos_map, const Tensor& dev_feats, const Tensor& uva_feats, int64_t num_nodes,
+              int64_t column, const Tensor& words) {
+  const Tensor id = ids(node_id, "node_id");
+  const int64_t n = id.numel(), size = dev_feats.element_size(), dim = dev_feats.size(1);
+  Tensor out = at::empty({n, dim}, dev_feats.options());
+  if (n == 0) return out;
+  const size_t bytes = apt_gather_workspace_bytes(n);
+  const Tensor ws = scratch(out, bytes);
+  check(apt_gather_rows(ptr(id), n, nullptr, ptr(pos_map), num_nodes, data(dev_feats), dev_feats.size(0), dim * size,
+                        data(uva_feats), uva_feats.size(0), uva_feats.size(1) * size, column * size, mut(out),
+                        ws.mutable_data_ptr(), bytes, status_word(words), stream()));
+  return out;
+}
+
+Tensor rows_gather(const Tensor& inp, const Tensor& index) {
+  const Tensor in = cuda(inp, "inp"), at = ids(index, "index");
+  Tensor out = at::empty({at.numel(), in.size(1)}, in.options());
+  check(apt_rows_gather(data(in), ptr(at), at.numel(), in.size(1) * in.element_size(), mut(out), stream()));
+  return out;
+}
+
+Tensor rows_scatter(const Tensor& inp, const Tensor& index, int64_t num_out_rows) {
+  const Tensor in = cuda(inp, "inp"), at = ids(index, "index");
+  Tensor out = at.numel() == num_out_rows ? at::empty({num_out_rows, in.size(1)}, in.options())
+                                          : at::zeros({num_out_rows, in.size(1)}, in.options());
+  check(apt_rows_scatter(data(in), ptr(at), at.numel(), in.size(1) * in.element_size(), mut(out), stream()));
+  return out;
+}
+
 // ---------------------------------------------------------------------------------------- attention block
 struct GatShape {
   int code;
@@ -200,6 +231,9 @@ PYBIND11_MODULE(_native, m) {
   });
   m.def("spmm", &spmm);
   m.def("sddmm", &sddmm);
+  m.def("gather", &gather);
+  m.def("rows_gather", &rows_gather);
+  m.def("rows_scatter", &rows_scatter);
   m.def("gat_forward", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
                           int64_t num_dst, double slope, bool want_attention, const Tensor& words) {
     auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, want_attention, words);

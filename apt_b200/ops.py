@@ -732,14 +732,15 @@ def load_subtensor(node_id: torch.Tensor) -> torch.Tensor:
     f = STATE.feat
     if f.feat_pos_map is None:
         raise RuntimeError("cache_feats_shared has not been called")
-    node_id = _need_cuda(node_id, "node_id")
     pre = STATE.prefetched
     if pre is not None:
         STATE.prefetched = None
         ids, rows = pre
-        if ids.data_ptr() == node_id.data_ptr() and ids.numel() == node_id.numel():
+        if ids is node_id or (ids.data_ptr() == node_id.data_ptr() and ids.numel() == node_id.numel()
+                              and node_id.is_contiguous()):
             return rows
-    return _gather_enqueue(node_id, None)
+    return _native.gather(node_id, f.feat_pos_map, f.dev_feats, f.uva_feats, f.num_total_nodes, f.feat_dim_offset,
+                          STATE.words())
 
 
 def _gather_enqueue(node_id: torch.Tensor, n_dev: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
@@ -861,20 +862,9 @@ class GATEdgeSoftmaxSum:
 def rows_gather(inp: torch.Tensor, index: torch.Tensor) -> torch.Tensor:
     """out[i] = inp[index[i]] for 2-D inp (the model's h[inverse_idx],
     python/npc/model/sage_model.py:67)."""
-    inp = _need_cuda(inp, "inp", dtype=None)
-    index = _need_cuda(index, "index")
-    out = torch.empty((index.numel(), inp.shape[1]), dtype=inp.dtype, device=inp.device)
-    check(lib.apt_rows_gather(_ptr(inp), _ptr(index), index.numel(), inp.shape[1] * inp.element_size(),
-                              _ptr(out), _stream()))
-    return out
+    return _native.rows_gather(inp, index)
 
 
 def rows_scatter(inp: torch.Tensor, index: torch.Tensor, num_out_rows: int) -> torch.Tensor:
     """out[index[i]] = inp[i]; rows of out not named by index are zero."""
-    inp = _need_cuda(inp, "inp", dtype=None)
-    index = _need_cuda(index, "index")
-    alloc = torch.empty if index.numel() == num_out_rows else torch.zeros
-    out = alloc((num_out_rows, inp.shape[1]), dtype=inp.dtype, device=inp.device)
-    check(lib.apt_rows_scatter(_ptr(inp), _ptr(index), index.numel(), inp.shape[1] * inp.element_size(),
-                               _ptr(out), _stream()))
-    return out
+    return _native.rows_scatter(inp, index, int(num_out_rows))

@@ -91,18 +91,6 @@ class _Plan:
 _CALL_BASE_SLOT = 100  # device word holding the sampler's call-id base for graph replays
 
 
-def _tunable_from_env(name: str, default: int = 0) -> int:
-    for pair in os.environ.get("APT_TUNABLES", "").split(","):
-        key, _, value = pair.partition("=")
-        if key.strip() == name and value.strip():
-            return int(value)
-    return default
-
-
-# what the process runs with outside a lane's capture (APT_TUNABLES may have set it)
-_MISS_KB_DEFAULT = _tunable_from_env("gather_miss_kb_per_block")
-
-
 class _Ring:
     """The buffer sets (plans) of one batch shape, taken in turn."""
 
@@ -142,8 +130,6 @@ class _GraphReplay:
         self._plans = {}
         # device memory the buffer sets of one batch shape may take together (APT_SAMPLER_PLAN_GB)
         self.plan_budget_bytes = int(float(os.environ.get("APT_SAMPLER_PLAN_GB", "40")) * (1 << 30))
-        # KiB to fetch per block of the copy from host memory inside a lane's graph (0: all blocks)
-        self.miss_kb_per_block = int(os.environ.get("APT_SAMPLER_MISS_KB_PER_BLOCK", "128"))
         # launches of sample_iter on a thread of their own (APT_SAMPLER_THREAD)
         self.launch_thread = os.environ.get("APT_SAMPLER_THREAD", "0") == "1"
 
@@ -199,11 +185,6 @@ class _GraphReplay:
             torch.cuda.synchronize()     # no other lane's mini-batch is in flight while this one is built
         st.lane = plan.lane
         try:
-            if on_lanes:
-                # a launch's grid is fixed when it is captured: on a lane the copy from host memory keeps
-                # only the blocks its bytes ask for, the SM slots of the others go to the kernels of the
-                # mini-batches beside it (C1, eight lanes: 6700 -> 7460 mini-batches/s)
-                check(lib.apt_set_tunable(b"gather_miss_kb_per_block", self.miss_kb_per_block))
             base_dev = st.word(_CALL_BASE_SLOT)
             # one eager run first: it sizes the cached workspaces and surfaces errors outside capture
             bufs = self._enqueue(plan.seeds_buf, base_dev)
@@ -224,8 +205,6 @@ class _GraphReplay:
             plan.keepalive = [v for k, v in st._ws.items() if k[2] == plan.lane]
         finally:
             st.lane = 0
-            if on_lanes:
-                check(lib.apt_set_tunable(b"gather_miss_kb_per_block", _MISS_KB_DEFAULT))
         ring.plans[i] = plan
         if piped and not ring.sized:
             # the first buffer set of a shape tells what one costs: keep as many as fit the budget

@@ -37,15 +37,14 @@ import torch.distributed as dist  # noqa: E402
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-STAGE_TAGS = ("sample", "relabel", "bucket", "unique_sorted", "gather_classify", "gather_hit", "gather_miss",
-              "p2p_push", "p2p_wait", "p2p_pull")
-# DRAM bytes (read + written) per algorithmic byte of the hit kernel, from an ncu capture of that kernel
+STAGE_TAGS = ("sample", "relabel", "bucket", "unique_sorted", "gather_hit", "p2p_push", "p2p_wait", "p2p_pull")
+# DRAM bytes (read + written) per algorithmic byte of the gather kernel, from an ncu capture of that kernel
 # alone at the mini-batch's size: 143 000 random rows of 512 bytes out of a 2 GB cache table moved
-# 73.3 MB of DRAM reads (every row once) and 21.5 MB of DRAM writes (the rest of the 73.2 MB written was
-# still in the 126 MB L2 when the kernel ended) for 147.6 MB algorithmic. Traffic grows with the rows.
-HIT_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (73.3 + 21.5) / 147.6
-HIT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_copy_hits at 143 000 rows x 512 B "
-                      "(94.8 MB per 147.6 MB algorithmic), scaled by this launch's algorithmic bytes; writes that "
+# 88.5 MB of DRAM reads (every row once, and a sector for each id's position) and 17.7 MB of DRAM writes (the rest of
+# the 73.2 MB written was still in the 126 MB L2 when the kernel ended) for 148.7 MB algorithmic.
+HIT_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (88.5 + 17.7) / 148.7
+HIT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_gather at 143 000 rows x 512 B "
+                      "(106.2 MB per 148.7 MB algorithmic), scaled by this launch's algorithmic bytes; writes that "
                       "stay in L2 past the kernel's end are not in it")
 # the pool's reference figure for a peer copy over NVLink, GB/s per direction (900 nominal); the benchmark
 # also measures a copy-engine peer copy in its own run and reports fractions of all three
@@ -298,7 +297,7 @@ class CpuPath:
 def stage_gather(args):
     """The cached feature gather alone: `rows` random rows out of a cache table of
     `table_rows` rows (larger than L2), a share `miss_frac` of them from pinned
-    host memory instead. One JSON line with the hit-copy kernel's roofline."""
+    host memory instead. One JSON line with the gather kernel's roofline."""
     import apt_b200  # noqa: F401
     from apt_b200 import ops
     from apt_b200._lib import lib
@@ -323,9 +322,8 @@ def stage_gather(args):
                          torch.randint(n_dev, n, (n_miss,), generator=g, device="cuda")])
         ids = ids[torch.randperm(args.rows, generator=g, device="cuda")].contiguous()
         if it == args.warmup:
-            for tag in (b"gather_hit", b"gather_miss", b"gather_classify"):
-                t, k = ctypes.c_double(), ctypes.c_int64()
-                lib.apt_profile_read(tag, ctypes.byref(t), ctypes.byref(k))
+            t, k = ctypes.c_double(), ctypes.c_int64()
+            lib.apt_profile_read(b"gather_hit", ctypes.byref(t), ctypes.byref(k))
         torch.cuda.nvtx.range_push("apt_timed")
         ev0.record()
         out = ops.load_subtensor(ids)
@@ -335,26 +333,22 @@ def stage_gather(args):
         if it >= args.warmup:
             total_ms += ev0.elapsed_time(ev1)
     ops.check_status()
-    res = {}
-    for tag in ("gather_hit", "gather_miss", "gather_classify"):
-        t, k = ctypes.c_double(), ctypes.c_int64()
-        lib.apt_profile_read(tag.encode(), ctypes.byref(t), ctypes.byref(k))
-        res[tag] = (t.value, k.value)
-    hit_ms, hit_n = res["gather_hit"]
-    # the hit kernel reads the 8-byte position of every requested row and moves every cached row once in
-    # and once out
-    hit_bytes = (args.rows - n_miss) * 2 * row_bytes + args.rows * 8
+    t, k = ctypes.c_double(), ctypes.c_int64()
+    lib.apt_profile_read(b"gather_hit", ctypes.byref(t), ctypes.byref(k))
+    hit_ms, hit_n = t.value, k.value
+    # every row once in and once out, its id and its position once in
+    hit_bytes = args.rows * (2 * row_bytes + 16)
     gbs = hit_bytes / (hit_ms / hit_n * 1e-3) / 1e9
     call_gbs = args.rows * (2 * row_bytes + 16) / (total_ms / args.steps * 1e-3) / 1e9
     print(json.dumps({
-        "metric": "cached feature gather GB/s (hit-copy kernel)", "value": gbs, "unit": "GB/s", "n_gpus": 1,
+        "metric": "cached feature gather GB/s (gather kernel)", "value": gbs, "unit": "GB/s", "n_gpus": 1,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
         "dtype": args.feat_dtype, "data": "synthetic",
         "config": {"workload": "stage gather", "rows": args.rows, "table_rows": n_dev, "row_bytes": row_bytes,
                    "miss_frac": args.miss_frac, "l2": "cache table larger than the 126 MB L2, new random ids every call"},
         "whole_call_gbs": call_gbs,
-        "stage_us": {k: 1000.0 * v[0] / max(v[1], 1) for k, v in res.items()},
-        "roofline": {"kernel": "k_copy_hits", "bound": "hbm", "achieved": round(gbs, 1), "peak": peak,
+        "stage_us": {"gather_hit": 1000.0 * hit_ms / max(hit_n, 1)},
+        "roofline": {"kernel": "k_gather", "bound": "hbm", "achieved": round(gbs, 1), "peak": peak,
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": round(gbs / peak, 4), "traffic": None}}))
 
 
@@ -1242,21 +1236,24 @@ def run():
     torch.cuda.synchronize()
     ops.profile_enable(False)
     empty_ms, empty_n = prof("gather_hit")
-    for tag in ("gather_classify", "gather_miss"):
-        prof(tag)
     bracket_us = 1000.0 * empty_ms / max(empty_n, 1)
     pos_map = ops.STATE.feat.feat_pos_map
+    # the gather of each step's cached rows alone: the step's own launch also reads rows over the host link
+    ops.profile_enable(True)
+    for k in kept:
+        ops._gather_enqueue(k[pos_map[k] >= 0], None)
+    torch.cuda.synchronize()
+    ops.profile_enable(False)
+    hit_ms, hit_n = prof("gather_hit")
     rows_total = sum(int(k.numel()) for k in kept)
     hits_total = sum(int((pos_map[k] >= 0).sum().item()) for k in kept)
     miss_total = rows_total - hits_total
     peak, peak_kind = peaks()
-    hit_ms, hit_n = stage_ms["gather_hit"]
-    miss_ms, miss_n = stage_ms["gather_miss"]
-    # algorithmic bytes of one launch of the hit kernel: each cached row once in and once out, plus the
-    # 8-byte position of every requested row
-    hit_bytes = (hits_total * 2 * row_bytes + rows_total * 8) / max(hit_n, 1)
+    miss_ms, miss_n = stage_ms["gather_hit"]
+    # algorithmic bytes of one launch: each cached row once in and once out, plus its 8-byte id and position
+    hit_bytes = hits_total * (2 * row_bytes + 16) / max(hit_n, 1)
     hit_gbs = hit_bytes / (hit_ms / max(hit_n, 1) * 1e-3) / 1e9 if hit_ms > 0 else 0.0
-    roofline = {"kernel": "k_copy_hits (gather, cache hits)", "bound": "hbm",
+    roofline = {"kernel": "k_gather (the step's cached rows)", "bound": "hbm",
                 "achieved": round(hit_gbs, 1), "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": round(hit_gbs / peak, 4),
                 # the capture holds for launches of its kind: 512-byte rows, a batch that fits the L2 twice over
@@ -1264,7 +1261,7 @@ def run():
                 if row_bytes == 512 and hit_bytes < 4e8 else None,
                 "traffic_source": HIT_TRAFFIC_SOURCE if row_bytes == 512 and hit_bytes < 4e8 else
                 "not captured for launches of this size",
-                "measured_in": "the pass that enqueues the kernels one by one with an event pair around each",
+                "measured_in": "a gather of each step's cached rows alone, an event pair around each launch",
                 "rows_per_launch": rows_total / max(hit_n, 1),
                 "hit_rows_per_launch": hits_total / max(hit_n, 1), "us_per_launch": 1000.0 * hit_ms / max(hit_n, 1),
                 "us_per_empty_launch": round(bracket_us, 2),
@@ -1273,7 +1270,7 @@ def run():
     miss_bytes = miss_total * row_bytes / max(miss_n, 1)
     miss_gbs = miss_bytes / (miss_ms / max(miss_n, 1) * 1e-3) / 1e9 if miss_ms > 0 else 0.0
 
-    # ---- measured host-link rate (pinned host -> device copy), the miss kernel's ceiling
+    # ---- measured host-link rate (pinned host -> device copy), the ceiling of the rows read from host memory
     phase("host_link_probe")
     probe_rows = min(int(inst.host_feats.shape[0]), (1 << 30) // row_bytes)
     dst = torch.empty((probe_rows, w.feat_dim), dtype=inst.host_feats.dtype, device="cuda")
@@ -1286,7 +1283,8 @@ def run():
     torch.cuda.synchronize()
     link_gbs = probe_rows * row_bytes / (e0.elapsed_time(e1) * 1e-3) / 1e9
     del dst
-    roofline_link = {"kernel": "k_copy_miss (gather, rows from pinned host memory)", "bound": "host_link",
+    roofline_link = {"kernel": "k_gather (the step's whole request: the rows from pinned host memory beside the cached ones)",
+                     "bound": "host_link",
                      "achieved": round(miss_gbs, 2), "peak": round(link_gbs, 2),
                      "peak_kind": "pinned host->device copy of 1 GiB measured in this run", "unit": "GB/s",
                      "frac": round(miss_gbs / link_gbs, 4) if link_gbs else None,
