@@ -108,6 +108,19 @@ k_bucket_scatter(const int64_t* __restrict__ ids, int64_t n, const int64_t* __re
   }
 }
 
+// One rank owns every id: the partition is the input, in one launch.
+__global__ void __launch_bounds__(256)
+k_bucket_one_rank(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev, int64_t* __restrict__ sorted,
+                  int64_t* __restrict__ perm, int64_t* __restrict__ sizes, int64_t* __restrict__ offsets) {
+  n = effective_n(n, n_dev);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    sorted[i] = ids[i];
+    perm[i] = i;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) sizes[0] = sizes[1] = offsets[0] = n;
+}
+
 // out = cat(a[0:na], b[0:nb]) with both lengths taken from device words (the input nodes of an
 // SNP-GAT mini-batch: the local destination nodes followed by the ids received from the peers,
 // python/npc/sampler.py:230).
@@ -129,90 +142,147 @@ k_concat_ids(const int64_t* __restrict__ a, int64_t na, const int64_t* __restric
 // bit per id, level 1 one bit per level-0 word that is not zero. Counting,
 // ranking and emitting walk level 1 only (range/1024 words), so the cost of a
 // call follows the number of ids, not the width of the range. Both levels are
-// all-zero between calls: the call clears exactly the words it set. Four launches:
-// mark, emit (count + ordered ranks in one pass), inverse, clear.
-constexpr int kUniqBlock = 1024;
+// all-zero between calls: the pass that emits the ids also clears what it read.
+// Three launches: mark, emit (count, ordered ranks, clear), inverse.
+constexpr int kUniqBlock = 256;
 
+// Runs of lanes whose ids share a word (the virtual ids of a sampled hop come in runs of its fanout) are joined
+// first: one atomic a run. 23 000 ids in runs of 25: 24 us with one an id.
 __global__ void __launch_bounds__(256)
 k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
             int64_t lo, int64_t hi, uint32_t* __restrict__ l0, uint32_t* __restrict__ l1,
             int32_t* status) {
   n = effective_n(n, n_dev);
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int flags = 0;
-  for (; i < n; i += stride) {
-    const int64_t v = ids[i];
-    if (v < lo || v >= hi) {
-      flags |= APT_FLAG_ID_OUT_OF_RANGE;
-      continue;
+  // whole warps iterate together
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i - lane < n; i += stride) {
+    uint32_t w = 0xffffffffu, bits = 0u;      // words of the range number less than 2^31
+    if (i < n) {
+      const int64_t v = ids[i];
+      if (v < lo || v >= hi) {
+        flags |= APT_FLAG_ID_OUT_OF_RANGE;
+      } else {
+        w = (uint32_t)((v - lo) >> 5);
+        bits = 1u << ((v - lo) & 31);
+      }
     }
-    const int64_t r = v - lo;
-    const uint32_t bit = 1u << (r & 31);
-    const int64_t w = r >> 5;
-    if (*(volatile uint32_t*)(l0 + w) & bit) continue;
-    const uint32_t old = atomicOr(l0 + w, bit);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t w2 = __shfl_down_sync(0xffffffffu, w, o), b2 = __shfl_down_sync(0xffffffffu, bits, o);
+      if (lane + o < 32 && w2 == w) bits |= b2;
+    }
+    const uint32_t before = __shfl_up_sync(0xffffffffu, w, 1);
+    if (w == 0xffffffffu || (lane > 0 && before == w)) continue;
+    if ((*(volatile uint32_t*)(l0 + w) & bits) == bits) continue;
+    const uint32_t old = atomicOr(l0 + w, bits);
     if (old == 0) atomicOr(l1 + (w >> 5), 1u << (w & 31));  // first bit of this word
   }
   if (flags) atomicOr(status, flags);
 }
 
-// Ids under one level-1 word (up to 1024 of them).
-__device__ __forceinline__ int l1_word_count(const uint32_t* __restrict__ l0, int64_t w1, uint32_t bits) {
-  int c = 0;
-  while (bits) {
-    const int b = __ffs(bits) - 1;
-    bits &= bits - 1;
-    c += __popc(l0[(w1 << 5) + b]);
-  }
-  return c;
-}
+// Counting, ranking, emitting and clearing in one launch. A warp has `per_warp` (up to 32) consecutive level-1 words,
+// a lane to each. A lane with few level-0 words below its own (a wide range) walks them itself, all loads in flight;
+// where there are many the warp's lanes take the 32 words together, one level-1 word after another (a dense range: a
+// million ids below one thousand level-1 words; one thread to a word walked 1024 ids alone, 75 to 430 us).
+// The blocks' counts are chained by the look-back of common.cuh. info[w] = (rank of the word's first id, its bits).
+constexpr int kOwnWords = 8, kOwnIds = 32;
 
-// Counting, ranking and emitting in one launch: a tile of kUniqBlock level-1 words counts its ids,
-// the tiles' counts are chained by the look-back of common.cuh, and the tile writes its ids in order.
 __global__ void __launch_bounds__(kUniqBlock)
-k_uniq_emit(const uint32_t* __restrict__ l0, const uint32_t* __restrict__ l1, int64_t nwords1,
-            int64_t lo, ScanCtrl* ctrl, uint64_t* tile_state,
-            uint32_t* __restrict__ word_prefix, int64_t* __restrict__ out_unique,
-            int64_t* __restrict__ out_num_unique, int32_t* status) {
-  __shared__ int warp_sums[33];
+k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords1, int per_warp,
+            int64_t lo, ScanCtrl* ctrl, uint64_t* tile_state, uint2* __restrict__ info,
+            int64_t* __restrict__ out_unique, int64_t* __restrict__ out_num_unique, int32_t* status) {
+  __shared__ uint32_t warp_total[kUniqBlock / 32];
   __shared__ uint32_t s_tile, s_epoch, s_before;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) tile_ticket(ctrl, &s_tile, &s_epoch);
   __syncthreads();
   const uint32_t tile = s_tile;
-  const int64_t w1 = (int64_t)tile * blockDim.x + threadIdx.x;
-  uint32_t bits1 = w1 < nwords1 ? l1[w1] : 0u;
-  int total;
-  const int ex = block_exclusive_scan(l1_word_count(l0, w1, bits1), warp_sums, &total);
-  if (threadIdx.x < 32) {
-    const uint32_t before = tile_lookback(tile_state, tile, s_epoch, (uint32_t)total, status, APT_FLAG_TABLE_FULL);
-    if (threadIdx.x == 0) s_before = before;
+  const int64_t first = ((int64_t)tile * (kUniqBlock / 32) + warp) * per_warp;
+  const uint32_t mine = lane < per_warp && first + lane < nwords1 ? l1[first + lane] : 0u;
+  uint32_t word[kOwnWords], count = 0;
+  const bool few = __popc(mine) <= kOwnWords;
+  uint32_t rest = mine;
+#pragma unroll
+  for (int q = 0; q < kOwnWords; ++q) {
+    word[q] = few && rest ? l0[((first + lane) << 5) + __ffs(rest) - 1] : 0u;
+    rest &= rest - 1;
+  }
+#pragma unroll
+  for (int q = 0; q < kOwnWords; ++q) count += __popc(word[q]);
+  for (unsigned m = __ballot_sync(0xffffffffu, !few); m; m &= m - 1) {
+    const int k = __ffs(m) - 1;
+    const uint32_t mask = __shfl_sync(0xffffffffu, mine, k);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, mask >> lane & 1u ? __popc(l0[((first + k) << 5) + lane]) : 0u);
+    if (lane == k) count = c;
+  }
+  uint32_t upto_lane = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, upto_lane, o);
+    if (lane >= o) upto_lane += t;
+  }
+  if (lane == 31) warp_total[warp] = upto_lane;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int k = 0; k < kUniqBlock / 32; ++k) {
+    if (k < warp) before += warp_total[k];
+    total += warp_total[k];
+  }
+  if (warp == 0) {
+    const uint32_t b = tile_lookback(tile_state, tile, s_epoch, total, status, APT_FLAG_TABLE_FULL);
+    if (lane == 0) s_before = b;
   }
   __syncthreads();
   if (tile == gridDim.x - 1 && threadIdx.x == 0) *out_num_unique = (int64_t)s_before + total;
-  int64_t at = (int64_t)s_before + ex;
-  while (bits1) {
-    const int b1 = __ffs(bits1) - 1;
-    bits1 &= bits1 - 1;
-    const int64_t w = (w1 << 5) + b1;
-    uint32_t bits = l0[w];
-    word_prefix[w] = (uint32_t)at;      // rank of the word's first id; only non-zero words are ever looked up
-    const int64_t base = lo + (w << 5);
-    while (bits) {
-      const int b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      out_unique[at++] = base + b;
+  int64_t at = (int64_t)s_before + before + upto_lane - count;      // rank of the first id below this lane's word
+  const bool own = few && count <= kOwnIds;
+  for (unsigned m = __ballot_sync(0xffffffffu, !own); m; m &= m - 1) {
+    const int k = __ffs(m) - 1;
+    const uint32_t mask = __shfl_sync(0xffffffffu, mine, k);
+    const int64_t start = __shfl_sync(0xffffffffu, at, k);
+    const int64_t w = ((first + k) << 5) + lane;
+    const uint32_t bits = mask >> lane & 1u ? l0[w] : 0u;
+    uint32_t upto = __popc(bits);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    const uint32_t here = upto - __popc(bits);
+    if (bits) {
+      info[w] = make_uint2((uint32_t)(start + here), bits);
+      l0[w] = 0u;
+    }
+    // the ids of one level-0 word at a time, a lane to a bit
+    for (uint32_t q = mask; q; q &= q - 1) {
+      const int j = __ffs(q) - 1;
+      const uint32_t x = __shfl_sync(0xffffffffu, bits, j), rank = __shfl_sync(0xffffffffu, here, j);
+      if (x >> lane & 1u) out_unique[start + rank + __popc(x & ((1u << lane) - 1u))] = lo + ((((first + k) << 5) + j) << 5) + lane;
     }
   }
+  if (own) {
+    rest = mine;
+#pragma unroll
+    for (int q = 0; q < kOwnWords; ++q) {
+      if (!rest) break;
+      const int64_t w = ((first + lane) << 5) + __ffs(rest) - 1;
+      rest &= rest - 1;
+      info[w] = make_uint2((uint32_t)at, word[q]);
+      l0[w] = 0u;
+      for (uint32_t bits = word[q]; bits; bits &= bits - 1) out_unique[at++] = lo + (w << 5) + __ffs(bits) - 1;
+    }
+  }
+  if (lane < per_warp && mine) l1[first + lane] = 0u;
   __syncthreads();
   if (threadIdx.x == 0) tile_done(ctrl, s_epoch);
 }
 
 __global__ void __launch_bounds__(256)
 k_uniq_inverse(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
-               int64_t lo, int64_t hi, const uint32_t* __restrict__ l0,
-               const uint32_t* __restrict__ word_prefix,
-               int64_t* __restrict__ out_inverse) {
+               int64_t lo, int64_t hi, const uint2* __restrict__ info, int64_t* __restrict__ out_inverse) {
   n = effective_n(n, n_dev);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -223,25 +293,8 @@ k_uniq_inverse(const int64_t* __restrict__ ids, int64_t n, const int64_t* __rest
       continue;
     }
     const int64_t r = v - lo;
-    const uint32_t bits = l0[r >> 5];
-    out_inverse[i] = (int64_t)word_prefix[r >> 5] +
-                     __popc(bits & ((1u << (r & 31)) - 1u));
-  }
-}
-
-// Puts both levels back to zero by revisiting the ids that set them.
-__global__ void __launch_bounds__(256)
-k_uniq_clear(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
-             int64_t lo, int64_t hi, uint32_t* __restrict__ l0, uint32_t* __restrict__ l1) {
-  n = effective_n(n, n_dev);
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) {
-    const int64_t v = ids[i];
-    if (v < lo || v >= hi) continue;
-    const int64_t w = (v - lo) >> 5;
-    l0[w] = 0u;
-    l1[w >> 5] = 0u;
+    const uint2 w = info[r >> 5];
+    out_inverse[i] = (int64_t)w.x + __popc(w.y & ((1u << (r & 31)) - 1u));
   }
 }
 
@@ -290,6 +343,11 @@ extern "C" int apt_bucket_by_owner(const int64_t* ids, int64_t num_ids,
   const int nblocks = (int)ceil_div(num_ids, kBucketBlock);
   int32_t* hist = (int32_t*)workspace;
   ProfScope prof("bucket", s);
+  if (world_size == 1) {
+    APT_LAUNCH(k_bucket_one_rank, wave_grid(ceil_div(num_ids, 256), 8, 1), 256, 0, s, ids, num_ids, num_ids_dev, out_sorted,
+               out_perm, out_bucket_sizes, out_bucket_offsets);
+    return APT_OK;
+  }
   APT_LAUNCH(k_bucket_count, nblocks, kBucketBlock, 0, s, ids, num_ids, num_ids_dev, min_vids, p, hist, nblocks);
   APT_LAUNCH(k_bucket_scatter, nblocks, kBucketBlock, 0, s, ids, num_ids, num_ids_dev, min_vids, p, hist,
              nblocks, out_sorted, out_perm, out_bucket_sizes, out_bucket_offsets);
@@ -300,30 +358,34 @@ namespace apt {
 struct UniqWs {
   uint32_t* l0;           // [nwords0] one bit per id
   uint32_t* l1;           // [nwords1] one bit per level-0 word
-  uint32_t* word_prefix;  // [nwords0]
+  uint2* info;            // [nwords1 * 32] rank of the word's first id and its bits, of the words the call set
   ScanCtrl* ctrl;         // [1]        control words of the ordered emit, zero once
   uint64_t* tile_state;   // [nblocks]  its tile states, tagged by call
   int64_t nwords0, nwords1;
-  int nblocks;
+  int nblocks, per_warp;
   size_t bitmap_bytes;    // l0 + l1: the part that has to be zero between calls
 };
 static size_t uniq_layout(int64_t range, char* base, UniqWs* ws) {
   const int64_t nwords0 = ceil_div(range > 0 ? range : 1, 32);
   const int64_t nwords1 = ceil_div(nwords0, 32);
-  const int nblocks = (int)ceil_div(nwords1, kUniqBlock);
+  // level-1 words a warp: few enough that a narrow range still spreads over the SMs, 32 at most
+  int per_warp = 1;
+  while (per_warp < 32 && (int64_t)per_warp * kNumSMs * (kUniqBlock / 32) < nwords1) per_warp <<= 1;
+  const int nblocks = (int)ceil_div(nwords1, (int64_t)per_warp * (kUniqBlock / 32));
   const size_t b0 = align_up((size_t)nwords1 * 32 * 4, 256);  // level 0, padded to whole level-1 words
   const size_t b1 = align_up((size_t)nwords1 * 4, 256);
-  const size_t b2 = align_up((size_t)nwords0 * 4, 256);
+  const size_t b2 = align_up((size_t)nwords1 * 32 * 8, 256);
   const size_t b3 = align_up(sizeof(ScanCtrl) + (size_t)nblocks * 8, 256);
   if (ws) {
     ws->l0 = (uint32_t*)base;
     ws->l1 = (uint32_t*)(base + b0);
-    ws->word_prefix = (uint32_t*)(base + b0 + b1);
+    ws->info = (uint2*)(base + b0 + b1);
     ws->ctrl = (ScanCtrl*)(base + b0 + b1 + b2);
     ws->tile_state = (uint64_t*)(base + b0 + b1 + b2 + sizeof(ScanCtrl));
     ws->nwords0 = nwords0;
     ws->nwords1 = nwords1;
     ws->nblocks = nblocks;
+    ws->per_warp = per_warp;
     ws->bitmap_bytes = b0 + b1;
   }
   return b0 + b1 + b2 + b3;
@@ -371,11 +433,9 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
   ProfScope prof("unique_sorted", s);
   const int g = wave_grid(ceil_div(num_ids, 256), 8);
   APT_LAUNCH(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, status_word);
-  APT_LAUNCH(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, id_lo, ws.ctrl, ws.tile_state,
-             ws.word_prefix, out_unique, out_num_unique, status_word);
-  APT_LAUNCH(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0,
-             ws.word_prefix, out_inverse);
-  APT_LAUNCH(k_uniq_clear, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1);
+  APT_LAUNCH(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.ctrl, ws.tile_state,
+             ws.info, out_unique, out_num_unique, status_word);
+  APT_LAUNCH(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.info, out_inverse);
   return APT_OK;
 }
 
