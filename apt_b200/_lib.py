@@ -42,6 +42,8 @@ PROTOTYPES = {
     "apt_relabel_csc": (c_int, [P, c_int64, P, P, c_int64, P, c_size_t, P, P, P, P, P]),
     "apt_sample_relabel_csc": (c_int, [P, c_int64, P, c_int, P, c_int64, P, P, P, P, c_uint64, c_uint32, P, P, c_size_t,
                                        P, P, P, P, P, P]),
+    "apt_sample_relabel_block": (c_int, [P, c_int64, P, c_int, P, c_int64, P, P, P, P, c_uint64, c_uint32, P, P, c_size_t,
+                                         P, P, P, P, P, P, P]),
     "apt_bucket_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "apt_bucket_by_owner": (c_int, [P, c_int64, P, P, c_int, c_int64, c_int, c_int, c_int, P, c_size_t, P, P, P, P, P]),
     "apt_unique_workspace_bytes": (c_size_t, [c_int64]),

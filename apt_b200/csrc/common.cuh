@@ -133,6 +133,13 @@ __device__ __forceinline__ uint4 ld_plain_16(const void* p) {
   return v;
 }
 
+// Two 8-byte words in one load that is not served from L1: for words that other blocks change meanwhile.
+__device__ __forceinline__ ulonglong2 ld_volatile_2x8(const void* p) {
+  ulonglong2 v;
+  asm volatile("ld.volatile.global.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ uint64_t global_timer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -13,12 +13,14 @@
 //                   library the sampling kernel does this itself
 //                   (sample_replace_kernel<G, true>, apt_sample_relabel_csc) and the
 //                   neighbour list is never read back.
-//   k_scan_assign   single-pass ordered compaction (tile counts chained by a
-//                   look-back over the tiles before): new id = first occurrences
-//                   before the item; writes unique[], the slot's new id and the
-//                   number of unique ids
-//   k_relabel       neighbours -> new id through the remembered slot; the first
-//                   occurrence of every id also empties its slot again
+//   k_first         which items are first occurrences: one bit an item, and the number of
+//                   ones before every 32 items of a tile and in every tile. Leaves the
+//                   position of an id's first occurrence beside every other item.
+//   k_relabel       the new id of an id is the number of ones before its first occurrence: a
+//                   tile's share (added up by every block in shared memory) plus a look at
+//                   the bits. No block waits for another one; the form before this chained its
+//                   tiles by a look-back and sent the ids through the table (1.08 M items:
+//                   29 + 20 us). The first occurrence also empties its id's slot.
 //
 // Layers of up to 8192 items run in one block with the table in shared memory
 // (k_relabel_small below).
@@ -35,23 +37,23 @@ constexpr int kRelabelBlock = 1024;
 static size_t relabel_bytes_for(int64_t items) {
   const int64_t n = items > 0 ? items : 1;
   return align_up((size_t)relabel_capacity(n) * sizeof(Slot), 256) + align_up((size_t)n * 4, 256) +
-         align_up(sizeof(ScanCtrl) + (size_t)(ceil_div(n, kScanTile) + 1) * 8, 256);
+         align_up((size_t)(n / 32 + 1) * 8, 256) + (size_t)kMaxTiles * 4;
 }
 
 // The layout depends only on the size of the workspace, not on the call, so
 // that "empty between calls" holds for one fixed slot region.
 static bool relabel_layout(char* base, size_t bytes, RelabelWs* ws) {
-  // 16 * 1.5 + 4 bytes per item plus a little: first guess, then shrink until it fits
-  int64_t items = bytes > 4096 ? (int64_t)((bytes - 4096) / 281 * 10) : 0;
+  // 16 * 1.5 + 4 + 8 / 32 bytes per item plus the tiles: first guess, then shrink until it fits
+  int64_t items = bytes > 20480 ? (int64_t)((bytes - 20480) / 283 * 10) : 0;
   while (items > 0 && relabel_bytes_for(items) > bytes) items -= 1 + items / 4096;
   ws->items_ws = items;
   if (items <= 0) return false;
   const size_t o_slot_of = align_up((size_t)relabel_capacity(items) * sizeof(Slot), 256);
-  const size_t o_ctrl = o_slot_of + align_up((size_t)items * 4, 256);
+  const size_t o_words = o_slot_of + align_up((size_t)items * 4, 256);
   ws->slots = (Slot*)base;
   ws->slot_of = (int32_t*)(base + o_slot_of);
-  ws->ctrl = (ScanCtrl*)(base + o_ctrl);
-  ws->tile_state = (uint64_t*)(base + o_ctrl + sizeof(ScanCtrl));
+  ws->words = (uint2*)(base + o_words);
+  ws->tile_count = (int32_t*)(base + o_words + align_up((size_t)(items / 32 + 1) * 8, 256));
   return true;
 }
 
@@ -73,92 +75,128 @@ k_insert(const int64_t* __restrict__ seeds, int64_t S_host, const int64_t* __res
   if (flags) atomicOr(status, flags);
 }
 
-// ---- pass 2: ordered compaction in one launch ----------------------------------------
-// An item is a first occurrence iff its slot's smallest position is its own. Tiles of
-// kScanTile consecutive items; their counts are chained by the look-back of common.cuh.
-__global__ void __launch_bounds__(kScanThreads)
-k_scan_assign(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed,
-              RelabelWs ws, int64_t* __restrict__ out_unique, int64_t* __restrict__ out_num_unique,
-              int32_t* status) {
-  __shared__ int scratch[33];
-  __shared__ uint32_t s_tile, s_epoch, s_before;
+// ---- pass 2: first occurrences --------------------------------------------------------
+// One block to a tile of 2^tile_shift (at least kSubTile) consecutive items.
+constexpr int kFirstThreads = 256;
+constexpr int kFirstItems = 4;
+constexpr int kSubTile = kFirstThreads * kFirstItems;
+static_assert(kSubTile / 32 == 32, "a sub-tile's words are scanned by one warp");
+
+__global__ void __launch_bounds__(kFirstThreads)
+k_first(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, RelabelWs ws, int tile_shift) {
+  __shared__ uint32_t counts[32], bases[32];
   const RelabelDims d = relabel_dims(S_host, M_host, S_dev, per_seed);
-  if (threadIdx.x == 0) tile_ticket(ws.ctrl, &s_tile, &s_epoch);
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  const int64_t first = (int64_t)tile * kScanTile;
-  if (first < d.n || tile == 0) {
-    // consecutive items of one thread: the block scan over thread sums keeps item order
-    const int64_t i0 = first + (int64_t)threadIdx.x * kScanItems;
-    int32_t slot[kScanItems];
-    uint4 sv[kScanItems];
-    int f[kScanItems];
-    int mine = 0;
+  const int64_t first = (int64_t)blockIdx.x << tile_shift;
+  if (first >= d.n) return;
+  const int64_t last = min(d.n, first + ((int64_t)1 << tile_shift));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t running = 0;
+  for (int64_t base = first; base < last; base += kSubTile) {
+    int32_t slot[kFirstItems];
+    uint32_t min_pos[kFirstItems];
+    unsigned ones[kFirstItems];
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) slot[k] = i0 + k < d.n ? ws.slot_of[i0 + k] : -1;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k)
-      if (slot[k] >= 0) sv[k] = ld_plain_16((const uint4*)(ws.slots + slot[k]));
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      f[k] = slot[k] >= 0 && sv[k].z == (uint32_t)(i0 + k);
-      mine += f[k];
+    for (int k = 0; k < kFirstItems; ++k) {
+      const int64_t i = base + k * kFirstThreads + threadIdx.x;
+      slot[k] = i < last ? ws.slot_of[i] : -1;
     }
-    int total;
-    const int ex = block_exclusive_scan(mine, scratch, &total);
-    if (threadIdx.x < 32) {
-      const uint32_t before = tile_lookback(ws.tile_state, tile, s_epoch, (uint32_t)total, status, APT_FLAG_TABLE_FULL);
-      if (threadIdx.x == 0) s_before = before;
+#pragma unroll
+    for (int k = 0; k < kFirstItems; ++k) min_pos[k] = slot[k] >= 0 ? ws.slots[slot[k]].min_pos : kNoPos;
+#pragma unroll
+    for (int k = 0; k < kFirstItems; ++k) {
+      const int64_t i = base + k * kFirstThreads + threadIdx.x;
+      const bool one = slot[k] >= 0 && min_pos[k] == (uint32_t)i;
+      ones[k] = __ballot_sync(0xffffffffu, one);
+      if (lane == 0) counts[k * (kFirstThreads / 32) + warp] = __popc(ones[k]);
+      if (slot[k] >= 0 && !one) ws.slot_of[i] = (int32_t)min_pos[k];
     }
     __syncthreads();
-    uint32_t id = s_before + (uint32_t)ex;
+    if (warp == 0) {
+      const uint32_t c = counts[lane];
+      uint32_t upto = c;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (f[k]) {
-        out_unique[id] = (int64_t)(((uint64_t)sv[k].y << 32) | sv[k].x);   // the slot's key is the id
-        ws.slots[slot[k]].new_id = id;
-        ++id;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += t;
       }
+      bases[lane] = running + upto - c;
+      running += __shfl_sync(0xffffffffu, upto, 31);
     }
-    // the tile that holds the last item (or the only, empty tile) knows the number of unique ids
-    if (threadIdx.x == 0 && first + kScanTile >= d.n) *out_num_unique = (int64_t)s_before + total;
+    __syncthreads();
+    if (lane < kFirstItems) {
+      const int w = lane * (kFirstThreads / 32) + warp;
+      unsigned mine = ones[0];
+#pragma unroll
+      for (int k = 1; k < kFirstItems; ++k)
+        if (lane == k) mine = ones[k];
+      if (base + w * 32 < last) ws.words[(base >> 5) + w] = make_uint2(bases[w], mine);
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) tile_done(ws.ctrl, s_epoch);
+  if (threadIdx.x == 0) ws.tile_count[blockIdx.x] = (int32_t)running;
 }
 
-// ---- pass 3: neighbours -> new id through the remembered slot; the first occurrence
-// of every id also empties its slot again with one 16-byte store.
+// ---- pass 3: new ids ------------------------------------------------------------------
+// out_col (may be null): the position of each neighbour's seed, the other side of the block's edges.
 __global__ void __launch_bounds__(256)
-k_relabel(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed,
-          RelabelWs ws, int64_t* __restrict__ out) {
+k_relabel(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, RelabelWs ws, int tile_shift,
+          int64_t* __restrict__ out_unique, int64_t* __restrict__ out, int64_t* __restrict__ out_col,
+          int64_t* __restrict__ out_num_unique) {
+  __shared__ int tile_base[kMaxTiles];
+  __shared__ int scratch[33];
   const RelabelDims d = relabel_dims(S_host, M_host, S_dev, per_seed);
+  const int tiles = (int)((d.n + ((int64_t)1 << tile_shift) - 1) >> tile_shift);
+  const int each = (tiles + (int)blockDim.x - 1) / (int)blockDim.x;
+  for (int t = threadIdx.x; t < tiles; t += blockDim.x) tile_base[t] = ws.tile_count[t];
+  __syncthreads();
+  int mine = 0;
+  const int t0 = threadIdx.x * each, t1 = min(tiles, t0 + each);
+  for (int t = t0; t < t1; ++t) mine += tile_base[t];
+  int total;
+  int at = block_exclusive_scan(mine, scratch, &total);
+  for (int t = t0; t < t1; ++t) {
+    const int c = tile_base[t];
+    tile_base[t] = at;
+    at += c;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *out_num_unique = total;
+  __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   constexpr int K = 4;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; base < d.n; base += stride * K) {
-    int32_t slot[K];
-    uint4 v[K];
+    int32_t v[K];
+    uint2 word[K];
+    unsigned long long key[K];
+    bool one[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int64_t i = base + k * stride;
-      slot[k] = i < d.n ? ws.slot_of[i] : -2;
+      v[k] = i < d.n ? ws.slot_of[i] : -1;
+      one[k] = v[k] >= 0 && (ws.words[i >> 5].y >> (i & 31) & 1u);
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (slot[k] >= 0) v[k] = ld_plain_16((const uint4*)(ws.slots + slot[k]));
+    for (int k = 0; k < K; ++k) {
+      if (v[k] < 0) continue;
+      // where the id occurs first: here, or at the position that pass 2 left
+      const uint32_t pos = one[k] ? (uint32_t)(base + k * stride) : (uint32_t)v[k];
+      word[k] = ws.words[pos >> 5];
+      if (one[k]) key[k] = ws.slots[v[k]].key;
+    }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int64_t i = base + k * stride;
-      if (slot[k] == -2) continue;
-      if (slot[k] < 0) {
+      if (i >= d.n) continue;
+      if (out_col && i >= d.S) out_col[i - d.S] = (int64_t)((uint32_t)(i - d.S) / (uint32_t)per_seed);
+      if (v[k] < 0) {
         if (i >= d.S) out[i - d.S] = -1;
         continue;
       }
-      if (i >= d.S) out[i - d.S] = (int64_t)v[k].w;
-      // Nothing reads keys any more and only the first occurrence itself compares positions:
-      // that item empties the slot (the new id stays for the items that have not read it yet).
-      if (v[k].z == (uint32_t)i)
-        st_plain_16((uint4*)(ws.slots + slot[k]), make_uint4(0xffffffffu, 0xffffffffu, kNoPos, v[k].w));
+      const uint32_t pos = one[k] ? (uint32_t)i : (uint32_t)v[k];
+      const int64_t id = (int64_t)tile_base[pos >> tile_shift] + word[k].x + __popc(word[k].y & ((1u << (pos & 31)) - 1u));
+      if (i >= d.S) out[i - d.S] = id;
+      if (one[k]) {
+        out_unique[id] = (int64_t)key[k];
+        st_plain_16((uint4*)(ws.slots + v[k]), make_uint4(0xffffffffu, 0xffffffffu, kNoPos, 0xffffffffu));
+      }
     }
   }
 }
@@ -186,7 +224,7 @@ constexpr size_t kSmallSmem = (size_t)kSmallCap * sizeof(Slot) + (size_t)kSmallI
 __global__ void __launch_bounds__(kRelabelBlock)
 k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __restrict__ nbrs,
                 int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, int erase_nbrs,
-                int64_t* __restrict__ out_unique, int64_t* __restrict__ out_relabeled,
+                int64_t* __restrict__ out_unique, int64_t* __restrict__ out_relabeled, int64_t* __restrict__ out_col,
                 int64_t* __restrict__ out_num_unique, int32_t* status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int scratch[33];
@@ -197,7 +235,7 @@ k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __re
   for (uint32_t t = threadIdx.x; t < kSmallCap; t += blockDim.x) {
     slots[t].key = kEmptyKey;
     slots[t].min_pos = kNoPos;
-    slots[t].new_id = 0;
+    slots[t].pad = 0;
   }
   __syncthreads();
   int flags = 0;
@@ -234,14 +272,16 @@ k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __re
     if (f) {
       const int id = running + ex;
       out_unique[id] = (int64_t)slots[slot_of[i]].key;
-      slots[slot_of[i]].new_id = (uint32_t)id;
+      slots[slot_of[i]].pad = (uint32_t)id;
     }
     running += total;
   }
   if (threadIdx.x == 0) *out_num_unique = running;
   __syncthreads();
-  for (int i = (int)d.S + threadIdx.x; i < n; i += blockDim.x)
-    out_relabeled[i - d.S] = slot_of[i] == kSmallNoSlot ? (int64_t)-1 : (int64_t)slots[slot_of[i]].new_id;
+  for (int i = (int)d.S + threadIdx.x; i < n; i += blockDim.x) {
+    out_relabeled[i - d.S] = slot_of[i] == kSmallNoSlot ? (int64_t)-1 : (int64_t)slots[slot_of[i]].pad;
+    if (out_col) out_col[i - d.S] = (int64_t)((uint32_t)(i - d.S) / (uint32_t)per_seed);
+  }
 }
 
 static int set_small_smem() {
@@ -256,14 +296,17 @@ static int set_small_smem() {
 }
 
 // Passes 2 and 3 of the multi-block path (the table already holds every item).
-static int scan_and_relabel(int64_t num_seeds, int64_t num_neighbors, const int64_t* num_seeds_dev,
-                            int64_t per_seed, const RelabelWs& ws, int64_t* out_unique, int64_t* out_relabeled,
-                            int64_t* out_num_unique, int32_t* status_word, cudaStream_t s) {
+static int first_and_relabel(int64_t num_seeds, int64_t num_neighbors, const int64_t* num_seeds_dev,
+                             int64_t per_seed, const RelabelWs& ws, int64_t* out_unique, int64_t* out_relabeled,
+                             int64_t* out_col, int64_t* out_num_unique, cudaStream_t s) {
   const int64_t n = num_seeds + num_neighbors;
-  APT_LAUNCH(k_scan_assign, (int)ceil_div(n, kScanTile), kScanThreads, 0, s, num_seeds, num_neighbors,
-             num_seeds_dev, per_seed, ws, out_unique, out_num_unique, status_word);
+  int tile_shift = 10;
+  while (ceil_div(n, (int64_t)1 << tile_shift) > kMaxTiles) ++tile_shift;
+  APT_LAUNCH(k_first, (int)ceil_div(n, (int64_t)1 << tile_shift), kFirstThreads, 0, s, num_seeds, num_neighbors, num_seeds_dev,
+             per_seed, ws, tile_shift);
   const int grid = wave_grid(ceil_div(n, 256 * 4), 8, 1);
-  APT_LAUNCH(k_relabel, grid, 256, 0, s, num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, out_relabeled);
+  APT_LAUNCH(k_relabel, grid, 256, 0, s, num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, tile_shift, out_unique,
+             out_relabeled, out_col, out_num_unique);
   return APT_OK;
 }
 
@@ -279,12 +322,6 @@ extern "C" int apt_relabel_workspace_init(void* workspace, size_t workspace_byte
   using namespace apt;
   APT_CHECK_ARG(workspace && workspace_bytes > 0, "apt_relabel_workspace_init: null workspace");
   APT_CUDA(cudaMemsetAsync(workspace, 0xff, workspace_bytes, (cudaStream_t)stream));
-  // the control words and tile states of the ordered compaction start at zero
-  RelabelWs ws;
-  if (relabel_layout((char*)workspace, workspace_bytes, &ws)) {
-    const size_t off = (size_t)((char*)ws.ctrl - (char*)workspace);
-    APT_CUDA(cudaMemsetAsync(ws.ctrl, 0, workspace_bytes - off, (cudaStream_t)stream));
-  }
   return APT_OK;
 }
 
@@ -319,7 +356,7 @@ extern "C" int apt_relabel_csc(const int64_t* seeds, int64_t num_seeds,
     if (rc != APT_OK) return rc;
     ProfScope prof("relabel", s);
     APT_LAUNCH(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, (int64_t*)neighbors, num_neighbors,
-               num_seeds_dev, per_seed, 0, out_unique, out_relabeled, out_num_unique, status_word);
+               num_seeds_dev, per_seed, 0, out_unique, out_relabeled, nullptr, out_num_unique, status_word);
     return APT_OK;
   }
   RelabelWs ws;
@@ -331,17 +368,17 @@ extern "C" int apt_relabel_csc(const int64_t* seeds, int64_t num_seeds,
   ProfScope prof("relabel", s);
   APT_LAUNCH(k_insert, wave_grid(ceil_div(n, 256 * 2), 8, 2), 256, 0, s, seeds, num_seeds, neighbors, num_neighbors,
              num_seeds_dev, per_seed, ws, status_word);
-  return scan_and_relabel(num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, out_unique, out_relabeled,
-                          out_num_unique, status_word, s);
+  return first_and_relabel(num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, out_unique, out_relabeled, nullptr,
+                           out_num_unique, s);
 }
 
-extern "C" int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds, const int64_t* num_seeds_dev,
+extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds, const int64_t* num_seeds_dev,
                                       int fanout, const int64_t* adj_pos_map, int64_t num_nodes,
                                       const int64_t* dev_indptr, const int64_t* dev_indices,
                                       const int64_t* uva_indptr, const int64_t* uva_indices, uint64_t key,
                                       uint32_t call_id, const int64_t* call_id_base_dev, void* workspace,
                                       size_t workspace_bytes, int64_t* out_neighbors, int64_t* out_unique,
-                                      int64_t* out_relabeled, int64_t* out_num_unique, int32_t* status_word,
+                                      int64_t* out_relabeled, int64_t* out_col, int64_t* out_num_unique, int32_t* status_word,
                                       void* stream) {
   using namespace apt;
   APT_CHECK_ARG(num_seeds >= 0 && fanout > 0 && num_nodes >= 0,
@@ -399,10 +436,23 @@ extern "C" int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds, c
     const int rc = set_small_smem();
     if (rc != APT_OK) return rc;
     APT_LAUNCH(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, nbr_buf, num_neighbors,
-               num_seeds_dev, (int64_t)fanout, out_neighbors ? 0 : 1, out_unique, out_relabeled, out_num_unique,
+               num_seeds_dev, (int64_t)fanout, out_neighbors ? 0 : 1, out_unique, out_relabeled, out_col, out_num_unique,
                status_word);
     return APT_OK;
   }
-  return scan_and_relabel(num_seeds, num_neighbors, num_seeds_dev, (int64_t)fanout, ws, out_unique, out_relabeled,
-                          out_num_unique, status_word, s);
+  return first_and_relabel(num_seeds, num_neighbors, num_seeds_dev, (int64_t)fanout, ws, out_unique, out_relabeled, out_col,
+                           out_num_unique, s);
+}
+
+extern "C" int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds, const int64_t* num_seeds_dev,
+                                      int fanout, const int64_t* adj_pos_map, int64_t num_nodes,
+                                      const int64_t* dev_indptr, const int64_t* dev_indices,
+                                      const int64_t* uva_indptr, const int64_t* uva_indices, uint64_t key,
+                                      uint32_t call_id, const int64_t* call_id_base_dev, void* workspace,
+                                      size_t workspace_bytes, int64_t* out_neighbors, int64_t* out_unique,
+                                      int64_t* out_relabeled, int64_t* out_num_unique, int32_t* status_word,
+                                      void* stream) {
+  return apt_sample_relabel_block(seeds, num_seeds, num_seeds_dev, fanout, adj_pos_map, num_nodes, dev_indptr, dev_indices,
+                                  uva_indptr, uva_indices, key, call_id, call_id_base_dev, workspace, workspace_bytes,
+                                  out_neighbors, out_unique, out_relabeled, nullptr, out_num_unique, status_word, stream);
 }

@@ -10,23 +10,21 @@ namespace apt {
 constexpr unsigned long long kEmptyKey = ~0ull;
 constexpr uint32_t kNoPos = 0xffffffffu;
 
-// key, smallest position and new id of one distinct id: 16 bytes, one sector.
+// key and smallest position of one distinct id: 16 bytes, half a sector. `pad` carries the new id in the one-block
+// form (k_relabel_small).
 struct Slot {
   unsigned long long key;
   uint32_t min_pos;
-  uint32_t new_id;
+  uint32_t pad;
 };
 
-// Items per tile of the ordered compaction: 512 threads x 4 consecutive items.
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kMaxTiles = 4096;   // tiles of items whose counts one block of the last pass adds up
 
 struct RelabelWs {
   Slot* slots;            // [cap_ws] all-0xff between calls
   int32_t* slot_of;       // [items_ws] slot of every item of the running call, -1: not in the table
-  ScanCtrl* ctrl;         // [1]
-  uint64_t* tile_state;   // [tiles_ws] epoch << 34 | status << 32 | count
+  uint2* words;           // [items_ws / 32 + 1] of 32 items: first occurrences before them in their tile, which are ones
+  int32_t* tile_count;    // [kMaxTiles] first occurrences of every tile
   int64_t items_ws;       // items this workspace was sized for
 };
 
@@ -83,12 +81,18 @@ __device__ __forceinline__ int32_t table_insert(Slot* slots, uint32_t cap, int64
   uint32_t at = (uint32_t)(((uint64_t)hash_id(id) * cap) >> 32);
   for (uint32_t probe = 0; probe < cap; ++probe) {
     Slot* s = slots + at;
-    unsigned long long prev = *(volatile unsigned long long*)&s->key;
-    if (prev == kEmptyKey) prev = atomicCAS(&s->key, kEmptyKey, key);
+    // key and smallest position in one 16-byte load: an id that is in the table with an earlier position, which is
+    // what most items of a hub find, is done after it. The position only falls, so one read too early costs an
+    // atomic and nothing else.
+    const ulonglong2 v = ld_volatile_2x8(s);
+    unsigned long long prev = v.x;
+    uint32_t min_pos = (uint32_t)v.y;
+    if (prev == kEmptyKey) {
+      prev = atomicCAS(&s->key, kEmptyKey, key);
+      min_pos = kNoPos;
+    }
     if (prev == kEmptyKey || prev == key) {
-      // the minimum only falls: an id that many items share (a hub) stops costing atomics on one
-      // address as soon as an early position has arrived
-      if (*(volatile uint32_t*)&s->min_pos > pos) atomicMin(&s->min_pos, pos);
+      if (min_pos > pos) atomicMin(&s->min_pos, pos);
       return (int32_t)at;
     }
     at = at + 1 == cap ? 0 : at + 1;

@@ -80,17 +80,8 @@ int apt_profile_enable(int on);
 int apt_profile_read(const char* tag, double* total_ms, int64_t* launches);
 
 /* Tuning knobs for measurements; the defaults are what the benchmark uses.
- *   gather_miss_mode   0 16-byte ld.global.nc loads (default),
- *                      1 bulk copies (cp.async.bulk) staged through shared memory
- *   gather_miss_blocks blocks of the miss-copy kernel (default 148)
- *   gather_miss_kb_per_block  0 (default): every block of the miss copy takes part; k > 0: one block per
- *                      k KiB to fetch (at least 16), the rest leave at once and keep their SM slots free.
- *                      The samplers set 128 for the launches they capture on a lane, where other
- *                      mini-batches' kernels run beside the copy.
- *   gather_hit_mode    copy of the cache hits: 0 one resident wave, two groups of rows in flight per warp,
- *                      1 bulk copies (cp.async.bulk) staged through shared memory,
- *                      2 grid-stride blocks, one group of rows per warp at a time
- *   gather_hit_waves   mode 2: cap on the grid, in units of 148 x 8 blocks (default 4)
+ *   gather_miss_mode, gather_miss_blocks, gather_miss_kb_per_block, gather_hit_mode, gather_hit_waves
+ *                      accepted and without effect (they chose between forms of the gather that are gone)
  *   relabel_small      1 (default): layers of up to 8192 items are relabelled by one block with
  *                      the hash table in shared memory; 0: always the multi-block path */
 int apt_set_tunable(const char* name, int64_t value);
@@ -177,6 +168,19 @@ int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds,
                            int64_t* out_neighbors, int64_t* out_unique,
                            int64_t* out_relabeled, int64_t* out_num_unique,
                            int32_t* status_word, void* stream);
+/* The same with the other side of the block's edges: out_col[j * fanout + i] = j (may be
+ * null), what arange(num_seeds).repeat_interleave(fanout) gives (python/npc/sampler.py:78). */
+int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
+                           const int64_t* num_seeds_dev, int fanout,
+                           const int64_t* adj_pos_map, int64_t num_nodes,
+                           const int64_t* dev_indptr, const int64_t* dev_indices,
+                           const int64_t* uva_indptr, const int64_t* uva_indices,
+                           uint64_t key, uint32_t call_id,
+                           const int64_t* call_id_base_dev,
+                           void* workspace, size_t workspace_bytes,
+                           int64_t* out_neighbors, int64_t* out_unique,
+                           int64_t* out_relabeled, int64_t* out_col, int64_t* out_num_unique,
+                           int32_t* status_word, void* stream);
 
 /* ----------------------------------------------------------- owner bucketing
  * Stable partition of ids by owning rank. Takes the role of ClusterAndPermute
@@ -234,9 +238,8 @@ int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
  *   p == -1: out[r] = 0 and APT_FLAG_FEAT_NOT_EXIST (the reference reads out
  *            of bounds here)
  * Rows are opaque bytes, so fp32/bf16/fp16 tables share the code.
- * Three kernels on `stream`: classify (decode p, compact the miss list), the
- * hit copy out of the HBM cache and the miss copy over the host link.
- * workspace: apt_gather_workspace_bytes(num_rows) bytes; needs no initialisation.
+ * One kernel on `stream`. workspace: apt_gather_workspace_bytes(num_rows) bytes, 256-byte
+ * aligned (an argument of the interface: nothing is kept there).
  * apt_gather_rows_from only produces output rows [*first_row_dev, num_rows) (a
  * device word; NULL: 0): a caller that already holds the leading rows, e.g. the
  * destination nodes of a block whose rows it fetched while the block was still
@@ -268,25 +271,14 @@ int apt_gather_rows(const int64_t* index, int64_t num_rows,
  * server that pre-plans all device memory at start-up), in a callback or a
  * real-time loop where an allocator call may block or synchronise the
  * device, or in a process whose allocator hooks forbid allocation after
- * initialisation. Such a caller passes its own inputs and output; the scratch
- * apt_gather_rows would take as `workspace` is a fixed array built into the
- * library's device image instead (about 12.6 MB, held by every GPU that loads
- * the library until the process exits).
+ * initialisation.
  *
- * Same arguments (minus the workspace) and result as apt_gather_rows, with these differences:
- *  - at most apt_gather_static_max_rows() (1 048 576) rows per call; more
- *    returns APT_ERR_CAPACITY with a message and launches nothing;
- *  - it calls no cudaMalloc, cudaFree or other allocating routine. Every call
- *    looks up the array's device address (cudaGetSymbolAddress) with the
- *    calling thread's device current, so the address is never stale, not even
- *    after the device's context has been torn down and made anew. The first
- *    call on each device makes the CUDA runtime load the library's device
- *    image if it has not yet: make that first call before any stream capture
- *    begins;
- *  - every call on a device uses the same array, which still holds the
- *    previous call's contents (the call clears what has to start at zero).
- *    Two calls that overlap on the GPU — different streams, or different host
- *    threads — race on it: issue them on one stream, or order them yourself.
+ * Same arguments (minus the workspace) and result as apt_gather_rows, for at most
+ * apt_gather_static_max_rows() (1 048 576) rows per call; more returns
+ * APT_ERR_CAPACITY with a message and launches nothing. It calls no cudaMalloc,
+ * cudaFree or other allocating routine and keeps no state. The first call on each
+ * device makes the CUDA runtime load the library's device image if it has not yet:
+ * make that first call before any stream capture begins.
  */
 int64_t apt_gather_static_max_rows(void);
 int apt_gather_rows_static(const int64_t* index, int64_t num_rows,
