@@ -33,6 +33,8 @@ PROTOTYPES = {
     "apt_launch_count": (c_int64, []),
     "apt_launch_count_reset": (None, []),
     "apt_memcpy_async": (c_int, [P, P, c_size_t, P]),
+    "apt_publish_words": (c_int, [P, c_int, P, c_int64, P, P]),
+    "apt_wait_published": (c_int, [P, c_int, c_int64, P]),
     "apt_set_tunable": (c_int, [c_char_p, c_int64]),
     "apt_profile_enable": (c_int, [c_int]),
     "apt_profile_read": (c_int, [c_char_p, ctypes.POINTER(c_double), ctypes.POINTER(c_int64)]),
@@ -43,13 +45,14 @@ PROTOTYPES = {
     "apt_sample_relabel_csc": (c_int, [P, c_int64, P, c_int, P, c_int64, P, P, P, P, c_uint64, c_uint32, P, P, c_size_t,
                                        P, P, P, P, P, P]),
     "apt_sample_relabel_block": (c_int, [P, c_int64, P, c_int, P, c_int64, P, P, P, P, c_uint64, c_uint32, P, P, c_size_t,
-                                         P, P, P, P, P, P, P]),
+                                         P, P, P, P, P, P, c_int64, c_int64, c_int64, P, P]),
     "apt_bucket_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "apt_bucket_by_owner": (c_int, [P, c_int64, P, P, c_int, c_int64, c_int, c_int, c_int, P, c_size_t, P, P, P, P, P]),
     "apt_unique_workspace_bytes": (c_size_t, [c_int64]),
     "apt_unique_workspace_init": (c_int, [P, c_size_t, P]),
     "apt_unique_sorted": (c_int, [P, c_int64, P, c_int64, c_int64, P, c_size_t, P, P, P, P, P]),
     "apt_concat_ids": (c_int, [P, c_int64, P, P, c_int64, P, P, P, P]),
+    "apt_concat_row_ids": (c_int, [P, c_int64, P, P, c_int64, P, P, P, P, c_int64, c_int64, c_int64, P, P]),
     "apt_gather_workspace_bytes": (c_size_t, [c_int64]),
     "apt_gather_rows": (c_int, [P, c_int64, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P, c_size_t, P, P]),
     "apt_gather_rows_from": (c_int, [P, c_int64, P, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P,

@@ -55,8 +55,20 @@ def _native_command(out):
     src = sorted(os.path.join(NATIVE, f) for f in os.listdir(NATIVE) if f.endswith(".cpp"))
     return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w", "-DTORCH_EXTENSION_NAME=_native",
             *[a for d in inc for a in ("-isystem", d)], *src, "-o", out,
-            "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+            "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", *_cudart(), "-ltorch_cpu", "-ltorch", "-ltorch_python",
             "-Wl,-rpath," + os.path.join(torch_dir, "lib"), "-Wl,-rpath,$ORIGIN", LIB_PATH]
+
+
+def _cudart():
+    """The CUDA runtime PyTorch has loaded: one runtime in the process knows all streams and events."""
+    import glob
+    import importlib.util
+
+    site = os.path.dirname(list(importlib.util.find_spec("torch").submodule_search_locations)[0])
+    found = sorted(glob.glob(os.path.join(site, "nvidia", "*", "lib", "libcudart.so.*")))
+    if not found:
+        return ["-L" + os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "lib64"), "-lcudart"]
+    return [found[0], "-Wl,-rpath," + os.path.dirname(found[0])]
 
 
 def _build_native(verbose=False):

@@ -127,13 +127,18 @@ k_bucket_one_rank(const int64_t* __restrict__ ids, int64_t n, const int64_t* __r
 __global__ void __launch_bounds__(256)
 k_concat_ids(const int64_t* __restrict__ a, int64_t na, const int64_t* __restrict__ na_dev,
              const int64_t* __restrict__ b, int64_t nb, const int64_t* __restrict__ nb_dev,
-             int64_t* __restrict__ out, int64_t* __restrict__ out_count) {
+             int64_t* __restrict__ out, int64_t* __restrict__ out_count, const RowTables tables, int32_t* status) {
   na = effective_n(na, na_dev);
   nb = effective_n(nb, nb_dev);
   const int64_t total = na + nb;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride)
-    out[i] = i < na ? a[i] : b[i - na];
+  int flags = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const int64_t id = i < na ? a[i] : b[i - na];
+    out[i] = id;
+    flags |= check_row(tables, id);
+  }
+  if (flags) atomicOr(status, flags);
   if (out_count && blockIdx.x == 0 && threadIdx.x == 0) *out_count = total;
 }
 
@@ -182,8 +187,8 @@ k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restric
   if (flags) atomicOr(status, flags);
 }
 
-// Counting, ranking, emitting and clearing in one launch. A warp has `per_warp` (up to 32) consecutive level-1 words,
-// a lane to each. A lane with few level-0 words below its own (a wide range) walks them itself, all loads in flight;
+// Counting, ranking, emitting and clearing in one launch. A block has 8 * `per_warp` consecutive level-1 words, dealt to
+// its warps in turn (a dense run of ids in a wide range is a few neighbouring words), a lane to each. A lane with few level-0 words below its own (a wide range) walks them itself, all loads in flight;
 // where there are many the warp's lanes take the 32 words together, one level-1 word after another (a dense range: a
 // million ids below one thousand level-1 words; one thread to a word walked 1024 ids alone, 75 to 430 us).
 // The blocks' counts are chained by the look-back of common.cuh. info[w] = (rank of the word's first id, its bits).
@@ -193,20 +198,23 @@ __global__ void __launch_bounds__(kUniqBlock)
 k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords1, int per_warp,
             int64_t lo, ScanCtrl* ctrl, uint64_t* tile_state, uint2* __restrict__ info,
             int64_t* __restrict__ out_unique, int64_t* __restrict__ out_num_unique, int32_t* status) {
-  __shared__ uint32_t warp_total[kUniqBlock / 32];
+  constexpr int W = kUniqBlock / 32;
+  __shared__ uint32_t counts[kUniqBlock];
+  __shared__ int scratch[33];
   __shared__ uint32_t s_tile, s_epoch, s_before;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) tile_ticket(ctrl, &s_tile, &s_epoch);
   __syncthreads();
   const uint32_t tile = s_tile;
-  const int64_t first = ((int64_t)tile * (kUniqBlock / 32) + warp) * per_warp;
-  const uint32_t mine = lane < per_warp && first + lane < nwords1 ? l1[first + lane] : 0u;
+  const int64_t first = (int64_t)tile * W * per_warp + warp;      // word of lane k: first + k * W
+  const int64_t w1 = first + lane * W;
+  const uint32_t mine = lane < per_warp && w1 < nwords1 ? l1[w1] : 0u;
   uint32_t word[kOwnWords], count = 0;
   const bool few = __popc(mine) <= kOwnWords;
   uint32_t rest = mine;
 #pragma unroll
   for (int q = 0; q < kOwnWords; ++q) {
-    word[q] = few && rest ? l0[((first + lane) << 5) + __ffs(rest) - 1] : 0u;
+    word[q] = few && rest ? l0[(w1 << 5) + __ffs(rest) - 1] : 0u;
     rest &= rest - 1;
   }
 #pragma unroll
@@ -214,36 +222,29 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
   for (unsigned m = __ballot_sync(0xffffffffu, !few); m; m &= m - 1) {
     const int k = __ffs(m) - 1;
     const uint32_t mask = __shfl_sync(0xffffffffu, mine, k);
-    const uint32_t c = __reduce_add_sync(0xffffffffu, mask >> lane & 1u ? __popc(l0[((first + k) << 5) + lane]) : 0u);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, mask >> lane & 1u ? __popc(l0[((first + k * W) << 5) + lane]) : 0u);
     if (lane == k) count = c;
   }
-  uint32_t upto_lane = count;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, upto_lane, o);
-    if (lane >= o) upto_lane += t;
-  }
-  if (lane == 31) warp_total[warp] = upto_lane;
+  // ranks inside the block, in the order of the words
+  counts[lane * W + warp] = count;
   __syncthreads();
-  uint32_t before = 0, total = 0;
-#pragma unroll
-  for (int k = 0; k < kUniqBlock / 32; ++k) {
-    if (k < warp) before += warp_total[k];
-    total += warp_total[k];
-  }
+  int total_i;
+  const int before_word = block_exclusive_scan((int)counts[threadIdx.x], scratch, &total_i);
+  counts[threadIdx.x] = (uint32_t)before_word;
+  const uint32_t total = (uint32_t)total_i;
   if (warp == 0) {
     const uint32_t b = tile_lookback(tile_state, tile, s_epoch, total, status, APT_FLAG_TABLE_FULL);
     if (lane == 0) s_before = b;
   }
   __syncthreads();
   if (tile == gridDim.x - 1 && threadIdx.x == 0) *out_num_unique = (int64_t)s_before + total;
-  int64_t at = (int64_t)s_before + before + upto_lane - count;      // rank of the first id below this lane's word
+  int64_t at = (int64_t)s_before + counts[lane * W + warp];      // rank of the first id below this lane's word
   const bool own = few && count <= kOwnIds;
   for (unsigned m = __ballot_sync(0xffffffffu, !own); m; m &= m - 1) {
     const int k = __ffs(m) - 1;
     const uint32_t mask = __shfl_sync(0xffffffffu, mine, k);
     const int64_t start = __shfl_sync(0xffffffffu, at, k);
-    const int64_t w = ((first + k) << 5) + lane;
+    const int64_t w = ((first + k * W) << 5) + lane;
     const uint32_t bits = mask >> lane & 1u ? l0[w] : 0u;
     uint32_t upto = __popc(bits);
 #pragma unroll
@@ -260,7 +261,7 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
     for (uint32_t q = mask; q; q &= q - 1) {
       const int j = __ffs(q) - 1;
       const uint32_t x = __shfl_sync(0xffffffffu, bits, j), rank = __shfl_sync(0xffffffffu, here, j);
-      if (x >> lane & 1u) out_unique[start + rank + __popc(x & ((1u << lane) - 1u))] = lo + ((((first + k) << 5) + j) << 5) + lane;
+      if (x >> lane & 1u) out_unique[start + rank + __popc(x & ((1u << lane) - 1u))] = lo + ((((first + k * W) << 5) + j) << 5) + lane;
     }
   }
   if (own) {
@@ -268,14 +269,14 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
 #pragma unroll
     for (int q = 0; q < kOwnWords; ++q) {
       if (!rest) break;
-      const int64_t w = ((first + lane) << 5) + __ffs(rest) - 1;
+      const int64_t w = (w1 << 5) + __ffs(rest) - 1;
       rest &= rest - 1;
       info[w] = make_uint2((uint32_t)at, word[q]);
       l0[w] = 0u;
       for (uint32_t bits = word[q]; bits; bits &= bits - 1) out_unique[at++] = lo + (w << 5) + __ffs(bits) - 1;
     }
   }
-  if (lane < per_warp && mine) l1[first + lane] = 0u;
+  if (lane < per_warp && mine) l1[w1] = 0u;
   __syncthreads();
   if (threadIdx.x == 0) tile_done(ctrl, s_epoch);
 }
@@ -442,7 +443,15 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
 extern "C" int apt_concat_ids(const int64_t* a, int64_t num_a, const int64_t* num_a_dev, const int64_t* b,
                               int64_t num_b, const int64_t* num_b_dev, int64_t* out, int64_t* out_count_dev,
                               void* stream) {
+  return apt_concat_row_ids(a, num_a, num_a_dev, b, num_b, num_b_dev, out, out_count_dev, nullptr, 0, 0, 0, nullptr, stream);
+}
+
+extern "C" int apt_concat_row_ids(const int64_t* a, int64_t num_a, const int64_t* num_a_dev, const int64_t* b,
+                                  int64_t num_b, const int64_t* num_b_dev, int64_t* out, int64_t* out_count_dev,
+                                  const int64_t* feat_pos_map, int64_t feat_num_nodes, int64_t num_dev_rows,
+                                  int64_t num_uva_rows, int32_t* status_word, void* stream) {
   using namespace apt;
+  APT_CHECK_ARG(!feat_pos_map || status_word, "apt_concat_ids: null status word");
   APT_CHECK_ARG(num_a >= 0 && num_b >= 0 && (num_a == 0 || a) && (num_b == 0 || b), "apt_concat_ids: bad argument");
   APT_CHECK_ARG(out || num_a + num_b == 0, "apt_concat_ids: null output");
   cudaStream_t s = (cudaStream_t)stream;
@@ -451,6 +460,6 @@ extern "C" int apt_concat_ids(const int64_t* a, int64_t num_a, const int64_t* nu
     return APT_OK;
   }
   APT_LAUNCH(k_concat_ids, wave_grid(ceil_div(num_a + num_b, 256), 8, 1), 256, 0, s, a, num_a, num_a_dev, b, num_b,
-             num_b_dev, out, out_count_dev);
+             num_b_dev, out, out_count_dev, RowTables{feat_pos_map, feat_num_nodes, num_dev_rows, num_uva_rows}, status_word);
   return APT_OK;
 }

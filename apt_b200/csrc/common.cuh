@@ -164,6 +164,20 @@ __device__ __forceinline__ int owner_of(int64_t v, const int64_t* mv, const Owne
   return d;
 }
 
+// Where the rows of a gather come from, for the kernels that make its ids: they look an id up as soon as they have it
+// and flag what the gather would flag (no table: pos_map null), so that the flags are there before the rows are.
+struct RowTables {
+  const int64_t* pos_map;
+  int64_t num_nodes, num_dev_rows, num_uva_rows;
+};
+__device__ __forceinline__ int check_row(const RowTables& t, int64_t id) {
+  if (!t.pos_map) return 0;
+  if (id < 0 || id >= t.num_nodes) return APT_FLAG_ID_OUT_OF_RANGE;
+  const int64_t p = t.pos_map[id];
+  if (p == -1) return APT_FLAG_FEAT_NOT_EXIST;
+  return p >= t.num_dev_rows || (-p - 2) >= t.num_uva_rows ? APT_FLAG_ID_OUT_OF_RANGE : 0;
+}
+
 // Sizes may live on the device: an operator chained behind another one takes
 // its element count from a device word (what the previous kernel produced), so
 // that the host never has to wait for it. `n_host` is then only an upper bound

@@ -67,9 +67,48 @@ ProfScope::~ProfScope() {
   if ((size_t)slot < g_prof.size()) cudaEventRecord(g_prof[slot].end, stream);
 }
 
+// The word block goes to page-locked host memory, a sequence number behind it last: the host polls for that, which
+// takes the place of a copy, an event and a wake-up.
+__global__ void __launch_bounds__(256)
+k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __restrict__ sequence_dev, int64_t sequence,
+                volatile int64_t* host) {
+  for (int t = threadIdx.x; t < count; t += blockDim.x) host[t] = words[t];
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) host[count] = sequence_dev ? *sequence_dev : sequence;
+}
+
 }  // namespace apt
 
 extern "C" {
+
+int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_dev, int64_t sequence, int64_t* host,
+                      void* stream) {
+  using namespace apt;
+  APT_CHECK_ARG(words && host && count >= 0 && count <= 4096, "apt_publish_words: bad argument");
+  APT_LAUNCH(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, sequence_dev, sequence, host);
+  return APT_OK;
+}
+
+int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream) {
+  APT_CHECK_ARG(host && count >= 0, "apt_wait_published: bad argument");
+  const volatile int64_t* word = host + count;
+  for (int64_t spin = 1; *word != sequence; ++spin) {
+    if ((spin & 0x3fff) == 0) {
+      // now and then the stream is asked, so that an error on it ends the wait
+      const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+      if (e == cudaErrorNotReady) continue;
+      APT_CUDA(e);
+      if (*word == sequence) break;
+      apt::set_error("apt_wait_published: the stream is idle and the words have not arrived");
+      return APT_ERR_TIMEOUT;
+    }
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+  }
+  return APT_OK;
+}
 
 const char* apt_last_error(void) { return apt::g_err; }
 int apt_version(void) { return 100; }

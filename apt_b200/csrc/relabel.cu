@@ -140,7 +140,7 @@ k_first(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64
 __global__ void __launch_bounds__(256)
 k_relabel(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, RelabelWs ws, int tile_shift,
           int64_t* __restrict__ out_unique, int64_t* __restrict__ out, int64_t* __restrict__ out_col,
-          int64_t* __restrict__ out_num_unique) {
+          int64_t* __restrict__ out_num_unique, const RowTables tables, int32_t* status) {
   __shared__ int tile_base[kMaxTiles];
   __shared__ int scratch[33];
   const RelabelDims d = relabel_dims(S_host, M_host, S_dev, per_seed);
@@ -162,6 +162,7 @@ k_relabel(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int
   __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   constexpr int K = 4;
+  int flags = 0;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; base < d.n; base += stride * K) {
     int32_t v[K];
     uint2 word[K];
@@ -194,11 +195,13 @@ k_relabel(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int
       const int64_t id = (int64_t)tile_base[pos >> tile_shift] + word[k].x + __popc(word[k].y & ((1u << (pos & 31)) - 1u));
       if (i >= d.S) out[i - d.S] = id;
       if (one[k]) {
+        flags |= check_row(tables, (int64_t)key[k]);
         out_unique[id] = (int64_t)key[k];
         st_plain_16((uint4*)(ws.slots + v[k]), make_uint4(0xffffffffu, 0xffffffffu, kNoPos, 0xffffffffu));
       }
     }
   }
+  if (flags) atomicOr(status, flags);
 }
 
 // ---- small layers: the whole relabelling in one block, table in shared memory ----------
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(kRelabelBlock)
 k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __restrict__ nbrs,
                 int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, int erase_nbrs,
                 int64_t* __restrict__ out_unique, int64_t* __restrict__ out_relabeled, int64_t* __restrict__ out_col,
-                int64_t* __restrict__ out_num_unique, int32_t* status) {
+                int64_t* __restrict__ out_num_unique, const RowTables tables, int32_t* status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int scratch[33];
   Slot* slots = (Slot*)smem;
@@ -261,7 +264,6 @@ k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __re
       pos = pos + 1 == kSmallCap ? 0 : pos + 1;
     }
   }
-  if (flags) atomicOr(status, flags);
   __syncthreads();
   int running = 0;
   for (int base = 0; base < n; base += blockDim.x) {
@@ -271,12 +273,14 @@ k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __re
     const int ex = block_exclusive_scan(f, scratch, &total);
     if (f) {
       const int id = running + ex;
+      flags |= check_row(tables, (int64_t)slots[slot_of[i]].key);
       out_unique[id] = (int64_t)slots[slot_of[i]].key;
       slots[slot_of[i]].pad = (uint32_t)id;
     }
     running += total;
   }
   if (threadIdx.x == 0) *out_num_unique = running;
+  if (flags) atomicOr(status, flags);
   __syncthreads();
   for (int i = (int)d.S + threadIdx.x; i < n; i += blockDim.x) {
     out_relabeled[i - d.S] = slot_of[i] == kSmallNoSlot ? (int64_t)-1 : (int64_t)slots[slot_of[i]].pad;
@@ -298,7 +302,8 @@ static int set_small_smem() {
 // Passes 2 and 3 of the multi-block path (the table already holds every item).
 static int first_and_relabel(int64_t num_seeds, int64_t num_neighbors, const int64_t* num_seeds_dev,
                              int64_t per_seed, const RelabelWs& ws, int64_t* out_unique, int64_t* out_relabeled,
-                             int64_t* out_col, int64_t* out_num_unique, cudaStream_t s) {
+                             int64_t* out_col, int64_t* out_num_unique, const RowTables& tables, int32_t* status_word,
+                             cudaStream_t s) {
   const int64_t n = num_seeds + num_neighbors;
   int tile_shift = 10;
   while (ceil_div(n, (int64_t)1 << tile_shift) > kMaxTiles) ++tile_shift;
@@ -306,7 +311,7 @@ static int first_and_relabel(int64_t num_seeds, int64_t num_neighbors, const int
              per_seed, ws, tile_shift);
   const int grid = wave_grid(ceil_div(n, 256 * 4), 8, 1);
   APT_LAUNCH(k_relabel, grid, 256, 0, s, num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, tile_shift, out_unique,
-             out_relabeled, out_col, out_num_unique);
+             out_relabeled, out_col, out_num_unique, tables, status_word);
   return APT_OK;
 }
 
@@ -356,7 +361,8 @@ extern "C" int apt_relabel_csc(const int64_t* seeds, int64_t num_seeds,
     if (rc != APT_OK) return rc;
     ProfScope prof("relabel", s);
     APT_LAUNCH(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, (int64_t*)neighbors, num_neighbors,
-               num_seeds_dev, per_seed, 0, out_unique, out_relabeled, nullptr, out_num_unique, status_word);
+               num_seeds_dev, per_seed, 0, out_unique, out_relabeled, nullptr, out_num_unique, RowTables{},
+               status_word);
     return APT_OK;
   }
   RelabelWs ws;
@@ -369,7 +375,7 @@ extern "C" int apt_relabel_csc(const int64_t* seeds, int64_t num_seeds,
   APT_LAUNCH(k_insert, wave_grid(ceil_div(n, 256 * 2), 8, 2), 256, 0, s, seeds, num_seeds, neighbors, num_neighbors,
              num_seeds_dev, per_seed, ws, status_word);
   return first_and_relabel(num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, out_unique, out_relabeled, nullptr,
-                           out_num_unique, s);
+                           out_num_unique, RowTables{}, status_word, s);
 }
 
 extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds, const int64_t* num_seeds_dev,
@@ -378,9 +384,11 @@ extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
                                       const int64_t* uva_indptr, const int64_t* uva_indices, uint64_t key,
                                       uint32_t call_id, const int64_t* call_id_base_dev, void* workspace,
                                       size_t workspace_bytes, int64_t* out_neighbors, int64_t* out_unique,
-                                      int64_t* out_relabeled, int64_t* out_col, int64_t* out_num_unique, int32_t* status_word,
+                                      int64_t* out_relabeled, int64_t* out_col, int64_t* out_num_unique, const int64_t* feat_pos_map, int64_t feat_num_nodes,
+                                        int64_t num_dev_rows, int64_t num_uva_rows, int32_t* status_word,
                                       void* stream) {
   using namespace apt;
+  const RowTables tables{feat_pos_map, feat_num_nodes, num_dev_rows, num_uva_rows};
   APT_CHECK_ARG(num_seeds >= 0 && fanout > 0 && num_nodes >= 0,
                 "apt_sample_relabel_csc: bad sizes (seeds %lld fanout %d)", (long long)num_seeds, fanout);
   const int64_t num_neighbors = num_seeds * fanout, n = num_seeds + num_neighbors;
@@ -437,11 +445,11 @@ extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
     if (rc != APT_OK) return rc;
     APT_LAUNCH(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, nbr_buf, num_neighbors,
                num_seeds_dev, (int64_t)fanout, out_neighbors ? 0 : 1, out_unique, out_relabeled, out_col, out_num_unique,
-               status_word);
+               tables, status_word);
     return APT_OK;
   }
   return first_and_relabel(num_seeds, num_neighbors, num_seeds_dev, (int64_t)fanout, ws, out_unique, out_relabeled, out_col,
-                           out_num_unique, s);
+                           out_num_unique, tables, status_word, s);
 }
 
 extern "C" int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds, const int64_t* num_seeds_dev,
@@ -454,5 +462,6 @@ extern "C" int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds, c
                                       void* stream) {
   return apt_sample_relabel_block(seeds, num_seeds, num_seeds_dev, fanout, adj_pos_map, num_nodes, dev_indptr, dev_indices,
                                   uva_indptr, uva_indices, key, call_id, call_id_base_dev, workspace, workspace_bytes,
-                                  out_neighbors, out_unique, out_relabeled, nullptr, out_num_unique, status_word, stream);
+                                  out_neighbors, out_unique, out_relabeled, nullptr, out_num_unique, nullptr, 0, 0, 0, status_word,
+                                  stream);
 }

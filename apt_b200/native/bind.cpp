@@ -7,6 +7,7 @@
 // or threads never share it.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -215,6 +216,197 @@ struct GatFunction : public torch::autograd::Function<GatFunction> {
   }
 };
 
+// ------------------------------------------------------------------------------------------------ samplers
+void cuda_ok(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) fail(std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+// Copies the word block to the host (one kernel, polled for) and returns its status flags.
+int64_t read_words(const Tensor& words, const Tensor& host, int64_t sequence) {
+  const int count = (int)words.numel();
+  void* const s = stream();
+  int64_t* const h = host.mutable_data_ptr<int64_t>();
+  py::gil_scoped_release nogil;
+  check(apt_publish_words(words.const_data_ptr<int64_t>(), count, nullptr, sequence, h, s));
+  check(apt_wait_published(h, count, sequence, s));
+  return h[count - 1] & 0xffffffff;
+}
+
+// One captured mini-batch: launches its graph, waits for its counts, orders other streams behind its last kernel.
+class Plan {
+ public:
+  // host_in: page-locked [call-id base, sequence]; host_words: page-locked, count words and the sequence; own_stream:
+  // 0 for the caller's current stream.
+  Plan(uintptr_t exec, Tensor seeds_buf, Tensor host_in, Tensor host_words, uintptr_t own_stream)
+      : exec_((cudaGraphExec_t)exec), seeds_buf_(std::move(seeds_buf)), host_in_(std::move(host_in)),
+        host_words_(std::move(host_words)), own_((cudaStream_t)own_stream) {
+    cuda_ok(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming), "cudaEventCreate");
+    cuda_ok(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming), "cudaEventCreate");
+  }
+  ~Plan() {
+    cudaEventDestroy(done_);
+    cudaEventDestroy(ready_);
+  }
+  Plan(const Plan&) = delete;
+
+  void launch(const Tensor& seeds, int64_t call_base) {
+    if (seeds.scalar_type() != at::kLong || !seeds.is_contiguous() || seeds.numel() != seeds_buf_.numel())
+      fail("sampler plan: seeds must be contiguous int64 of the plan's length");
+    const cudaStream_t cur = (cudaStream_t)stream();
+    const cudaStream_t s = own_ ? own_ : cur;
+    int64_t* const in = host_in_.mutable_data_ptr<int64_t>();
+    in[0] = call_base;
+    in[1] = ++sequence_;
+    py::gil_scoped_release nogil;
+    if (own_) {
+      // behind everything the caller's stream holds so far: the seeds' producer, the consumer of the last results
+      cuda_ok(cudaEventRecord(ready_, cur), "cudaEventRecord");
+      cuda_ok(cudaStreamWaitEvent(own_, ready_, 0), "cudaStreamWaitEvent");
+    } else if (stream_ && stream_ != cur) {
+      cuda_ok(cudaStreamWaitEvent(cur, done_, 0), "cudaStreamWaitEvent");
+    }
+    if (seeds.numel() && seeds.const_data_ptr() != seeds_buf_.const_data_ptr())
+      cuda_ok(cudaMemcpyAsync(seeds_buf_.mutable_data_ptr(), seeds.const_data_ptr(), seeds.nbytes(), cudaMemcpyDefault, s),
+              "cudaMemcpyAsync");
+    cuda_ok(cudaGraphLaunch(exec_, s), "cudaGraphLaunch");
+    cuda_ok(cudaEventRecord(done_, s), "cudaEventRecord");
+    seeds_ = seeds;       // the copy reads it when the stream gets there
+    stream_ = s;
+  }
+  // Until the counts of the last launch are in host_words; returns the status flags.
+  int64_t wait() {
+    const int count = (int)host_words_.numel() - 1;
+    const int64_t* const h = host_words_.const_data_ptr<int64_t>();
+    py::gil_scoped_release nogil;
+    check(apt_wait_published(h, count, sequence_, stream_));
+    return h[count - 1] & 0xffffffff;
+  }
+  void finish() {
+    py::gil_scoped_release nogil;
+    if (stream_) cudaEventSynchronize(done_);
+  }
+  // The current stream runs on behind everything the last launch enqueued (the gathered rows among it).
+  void order_current_stream() {
+    const cudaStream_t cur = (cudaStream_t)stream();
+    if (stream_ && stream_ != cur) cuda_ok(cudaStreamWaitEvent(cur, done_, 0), "cudaStreamWaitEvent");
+  }
+
+ private:
+  cudaGraphExec_t exec_;
+  Tensor seeds_buf_, host_in_, host_words_, seeds_;
+  cudaStream_t own_, stream_ = nullptr;
+  cudaEvent_t done_, ready_;
+  int64_t sequence_ = 0;
+};
+
+Tensor front(const Tensor& t, int64_t n) { return t.narrow(0, 0, n); }
+
+Tensor offsets_cpu(const int64_t* v, int64_t n, bool sum) {
+  Tensor t = at::empty({n}, at::TensorOptions().dtype(at::kLong));
+  int64_t* const o = t.mutable_data_ptr<int64_t>();
+  int64_t run = 0;
+  for (int64_t k = 0; k < n; ++k) o[k] = sum ? (run += v[k]) : v[k];
+  return t;
+}
+
+// The hops of a mini-batch cut to their real sizes. `layers`: innermost first, (relabelled rows, unique ids, columns,
+// fanout, count slot). Returns the blocks, outermost first, and the number of nodes of the last frontier.
+std::pair<py::list, int64_t> narrow_blocks(const int64_t* w, int64_t num_dst, const py::list& layers, const py::object& block) {
+  py::list blocks;
+  for (const auto& item : layers) {
+    const py::tuple l = item.cast<py::tuple>();
+    const int64_t fanout = l[3].cast<int64_t>(), num_src = w[l[4].cast<int64_t>()];
+    blocks.insert(0, block(front(l[0].cast<Tensor>(), num_dst * fanout), front(l[2].cast<Tensor>(), num_dst * fanout), num_src,
+                           num_dst, front(l[1].cast<Tensor>(), num_src), fanout));
+    num_dst = num_src;
+  }
+  return {blocks, num_dst};
+}
+
+// Node-partitioned: blocks, permutation, exchange counts and inverse index. `outer` = the outermost hop as a layer; the
+// words hold [0..] hop counts, [16..] ids received per peer, [64..] bucket offsets.
+py::tuple np_finish(const Tensor& host, const Tensor& seeds, const py::list& layers, const py::tuple& outer, int64_t frontier_slot,
+                    const Tensor& perm, const Tensor& inverse, const OptTensor& rows, int64_t world_size, const py::object& block) {
+  const int64_t* const w = host.const_data_ptr<int64_t>();
+  auto [blocks, frontier] = narrow_blocks(w, seeds.numel(), layers, block);
+  const Tensor recv = offsets_cpu(w + 16, world_size, true), sent = offsets_cpu(w + 64, world_size, false);
+  const int64_t received = recv.const_data_ptr<int64_t>()[world_size - 1];
+  if (received > inverse.numel())
+    fail("chained NP sampler: more ids received than the buffer sized from this rank's own batch holds; use chained=False for "
+         "batches that differ this much between the ranks");
+  py::list last;
+  last.append(outer);
+  auto [outer_block, num_in] = narrow_blocks(w, w[frontier_slot], last, block);
+  blocks.insert(0, outer_block[0]);
+  const Tensor input = front(outer[1].cast<Tensor>(), num_in);
+  py::object row_view = py::none();
+  if (rows) row_view = py::cast(front(*rows, num_in));
+  return py::make_tuple(py::make_tuple(input, seeds, blocks, front(perm, frontier), recv, sent, front(inverse, received)), row_view);
+}
+
+// Data-parallel: every hop sampled and relabelled on this GPU, the rows of the input nodes gathered behind the counts. One
+// read at the end; all results are tensors of their own.
+py::tuple dp_sample(const Tensor& seeds, const std::vector<int64_t>& fanouts, const OptTensor& adj_pos_map, int64_t num_nodes,
+                    const OptTensor& dev_indptr, const OptTensor& dev_indices, const Tensor& uva_indptr, const Tensor& uva_indices,
+                    int64_t key, int64_t call, const Tensor& relabel_ws, const Tensor& words, const Tensor& host, int64_t sequence,
+                    const py::object& features, int64_t row_limit_bytes, const py::object& block) {
+  const auto opt = [](const OptTensor& t) { return t ? ptr(*t) : nullptr; };
+  Tensor pos_map, dev_feats, uva_feats;
+  int64_t feat_nodes = 0, column = 0;
+  bool gather = !features.is_none();
+  if (gather) {
+    const py::tuple f = features.cast<py::tuple>();
+    pos_map = f[0].cast<Tensor>(), dev_feats = f[1].cast<Tensor>(), uva_feats = f[2].cast<Tensor>();
+    feat_nodes = f[3].cast<int64_t>(), column = f[4].cast<int64_t>();
+  }
+  int64_t bound = seeds.numel();
+  for (const int64_t f : fanouts) bound *= 1 + f;
+  if (gather && bound * dev_feats.size(1) * (int64_t)dev_feats.element_size() > row_limit_bytes) gather = false;
+  int64_t* const word = words.mutable_data_ptr<int64_t>();
+  int64_t* const h = host.mutable_data_ptr<int64_t>();
+  const int count = (int)words.numel();
+  void* const s = stream();
+  struct Hop { Tensor rel, uniq, col; };
+  std::vector<Hop> hops;
+  Tensor rows;
+  const auto ids_like = [&](int64_t n) { return at::empty({n}, seeds.options()); };
+  {
+    py::gil_scoped_release nogil;
+    Tensor cur = seeds;
+    for (size_t k = 0; k < fanouts.size(); ++k) {
+      const int64_t n = cur.numel(), f = fanouts[k];
+      Hop hop{ids_like(n * f), ids_like(n * (1 + f)), ids_like(n * f)};
+      const bool last = gather && k + 1 == fanouts.size();
+      check(apt_sample_relabel_block(ptr(cur), n, k ? word + k - 1 : nullptr, (int)f, opt(adj_pos_map), num_nodes, opt(dev_indptr),
+                                     opt(dev_indices), ptr(uva_indptr), ptr(uva_indices), (uint64_t)key,
+                                     (uint32_t)(call + (int64_t)k), nullptr, relabel_ws.mutable_data_ptr(), relabel_ws.numel(),
+                                     nullptr, hop.uniq.mutable_data_ptr<int64_t>(), hop.rel.mutable_data_ptr<int64_t>(),
+                                     hop.col.mutable_data_ptr<int64_t>(), word + k, last ? ptr(pos_map) : nullptr, feat_nodes,
+                                     last ? dev_feats.size(0) : 0, last ? uva_feats.size(0) : 0, status_word(words), s));
+      cur = hop.uniq;
+      hops.push_back(std::move(hop));
+    }
+    check(apt_publish_words(word, count, nullptr, sequence, h, s));
+    if (gather) {
+      const int64_t size = dev_feats.element_size(), dim = dev_feats.size(1);
+      rows = at::empty({cur.numel(), dim}, dev_feats.options());
+      const size_t bytes = apt_gather_workspace_bytes(cur.numel());
+      const Tensor ws = scratch(rows, bytes);
+      check(apt_gather_rows(ptr(cur), cur.numel(), word + fanouts.size() - 1, ptr(pos_map), feat_nodes, data(dev_feats),
+                            dev_feats.size(0), dim * size, data(uva_feats), uva_feats.size(0), uva_feats.size(1) * size,
+                            column * size, mut(rows), ws.mutable_data_ptr(), bytes, status_word(words), s));
+    }
+    check(apt_wait_published(h, count, sequence, s));
+  }
+  py::list layers;
+  for (size_t k = 0; k < hops.size(); ++k)
+    layers.append(py::make_tuple(hops[k].rel, hops[k].uniq, hops[k].col, fanouts[k], (int64_t)k));
+  auto [blocks, num_in] = narrow_blocks(h, seeds.numel(), layers, block);
+  py::object row_view = py::none();
+  if (gather) row_view = py::cast(front(rows, num_in));
+  return py::make_tuple(front(hops.back().uniq, num_in), blocks, row_view, h[count - 1] & 0xffffffff);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -231,6 +423,23 @@ PYBIND11_MODULE(_native, m) {
   });
   m.def("spmm", &spmm);
   m.def("sddmm", &sddmm);
+  py::class_<Plan>(m, "Plan")
+      .def(py::init<uintptr_t, Tensor, Tensor, Tensor, uintptr_t>())
+      .def("launch", &Plan::launch)
+      .def("wait", &Plan::wait)
+      .def("finish", &Plan::finish)
+      .def("order_current_stream", &Plan::order_current_stream);
+  m.def("read_words", &read_words);
+  m.def("narrow_blocks", [](const Tensor& host, int64_t num_dst, const py::list& layers, const py::object& block) {
+    return narrow_blocks(host.const_data_ptr<int64_t>(), num_dst, layers, block);
+  });
+  m.def("fronts", [](const std::vector<Tensor>& tensors, const std::vector<int64_t>& sizes) {
+    std::vector<Tensor> out;
+    for (size_t k = 0; k < tensors.size(); ++k) out.push_back(front(tensors[k], sizes.at(k)));
+    return out;
+  });
+  m.def("np_finish", &np_finish);
+  m.def("dp_sample", &dp_sample);
   m.def("gather", &gather);
   m.def("rows_gather", &rows_gather);
   m.def("rows_scatter", &rows_scatter);

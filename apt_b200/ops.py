@@ -117,7 +117,11 @@ class NPCState:
         self._tls = threading.local()
         self._lane_exchange = {}
         self._lane_streams = {}
-        self.prefetched = None  # (input ids, gathered rows) left by a sampler that gathers ahead
+        # (input ids, gathered rows, plan or None) left by a sampler that gathers ahead; the rows of a plan may
+        # still be on their way on its stream
+        self.prefetched = None
+        self._publish_seq = 0
+        self._seq_lock = threading.Lock()
         self.generation = 0     # bumped whenever installed state changes; captured graphs check it
         self.profiling = False
         self.exchange = None  # set by apt_b200.exchange.make_exchange at init
@@ -173,7 +177,7 @@ class NPCState:
         pair = self._lane_words.get(self.lane)
         if pair is None or pair[0].device != self.device():
             pair = (torch.zeros(self.NUM_WORDS, dtype=torch.int64, device=self.device()),
-                    torch.zeros(self.NUM_WORDS, dtype=torch.int64).pin_memory())
+                    torch.zeros(self.NUM_WORDS + 1, dtype=torch.int64).pin_memory())
             self._lane_words[self.lane] = pair
         return pair[0]
 
@@ -189,14 +193,20 @@ class NPCState:
         any status flag except zero-degree, which is only a notice."""
         w = self.words()
         host = self._lane_words[self.lane][1]
-        host.copy_(w, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
-        self.check_host_words(host)
+        self.check_flags(_native.read_words(w, host, self.next_sequence()))
         return host
+
+    def next_sequence(self) -> int:
+        """A number no earlier publication of a word block carries."""
+        with self._seq_lock:
+            self._publish_seq += 1
+            return self._publish_seq
 
     def check_host_words(self, host: torch.Tensor):
         """Raises if a host copy of the word block carries a status flag (zero-degree is a notice)."""
-        flags = int(host[self.NUM_WORDS - 1]) & 0xFFFFFFFF
+        self.check_flags(int(host[self.NUM_WORDS - 1]) & 0xFFFFFFFF)
+
+    def check_flags(self, flags: int):
         if flags & ~_lib.FLAG_ZERO_DEGREE:
             self.words()[self.NUM_WORDS - 1] = 0
             raise RuntimeError(f"apt_b200 device status flags 0x{flags:x}: " + _flag_text(flags))
@@ -337,8 +347,10 @@ def cache_feats_shared(num_total_nodes: int, localnode_feats: torch.Tensor, cach
 
 def set_sampling(key: Optional[int] = None, call_id: Optional[int] = None, replace: Optional[bool] = None):
     """Sampler stream control: draws depend only on (key, call_id, seed slot,
-    draw slot); call_id advances by one per sampling call."""
-    STATE.generation += 1
+    draw slot); call_id advances by one per sampling call. Captured mini-batches carry the key and the mode, not the
+    call id: they stay as they are when only that changes."""
+    if (key is not None and int(key) != STATE.sample_key) or (replace is not None and bool(replace) != STATE.sample_replace):
+        STATE.generation += 1
     if key is not None:
         STATE.sample_key = int(key)
     if call_id is not None:
@@ -396,16 +408,29 @@ def _relabel_workspace(n):
     return ws
 
 
-def _sample_relabel_enqueue(seeds, fanout, n_dev, count_out, call_id=None, call_base_dev=None, want_neighbors=False):
-    """One sampled layer, sampling and relabelling together (apt_sample_relabel_csc): returns the
+def _row_tables():
+    """(position map, nodes, cached rows, host rows) for the kernels that look ids of a gather up."""
+    f = STATE.feat
+    if f.feat_pos_map is None:
+        return None, 0, 0, 0
+    return _ptr(f.feat_pos_map), f.num_total_nodes, f.dev_feats.shape[0], f.uva_feats.shape[0]
+
+
+def _sample_relabel_enqueue(seeds, fanout, n_dev, count_out, call_id=None, call_base_dev=None, want_neighbors=False,
+                            look_up=False):
+    """One sampled layer, sampling and relabelling together (apt_sample_relabel_block): returns the
     upper-bound buffers (unique ids, relabelled neighbours, neighbours or None); the number of
-    unique ids lands in the device word `count_out`."""
+    unique ids lands in the device word `count_out`. `look_up`: the unique ids are those of a gather,
+    flag what it would flag."""
     g = STATE.graph
     if g.uva_indptr is None:
         raise RuntimeError("mix_cache_graphs has not been called")
     if not STATE.sample_replace:
         nbr = _sample(seeds, fanout, n_dev, call_id, call_base_dev)
         uniq, rel = _relabel_enqueue(seeds, nbr, n_dev, count_out)
+        if look_up:
+            none = torch.empty(0, dtype=torch.int64, device=uniq.device)
+            concat_ids(none, None, uniq, count_out, None, look_up=True)
         return uniq, rel, nbr
     seeds = _need_cuda(seeds, "seeds")
     S, f = seeds.numel(), int(fanout)
@@ -416,11 +441,11 @@ def _sample_relabel_enqueue(seeds, fanout, n_dev, count_out, call_id=None, call_
     if call_id is None:
         call_id = STATE.sample_calls
         STATE.sample_calls += 1
-    check(lib.apt_sample_relabel_csc(
+    check(lib.apt_sample_relabel_block(
         _ptr(seeds), S, _ptr(n_dev), f, _ptr(g.adj_pos_map), g.num_total_nodes, _ptr(g.dev_indptr),
         _ptr(g.dev_indices), _ptr(g.uva_indptr), _ptr(g.uva_indices), STATE.sample_key, call_id & 0xFFFFFFFF,
-        _ptr(call_base_dev), _ptr(ws), ws.numel(), _ptr(nbr), _ptr(uniq), _ptr(rel), _ptr(count_out),
-        STATE.status_ptr(), _stream()))
+        _ptr(call_base_dev), _ptr(ws), ws.numel(), _ptr(nbr), _ptr(uniq), _ptr(rel), None, _ptr(count_out),
+        *(_row_tables() if look_up else (None, 0, 0, 0)), STATE.status_ptr(), _stream()))
     return uniq, rel, nbr
 
 
@@ -503,12 +528,14 @@ def _unique_enqueue(ids, n_dev, id_lo, id_hi, count_out, ws_name="unique"):
 
 
 def concat_ids(a: torch.Tensor, na_dev: Optional[torch.Tensor], b: torch.Tensor, nb_dev: Optional[torch.Tensor],
-               count_out: torch.Tensor) -> torch.Tensor:
+               count_out: Optional[torch.Tensor], look_up: bool = False) -> torch.Tensor:
     """cat(a[:na], b[:nb]) with device-side lengths (None: the whole tensor); the result buffer holds
-    a.numel() + b.numel() ids and the device word `count_out` receives na + nb."""
+    a.numel() + b.numel() ids and the device word `count_out` receives na + nb. `look_up`: the ids are those of
+    a gather, flag what it would flag."""
     out = torch.empty(a.numel() + b.numel(), dtype=torch.int64, device=a.device)
-    check(lib.apt_concat_ids(_ptr(a), a.numel(), _ptr(na_dev), _ptr(b), b.numel(), _ptr(nb_dev), _ptr(out),
-                             _ptr(count_out), _stream()))
+    check(lib.apt_concat_row_ids(_ptr(a), a.numel(), _ptr(na_dev), _ptr(b), b.numel(), _ptr(nb_dev), _ptr(out),
+                                 _ptr(count_out), *(_row_tables() if look_up else (None, 0, 0, 0)), STATE.status_ptr(),
+                                 _stream()))
     return out
 
 
@@ -735,9 +762,11 @@ def load_subtensor(node_id: torch.Tensor) -> torch.Tensor:
     pre = STATE.prefetched
     if pre is not None:
         STATE.prefetched = None
-        ids, rows = pre
+        ids, rows, plan = pre
         if ids is node_id or (ids.data_ptr() == node_id.data_ptr() and ids.numel() == node_id.numel()
                               and node_id.is_contiguous()):
+            if plan is not None:
+                plan.order_current_stream()
             return rows
     return _native.gather(node_id, f.feat_pos_map, f.dev_feats, f.uva_feats, f.num_total_nodes, f.feat_dim_offset,
                           STATE.words())

@@ -22,7 +22,7 @@ from typing import List
 import torch
 import torch.distributed as dist
 
-from . import ops
+from . import _native, ops
 from ._lib import check, lib
 
 
@@ -54,6 +54,22 @@ def _coo_col(num_dst_max: int, num_dst: int, fanout: int, device) -> torch.Tenso
     return col[:num_dst * fanout]
 
 
+def _layer(dst_buf, rel, uniq, fanout, slot):
+    """A hop as _native.narrow_blocks takes it: upper-bound buffers and the word slot of its unique ids."""
+    return rel, uniq, _coo_col(dst_buf.numel(), dst_buf.numel(), fanout, rel.device), fanout, slot
+
+
+_ARANGE = {}
+
+
+def _arange(n, device):
+    """arange(n) as a prefix of a cached longer one."""
+    t = _ARANGE.get(device)
+    if t is None or t.numel() < n:
+        t = _ARANGE[device] = torch.arange(max(2 * n, 1 << 14), device=device)
+    return t[:n]
+
+
 def create_block(seeds: torch.Tensor, neighbors: torch.Tensor, fanout: int) -> Block:
     unique_frontier, indices = ops.relabel_csc(seeds, neighbors)
     coo_col = torch.arange(0, seeds.numel(), device=indices.device).repeat_interleave(fanout)
@@ -63,6 +79,12 @@ def create_block(seeds: torch.Tensor, neighbors: torch.Tensor, fanout: int) -> B
 # Upper-bound buffers beyond this many bytes of gathered rows are not gathered
 # ahead of the size read; the gather then runs right after it with exact sizes.
 _PREFETCH_LIMIT_BYTES = 6 << 30
+
+
+def _fits_prefetch(rows: int) -> bool:
+    f = ops.STATE.feat
+    return f.feat_pos_map is not None and \
+        rows * f.rank_feat_dim * f.dev_feats.element_size() <= _PREFETCH_LIMIT_BYTES
 
 
 class _Plan:
@@ -75,20 +97,22 @@ class _Plan:
         self.graph = None
         self.generation = -1
         self.keepalive = None
-        # pipelined use (sample_iter): the batch's own copy of the word block, the event behind that
-        # copy, and its own pinned word for the call-id base
+        # the batch's own copy of the word block (a sequence number behind it) and the pinned words a replay
+        # reads: the call-id base and that number
         self.host_words = None
-        self.done = None
-        self.host_base = None
+        self.host_in = None
+        self.handle = None      # _native.Plan: launches the graph, waits for the counts, orders streams
         # the lane whose scratch the plan was built on; with more than one lane, the lane's stream
-        # and the event that orders a new launch behind the consumer of the plan's last results
         self.lane = 0
         self.stream = None
-        self.ready = None
         self.ring_size = 1      # buffer sets of this plan's shape: as many mini-batches may be in flight
 
+    def __del__(self):
+        if self.handle is not None:
+            self.handle.finish()     # the last launch may still be running: its graph and buffers go only then
 
-_CALL_BASE_SLOT = 100  # device word holding the sampler's call-id base for graph replays
+
+_CALL_BASE_SLOT = 100  # device words holding the call-id base and the sequence number of a graph replay
 
 
 class _Ring:
@@ -101,9 +125,10 @@ class _Ring:
 
 
 class _GraphReplay:
-    """What the chained samplers share: the whole mini-batch is enqueued by `_enqueue(seeds, base_dev)`
-    without a host read and narrowed by `_finish(seeds, bufs, host)` after one copy of the device word
-    block; the enqueue is captured once per batch shape as a CUDA graph and replayed, from
+    """What the chained samplers share: the whole mini-batch is enqueued by `_enqueue(seeds, base_dev, publish)`
+    without a host read and narrowed by `_finish(seeds, bufs, host)` after one look at the device word
+    block, which `publish()` sends to the host as soon as it is complete (a gather of the rows goes behind it
+    and runs on while the host narrows); the enqueue is captured once per batch shape as a CUDA graph and replayed, from
     `graph_buffers` buffer sets in turn. `sample_iter` launches mini-batch k + 1 before it reads
     mini-batch k back. Subclasses set `num_calls` (sampling calls per mini-batch).
 
@@ -173,15 +198,13 @@ class _GraphReplay:
         plan.generation = st.generation
         plan.seeds_buf = torch.empty(seeds.numel(), dtype=torch.int64, device=dev)
         plan.seeds_buf.copy_(seeds)
-        plan.host_words = torch.zeros(st.NUM_WORDS, dtype=torch.int64).pin_memory()
-        plan.host_base = torch.zeros(1, dtype=torch.int64).pin_memory()
-        plan.done = torch.cuda.Event()
+        plan.host_words = torch.zeros(st.NUM_WORDS + 1, dtype=torch.int64).pin_memory()
+        plan.host_in = torch.zeros(2, dtype=torch.int64).pin_memory()
         if on_lanes:
             # lane 0 stays with the caller: its exchange context also carries the feature shuffles
             # the model side runs on its own stream while the samplers' lanes are in flight
             plan.lane = 1 + i % self.lanes
             plan.stream = st.lane_stream(plan.lane)
-            plan.ready = torch.cuda.Event()
             torch.cuda.synchronize()     # no other lane's mini-batch is in flight while this one is built
         st.lane = plan.lane
         try:
@@ -192,16 +215,24 @@ class _GraphReplay:
             st.prefetched = None
             del bufs
             plan.graph = torch.cuda.CUDAGraph()
+            replay_in = st.words()[_CALL_BASE_SLOT:_CALL_BASE_SLOT + 2]
+            published = []
+
+            def publish():
+                published.append(True)
+                check(lib.apt_publish_words(ops._ptr(st.words()), st.NUM_WORDS, ops._ptr(replay_in[1:2]), 0,
+                                            ops._ptr(plan.host_words), ops._stream()))
+
             with torch.cuda.graph(plan.graph):
-                # the two small host copies are nodes of the graph: the call-id base is read from the
-                # plan's pinned word when the replay runs, and the word block lands in the plan's
-                # pinned copy behind the last kernel
-                # (apt_memcpy_async and not Tensor.copy_: the latter also records an event for the
+                # the call-id base and the sequence number are read from the plan's pinned words when the replay
+                # runs (apt_memcpy_async and not Tensor.copy_: the latter also records an event for the
                 # pinned block, which may not be queried once it was recorded in a capture)
-                check(lib.apt_memcpy_async(ops._ptr(base_dev), ops._ptr(plan.host_base), 8, ops._stream()))
-                plan.bufs = self._enqueue(plan.seeds_buf, base_dev)
-                check(lib.apt_memcpy_async(ops._ptr(plan.host_words), ops._ptr(st.words()), 8 * st.NUM_WORDS,
-                                           ops._stream()))
+                check(lib.apt_memcpy_async(ops._ptr(replay_in), ops._ptr(plan.host_in), 16, ops._stream()))
+                plan.bufs = self._enqueue(plan.seeds_buf, base_dev, publish)
+                if not published:
+                    publish()
+            plan.handle = _native.Plan(plan.graph.raw_cuda_graph_exec(), plan.seeds_buf, plan.host_in, plan.host_words,
+                                       plan.stream.cuda_stream if on_lanes else 0)
             plan.keepalive = [v for k, v in st._ws.items() if k[2] == plan.lane]
         finally:
             st.lane = 0
@@ -223,28 +254,13 @@ class _GraphReplay:
         return plan
 
     def _replay(self, plan, seeds):
-        """Enqueues one replay of `plan` for `seeds` and records `plan.done` behind it: on the current
-        stream, or, with lanes, on the plan's own stream behind everything the current stream holds
-        so far (the seeds' producer and the consumer of the plan's previous results)."""
+        """Enqueues one replay of `plan` for `seeds`: on the current stream, or, with lanes, on the plan's own
+        stream behind everything the current stream holds so far (the seeds' producer and the consumer of the
+        plan's previous results)."""
         st = ops.STATE
-        plan.host_base[0] = st.sample_calls
+        base = st.sample_calls
         st.sample_calls += self.num_calls
-        # explicit streams throughout: looking the current stream up costs more host time than a launch
-        cur = torch.cuda.current_stream()
-        if plan.stream is None:
-            plan.seeds_buf.copy_(seeds, non_blocking=True)
-            plan.graph.replay()
-            plan.done.record(cur)
-            return
-        plan.ready.record(cur)
-        plan.stream.wait_event(plan.ready)
-        torch.cuda.set_stream(plan.stream)
-        try:
-            plan.seeds_buf.copy_(seeds, non_blocking=True)
-            plan.graph.replay()
-        finally:
-            torch.cuda.set_stream(cur)
-        plan.done.record(plan.stream)
+        plan.handle.launch(seeds, base)
 
     def _sample_chained(self, seeds: torch.Tensor):
         seeds = ops._need_cuda(seeds, "seeds")
@@ -351,15 +367,20 @@ class _GraphReplay:
 
     def _collect(self, launched):
         plan, seeds = launched
-        plan.done.synchronize()
+        flags = plan.handle.wait()
         st = ops.STATE
+        if plan.lane == 0:
+            if flags:
+                st.check_flags(flags)
+            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle)
         st.lane = plan.lane
         try:
-            st.check_host_words(plan.host_words)
-            return self._finish(seeds, plan.bufs, plan.host_words)
+            if flags:
+                plan.handle.order_current_stream()
+                st.check_flags(flags)
+            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle)
         finally:
             st.lane = 0
-
 
 
 class MixedNeighborSampler(_GraphReplay):
@@ -418,7 +439,7 @@ class MixedNeighborSampler(_GraphReplay):
         return seeds, output_nodes, blocks, perm, send_offset, recv_offset, inverse_idx
 
     # ------------------------------------------------------------ chained path
-    def _enqueue(self, seeds: torch.Tensor, call_base_dev):
+    def _enqueue(self, seeds: torch.Tensor, call_base_dev, publish=None):
         """Enqueues every kernel of the mini-batch on the current stream; no host
         read. With call_base_dev the k-th sampling call uses call id base + k."""
         st = ops.STATE
@@ -429,13 +450,13 @@ class MixedNeighborSampler(_GraphReplay):
         slot = 0
         call = 0
         cur, cur_n = seeds, None
-        layers = []                      # (dst buffer, rel, uniq, uniq count slot, fanout)
+        layers = []
         for fanout in reversed(self.fir_fanouts):
             cnt = st.word(slot)
             uniq, rel, _ = ops._sample_relabel_enqueue(cur, fanout, cur_n, cnt, call if explicit else None,
                                                        call_base_dev)
             call += 1
-            layers.append((cur, rel, uniq, slot, fanout))
+            layers.append(_layer(cur, rel, uniq, fanout, slot))
             cur, cur_n = uniq, cnt
             slot += 1
         # outermost hop at the owners (NPSampleAndShuffle, src/sampling.cc:52-69)
@@ -456,8 +477,7 @@ class MixedNeighborSampler(_GraphReplay):
         # rows are fetched on a second stream while the hop is still being sampled and relabelled,
         # and only the rows of the newly met nodes wait for the relabelling.
         f = st.feat
-        prefetch = self.prefetch_features and f.feat_pos_map is not None and \
-            uniq2.numel() * (1 + self.las_fanouts) * f.rank_feat_dim * f.dev_feats.element_size() <= _PREFETCH_LIMIT_BYTES
+        prefetch = self.prefetch_features and _fits_prefetch(uniq2.numel() * (1 + self.las_fanouts))
         split = self.gather_split if prefetch and not st.profiling else 0
         rows = None
         side = None
@@ -471,53 +491,29 @@ class MixedNeighborSampler(_GraphReplay):
             with torch.cuda.stream(side):
                 ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier")
         uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
-                                                     call if explicit else None, call_base_dev)
+                                                     call if explicit else None, call_base_dev, look_up=prefetch)
+        if publish is not None and not split:
+            publish()
         if split == 1:
             main.wait_stream(side)
         if prefetch:
             ops._gather_enqueue(uniq3, st.word(in_slot), out=rows, first_dev=st.word(u_slot) if split else None)
         if split == 2:
             main.wait_stream(side)
-        return dict(layers=layers, perm=perm, inv=inv, uniq2=uniq2, uniq3=uniq3, rel3=rel3, rows=rows,
-                    u_slot=u_slot, in_slot=in_slot)
+        return dict(layers=layers, perm=perm, inv=inv, rows=rows, u_slot=u_slot,
+                    outer=_layer(uniq2, rel3, uniq3, self.las_fanouts, in_slot))
 
-    def _finish(self, seeds, bufs, host=None):
-        """The one host read of the mini-batch (or the copy of the word block a pipelined launch
+    def _finish(self, seeds, bufs, host=None, plan=None):
+        """The one host read of the mini-batch (or the copy of the word block a captured launch
         left in `host`), then buffers narrowed to their real sizes."""
         st = ops.STATE
-        ws = st.world_size
         if host is None:
             host = st.read_words()
-        u_slot, in_slot = bufs["u_slot"], bufs["in_slot"]
-        # one tolist() of the word block: python ints from here on (every slice, clone or int() of the
-        # pinned block costs microseconds of host time per mini-batch)
-        h = host.tolist()
-        count = h[:in_slot + 1]
-        recv_cum = list(itertools.accumulate(h[16:16 + ws]))
-        recv_offset = torch.tensor(recv_cum, dtype=torch.int64)
-        dev_offset = torch.tensor(h[64:64 + ws], dtype=torch.int64)
-        total_recv = recv_cum[-1]
-        if total_recv > bufs["inv"].numel():
-            raise RuntimeError("chained NP sampler: more ids received than the buffer sized from this rank's own "
-                               "batch holds; use chained=False for batches that differ this much between the ranks")
-        blocks = []
-        n_dst = seeds.numel()
-        for dst_buf, rel, uniq, u_s, fanout in bufs["layers"]:
-            n_src = count[u_s]
-            blocks.insert(0, Block(rel[:n_dst * fanout], _coo_col(dst_buf.numel(), n_dst, fanout, rel.device),
-                                   n_src, n_dst, uniq[:n_src], fanout))
-            n_dst = n_src
-        n_frontier = n_dst
-        n_owner_dst, n_in = count[u_slot], count[in_slot]
-        f0 = self.las_fanouts
-        uniq2, uniq3, rel3 = bufs["uniq2"], bufs["uniq3"], bufs["rel3"]
-        blocks.insert(0, Block(rel3[:n_owner_dst * f0], _coo_col(uniq2.numel(), n_owner_dst, f0, rel3.device),
-                               n_in, n_owner_dst, uniq3[:n_in], f0))
-        input_nodes = uniq3[:n_in]
-        if bufs["rows"] is not None:
-            st.prefetched = (input_nodes, bufs["rows"][:n_in])
-        return (input_nodes, seeds, blocks, bufs["perm"][:n_frontier], recv_offset, dev_offset,
-                bufs["inv"][:total_recv])
+        got, rows = _native.np_finish(host, seeds, bufs["layers"], bufs["outer"], bufs["u_slot"], bufs["perm"], bufs["inv"],
+                                      bufs["rows"], st.world_size, Block)
+        if rows is not None:
+            st.prefetched = (got[0], rows, plan)
+        return got
 
 
 class SPGATSampler(_GraphReplay):
@@ -551,7 +547,7 @@ class SPGATSampler(_GraphReplay):
         self.use_graph = self.use_graph and self.chained
         self.num_calls = len(self.fanouts)
 
-    def _enqueue(self, seeds: torch.Tensor, call_base_dev):
+    def _enqueue(self, seeds: torch.Tensor, call_base_dev, publish=None):
         """Every kernel of the mini-batch on the current stream, no host read."""
         st = ops.STATE
         ws = st.world_size
@@ -568,7 +564,7 @@ class SPGATSampler(_GraphReplay):
             uniq, rel, _ = ops._sample_relabel_enqueue(cur, fanout, cur_n, cnt, call if explicit else None,
                                                        call_base_dev)
             call += 1
-            layers.append((cur, rel, uniq, slot, fanout))
+            layers.append(_layer(cur, rel, uniq, fanout, slot))
             cur, cur_n = uniq, cnt
             slot += 1
         f = self.fanouts[0]
@@ -587,41 +583,32 @@ class SPGATSampler(_GraphReplay):
         sorted_ids, perm, sizes, offsets = ops._bucket(unique_neigh, u_word, sizes_view, words[64:64 + ws])
         recv, recv_counts = ops._exchange().exchange_ids_enqueue(sorted_ids, sizes, offsets, recv_view)
         in_word = st.word(self._IN)
-        input_nodes = ops.concat_ids(cur, cur_n, recv, recv_counts[ws:ws + 1], in_word)
-        rows = None
-        ft = st.feat
-        if self.prefetch_features and ft.feat_pos_map is not None and \
-                input_nodes.numel() * ft.rank_feat_dim * ft.dev_feats.element_size() <= _PREFETCH_LIMIT_BYTES:
-            rows = ops._gather_enqueue(input_nodes, in_word)
-        return dict(layers=layers, slot=slot, cur=cur, arange_src=arange_src, unique_neigh=unique_neigh, perm=perm,
+        prefetch = self.prefetch_features and _fits_prefetch(cur.numel() + recv.numel())
+        input_nodes = ops.concat_ids(cur, cur_n, recv, recv_counts[ws:ws + 1], in_word, look_up=prefetch)
+        if publish is not None:
+            publish()
+        rows = ops._gather_enqueue(input_nodes, in_word) if prefetch else None
+        return dict(layers=layers, outer=_layer(cur, arange_src, unique_neigh, f, self._U), perm=perm,
                     input_nodes=input_nodes, rows=rows)
 
-    def _finish(self, seeds, b, host=None):
+    def _finish(self, seeds, b, host=None, plan=None):
         st = ops.STATE
         ws = st.world_size
         if host is None:
             host = st.read_words()
-        dev = seeds.device
-        f = self.fanouts[0]
-        blocks = []
-        n_dst = seeds.numel()
-        for dst_buf, rel, uniq, u_s, fanout in b["layers"]:
-            n_src = int(host[u_s])
-            blocks.insert(0, Block(rel[:n_dst * fanout], _coo_col(dst_buf.numel(), n_dst, fanout, dev), n_src, n_dst,
-                                   uniq[:n_src], fanout))
-            n_dst = n_src
-        n_u, n_in = int(host[self._U]), int(host[self._IN])
+        blocks, n_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
+        h = host.tolist()
+        n_u, n_in = h[self._U], h[self._IN]
         if n_in > b["input_nodes"].numel():
             raise RuntimeError("chained SNP-GAT sampler: more ids received than the buffer sized from this rank's own "
                                "batch holds; use chained=False for batches that differ this much between the ranks")
-        blocks.insert(0, Block(b["arange_src"][:n_dst * f], _coo_col(b["cur"].numel(), n_dst, f, dev), n_u, n_dst,
-                               b["unique_neigh"][:n_u], f))
-        h = host.tolist()
+        outer, _ = _native.narrow_blocks(host, n_dst, [b["outer"]], Block)
+        blocks.insert(0, outer[0])
         send_offset = torch.tensor(list(itertools.accumulate(h[16:16 + ws])), dtype=torch.int64)
         recv_offset = torch.tensor(h[64:64 + ws], dtype=torch.int64)
         input_nodes = b["input_nodes"][:n_in]
         if b["rows"] is not None:
-            st.prefetched = (input_nodes, b["rows"][:n_in])
+            st.prefetched = (input_nodes, b["rows"][:n_in], plan)
         return input_nodes, seeds, blocks, b["perm"][:n_u], send_offset, recv_offset
 
     def sample(self, graph, seeds: torch.Tensor):
@@ -666,7 +653,7 @@ class SPVirtualSampler(_GraphReplay):
     (`self.last["unique_dst"]`)."""
 
     def __init__(self, rank: int, fanouts: List[int], model: str = "SAGE", shuffle_with_dst: bool = False,
-                 chained: bool = None, use_graph: bool = None, lanes: int = None):
+                 chained: bool = None, use_graph: bool = None, lanes: int = None, prefetch_features: bool = True):
         if model not in ("SAGE", "GCN"):
             raise ValueError("SPVirtualSampler serves SAGE and GCN; GAT uses SPGATSampler")
         self.rank = rank
@@ -679,15 +666,17 @@ class SPVirtualSampler(_GraphReplay):
         self._init_replay(use_graph, 2, lanes)
         self.use_graph = self.use_graph and self.chained
         self.num_calls = len(self.fanouts)
+        self.prefetch_features = prefetch_features
         self.last = {}
 
     # word slots of the chained form: [0..13] hop counts, [16..48] packed ids received per peer (+ total),
     # [50] neighbours, [51] unique virtual nodes, [52] unique received neighbours, [53] unique received
-    # virtual nodes, [54] destinations + neighbours, [64..96] destinations received per peer (+ total),
-    # [128..191] send sizes, [192..253] receive sizes
-    _N, _UF, _US, _UD, _ALL, _RDST, _SEND, _RECV = 50, 51, 52, 53, 54, 64, 128, 192
+    # virtual nodes, [54] destinations + neighbours, [55] input nodes, [64..96] destinations received per peer
+    # (+ total), [128..191] send sizes, [192..253] receive sizes. With one rank and no destinations sent along, the
+    # sizes are [50] and [51] and nothing is exchanged.
+    _N, _UF, _US, _UD, _ALL, _IN, _RDST, _SEND, _RECV = 50, 51, 52, 53, 54, 55, 64, 128, 192
 
-    def _enqueue(self, seeds: torch.Tensor, call_base_dev):
+    def _enqueue(self, seeds: torch.Tensor, call_base_dev, publish=None):
         """Every kernel of the mini-batch on the current stream, no host read."""
         st = ops.STATE
         ws = st.world_size
@@ -707,7 +696,7 @@ class SPVirtualSampler(_GraphReplay):
             uniq, rel, _ = ops._sample_relabel_enqueue(cur, fanout, cur_n, cnt, call if explicit else None,
                                                        call_base_dev)
             call += 1
-            layers.append((cur, rel, uniq, slot, fanout))
+            layers.append(_layer(cur, rel, uniq, fanout, slot))
             cur, cur_n = uniq, cnt
             slot += 1
         f = self.fanouts[0]
@@ -746,30 +735,32 @@ class SPVirtualSampler(_GraphReplay):
             all_word = st.word(self._ALL)
         else:
             sorted_all, all_word = sorted_vir, n_word
-        send_sizes = words[self._SEND:self._SEND + k * ws]
-        recv_sizes = words[self._RECV:self._RECV + k * ws]
-        check(lib.apt_vir_send_sizes(ops._ptr(sorted_all), sorted_all.numel(), ops._ptr(all_word),
-                                     ops._ptr(unique_frontier), unique_frontier.numel(), ops._ptr(uf_word), ws, s_max,
-                                     ops._ptr(cur_n), int(with_dst), None, ops._ptr(send_sizes), ops._stream()))
-        ex = ops._exchange()
-        ex.exchange_fixed(send_sizes.view(ws, k), recv_sizes.view(ws, k))
         counts = words[16:16 + ws + 1]
         dst_counts = words[self._RDST:self._RDST + ws + 1]
         recv_dst = None
-        ids_at = 1 if with_dst else 0
-        if ws == 1:
-            recv = packed
-            counts[0:1].copy_(send_sizes[ids_at:ids_at + 1])
-            counts[1:2].copy_(send_sizes[ids_at:ids_at + 1])
-            if with_dst:
+        if ws == 1 and not with_dst:
+            recv, total = packed, n_word
+        else:
+            send_sizes = words[self._SEND:self._SEND + k * ws]
+            recv_sizes = words[self._RECV:self._RECV + k * ws]
+            check(lib.apt_vir_send_sizes(ops._ptr(sorted_all), sorted_all.numel(), ops._ptr(all_word),
+                                         ops._ptr(unique_frontier), unique_frontier.numel(), ops._ptr(uf_word), ws, s_max,
+                                         ops._ptr(cur_n), int(with_dst), None, ops._ptr(send_sizes), ops._stream()))
+            ex = ops._exchange()
+            ex.exchange_fixed(send_sizes.view(ws, k), recv_sizes.view(ws, k))
+            ids_at = 1 if with_dst else 0
+            if ws == 1:
+                recv = packed
+                counts[0:1].copy_(send_sizes[ids_at:ids_at + 1])
+                counts[1:2].copy_(send_sizes[ids_at:ids_at + 1])
                 recv_dst = dst_sorted
                 dst_counts[0:1].copy_(send_sizes[0:1])
                 dst_counts[1:2].copy_(send_sizes[0:1])
-        else:
-            if with_dst:
-                recv_dst, _ = ex.exchange_ids_enqueue(dst_sorted, None, torch.cumsum(send_sizes[0::k], 0), dst_counts)
-            recv, _ = ex.exchange_ids_enqueue(packed, None, torch.cumsum(send_sizes[ids_at::k], 0), counts)
-        total = counts[ws:ws + 1]
+            else:
+                if with_dst:
+                    recv_dst, _ = ex.exchange_ids_enqueue(dst_sorted, None, torch.cumsum(send_sizes[0::k], 0), dst_counts)
+                recv, _ = ex.exchange_ids_enqueue(packed, None, torch.cumsum(send_sizes[ids_at::k], 0), counts)
+            total = counts[ws:ws + 1]
         vir_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
         ori_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
         check(lib.apt_sp_unpack_frontier(ops._ptr(recv), recv.numel(), ops._ptr(total), n_total,
@@ -777,64 +768,70 @@ class SPVirtualSampler(_GraphReplay):
         lo, hi = ops._owned_range()
         unique_src, a_src = ops._unique_enqueue(ori_src, total, lo, hi, st.word(self._US), "unique_sp_src")
         unique_dst, a_dst = ops._unique_enqueue(vir_src, total, 0, ws * ops.SP_BASE, st.word(self._UD), "unique_vdst")
-        div = cur_n if cur_n is not None else max(s_max, 1)
-        arange_dst = torch.remainder(unique_frontier, div)
-        return dict(layers=layers, slot=slot, cur=cur, nbr=nbr, sorted_all=sorted_all, packed=packed,
+        if ws == 1 and not with_dst:
+            arange_dst = unique_frontier        # owner 0: a virtual node is its destination's index
+        else:
+            arange_dst = torch.remainder(unique_frontier, cur_n if cur_n is not None else max(s_max, 1))
+        # the input nodes (the reference's torch.cat of destinations and received neighbours)
+        us_word = st.word(self._US)
+        none = torch.empty(0, dtype=torch.int64, device=dev)
+        if with_dst:
+            head, head_n = recv_dst, dst_counts[ws:ws + 1]
+        elif self.model == "GCN":
+            head, head_n = none, None
+        else:
+            head, head_n = cur, cur_n
+        in_word = st.word(self._IN)
+        prefetch = self.prefetch_features and _fits_prefetch(head.numel() + unique_src.numel())
+        input_nodes = ops.concat_ids(head, head_n, unique_src, us_word, in_word, look_up=prefetch)
+        if publish is not None:
+            publish()
+        rows = ops._gather_enqueue(input_nodes, in_word) if prefetch else None
+        return dict(layers=layers, cur=cur, nbr=nbr, sorted_all=sorted_all, packed=packed,
                     unique_frontier=unique_frontier, arange_dst=arange_dst, vir_src=vir_src, ori_src=ori_src,
                     unique_src=unique_src, a_src=a_src, unique_dst=unique_dst, a_dst=a_dst, dst_sorted=dst_sorted,
-                    recv_dst=recv_dst)
+                    recv_dst=recv_dst, input_nodes=input_nodes, rows=rows)
 
-    def _finish(self, seeds, b, host=None):
+    def _finish(self, seeds, b, host=None, plan=None):
         """The one host read of the mini-batch, then everything is narrowed to its real size."""
         st = ops.STATE
         ws = st.world_size
-        dev = seeds.device
         f = self.fanouts[0]
         if host is None:
             host = st.read_words()
-        count = [int(host[k]) for k in range(b["slot"])]
-        blocks = []
-        n_dst = seeds.numel()
-        for dst_buf, rel, uniq, u_s, fanout in b["layers"]:
-            n_src = count[u_s]
-            blocks.insert(0, Block(rel[:n_dst * fanout], _coo_col(dst_buf.numel(), n_dst, fanout, dev), n_src, n_dst,
-                                   uniq[:n_src], fanout))
-            n_dst = n_src
-        num_dst = n_dst
-        n_uf, n_us, n_ud = int(host[self._UF]), int(host[self._US]), int(host[self._UD])
-        n_recv = int(host[16 + ws])
+        blocks, num_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
+        h = host.tolist()
+        n_uf, n_us, n_ud, n_in = h[self._UF], h[self._US], h[self._UD], h[self._IN]
         with_dst = self.shuffle_with_dst
         k = 3 if with_dst else 2
-        n_rdst = int(host[self._RDST + ws]) if with_dst else 0
+        if ws == 1 and not with_dst:
+            send, recv = [num_dst * f, n_uf], [num_dst * f, n_uf]
+            n_recv = num_dst * f
+        else:
+            send, recv = h[self._SEND:self._SEND + k * ws], h[self._RECV:self._RECV + k * ws]
+            n_recv = h[16 + ws]
+        n_rdst = h[self._RDST + ws] if with_dst else 0
         if n_recv > b["vir_src"].numel() or (with_dst and n_rdst > b["recv_dst"].numel()):
             raise RuntimeError("chained SNP sampler: more ids received than the buffer sized from this rank's own "
                                "batch holds; use chained=False for batches that differ this much between the ranks")
-        h = host.tolist()
-        send_sizes_cpu = torch.tensor(h[self._SEND:self._SEND + k * ws], dtype=torch.int64)
-        recv_sizes_cpu = torch.tensor(h[self._RECV:self._RECV + k * ws], dtype=torch.int64)
-        unique_frontier, unique_src = b["unique_frontier"], b["unique_src"]
-        block1 = Block(torch.arange(n_uf, device=dev), b["arange_dst"][:n_uf], n_uf, num_dst, unique_frontier[:n_uf], f)
-        block2 = Block(b["a_src"][:n_recv], b["a_dst"][:n_recv], n_us, n_ud, unique_src[:n_us], f)
-        blocks.insert(0, block1)
-        blocks.insert(0, block2)
-        dst_nodes = b["cur"][:num_dst]
-        n_all = num_dst * f + (num_dst if with_dst else 0)
-        send_frontier = b["packed"][:num_dst * f]
+        send_sizes_cpu, recv_sizes_cpu = torch.tensor(send, dtype=torch.int64), torch.tensor(recv, dtype=torch.int64)
+        n_nbr = num_dst * f
+        (unique_frontier, unique_src, arange_dst, a_src, a_dst, input_nodes, neighbors, sorted_all, packed, vir_src, ori_src,
+         unique_dst) = _native.fronts(
+            [b["unique_frontier"], b["unique_src"], b["arange_dst"], b["a_src"], b["a_dst"], b["input_nodes"], b["nbr"],
+             b["sorted_all"], b["packed"], b["vir_src"], b["ori_src"], b["unique_dst"]],
+            [n_uf, n_us, n_uf, n_recv, n_recv, n_in, n_nbr, n_nbr + (num_dst if with_dst else 0), n_nbr, n_recv, n_recv, n_ud])
+        blocks.insert(0, Block(_arange(n_uf, seeds.device), arange_dst, n_uf, num_dst, unique_frontier, f))
+        blocks.insert(0, Block(a_src, a_dst, n_us, n_ud, unique_src, f))
         recv_dst = None
         if with_dst:
-            send_frontier = torch.cat((b["dst_sorted"][:num_dst], send_frontier))
+            packed = torch.cat((b["dst_sorted"][:num_dst], packed))
             recv_dst = b["recv_dst"][:n_rdst]
-        self.last = dict(neighbors=b["nbr"][:num_dst * f], sorted_allnodes=b["sorted_all"][:n_all],
-                         unique_frontier=unique_frontier[:n_uf], send_frontier=send_frontier, recv_dst=recv_dst,
-                         vir_src=b["vir_src"][:n_recv], ori_src=b["ori_src"][:n_recv],
-                         unique_dst=b["unique_dst"][:n_ud])
-        if with_dst:
-            nxt = torch.cat((recv_dst, unique_src[:n_us]))
-        elif self.model == "GCN":
-            nxt = unique_src[:n_us]
-        else:
-            nxt = torch.cat((dst_nodes, unique_src[:n_us]))
-        return nxt, seeds, blocks, send_sizes_cpu, recv_sizes_cpu
+        self.last = dict(neighbors=neighbors, sorted_allnodes=sorted_all, unique_frontier=unique_frontier,
+                         send_frontier=packed, recv_dst=recv_dst, vir_src=vir_src, ori_src=ori_src, unique_dst=unique_dst)
+        if b["rows"] is not None:
+            st.prefetched = (input_nodes, b["rows"][:n_in], plan)
+        return input_nodes, seeds, blocks, send_sizes_cpu, recv_sizes_cpu
 
     def _outer(self, seeds, neighbors, fanout):
         st = ops.STATE
@@ -929,7 +926,7 @@ class MPSampler(_GraphReplay):
     # for the two broadcasts, [128..223] every rank's three sizes
     _MINE, _ALL = 54, 128
 
-    def _enqueue(self, seeds: torch.Tensor, call_base_dev):
+    def _enqueue(self, seeds: torch.Tensor, call_base_dev, publish=None):
         """Every kernel of the mini-batch on the current stream without a host read: sizes stay in the
         device word block, buffers are upper bounds, the broadcasts take device-side counts."""
         st = ops.STATE
@@ -948,7 +945,7 @@ class MPSampler(_GraphReplay):
             uniq, rel, _ = ops._sample_relabel_enqueue(cur, fanout, cur_n, cnt, call if explicit else None,
                                                        call_base_dev)
             call += 1
-            layers.append((cur, rel, uniq, slot, fanout))
+            layers.append(_layer(cur, rel, uniq, fanout, slot))
             cur, cur_n = uniq, cnt
             slot += 1
         f = self.fanouts[0]
@@ -972,9 +969,9 @@ class MPSampler(_GraphReplay):
             all_sizes.copy_(got[:ws])
         recv_frontier, _ = ex.allbroadcast_enqueue(unique_frontier.view(-1, 1), mine[1:2], words[16:16 + ws + 1])
         recv_coo, _ = ex.allbroadcast_enqueue(coo_row.view(-1, 1), mine[2:3], words[64:64 + ws + 1])
-        return dict(layers=layers, slot=slot, recv_frontier=recv_frontier, recv_coo=recv_coo)
+        return dict(layers=layers, recv_frontier=recv_frontier, recv_coo=recv_coo)
 
-    def _finish(self, seeds, b, host=None):
+    def _finish(self, seeds, b, host=None, plan=None):
         """The one host read of the mini-batch, then everything is narrowed to its real size."""
         st = ops.STATE
         ws = st.world_size
@@ -982,14 +979,7 @@ class MPSampler(_GraphReplay):
         f = self.fanouts[0]
         if host is None:
             host = st.read_words()
-        count = [int(host[k]) for k in range(b["slot"])]
-        blocks = []
-        n_dst = seeds.numel()
-        for dst_buf, rel, uniq, u_s, fanout in b["layers"]:
-            n_src = count[u_s]
-            blocks.insert(0, Block(rel[:n_dst * fanout], _coo_col(dst_buf.numel(), n_dst, fanout, dev), n_src, n_dst,
-                                   uniq[:n_src], fanout))
-            n_dst = n_src
+        blocks, n_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
         sizes = host[self._ALL:self._ALL + 3 * ws].view(ws, 3)
         sizes = torch.tensor(sizes.tolist(), dtype=torch.int64)        # off the pinned block
         recv_size = sizes[:, 0].contiguous()
@@ -1028,13 +1018,24 @@ class MPSampler(_GraphReplay):
 
 class DPNeighborSampler:
     """GDP strategy: every hop local (python/npc/sampler.py:202-203 with the
-    common block construction)."""
+    common block construction).
 
-    def __init__(self, rank: int, fanouts: List[int]):
+    chained            enqueue the whole mini-batch with device-side sizes and one host read (one C++ call; every result
+                       is a tensor of its own) instead of one read per hop
+    prefetch_features  also enqueue the feature gather of the input nodes behind that read; the next
+                       ops.load_subtensor(input_nodes) returns it"""
+
+    def __init__(self, rank: int, fanouts: List[int], chained: bool = None, prefetch_features: bool = True):
         self.rank = rank
         self.fanouts = list(fanouts)
+        if chained is None:
+            chained = os.environ.get("APT_CHAINED_SAMPLER", "1") != "0"
+        self.chained = bool(chained)
+        self.prefetch_features = prefetch_features
 
     def sample(self, graph, seeds: torch.Tensor):
+        if self._chained_fits(seeds):
+            return self._sample_chained(seeds)
         output_nodes = seeds
         blocks = []
         for fanout in reversed(self.fanouts):
@@ -1043,3 +1044,37 @@ class DPNeighborSampler:
             seeds = block.src_ids
             blocks.insert(0, block)
         return seeds, output_nodes, blocks
+
+    # Upper-bound buffers (no id met twice) beyond this many ids are not worth one read: hop by hop then.
+    _CHAINED_IDS = 1 << 25
+
+    def _chained_fits(self, seeds) -> bool:
+        st = ops.STATE
+        bound = seeds.numel()
+        for f in self.fanouts:
+            bound *= 1 + f
+        return self.chained and st.sample_replace and not st.profiling and st.graph.uva_indptr is not None and \
+            0 < bound <= self._CHAINED_IDS and 0 < len(self.fanouts) <= 14 and min(self.fanouts) > 0
+
+    def _sample_chained(self, seeds):
+        st = ops.STATE
+        g, f = st.graph, st.feat
+        ids = ops._need_cuda(seeds, "seeds")
+        order = [int(x) for x in reversed(self.fanouts)]
+        bound = ids.numel()
+        for x in order:
+            bound *= 1 + x
+        features = (f.feat_pos_map, f.dev_feats, f.uva_feats, f.num_total_nodes, f.feat_dim_offset) \
+            if self.prefetch_features and f.feat_pos_map is not None else None
+        call = st.sample_calls
+        st.sample_calls += len(order)
+        words = st.words()
+        input_nodes, blocks, rows, flags = _native.dp_sample(
+            ids, order, g.adj_pos_map, g.num_total_nodes, g.dev_indptr, g.dev_indices, g.uva_indptr, g.uva_indices, st.sample_key,
+            call, ops._relabel_workspace(bound), words, st._lane_words[st.lane][1], st.next_sequence(), features,
+            _PREFETCH_LIMIT_BYTES, Block)
+        if flags:
+            st.check_flags(flags)
+        if rows is not None:
+            st.prefetched = (input_nodes, rows, None)
+        return input_nodes, seeds, blocks

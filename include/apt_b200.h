@@ -71,6 +71,15 @@ void apt_launch_count_reset(void);
  * its sizes with blocking copies (src/sampling.cc:176-185). */
 int apt_memcpy_async(void* dst, const void* src, size_t nbytes, void* stream);
 
+/* Small results for the host without a copy and an event: a kernel on `stream` stores
+ * count words into page-locked host memory and then, behind them, a sequence number
+ * (*sequence_dev when given: a word that a captured graph's replay brings along);
+ * apt_wait_published polls host[count] for it. An error on the stream, or an idle
+ * stream without an answer, ends the wait with a status. host holds count + 1 words. */
+int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_dev,
+                      int64_t sequence, int64_t* host, void* stream);
+int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream);
+
 /* Optional per-kernel timing. When enabled, every launch of a tagged kernel
  * is bracketed by CUDA events on its own stream; apt_profile_read
  * synchronises those events and returns the summed milliseconds and launch
@@ -169,18 +178,23 @@ int apt_sample_relabel_csc(const int64_t* seeds, int64_t num_seeds,
                            int64_t* out_relabeled, int64_t* out_num_unique,
                            int32_t* status_word, void* stream);
 /* The same with the other side of the block's edges: out_col[j * fanout + i] = j (may be
- * null), what arange(num_seeds).repeat_interleave(fanout) gives (python/npc/sampler.py:78). */
+ * null), what arange(num_seeds).repeat_interleave(fanout) gives (python/npc/sampler.py:78);
+ * and, with feat_pos_map (may be null), every unique id is looked up as apt_gather_rows
+ * will and what that would flag is flagged here, so that the flags are complete before a
+ * gather of the ids has run. */
 int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
-                           const int64_t* num_seeds_dev, int fanout,
-                           const int64_t* adj_pos_map, int64_t num_nodes,
-                           const int64_t* dev_indptr, const int64_t* dev_indices,
-                           const int64_t* uva_indptr, const int64_t* uva_indices,
-                           uint64_t key, uint32_t call_id,
-                           const int64_t* call_id_base_dev,
-                           void* workspace, size_t workspace_bytes,
-                           int64_t* out_neighbors, int64_t* out_unique,
-                           int64_t* out_relabeled, int64_t* out_col, int64_t* out_num_unique,
-                           int32_t* status_word, void* stream);
+                             const int64_t* num_seeds_dev, int fanout,
+                             const int64_t* adj_pos_map, int64_t num_nodes,
+                             const int64_t* dev_indptr, const int64_t* dev_indices,
+                             const int64_t* uva_indptr, const int64_t* uva_indices,
+                             uint64_t key, uint32_t call_id,
+                             const int64_t* call_id_base_dev,
+                             void* workspace, size_t workspace_bytes,
+                             int64_t* out_neighbors, int64_t* out_unique,
+                             int64_t* out_relabeled, int64_t* out_col,
+                             int64_t* out_num_unique, const int64_t* feat_pos_map,
+                             int64_t feat_num_nodes, int64_t num_dev_rows,
+                             int64_t num_uva_rows, int32_t* status_word, void* stream);
 
 /* ----------------------------------------------------------- owner bucketing
  * Stable partition of ids by owning rank. Takes the role of ClusterAndPermute
@@ -507,6 +521,12 @@ int apt_cached_access(const int32_t* counters, int64_t num_nodes,
 int apt_concat_ids(const int64_t* a, int64_t num_a, const int64_t* num_a_dev,
                    const int64_t* b, int64_t num_b, const int64_t* num_b_dev,
                    int64_t* out, int64_t* out_count_dev, void* stream);
+/* The same for ids of a gather: see apt_sample_relabel_block for the look-up. */
+int apt_concat_row_ids(const int64_t* a, int64_t num_a, const int64_t* num_a_dev,
+                       const int64_t* b, int64_t num_b, const int64_t* num_b_dev,
+                       int64_t* out, int64_t* out_count_dev, const int64_t* feat_pos_map,
+                       int64_t feat_num_nodes, int64_t num_dev_rows,
+                       int64_t num_uva_rows, int32_t* status_word, void* stream);
 
 /* ------------------------------------------------------- local row movers
  * out[i] = in[index[i]] and out[index[i]] = in[i] over rows of row_bytes
