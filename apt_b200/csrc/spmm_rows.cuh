@@ -100,7 +100,9 @@ inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t n
   RowSplit r;
   const int64_t nvec = feat_dim / ve;
   r.ve = ve;
-  // one slice a lane while 32 lanes cover the row; two, then four, beyond (wider rows are walked in column blocks)
+  // one slice a lane while 32 lanes cover the row; two, then four, beyond (wider rows are walked in column blocks). Half as
+  // many lanes with twice the slices, two edges side by side, take half the address arithmetic but more registers:
+  // 64 -> 98 us for bf16 x 256.
   r.vpl = nvec <= 32 ? 1 : nvec <= 64 ? 2 : 4;
   r.lpe = pow2_ge(ceil_div(nvec, r.vpl));
   // edges side by side: never more than half the mean row, whose second half would idle those lanes
@@ -193,7 +195,7 @@ __device__ __forceinline__ void slice_add(Acc<VE>& acc, float& acc2, const EdgeS
 // The sums of the edges read side by side meet, and the lanes of the first of them write the row's column block.
 template <typename T, int VE, int VPL, int OP>
 __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], float (&acc2)[VPL], const int (&col)[VPL],
-                                           const int (&head)[VPL], int d, int c0, int nvec, int per, int lpe, int lpr, int vl,
+                                           const int (&head)[VPL], unsigned lead, int d, int c0, int nvec, int lpe, int lpr, int vl,
                                            int epi, unsigned gmask) {
 #pragma unroll 1
   for (int o = lpe; o < lpr; o <<= 1)
@@ -208,7 +210,7 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[V
     if (c0 + vl + i * lpe >= nvec) continue;
     store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
     if constexpr (OP == kGatSrc)
-      if (col[i] % per == 0) a.out2[(int64_t)d * a.edata_dim + head[i]] = Elem<T>::from_f(acc2[i]);
+      if (lead >> i & 1u) a.out2[(int64_t)d * a.edata_dim + head[i]] = Elem<T>::from_f(acc2[i]);
   }
 }
 
@@ -310,6 +312,29 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   };
   if (items) start_item(); else start_rows();
 
+  // the lane's columns: worked out once for rows of one column block (the divisions by the head width took a quarter of
+  // a short row's instructions)
+  const T *lane_in = nullptr, *lane_ed[VPL];
+  uint32_t off[VPL];      // bytes from the lane's first slice; lanes past the row's last slice read their first one again
+  int head[VPL], col[VPL], at_block = 0;
+  unsigned lead = 0;      // slices that open a head
+  auto set_block = [&](int c0) {
+    at_block = c0;
+    lead = 0;
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      col[i] = (c0 + vl + i * lpe < nvec ? c0 + vl + i * lpe : i == 0 ? nvec - 1 : c0 + vl < nvec ? c0 + vl : nvec - 1) * VE;
+      head[i] = (OP == kGatSrc || OP == kUMulW || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
+      if (OP == kGatSrc && head[i] * per == col[i]) lead |= 1u << i;
+      off[i] = (uint32_t)((col[i] - col[0]) * (int)sizeof(T));
+      lane_ed[i] = OP == kGatSrc  ? (const T*)((const float2*)a.edata + head[i])
+                   : OP == kUMulW ? (const T*)((const float*)a.edata + head[i])
+                                  : a.edata + (head[i] >= 0 ? head[i] : col[i]);
+    }
+    lane_in = a.in + col[0];
+  };
+  set_block(0);
+
   while (items || d < num_rows) {
     int nnb = 0, nne = 0;
     if (!items) {
@@ -320,21 +345,14 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     const bool skip = !items && mode == kOrder && e - b > a.split.long_edges;
 #pragma unroll 1
     for (int c0 = 0; c0 < nvec && !skip; c0 += lpe * VPL) {
+      if (c0 != at_block) set_block(c0);
       Acc<VE> acc[VPL];
       float acc2[VPL];
-      int head[VPL], col[VPL];
-      const T* lane_ed[VPL];
-      uint32_t off[VPL];      // bytes from the lane's first slice; lanes past the row's last slice read their first one again
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
         acc2[i] = 0.f;
         acc[i].zero();
-        col[i] = (c0 + vl + i * lpe < nvec ? c0 + vl + i * lpe : i == 0 ? nvec - 1 : c0 + vl < nvec ? c0 + vl : nvec - 1) * VE;
-        head[i] = (OP == kGatSrc || OP == kUMulW || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
-        off[i] = (uint32_t)((col[i] - col[0]) * (int)sizeof(T));
-        lane_ed[i] = OP == kGatSrc ? (const T*)((const float2*)a.edata + head[i]) : OP == kUMulW ? (const T*)((const float*)a.edata + head[i]) : a.edata + (head[i] >= 0 ? head[i] : col[i]);
       }
-      const T* const lane_in = a.in + col[0];
       uint32_t my_src = src, my_e = eid;
 #pragma unroll 1
       for (int k0 = b; k0 < e; k0 += LPR) {
@@ -395,7 +413,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
 #pragma unroll
             for (int t = 0; t < VE; ++t) __stcg(p + col[i] + t, acc[i].get(t));
             if constexpr (OP == kGatSrc)
-              if (col[i] % per == 0) __stcg(p + a.feat_dim + head[i], acc2[i]);
+              if (lead >> i & 1u) __stcg(p + a.feat_dim + head[i], acc2[i]);
           }
         }
         if (c0 + lpe * VPL < nvec) continue;
@@ -411,10 +429,9 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
         __threadfence();
 #pragma unroll 1
         for (int cc = 0; cc < nvec; cc += lpe * VPL) {
+          if (cc != at_block) set_block(cc);
 #pragma unroll
           for (int i = 0; i < VPL; ++i) {
-            col[i] = min(cc + vl + i * lpe, nvec - 1) * VE;
-            head[i] = OP == kGatSrc ? col[i] / per : -1;
             acc2[i] = 0.f;
             acc[i].zero();
 #pragma unroll 1
@@ -428,11 +445,11 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
           }
           c0 = cc;
           if (cc + lpe * VPL < nvec) {
-            rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, d, c0, nvec, per, lpe, LPR, vl, EPI, GMASK);
+            rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, lead, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
           }
         }
       }
-      rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, d, c0, nvec, per, lpe, LPR, vl, EPI, GMASK);
+      rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, lead, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
     }
     if (items) {
       it += warps;
