@@ -18,8 +18,12 @@
 //   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination. The four partial dots of a
 //                   lane are reduced together: each step halves the values a lane keeps, log2(lph) + 1 shuffles
 //                   for four edges instead of 4 log2(lph).
-//   k_gat_scores    backward: t, grad_s and grad_er, one thread per destination and head
-//   row kernel      both sums over the source side in one walk (kGatSrc) behind one counting sort by source
+//   k_gat_scores    backward: t, grad_s and grad_er, one thread per destination and head; grad_el is added up in fp32 with
+//                   one reduction per edge and head (the heads of an edge are neighbours: one sector)
+//   row kernel      grad_ft: the weighted sum of the forward with the sides swapped, behind one counting sort by source.
+//                   With grad_el as a second accumulator of the same walk it held two blocks an SM instead of three:
+//                   150 us against 116, and the scores had to be written out for it.
+//   k_gat_source    grad_el in T
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
@@ -152,14 +156,15 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
       // lanes without a slice read one that exists and contribute zero
       const int64_t col = (int64_t)(rows ? h : h0) * head_dim;
       const T* const grad = grad_out + (int64_t)d * num_heads * head_dim + col;
-      Raw<T, VE> g;
+      F2 g[Acc<VE>::P];      // the gradient's slice, unpacked
       int at = 0;
       auto block = [&](int c0) {
         at = min(c0 + p, nvh - 1) * VE;
-        g = load_raw<T, VE>(grad + at);
-        if (c0 + p >= nvh) {
+        const Raw<T, VE> raw = load_raw<T, VE>(grad + at);
 #pragma unroll
-          for (int q = 0; q < (int)(sizeof(g.w) / 4); ++q) g.w[q] = 0u;
+        for (int q = 0; q < Acc<VE>::P; ++q) {
+          if constexpr (VE > 1) g[q] = pair_of(raw, q); else g[q] = f2_pack(raw.get(0), 0.f);
+          if (c0 + p >= nvh) g[q] = 0ull;
         }
       };
       block(0);
@@ -181,15 +186,15 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
               v[u] = load_raw<T, VE>(at_row(lane_ft, __shfl_sync(0xffffffffu, my_src, (j0 + u * ep + epi) & 31), row_bytes));
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              Acc<VE> acc;
-              acc.zero();
-              acc.fma(g, v[u]);
-              F2 pair = acc.p[0];
+              F2 pair = 0ull;
 #pragma unroll
-              for (int q = 1; q < Acc<VE>::P; ++q) pair = f2_add(pair, acc.p[q]);
+              for (int q = 0; q < Acc<VE>::P; ++q) {
+                if constexpr (VE > 1) pair = f2_fma(g[q], pair_of(v[u], q), pair);
+                else pair = f2_fma(g[q], f2_pack(v[u].get(0), 0.f), pair);
+              }
               float lo, hi;
               f2_unpack(pair, lo, hi);
-              dt[u] += VE > 1 ? lo + hi : lo;
+              dt[u] += lo + hi;
             }
           }
           float* const out = dots + (int64_t)(base + j0 + epi) * num_heads + h;
@@ -216,25 +221,25 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
   }
 }
 
-// Score gradients. Writes (weight, gradient) pairs for the source side, or both in T for callers of the edge part alone.
+// Score gradients: added to sums[source][head] (if sums), or written with the weights, both in T, for callers of the
+// edge part alone.
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
-             int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
-             const float* __restrict__ weight, const float* __restrict__ dots, float2* __restrict__ pair, T* __restrict__ attn,
+             int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
+             float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, T* __restrict__ attn,
              T* __restrict__ grad_score, T* __restrict__ grad_er) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  auto put = [&](int64_t o, float w, float gs) {
-    if (pair) {
-      pair[o] = make_float2(w, gs);
-    } else {
-      attn[o] = Elem<T>::from_f(w);
-      grad_score[o] = Elem<T>::from_f(gs);
-    }
-  };
   const bool empty = *none != 0;
-  if (empty)
-    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += stride) put(o, 0.f, 0.f);
+  if (empty)   // no edge belongs to anybody
+    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += stride) {
+      if (sums) {
+        weight[o] = 0.f;
+      } else {
+        attn[o] = Elem<T>::from_f(0.f);
+        grad_score[o] = Elem<T>::from_f(0.f);
+      }
+    }
   const int64_t total = num_dst * num_heads;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
@@ -249,14 +254,26 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
     }
 #pragma unroll 4
     for (int e = r.x; e < r.y; ++e) {
-      const int64_t o = (int64_t)e * num_heads + h;
+      const int64_t o = (int64_t)e * num_heads + h, src = row[e];
       const float w = weight[o];
-      const float gs = w * (dots[o] - t) * (Elem<T>::to_f(el[row[e] * num_heads + h]) + bias > 0.f ? 1.f : slope);
+      const float gs = w * (dots[o] - t) * (Elem<T>::to_f(el[src * num_heads + h]) + bias > 0.f ? 1.f : slope);
       ger += gs;
-      put(o, w, gs);
+      if (sums) {
+        if ((uint64_t)src < (uint64_t)num_src) atomicAdd(sums + src * num_heads + h, gs);
+      } else {
+        attn[o] = Elem<T>::from_f(w);
+        grad_score[o] = Elem<T>::from_f(gs);
+      }
     }
     grad_er[i] = Elem<T>::from_f(ger);
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_gat_source(const float* __restrict__ sums, int64_t n, T* __restrict__ grad_el) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    grad_el[i] = Elem<T>::from_f(sums[i]);
 }
 
 // ---- host side ----------------------------------------------------------------------
@@ -280,18 +297,20 @@ static size_t gat_edges_layout(int64_t num_dst, int64_t E, int H, char* base, Ga
 }
 
 struct GatBwdWs {
+  float* sums;      // [num_src][heads], cleared with the front of the sort
   SpmmWs sort;
   float* dots;      // [E][heads]
-  float2* pair;     // [E][heads]
+  size_t zero_bytes;
 };
 static size_t gat_bwd_layout(int64_t num_src, int64_t E, int H, char* base, GatBwdWs* ws) {
-  const size_t o_dots = spmm_layout(num_src, E, base, ws ? &ws->sort : nullptr);
-  const size_t o_pair = o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
+  const size_t o_sort = align_up((size_t)(num_src > 0 ? num_src : 1) * H * 4, 256);
+  const size_t o_dots = o_sort + spmm_layout(num_src, E, base + o_sort, ws ? &ws->sort : nullptr);
   if (ws) {
+    ws->sums = (float*)base;
     ws->dots = (float*)(base + o_dots);
-    ws->pair = (float2*)(base + o_pair);
+    ws->zero_bytes = o_sort + ws->sort.zero_bytes;
   }
-  return o_pair + align_up((size_t)(E > 0 ? E : 1) * H * 8, 256);
+  return o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
 }
 
 struct GatProblem {
@@ -337,7 +356,7 @@ static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* 
   SpmmWs ws{};
   ws.range = g.range;
   const RowArgs<T> a{q.row, (const T*)q.ft, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, ws,
-                     (T*)out, nullptr, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none};
+                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none};
   ProfScope prof("gat_rows", s);
   return launch_spmm_rows<T>(kUMulW, a, s);
 }
@@ -357,8 +376,8 @@ static int launch_dots(const GatProblem& q, const GatEdges& g, float* dots, cuda
 
 // The edge part of the backward: weights are there already.
 template <typename T>
-static int gat_edge_backward(const GatProblem& q, const GatEdges& g, float* dots, float2* pair, void* attn, void* grad_score,
-                             void* grad_er, cudaStream_t s) {
+static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num_src, float* dots, float* sums, void* attn,
+                             void* grad_score, void* grad_er, cudaStream_t s) {
   ProfScope prof("gat_bwd_rows", s);
   int rc;
   switch (slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T)) {
@@ -369,26 +388,29 @@ static int gat_edge_backward(const GatProblem& q, const GatEdges& g, float* dots
   }
   if (rc != APT_OK) return rc;
   APT_LAUNCH(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-             q.slope, q.num_dst, q.E, g.range, g.none, g.weight, dots, pair, (T*)attn, (T*)grad_score, (T*)grad_er);
+             q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, (T*)attn, (T*)grad_score, (T*)grad_er);
   return APT_OK;
 }
 
 template <typename T>
 static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, char* workspace, int64_t num_src, void* grad_ft,
                         void* grad_el, void* grad_er, cudaStream_t s) {
-  int rc = gat_edge_backward<T>(q, g, ws.dots, ws.pair, nullptr, nullptr, grad_er, s);
+  APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
+  int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, nullptr, nullptr, grad_er, s);
   if (rc != APT_OK) return rc;
   const int64_t dim = q.H * q.Dh;
   const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
   const RowSplit split = row_split(dim, ve, q.E, num_src);
   const SegTable st{nullptr, nullptr, nullptr, 1};
-  APT_CUDA(cudaMemsetAsync(workspace, 0, ws.sort.zero_bytes, s));
-  rc = launch_group(q.col, q.row, q.E, st, num_src, ws.sort, kOrder, split.long_edges, (int)dim + q.H, s);
+  rc = launch_group(q.col, q.row, q.E, st, num_src, ws.sort, kOrder, split.long_edges, (int)dim, s);
   if (rc != APT_OK) return rc;
-  const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)ws.pair, q.H, dim, st, num_src, q.E, ws.sort,
-                     (T*)grad_ft, (T*)grad_el, kOrder, 0, split, (int)dim + q.H, nullptr};
+  const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, st, num_src, q.E, ws.sort,
+                     (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr};
   ProfScope prof("spmm_rows", s);
-  return launch_spmm_rows<T>(kGatSrc, a, s);
+  rc = launch_spmm_rows<T>(kUMulW, a, s);
+  if (rc != APT_OK) return rc;
+  APT_LAUNCH(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (T*)grad_el);
+  return APT_OK;
 }
 
 // Stream-ordered memory for the duration of a call, for the two entry points without a buffer for weights.
@@ -536,7 +558,7 @@ extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const in
 #define APT_RUN(T)                                                                                         \
   do {                                                                                                     \
     if ((rc = gat_weights<T>(q, g, nullptr, s)) != APT_OK) return rc;                                      \
-    return gat_edge_backward<T>(q, g, dots, nullptr, out_attn, out_grad_score, out_grad_er, s);            \
+    return gat_edge_backward<T>(q, g, 0, dots, nullptr, out_attn, out_grad_score, out_grad_er, s);                     \
   } while (0)
   switch (dtype) {
     case APT_F32: APT_RUN(float);

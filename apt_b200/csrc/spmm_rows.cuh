@@ -32,8 +32,8 @@
 namespace apt {
 
 constexpr int kMaxSegments = 64;
-// kUMulW: one fp32 weight per head. kGatSrc: the same with a second fp32 value per head that is summed beside the row.
-enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kUMulW = 4, kGatSrc = 5 };
+// kUMulW: one fp32 weight per edge and head.
+enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kUMulW = 4 };
 enum { kDevice = -1, kFixed = 0, kRanges = 1, kOrder = 2 };
 
 // Rows of more edges are left to whole warps. A group narrower than a warp hands over earlier: its own pace is
@@ -115,13 +115,12 @@ template <typename T>
 struct RowArgs {
   const int64_t* row;
   const T* in;
-  const T* edata;          // kUMulW: float[E][heads]; kGatSrc: float2[E][heads]
+  const T* edata;          // kUMulW: float[E][heads]
   int64_t edata_dim, feat_dim;
   SegTable st;
   int64_t num_rows, num_edges;
   SpmmWs ws;
   T* out;
-  T* out2;                 // kGatSrc: [rows][heads] sums of the score gradients
   int mode, fixed;
   RowSplit split;
   int part_stride;         // floats per part
@@ -134,7 +133,7 @@ template <typename T, int VE, int OP>
 struct EdgeSlice {
   Raw<T, VE> x;                                           // input slice (kCopyE: the edge's own)
   Raw<T, (OP == kUMulE || OP == kUAddE) ? VE : 2 / sizeof(T) + 1> w;   // per-column edge values
-  float s, s2;                                            // per-head edge value (kGatSrc: and gradient)
+  float s;                                                // per-head edge value
 };
 
 // `lane_in` and `lane_edata` point at the lane's column of row 0, `off` bytes before this slice.
@@ -160,15 +159,10 @@ __device__ __forceinline__ void slice_load(EdgeSlice<T, VE, OP>& v, const RowArg
     }
   }
   if constexpr (OP == kUMulW) v.s = __ldg((const float*)at_row(lane_edata, e, edata_bytes));
-  if constexpr (OP == kGatSrc) {
-    const float2 p = __ldg((const float2*)at_row(lane_edata, e, edata_bytes));
-    v.s = p.x;
-    v.s2 = p.y;
-  }
 }
 
 template <typename T, int VE, int OP>
-__device__ __forceinline__ void slice_add(Acc<VE>& acc, float& acc2, const EdgeSlice<T, VE, OP>& v, int per, int head) {
+__device__ __forceinline__ void slice_add(Acc<VE>& acc, const EdgeSlice<T, VE, OP>& v, int per, int head) {
   if constexpr (OP == kUMulE) {
     if (per != 1 && head >= 0) {
       acc.fma(v.x, v.s);
@@ -184,33 +178,26 @@ __device__ __forceinline__ void slice_add(Acc<VE>& acc, float& acc2, const EdgeS
     } else {
       acc.add(v.w);
     }
-  } else if constexpr (OP == kUMulW || OP == kGatSrc) {
+  } else if constexpr (OP == kUMulW) {
     acc.fma(v.x, v.s);
-    if constexpr (OP == kGatSrc) acc2 += v.s2;
   } else {
     acc.add(v.x);
   }
 }
 
 // The sums of the edges read side by side meet, and the lanes of the first of them write the row's column block.
-template <typename T, int VE, int VPL, int OP>
-__device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], float (&acc2)[VPL], const int (&col)[VPL],
-                                           const int (&head)[VPL], unsigned lead, int d, int c0, int nvec, int lpe, int lpr, int vl,
+template <typename T, int VE, int VPL>
+__device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], const int (&col)[VPL], int d, int c0, int nvec, int lpe, int lpr, int vl,
                                            int epi, unsigned gmask) {
 #pragma unroll 1
   for (int o = lpe; o < lpr; o <<= 1)
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      acc[i].join(gmask, o);
-      if constexpr (OP == kGatSrc) acc2[i] += __shfl_xor_sync(gmask, acc2[i], o);
-    }
+    for (int i = 0; i < VPL; ++i) acc[i].join(gmask, o);
   if (epi != 0) return;
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     if (c0 + vl + i * lpe >= nvec) continue;
     store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
-    if constexpr (OP == kGatSrc)
-      if (lead >> i & 1u) a.out2[(int64_t)d * a.edata_dim + head[i]] = Elem<T>::from_f(acc2[i]);
   }
 }
 
@@ -220,7 +207,6 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[V
 // four; bf16 x 256: 89 / 65 / 63 us; the reverse direction 186 / 149 / 158 and 104 / 82 / 90 us.
 constexpr int rows_min_blocks(int op, int elems) {
   if (op == kCopyU || op == kCopyE || op == kUMulW) return elems <= 4 ? 4 : elems <= 8 ? 3 : 2;
-  if (op == kGatSrc) return elems <= 8 ? 2 : 1;   // three blocks spill: 158 -> 188 us on the attention backward (bf16, 4 x 64)
   return elems <= 2 ? 3 : elems <= 8 ? 2 : 1;
 }
 
@@ -230,7 +216,7 @@ __global__ void __launch_bounds__(256, rows_min_blocks(OP, VE * VPL))
 k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   constexpr int U = VPL >= 2 ? 2 : 4;
   __shared__ int64_t coo[kMaxSegments + 1], ioff[kMaxSegments + 1];
-  int mode = OP == kGatSrc ? kOrder : a.mode, fixed = a.fixed;
+  int mode = a.mode, fixed = a.fixed;
   if (mode == kDevice) {
     const int64_t w = *a.ws.result;
     mode = probe_mode(w);
@@ -249,7 +235,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   const int nvec = (int)(a.feat_dim / VE);
   const int per = (int)(a.feat_dim / a.edata_dim);
   const uint32_t row_bytes = (uint32_t)(a.feat_dim * sizeof(T));
-  const uint32_t ed_bytes = (uint32_t)(a.edata_dim * (OP == kGatSrc ? sizeof(float2) : OP == kUMulW ? sizeof(float) : sizeof(T)));
+  const uint32_t ed_bytes = (uint32_t)(a.edata_dim * (OP == kUMulW ? sizeof(float) : sizeof(T)));
   const bool none = a.none && *a.none != 0;
   // rows and edges fit 31 bits, and so does everything that counts them
   const int num_rows = (int)a.num_rows;
@@ -317,19 +303,14 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   const T *lane_in = nullptr, *lane_ed[VPL];
   uint32_t off[VPL];      // bytes from the lane's first slice; lanes past the row's last slice read their first one again
   int head[VPL], col[VPL], at_block = 0;
-  unsigned lead = 0;      // slices that open a head
   auto set_block = [&](int c0) {
     at_block = c0;
-    lead = 0;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       col[i] = (c0 + vl + i * lpe < nvec ? c0 + vl + i * lpe : i == 0 ? nvec - 1 : c0 + vl < nvec ? c0 + vl : nvec - 1) * VE;
-      head[i] = (OP == kGatSrc || OP == kUMulW || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
-      if (OP == kGatSrc && head[i] * per == col[i]) lead |= 1u << i;
+      head[i] = (OP == kUMulW || (per > 1 && per % VE == 0)) ? col[i] / per : -1;
       off[i] = (uint32_t)((col[i] - col[0]) * (int)sizeof(T));
-      lane_ed[i] = OP == kGatSrc  ? (const T*)((const float2*)a.edata + head[i])
-                   : OP == kUMulW ? (const T*)((const float*)a.edata + head[i])
-                                  : a.edata + (head[i] >= 0 ? head[i] : col[i]);
+      lane_ed[i] = OP == kUMulW ? (const T*)((const float*)a.edata + head[i]) : a.edata + (head[i] >= 0 ? head[i] : col[i]);
     }
     lane_in = a.in + col[0];
   };
@@ -347,12 +328,8 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     for (int c0 = 0; c0 < nvec && !skip; c0 += lpe * VPL) {
       if (c0 != at_block) set_block(c0);
       Acc<VE> acc[VPL];
-      float acc2[VPL];
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        acc2[i] = 0.f;
-        acc[i].zero();
-      }
+      for (int i = 0; i < VPL; ++i) acc[i].zero();
       uint32_t my_src = src, my_e = eid;
 #pragma unroll 1
       for (int k0 = b; k0 < e; k0 += LPR) {
@@ -373,7 +350,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
 #pragma unroll
           for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int i = 0; i < VPL; ++i) slice_add<T, VE, OP>(acc[i], acc2[i], v[u][i], per, head[i]);
+            for (int i = 0; i < VPL; ++i) slice_add<T, VE, OP>(acc[i], v[u][i], per, head[i]);
         }
         if (full < cnt) {
           EdgeSlice<T, VE, OP> v[U][VPL];
@@ -390,7 +367,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
           for (int u = 0; u < U; ++u)
             if (j + u * EP < cnt) {
 #pragma unroll
-              for (int i = 0; i < VPL; ++i) slice_add<T, VE, OP>(acc[i], acc2[i], v[u][i], per, head[i]);
+              for (int i = 0; i < VPL; ++i) slice_add<T, VE, OP>(acc[i], v[u][i], per, head[i]);
             }
         }
       }
@@ -402,18 +379,13 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
 #pragma unroll 1
         for (int o = lpe; o < LPR; o <<= 1)
 #pragma unroll
-          for (int i = 0; i < VPL; ++i) {
-            acc[i].join(GMASK, o);
-            if constexpr (OP == kGatSrc) acc2[i] += __shfl_xor_sync(GMASK, acc2[i], o);
-          }
+          for (int i = 0; i < VPL; ++i) acc[i].join(GMASK, o);
         if (EPI == 0) {
 #pragma unroll
           for (int i = 0; i < VPL; ++i) {
             if (c0 + vl + i * lpe >= nvec) continue;
 #pragma unroll
             for (int t = 0; t < VE; ++t) __stcg(p + col[i] + t, acc[i].get(t));
-            if constexpr (OP == kGatSrc)
-              if (lead >> i & 1u) __stcg(p + a.feat_dim + head[i], acc2[i]);
           }
         }
         if (c0 + lpe * VPL < nvec) continue;
@@ -432,7 +404,6 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
           if (cc != at_block) set_block(cc);
 #pragma unroll
           for (int i = 0; i < VPL; ++i) {
-            acc2[i] = 0.f;
             acc[i].zero();
 #pragma unroll 1
             for (int q = EPI; q < parts; q += EP) {
@@ -440,16 +411,15 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
 #pragma unroll
               for (int t = 0; t < VE; t += 2)
                 acc[i].p[t / 2] = f2_add(acc[i].p[t / 2], f2_pack(__ldcg(src_part + col[i] + t), VE > 1 ? __ldcg(src_part + col[i] + (VE > 1 ? t + 1 : t)) : 0.f));
-              if constexpr (OP == kGatSrc) acc2[i] += __ldcg(src_part + a.feat_dim + head[i]);
             }
           }
           c0 = cc;
           if (cc + lpe * VPL < nvec) {
-            rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, lead, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
+            rows_write<T, VE, VPL>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
           }
         }
       }
-      rows_write<T, VE, VPL, OP>(a, acc, acc2, col, head, lead, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
+      rows_write<T, VE, VPL>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
     }
     if (items) {
       it += warps;
@@ -513,8 +483,7 @@ int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
       case kCopyE: return launch_rows_ve<T, kCopyE>(a, s);                                \
       case kUMulE: return launch_rows_ve<T, kUMulE>(a, s);                                \
       case kUAddE: return launch_rows_ve<T, kUAddE>(a, s);                                \
-      case kUMulW: return launch_rows_ve<T, kUMulW>(a, s);                                \
-      default: return launch_rows_ve<T, kGatSrc>(a, s);                                   \
+      default: return launch_rows_ve<T, kUMulW>(a, s);                                   \
     }                                                                                                    \
   }
 
