@@ -148,15 +148,32 @@ k_concat_ids(const int64_t* __restrict__ a, int64_t na, const int64_t* __restric
 // ranking and emitting walk level 1 only (range/1024 words), so the cost of a
 // call follows the number of ids, not the width of the range. Both levels are
 // all-zero between calls: the pass that emits the ids also clears what it read.
-// Three launches: mark, emit (count, ordered ranks, clear), inverse.
+// Three launches: mark (and count per tile of words), emit (ranks, ids, clear), inverse.
 constexpr int kUniqBlock = 256;
+constexpr int kSharedTiles = 1024;    // up to here a block adds its counts up in shared memory first
+constexpr int kGroup = 256;           // tiles whose counts are added up once more where there are many
+constexpr int kManyTiles = 8192;      // (every block of the emit reads the counts before its own: 32 a thread here)
+
+// Ids set per tile; all zero between calls.
+struct TileCounts {
+  int32_t* tile;       // [tiles]
+  int32_t* group;      // [tiles / kGroup + 1], used above kManyTiles
+  int tiles;
+  int shift;           // level-0 word -> tile
+};
 
 // Runs of lanes whose ids share a word (the virtual ids of a sampled hop come in runs of its fanout) are joined
 // first: one atomic a run. 23 000 ids in runs of 25: 24 us with one an id.
 __global__ void __launch_bounds__(256)
 k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
             int64_t lo, int64_t hi, uint32_t* __restrict__ l0, uint32_t* __restrict__ l1,
-            int32_t* status) {
+            TileCounts counts, int32_t* status) {
+  __shared__ int here[kSharedTiles];
+  const bool shared = counts.tiles <= kSharedTiles;
+  if (shared) {
+    for (int t = threadIdx.x; t < counts.tiles; t += 256) here[t] = 0;
+    __syncthreads();
+  }
   n = effective_n(n, n_dev);
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -183,32 +200,53 @@ k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restric
     if ((*(volatile uint32_t*)(l0 + w) & bits) == bits) continue;
     const uint32_t old = atomicOr(l0 + w, bits);
     if (old == 0) atomicOr(l1 + (w >> 5), 1u << (w & 31));  // first bit of this word
+    const int set = __popc(bits & ~old);
+    if (!set) continue;
+    const uint32_t tile = w >> counts.shift;
+    if (shared) {
+      atomicAdd(here + tile, set);
+    } else {
+      atomicAdd(counts.tile + tile, set);
+      if (counts.tiles > kManyTiles) atomicAdd(counts.group + tile / kGroup, set);
+    }
   }
   if (flags) atomicOr(status, flags);
+  if (!shared) return;
+  __syncthreads();
+  for (int t = threadIdx.x; t < counts.tiles; t += 256)
+    if (here[t]) atomicAdd(counts.tile + t, here[t]);
 }
 
-// Counting, ranking, emitting and clearing in one launch. A block has 8 * `per_warp` consecutive level-1 words, dealt to
-// its warps in turn (a dense run of ids in a wide range is a few neighbouring words), a lane to each. A lane with few level-0 words below its own (a wide range) walks them itself, all loads in flight;
-// where there are many the warp's lanes take the 32 words together, one level-1 word after another (a dense range: a
-// million ids below one thousand level-1 words; one thread to a word walked 1024 ids alone, 75 to 430 us).
-// The blocks' counts are chained by the look-back of common.cuh. info[w] = (rank of the word's first id, its bits).
+// Ranking, emitting and clearing in one launch. A block (a tile) has 8 * `per_warp` consecutive level-1 words, dealt to
+// its warps in turn (a dense run of ids in a wide range is a few neighbouring words), a lane to each. A lane with few
+// level-0 words below its own (a wide range) walks them itself, all loads in flight; where there are many the warp's lanes
+// take the 32 words together, one level-1 word after another (a dense range: a million ids below one thousand level-1
+// words; one thread to a word walked 1024 ids alone, 75 to 430 us). The first rank of a tile is the sum of the counts
+// the marks left for the tiles before it, read beside the tile's own words: with counts found here and chained by a
+// decoupled look-back the launch took 11 us instead of 4 (67 584 ids of 111 million), most of it waiting in
+// turn for the ticket, the look-back's windows and the closing counter.
+// info[w] = (rank of the word's first id, its bits).
 constexpr int kOwnWords = 8, kOwnIds = 32;
 
 __global__ void __launch_bounds__(kUniqBlock)
 k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords1, int per_warp,
-            int64_t lo, ScanCtrl* ctrl, uint64_t* tile_state, uint2* __restrict__ info,
-            int64_t* __restrict__ out_unique, int64_t* __restrict__ out_num_unique, int32_t* status) {
+            int64_t lo, const TileCounts tc, uint2* __restrict__ info, int64_t* __restrict__ out_unique,
+            int64_t* __restrict__ out_num_unique) {
   constexpr int W = kUniqBlock / 32;
   __shared__ uint32_t counts[kUniqBlock];
-  __shared__ int scratch[33];
-  __shared__ uint32_t s_tile, s_epoch, s_before;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) tile_ticket(ctrl, &s_tile, &s_epoch);
-  __syncthreads();
-  const uint32_t tile = s_tile;
+  __shared__ int scratch[33], s_before[W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = blockIdx.x;
   const int64_t first = (int64_t)tile * W * per_warp + warp;      // word of lane k: first + k * W
   const int64_t w1 = first + lane * W;
   const uint32_t mine = lane < per_warp && w1 < nwords1 ? l1[w1] : 0u;
+  int before = 0;
+  {
+    const bool many = tc.tiles > kManyTiles;
+    const int start = many ? tile / kGroup * kGroup : 0;
+    for (int t = start + threadIdx.x; t < tile; t += kUniqBlock) before += tc.tile[t];
+    if (many)
+      for (int t = threadIdx.x; t < tile / kGroup; t += kUniqBlock) before += tc.group[t];
+  }
   uint32_t word[kOwnWords], count = 0;
   const bool few = __popc(mine) <= kOwnWords;
   uint32_t rest = mine;
@@ -227,18 +265,19 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
   }
   // ranks inside the block, in the order of the words
   counts[lane * W + warp] = count;
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) s_before[warp] = before;
   __syncthreads();
   int total_i;
   const int before_word = block_exclusive_scan((int)counts[threadIdx.x], scratch, &total_i);
   counts[threadIdx.x] = (uint32_t)before_word;
   const uint32_t total = (uint32_t)total_i;
-  if (warp == 0) {
-    const uint32_t b = tile_lookback(tile_state, tile, s_epoch, total, status, APT_FLAG_TABLE_FULL);
-    if (lane == 0) s_before = b;
-  }
   __syncthreads();
-  if (tile == gridDim.x - 1 && threadIdx.x == 0) *out_num_unique = (int64_t)s_before + total;
-  int64_t at = (int64_t)s_before + counts[lane * W + warp];      // rank of the first id below this lane's word
+  int64_t base = 0;
+#pragma unroll
+  for (int q = 0; q < W; ++q) base += s_before[q];
+  if (tile == (int)gridDim.x - 1 && threadIdx.x == 0) *out_num_unique = base + total;
+  int64_t at = base + counts[lane * W + warp];      // rank of the first id below this lane's word
   const bool own = few && count <= kOwnIds;
   for (unsigned m = __ballot_sync(0xffffffffu, !own); m; m &= m - 1) {
     const int k = __ffs(m) - 1;
@@ -277,16 +316,18 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
     }
   }
   if (lane < per_warp && mine) l1[w1] = 0u;
-  __syncthreads();
-  if (threadIdx.x == 0) tile_done(ctrl, s_epoch);
 }
 
 __global__ void __launch_bounds__(256)
 k_uniq_inverse(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
-               int64_t lo, int64_t hi, const uint2* __restrict__ info, int64_t* __restrict__ out_inverse) {
+               int64_t lo, int64_t hi, const uint2* __restrict__ info, TileCounts counts, int64_t* __restrict__ out_inverse) {
   n = effective_n(n, n_dev);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t t = i; t < counts.tiles; t += stride) {      // the emit is done with them
+    counts.tile[t] = 0;
+    if (t % kGroup == 0) counts.group[t / kGroup] = 0;
+  }
   for (; i < n; i += stride) {
     const int64_t v = ids[i];
     if (v < lo || v >= hi) {
@@ -360,11 +401,9 @@ struct UniqWs {
   uint32_t* l0;           // [nwords0] one bit per id
   uint32_t* l1;           // [nwords1] one bit per level-0 word
   uint2* info;            // [nwords1 * 32] rank of the word's first id and its bits, of the words the call set
-  ScanCtrl* ctrl;         // [1]        control words of the ordered emit, zero once
-  uint64_t* tile_state;   // [nblocks]  its tile states, tagged by call
-  int64_t nwords0, nwords1;
+  TileCounts counts;
+  int64_t nwords1;
   int nblocks, per_warp;
-  size_t bitmap_bytes;    // l0 + l1: the part that has to be zero between calls
 };
 static size_t uniq_layout(int64_t range, char* base, UniqWs* ws) {
   const int64_t nwords0 = ceil_div(range > 0 ? range : 1, 32);
@@ -376,20 +415,20 @@ static size_t uniq_layout(int64_t range, char* base, UniqWs* ws) {
   const size_t b0 = align_up((size_t)nwords1 * 32 * 4, 256);  // level 0, padded to whole level-1 words
   const size_t b1 = align_up((size_t)nwords1 * 4, 256);
   const size_t b2 = align_up((size_t)nwords1 * 32 * 8, 256);
-  const size_t b3 = align_up(sizeof(ScanCtrl) + (size_t)nblocks * 8, 256);
+  const size_t b3 = align_up((size_t)nblocks * 4, 256);
+  const size_t b4 = align_up((size_t)(nblocks / kGroup + 1) * 4, 256);
   if (ws) {
     ws->l0 = (uint32_t*)base;
     ws->l1 = (uint32_t*)(base + b0);
     ws->info = (uint2*)(base + b0 + b1);
-    ws->ctrl = (ScanCtrl*)(base + b0 + b1 + b2);
-    ws->tile_state = (uint64_t*)(base + b0 + b1 + b2 + sizeof(ScanCtrl));
-    ws->nwords0 = nwords0;
+    int shift = 5 + 3;      // 32 level-0 words to a level-1 word, 8 warps
+    for (int k = per_warp; k > 1; k >>= 1) ++shift;
+    ws->counts = TileCounts{(int32_t*)(base + b0 + b1 + b2), (int32_t*)(base + b0 + b1 + b2 + b3), nblocks, shift};
     ws->nwords1 = nwords1;
     ws->nblocks = nblocks;
     ws->per_warp = per_warp;
-    ws->bitmap_bytes = b0 + b1;
   }
-  return b0 + b1 + b2 + b3;
+  return b0 + b1 + b2 + b3 + b4;
 }
 }  // namespace apt
 
@@ -433,10 +472,10 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
   }
   ProfScope prof("unique_sorted", s);
   const int g = wave_grid(ceil_div(num_ids, 256), 8);
-  APT_LAUNCH(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, status_word);
-  APT_LAUNCH(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.ctrl, ws.tile_state,
-             ws.info, out_unique, out_num_unique, status_word);
-  APT_LAUNCH(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.info, out_inverse);
+  APT_LAUNCH(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, ws.counts, status_word);
+  APT_LAUNCH(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.counts, ws.info,
+             out_unique, out_num_unique);
+  APT_LAUNCH(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.info, ws.counts, out_inverse);
   return APT_OK;
 }
 

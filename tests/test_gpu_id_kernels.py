@@ -5,10 +5,11 @@ import numpy as np
 import pytest
 import torch
 
-from apt_b200 import ops
+from apt_b200 import DPNeighborSampler, ops
 from apt_b200._lib import check, lib
 from oracle import oracle as orc
-from tests.gpu_util import dev, host
+from tests.gpu_util import dev, host, install_graph
+from tests.helpers import small_graph
 
 pytestmark = pytest.mark.gpu
 I64 = np.int64
@@ -81,3 +82,32 @@ def test_relabel_beyond_the_tiles_of_one_size():
     first = torch.full((3_000_000,), n, device="cuda").scatter_reduce_(0, items, torch.arange(n, device="cuda"), "amin")
     order = first[uniq]                                # positions of first occurrence: rising, and all of them
     assert bool((order[1:] > order[:-1]).all()) and uniq.numel() == int((first < n).sum())
+
+
+@pytest.mark.parametrize("id_range", [1 << 18, (1 << 18) + 1, 1 << 28, (1 << 28) + 1, (1 << 31) + 1])
+def test_unique_around_the_numbers_of_tiles(id_range):
+    # one tile and two; the most whose counts a block adds up first and one more; enough for sums over groups of tiles
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    edge = torch.tensor([0, id_range - 1, id_range - 1, id_range // 2], device="cuda")
+    ids = torch.cat([torch.randint(0, id_range, (20_000,), device="cuda", generator=gen), edge])
+    for _ in range(2):
+        uniq, inv = ops.unique_sorted(ids, 0, id_range)
+        want, want_inv = torch.unique(ids, return_inverse=True)
+        assert torch.equal(uniq, want) and torch.equal(inv, want_inv)
+    for key in [k for k in ops.STATE._ws if k[0].startswith("unique")]:
+        del ops.STATE._ws[key]                         # the widest bitmap is 0.8 GB
+
+
+@pytest.mark.parametrize("fanout", [1, 7, 8, 9, 15, 16, 31, 32, 33])
+def test_sample_and_relabel_around_the_group_widths(fanout):
+    # with a lane left over the seed enters the table beside its draws, without one behind them
+    n, indptr, indices = small_graph(scale=12, edge_factor=8)
+    install_graph(indptr, indices)
+    seeds = dev(np.random.default_rng(fanout).permutation(n)[:1003].astype(I64))
+    ops.set_sampling(key=5, call_id=9)
+    _, neighbours = ops.local_sample_one_layer(seeds, fanout)
+    uniq, rel = ops.relabel_csc(seeds, neighbours)
+    got = DPNeighborSampler(0, [fanout], prefetch_features=False)
+    ops.set_sampling(key=5, call_id=9)
+    input_nodes, _, blocks = got.sample(None, seeds)[:3]
+    assert torch.equal(input_nodes, uniq) and torch.equal(blocks[0].coo_row, rel)
