@@ -44,7 +44,7 @@ size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) 
   const size_t o_part = take((size_t)part_floats * 4);
   if (ws) {
     ws->result = (int64_t*)(base + o_words);
-    ws->probe = (uint32_t*)(base + o_words + 8);
+    ws->probe = (unsigned long long*)(base + o_words + 8);
     ws->num_items = (int32_t*)(base + o_words + 16);
     ws->num_slots = (int32_t*)(base + o_words + 20);
     ws->num_parts = (int32_t*)(base + o_words + 24);
@@ -70,12 +70,28 @@ __device__ __forceinline__ int64_t out_row(const int64_t* coo, const int64_t* oo
   return ooff[nseg > 1 ? seg_of(coo, nseg, e) : 0] + col[e];
 }
 
-// `agg` (two words) is zero before and after; `result` may be mapped host memory.
+// One 64-bit word collects the blocks' answers: blocks done, and how many of them saw each of the three. The add that
+// counts a block also returns what the others saw, so the last block has the answer without a fence or a second
+// read (fence, counter and read in turn: 5.6 -> 4.5 us for 10 240 edges). `agg` is zero before and after; `result` may
+// be mapped host memory.
+__device__ __forceinline__ unsigned long long probe_votes(uint32_t bits) {
+  return 1ull | (bits & kNotGrouped ? 1ull << 16 : 0ull) | (bits & kNotFixed ? 1ull << 32 : 0ull) |
+         (bits & kHasLong ? 1ull << 48 : 0ull);
+}
+
 __global__ void __launch_bounds__(256)
-k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, uint32_t* agg, volatile int64_t* result,
+k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned long long* agg, volatile int64_t* result,
              int64_t sequence) {
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   __shared__ uint32_t s_bits;
+  constexpr int K = 4;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, c[K];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int k = 0; k < K; ++k) c[k] = e0 + k * stride < E ? col[e0 + k * stride] : 0;
+  };
+  fetch();     // on its way while the offsets are
   for (int t = threadIdx.x; t <= st.nseg; t += blockDim.x) {
     coo[t] = st.coo_off[t];
     ooff[t] = st.out_off[t];
@@ -86,38 +102,41 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, uint32_t* 
   // the one fanout that fits the sizes
   const uint32_t f = rows > 0 && E % rows == 0 ? (uint32_t)(E / rows) : 0u;
   uint32_t bits = f ? 0u : kNotFixed;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-#pragma unroll 4
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
-    const int64_t d = out_row(coo, ooff, st.nseg, col, e);
-    if (f && d == (int64_t)((uint32_t)e / f)) continue;
-    bits |= kNotFixed;
-    const int64_t prev = e > 0 ? out_row(coo, ooff, st.nseg, col, e - 1) : (int64_t)-1;
-    if (d < prev || d < 0 || d >= rows) bits |= kNotGrouped;
-    // the next edge may match the fanout and then does not look back itself
-    if (e + 1 < E && out_row(coo, ooff, st.nseg, col, e + 1) < d) bits |= kNotGrouped;
-    // a run of kLongRun edges covers two neighbouring multiples of half that length
-    if (e % (kLongRun / 2) == 0 && e >= kLongRun / 2 && out_row(coo, ooff, st.nseg, col, e - kLongRun / 2) == d)
-      bits |= kHasLong;
+  while (e0 < E) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int64_t e = e0 + k * stride;
+      if (e >= E) break;
+      const int64_t d = ooff[st.nseg > 1 ? seg_of(coo, st.nseg, e) : 0] + c[k];
+      if (f && d == (int64_t)((uint32_t)e / f)) continue;
+      bits |= kNotFixed;
+      const int64_t prev = e > 0 ? out_row(coo, ooff, st.nseg, col, e - 1) : (int64_t)-1;
+      if (d < prev || d < 0 || d >= rows) bits |= kNotGrouped;
+      // the next edge may match the fanout and then does not look back itself
+      if (e + 1 < E && out_row(coo, ooff, st.nseg, col, e + 1) < d) bits |= kNotGrouped;
+      // a run of kLongRun edges covers two neighbouring multiples of half that length
+      if (e % (kLongRun / 2) == 0 && e >= kLongRun / 2 && out_row(coo, ooff, st.nseg, col, e - kLongRun / 2) == d)
+        bits |= kHasLong;
+    }
+    e0 += K * stride;
+    if (e0 < E) fetch();
   }
   bits = __reduce_or_sync(0xffffffffu, bits);
   if ((threadIdx.x & 31) == 0 && bits) atomicOr(&s_bits, bits);
   __syncthreads();
   if (threadIdx.x != 0) return;
-  uint32_t all = s_bits;
+  unsigned long long all = probe_votes(s_bits);
   if (gridDim.x > 1) {
-    if (all) atomicOr(agg, all);
-    __threadfence();
-    if (atomicAdd(agg + 1, 1u) != gridDim.x - 1) return;
-    all = atomicExch(agg, 0u);
-    atomicExch(agg + 1, 0u);
+    all += atomicAdd(agg, all);
+    if ((all & 0xffffu) != gridDim.x) return;
+    atomicExch(agg, 0ull);
   }
+  const bool fixed = !(all >> 32 & 0xffffu), grouped = !(all >> 16 & 0xffffu), has_long = (all >> 48) != 0;
   const bool fits = rows >= 0 && rows < 0x7fffffff;
-  *result = probe_pack(fits ? rows : 0, !fits ? 3 : !(all & kNotFixed) ? kFixed : (all & (kNotGrouped | kHasLong)) ? kOrder : kRanges,
-                       sequence);
+  *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, sequence);
 }
 
-static int launch_probe(const int64_t* col, int64_t E, SegTable st, uint32_t* agg, int64_t* result, int64_t sequence,
+static int launch_probe(const int64_t* col, int64_t E, SegTable st, unsigned long long* agg, int64_t* result, int64_t sequence,
                         cudaStream_t s) {
   // a thousand edges a block and one wave at most: small blocks of edges are looked over by one thread block
   const int grid = wave_grid(ceil_div(E, 1024), 4, 1);
@@ -133,7 +152,7 @@ struct ProbeSlots {
   std::mutex mu;
   std::condition_variable cv;
   int64_t* host = nullptr;            // mapped: 8 words a slot
-  uint32_t* agg[64] = {};             // device words of each device: 2 a slot, zero between calls
+  unsigned long long* agg[64] = {};   // device words of each device: one a slot, zero between calls
   uint64_t taken = 0;
   int64_t sequence = 0;
 };
@@ -156,7 +175,7 @@ static int take_slot(int dev, int* slot, int64_t* sequence) {
       cudaFree(p);
       APT_CUDA(e);
     }
-    g_probe.agg[dev] = (uint32_t*)p;
+    g_probe.agg[dev] = (unsigned long long*)p;
   }
   g_probe.cv.wait(lk, [] { return g_probe.taken != ~0ull; });
   *slot = __builtin_ctzll(~g_probe.taken);
@@ -514,7 +533,7 @@ extern "C" int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges, const i
   if (rc != APT_OK) return rc;
   int64_t* host = g_probe.host + slot * 8;
   SegTable st{coo_offset, nullptr, output_offset, num_segments};
-  rc = launch_probe(coo_col, num_edges, st, g_probe.agg[dev] + slot * 2, host, sequence, s);
+  rc = launch_probe(coo_col, num_edges, st, g_probe.agg[dev] + slot, host, sequence, s);
   if (rc == APT_OK) rc = wait_for(host, sequence, s);
   if (rc == APT_OK) {
     const int64_t w = *(volatile int64_t*)host, rows = probe_rows(w);

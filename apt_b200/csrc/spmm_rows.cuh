@@ -62,7 +62,7 @@ __host__ __device__ inline int64_t probe_sequence(int64_t w) { return (int64_t)(
 struct SpmmWs {
   // zero when a call starts that groups edges or asks the device for the mode
   int64_t* result;      // [1] the probe's answer (probe_pack)
-  uint32_t* probe;      // [2] what the blocks of the probe found, blocks done
+  unsigned long long* probe;   // what the blocks of the probe found (probe_votes)
   int32_t* num_items;   // [1]
   int32_t* num_slots;   // [1] slots of order[] given out
   int32_t* num_parts;   // [1] rows of part[] given out

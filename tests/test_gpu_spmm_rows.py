@@ -116,6 +116,25 @@ def test_probe_and_enqueue_only_form(name):
     _close(out, want, magnitude, torch.float32)
 
 
+@pytest.mark.parametrize("E", [2, 5, 1023, 1024, 1025, 700_001])
+def test_probe_finds_one_edge_out_of_order(E):
+    # one thread block and several, the last of them ragged; more edges than one wave of blocks holds at a time
+    gen = torch.Generator(device="cuda").manual_seed(E)
+    n_out, n_in = E // 2 + 1, 50
+    row = torch.randint(0, n_in, (E,), device="cuda", generator=gen)
+    x = torch.arange(n_in, dtype=torch.float32, device="cuda")[:, None].contiguous()      # small integers: exact sums
+    off = [torch.tensor([0, n], device="cuda") for n in (E, n_in, n_out)]
+    for at in {1, E // 2, E - 1}:
+        col = torch.arange(E, device="cuda") // 2
+        col[at] = (col[at] + n_out // 2 + 1) % n_out
+        want = torch.zeros(n_out, 1, device="cuda").index_add_(0, col, x[row])
+        got = (ctypes.c_int64 * 3)()
+        check(lib.apt_spmm_probe(col.data_ptr(), E, off[0].data_ptr(), off[2].data_ptr(), 1, got, None))
+        rising = bool((col[1:] >= col[:-1]).all())
+        assert got[0] == n_out and got[1] == (1 if rising else 2)
+        assert torch.equal(ops.spmm_copy_u_sum(row, col, x, *off), want)
+
+
 def test_probe_is_refused_inside_a_capture():
     one = torch.zeros(1, dtype=torch.int64, device="cuda")
     off = torch.tensor([0, 1], device="cuda")
