@@ -77,26 +77,30 @@ sample_replace_kernel(const int64_t* __restrict__ seeds, int64_t num_seeds,
                       const int64_t* __restrict__ num_seeds_dev, int fanout, CscView g, uint32_t k0,
                       uint32_t k1, uint32_t call_id, const int64_t* __restrict__ call_base_dev,
                       int64_t* __restrict__ out, int32_t* status, SampleInsert ins) {
+  const int64_t groups_per_block = blockDim.x / G;
+  int64_t j = (int64_t)blockIdx.x * groups_per_block + threadIdx.x / G;
+  // the first id is on its way before the count is known: `seeds` holds the upper bound
+  int64_t v = j < num_seeds ? seeds[j] : 0;
   num_seeds = effective_n(num_seeds, num_seeds_dev);
   if (call_base_dev) call_id += (uint32_t)*call_base_dev;
   const uint32_t cap = INSERT ? relabel_capacity(num_seeds + num_seeds * fanout) : 0u;
   const int sub = threadIdx.x % G;
-  const int64_t groups_per_block = blockDim.x / G;
-  int64_t j = (int64_t)blockIdx.x * groups_per_block + threadIdx.x / G;
   const int64_t stride = (int64_t)gridDim.x * groups_per_block;
   int flags = 0;
   for (; j < num_seeds; j += stride) {
-    const int64_t v = seeds[j];
-    int64_t* orow = out ? out + j * fanout : nullptr;
     const int64_t* nbr = nullptr;
     const int64_t deg = csc_row(g, v, &nbr, &flags);
-    if (INSERT && sub == 0) ins.slot_of[j] = table_insert(ins.slots, cap, v, (uint32_t)j, &flags);
-    for (int i = sub; i < fanout; i += G) {
-      int64_t u = v;   // a seed that is no node, or has no in-neighbour, fills its row with itself
-      if (deg > 0) u = nbr[mod_deg(draw_word((uint64_t)j, (uint32_t)i, call_id, k0, k1), deg)];
-      if (orow) orow[i] = u;
+    const int64_t here = v;
+    if (j + stride < num_seeds) v = seeds[j + stride];     // the next seed's id travels while this one's row is drawn
+    int64_t* orow = out ? out + j * fanout : nullptr;
+    // with INSERT the seed is one item more, behind its draws: its way through the table runs beside theirs
+    for (int i = sub; i < fanout + (INSERT ? 1 : 0); i += G) {
+      int64_t u = here;   // a seed that is no node, or has no in-neighbour, fills its row with itself
+      const bool drawn = !INSERT || i < fanout;
+      if (drawn && deg > 0) u = nbr[mod_deg(draw_word((uint64_t)j, (uint32_t)i, call_id, k0, k1), deg)];
+      if (drawn && orow) orow[i] = u;
       if (INSERT) {
-        const int64_t item = num_seeds + j * fanout + i;
+        const int64_t item = drawn ? num_seeds + j * fanout + i : j;
         ins.slot_of[item] = table_insert(ins.slots, cap, u, (uint32_t)item, &flags);
       }
     }
