@@ -72,10 +72,21 @@ ProfScope::~ProfScope() {
 __global__ void __launch_bounds__(256)
 k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __restrict__ sequence_dev, int64_t sequence,
                 volatile int64_t* host) {
+  if (threadIdx.x == 0 && sequence_dev) sequence = *sequence_dev;
   for (int t = threadIdx.x; t < count; t += blockDim.x) host[t] = words[t];
   __threadfence_system();
   __syncthreads();
-  if (threadIdx.x == 0) host[count] = sequence_dev ? *sequence_dev : sequence;
+  if (threadIdx.x == 0) host[count] = sequence;
+}
+
+// What a replay starts from, in one kernel in front of it: the seeds, the call-id base and the sequence number of its
+// counts. (A copy of the seeds, and one of the two words inside the graph, cost a launch more on the host and put a copy
+// engine between kernels twice.)
+__global__ void __launch_bounds__(256)
+k_stage_replay(const int64_t* __restrict__ seeds, int64_t n, int64_t* __restrict__ seeds_buf, int64_t call_base, int64_t sequence,
+               int64_t* __restrict__ words) {
+  for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < n; t += (int64_t)gridDim.x * 256) seeds_buf[t] = seeds[t];
+  if (blockIdx.x == 0 && threadIdx.x < 2) words[threadIdx.x] = threadIdx.x ? sequence : call_base;
 }
 
 }  // namespace apt
@@ -87,6 +98,15 @@ int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_d
   using namespace apt;
   APT_CHECK_ARG(words && host && count >= 0 && count <= 4096, "apt_publish_words: bad argument");
   APT_LAUNCH(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, sequence_dev, sequence, host);
+  return APT_OK;
+}
+
+int apt_stage_replay(const int64_t* seeds, int64_t num_seeds, int64_t* seeds_buf, int64_t call_base, int64_t sequence,
+                     int64_t* words, void* stream) {
+  using namespace apt;
+  APT_CHECK_ARG(num_seeds >= 0 && words && (num_seeds == 0 || (seeds && seeds_buf)), "apt_stage_replay: bad argument");
+  APT_LAUNCH(k_stage_replay, wave_grid(ceil_div(num_seeds, 256), 4, 1), 256, 0, (cudaStream_t)stream, seeds, num_seeds,
+             seeds_buf, call_base, sequence, words);
   return APT_OK;
 }
 

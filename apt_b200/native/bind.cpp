@@ -235,10 +235,10 @@ int64_t read_words(const Tensor& words, const Tensor& host, int64_t sequence) {
 // One captured mini-batch: launches its graph, waits for its counts, orders other streams behind its last kernel.
 class Plan {
  public:
-  // host_in: page-locked [call-id base, sequence]; host_words: page-locked, count words and the sequence; own_stream:
+  // replay_in: device words [call-id base, sequence]; host_words: page-locked, count words and the sequence; own_stream:
   // 0 for the caller's current stream.
-  Plan(uintptr_t exec, Tensor seeds_buf, Tensor host_in, Tensor host_words, uintptr_t own_stream)
-      : exec_((cudaGraphExec_t)exec), seeds_buf_(std::move(seeds_buf)), host_in_(std::move(host_in)),
+  Plan(uintptr_t exec, Tensor seeds_buf, Tensor replay_in, Tensor host_words, uintptr_t own_stream)
+      : exec_((cudaGraphExec_t)exec), seeds_buf_(std::move(seeds_buf)), replay_in_(std::move(replay_in)),
         host_words_(std::move(host_words)), own_((cudaStream_t)own_stream) {
     cuda_ok(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming), "cudaEventCreate");
     cuda_ok(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming), "cudaEventCreate");
@@ -254,9 +254,9 @@ class Plan {
       fail("sampler plan: seeds must be contiguous int64 of the plan's length");
     const cudaStream_t cur = (cudaStream_t)stream();
     const cudaStream_t s = own_ ? own_ : cur;
-    int64_t* const in = host_in_.mutable_data_ptr<int64_t>();
-    in[0] = call_base;
-    in[1] = ++sequence_;
+    const int64_t* from = seeds.const_data_ptr<int64_t>();
+    int64_t* const to = seeds_buf_.mutable_data_ptr<int64_t>();
+    int64_t count = from != to ? seeds.numel() : 0;
     py::gil_scoped_release nogil;
     if (own_) {
       // behind everything the caller's stream holds so far: the seeds' producer, the consumer of the last results
@@ -265,9 +265,11 @@ class Plan {
     } else if (stream_ && stream_ != cur) {
       cuda_ok(cudaStreamWaitEvent(cur, done_, 0), "cudaStreamWaitEvent");
     }
-    if (seeds.numel() && seeds.const_data_ptr() != seeds_buf_.const_data_ptr())
-      cuda_ok(cudaMemcpyAsync(seeds_buf_.mutable_data_ptr(), seeds.const_data_ptr(), seeds.nbytes(), cudaMemcpyDefault, s),
-              "cudaMemcpyAsync");
+    if (count && !(seeds.is_cuda() && seeds.device() == seeds_buf_.device())) {
+      cuda_ok(cudaMemcpyAsync(to, from, count * 8, cudaMemcpyDefault, s), "cudaMemcpyAsync");
+      count = 0;
+    }
+    check(apt_stage_replay(from, count, to, call_base, ++sequence_, replay_in_.mutable_data_ptr<int64_t>(), s));
     cuda_ok(cudaGraphLaunch(exec_, s), "cudaGraphLaunch");
     cuda_ok(cudaEventRecord(done_, s), "cudaEventRecord");
     seeds_ = seeds;       // the copy reads it when the stream gets there
@@ -293,13 +295,17 @@ class Plan {
 
  private:
   cudaGraphExec_t exec_;
-  Tensor seeds_buf_, host_in_, host_words_, seeds_;
+  Tensor seeds_buf_, replay_in_, host_words_, seeds_;
   cudaStream_t own_, stream_ = nullptr;
   cudaEvent_t done_, ready_;
   int64_t sequence_ = 0;
 };
 
-Tensor front(const Tensor& t, int64_t n) { return t.narrow(0, 0, n); }
+// The first n rows. Below autograd: a sampler's buffers have no history to carry on, and the view costs half as much.
+Tensor front(const Tensor& t, int64_t n) {
+  at::AutoDispatchBelowADInplaceOrView below;
+  return t.narrow(0, 0, n);
+}
 
 Tensor offsets_cpu(const int64_t* v, int64_t n, bool sum) {
   Tensor t = at::empty({n}, at::TensorOptions().dtype(at::kLong));

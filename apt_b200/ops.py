@@ -9,6 +9,7 @@ every operator except ``cpu_load_subtensor`` requires CUDA tensors.
 State lives in one process-wide object like the reference's ``NPCState``
 (src/state.h:32-63): one process drives one GPU.
 """
+import contextlib
 import ctypes
 import os
 import threading
@@ -126,7 +127,7 @@ class NPCState:
         self.profiling = False
         self.exchange = None  # set by apt_b200.exchange.make_exchange at init
         self.exchange_generation = 0
-        self._side_stream = None
+        self._side_streams = {}
         self.shuffle_backend = os.environ.get("APT_SHUFFLE_BACKEND", "p2p")
         self.p2p_region_bytes = int(os.environ.get("APT_P2P_REGION_MB", "256")) << 20
         # inboxes of the lanes beside the first carry the samplers' id exchanges only
@@ -154,11 +155,25 @@ class NPCState:
             self._ws[key] = buf
         return buf
 
-    def side_stream(self) -> torch.cuda.Stream:
-        """A second stream of this device for work that runs beside the main chain of a mini-batch."""
-        if self._side_stream is None or self._side_stream.device != self.device():
-            self._side_stream = torch.cuda.Stream(device=self.device())
-        return self._side_stream
+    def side_stream(self, k: int = 0) -> torch.cuda.Stream:
+        """Further streams of this device for work that runs beside the main chain of a mini-batch."""
+        key = (k, torch.cuda.current_device())
+        stream = self._side_streams.get(key)
+        if stream is None:
+            stream = self._side_streams[key] = torch.cuda.Stream(device=self.device())
+        return stream
+
+    @contextlib.contextmanager
+    def beside(self, k: int):
+        """Enqueues the block's work on side stream k, behind what the current stream holds so far. The current stream
+        waits for it with `join(k)`."""
+        side = self.side_stream(k)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            yield
+
+    def join(self, k: int):
+        torch.cuda.current_stream().wait_stream(self.side_stream(k))
 
     def lane_stream(self, lane: int) -> torch.cuda.Stream:
         """The one stream on which work that uses lane `lane`'s scratch is enqueued: everything on

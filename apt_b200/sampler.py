@@ -12,6 +12,7 @@ buffers are narrowed to their real lengths. The results are identical to
 calling the operators one by one (``chained=False``), which reads a count
 after every relabelling like the reference does (src/cuda/relabel.cu:119).
 """
+import contextlib
 import itertools
 import os
 import queue
@@ -97,10 +98,7 @@ class _Plan:
         self.graph = None
         self.generation = -1
         self.keepalive = None
-        # the batch's own copy of the word block (a sequence number behind it) and the pinned words a replay
-        # reads: the call-id base and that number
-        self.host_words = None
-        self.host_in = None
+        self.host_words = None  # the batch's own copy of the word block, a sequence number behind it
         self.handle = None      # _native.Plan: launches the graph, waits for the counts, orders streams
         # the lane whose scratch the plan was built on; with more than one lane, the lane's stream
         self.lane = 0
@@ -199,7 +197,6 @@ class _GraphReplay:
         plan.seeds_buf = torch.empty(seeds.numel(), dtype=torch.int64, device=dev)
         plan.seeds_buf.copy_(seeds)
         plan.host_words = torch.zeros(st.NUM_WORDS + 1, dtype=torch.int64).pin_memory()
-        plan.host_in = torch.zeros(2, dtype=torch.int64).pin_memory()
         if on_lanes:
             # lane 0 stays with the caller: its exchange context also carries the feature shuffles
             # the model side runs on its own stream while the samplers' lanes are in flight
@@ -224,14 +221,10 @@ class _GraphReplay:
                                             ops._ptr(plan.host_words), ops._stream()))
 
             with torch.cuda.graph(plan.graph):
-                # the call-id base and the sequence number are read from the plan's pinned words when the replay
-                # runs (apt_memcpy_async and not Tensor.copy_: the latter also records an event for the
-                # pinned block, which may not be queried once it was recorded in a capture)
-                check(lib.apt_memcpy_async(ops._ptr(replay_in), ops._ptr(plan.host_in), 16, ops._stream()))
                 plan.bufs = self._enqueue(plan.seeds_buf, base_dev, publish)
                 if not published:
                     publish()
-            plan.handle = _native.Plan(plan.graph.raw_cuda_graph_exec(), plan.seeds_buf, plan.host_in, plan.host_words,
+            plan.handle = _native.Plan(plan.graph.raw_cuda_graph_exec(), plan.seeds_buf, replay_in, plan.host_words,
                                        plan.stream.cuda_stream if on_lanes else 0)
             plan.keepalive = [v for k, v in st._ws.items() if k[2] == plan.lane]
         finally:
@@ -717,7 +710,11 @@ class SPVirtualSampler(_GraphReplay):
         uf_word = st.word(self._UF)
         # the unique virtual nodes come from the ids as they stand (owner x num_dst + destination); with
         # destinations every neighbour's id is shifted by world_size x num_dst afterwards, which keeps the order
-        unique_frontier, _ = ops._unique_enqueue(sorted_vir, n_word, 0, ws * max(s_max, 1), uf_word, "unique_vir")
+        # the three uniques of this sampler are small and wait mostly for memory: where they do not need one another's
+        # results they run side by side
+        beside = ws == 1 and not with_dst and not st.profiling
+        with st.beside(0) if beside else contextlib.nullcontext():
+            unique_frontier, _ = ops._unique_enqueue(sorted_vir, n_word, 0, ws * max(s_max, 1), uf_word, "unique_vir")
         dst_sorted = None
         if with_dst:
             dst_sorted, dst_pos, _, _ = ops._bucket(cur, cur_n)
@@ -766,8 +763,12 @@ class SPVirtualSampler(_GraphReplay):
         check(lib.apt_sp_unpack_frontier(ops._ptr(recv), recv.numel(), ops._ptr(total), n_total,
                                          ops._ptr(vir_src), ops._ptr(ori_src), ops._stream()))
         lo, hi = ops._owned_range()
+        with st.beside(1) if beside else contextlib.nullcontext():
+            unique_dst, a_dst = ops._unique_enqueue(vir_src, total, 0, ws * ops.SP_BASE, st.word(self._UD), "unique_vdst")
         unique_src, a_src = ops._unique_enqueue(ori_src, total, lo, hi, st.word(self._US), "unique_sp_src")
-        unique_dst, a_dst = ops._unique_enqueue(vir_src, total, 0, ws * ops.SP_BASE, st.word(self._UD), "unique_vdst")
+        if beside:
+            st.join(0)
+            st.join(1)
         if ws == 1 and not with_dst:
             arange_dst = unique_frontier        # owner 0: a virtual node is its destination's index
         else:

@@ -79,6 +79,10 @@ int apt_memcpy_async(void* dst, const void* src, size_t nbytes, void* stream);
 int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_dev,
                       int64_t sequence, int64_t* host, void* stream);
 int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream);
+/* The inputs of a captured mini-batch in one kernel: copies the seeds (device memory) into the buffer
+ * the graph reads and writes words[0] = call_base, words[1] = sequence. */
+int apt_stage_replay(const int64_t* seeds, int64_t num_seeds, int64_t* seeds_buf, int64_t call_base,
+                     int64_t sequence, int64_t* words, void* stream);
 
 /* Optional per-kernel timing. When enabled, every launch of a tagged kernel
  * is bracketed by CUDA events on its own stream; apt_profile_read
