@@ -226,7 +226,9 @@ k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restric
 // decoupled look-back the launch took 11 us instead of 4 (67 584 ids of 111 million), most of it waiting in
 // turn for the ticket, the look-back's windows and the closing counter.
 // info[w] = (rank of the word's first id, its bits).
-constexpr int kOwnWords = 8, kOwnIds = 32;
+// 16 words: 50 000 ids of 8.2 million, six to a level-1 word on average, take 5.0 us; with 8 a sixth of the lanes went the
+// warp's way and it took 11.7.
+constexpr int kOwnWords = 16, kOwnIds = 32;
 
 __global__ void __launch_bounds__(kUniqBlock)
 k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords1, int per_warp,
