@@ -146,6 +146,47 @@ Tensor rows_scatter(const Tensor& inp, const Tensor& index, int64_t num_out_rows
   return out;
 }
 
+// ---------------------------------------------------------------------------- feature shuffles of a world of one
+void cuda_ok(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) fail(std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+// What travels nowhere still changes its order.
+Tensor feat_shuffle_local(const Tensor& inputs, const Tensor& recv_offset, const Tensor& permutation, int64_t feat_dim, bool fwd) {
+  if (dtype_code(inputs.scalar_type()) < 0) fail("feat_shuffle: unsupported dtype " + dtype_name(inputs));
+  const Tensor in = cuda(inputs, "inputs");
+  ids(permutation, "permutation");
+  const int64_t rows = in.numel() / feat_dim;
+  const Tensor flat = in.dim() == 2 && in.size(1) == feat_dim ? in : in.view({rows, feat_dim});
+  return fwd ? rows_gather(flat, permutation) : rows_scatter(flat, permutation, recv_offset[-1].item<int64_t>());
+}
+
+// The parts' sizes are checked and each part is one copy.
+Tensor sp_feat_shuffle_local(const Tensor& inputs, const Tensor& send_sizes, const Tensor& recv_sizes, int64_t total_recv,
+                             int64_t expand, bool with_dst) {
+  if (dtype_code(inputs.scalar_type()) < 0) fail("sp_feat_shuffle: unsupported dtype " + dtype_name(inputs));
+  const Tensor in = cuda(inputs, "inputs");
+  const int64_t rows = in.numel() / expand;
+  if (rows * expand != in.numel()) fail("sp_feat_shuffle: the input is no whole number of rows");
+  Tensor out = at::empty({total_recv, expand}, in.options());
+  const Tensor send = send_sizes.to(at::kCPU, at::kLong).contiguous(), recv = recv_sizes.to(at::kCPU, at::kLong).contiguous();
+  const auto sum = [](const Tensor& t, int64_t first, int64_t step) {
+    const int64_t* const v = t.const_data_ptr<int64_t>();
+    int64_t total = 0;
+    for (int64_t k = first; k < t.numel(); k += step) total += v[k];
+    return total;
+  };
+  const int64_t step = with_dst ? 3 : 2;
+  const int64_t sent_dst = with_dst ? sum(send, 0, step) : 0, got_dst = with_dst ? sum(recv, 0, step) : 0;
+  const int64_t sent = sum(send, step - 1, step), got = sum(recv, step - 1, step);
+  if (sent_dst + sent != rows || got_dst + got != total_recv) fail("sp_feat_shuffle: sizes do not add up to the rows given");
+  if (sent_dst != got_dst || sent != got) fail("sp_feat_shuffle: one rank receives what it sends");
+  if (in.nbytes())      // the parts follow one another on both sides
+    cuda_ok(cudaMemcpyAsync(out.mutable_data_ptr(), in.const_data_ptr(), in.nbytes(), cudaMemcpyDeviceToDevice,
+                            (cudaStream_t)stream()), "cudaMemcpyAsync");
+  return out;
+}
+
 // ---------------------------------------------------------------------------------------- attention block
 struct GatShape {
   int code;
@@ -217,10 +258,6 @@ struct GatFunction : public torch::autograd::Function<GatFunction> {
 };
 
 // ------------------------------------------------------------------------------------------------ samplers
-void cuda_ok(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) fail(std::string(what) + ": " + cudaGetErrorString(e));
-}
-
 // Copies the word block to the host (one kernel, polled for) and returns its status flags.
 int64_t read_words(const Tensor& words, const Tensor& host, int64_t sequence) {
   const int count = (int)words.numel();
@@ -350,6 +387,27 @@ py::tuple np_finish(const Tensor& host, const Tensor& seeds, const py::list& lay
   return py::make_tuple(py::make_tuple(input, seeds, blocks, front(perm, frontier), recv, sent, front(inverse, received)), row_view);
 }
 
+// Source-split, attention: the words hold what np_finish's do, with the unique neighbours and the input nodes in slots of
+// their own.
+py::tuple snp_gat_finish(const Tensor& host, const Tensor& seeds, const py::list& layers, const py::tuple& outer, const Tensor& perm,
+                         const Tensor& input_nodes, const OptTensor& rows, int64_t world_size, int64_t unique_slot,
+                         int64_t input_slot, const py::object& block) {
+  const int64_t* const w = host.const_data_ptr<int64_t>();
+  auto [blocks, num_dst] = narrow_blocks(w, seeds.numel(), layers, block);
+  const int64_t num_in = w[input_slot];
+  if (num_in > input_nodes.numel())
+    fail("chained SNP-GAT sampler: more ids received than the buffer sized from this rank's own batch holds; use chained=False "
+         "for batches that differ this much between the ranks");
+  py::list last;
+  last.append(outer);
+  blocks.insert(0, narrow_blocks(w, num_dst, last, block).first[0]);
+  py::object row_view = py::none();
+  if (rows) row_view = py::cast(front(*rows, num_in));
+  return py::make_tuple(py::make_tuple(front(input_nodes, num_in), seeds, blocks, front(perm, w[unique_slot]),
+                                       offsets_cpu(w + 16, world_size, true), offsets_cpu(w + 64, world_size, false)),
+                        row_view);
+}
+
 // Data-parallel: every hop sampled and relabelled on this GPU, the rows of the input nodes gathered behind the counts. One
 // read at the end; all results are tensors of their own.
 py::tuple dp_sample(const Tensor& seeds, const std::vector<int64_t>& fanouts, const OptTensor& adj_pos_map, int64_t num_nodes,
@@ -445,6 +503,15 @@ PYBIND11_MODULE(_native, m) {
     return out;
   });
   m.def("np_finish", &np_finish);
+  m.def("snp_gat_finish", &snp_gat_finish);
+  m.def("pick", [](const Tensor& host, const std::vector<int64_t>& at) {
+    std::vector<int64_t> out;
+    for (const int64_t k : at) out.push_back(host.const_data_ptr<int64_t>()[k]);
+    return out;
+  });
+  m.def("sizes", [](const std::vector<int64_t>& v) { return offsets_cpu(v.data(), (int64_t)v.size(), false); });
+  m.def("feat_shuffle_local", &feat_shuffle_local);
+  m.def("sp_feat_shuffle_local", &sp_feat_shuffle_local);
   m.def("dp_sample", &dp_sample);
   m.def("gather", &gather);
   m.def("rows_gather", &rows_gather);

@@ -249,14 +249,16 @@ def _exchange():
     than the first get a context of their own on first use (a collective step: every rank has to
     reach it, which holds when the ranks run the same sampler), since the flags of one context
     order its exchanges as one sequence."""
-    from .exchange import P2PExchange, make_exchange
-
     if STATE.exchange is None:
+        from .exchange import make_exchange
+
         STATE.exchange = make_exchange(STATE)
     if STATE.lane == 0 or STATE.exchange.name != "p2p" or STATE.world_size == 1:
         return STATE.exchange
     ex = STATE._lane_exchange.get(STATE.lane)
     if ex is None or ex.generation != STATE.exchange_generation:
+        from .exchange import P2PExchange
+
         ex = P2PExchange(STATE, min(STATE.p2p_region_bytes, STATE.p2p_lane_region_bytes))
         ex.generation = STATE.exchange_generation
         STATE._lane_exchange[STATE.lane] = ex
@@ -691,6 +693,9 @@ def sp_feat_shuffle(inputs: torch.Tensor, send_sizes: torch.Tensor, recv_sizes: 
     """SPFeatShuffle, src/feat_shuffle.cc:32-52: rows of `expand` elements; per
     peer q the last of its k sizes (partial sums per virtual node), preceded,
     with destinations, by sizes[3 q] destination rows for every q."""
+    ex = _exchange()
+    if ex.name == "local":
+        return _native.sp_feat_shuffle_local(inputs, send_sizes, recv_sizes, int(total_recv_size), int(expand), bool(shuffle_with_dst))
     if inputs.dtype not in _DTYPE_CODE:
         raise RuntimeError(f"sp_feat_shuffle: unsupported dtype {inputs.dtype}")
     inputs = _need_cuda(inputs, "inputs", dtype=None)
@@ -699,7 +704,6 @@ def sp_feat_shuffle(inputs: torch.Tensor, send_sizes: torch.Tensor, recv_sizes: 
     flat = inputs.view(rows, expand)
     out = torch.empty((int(total_recv_size), expand), dtype=inputs.dtype, device=inputs.device)
     send_sizes, recv_sizes = send_sizes.cpu(), recv_sizes.cpu()
-    ex = _exchange()
     if shuffle_with_dst:
         sd, rd = send_sizes[0::3], recv_sizes[0::3]
         sv, rv = send_sizes[2::3], recv_sizes[2::3]
@@ -823,13 +827,15 @@ def feat_shuffle(inputs: torch.Tensor, send_offset: torch.Tensor, recv_offset: t
     cumulative row counts. fwd: rows travel to the ranks that asked for them
     and come out in the asker's original seed order (``buf[permutation]``);
     bwd: rows are scattered by permutation and travel back."""
+    ex = _exchange()
+    if ex.name == "local":
+        return _native.feat_shuffle_local(inputs, recv_offset, permutation, int(feat_dim), bool(fwd_flag))
     if inputs.dtype not in _DTYPE_CODE:
         raise RuntimeError(f"feat_shuffle: unsupported dtype {inputs.dtype}")
     inputs = _need_cuda(inputs, "inputs", dtype=None)
     permutation = _need_cuda(permutation, "permutation")
     rows_in = inputs.numel() // int(feat_dim)
-    return _exchange().exchange_rows(inputs.view(rows_in, int(feat_dim)), send_offset, recv_offset,
-                                        permutation, bool(fwd_flag))
+    return ex.exchange_rows(inputs.view(rows_in, int(feat_dim)), send_offset, recv_offset, permutation, bool(fwd_flag))
 
 
 def alltoall(input: torch.Tensor, output: torch.Tensor, send_offset: torch.Tensor, recv_offset: torch.Tensor,

@@ -13,7 +13,6 @@ calling the operators one by one (``chained=False``), which reads a count
 after every relabelling like the reference does (src/cuda/relabel.cu:119).
 """
 import contextlib
-import itertools
 import os
 import queue
 import threading
@@ -586,23 +585,13 @@ class SPGATSampler(_GraphReplay):
 
     def _finish(self, seeds, b, host=None, plan=None):
         st = ops.STATE
-        ws = st.world_size
         if host is None:
             host = st.read_words()
-        blocks, n_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
-        h = host.tolist()
-        n_u, n_in = h[self._U], h[self._IN]
-        if n_in > b["input_nodes"].numel():
-            raise RuntimeError("chained SNP-GAT sampler: more ids received than the buffer sized from this rank's own "
-                               "batch holds; use chained=False for batches that differ this much between the ranks")
-        outer, _ = _native.narrow_blocks(host, n_dst, [b["outer"]], Block)
-        blocks.insert(0, outer[0])
-        send_offset = torch.tensor(list(itertools.accumulate(h[16:16 + ws])), dtype=torch.int64)
-        recv_offset = torch.tensor(h[64:64 + ws], dtype=torch.int64)
-        input_nodes = b["input_nodes"][:n_in]
-        if b["rows"] is not None:
-            st.prefetched = (input_nodes, b["rows"][:n_in], plan)
-        return input_nodes, seeds, blocks, b["perm"][:n_u], send_offset, recv_offset
+        got, rows = _native.snp_gat_finish(host, seeds, b["layers"], b["outer"], b["perm"], b["input_nodes"], b["rows"],
+                                           st.world_size, self._U, self._IN, Block)
+        if rows is not None:
+            st.prefetched = (got[0], rows, plan)
+        return got
 
     def sample(self, graph, seeds: torch.Tensor):
         if self.chained and ops._exchange().name in ("local", "p2p"):
@@ -801,21 +790,20 @@ class SPVirtualSampler(_GraphReplay):
         if host is None:
             host = st.read_words()
         blocks, num_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
-        h = host.tolist()
-        n_uf, n_us, n_ud, n_in = h[self._UF], h[self._US], h[self._UD], h[self._IN]
+        n_uf, n_us, n_ud, n_in, n_recv, n_rdst = _native.pick(host, [self._UF, self._US, self._UD, self._IN, 16 + ws,
+                                                                     self._RDST + ws])
         with_dst = self.shuffle_with_dst
         k = 3 if with_dst else 2
         if ws == 1 and not with_dst:
             send, recv = [num_dst * f, n_uf], [num_dst * f, n_uf]
             n_recv = num_dst * f
         else:
-            send, recv = h[self._SEND:self._SEND + k * ws], h[self._RECV:self._RECV + k * ws]
-            n_recv = h[16 + ws]
-        n_rdst = h[self._RDST + ws] if with_dst else 0
+            send = _native.pick(host, list(range(self._SEND, self._SEND + k * ws)))
+            recv = _native.pick(host, list(range(self._RECV, self._RECV + k * ws)))
         if n_recv > b["vir_src"].numel() or (with_dst and n_rdst > b["recv_dst"].numel()):
             raise RuntimeError("chained SNP sampler: more ids received than the buffer sized from this rank's own "
                                "batch holds; use chained=False for batches that differ this much between the ranks")
-        send_sizes_cpu, recv_sizes_cpu = torch.tensor(send, dtype=torch.int64), torch.tensor(recv, dtype=torch.int64)
+        send_sizes_cpu, recv_sizes_cpu = _native.sizes(send), _native.sizes(recv)
         n_nbr = num_dst * f
         (unique_frontier, unique_src, arange_dst, a_src, a_dst, input_nodes, neighbors, sorted_all, packed, vir_src, ori_src,
          unique_dst) = _native.fronts(
