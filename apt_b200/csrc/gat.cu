@@ -20,15 +20,19 @@
 //                   for four edges instead of 4 log2(lph).
 //   k_gat_scores    backward: t, grad_s and grad_er, one thread per destination and head; grad_el is added up in fp32 with
 //                   one reduction per edge and head (the heads of an edge are neighbours: one sector)
-//   row kernel      grad_ft: the weighted sum of the forward with the sides swapped, behind one counting sort by source.
-//                   With grad_el as a second accumulator of the same walk it held two blocks an SM instead of three:
-//                   150 us against 116, and the scores had to be written out for it.
+//   row kernel      grad_ft: the weighted sum of the forward with the sides swapped. With grad_el as a second accumulator
+//                   of the same walk it held two blocks an SM instead of three: 150 us against 116, and the scores had to
+//                   be written out for it.
+//   The counting sort by source that grad_ft needs rides along: k_gat_dots has every edge's source in a register and waits
+//                   for rows most of the time, so it also counts the edges (the add returns an edge's place in its
+//                   row); k_dst_slots gives the rows their places; k_gat_scores writes the order. As launches of
+//                   their own the first and the last pass took 23 + 16 us.
 //   k_gat_source    grad_el in T
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 28, then 45 us of sort and 158 us
-// for both source-side sums, where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
+// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 48 + 116 + 5 us,
+// where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 
 #include <algorithm>
@@ -133,7 +137,7 @@ template <typename T, int VE>
 __global__ void __launch_bounds__(256, 3)
 k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ grad_out, int num_heads, int head_dim,
            int64_t num_dst_, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ dots, int lph,
-           int hpp) {
+           int hpp, uint32_t num_src, int32_t* __restrict__ src_count /* null: not wanted */, uint32_t* __restrict__ rank) {
   if (*none != 0) return;
   const int lane = threadIdx.x & 31, G = gridDim.x * 8, num_dst = (int)num_dst_;
   const int lpe = lph * hpp, ep = 32 / lpe;
@@ -173,6 +177,9 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
         const int cnt = min(32, r.y - base);
         uint32_t my_src = src;
         if (base != r.x) my_src = (uint32_t)row[min(base + lane, r.y - 1)];
+        const bool ranked = src_count && h0 == 0 && lane < cnt;
+        uint32_t place = kNoRank;
+        if (ranked && my_src < num_src) place = (uint32_t)atomicAdd(src_count + my_src, 1);
 #pragma unroll 1
         for (int j0 = 0; j0 < cnt; j0 += ep * 4) {
           float dt[4] = {0.f, 0.f, 0.f, 0.f};
@@ -215,6 +222,7 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
             }
           }
         }
+        if (ranked) rank[base + lane] = place;
       }
     }
     r = nr, src = nsrc, nr = nnr;
@@ -227,8 +235,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
              int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
-             float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, T* __restrict__ attn,
-             T* __restrict__ grad_score, T* __restrict__ grad_er) {
+             float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort,
+             T* __restrict__ attn, T* __restrict__ grad_score, T* __restrict__ grad_er) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const bool empty = *none != 0;
   if (empty)   // no edge belongs to anybody
@@ -266,6 +274,13 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
       }
     }
     grad_er[i] = Elem<T>::from_f(ger);
+    if (!sums) continue;
+    // the destination's edges to their places in the order by source, a share for every head's thread
+#pragma unroll 4
+    for (int e = r.x + (int)h; e < r.y; e += num_heads) {
+      const uint32_t place = sort.rank[e];
+      if (place != kNoRank) sort.order[(uint32_t)sort.range[row[e]].x + place] = make_uint2(d, (uint32_t)e);
+    }
   }
 }
 
@@ -362,7 +377,7 @@ static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* 
 }
 
 template <typename T, int VE>
-static int launch_dots(const GatProblem& q, const GatEdges& g, float* dots, cudaStream_t s) {
+static int launch_dots(const GatProblem& q, const GatEdges& g, int64_t num_src, float* dots, const SpmmWs& sort, cudaStream_t s) {
   static int occupancy[64] = {};
   int per_sm = 0;
   const int rc = blocks_per_sm(k_gat_dots<T, VE>, 256, occupancy, &per_sm);
@@ -370,39 +385,39 @@ static int launch_dots(const GatProblem& q, const GatEdges& g, float* dots, cuda
   const int lph = pow2_ge(q.Dh / VE), hpp = pow2_ge(q.H, 32 / lph);
   const int64_t want = ceil_div(q.num_dst, 8), wave = (int64_t)kNumSMs * per_sm;
   APT_LAUNCH((k_gat_dots<T, VE>), (int)(want < wave ? want : wave), 256, 0, s, q.row, (const T*)q.ft, (const T*)q.grad_out, q.H,
-             (int)q.Dh, q.num_dst, g.range, g.none, dots, lph, hpp);
+             (int)q.Dh, q.num_dst, g.range, g.none, dots, lph, hpp, (uint32_t)num_src, sort.cnt, sort.rank);
   return APT_OK;
 }
 
-// The edge part of the backward: weights are there already.
+// The edge part of the backward: weights are there already. With `sums` also the source side's sums of the score gradients
+// and the order of its edges (`sort`, all of it zero where it has to be).
 template <typename T>
-static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num_src, float* dots, float* sums, void* attn,
-                             void* grad_score, void* grad_er, cudaStream_t s) {
+static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num_src, float* dots, float* sums, const SpmmWs& sort,
+                             int long_edges, void* attn, void* grad_score, void* grad_er, cudaStream_t s) {
   ProfScope prof("gat_bwd_rows", s);
   int rc;
   switch (slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T)) {
-    case 16: rc = launch_dots<T, 16 / sizeof(T)>(q, g, dots, s); break;
-    case 8: rc = launch_dots<T, 8 / sizeof(T)>(q, g, dots, s); break;
-    case 4: rc = launch_dots<T, 4 / sizeof(T)>(q, g, dots, s); break;
-    default: rc = launch_dots<T, 1>(q, g, dots, s); break;
+    case 16: rc = launch_dots<T, 16 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
+    case 8: rc = launch_dots<T, 8 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
+    case 4: rc = launch_dots<T, 4 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
+    default: rc = launch_dots<T, 1>(q, g, num_src, dots, sort, s); break;
   }
+  if (rc == APT_OK && sums) rc = launch_slots(num_src, sort, kOrder, long_edges, (int)(q.H * q.Dh), s);
   if (rc != APT_OK) return rc;
   APT_LAUNCH(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-             q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, (T*)attn, (T*)grad_score, (T*)grad_er);
+             q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, sort, (T*)attn, (T*)grad_score, (T*)grad_er);
   return APT_OK;
 }
 
 template <typename T>
 static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, char* workspace, int64_t num_src, void* grad_ft,
                         void* grad_el, void* grad_er, cudaStream_t s) {
-  APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
-  int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, nullptr, nullptr, grad_er, s);
-  if (rc != APT_OK) return rc;
   const int64_t dim = q.H * q.Dh;
   const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
   const RowSplit split = row_split(dim, ve, q.E, num_src);
   const SegTable st{nullptr, nullptr, nullptr, 1};
-  rc = launch_group(q.col, q.row, q.E, st, num_src, ws.sort, kOrder, split.long_edges, (int)dim, s);
+  APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
+  int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, ws.sort, split.long_edges, nullptr, nullptr, grad_er, s);
   if (rc != APT_OK) return rc;
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, st, num_src, q.E, ws.sort,
                      (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr};
@@ -558,7 +573,7 @@ extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const in
 #define APT_RUN(T)                                                                                         \
   do {                                                                                                     \
     if ((rc = gat_weights<T>(q, g, nullptr, s)) != APT_OK) return rc;                                      \
-    return gat_edge_backward<T>(q, g, 0, dots, nullptr, out_attn, out_grad_score, out_grad_er, s);                     \
+    return gat_edge_backward<T>(q, g, 0, dots, nullptr, SpmmWs{}, 0, out_attn, out_grad_score, out_grad_er, s);    \
   } while (0)
   switch (dtype) {
     case APT_F32: APT_RUN(float);

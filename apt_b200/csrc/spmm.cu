@@ -245,8 +245,6 @@ k_edge_ranges(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t n
 
 // Counting sort by output row. The add that counts an edge also returns its place inside its row, so the pass
 // that writes the order needs no second round of atomics (1.01 M edges: 25 + 28 us with one in both passes).
-constexpr uint32_t kNoRank = 0xffffffffu;
-
 __global__ void __launch_bounds__(256)
 k_dst_rank(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_rows, SpmmWs ws, int mode) {
   if (resolve_mode(mode, ws) != kOrder) return;
@@ -351,12 +349,18 @@ k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int
   }
 }
 
-int launch_group(const int64_t* row, const int64_t* col, int64_t num_edges, SegTable st, int64_t num_rows,
+int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s) {
+  APT_LAUNCH(k_dst_slots, (int)ceil_div(num_rows, 256 * kScanRows), 256, 0, s, num_rows, ws, mode, long_edges, part_stride);
+  return APT_OK;
+}
+
+static int launch_group(const int64_t* row, const int64_t* col, int64_t num_edges, SegTable st, int64_t num_rows,
                  const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s) {
   ProfScope prof("spmm_group", s);
   const int ge = wave_grid(ceil_div(num_edges, 256 * 4), 8, 1);
   APT_LAUNCH(k_dst_rank, ge, 256, 0, s, col, num_edges, st, num_rows, ws, mode);
-  APT_LAUNCH(k_dst_slots, (int)ceil_div(num_rows, 256 * kScanRows), 256, 0, s, num_rows, ws, mode, long_edges, part_stride);
+  const int rc = launch_slots(num_rows, ws, mode, long_edges, part_stride, s);
+  if (rc != APT_OK) return rc;
   APT_LAUNCH(k_dst_fill, ge, 256, 0, s, row, col, num_edges, st, ws, mode);
   return APT_OK;
 }

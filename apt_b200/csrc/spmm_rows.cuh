@@ -78,6 +78,8 @@ struct SpmmWs {
   int64_t max_items, max_parts, part_floats;
 };
 
+constexpr uint32_t kNoRank = 0xffffffffu;     // rank of an edge that belongs to no row
+
 __device__ __forceinline__ int seg_of(const int64_t* coo, int nseg, int64_t e) {
   int k = 0;
   while (k + 1 < nseg && coo[k + 1] <= e) ++k;
@@ -489,8 +491,7 @@ int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
 
 // ---- shared by spmm.cu and gat.cu -----------------------------------------------------
 size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws);
-// Groups the edges by output row into ws.order / ws.range / ws.items (three launches behind one memset).
-int launch_group(const int64_t* row, const int64_t* col, int64_t num_edges, SegTable st, int64_t num_rows,
-                 const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s);
+// Counted edges (ws.cnt) to places: ws.range, and the items of long rows.
+int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s);
 
 }  // namespace apt
