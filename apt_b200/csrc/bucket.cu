@@ -11,6 +11,7 @@ k_bucket_count(const int64_t* __restrict__ ids, int64_t n, const int64_t* __rest
                const int64_t* __restrict__ min_vids, OwnerParams p,
                int32_t* __restrict__ hist /* [world_size][nblocks] */,
                int nblocks) {
+  wait_for_previous();
   __shared__ int64_t mv[kMaxRanks + 1];
   __shared__ int cnt[kMaxRanks];
   n = effective_n(n, n_dev);
@@ -39,6 +40,7 @@ k_bucket_scatter(const int64_t* __restrict__ ids, int64_t n, const int64_t* __re
                  const int32_t* __restrict__ hist, int nblocks,
                  int64_t* __restrict__ sorted, int64_t* __restrict__ perm,
                  int64_t* __restrict__ sizes, int64_t* __restrict__ offsets) {
+  wait_for_previous();
   __shared__ int64_t mv[kMaxRanks + 1];
   __shared__ int warp_cnt[kBucketBlock / 32][kMaxRanks];
   __shared__ int row_total[kMaxRanks], row_before[kMaxRanks], bucket_base[kMaxRanks];
@@ -112,6 +114,7 @@ k_bucket_scatter(const int64_t* __restrict__ ids, int64_t n, const int64_t* __re
 __global__ void __launch_bounds__(256)
 k_bucket_one_rank(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev, int64_t* __restrict__ sorted,
                   int64_t* __restrict__ perm, int64_t* __restrict__ sizes, int64_t* __restrict__ offsets) {
+  wait_for_previous();
   n = effective_n(n, n_dev);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -128,6 +131,7 @@ __global__ void __launch_bounds__(256)
 k_concat_ids(const int64_t* __restrict__ a, int64_t na, const int64_t* __restrict__ na_dev,
              const int64_t* __restrict__ b, int64_t nb, const int64_t* __restrict__ nb_dev,
              int64_t* __restrict__ out, int64_t* __restrict__ out_count, const RowTables tables, int32_t* status) {
+  wait_for_previous();
   na = effective_n(na, na_dev);
   nb = effective_n(nb, nb_dev);
   const int64_t total = na + nb;
@@ -168,6 +172,7 @@ __global__ void __launch_bounds__(256)
 k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
             int64_t lo, int64_t hi, uint32_t* __restrict__ l0, uint32_t* __restrict__ l1,
             TileCounts counts, int32_t* status) {
+  wait_for_previous();
   __shared__ int here[kSharedTiles];
   const bool shared = counts.tiles <= kSharedTiles;
   if (shared) {
@@ -234,6 +239,7 @@ __global__ void __launch_bounds__(kUniqBlock)
 k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords1, int per_warp,
             int64_t lo, const TileCounts tc, uint2* __restrict__ info, int64_t* __restrict__ out_unique,
             int64_t* __restrict__ out_num_unique) {
+  wait_for_previous();
   constexpr int W = kUniqBlock / 32;
   __shared__ uint32_t counts[kUniqBlock];
   __shared__ int scratch[33], s_before[W];
@@ -323,6 +329,7 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
 __global__ void __launch_bounds__(256)
 k_uniq_inverse(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
                int64_t lo, int64_t hi, const uint2* __restrict__ info, TileCounts counts, int64_t* __restrict__ out_inverse) {
+  wait_for_previous();
   n = effective_n(n, n_dev);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -388,12 +395,12 @@ extern "C" int apt_bucket_by_owner(const int64_t* ids, int64_t num_ids,
   int32_t* hist = (int32_t*)workspace;
   ProfScope prof("bucket", s);
   if (world_size == 1) {
-    APT_LAUNCH(k_bucket_one_rank, wave_grid(ceil_div(num_ids, 256), 8, 1), 256, 0, s, ids, num_ids, num_ids_dev, out_sorted,
+    APT_FOLLOW(k_bucket_one_rank, wave_grid(ceil_div(num_ids, 256), 8, 1), 256, 0, s, ids, num_ids, num_ids_dev, out_sorted,
                out_perm, out_bucket_sizes, out_bucket_offsets);
     return APT_OK;
   }
-  APT_LAUNCH(k_bucket_count, nblocks, kBucketBlock, 0, s, ids, num_ids, num_ids_dev, min_vids, p, hist, nblocks);
-  APT_LAUNCH(k_bucket_scatter, nblocks, kBucketBlock, 0, s, ids, num_ids, num_ids_dev, min_vids, p, hist,
+  APT_FOLLOW(k_bucket_count, nblocks, kBucketBlock, 0, s, ids, num_ids, num_ids_dev, min_vids, p, hist, nblocks);
+  APT_FOLLOW(k_bucket_scatter, nblocks, kBucketBlock, 0, s, ids, num_ids, num_ids_dev, min_vids, p, hist,
              nblocks, out_sorted, out_perm, out_bucket_sizes, out_bucket_offsets);
   return APT_OK;
 }
@@ -474,10 +481,10 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
   }
   ProfScope prof("unique_sorted", s);
   const int g = wave_grid(ceil_div(num_ids, 256), 8);
-  APT_LAUNCH(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, ws.counts, status_word);
-  APT_LAUNCH(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.counts, ws.info,
+  APT_FOLLOW(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, ws.counts, status_word);
+  APT_FOLLOW(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.counts, ws.info,
              out_unique, out_num_unique);
-  APT_LAUNCH(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.info, ws.counts, out_inverse);
+  APT_FOLLOW(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.info, ws.counts, out_inverse);
   return APT_OK;
 }
 
@@ -500,7 +507,7 @@ extern "C" int apt_concat_row_ids(const int64_t* a, int64_t num_a, const int64_t
     if (out_count_dev) APT_CUDA(cudaMemsetAsync(out_count_dev, 0, sizeof(int64_t), s));
     return APT_OK;
   }
-  APT_LAUNCH(k_concat_ids, wave_grid(ceil_div(num_a + num_b, 256), 8, 1), 256, 0, s, a, num_a, num_a_dev, b, num_b,
+  APT_FOLLOW(k_concat_ids, wave_grid(ceil_div(num_a + num_b, 256), 8, 1), 256, 0, s, a, num_a, num_a_dev, b, num_b,
              num_b_dev, out, out_count_dev, RowTables{feat_pos_map, feat_num_nodes, num_dev_rows, num_uva_rows}, status_word);
   return APT_OK;
 }

@@ -55,6 +55,30 @@ struct ProfScope {
     }                                                                         \
   } while (0)
 
+// The same for a kernel that opens with wait_for_previous(): its launch overlaps the end of the kernel before it on the
+// stream (programmatic dependent launch), in captured graphs too. Chains of kernels of a few microseconds are what this
+// framework's mini-batches consist of: three edge operators over 61 310 edges 38 -> 31 us, a data-parallel batch 151 -> 135.
+#define APT_FOLLOW(kernel, grid_, block_, smem_, stream_, ...)                \
+  do {                                                                        \
+    cudaLaunchAttribute attr__ = {};                                          \
+    attr__.id = cudaLaunchAttributeProgrammaticStreamSerialization;           \
+    attr__.val.programmaticStreamSerializationAllowed = 1;                    \
+    cudaLaunchConfig_t cfg__ = {};                                            \
+    cfg__.gridDim = dim3((unsigned)(grid_));                                  \
+    cfg__.blockDim = dim3((unsigned)(block_));                                \
+    cfg__.dynamicSmemBytes = (smem_);                                         \
+    cfg__.stream = (stream_);                                                 \
+    cfg__.attrs = &attr__;                                                    \
+    cfg__.numAttrs = 1;                                                       \
+    const cudaError_t e__ = cudaLaunchKernelEx(&cfg__, kernel, __VA_ARGS__);  \
+    apt::count_launch();                                                      \
+    if (e__ != cudaSuccess) {                                                 \
+      apt::set_error("%s:%d launch of %s -> %s", __FILE__, __LINE__, #kernel, \
+                     cudaGetErrorString(e__));                                \
+      return APT_ERR_CUDA;                                                    \
+    }                                                                         \
+  } while (0)
+
 void set_relabel_small(bool on);   // relabel.cu: one-block shared-memory path for small layers
 
 constexpr int kNumSMs = 148;  // B200: 2 dies x 74 SMs
@@ -177,6 +201,12 @@ __device__ __forceinline__ int check_row(const RowTables& t, int64_t id) {
   if (p == -1) return APT_FLAG_FEAT_NOT_EXIST;
   return p >= t.num_dev_rows || (-p - 2) >= t.num_uva_rows ? APT_FLAG_ID_OUT_OF_RANGE : 0;
 }
+
+// First statement of every kernel launched with APT_FOLLOW: until the kernels before it are done and what they wrote can
+// be read. None of them announces its end early (griddepcontrol.launch_dependents): this kernel's blocks would then sit
+// on an SM beside blocks that still read lines about to be rewritten, and a load through the read-only path may find
+// the old line in L1. Waiting for their exit gives the same times.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Sizes may live on the device: an operator chained behind another one takes
 // its element count from a device word (what the previous kernel produced), so

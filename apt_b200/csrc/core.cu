@@ -72,6 +72,7 @@ ProfScope::~ProfScope() {
 __global__ void __launch_bounds__(256)
 k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __restrict__ sequence_dev, int64_t sequence,
                 volatile int64_t* host) {
+  wait_for_previous();
   if (threadIdx.x == 0 && sequence_dev) sequence = *sequence_dev;
   for (int t = threadIdx.x; t < count; t += blockDim.x) host[t] = words[t];
   __threadfence_system();
@@ -85,6 +86,7 @@ k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __r
 __global__ void __launch_bounds__(256)
 k_stage_replay(const int64_t* __restrict__ seeds, int64_t n, int64_t* __restrict__ seeds_buf, int64_t call_base, int64_t sequence,
                int64_t* __restrict__ words) {
+  wait_for_previous();
   for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < n; t += (int64_t)gridDim.x * 256) seeds_buf[t] = seeds[t];
   if (blockIdx.x == 0 && threadIdx.x < 2) words[threadIdx.x] = threadIdx.x ? sequence : call_base;
 }
@@ -97,7 +99,7 @@ int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_d
                       void* stream) {
   using namespace apt;
   APT_CHECK_ARG(words && host && count >= 0 && count <= 4096, "apt_publish_words: bad argument");
-  APT_LAUNCH(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, sequence_dev, sequence, host);
+  APT_FOLLOW(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, sequence_dev, sequence, host);
   return APT_OK;
 }
 
@@ -105,7 +107,7 @@ int apt_stage_replay(const int64_t* seeds, int64_t num_seeds, int64_t* seeds_buf
                      int64_t* words, void* stream) {
   using namespace apt;
   APT_CHECK_ARG(num_seeds >= 0 && words && (num_seeds == 0 || (seeds && seeds_buf)), "apt_stage_replay: bad argument");
-  APT_LAUNCH(k_stage_replay, wave_grid(ceil_div(num_seeds, 256), 4, 1), 256, 0, (cudaStream_t)stream, seeds, num_seeds,
+  APT_FOLLOW(k_stage_replay, wave_grid(ceil_div(num_seeds, 256), 4, 1), 256, 0, (cudaStream_t)stream, seeds, num_seeds,
              seeds_buf, call_base, sequence, words);
   return APT_OK;
 }

@@ -52,6 +52,7 @@ __device__ __forceinline__ float group_sum(float v, int n) {
 // First and last edge of every destination; *none when the edges are not grouped (nothing then belongs to anybody).
 __global__ void __launch_bounds__(256)
 k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* __restrict__ range, int32_t* none, int32_t* status) {
+  wait_for_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   bool bad = false;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(256)
 k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
               int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ weight,
               T* __restrict__ attn) {
+  wait_for_previous();
   constexpr int K = 16;
   if (*none != 0) return;
   const int64_t total = num_dst * num_heads, stride = (int64_t)gridDim.x * blockDim.x;
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(256, 3)
 k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ grad_out, int num_heads, int head_dim,
            int64_t num_dst_, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ dots, int lph,
            int hpp, uint32_t num_src, int32_t* __restrict__ src_count /* null: not wanted */, uint32_t* __restrict__ rank) {
+  wait_for_previous();
   if (*none != 0) return;
   const int lane = threadIdx.x & 31, G = gridDim.x * 8, num_dst = (int)num_dst_;
   const int lpe = lph * hpp, ep = 32 / lpe;
@@ -237,6 +240,7 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
              int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
              float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort,
              T* __restrict__ attn, T* __restrict__ grad_score, T* __restrict__ grad_er) {
+  wait_for_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const bool empty = *none != 0;
   if (empty)   // no edge belongs to anybody
@@ -287,6 +291,7 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_source(const float* __restrict__ sums, int64_t n, T* __restrict__ grad_el) {
+  wait_for_previous();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     grad_el[i] = Elem<T>::from_f(sums[i]);
 }
@@ -353,10 +358,10 @@ static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaS
   APT_CUDA(cudaMemsetAsync(g.none, 0, 4, s));
   {
     ProfScope prof("spmm_ranges", s);
-    APT_LAUNCH(k_gat_ranges, wave_grid(ceil_div(q.E, 256), 8), 256, 0, s, q.col, q.E, q.num_dst, g.range, g.none, q.status);
+    APT_FOLLOW(k_gat_ranges, wave_grid(ceil_div(q.E, 256), 8), 256, 0, s, q.col, q.E, q.num_dst, g.range, g.none, q.status);
   }
   ProfScope prof("gat_rows", s);
-  APT_LAUNCH(k_gat_weights<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
+  APT_FOLLOW(k_gat_weights<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
              q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn);
   return APT_OK;
 }
@@ -384,7 +389,7 @@ static int launch_dots(const GatProblem& q, const GatEdges& g, int64_t num_src, 
   if (rc != APT_OK) return rc;
   const int lph = pow2_ge(q.Dh / VE), hpp = pow2_ge(q.H, 32 / lph);
   const int64_t want = ceil_div(q.num_dst, 8), wave = (int64_t)kNumSMs * per_sm;
-  APT_LAUNCH((k_gat_dots<T, VE>), (int)(want < wave ? want : wave), 256, 0, s, q.row, (const T*)q.ft, (const T*)q.grad_out, q.H,
+  APT_FOLLOW((k_gat_dots<T, VE>), (int)(want < wave ? want : wave), 256, 0, s, q.row, (const T*)q.ft, (const T*)q.grad_out, q.H,
              (int)q.Dh, q.num_dst, g.range, g.none, dots, lph, hpp, (uint32_t)num_src, sort.cnt, sort.rank);
   return APT_OK;
 }
@@ -404,7 +409,7 @@ static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num
   }
   if (rc == APT_OK && sums) rc = launch_slots(num_src, sort, kOrder, long_edges, (int)(q.H * q.Dh), s);
   if (rc != APT_OK) return rc;
-  APT_LAUNCH(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
+  APT_FOLLOW(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
              q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, sort, (T*)attn, (T*)grad_score, (T*)grad_er);
   return APT_OK;
 }
@@ -424,7 +429,7 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
   ProfScope prof("spmm_rows", s);
   rc = launch_spmm_rows<T>(kUMulW, a, s);
   if (rc != APT_OK) return rc;
-  APT_LAUNCH(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (T*)grad_el);
+  APT_FOLLOW(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (T*)grad_el);
   return APT_OK;
 }
 

@@ -114,6 +114,7 @@ k_gather(const int64_t* __restrict__ index, int64_t n, const int64_t* __restrict
          const int64_t* __restrict__ pos_map, int64_t num_nodes, const char* __restrict__ dev_feats, int64_t num_dev_rows,
          const char* __restrict__ uva_feats, int64_t num_uva_rows, int64_t uva_row_bytes, int64_t col_offset_bytes,
          int64_t row_bytes, int rows_per_chunk, int lpr, char* __restrict__ out, int32_t* status) {
+  wait_for_previous();
   n = effective_n(n, n_dev);
   const int64_t first = first_row(first_dev, n);
   const int lane = threadIdx.x & 31;
@@ -193,7 +194,7 @@ static int gather_launch(const GatherArgs& a, cudaStream_t s) {
   const int grid = wave_grid(ceil_div(a.num_rows, (int64_t)per * (kGatherBlock / 32)), 8, kGatherWaves);
   ProfScope prof("gather_hit", s);
 #define APT_GATHER(V)                                                                                                     \
-  APT_LAUNCH(k_gather<V>, grid, kGatherBlock, 0, s, a.index, a.num_rows, a.num_rows_dev, a.first_row_dev, a.feat_pos_map, \
+  APT_FOLLOW(k_gather<V>, grid, kGatherBlock, 0, s, a.index, a.num_rows, a.num_rows_dev, a.first_row_dev, a.feat_pos_map, \
              a.num_nodes, a.dev_feats, a.num_dev_rows, a.uva_feats, a.num_uva_rows, a.uva_row_bytes,                      \
              a.uva_col_offset_bytes, a.dev_row_bytes, per, lpr, a.out, a.status_word)
   switch (width) {

@@ -68,6 +68,7 @@ template <typename V, int MODE>
 __global__ void __launch_bounds__(kMoveBlock)
 k_rows_move(const char* __restrict__ in, const int64_t* __restrict__ index, int64_t n,
             int64_t row_bytes, char* __restrict__ out) {
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -112,11 +113,11 @@ static int rows_move(const void* in, const int64_t* index, int64_t n, int64_t ro
   const char* ip = (const char*)in;
   char* op = (char*)out;
   switch (w) {
-    case 16: APT_LAUNCH((k_rows_move<uint4, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
-    case 8: APT_LAUNCH((k_rows_move<uint2, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
-    case 4: APT_LAUNCH((k_rows_move<uint32_t, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
-    case 2: APT_LAUNCH((k_rows_move<uint16_t, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
-    default: APT_LAUNCH((k_rows_move<uint8_t, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
+    case 16: APT_FOLLOW((k_rows_move<uint4, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
+    case 8: APT_FOLLOW((k_rows_move<uint2, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
+    case 4: APT_FOLLOW((k_rows_move<uint32_t, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
+    case 2: APT_FOLLOW((k_rows_move<uint16_t, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
+    default: APT_FOLLOW((k_rows_move<uint8_t, MODE>), grid, kMoveBlock, 0, s, ip, index, n, row_bytes, op); break;
   }
   return APT_OK;
 }

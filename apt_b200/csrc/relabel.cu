@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(256)
 k_insert(const int64_t* __restrict__ seeds, int64_t S_host, const int64_t* __restrict__ nbrs,
          int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, RelabelWs ws,
          int32_t* status) {
+  wait_for_previous();
   const RelabelDims d = relabel_dims(S_host, M_host, S_dev, per_seed);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int flags = 0;
@@ -84,6 +85,7 @@ static_assert(kSubTile / 32 == 32, "a sub-tile's words are scanned by one warp")
 
 __global__ void __launch_bounds__(kFirstThreads)
 k_first(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, RelabelWs ws, int tile_shift) {
+  wait_for_previous();
   __shared__ uint32_t counts[32], bases[32];
   const RelabelDims d = relabel_dims(S_host, M_host, S_dev, per_seed);
   const int64_t first = (int64_t)blockIdx.x << tile_shift;
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(256)
 k_relabel(int64_t S_host, int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, RelabelWs ws, int tile_shift,
           int64_t* __restrict__ out_unique, int64_t* __restrict__ out, int64_t* __restrict__ out_col,
           int64_t* __restrict__ out_num_unique, const RowTables tables, int32_t* status) {
+  wait_for_previous();
   __shared__ int tile_base[kMaxTiles];
   __shared__ int scratch[33];
   const RelabelDims d = relabel_dims(S_host, M_host, S_dev, per_seed);
@@ -232,6 +235,7 @@ k_relabel_small(const int64_t* __restrict__ seeds, int64_t S_host, int64_t* __re
                 int64_t M_host, const int64_t* __restrict__ S_dev, int64_t per_seed, int erase_nbrs,
                 int64_t* __restrict__ out_unique, int64_t* __restrict__ out_relabeled, int64_t* __restrict__ out_col,
                 int64_t* __restrict__ out_num_unique, const RowTables tables, int32_t* status) {
+  wait_for_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int scratch[33];
   Slot* slots = (Slot*)smem;
@@ -310,10 +314,10 @@ static int first_and_relabel(int64_t num_seeds, int64_t num_neighbors, const int
   const int64_t n = num_seeds + num_neighbors;
   int tile_shift = 10;
   while (ceil_div(n, (int64_t)1 << tile_shift) > kMaxTiles) ++tile_shift;
-  APT_LAUNCH(k_first, (int)ceil_div(n, (int64_t)1 << tile_shift), kFirstThreads, 0, s, num_seeds, num_neighbors, num_seeds_dev,
+  APT_FOLLOW(k_first, (int)ceil_div(n, (int64_t)1 << tile_shift), kFirstThreads, 0, s, num_seeds, num_neighbors, num_seeds_dev,
              per_seed, ws, tile_shift);
   const int grid = wave_grid(ceil_div(n, 256 * 4), 8, 1);
-  APT_LAUNCH(k_relabel, grid, 256, 0, s, num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, tile_shift, out_unique,
+  APT_FOLLOW(k_relabel, grid, 256, 0, s, num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, tile_shift, out_unique,
              out_relabeled, out_col, out_num_unique, tables, status_word);
   return APT_OK;
 }
@@ -363,7 +367,7 @@ extern "C" int apt_relabel_csc(const int64_t* seeds, int64_t num_seeds,
     const int rc = set_small_smem();
     if (rc != APT_OK) return rc;
     ProfScope prof("relabel", s);
-    APT_LAUNCH(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, (int64_t*)neighbors, num_neighbors,
+    APT_FOLLOW(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, (int64_t*)neighbors, num_neighbors,
                num_seeds_dev, per_seed, 0, out_unique, out_relabeled, nullptr, out_num_unique, RowTables{},
                status_word);
     return APT_OK;
@@ -375,7 +379,7 @@ extern "C" int apt_relabel_csc(const int64_t* seeds, int64_t num_seeds,
     return APT_ERR_CAPACITY;
   }
   ProfScope prof("relabel", s);
-  APT_LAUNCH(k_insert, wave_grid(ceil_div(n, 256 * 2), 8, 2), 256, 0, s, seeds, num_seeds, neighbors, num_neighbors,
+  APT_FOLLOW(k_insert, wave_grid(ceil_div(n, 256 * 2), 8, 2), 256, 0, s, seeds, num_seeds, neighbors, num_neighbors,
              num_seeds_dev, per_seed, ws, status_word);
   return first_and_relabel(num_seeds, num_neighbors, num_seeds_dev, per_seed, ws, out_unique, out_relabeled, nullptr,
                            out_num_unique, RowTables{}, status_word, s);
@@ -426,11 +430,11 @@ extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
   do {                                                                                               \
     const int grid = wave_grid(ceil_div(num_seeds, 256 / G), 8);                                     \
     if (small)                                                                                       \
-      APT_LAUNCH((sample_replace_kernel<G, false>), grid, 256, 0, s, seeds, num_seeds,               \
+      APT_FOLLOW((sample_replace_kernel<G, false>), grid, 256, 0, s, seeds, num_seeds,               \
                  num_seeds_dev, fanout, g, k0, k1, call_id, call_id_base_dev, nbr_buf, status_word,  \
                  SampleInsert{nullptr, nullptr});                                                    \
     else                                                                                             \
-      APT_LAUNCH((sample_replace_kernel<G, true>), grid, 256, 0, s, seeds, num_seeds, num_seeds_dev, \
+      APT_FOLLOW((sample_replace_kernel<G, true>), grid, 256, 0, s, seeds, num_seeds, num_seeds_dev, \
                  fanout, g, k0, k1, call_id, call_id_base_dev, out_neighbors, status_word, ins);     \
   } while (0)
     if (fanout <= 8) {
@@ -446,7 +450,7 @@ extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
   if (small) {
     const int rc = set_small_smem();
     if (rc != APT_OK) return rc;
-    APT_LAUNCH(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, nbr_buf, num_neighbors,
+    APT_FOLLOW(k_relabel_small, 1, kRelabelBlock, kSmallSmem, s, seeds, num_seeds, nbr_buf, num_neighbors,
                num_seeds_dev, (int64_t)fanout, out_neighbors ? 0 : 1, out_unique, out_relabeled, out_col, out_num_unique,
                tables, status_word);
     return APT_OK;

@@ -17,6 +17,7 @@ sample_floyd_kernel(const int64_t* __restrict__ seeds, int64_t num_seeds,
                     const int64_t* __restrict__ uva_indices, uint32_t k0,
                     uint32_t k1, uint32_t call_id, const int64_t* __restrict__ call_base_dev,
                     int64_t* __restrict__ out, int32_t* status) {
+  wait_for_previous();
   num_seeds = effective_n(num_seeds, num_seeds_dev);
   if (call_base_dev) call_id += (uint32_t)*call_base_dev;
   const int lane = threadIdx.x & 31;
@@ -97,7 +98,7 @@ extern "C" int apt_sample_csc_fanout(
   ProfScope prof("sample", s);
   if (!replace) {
     const int grid = wave_grid(ceil_div(num_seeds, 8), 8);
-    APT_LAUNCH(sample_floyd_kernel, grid, 256, 0, s, seeds, num_seeds, num_seeds_dev, fanout,
+    APT_FOLLOW(sample_floyd_kernel, grid, 256, 0, s, seeds, num_seeds, num_seeds_dev, fanout,
                adj_pos_map, num_nodes, dev_indptr, dev_indices, uva_indptr,
                uva_indices, k0, k1, call_id, call_id_base_dev, out_neighbors, status_word);
     return APT_OK;
@@ -105,7 +106,7 @@ extern "C" int apt_sample_csc_fanout(
 #define APT_SAMPLE_G(G)                                                        \
   do {                                                                         \
     const int grid = wave_grid(ceil_div(num_seeds, 256 / G), 8);               \
-    APT_LAUNCH((sample_replace_kernel<G, false>), grid, 256, 0, s, seeds, num_seeds,    \
+    APT_FOLLOW((sample_replace_kernel<G, false>), grid, 256, 0, s, seeds, num_seeds,    \
                num_seeds_dev, fanout, g, k0, k1, call_id, call_id_base_dev,    \
                out_neighbors, status_word, SampleInsert{nullptr, nullptr});    \
   } while (0)

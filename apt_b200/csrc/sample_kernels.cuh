@@ -77,6 +77,7 @@ sample_replace_kernel(const int64_t* __restrict__ seeds, int64_t num_seeds,
                       const int64_t* __restrict__ num_seeds_dev, int fanout, CscView g, uint32_t k0,
                       uint32_t k1, uint32_t call_id, const int64_t* __restrict__ call_base_dev,
                       int64_t* __restrict__ out, int32_t* status, SampleInsert ins) {
+  wait_for_previous();
   const int64_t groups_per_block = blockDim.x / G;
   int64_t j = (int64_t)blockIdx.x * groups_per_block + threadIdx.x / G;
   // the first id is on its way before the count is known: `seeds` holds the upper bound

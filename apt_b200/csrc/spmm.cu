@@ -82,6 +82,7 @@ __device__ __forceinline__ unsigned long long probe_votes(uint32_t bits) {
 __global__ void __launch_bounds__(256)
 k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned long long* agg, volatile int64_t* result,
              int64_t sequence) {
+  wait_for_previous();
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   __shared__ uint32_t s_bits;
   constexpr int K = 4;
@@ -141,7 +142,7 @@ static int launch_probe(const int64_t* col, int64_t E, SegTable st, unsigned lon
   // a thousand edges a block and one wave at most: small blocks of edges are looked over by one thread block
   const int grid = wave_grid(ceil_div(E, 1024), 4, 1);
   ProfScope prof("spmm_ranges", s);
-  APT_LAUNCH(k_spmm_probe, grid, 256, 0, s, col, E, st, agg, (volatile int64_t*)result, sequence);
+  APT_FOLLOW(k_spmm_probe, grid, 256, 0, s, col, E, st, agg, (volatile int64_t*)result, sequence);
   return APT_OK;
 }
 
@@ -219,6 +220,7 @@ __device__ __forceinline__ int resolve_mode(int mode, const SpmmWs& ws) {
 // Grouped edges: the edge that opens a row closes the one before and leaves the rows in between empty.
 __global__ void __launch_bounds__(256)
 k_edge_ranges(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_rows, SpmmWs ws, int mode) {
+  wait_for_previous();
   if (resolve_mode(mode, ws) != kRanges) return;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   for (int t = threadIdx.x; t <= st.nseg; t += blockDim.x) {
@@ -247,6 +249,7 @@ k_edge_ranges(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t n
 // that writes the order needs no second round of atomics (1.01 M edges: 25 + 28 us with one in both passes).
 __global__ void __launch_bounds__(256)
 k_dst_rank(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_rows, SpmmWs ws, int mode) {
+  wait_for_previous();
   if (resolve_mode(mode, ws) != kOrder) return;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   for (int t = threadIdx.x; t <= st.nseg; t += blockDim.x) {
@@ -277,6 +280,7 @@ k_dst_rank(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_
 constexpr int kScanRows = 4;
 __global__ void __launch_bounds__(256)
 k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, int long_edges, int part_stride) {
+  wait_for_previous();
   if (resolve_mode(mode, ws) != kOrder) return;
   __shared__ int scratch[33];
   __shared__ int s_base;
@@ -317,6 +321,7 @@ k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, int long_edges, int part_stri
 
 __global__ void __launch_bounds__(256)
 k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E, SegTable st, SpmmWs ws, int mode) {
+  wait_for_previous();
   if (resolve_mode(mode, ws) != kOrder) return;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1], ioff[kMaxSegments + 1];
   for (int t = threadIdx.x; t <= st.nseg; t += blockDim.x) {
@@ -350,7 +355,7 @@ k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int
 }
 
 int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s) {
-  APT_LAUNCH(k_dst_slots, (int)ceil_div(num_rows, 256 * kScanRows), 256, 0, s, num_rows, ws, mode, long_edges, part_stride);
+  APT_FOLLOW(k_dst_slots, (int)ceil_div(num_rows, 256 * kScanRows), 256, 0, s, num_rows, ws, mode, long_edges, part_stride);
   return APT_OK;
 }
 
@@ -358,10 +363,10 @@ static int launch_group(const int64_t* row, const int64_t* col, int64_t num_edge
                  const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s) {
   ProfScope prof("spmm_group", s);
   const int ge = wave_grid(ceil_div(num_edges, 256 * 4), 8, 1);
-  APT_LAUNCH(k_dst_rank, ge, 256, 0, s, col, num_edges, st, num_rows, ws, mode);
+  APT_FOLLOW(k_dst_rank, ge, 256, 0, s, col, num_edges, st, num_rows, ws, mode);
   const int rc = launch_slots(num_rows, ws, mode, long_edges, part_stride, s);
   if (rc != APT_OK) return rc;
-  APT_LAUNCH(k_dst_fill, ge, 256, 0, s, row, col, num_edges, st, ws, mode);
+  APT_FOLLOW(k_dst_fill, ge, 256, 0, s, row, col, num_edges, st, ws, mode);
   return APT_OK;
 }
 
@@ -372,6 +377,7 @@ __global__ void __launch_bounds__(256)
 k_sddmm(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E,
         const T* __restrict__ lhs, const T* __restrict__ rhs, int64_t feat_dim,
         SegTable st, const int64_t* __restrict__ rhs_off, T* __restrict__ out, int lpe) {
+  wait_for_previous();
   constexpr int U = 4;
   __shared__ int64_t coo[kMaxSegments + 1], loff[kMaxSegments + 1], roff[kMaxSegments + 1];
   for (int t = threadIdx.x; t <= st.nseg; t += blockDim.x) {
@@ -424,9 +430,9 @@ static int launch_sddmm(int op, const int64_t* row, const int64_t* col, int64_t 
   const int lpe = pow2_ge(feat_dim / VE);
   const int grid = wave_grid(ceil_div(E, (int64_t)(256 / lpe) * 4), 8);
   if (op == 0) {
-    APT_LAUNCH((k_sddmm<T, VE, 0>), grid, 256, 0, s, row, col, E, lhs, rhs, feat_dim, st, rhs_off, out, lpe);
+    APT_FOLLOW((k_sddmm<T, VE, 0>), grid, 256, 0, s, row, col, E, lhs, rhs, feat_dim, st, rhs_off, out, lpe);
   } else {
-    APT_LAUNCH((k_sddmm<T, VE, 1>), grid, 256, 0, s, row, col, E, lhs, rhs, feat_dim, st, rhs_off, out, lpe);
+    APT_FOLLOW((k_sddmm<T, VE, 1>), grid, 256, 0, s, row, col, E, lhs, rhs, feat_dim, st, rhs_off, out, lpe);
   }
   return APT_OK;
 }
@@ -481,7 +487,7 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
   }
   if (mode == kDevice || mode == kRanges) {
     ProfScope prof("spmm_ranges", s);
-    APT_LAUNCH(k_edge_ranges, wave_grid(ceil_div(E, 256), 8), 256, 0, s, coo_col, E, st, num_rows, ws, mode);
+    APT_FOLLOW(k_edge_ranges, wave_grid(ceil_div(E, 256), 8), 256, 0, s, coo_col, E, st, num_rows, ws, mode);
   }
   if (mode == kDevice || mode == kOrder) {
     const int rc = launch_group(coo_row, coo_col, E, st, num_rows, ws, mode, split.long_edges, (int)feat_dim, s);

@@ -216,6 +216,7 @@ constexpr int rows_min_blocks(int op, int elems) {
 template <typename T, int VE, int VPL, int OP, bool WIDE>
 __global__ void __launch_bounds__(256, rows_min_blocks(OP, VE * VPL))
 k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
+  wait_for_previous();
   constexpr int U = VPL >= 2 ? 2 : 4;
   __shared__ int64_t coo[kMaxSegments + 1], ioff[kMaxSegments + 1];
   int mode = a.mode, fixed = a.fixed;
@@ -448,7 +449,7 @@ static int launch_rows_kernel(const RowArgs<T>& a, cudaStream_t s) {
   if (rc != APT_OK) return rc;
   const int64_t want = ceil_div(a.num_rows, 256 / (a.split.lpe * a.split.ep));
   const int64_t wave = (int64_t)kNumSMs * per_sm;
-  APT_LAUNCH((k_spmm_rows<T, VE, VPL, OP, WIDE>), (int)(want < wave ? want : wave), 256, 0, s, a);
+  APT_FOLLOW((k_spmm_rows<T, VE, VPL, OP, WIDE>), (int)(want < wave ? want : wave), 256, 0, s, a);
   return APT_OK;
 }
 

@@ -10,6 +10,7 @@ __global__ void __launch_bounds__(256)
 k_src_to_vir(const int64_t* __restrict__ dst, int64_t num_dst, const int64_t* __restrict__ src,
              int64_t num_src, int64_t fanout, const int64_t* __restrict__ min_vids, OwnerParams p,
              int with_dst, int64_t* __restrict__ out) {
+  wait_for_previous();
   __shared__ int64_t mv[kMaxRanks + 1];
   if (threadIdx.x <= p.world_size) mv[threadIdx.x] = min_vids[threadIdx.x];
   __syncthreads();
@@ -50,6 +51,7 @@ k_vir_send_sizes(const int64_t* __restrict__ sorted_nodes, int64_t num_sorted,
                  const int64_t* __restrict__ num_unique_dev, int ws, int64_t base,
                  const int64_t* __restrict__ base_dev, int with_dst,
                  int64_t* __restrict__ out_offset, int64_t* __restrict__ out_sizes) {
+  wait_for_previous();
   __shared__ int64_t off[3 * kMaxRanks + 1];
   const int K = with_dst ? 2 * ws : ws;
   const int total = K + 1 + ws;
@@ -76,6 +78,7 @@ k_vir_send_sizes(const int64_t* __restrict__ sorted_nodes, int64_t num_sorted,
 __global__ void __launch_bounds__(256)
 k_sp_pack(const int64_t* __restrict__ sorted_vir, const int64_t* __restrict__ sorted_ids, int64_t n,
           int64_t num_dst, int64_t rank_term, int64_t num_total_nodes, int64_t* __restrict__ out) {
+  wait_for_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
     out[i] = rank_term + (sorted_vir[i] % num_dst) * num_total_nodes + sorted_ids[i];
@@ -84,6 +87,7 @@ k_sp_pack(const int64_t* __restrict__ sorted_vir, const int64_t* __restrict__ so
 __global__ void __launch_bounds__(256)
 k_sp_unpack(const int64_t* __restrict__ packed, int64_t n, const int64_t* __restrict__ n_dev,
             int64_t num_total_nodes, int64_t* __restrict__ out_vir, int64_t* __restrict__ out_ori) {
+  wait_for_previous();
   n = effective_n(n, n_dev);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -107,6 +111,7 @@ k_sp_map_place_pack(const int64_t* __restrict__ nbr, const int64_t* __restrict__
                     const int64_t* __restrict__ min_vids, OwnerParams p, int64_t rank_term,
                     int64_t num_total_nodes, int64_t* __restrict__ sorted_vir,
                     int64_t* __restrict__ packed, int64_t* __restrict__ out_count) {
+  wait_for_previous();
   __shared__ int64_t mv[kMaxRanks + 1];
   if (threadIdx.x <= p.world_size) mv[threadIdx.x] = min_vids[threadIdx.x];
   __syncthreads();
@@ -146,7 +151,7 @@ extern "C" int apt_src_to_vir(const int64_t* src, int64_t num_src, int64_t fanou
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("src_to_vir", s);
   OwnerParams p{world_size, shuffle_id_offset, rank, node_beg, node_end};
-  APT_LAUNCH(k_src_to_vir, wave_grid(ceil_div(num_src, 256), 8), 256, 0, s, nullptr, num_dst, src, num_src,
+  APT_FOLLOW(k_src_to_vir, wave_grid(ceil_div(num_src, 256), 8), 256, 0, s, nullptr, num_dst, src, num_src,
              fanout, min_vids, p, 0, out_vir);
   return APT_OK;
 }
@@ -165,7 +170,7 @@ extern "C" int apt_srcdst_to_vir(const int64_t* dst, int64_t num_dst, const int6
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("src_to_vir", s);
   OwnerParams p{world_size, shuffle_id_offset, rank, node_beg, node_end};
-  APT_LAUNCH(k_src_to_vir, wave_grid(ceil_div(num_src + num_dst, 256), 8), 256, 0, s, dst, num_dst, src,
+  APT_FOLLOW(k_src_to_vir, wave_grid(ceil_div(num_src + num_dst, 256), 8), 256, 0, s, dst, num_dst, src,
              num_src, fanout, min_vids, p, 1, out_vir);
   return APT_OK;
 }
@@ -183,7 +188,7 @@ extern "C" int apt_vir_send_sizes(const int64_t* sorted_nodes, int64_t num_sorte
                 "apt_vir_send_sizes: null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("vir_send_sizes", s);
-  APT_LAUNCH(k_vir_send_sizes, 1, 128, 0, s, sorted_nodes, num_sorted, num_sorted_dev, unique_nodes, num_unique,
+  APT_FOLLOW(k_vir_send_sizes, 1, 128, 0, s, sorted_nodes, num_sorted, num_sorted_dev, unique_nodes, num_unique,
              num_unique_dev, world_size, base, base_dev, with_dst ? 1 : 0, out_send_offset, out_send_sizes);
   return APT_OK;
 }
@@ -203,7 +208,7 @@ extern "C" int apt_sp_pack_frontier(const int64_t* sorted_vir, const int64_t* so
   APT_CHECK_ARG(sorted_vir && sorted_ids && out && num_dst > 0, "apt_sp_pack_frontier: null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("sp_pack", s);
-  APT_LAUNCH(k_sp_pack, wave_grid(ceil_div(n, 256), 8), 256, 0, s, sorted_vir, sorted_ids, n, num_dst,
+  APT_FOLLOW(k_sp_pack, wave_grid(ceil_div(n, 256), 8), 256, 0, s, sorted_vir, sorted_ids, n, num_dst,
              (int64_t)rank * sp_base * num_total_nodes, num_total_nodes, out);
   return APT_OK;
 }
@@ -217,7 +222,7 @@ extern "C" int apt_sp_unpack_frontier(const int64_t* packed, int64_t n, const in
   APT_CHECK_ARG(packed && out_vir && out_ori, "apt_sp_unpack_frontier: null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("sp_unpack", s);
-  APT_LAUNCH(k_sp_unpack, wave_grid(ceil_div(n, 256), 8), 256, 0, s, packed, n, n_dev, num_total_nodes, out_vir,
+  APT_FOLLOW(k_sp_unpack, wave_grid(ceil_div(n, 256), 8), 256, 0, s, packed, n, n_dev, num_total_nodes, out_vir,
              out_ori);
   return APT_OK;
 }
@@ -244,7 +249,7 @@ extern "C" int apt_sp_map_place_pack(const int64_t* neighbors, const int64_t* po
                 "apt_sp_map_place_pack: null pointer");
   ProfScope prof("sp_map_place_pack", s);
   OwnerParams p{world_size, shuffle_id_offset, rank, node_beg, node_end};
-  APT_LAUNCH(k_sp_map_place_pack, wave_grid(ceil_div(num_dst * fanout, 256), 8), 256, 0, s, neighbors, positions,
+  APT_FOLLOW(k_sp_map_place_pack, wave_grid(ceil_div(num_dst * fanout, 256), 8), 256, 0, s, neighbors, positions,
              num_dst, num_dst_dev, fanout, min_vids, p, (int64_t)rank * sp_base * num_total_nodes, num_total_nodes,
              out_sorted_vir, out_packed, out_count);
   return APT_OK;
