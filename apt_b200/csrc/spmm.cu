@@ -63,6 +63,8 @@ size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) 
   return at;
 }
 
+int bulk_gave_up(int32_t** word);   // spmm_bulk.cuh
+
 // ---- the probe -------------------------------------------------------------------------
 constexpr uint32_t kNotGrouped = 1u, kNotFixed = 2u, kHasLong = 4u;
 
@@ -191,6 +193,23 @@ static void give_slot(int slot) {
     g_probe.taken &= ~(1ull << slot);
   }
   g_probe.cv.notify_one();
+}
+
+int bulk_gave_up(int32_t** word) {
+  static std::mutex mu;
+  static int32_t* mapped = nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!mapped) {
+    void* p = nullptr;
+    APT_CUDA(cudaHostAlloc(&p, 64, cudaHostAllocMapped | cudaHostAllocPortable));
+    *(int32_t*)p = 0;
+    mapped = (int32_t*)p;
+  }
+  *word = mapped;
+  if (*(volatile int32_t*)mapped == 0) return APT_OK;
+  *(volatile int32_t*)mapped = 0;
+  set_error("spmm: a row's copy to shared memory did not complete in an earlier call");
+  return APT_ERR_TIMEOUT;
 }
 
 // Polls a mapped word until it carries `sequence`. The stream is asked now and then, so that an error on it ends the wait.

@@ -18,6 +18,8 @@
 //                block of 1024 threads per long row, the form before this, kept 26 of 148 SMs busy for
 //                62 us behind the row kernel.
 //
+// Wide rows of many edges have a kernel of their own (spmm_bulk.cuh).
+//
 // Where a row's edges are (`mode`):
 //   kFixed    every row has `fixed` consecutive edges: what a fanout sampler produces. No table.
 //   kRanges   grouped by row, any length: range[] (k_edge_ranges)
@@ -465,7 +467,15 @@ static int launch_rows_vpl(const RowArgs<T>& a, cudaStream_t s) {
 }
 
 template <typename T, int OP>
+static int launch_bulk(const RowArgs<T>& a, cudaStream_t s, bool* taken);     // spmm_bulk.cuh
+
+template <typename T, int OP>
 static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
+  if constexpr (OP == kCopyU || OP == kUMulW) {
+    bool taken = false;
+    const int rc = launch_bulk<T, OP>(a, s, &taken);
+    if (taken || rc != APT_OK) return rc;
+  }
   switch (a.split.ve * (int)sizeof(T)) {
     case 16: return launch_rows_vpl<T, 16 / sizeof(T), OP>(a, s);
     case 8: return launch_rows_vpl<T, 8 / sizeof(T), OP>(a, s);

@@ -93,3 +93,23 @@ def test_ungrouped_backward_is_zero_and_flagged():
     assert not any(host(g).any() for g in grads)
     with pytest.raises(RuntimeError, match="not grouped"):
         ops.check_status()
+
+
+@pytest.mark.parametrize("dtype,H,Dh", [(torch.float32, 4, 64), (torch.float32, 3, 44), (torch.float32, 16, 16),
+                                        (torch.float32, 17, 12), (torch.bfloat16, 4, 128), (torch.float16, 1, 272)])
+def test_source_rows_of_many_edges(dtype, H, Dh):
+    # enough edges of rows above 512 bytes for the copies through shared memory: hubs, short rows and rows without edges
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    S, n_src = 14_001, 20_003
+    lengths = torch.randint(0, 31, (S,), device="cuda", generator=gen)
+    col = torch.repeat_interleave(torch.arange(S, device="cuda"), lengths)
+    u = torch.rand(col.numel(), device="cuda", generator=gen, dtype=torch.float64)
+    row = (u ** 3 * n_src).long()
+    rand = lambda *shape: torch.randn(shape, device="cuda", generator=gen).to(dtype)
+    ft, el, er, go = rand(n_src, H, Dh), rand(n_src, H, 1), rand(S, H, 1), rand(S, H, Dh)
+    _, attn = ops.gat_edge_softmax_sum(row, col, ft, el, er, S, 0.2, return_attention=True)
+    got = ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, go, 0.2)[0]
+    want = torch.zeros((n_src, H, Dh), device="cuda", dtype=torch.float64)
+    want.index_add_(0, row, attn.double() * go.double()[col])
+    assert col.numel() >= 200_000
+    _near(got, host(want), dtype, "grad_ft")

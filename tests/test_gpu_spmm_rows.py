@@ -116,6 +116,34 @@ def test_probe_and_enqueue_only_form(name):
     _close(out, want, magnitude, torch.float32)
 
 
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 132), (torch.float32, 200), (torch.float32, 256),
+                                     (torch.bfloat16, 264), (torch.bfloat16, 512), (torch.float16, 384)])
+@pytest.mark.parametrize("shape", ["fixed", "ragged", "reverse", "segments"])
+def test_wide_rows_of_many_edges(dtype, D, shape):
+    # rows that travel through shared memory. Small whole numbers: exact in fp32, one rounding of the sum in 16 bits.
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    fixed = shape in ("fixed", "segments")
+    n_out, n_in, f = (20_002, 5001, 10) if fixed else (20_003, 5001, 21)
+    lengths = torch.full((n_out,), f, device="cuda") if fixed else torch.randint(0, f, (n_out,), device="cuda", generator=gen)
+    col = torch.repeat_interleave(torch.arange(n_out, device="cuda"), lengths)
+    u = torch.rand(col.numel(), device="cuda", generator=gen, dtype=torch.float64)
+    row = (u * u * n_in).long()
+    if shape == "reverse":                      # hubs of thousands of edges, items of their own
+        row, col, n_in, n_out = col, (u ** 4 * 50_000).long(), n_out, 50_000
+    E = col.numel()
+    assert E >= 196_608
+    x = torch.randint(-4, 5, (n_in, D), device="cuda", generator=gen).to(dtype)
+    T = lambda *v: torch.tensor(v, device="cuda")
+    offsets = T(0, E), T(0, n_in), T(0, n_out)
+    want = torch.zeros((n_out, D), device="cuda").index_add_(0, col, x.float()[row])
+    if shape == "segments":                     # two blocks with ids of their own
+        half, first = n_out // 2, col < n_out // 2
+        row = torch.where(first, row % 2000, row % 3001)
+        want = torch.zeros((n_out, D), device="cuda").index_add_(0, col, x.float()[torch.where(first, row, row + 2000)])
+        col, offsets = col % half, (T(0, E // 2, E), T(0, 2000, n_in), T(0, half, n_out))
+    assert torch.equal(ops.spmm_copy_u_sum(row, col, x, *offsets), want.to(dtype))
+
+
 @pytest.mark.parametrize("E", [2, 5, 1023, 1024, 1025, 700_001])
 def test_probe_finds_one_edge_out_of_order(E):
     # one thread block and several, the last of them ragged; more edges than one wave of blocks holds at a time
