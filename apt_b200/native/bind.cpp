@@ -352,61 +352,114 @@ Tensor offsets_cpu(const int64_t* v, int64_t n, bool sum) {
   return t;
 }
 
-// The hops of a mini-batch cut to their real sizes. `layers`: innermost first, (relabelled rows, unique ids, columns,
-// fanout, count slot). Returns the blocks, outermost first, and the number of nodes of the last frontier.
-std::pair<py::list, int64_t> narrow_blocks(const int64_t* w, int64_t num_dst, const py::list& layers, const py::object& block) {
-  py::list blocks;
-  for (const auto& item : layers) {
-    const py::tuple l = item.cast<py::tuple>();
-    const int64_t fanout = l[3].cast<int64_t>(), num_src = w[l[4].cast<int64_t>()];
-    blocks.insert(0, block(front(l[0].cast<Tensor>(), num_dst * fanout), front(l[2].cast<Tensor>(), num_dst * fanout), num_src,
-                           num_dst, front(l[1].cast<Tensor>(), num_src), fanout));
-    num_dst = num_src;
+// A view of all of `t` that is cut to its real length once that is known: the views, their Python objects and the blocks
+// around them (10 to 15 us a mini-batch) are made while the GPU is still sampling.
+Tensor whole(const Tensor& t) { return front(t, t.size(0)); }
+void cut(const Tensor& t, int64_t n) {
+  if (n < 0 || n > t.size(0)) fail("sampler: a count of " + std::to_string(n) + " exceeds a buffer of " + std::to_string(t.size(0)));
+  c10::SmallVector<int64_t, 4> sizes(t.sizes().begin(), t.sizes().end());
+  sizes[0] = n;
+  t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+}
+
+// The hops of a mini-batch, innermost first: (relabelled rows, unique ids, columns, fanout, count slot) each. `blocks`
+// lists them outermost first.
+class Hops {
+ public:
+  Hops(const py::list& layers, const py::object& block) {
+    for (const auto& item : layers) {
+      const py::tuple l = item.cast<py::tuple>();
+      Hop h{whole(l[0].cast<Tensor>()), whole(l[1].cast<Tensor>()), whole(l[2].cast<Tensor>()), py::none(),
+            l[3].cast<int64_t>(), l[4].cast<int64_t>()};
+      h.block = block(h.rows, h.cols, 0, 0, h.ids, h.fanout);
+      blocks.insert(0, h.block);
+      hops_.push_back(std::move(h));
+    }
   }
-  return {blocks, num_dst};
-}
+  // Cuts everything to the counts `w`; returns the number of nodes of the last frontier.
+  int64_t fill(const int64_t* w, int64_t num_dst) {
+    for (Hop& h : hops_) {
+      const int64_t num_src = w[h.slot];
+      cut(h.rows, num_dst * h.fanout);
+      cut(h.cols, num_dst * h.fanout);
+      cut(h.ids, num_src);
+      h.block.attr("num_src") = num_src;
+      h.block.attr("num_dst") = num_dst;
+      num_dst = num_src;
+    }
+    return num_dst;
+  }
+  py::list blocks;
 
-// Node-partitioned: blocks, permutation, exchange counts and inverse index. `outer` = the outermost hop as a layer; the
-// words hold [0..] hop counts, [16..] ids received per peer, [64..] bucket offsets.
-py::tuple np_finish(const Tensor& host, const Tensor& seeds, const py::list& layers, const py::tuple& outer, int64_t frontier_slot,
-                    const Tensor& perm, const Tensor& inverse, const OptTensor& rows, int64_t world_size, const py::object& block) {
-  const int64_t* const w = host.const_data_ptr<int64_t>();
-  auto [blocks, frontier] = narrow_blocks(w, seeds.numel(), layers, block);
-  const Tensor recv = offsets_cpu(w + 16, world_size, true), sent = offsets_cpu(w + 64, world_size, false);
-  const int64_t received = recv.const_data_ptr<int64_t>()[world_size - 1];
-  if (received > inverse.numel())
-    fail("chained NP sampler: more ids received than the buffer sized from this rank's own batch holds; use chained=False for "
-         "batches that differ this much between the ranks");
-  py::list last;
-  last.append(outer);
-  auto [outer_block, num_in] = narrow_blocks(w, w[frontier_slot], last, block);
-  blocks.insert(0, outer_block[0]);
-  const Tensor input = front(outer[1].cast<Tensor>(), num_in);
-  py::object row_view = py::none();
-  if (rows) row_view = py::cast(front(*rows, num_in));
-  return py::make_tuple(py::make_tuple(input, seeds, blocks, front(perm, frontier), recv, sent, front(inverse, received)), row_view);
-}
+ private:
+  struct Hop {
+    Tensor rows, ids, cols;
+    py::object block;
+    int64_t fanout, slot;
+  };
+  std::vector<Hop> hops_;
+};
 
-// Source-split, attention: the words hold what np_finish's do, with the unique neighbours and the input nodes in slots of
-// their own.
-py::tuple snp_gat_finish(const Tensor& host, const Tensor& seeds, const py::list& layers, const py::tuple& outer, const Tensor& perm,
-                         const Tensor& input_nodes, const OptTensor& rows, int64_t world_size, int64_t unique_slot,
-                         int64_t input_slot, const py::object& block) {
-  const int64_t* const w = host.const_data_ptr<int64_t>();
-  auto [blocks, num_dst] = narrow_blocks(w, seeds.numel(), layers, block);
-  const int64_t num_in = w[input_slot];
-  if (num_in > input_nodes.numel())
-    fail("chained SNP-GAT sampler: more ids received than the buffer sized from this rank's own batch holds; use chained=False "
-         "for batches that differ this much between the ranks");
-  py::list last;
-  last.append(outer);
-  blocks.insert(0, narrow_blocks(w, num_dst, last, block).first[0]);
-  py::object row_view = py::none();
-  if (rows) row_view = py::cast(front(*rows, num_in));
-  return py::make_tuple(py::make_tuple(front(input_nodes, num_in), seeds, blocks, front(perm, w[unique_slot]),
-                                       offsets_cpu(w + 16, world_size, true), offsets_cpu(w + 64, world_size, false)),
-                        row_view);
-}
+// What sample() of a chained sampler returns, (input nodes, seeds, blocks, permutation, ids received per peer, bucket
+// offsets[, inverse]) and the gathered rows, but for the lengths. `layers`: the inner hops, `outer` the outermost. The words
+// hold [0..] hop counts, [16..] ids received per peer, [64..] bucket offsets.
+//   node-partitioned        the outermost hop starts from w[frontier_slot] nodes and its sources are the input nodes
+//   source-split, attention it starts from the inner hops' frontier; the input nodes are a buffer of their own
+class Outline {
+ public:
+  Outline(const Tensor& seeds, const py::list& layers, const py::tuple& outer, const Tensor& perm, const OptTensor& inverse,
+          const OptTensor& input, const OptTensor& rows, int64_t world_size, int64_t frontier_slot, int64_t unique_slot,
+          int64_t input_slot, const py::object& block)
+      : inner_(layers, block), outer_(only(outer), block), world_(world_size), frontier_slot_(frontier_slot),
+        unique_slot_(unique_slot), input_slot_(input_slot), seeds_(seeds.numel()) {
+    const auto longs = at::TensorOptions().dtype(at::kLong);
+    perm_ = whole(perm);
+    input_ = whole(input ? *input : outer[1].cast<Tensor>());
+    recv_ = at::empty({world_size}, longs);
+    sent_ = at::empty({world_size}, longs);
+    inner_.blocks.insert(0, outer_.blocks[0]);
+    if (inverse) {
+      inverse_ = whole(*inverse);
+      got_ = py::make_tuple(input_, seeds, inner_.blocks, perm_, recv_, sent_, inverse_);
+    } else {
+      got_ = py::make_tuple(input_, seeds, inner_.blocks, perm_, recv_, sent_);
+    }
+    if (rows) {
+      rows_ = whole(*rows);
+      row_view_ = py::cast(rows_);
+    }
+  }
+  py::tuple finish(const Tensor& host) {
+    const int64_t* const w = host.const_data_ptr<int64_t>();
+    int64_t* const recv = recv_.mutable_data_ptr<int64_t>();
+    int64_t received = 0;
+    for (int64_t k = 0; k < world_; ++k) recv[k] = received += w[16 + k];
+    std::copy_n(w + 64, world_, sent_.mutable_data_ptr<int64_t>());
+    const int64_t frontier = inner_.fill(w, seeds_);
+    const bool np = inverse_.defined();
+    if (np ? received > inverse_.numel() : w[input_slot_] > input_.numel())
+      fail(std::string(np ? "chained NP sampler" : "chained SNP-GAT sampler") + ": more ids received than the buffer sized from "
+           "this rank's own batch holds; use chained=False for batches that differ this much between the ranks");
+    const int64_t sources = outer_.fill(w, np ? w[frontier_slot_] : frontier), num_in = np ? sources : w[input_slot_];
+    cut(input_, num_in);
+    cut(perm_, np ? frontier : w[unique_slot_]);
+    if (np) cut(inverse_, received);
+    if (rows_.defined()) cut(rows_, num_in);
+    return py::make_tuple(got_, row_view_);
+  }
+
+ private:
+  static py::list only(const py::tuple& layer) {
+    py::list l;
+    l.append(layer);
+    return l;
+  }
+  Hops inner_, outer_;
+  int64_t world_, frontier_slot_, unique_slot_, input_slot_, seeds_;
+  Tensor perm_, input_, inverse_, rows_, recv_, sent_;
+  py::object row_view_ = py::none();
+  py::tuple got_;
+};
 
 // Data-parallel: every hop sampled and relabelled on this GPU, the rows of the input nodes gathered behind the counts. One
 // read at the end; all results are tensors of their own.
@@ -430,45 +483,49 @@ py::tuple dp_sample(const Tensor& seeds, const std::vector<int64_t>& fanouts, co
   int64_t* const h = host.mutable_data_ptr<int64_t>();
   const int count = (int)words.numel();
   void* const s = stream();
-  struct Hop { Tensor rel, uniq, col; };
-  std::vector<Hop> hops;
+  py::list layers;
+  Tensor cur = seeds;
   Tensor rows;
   const auto ids_like = [&](int64_t n) { return at::empty({n}, seeds.options()); };
+  for (size_t k = 0; k < fanouts.size(); ++k) {
+    const int64_t n = cur.numel(), f = fanouts[k];
+    Tensor rel = ids_like(n * f), uniq = ids_like(n * (1 + f)), col = ids_like(n * f);
+    const bool last = gather && k + 1 == fanouts.size();
+    check(apt_sample_relabel_block(ptr(cur), n, k ? word + k - 1 : nullptr, (int)f, opt(adj_pos_map), num_nodes, opt(dev_indptr),
+                                   opt(dev_indices), ptr(uva_indptr), ptr(uva_indices), (uint64_t)key,
+                                   (uint32_t)(call + (int64_t)k), nullptr, relabel_ws.mutable_data_ptr(), relabel_ws.numel(),
+                                   nullptr, uniq.mutable_data_ptr<int64_t>(), rel.mutable_data_ptr<int64_t>(),
+                                   col.mutable_data_ptr<int64_t>(), word + k, last ? ptr(pos_map) : nullptr, feat_nodes,
+                                   last ? dev_feats.size(0) : 0, last ? uva_feats.size(0) : 0, status_word(words), s));
+    cur = uniq;
+    layers.append(py::make_tuple(rel, uniq, col, f, (int64_t)k));
+  }
+  check(apt_publish_words(word, count, nullptr, sequence, h, s));
+  if (gather) {
+    const int64_t size = dev_feats.element_size(), dim = dev_feats.size(1);
+    rows = at::empty({cur.numel(), dim}, dev_feats.options());
+    const size_t bytes = apt_gather_workspace_bytes(cur.numel());
+    const Tensor ws = scratch(rows, bytes);
+    check(apt_gather_rows(ptr(cur), cur.numel(), word + fanouts.size() - 1, ptr(pos_map), feat_nodes, data(dev_feats),
+                          dev_feats.size(0), dim * size, data(uva_feats), uva_feats.size(0), uva_feats.size(1) * size,
+                          column * size, mut(rows), ws.mutable_data_ptr(), bytes, status_word(words), s));
+  }
+  Hops hops(layers, block);
+  const Tensor input = whole(cur);
+  py::object input_view = py::cast(input), row_view = py::none();
+  Tensor cut_rows;
+  if (gather) {
+    cut_rows = whole(rows);
+    row_view = py::cast(cut_rows);
+  }
   {
     py::gil_scoped_release nogil;
-    Tensor cur = seeds;
-    for (size_t k = 0; k < fanouts.size(); ++k) {
-      const int64_t n = cur.numel(), f = fanouts[k];
-      Hop hop{ids_like(n * f), ids_like(n * (1 + f)), ids_like(n * f)};
-      const bool last = gather && k + 1 == fanouts.size();
-      check(apt_sample_relabel_block(ptr(cur), n, k ? word + k - 1 : nullptr, (int)f, opt(adj_pos_map), num_nodes, opt(dev_indptr),
-                                     opt(dev_indices), ptr(uva_indptr), ptr(uva_indices), (uint64_t)key,
-                                     (uint32_t)(call + (int64_t)k), nullptr, relabel_ws.mutable_data_ptr(), relabel_ws.numel(),
-                                     nullptr, hop.uniq.mutable_data_ptr<int64_t>(), hop.rel.mutable_data_ptr<int64_t>(),
-                                     hop.col.mutable_data_ptr<int64_t>(), word + k, last ? ptr(pos_map) : nullptr, feat_nodes,
-                                     last ? dev_feats.size(0) : 0, last ? uva_feats.size(0) : 0, status_word(words), s));
-      cur = hop.uniq;
-      hops.push_back(std::move(hop));
-    }
-    check(apt_publish_words(word, count, nullptr, sequence, h, s));
-    if (gather) {
-      const int64_t size = dev_feats.element_size(), dim = dev_feats.size(1);
-      rows = at::empty({cur.numel(), dim}, dev_feats.options());
-      const size_t bytes = apt_gather_workspace_bytes(cur.numel());
-      const Tensor ws = scratch(rows, bytes);
-      check(apt_gather_rows(ptr(cur), cur.numel(), word + fanouts.size() - 1, ptr(pos_map), feat_nodes, data(dev_feats),
-                            dev_feats.size(0), dim * size, data(uva_feats), uva_feats.size(0), uva_feats.size(1) * size,
-                            column * size, mut(rows), ws.mutable_data_ptr(), bytes, status_word(words), s));
-    }
     check(apt_wait_published(h, count, sequence, s));
   }
-  py::list layers;
-  for (size_t k = 0; k < hops.size(); ++k)
-    layers.append(py::make_tuple(hops[k].rel, hops[k].uniq, hops[k].col, fanouts[k], (int64_t)k));
-  auto [blocks, num_in] = narrow_blocks(h, seeds.numel(), layers, block);
-  py::object row_view = py::none();
-  if (gather) row_view = py::cast(front(rows, num_in));
-  return py::make_tuple(front(hops.back().uniq, num_in), blocks, row_view, h[count - 1] & 0xffffffff);
+  const int64_t num_in = hops.fill(h, seeds.numel());
+  cut(input, num_in);
+  if (gather) cut(cut_rows, num_in);
+  return py::make_tuple(input_view, hops.blocks, row_view, h[count - 1] & 0xffffffff);
 }
 
 }  // namespace
@@ -494,16 +551,22 @@ PYBIND11_MODULE(_native, m) {
       .def("finish", &Plan::finish)
       .def("order_current_stream", &Plan::order_current_stream);
   m.def("read_words", &read_words);
-  m.def("narrow_blocks", [](const Tensor& host, int64_t num_dst, const py::list& layers, const py::object& block) {
-    return narrow_blocks(host.const_data_ptr<int64_t>(), num_dst, layers, block);
-  });
-  m.def("fronts", [](const std::vector<Tensor>& tensors, const std::vector<int64_t>& sizes) {
+  py::class_<Hops>(m, "Hops")
+      .def(py::init<const py::list&, const py::object&>())
+      .def_readonly("blocks", &Hops::blocks)
+      .def("fill", [](Hops& hops, const Tensor& host, int64_t num_dst) { return hops.fill(host.const_data_ptr<int64_t>(), num_dst); });
+  py::class_<Outline>(m, "Outline")
+      .def(py::init<const Tensor&, const py::list&, const py::tuple&, const Tensor&, const OptTensor&, const OptTensor&,
+                    const OptTensor&, int64_t, int64_t, int64_t, int64_t, const py::object&>())
+      .def("finish", &Outline::finish);
+  m.def("wholes", [](const std::vector<Tensor>& tensors) {
     std::vector<Tensor> out;
-    for (size_t k = 0; k < tensors.size(); ++k) out.push_back(front(tensors[k], sizes.at(k)));
+    for (const Tensor& t : tensors) out.push_back(whole(t));
     return out;
   });
-  m.def("np_finish", &np_finish);
-  m.def("snp_gat_finish", &snp_gat_finish);
+  m.def("cut", [](const std::vector<Tensor>& tensors, const std::vector<int64_t>& sizes) {
+    for (size_t k = 0; k < tensors.size(); ++k) cut(tensors[k], sizes.at(k));
+  });
   m.def("pick", [](const Tensor& host, const std::vector<int64_t>& at) {
     std::vector<int64_t> out;
     for (const int64_t k : at) out.push_back(host.const_data_ptr<int64_t>()[k]);

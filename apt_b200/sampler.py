@@ -55,7 +55,7 @@ def _coo_col(num_dst_max: int, num_dst: int, fanout: int, device) -> torch.Tenso
 
 
 def _layer(dst_buf, rel, uniq, fanout, slot):
-    """A hop as _native.narrow_blocks takes it: upper-bound buffers and the word slot of its unique ids."""
+    """A hop as _native.Hops takes it: upper-bound buffers and the word slot of its unique ids."""
     return rel, uniq, _coo_col(dst_buf.numel(), dst_buf.numel(), fanout, rel.device), fanout, slot
 
 
@@ -123,7 +123,7 @@ class _Ring:
 
 class _GraphReplay:
     """What the chained samplers share: the whole mini-batch is enqueued by `_enqueue(seeds, base_dev, publish)`
-    without a host read and narrowed by `_finish(seeds, bufs, host)` after one look at the device word
+    without a host read, its result outlined by `_outline(seeds, bufs)` and narrowed by `_finish(seeds, bufs, host)` after one look at the device word
     block, which `publish()` sends to the host as soon as it is complete (a gather of the rows goes behind it
     and runs on while the host narrows); the enqueue is captured once per batch shape as a CUDA graph and replayed, from
     `graph_buffers` buffer sets in turn. `sample_iter` launches mini-batch k + 1 before it reads
@@ -257,7 +257,8 @@ class _GraphReplay:
     def _sample_chained(self, seeds: torch.Tensor):
         seeds = ops._need_cuda(seeds, "seeds")
         if not self._graph_ok():
-            return self._finish(seeds, self._enqueue(seeds, None))
+            bufs = self._enqueue(seeds, None)
+            return self._finish(seeds, bufs, outline=self._outline(seeds, bufs))
         return self._collect(self._launch(seeds, piped=False))
 
     def sample_iter(self, graph, seed_batches):
@@ -359,18 +360,19 @@ class _GraphReplay:
 
     def _collect(self, launched):
         plan, seeds = launched
+        outline = self._outline(seeds, plan.bufs)      # beside the GPU's work
         flags = plan.handle.wait()
         st = ops.STATE
         if plan.lane == 0:
             if flags:
                 st.check_flags(flags)
-            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle)
+            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle, outline)
         st.lane = plan.lane
         try:
             if flags:
                 plan.handle.order_current_stream()
                 st.check_flags(flags)
-            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle)
+            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle, outline)
         finally:
             st.lane = 0
 
@@ -495,14 +497,15 @@ class MixedNeighborSampler(_GraphReplay):
         return dict(layers=layers, perm=perm, inv=inv, rows=rows, u_slot=u_slot,
                     outer=_layer(uniq2, rel3, uniq3, self.las_fanouts, in_slot))
 
-    def _finish(self, seeds, bufs, host=None, plan=None):
+    def _outline(self, seeds, bufs):
+        return _native.Outline(seeds, bufs["layers"], bufs["outer"], bufs["perm"], bufs["inv"], None, bufs["rows"],
+                               ops.STATE.world_size, bufs["u_slot"], -1, -1, Block)
+
+    def _finish(self, seeds, bufs, host=None, plan=None, outline=None):
         """The one host read of the mini-batch (or the copy of the word block a captured launch
         left in `host`), then buffers narrowed to their real sizes."""
         st = ops.STATE
-        if host is None:
-            host = st.read_words()
-        got, rows = _native.np_finish(host, seeds, bufs["layers"], bufs["outer"], bufs["u_slot"], bufs["perm"], bufs["inv"],
-                                      bufs["rows"], st.world_size, Block)
+        got, rows = outline.finish(st.read_words() if host is None else host)
         if rows is not None:
             st.prefetched = (got[0], rows, plan)
         return got
@@ -583,12 +586,13 @@ class SPGATSampler(_GraphReplay):
         return dict(layers=layers, outer=_layer(cur, arange_src, unique_neigh, f, self._U), perm=perm,
                     input_nodes=input_nodes, rows=rows)
 
-    def _finish(self, seeds, b, host=None, plan=None):
+    def _outline(self, seeds, b):
+        return _native.Outline(seeds, b["layers"], b["outer"], b["perm"], None, b["input_nodes"], b["rows"],
+                               ops.STATE.world_size, -1, self._U, self._IN, Block)
+
+    def _finish(self, seeds, b, host=None, plan=None, outline=None):
         st = ops.STATE
-        if host is None:
-            host = st.read_words()
-        got, rows = _native.snp_gat_finish(host, seeds, b["layers"], b["outer"], b["perm"], b["input_nodes"], b["rows"],
-                                           st.world_size, self._U, self._IN, Block)
+        got, rows = outline.finish(st.read_words() if host is None else host)
         if rows is not None:
             st.prefetched = (got[0], rows, plan)
         return got
@@ -782,14 +786,26 @@ class SPVirtualSampler(_GraphReplay):
                     unique_src=unique_src, a_src=a_src, unique_dst=unique_dst, a_dst=a_dst, dst_sorted=dst_sorted,
                     recv_dst=recv_dst, input_nodes=input_nodes, rows=rows)
 
-    def _finish(self, seeds, b, host=None, plan=None):
+    _CUT = ("unique_frontier", "unique_src", "arange_dst", "a_src", "a_dst", "input_nodes", "nbr", "sorted_all", "packed", "vir_src",
+            "ori_src", "unique_dst")
+
+    def _outline(self, seeds, b):
+        hops = _native.Hops(b["layers"], Block)
+        views = _native.wholes([b[name] for name in self._CUT] + [_arange(b["unique_frontier"].numel(), seeds.device)])
+        uf, us, arange_dst, a_src, a_dst = views[:5]
+        outer = Block(a_src, a_dst, 0, 0, us, self.fanouts[0]), Block(views[12], arange_dst, 0, 0, uf, self.fanouts[0])
+        rows = None if b["rows"] is None else _native.wholes([b["rows"]])[0]
+        return hops, views, outer, rows
+
+    def _finish(self, seeds, b, host=None, plan=None, outline=None):
         """The one host read of the mini-batch, then everything is narrowed to its real size."""
         st = ops.STATE
         ws = st.world_size
         f = self.fanouts[0]
         if host is None:
             host = st.read_words()
-        blocks, num_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
+        hops, views, (block2, block1), rows = outline
+        num_dst = hops.fill(host, seeds.numel())
         n_uf, n_us, n_ud, n_in, n_recv, n_rdst = _native.pick(host, [self._UF, self._US, self._UD, self._IN, 16 + ws,
                                                                      self._RDST + ws])
         with_dst = self.shuffle_with_dst
@@ -805,21 +821,20 @@ class SPVirtualSampler(_GraphReplay):
                                "batch holds; use chained=False for batches that differ this much between the ranks")
         send_sizes_cpu, recv_sizes_cpu = _native.sizes(send), _native.sizes(recv)
         n_nbr = num_dst * f
-        (unique_frontier, unique_src, arange_dst, a_src, a_dst, input_nodes, neighbors, sorted_all, packed, vir_src, ori_src,
-         unique_dst) = _native.fronts(
-            [b["unique_frontier"], b["unique_src"], b["arange_dst"], b["a_src"], b["a_dst"], b["input_nodes"], b["nbr"],
-             b["sorted_all"], b["packed"], b["vir_src"], b["ori_src"], b["unique_dst"]],
-            [n_uf, n_us, n_uf, n_recv, n_recv, n_in, n_nbr, n_nbr + (num_dst if with_dst else 0), n_nbr, n_recv, n_recv, n_ud])
-        blocks.insert(0, Block(_arange(n_uf, seeds.device), arange_dst, n_uf, num_dst, unique_frontier, f))
-        blocks.insert(0, Block(a_src, a_dst, n_us, n_ud, unique_src, f))
+        _native.cut(views, [n_uf, n_us, n_uf, n_recv, n_recv, n_in, n_nbr, n_nbr + (num_dst if with_dst else 0), n_nbr, n_recv,
+                            n_recv, n_ud, n_uf])
+        unique_frontier, _, _, _, _, input_nodes, neighbors, sorted_all, packed, vir_src, ori_src, unique_dst, _ = views
+        block1.num_src, block1.num_dst, block2.num_src, block2.num_dst = n_uf, num_dst, n_us, n_ud
+        blocks = [block2, block1, *hops.blocks]
         recv_dst = None
         if with_dst:
             packed = torch.cat((b["dst_sorted"][:num_dst], packed))
             recv_dst = b["recv_dst"][:n_rdst]
         self.last = dict(neighbors=neighbors, sorted_allnodes=sorted_all, unique_frontier=unique_frontier,
                          send_frontier=packed, recv_dst=recv_dst, vir_src=vir_src, ori_src=ori_src, unique_dst=unique_dst)
-        if b["rows"] is not None:
-            st.prefetched = (input_nodes, b["rows"][:n_in], plan)
+        if rows is not None:
+            _native.cut([rows], [n_in])
+            st.prefetched = (input_nodes, rows, plan)
         return input_nodes, seeds, blocks, send_sizes_cpu, recv_sizes_cpu
 
     def _outer(self, seeds, neighbors, fanout):
@@ -960,7 +975,10 @@ class MPSampler(_GraphReplay):
         recv_coo, _ = ex.allbroadcast_enqueue(coo_row.view(-1, 1), mine[2:3], words[64:64 + ws + 1])
         return dict(layers=layers, recv_frontier=recv_frontier, recv_coo=recv_coo)
 
-    def _finish(self, seeds, b, host=None, plan=None):
+    def _outline(self, seeds, b):
+        return _native.Hops(b["layers"], Block)
+
+    def _finish(self, seeds, b, host=None, plan=None, outline=None):
         """The one host read of the mini-batch, then everything is narrowed to its real size."""
         st = ops.STATE
         ws = st.world_size
@@ -968,7 +986,7 @@ class MPSampler(_GraphReplay):
         f = self.fanouts[0]
         if host is None:
             host = st.read_words()
-        blocks, n_dst = _native.narrow_blocks(host, seeds.numel(), b["layers"], Block)
+        n_dst, blocks = outline.fill(host, seeds.numel()), outline.blocks
         sizes = host[self._ALL:self._ALL + 3 * ws].view(ws, 3)
         sizes = torch.tensor(sizes.tolist(), dtype=torch.int64)        # off the pinned block
         recv_size = sizes[:, 0].contiguous()
