@@ -56,6 +56,7 @@ PROTOTYPES = {
     "apt_concat_row_ids": (c_int, [P, c_int64, P, P, c_int64, P, P, P, P, c_int64, c_int64, c_int64, P, P]),
     "apt_gather_workspace_bytes": (c_size_t, [c_int64]),
     "apt_gather_rows": (c_int, [P, c_int64, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P, c_size_t, P, P]),
+    "apt_gather_rows_beside": (c_int, [P, c_int64, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P, c_size_t, P, P]),
     "apt_gather_rows_from": (c_int, [P, c_int64, P, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P,
                                      c_size_t, P, P]),
     "apt_gather_static_max_rows": (c_int64, []),

@@ -179,7 +179,12 @@ struct GatherArgs {
   int32_t* status_word;
 };
 
-static int gather_launch(const GatherArgs& a, cudaStream_t s) {
+// Blocks an SM for a gather that runs beside other kernels: enough reads over the host link for its full rate (one block's
+// warps have 16 KiB each in flight, of the 80 KB that rate times latency asks of the whole chip), and room for the others,
+// which at the full grid wait until it ends.
+constexpr int kNarrowBlocks = 1;
+
+static int gather_launch(const GatherArgs& a, cudaStream_t s, bool narrow = false) {
   uint64_t bits = (uint64_t)a.dev_row_bytes | (uintptr_t)a.out;
   if (a.num_dev_rows > 0) bits |= (uintptr_t)a.dev_feats;
   if (a.num_uva_rows > 0) bits |= (uint64_t)a.uva_row_bytes | (uint64_t)a.uva_col_offset_bytes | (uintptr_t)a.uva_feats;
@@ -191,7 +196,8 @@ static int gather_launch(const GatherArgs& a, cudaStream_t s) {
   const int64_t all_warps = (int64_t)kNumSMs * 8 * (kGatherBlock / 32);
   int per = 32 / lpr;
   while (per < 32 && (int64_t)per * all_warps < a.num_rows) per <<= 1;
-  const int grid = wave_grid(ceil_div(a.num_rows, (int64_t)per * (kGatherBlock / 32)), 8, kGatherWaves);
+  int grid = wave_grid(ceil_div(a.num_rows, (int64_t)per * (kGatherBlock / 32)), 8, kGatherWaves);
+  if (narrow && grid > kNumSMs * kNarrowBlocks) grid = kNumSMs * kNarrowBlocks;
   ProfScope prof("gather_hit", s);
 #define APT_GATHER(V)                                                                                                     \
   APT_FOLLOW(k_gather<V>, grid, kGatherBlock, 0, s, a.index, a.num_rows, a.num_rows_dev, a.first_row_dev, a.feat_pos_map, \
@@ -278,6 +284,28 @@ extern "C" int apt_gather_rows_from(const int64_t* index, int64_t num_rows,
     return APT_ERR_CAPACITY;
   }
   return gather_launch(a, (cudaStream_t)stream);
+}
+
+extern "C" int apt_gather_rows_beside(const int64_t* index, int64_t num_rows,
+                                    const int64_t* num_rows_dev, const int64_t* feat_pos_map,
+                                    int64_t num_nodes, const void* dev_feats, int64_t num_dev_rows,
+                                    int64_t dev_row_bytes, const void* uva_feats,
+                                    int64_t num_uva_rows, int64_t uva_row_bytes,
+                                    int64_t uva_col_offset_bytes, void* out, void* workspace,
+                                    size_t workspace_bytes, int32_t* status_word, void* stream) {
+  using namespace apt;
+  const GatherArgs a{index, num_rows, num_rows_dev, nullptr, feat_pos_map, num_nodes, (const char*)dev_feats,
+                     num_dev_rows, dev_row_bytes, (const char*)uva_feats, num_uva_rows, uva_row_bytes,
+                     uva_col_offset_bytes, (char*)out, status_word};
+  const int rc = gather_check("apt_gather_rows", a);
+  if (rc != APT_OK || num_rows == 0) return rc;
+  APT_CHECK_ARG(workspace && ((uintptr_t)workspace & 255) == 0,
+                "apt_gather_rows: workspace must be non-null and 256-byte aligned");
+  if (workspace_bytes < apt_gather_workspace_bytes(num_rows)) {
+    set_error("apt_gather_rows: workspace %zu < %zu bytes", workspace_bytes, apt_gather_workspace_bytes(num_rows));
+    return APT_ERR_CAPACITY;
+  }
+  return gather_launch(a, (cudaStream_t)stream, true);
 }
 
 // The same without a workspace argument, for callers that must not allocate. The limit on the rows of a call dates from

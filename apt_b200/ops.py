@@ -792,10 +792,10 @@ def load_subtensor(node_id: torch.Tensor) -> torch.Tensor:
 
 
 def _gather_enqueue(node_id: torch.Tensor, n_dev: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
-                    first_dev: Optional[torch.Tensor] = None, ws_name: str = "gather") -> torch.Tensor:
+                    first_dev: Optional[torch.Tensor] = None, ws_name: str = "gather", beside: bool = False) -> torch.Tensor:
     """Enqueues the gather of rows [first_dev, n_dev) of node_id (device words; None: 0 and
     node_id.numel()) into `out` (allocated here when None). Calls that may overlap on the GPU
-    need workspaces of their own (`ws_name`)."""
+    need workspaces of their own (`ws_name`). `beside`: on a few blocks, beside other kernels."""
     f = STATE.feat
     n = node_id.numel()
     esz = f.dev_feats.element_size()
@@ -803,8 +803,10 @@ def _gather_enqueue(node_id: torch.Tensor, n_dev: Optional[torch.Tensor], out: O
         out = torch.empty((n, f.rank_feat_dim), dtype=f.dev_feats.dtype, device=node_id.device)
     nbytes = lib.apt_gather_workspace_bytes(n)
     ws = STATE.workspace(ws_name, nbytes)
-    check(lib.apt_gather_rows_from(
-        _ptr(node_id), n, _ptr(n_dev), _ptr(first_dev), _ptr(f.feat_pos_map), f.num_total_nodes,
+    launch, counts = (lib.apt_gather_rows_beside, (_ptr(n_dev),)) if beside else \
+        (lib.apt_gather_rows_from, (_ptr(n_dev), _ptr(first_dev)))
+    check(launch(
+        _ptr(node_id), n, *counts, _ptr(f.feat_pos_map), f.num_total_nodes,
         _ptr(f.dev_feats), f.dev_feats.shape[0], f.rank_feat_dim * esz,
         _ptr(f.uva_feats), f.uva_feats.shape[0], f.feat_dim * esz, f.feat_dim_offset * esz,
         _ptr(out), _ptr(ws), ws.numel(), STATE.status_ptr(), _stream()))

@@ -81,6 +81,13 @@ def create_block(seeds: torch.Tensor, neighbors: torch.Tensor, fanout: int) -> B
 _PREFETCH_LIMIT_BYTES = 6 << 30
 
 
+def _gather_split() -> int:
+    """APT_GATHER_SPLIT. 0: one gather of the input nodes' rows behind the sampling; 2 (default): those of the outermost
+    hop's destinations, which come first among them, are fetched on a second stream while that hop is sampled, and the two
+    gathers meet at the end; 1: they meet before the second one starts."""
+    return int(os.environ.get("APT_GATHER_SPLIT", "2"))
+
+
 def _fits_prefetch(rows: int) -> bool:
     f = ops.STATE.feat
     return f.feat_pos_map is not None and \
@@ -168,6 +175,27 @@ class _GraphReplay:
         if self.lanes > 1:
             return max(self.graph_buffers, self.lanes * self.plans_per_lane)
         return self.graph_buffers
+
+    def _early_rows(self, cur, cur_n, more):
+        """The rows of the outermost hop's destinations, fetched beside its sampling into a buffer for `more` further
+        rows; None where that is not done."""
+        st = ops.STATE
+        f = st.feat
+        if not (self.prefetch_features and _gather_split() and st.world_size == 1 and cur_n is not None and not st.profiling
+                and _fits_prefetch(cur.numel() + more)):
+            return None
+        rows = torch.empty((cur.numel() + more, f.rank_feat_dim), dtype=f.dev_feats.dtype, device=cur.device)
+        with st.beside(2):
+            ops._gather_enqueue(cur, cur_n, out=rows, ws_name="gather_frontier", beside=True)
+        return rows
+
+    def _late_rows(self, input_nodes, in_word, cur_n, rows):
+        """The rows of the input nodes, those behind the first cur_n when `rows` holds these already."""
+        if rows is None:
+            return ops._gather_enqueue(input_nodes, in_word)
+        ops._gather_enqueue(input_nodes, in_word, out=rows, first_dev=cur_n)
+        ops.STATE.join(2)
+        return rows
 
     def buffer_sets(self):
         """Buffer sets sample_iter really takes turns with: the number asked for, or fewer once the
@@ -408,12 +436,7 @@ class MixedNeighborSampler(_GraphReplay):
         self._init_replay(use_graph, graph_buffers, lanes)
         self.use_graph = self.use_graph and chained
         self.num_calls = self.num_layers
-        # 0 (default): one gather after the outermost hop; 1: the frontier's rows are gathered on a second
-        # stream beside the outermost hop and the two meet before the remaining rows are gathered; 2: they
-        # meet at the end. Measured on the papers-shaped run, 1 and 2 are slower (0.371 and 0.374 ms per
-        # mini-batch against 0.340): kernels that share SMs with the host-memory reads of the miss copy
-        # slow down by more than the overlap wins.
-        self.gather_split = int(os.environ.get("APT_GATHER_SPLIT", "0"))
+        self.gather_split = _gather_split()
 
     def sample(self, graph, seeds: torch.Tensor):
         if self.chained:
@@ -474,26 +497,22 @@ class MixedNeighborSampler(_GraphReplay):
         prefetch = self.prefetch_features and _fits_prefetch(uniq2.numel() * (1 + self.las_fanouts))
         split = self.gather_split if prefetch and not st.profiling else 0
         rows = None
-        side = None
         if prefetch:
             rows = torch.empty((uniq2.numel() * (1 + self.las_fanouts), f.rank_feat_dim), dtype=f.dev_feats.dtype,
                                device=uniq2.device)
         if split:
-            main = torch.cuda.current_stream()
-            side = st.side_stream()
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier")
+            with st.beside(2):
+                ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier", beside=True)
         uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
                                                      call if explicit else None, call_base_dev, look_up=prefetch)
-        if publish is not None and not split:
+        if publish is not None:
             publish()
         if split == 1:
-            main.wait_stream(side)
+            st.join(2)
         if prefetch:
             ops._gather_enqueue(uniq3, st.word(in_slot), out=rows, first_dev=st.word(u_slot) if split else None)
         if split == 2:
-            main.wait_stream(side)
+            st.join(2)
         return dict(layers=layers, perm=perm, inv=inv, rows=rows, u_slot=u_slot,
                     outer=_layer(uniq2, rel3, uniq3, self.las_fanouts, in_slot))
 
@@ -563,6 +582,7 @@ class SPGATSampler(_GraphReplay):
             cur, cur_n = uniq, cnt
             slot += 1
         f = self.fanouts[0]
+        rows = self._early_rows(cur, cur_n, min(cur.numel() * f, int(st.graph.num_total_nodes)))
         nbr = ops._sample(cur, f, cur_n, call if explicit else None, call_base_dev)
         n_word = None
         if cur_n is not None:
@@ -582,7 +602,7 @@ class SPGATSampler(_GraphReplay):
         input_nodes = ops.concat_ids(cur, cur_n, recv, recv_counts[ws:ws + 1], in_word, look_up=prefetch)
         if publish is not None:
             publish()
-        rows = ops._gather_enqueue(input_nodes, in_word) if prefetch else None
+        rows = self._late_rows(input_nodes, in_word, cur_n, rows) if prefetch else None
         return dict(layers=layers, outer=_layer(cur, arange_src, unique_neigh, f, self._U), perm=perm,
                     input_nodes=input_nodes, rows=rows)
 
@@ -688,6 +708,10 @@ class SPVirtualSampler(_GraphReplay):
         f = self.fanouts[0]
         s_max = cur.numel()
         n_max = s_max * f
+        lo, hi = ops._owned_range()
+        rows = None
+        if self.model != "GCN" and not with_dst:
+            rows = self._early_rows(cur, cur_n, min(n_max, max(hi - lo, 0)))
         nbr = ops._sample(cur, f, cur_n, call if explicit else None, call_base_dev)
         n_word = None
         if cur_n is not None:
@@ -755,7 +779,6 @@ class SPVirtualSampler(_GraphReplay):
         ori_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
         check(lib.apt_sp_unpack_frontier(ops._ptr(recv), recv.numel(), ops._ptr(total), n_total,
                                          ops._ptr(vir_src), ops._ptr(ori_src), ops._stream()))
-        lo, hi = ops._owned_range()
         with st.beside(1) if beside else contextlib.nullcontext():
             unique_dst, a_dst = ops._unique_enqueue(vir_src, total, 0, ws * ops.SP_BASE, st.word(self._UD), "unique_vdst")
         unique_src, a_src = ops._unique_enqueue(ori_src, total, lo, hi, st.word(self._US), "unique_sp_src")
@@ -780,7 +803,7 @@ class SPVirtualSampler(_GraphReplay):
         input_nodes = ops.concat_ids(head, head_n, unique_src, us_word, in_word, look_up=prefetch)
         if publish is not None:
             publish()
-        rows = ops._gather_enqueue(input_nodes, in_word) if prefetch else None
+        rows = self._late_rows(input_nodes, in_word, cur_n, rows) if prefetch else None
         return dict(layers=layers, cur=cur, nbr=nbr, sorted_all=sorted_all, packed=packed,
                     unique_frontier=unique_frontier, arange_dst=arange_dst, vir_src=vir_src, ori_src=ori_src,
                     unique_src=unique_src, a_src=a_src, unique_dst=unique_dst, a_dst=a_dst, dst_sorted=dst_sorted,

@@ -280,6 +280,15 @@ int apt_gather_rows(const int64_t* index, int64_t num_rows,
                     int64_t num_uva_rows, int64_t uva_row_bytes,
                     int64_t uva_col_offset_bytes, void* out, void* workspace,
                     size_t workspace_bytes, int32_t* status_word, void* stream);
+/* The same on a few blocks, to run beside other kernels on another stream. */
+int apt_gather_rows_beside(const int64_t* index, int64_t num_rows,
+                    const int64_t* num_rows_dev,
+                    const int64_t* feat_pos_map, int64_t num_nodes,
+                    const void* dev_feats, int64_t num_dev_rows,
+                    int64_t dev_row_bytes, const void* uva_feats,
+                    int64_t num_uva_rows, int64_t uva_row_bytes,
+                    int64_t uva_col_offset_bytes, void* out, void* workspace,
+                    size_t workspace_bytes, int32_t* status_word, void* stream);
 
 /* Gather for callers that cannot allocate device memory. No counterpart in the
  * reference, whose gather allocates its output and keeps no scratch.
