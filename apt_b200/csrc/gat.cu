@@ -31,7 +31,7 @@
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 48 + 116 + 5 us,
+// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 44 + 116 + 5 us,
 // where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 
@@ -264,17 +264,34 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
       const int64_t o = (int64_t)e * num_heads + h;
       t += weight[o] * dots[o];
     }
-#pragma unroll 4
-    for (int e = r.x; e < r.y; ++e) {
-      const int64_t o = (int64_t)e * num_heads + h, src = row[e];
-      const float w = weight[o];
-      const float gs = w * (dots[o] - t) * (Elem<T>::to_f(el[src * num_heads + h]) + bias > 0.f ? 1.f : slope);
-      ger += gs;
-      if (sums) {
-        if ((uint64_t)src < (uint64_t)num_src) atomicAdd(sums + src * num_heads + h, gs);
-      } else {
-        attn[o] = Elem<T>::from_f(w);
-        grad_score[o] = Elem<T>::from_f(gs);
+    // four edges' loads ahead of their adds (44 us; eight or sixteen take the registers of half the warps: 51, 81)
+    constexpr int C = 4;
+#pragma unroll 1
+    for (int e0 = r.x; e0 < r.y; e0 += C) {
+      int64_t src[C];
+      float w[C], dot[C], x[C];
+#pragma unroll
+      for (int k = 0; k < C; ++k) src[k] = row[min(e0 + k, r.y - 1)];
+#pragma unroll
+      for (int k = 0; k < C; ++k) {
+        const int64_t o = (int64_t)min(e0 + k, r.y - 1) * num_heads + h;
+        w[k] = weight[o];
+        dot[k] = dots[o];
+      }
+#pragma unroll
+      for (int k = 0; k < C; ++k) x[k] = Elem<T>::to_f(el[src[k] * num_heads + h]);
+#pragma unroll
+      for (int k = 0; k < C; ++k) {
+        if (e0 + k >= r.y) break;
+        const int64_t o = (int64_t)(e0 + k) * num_heads + h;
+        const float gs = w[k] * (dot[k] - t) * (x[k] + bias > 0.f ? 1.f : slope);
+        ger += gs;
+        if (sums) {
+          if ((uint64_t)src[k] < (uint64_t)num_src) atomicAdd(sums + src[k] * num_heads + h, gs);
+        } else {
+          attn[o] = Elem<T>::from_f(w[k]);
+          grad_score[o] = Elem<T>::from_f(gs);
+        }
       }
     }
     grad_er[i] = Elem<T>::from_f(ger);

@@ -105,11 +105,12 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned l
   // the one fanout that fits the sizes
   const uint32_t f = rows > 0 && E % rows == 0 ? (uint32_t)(E / rows) : 0u;
   uint32_t bits = f ? 0u : kNotFixed;
-  while (e0 < E) {
+  // edges that are not grouped need the counting sort whatever the others are
+  while (e0 < E && !(bits & kNotGrouped)) {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int64_t e = e0 + k * stride;
-      if (e >= E) break;
+      if (e >= E || (bits & kNotGrouped)) break;
       const int64_t d = ooff[st.nseg > 1 ? seg_of(coo, st.nseg, e) : 0] + c[k];
       if (f && d == (int64_t)((uint32_t)e / f)) continue;
       bits |= kNotFixed;
