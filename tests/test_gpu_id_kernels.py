@@ -34,6 +34,22 @@ def test_gather_rows_and_widths(dtype, dim):
         ops.check_status()
 
 
+
+@pytest.mark.parametrize("rows", [1, 1184, 37_889, 200_001])
+def test_gather_on_few_blocks(rows):
+    # fewer rows than its warps, one chunk more than they take at once, many
+    table, n_host, dim = 5000, 700, 36
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    cached = torch.randn((table, dim), device="cuda", generator=gen)
+    hosted = torch.randn((n_host, dim), device="cuda", generator=gen)
+    ops.cache_feats_shared(table + n_host, hosted.cpu().pin_memory(), cached, torch.arange(table),
+                           torch.arange(table, table + n_host), 0)
+    ids = torch.randint(0, table + n_host, (rows,), device="cuda", generator=gen)
+    got = ops._gather_enqueue(ids, torch.tensor([rows], device="cuda"), beside=True)
+    assert torch.equal(got, torch.cat([cached, hosted])[ids])
+    ops.check_status()
+
+
 def _patterns():
     rng = np.random.default_rng(8)
     for words in (7, 8, 9, 32):                        # level-0 words below one level-1 word
