@@ -31,7 +31,7 @@
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 44 + 116 + 5 us,
+// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 44 + 112 + 5 us,
 // where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 

@@ -15,8 +15,8 @@
 //   67 584 x 15 edges, fp32 x 256                    112 -> 87      148 -> 122     (1.04 GB: 12 TB/s out of L2 forward)
 //   53 000 x 15, fp32 x 192 / x 132                  77 -> 56, 67 -> 57    103 -> 86, 95 -> 86
 //   53 000 x 15, bf16 x 512 / x 264                  122 -> 84, 102 -> 83  161 -> 121, 126 -> 117
-//   16 000 x 15, fp32 x 256                          30 -> 26       66 -> 56
-//   67 584 x 15, weights, fp32 x 4 x 64              133 -> 129     215 -> 160
+//   16 000 x 15, fp32 x 256                          30 -> 26       66 -> 46
+//   67 584 x 15, weights, fp32 x 4 x 64              133 -> 129     215 -> 156
 // and against it: 9 000 x 15, fp32 x 256 13 -> 17 forward (the stream's start costs three dependent rounds), rows of
 // one slice a lane 44 -> 56 (fp32 x 128; an SM issues a copy every 13 ns whatever its size). Hence the rule of launch_bulk:
 // rows of more than 32 slices, 196 608 edges, and with weights only where edges are ordered.
@@ -274,9 +274,13 @@ k_spmm_bulk(const __grid_constant__ RowArgs<T> a, volatile int32_t* gave_up) {
     return true;
   };
 
+  // Items are dealt from the last warp on, since the first rows, often the longest, are the first warps', while an item is
+  // a large part of a warp's edges: 16 000 x 15 edges, fp32 x 256, reverse 56 -> 46 us; with weights 160 -> 156. Plain sums
+  // of a million edges keep the other order (125 against 128 us).
+  const bool from_last = kWeights || a.num_edges < (int64_t)2 * kItemEdges * warps;
   bool ok = true;
 #pragma unroll 1
-  for (int64_t first = warp; first < num_items && ok; first += (int64_t)32 * warps) {
+  for (int64_t first = from_last ? warps - 1 - warp : warp; first < num_items && ok; first += (int64_t)32 * warps) {
     const int64_t it = first + (int64_t)lane * warps;
     const int4 m = it < num_items ? a.ws.items[it] : make_int4(0, 0, 0, -1);
     ok = run(m.y, m.z - m.y, m.x, m.w);

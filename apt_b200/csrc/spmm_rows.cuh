@@ -246,7 +246,10 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   const int num_rows = (int)a.num_rows;
   const int warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int num_items = mode == kOrder ? min(*a.ws.num_items, (int)a.ws.max_items) : 0;
-  bool items = warp < num_items;                     // whole warps first take items ...
+  // whole warps first take items, dealt from the last warp on (the first rows, often the longest, are the first warps': rows
+  // of 32 bf16 columns in reverse 12.8 -> 9.1 us, of 4 x 64 with weights 115 -> 110) ...
+  int it = warps - 1 - warp;
+  bool items = it < num_items;
   // ... then groups of lanes take rows: lpr lanes, ep edges side by side
   int g_ep = items ? 32 / lpe : a.split.ep, g_lpr = lpe * g_ep, g_sub = lane & (g_lpr - 1), g_epi = g_sub / lpe;
   unsigned g_mask = g_lpr == 32 ? 0xffffffffu : (((1u << g_lpr) - 1u) << (lane - g_sub));
@@ -277,7 +280,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     }
   };
 
-  int it = warp, d = 0, G = 0;
+  int d = 0, G = 0;
   int b = 0, e = 0, nb = 0, ne = 0, part = -1;
   uint32_t src = 0, eid = 0, nsrc = 0, neid = 0;
   auto start_item = [&]() {
