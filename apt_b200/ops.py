@@ -118,9 +118,7 @@ class NPCState:
         self._tls = threading.local()
         self._lane_exchange = {}
         self._lane_streams = {}
-        # (input ids, gathered rows, plan or None) left by a sampler that gathers ahead; the rows of a plan may
-        # still be on their way on its stream
-        self.prefetched = None
+        self.prefetched = None  # _RowsAhead a sampler left for the next load_subtensor
         self._publish_seq = 0
         self._seq_lock = threading.Lock()
         self.generation = 0     # bumped whenever installed state changes; captured graphs check it
@@ -242,6 +240,35 @@ def _flag_text(flags):
 
 
 STATE = NPCState()
+
+
+def _version(t: torch.Tensor):
+    """PyTorch's count of the in-place changes of a tensor (inference tensors keep none)."""
+    return None if t.is_inference() else t._version
+
+
+def _tables_key():
+    """What a gather's rows depend on beside their ids: a gather enqueued under one key is good for as long as the key is the
+    same. Covers another feature table being installed and changes of an installed one that PyTorch knows of."""
+    f = STATE.feat
+    return STATE.generation, _version(f.dev_feats), _version(f.uva_feats)
+
+
+class _RowsAhead:
+    """Feature rows that a sampler gathered for `ids`, its input nodes, under `key`. `pending` (None: nothing to wait for)
+    orders a stream behind the gather."""
+
+    def __init__(self, ids, rows, key, pending):
+        self.ids, self.rows, self.key, self.pending = ids, rows, key, pending
+        self.version = _version(ids)
+
+    def serves(self, node_id) -> bool:
+        ids = self.ids
+        if self.key != _tables_key() or self.version != _version(ids):
+            return False
+        return ids is node_id or (ids.data_ptr() == node_id.data_ptr() and ids.numel() == node_id.numel()
+                                  and ids.dtype == node_id.dtype and node_id.is_contiguous())
+
 
 
 def _exchange():
@@ -778,15 +805,13 @@ def load_subtensor(node_id: torch.Tensor) -> torch.Tensor:
     f = STATE.feat
     if f.feat_pos_map is None:
         raise RuntimeError("cache_feats_shared has not been called")
-    pre = STATE.prefetched
-    if pre is not None:
+    ahead = STATE.prefetched
+    if ahead is not None:
         STATE.prefetched = None
-        ids, rows, plan = pre
-        if ids is node_id or (ids.data_ptr() == node_id.data_ptr() and ids.numel() == node_id.numel()
-                              and node_id.is_contiguous()):
-            if plan is not None:
-                plan.order_current_stream()
-            return rows
+        if ahead.serves(node_id):
+            if ahead.pending is not None:
+                ahead.pending.order_current_stream()
+            return ahead.rows
     return _native.gather(node_id, f.feat_pos_map, f.dev_feats, f.uva_feats, f.num_total_nodes, f.feat_dim_offset,
                           STATE.words())
 

@@ -106,6 +106,7 @@ class _Plan:
         self.keepalive = None
         self.host_words = None  # the batch's own copy of the word block, a sequence number behind it
         self.handle = None      # _native.Plan: launches the graph, waits for the counts, orders streams
+        self.rows_key = None    # ops._tables_key() of the last launch
         # the lane whose scratch the plan was built on; with more than one lane, the lane's stream
         self.lane = 0
         self.stream = None
@@ -197,6 +198,14 @@ class _GraphReplay:
         ops.STATE.join(2)
         return rows
 
+    @staticmethod
+    def _leave_rows(input_nodes, rows, plan):
+        """For the next load_subtensor: the rows of a replay (under the tables it was launched with; they may still be on
+        their way) or of an enqueue that the host has waited for."""
+        st = ops.STATE
+        key, pending = (ops._tables_key(), None) if plan is None else (plan.rows_key, plan.handle)
+        st.prefetched = ops._RowsAhead(input_nodes, rows, key, pending)
+
     def buffer_sets(self):
         """Buffer sets sample_iter really takes turns with: the number asked for, or fewer once the
         memory budget has cut a shape's ring."""
@@ -280,6 +289,8 @@ class _GraphReplay:
         st = ops.STATE
         base = st.sample_calls
         st.sample_calls += self.num_calls
+        if st.feat.feat_pos_map is not None:
+            plan.rows_key = ops._tables_key()
         plan.handle.launch(seeds, base)
 
     def _sample_chained(self, seeds: torch.Tensor):
@@ -394,13 +405,13 @@ class _GraphReplay:
         if plan.lane == 0:
             if flags:
                 st.check_flags(flags)
-            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle, outline)
+            return self._finish(seeds, plan.bufs, plan.host_words, plan, outline)
         st.lane = plan.lane
         try:
             if flags:
                 plan.handle.order_current_stream()
                 st.check_flags(flags)
-            return self._finish(seeds, plan.bufs, plan.host_words, plan.handle, outline)
+            return self._finish(seeds, plan.bufs, plan.host_words, plan, outline)
         finally:
             st.lane = 0
 
@@ -526,7 +537,7 @@ class MixedNeighborSampler(_GraphReplay):
         st = ops.STATE
         got, rows = outline.finish(st.read_words() if host is None else host)
         if rows is not None:
-            st.prefetched = (got[0], rows, plan)
+            self._leave_rows(got[0], rows, plan)
         return got
 
 
@@ -614,7 +625,7 @@ class SPGATSampler(_GraphReplay):
         st = ops.STATE
         got, rows = outline.finish(st.read_words() if host is None else host)
         if rows is not None:
-            st.prefetched = (got[0], rows, plan)
+            self._leave_rows(got[0], rows, plan)
         return got
 
     def sample(self, graph, seeds: torch.Tensor):
@@ -857,7 +868,7 @@ class SPVirtualSampler(_GraphReplay):
                          send_frontier=packed, recv_dst=recv_dst, vir_src=vir_src, ori_src=ori_src, unique_dst=unique_dst)
         if rows is not None:
             _native.cut([rows], [n_in])
-            st.prefetched = (input_nodes, rows, plan)
+            self._leave_rows(input_nodes, rows, plan)
         return input_nodes, seeds, blocks, send_sizes_cpu, recv_sizes_cpu
 
     def _outer(self, seeds, neighbors, fanout):
@@ -1106,5 +1117,5 @@ class DPNeighborSampler:
         if flags:
             st.check_flags(flags)
         if rows is not None:
-            st.prefetched = (input_nodes, rows, None)
+            st.prefetched = ops._RowsAhead(input_nodes, rows, ops._tables_key(), None)
         return input_nodes, seeds, blocks

@@ -1,0 +1,96 @@
+"""Rows that a sampler gathered ahead: load_subtensor hands them out only while the tables and the ids they were gathered
+for are what they were. Rows are copied bytes: compared bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+import apt_b200
+from apt_b200 import ops
+from tests.gpu_util import dev, install_graph, reset_world
+from tests.helpers import small_graph
+from tests.test_gpu_counts_first import MAKE
+
+pytestmark = pytest.mark.gpu
+I64 = np.int64
+
+
+def _table(n, scale, dim=24):
+    """A feature table of its own, half of it cached: (table, what is to be kept alive)."""
+    table = (torch.arange(n, dtype=torch.float32, device="cuda")[:, None] + torch.zeros(dim, device="cuda")) * scale
+    cached, hosted = torch.arange(n)[::2], torch.arange(n)[1::2]
+    parts = table[hosted.cuda()].cpu().pin_memory(), table[cached.cuda()]
+    ops.cache_feats_shared(n, parts[0], parts[1], cached, hosted, 0)
+    return table, parts
+
+
+def _install():
+    n, indptr, indices = small_graph(scale=12, edge_factor=8)
+    install_graph(indptr, indices)
+    reset_world(1, 0)
+    ops.register_min_vids(torch.tensor([0, n]))
+    return n
+
+
+def _seeds(n, seed=2, count=300):
+    return dev(np.random.default_rng(seed).permutation(n)[:count].astype(I64))
+
+
+@pytest.mark.parametrize("kind", sorted(MAKE))
+def test_another_table_is_read(kind):
+    n = _install()
+    old = _table(n, 1.0)
+    smp = MAKE[kind]([6, 4])
+    for _ in range(2):                      # the first pass of a shape, and a replay
+        got = smp.sample(None, _seeds(n))
+        new = _table(n, -3.0)
+        assert torch.equal(ops.load_subtensor(got[0]), new[0][got[0]])
+        old = _table(n, 1.0)
+    ops.check_status()
+    del old
+
+
+@pytest.mark.parametrize("kind", sorted(MAKE))
+def test_changes_in_place_are_read(kind):
+    n = _install()
+    table, (host, cached) = _table(n, 1.0)
+    smp = MAKE[kind]([6, 4])
+    for _ in range(2):
+        got = smp.sample(None, _seeds(n))
+        cached.mul_(2)
+        table[::2] *= 2
+        assert torch.equal(ops.load_subtensor(got[0]), table[got[0]])
+        got = smp.sample(None, _seeds(n))
+        torch.cuda.synchronize()
+        host.add_(1)
+        table[1::2] += 1
+        assert torch.equal(ops.load_subtensor(got[0]), table[got[0]])
+        got = smp.sample(None, _seeds(n))
+        torch.cuda.synchronize()
+        got[0].copy_(got[0].flip(0))
+        assert torch.equal(ops.load_subtensor(got[0]), table[got[0]])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("kind", ["np", "snp_gat", "sage"])
+def test_batches_in_flight_meet_another_table(kind):
+    n = _install()
+    old = _table(n, 1.0)
+    it = MAKE[kind]([6, 4]).sample_iter(None, [_seeds(n, k) for k in range(6)])
+    got = next(it)
+    assert torch.equal(ops.load_subtensor(got[0]), old[0][got[0]])
+    new = _table(n, 5.0)                    # the batches launched by now were gathered from the old one
+    for got in it:
+        assert torch.equal(ops.load_subtensor(got[0]), new[0][got[0]])
+    ops.check_status()
+
+
+def test_rows_ahead_are_used_when_nothing_changed():
+    n = _install()
+    table, _ = _table(n, 1.0)
+    for kind in ("np", "dp", "sage"):
+        got = MAKE[kind]([6, 4]).sample(None, _seeds(n))
+        rows = ops.STATE.prefetched.rows
+        assert ops.load_subtensor(got[0]).data_ptr() == rows.data_ptr()
+        got = MAKE[kind]([6, 4]).sample(None, _seeds(n))
+        assert torch.equal(ops.load_subtensor(got[0].view(-1)), table[got[0]])
+    ops.check_status()
