@@ -1063,8 +1063,8 @@ class DPNeighborSampler:
 
     chained            enqueue the whole mini-batch with device-side sizes and one host read (one C++ call; every result
                        is a tensor of its own) instead of one read per hop
-    prefetch_features  also enqueue the feature gather of the input nodes behind that read; the next
-                       ops.load_subtensor(input_nodes) returns it"""
+    prefetch_features  also enqueue the feature gather of the input nodes, right after that read; the next
+                       ops.load_subtensor(input_nodes) returns it, on whichever stream it is called"""
 
     def __init__(self, rank: int, fanouts: List[int], chained: bool = None, prefetch_features: bool = True):
         self.rank = rank
@@ -1110,12 +1110,14 @@ class DPNeighborSampler:
         call = st.sample_calls
         st.sample_calls += len(order)
         words = st.words()
-        input_nodes, blocks, rows, flags = _native.dp_sample(
+        key = ops._tables_key() if features is not None else None
+        blocks, rows, pending, flags = _native.dp_sample(
             ids, order, g.adj_pos_map, g.num_total_nodes, g.dev_indptr, g.dev_indices, g.uva_indptr, g.uva_indices, st.sample_key,
             call, ops._relabel_workspace(bound), words, st._lane_words[st.lane][1], st.next_sequence(), features,
             _PREFETCH_LIMIT_BYTES, Block)
         if flags:
             st.check_flags(flags)
+        input_nodes = blocks[0].src_ids
         if rows is not None:
-            st.prefetched = ops._RowsAhead(input_nodes, rows, ops._tables_key(), None)
+            st.prefetched = ops._RowsAhead(input_nodes, rows, key, pending)
         return input_nodes, seeds, blocks

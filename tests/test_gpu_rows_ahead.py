@@ -94,3 +94,48 @@ def test_rows_ahead_are_used_when_nothing_changed():
         got = MAKE[kind]([6, 4]).sample(None, _seeds(n))
         assert torch.equal(ops.load_subtensor(got[0].view(-1)), table[got[0]])
     ops.check_status()
+
+
+def _wide_host_table(n, dim):
+    """Rows of several KiB in host memory: a gather of some thousands of them is still running when sample() returns."""
+    host = (torch.arange(n, dtype=torch.float32)[:, None] + torch.zeros(dim)).pin_memory()
+    ops.cache_feats_shared(n, host, host[:1].cuda(), torch.arange(1), torch.arange(n), 0)
+    return host
+
+
+@pytest.mark.parametrize("fanouts", [[10], [6, 4]])
+def test_data_parallel_rows_on_another_stream(fanouts):
+    # the rows are ordered behind their gather, and operators on other streams do not change how many there are
+    n = _install()
+    host = _wide_host_table(n, 1024)
+    smp = apt_b200.DPNeighborSampler(0, fanouts)
+    other = torch.cuda.Stream()
+    few = torch.arange(3, device="cuda")
+    for k in range(6):
+        seeds = _seeds(n, k, 2000)
+        torch.empty(4096 * 1024, device="cuda").fill_(-1.0)         # rows not written yet show
+        torch.cuda.synchronize()
+        got = smp.sample(None, seeds)
+        with torch.cuda.stream(other):
+            if k % 2:
+                ops.relabel_csc(few, few)                           # leaves its own count in the shared words
+            rows = ops.load_subtensor(got[0])
+            seen = rows[:, ::512].clone()
+        other.synchronize()
+        ids = got[0].cpu()
+        assert len(ids) > 2000 and torch.equal(seen.cpu(), host[ids][:, ::512])
+    ops.check_status()
+
+
+def test_data_parallel_batches_hold_what_they_consist_of():
+    n = _install()                          # 4096 nodes: three hops meet the same ones again and again
+    _table(n, 1.0, dim=256)
+    got = apt_b200.DPNeighborSampler(0, [15, 15, 15]).sample(None, _seeds(n, 0, 256))
+    rows = ops.load_subtensor(got[0])
+    assert got[0] is got[2][0].src_ids
+    held = [(rows.untyped_storage().nbytes(), rows.numel() * 4 + 512)]
+    for b in got[2]:
+        held += [(t.untyped_storage().nbytes(), 2 * t.numel() * 8 + (1 << 20)) for t in (b.coo_row, b.coo_col, b.src_ids)]
+        assert torch.equal(b.coo_col, torch.arange(b.num_dst, device="cuda").repeat_interleave(15))
+    assert all(size <= most for size, most in held), held
+    ops.check_status()
