@@ -34,6 +34,7 @@ PROTOTYPES = {
     "apt_launch_count_reset": (None, []),
     "apt_memcpy_async": (c_int, [P, P, c_size_t, P]),
     "apt_publish_words": (c_int, [P, c_int, P, c_int64, P, P]),
+    "apt_publish_words_from": (c_int, [P, c_int, P, P, c_int64, P, P]),
     "apt_stage_replay": (c_int, [P, c_int64, P, c_int64, c_int64, P, P]),
     "apt_wait_published": (c_int, [P, c_int, c_int64, P]),
     "apt_set_tunable": (c_int, [c_char_p, c_int64]),

@@ -70,11 +70,11 @@ ProfScope::~ProfScope() {
 // The word block goes to page-locked host memory, a sequence number behind it last: the host polls for that, which
 // takes the place of a copy, an event and a wake-up.
 __global__ void __launch_bounds__(256)
-k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __restrict__ sequence_dev, int64_t sequence,
-                volatile int64_t* host) {
+k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __restrict__ last, const int64_t* __restrict__ sequence_dev,
+                int64_t sequence, volatile int64_t* host) {
   wait_for_previous();
   if (threadIdx.x == 0 && sequence_dev) sequence = *sequence_dev;
-  for (int t = threadIdx.x; t < count; t += blockDim.x) host[t] = words[t];
+  for (int t = threadIdx.x; t < count; t += blockDim.x) host[t] = last && t == count - 1 ? *last : words[t];
   __threadfence_system();
   __syncthreads();
   if (threadIdx.x == 0) host[count] = sequence;
@@ -97,9 +97,14 @@ extern "C" {
 
 int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_dev, int64_t sequence, int64_t* host,
                       void* stream) {
+  return apt_publish_words_from(words, count, nullptr, sequence_dev, sequence, host, stream);
+}
+
+int apt_publish_words_from(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev, int64_t sequence,
+                           int64_t* host, void* stream) {
   using namespace apt;
   APT_CHECK_ARG(words && host && count >= 0 && count <= 4096, "apt_publish_words: bad argument");
-  APT_FOLLOW(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, sequence_dev, sequence, host);
+  APT_FOLLOW(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, last, sequence_dev, sequence, host);
   return APT_OK;
 }
 

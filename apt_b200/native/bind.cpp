@@ -258,13 +258,15 @@ struct GatFunction : public torch::autograd::Function<GatFunction> {
 };
 
 // ------------------------------------------------------------------------------------------------ samplers
-// Copies the word block to the host (one kernel, polled for) and returns its status flags.
-int64_t read_words(const Tensor& words, const Tensor& host, int64_t sequence) {
+// Copies a word block to the host (one kernel, polled for), the last word, the status flags, from the end of `status`, and
+// returns the flags.
+int64_t read_words(const Tensor& words, const Tensor& status, const Tensor& host, int64_t sequence) {
   const int count = (int)words.numel();
   void* const s = stream();
   int64_t* const h = host.mutable_data_ptr<int64_t>();
   py::gil_scoped_release nogil;
-  check(apt_publish_words(words.const_data_ptr<int64_t>(), count, nullptr, sequence, h, s));
+  check(apt_publish_words_from(words.const_data_ptr<int64_t>(), count, status.const_data_ptr<int64_t>() + status.numel() - 1, nullptr,
+                               sequence, h, s));
   check(apt_wait_published(h, count, sequence, s));
   return h[count - 1] & 0xffffffff;
 }

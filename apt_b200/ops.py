@@ -186,7 +186,23 @@ class NPCState:
 
     def words(self) -> torch.Tensor:
         """int64[256] device words: [0..254] small results (counts a kernel leaves for
-        the next kernel and, later, for the host), [255] status flags."""
+        the next kernel and, later, for the host), [255] status flags. Inside own_words() the small results are in
+        a block of the caller's."""
+        own = getattr(self._tls, "words", None)
+        return self.lane_words() if own is None else own
+
+    @contextlib.contextmanager
+    def own_words(self, words: torch.Tensor):
+        """Small results of the block's operators go to `words`; status flags stay in the lane's block. For operators that
+        are still reading their counts when others have begun to write theirs."""
+        self._tls.words = words
+        try:
+            yield
+        finally:
+            self._tls.words = None
+
+    def lane_words(self) -> torch.Tensor:
+        """The word block of the calling thread's lane, its status flags among them."""
         pair = self._lane_words.get(self.lane)
         if pair is None or pair[0].device != self.device():
             pair = (torch.zeros(self.NUM_WORDS, dtype=torch.int64, device=self.device()),
@@ -199,14 +215,14 @@ class NPCState:
         return self.words()[k:k + 1]
 
     def status_ptr(self):
-        return ctypes.c_void_p(self.words().data_ptr() + 8 * (self.NUM_WORDS - 1))
+        return ctypes.c_void_p(self.lane_words().data_ptr() + 8 * (self.NUM_WORDS - 1))
 
     def read_words(self) -> torch.Tensor:
         """Copies the device words to the host (one stream sync) and raises on
         any status flag except zero-degree, which is only a notice."""
-        w = self.words()
+        status = self.lane_words()
         host = self._lane_words[self.lane][1]
-        self.check_flags(_native.read_words(w, host, self.next_sequence()))
+        self.check_flags(_native.read_words(self.words(), status, host, self.next_sequence()))
         return host
 
     def next_sequence(self) -> int:
@@ -221,7 +237,7 @@ class NPCState:
 
     def check_flags(self, flags: int):
         if flags & ~_lib.FLAG_ZERO_DEGREE:
-            self.words()[self.NUM_WORDS - 1] = 0
+            self.lane_words()[self.NUM_WORDS - 1] = 0
             raise RuntimeError(f"apt_b200 device status flags 0x{flags:x}: " + _flag_text(flags))
 
 

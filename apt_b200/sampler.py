@@ -104,7 +104,10 @@ class _Plan:
         self.graph = None
         self.generation = -1
         self.keepalive = None
-        self.host_words = None  # the batch's own copy of the word block, a sequence number behind it
+        # The batch's own counts, on the device and, a sequence number behind them, on the host: the gather of its rows still
+        # reads them when the mini-batch has been handed out and another one, on another stream, writes its own.
+        self.words = None
+        self.host_words = None
         self.handle = None      # _native.Plan: launches the graph, waits for the counts, orders streams
         self.rows_key = None    # ops._tables_key() of the last launch
         # the lane whose scratch the plan was built on; with more than one lane, the lane's stream
@@ -232,6 +235,7 @@ class _GraphReplay:
         plan.generation = st.generation
         plan.seeds_buf = torch.empty(seeds.numel(), dtype=torch.int64, device=dev)
         plan.seeds_buf.copy_(seeds)
+        plan.words = torch.zeros(st.NUM_WORDS, dtype=torch.int64, device=dev)
         plan.host_words = torch.zeros(st.NUM_WORDS + 1, dtype=torch.int64).pin_memory()
         if on_lanes:
             # lane 0 stays with the caller: its exchange context also carries the feature shuffles
@@ -241,28 +245,8 @@ class _GraphReplay:
             torch.cuda.synchronize()     # no other lane's mini-batch is in flight while this one is built
         st.lane = plan.lane
         try:
-            base_dev = st.word(_CALL_BASE_SLOT)
-            # one eager run first: it sizes the cached workspaces and surfaces errors outside capture
-            bufs = self._enqueue(plan.seeds_buf, base_dev)
-            st.read_words()
-            st.prefetched = None
-            del bufs
-            plan.graph = torch.cuda.CUDAGraph()
-            replay_in = st.words()[_CALL_BASE_SLOT:_CALL_BASE_SLOT + 2]
-            published = []
-
-            def publish():
-                published.append(True)
-                check(lib.apt_publish_words(ops._ptr(st.words()), st.NUM_WORDS, ops._ptr(replay_in[1:2]), 0,
-                                            ops._ptr(plan.host_words), ops._stream()))
-
-            with torch.cuda.graph(plan.graph):
-                plan.bufs = self._enqueue(plan.seeds_buf, base_dev, publish)
-                if not published:
-                    publish()
-            plan.handle = _native.Plan(plan.graph.raw_cuda_graph_exec(), plan.seeds_buf, replay_in, plan.host_words,
-                                       plan.stream.cuda_stream if on_lanes else 0)
-            plan.keepalive = [v for k, v in st._ws.items() if k[2] == plan.lane]
+            with st.own_words(plan.words):
+                self._build(plan, on_lanes)
         finally:
             st.lane = 0
         ring.plans[i] = plan
@@ -281,6 +265,32 @@ class _GraphReplay:
                 del ring.plans[fit:]
         plan.ring_size = len(ring.plans)
         return plan
+
+    def _build(self, plan, on_lanes):
+        """Captures `plan`'s graph on the calling thread's lane and word block."""
+        st = ops.STATE
+        base_dev = st.word(_CALL_BASE_SLOT)
+        # one eager run first: it sizes the cached workspaces and surfaces errors outside capture
+        bufs = self._enqueue(plan.seeds_buf, base_dev)
+        st.read_words()
+        st.prefetched = None
+        del bufs
+        plan.graph = torch.cuda.CUDAGraph()
+        replay_in = plan.words[_CALL_BASE_SLOT:_CALL_BASE_SLOT + 2]
+        published = []
+
+        def publish():
+            published.append(True)
+            check(lib.apt_publish_words_from(ops._ptr(plan.words), st.NUM_WORDS, st.status_ptr(), ops._ptr(replay_in[1:2]), 0,
+                                             ops._ptr(plan.host_words), ops._stream()))
+
+        with torch.cuda.graph(plan.graph):
+            plan.bufs = self._enqueue(plan.seeds_buf, base_dev, publish)
+            if not published:
+                publish()
+        plan.handle = _native.Plan(plan.graph.raw_cuda_graph_exec(), plan.seeds_buf, replay_in, plan.host_words,
+                                   plan.stream.cuda_stream if on_lanes else 0)
+        plan.keepalive = [v for k, v in st._ws.items() if k[2] == plan.lane] + [st.lane_words()]
 
     def _replay(self, plan, seeds):
         """Enqueues one replay of `plan` for `seeds`: on the current stream, or, with lanes, on the plan's own

@@ -78,6 +78,9 @@ int apt_memcpy_async(void* dst, const void* src, size_t nbytes, void* stream);
  * stream without an answer, ends the wait with a status. host holds count + 1 words. */
 int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_dev,
                       int64_t sequence, int64_t* host, void* stream);
+/* The same with the last word taken from *last instead (counts of one block, status flags of another); NULL: from words. */
+int apt_publish_words_from(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev,
+                           int64_t sequence, int64_t* host, void* stream);
 int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream);
 /* The inputs of a captured mini-batch in one kernel: copies the seeds (device memory) into the buffer
  * the graph reads and writes words[0] = call_base, words[1] = sequence. */

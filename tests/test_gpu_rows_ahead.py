@@ -139,3 +139,23 @@ def test_data_parallel_batches_hold_what_they_consist_of():
         assert torch.equal(b.coo_col, torch.arange(b.num_dst, device="cuda").repeat_interleave(15))
     assert all(size <= most for size, most in held), held
     ops.check_status()
+
+
+@pytest.mark.parametrize("kind", ["np", "snp_gat", "sage", "gcn", "sage_dst"])
+def test_a_batch_keeps_its_counts_to_itself(kind):
+    # the gather behind a replay reads its counts when other operators, on other streams, may be writing theirs
+    n = _install()
+    table, _ = _table(n, 1.0)
+    smp = MAKE[kind]([6, 4])
+    smp.sample(None, _seeds(n))
+    ops.check_status()
+    words = ops.STATE.words()
+    words[:-1].fill_(-7)
+    got = smp.sample(None, _seeds(n, 3))
+    assert bool((words[:-1] == -7).all()) and int(words[-1]) & ~4 == 0
+    assert torch.equal(ops.load_subtensor(got[0]), table[got[0]])
+    # flags of operators outside the replay are still raised by it
+    ops.STATE.lane_words()[-1] = 32
+    with pytest.raises(RuntimeError, match="not grouped"):
+        smp.sample(None, _seeds(n, 3))
+    ops.check_status()
