@@ -22,6 +22,7 @@ APT_OK, APT_ERR_BAD_ARG, APT_ERR_CUDA, APT_ERR_TIMEOUT, APT_ERR_OOB, APT_ERR_CAP
 FLAG_ID_OUT_OF_RANGE, FLAG_FEAT_NOT_EXIST, FLAG_ZERO_DEGREE, FLAG_TABLE_FULL, FLAG_PEER_TIMEOUT = 1, 2, 4, 8, 16
 FLAG_NOT_GROUPED = 32
 FLAG_SIZE_MISMATCH = 64
+FLAG_COPY_TIMEOUT = 128
 F32, BF16, F16 = 0, 1, 2
 IPC_HANDLE_BYTES = 64
 
@@ -37,6 +38,7 @@ PROTOTYPES = {
     "apt_publish_words_from": (c_int, [P, c_int, P, P, c_int64, P, P]),
     "apt_stage_replay": (c_int, [P, c_int64, P, c_int64, c_int64, P, P]),
     "apt_wait_published": (c_int, [P, c_int, c_int64, P]),
+    "apt_pending_flags": (c_int, []),
     "apt_set_tunable": (c_int, [c_char_p, c_int64]),
     "apt_profile_enable": (c_int, [c_int]),
     "apt_profile_read": (c_int, [c_char_p, ctypes.POINTER(c_double), ctypes.POINTER(c_int64)]),

@@ -80,6 +80,7 @@ struct ProfScope {
   } while (0)
 
 void set_relabel_small(bool on);   // relabel.cu: one-block shared-memory path for small layers
+void set_bulk_wait_polls(int polls);   // spmm.cu: bound of k_spmm_bulk's waits
 
 constexpr int kNumSMs = 148;  // B200: 2 dies x 74 SMs
 

@@ -393,7 +393,7 @@ static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* 
   SpmmWs ws{};
   ws.range = g.range;
   const RowArgs<T> a{q.row, (const T*)q.ft, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, ws,
-                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none};
+                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status};
   ProfScope prof("gat_rows", s);
   return launch_spmm_rows<T>(kUMulW, a, s);
 }
@@ -442,7 +442,7 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
   int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, ws.sort, split.long_edges, nullptr, nullptr, grad_er, s);
   if (rc != APT_OK) return rc;
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, st, num_src, q.E, ws.sort,
-                     (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr};
+                     (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr, q.status};
   ProfScope prof("spmm_rows", s);
   rc = launch_spmm_rows<T>(kUMulW, a, s);
   if (rc != APT_OK) return rc;

@@ -244,6 +244,10 @@ extern "C" int apt_set_tunable(const char* name, int64_t value) {
     set_relabel_small(value != 0);
     return APT_OK;
   }
+  if (!strcmp(name, "bulk_wait_polls") && value >= 0 && value <= 1 << 20) {
+    set_bulk_wait_polls((int)value);
+    return APT_OK;
+  }
   set_error("apt_set_tunable: unknown name or bad value: %s = %lld", name, (long long)value);
   return APT_ERR_BAD_ARG;
 }

@@ -12,6 +12,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <mutex>
 
@@ -62,8 +63,6 @@ size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) 
   }
   return at;
 }
-
-int bulk_gave_up(int32_t** word);   // spmm_bulk.cuh
 
 // ---- the probe -------------------------------------------------------------------------
 constexpr uint32_t kNotGrouped = 1u, kNotFixed = 2u, kHasLong = 4u;
@@ -196,22 +195,39 @@ static void give_slot(int slot) {
   g_probe.cv.notify_one();
 }
 
-int bulk_gave_up(int32_t** word) {
+// Where kernels without a status word of their caller leave flags: mapped memory, made by the first call that may need it.
+static std::atomic<int32_t*> g_pending{nullptr};
+
+int pending_word(int32_t** word) {
   static std::mutex mu;
-  static int32_t* mapped = nullptr;
+  *word = g_pending.load(std::memory_order_acquire);
+  if (*word) return APT_OK;
   std::lock_guard<std::mutex> lk(mu);
-  if (!mapped) {
+  if (!g_pending.load()) {
     void* p = nullptr;
     APT_CUDA(cudaHostAlloc(&p, 64, cudaHostAllocMapped | cudaHostAllocPortable));
     *(int32_t*)p = 0;
-    mapped = (int32_t*)p;
+    g_pending.store((int32_t*)p, std::memory_order_release);
   }
-  *word = mapped;
-  if (*(volatile int32_t*)mapped == 0) return APT_OK;
-  *(volatile int32_t*)mapped = 0;
-  set_error("spmm: a row's copy to shared memory did not complete in an earlier call");
+  *word = g_pending.load();
+  return APT_OK;
+}
+
+static int32_t take_pending() {
+  int32_t* const word = g_pending.load(std::memory_order_acquire);
+  return word && *(volatile int32_t*)word ? __atomic_exchange_n(word, 0, __ATOMIC_ACQ_REL) : 0;
+}
+
+// Sums that came out wrong are reported by the next call that sums, whatever its size.
+static int check_pending(const char* who) {
+  if (!take_pending()) return APT_OK;
+  set_error("%s: in an earlier call input rows did not reach shared memory in time; some of its sums are zero", who);
   return APT_ERR_TIMEOUT;
 }
+
+static std::atomic<int> g_bulk_wait_polls{kBulkWaitPolls};
+void set_bulk_wait_polls(int polls) { g_bulk_wait_polls = polls; }
+int bulk_wait_polls() { return g_bulk_wait_polls; }
 
 // Polls a mapped word until it carries `sequence`. The stream is asked now and then, so that an error on it ends the wait.
 static int wait_for(const volatile int64_t* word, int64_t sequence, cudaStream_t s) {
@@ -476,7 +492,7 @@ static int run_rows(int op, const RowSplit& split, const int64_t* row, int64_t E
                     int64_t edata_dim, int64_t feat_dim, SegTable st, int64_t num_rows, const SpmmWs& ws, int mode, int fixed,
                     void* out, cudaStream_t s) {
   const RowArgs<T> a{row, (const T*)in, (const T*)edata, edata_dim, feat_dim, st, num_rows, E, ws, (T*)out,
-                     mode, fixed, split, (int)feat_dim, nullptr};
+                     mode, fixed, split, (int)feat_dim, nullptr, nullptr};
   ProfScope prof("spmm_rows", s);
   return launch_spmm_rows<T>(op, a, s);
 }
@@ -536,6 +552,8 @@ static int spmm_check(const char* who, int op, int dtype, int64_t num_edges, int
 
 }  // namespace apt
 
+extern "C" int32_t apt_pending_flags(void) { return apt::take_pending(); }
+
 extern "C" size_t apt_spmm_workspace_bytes(int64_t num_out_rows, int64_t num_edges) {
   if (num_out_rows < 0 || num_edges < 0) return 0;
   return apt::spmm_layout(num_out_rows, num_edges, nullptr, nullptr);
@@ -555,11 +573,13 @@ extern "C" int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges, const i
   APT_CUDA(cudaStreamIsCapturing(s, &capturing));
   APT_CHECK_ARG(capturing == cudaStreamCaptureStatusNone,
                 "apt_spmm_probe: the number of output rows is read on the host, which a stream capture does not allow");
+  int rc = check_pending("apt_spmm_probe");
+  if (rc != APT_OK) return rc;
   int dev = 0, slot = -1;
   APT_CUDA(cudaGetDevice(&dev));
   APT_CHECK_ARG(dev < 64, "apt_spmm_probe: device %d", dev);
   int64_t sequence = 0;
-  int rc = take_slot(dev, &slot, &sequence);
+  rc = take_slot(dev, &slot, &sequence);
   if (rc != APT_OK) return rc;
   int64_t* host = g_probe.host + slot * 8;
   SegTable st{coo_offset, nullptr, output_offset, num_segments};
@@ -586,7 +606,8 @@ extern "C" int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row, con
                                   int num_segments, int64_t num_out_rows, int mode, int fixed, void* out,
                                   void* workspace, size_t workspace_bytes, void* stream) {
   using namespace apt;
-  const int rc = spmm_check("apt_spmm_sum", op, dtype, num_edges, &edata_dim, feat_dim, num_segments, num_out_rows);
+  int rc = spmm_check("apt_spmm_sum", op, dtype, num_edges, &edata_dim, feat_dim, num_segments, num_out_rows);
+  if (rc == APT_OK && mode == kDevice) rc = check_pending("apt_spmm_sum");
   if (rc != APT_OK) return rc;
   APT_CHECK_ARG(mode >= kDevice && mode <= kOrder, "apt_spmm_sum: mode %d", mode);
   APT_CHECK_ARG(mode != kFixed || (fixed >= 0 && (int64_t)fixed * num_out_rows == num_edges),

@@ -31,8 +31,6 @@ constexpr int kBulkWarps = 12, kBulkStages = 2;
 // 80 registers; weights need more.
 constexpr int bulk_group(int op) { return op == kCopyU ? 4 : 8; }
 constexpr int bulk_blocks(int op) { return op == kCopyU ? 2 : 1; }
-constexpr int kBulkWaitLimit = 1 << 20;      // polls of an mbarrier, each of which may suspend for a while itself
-
 constexpr int kBulkMinSlices = 33, kBulkMinEdges = 3 << 16;
 constexpr int kBulkHeads = 16;               // weights an edge can bring along
 constexpr int kBulkVpl = 2;                  // 16-byte slices a lane
@@ -54,9 +52,10 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (int k = 0; k < kBulkWaitLimit; ++k)
-    if (mbar_try(bar, parity)) return true;
+// By all lanes of a warp, which agree on the answer.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int polls) {
+  for (int k = 0; k < polls; ++k)
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
   return false;
 }
 // `bytes` and both addresses are multiples of 16.
@@ -100,10 +99,12 @@ struct BulkRing {
   }
   __device__ __forceinline__ const unsigned char* group() const { return slots + taken % kBulkStages * GE * kBulkSlot; }
   __device__ __forceinline__ const float* group_weights() const { return weights + taken % kBulkStages * GE * kBulkHeads; }
-  __device__ __forceinline__ bool wait() const { return mbar_wait(bars + taken % kBulkStages, (uint32_t)(taken / kBulkStages) & 1u); }
-  // Copies that nobody will read: the block may go once they are done.
+  __device__ __forceinline__ bool wait(int polls) const {
+    return mbar_wait(bars + taken % kBulkStages, (uint32_t)(taken / kBulkStages) & 1u, polls);
+  }
+  // Copies that nobody will read: the block may go once they are done. (They have this long; the block goes all the same.)
   __device__ __forceinline__ void drain() {
-    for (; taken < issued; ++taken) wait();
+    for (; taken < issued; ++taken) wait(kBulkWaitPolls);
   }
 };
 
@@ -116,7 +117,7 @@ struct EdgeBatch {
 
 template <typename T, int OP>
 __global__ void __launch_bounds__(kBulkWarps * 32, bulk_blocks(OP))
-k_spmm_bulk(const __grid_constant__ RowArgs<T> a, volatile int32_t* gave_up) {
+k_spmm_bulk(const __grid_constant__ RowArgs<T> a, int polls, volatile int32_t* pending) {
   wait_for_previous();
   constexpr int VE = 16 / sizeof(T), GE = bulk_group(OP), VPL = kBulkVpl;
   constexpr bool kWeights = OP == kUMulW;
@@ -235,7 +236,7 @@ k_spmm_bulk(const __grid_constant__ RowArgs<T> a, volatile int32_t* gave_up) {
       for (int k = 0; k < 32 / GE; ++k) {
         const int at = base + k * GE, cnt = min(GE, n - at);
         if (cnt <= 0) break;
-        if (!ring.wait()) return false;
+        if (!ring.wait(polls)) return false;
         Raw<T, VE> v[GE][VPL];
         float wt[GE][VPL];
         const unsigned char* const g = ring.group() + lane * 16;
@@ -305,14 +306,20 @@ k_spmm_bulk(const __grid_constant__ RowArgs<T> a, volatile int32_t* gave_up) {
     for (unsigned m = __ballot_sync(0xffffffffu, empty); m; m &= m - 1) write(__shfl_sync(0xffffffffu, (int)d, __ffs(m) - 1));
     ok = run(b, len, (int)d, -1);
   }
-  if (!ok) {
-    ring.drain();
-    if (lane == 0) *gave_up = 1;
-  }
+  if (ok) return;
+  // waited in vain: zeros for all of this warp's rows, and a flag
+  ring.drain();
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) acc[i].zero();
+#pragma unroll 1
+  for (int64_t it = from_last ? warps - 1 - warp : warp; it < num_items; it += warps) write(a.ws.items[it].x);
+#pragma unroll 1
+  for (int64_t d = warp; d < num_rows; d += warps)
+    if (mode != kOrder || a.ws.range[d].y - a.ws.range[d].x <= a.split.long_edges) write((int)d);
+  if (lane != 0) return;
+  if (a.status) atomicOr(a.status, APT_FLAG_COPY_TIMEOUT);
+  else *pending = APT_FLAG_COPY_TIMEOUT;
 }
-
-// Where a warp that waited in vain says so: mapped memory, looked at by every later call.
-int bulk_gave_up(int32_t** word);
 
 // Wide rows of many edges: see the top of the file.
 template <typename T, int OP>
@@ -329,11 +336,14 @@ static int launch_bulk(const RowArgs<T>& a, cudaStream_t s, bool* taken) {
     APT_CUDA(cudaFuncSetAttribute(k_spmm_bulk<T, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (dev < 64) sized[dev] = true;
   }
-  int32_t* word = nullptr;
-  const int rc = bulk_gave_up(&word);
-  if (rc != APT_OK) return rc;
+  int32_t* pending = nullptr;
+  if (!a.status) {
+    const int rc = pending_word(&pending);
+    if (rc != APT_OK) return rc;
+  }
   const int64_t want = ceil_div(a.num_rows, kBulkWarps), wave = (int64_t)kNumSMs * bulk_blocks(OP);
-  APT_FOLLOW((k_spmm_bulk<T, OP>), (int)(want < wave ? want : wave), kBulkWarps * 32, smem, s, a, (volatile int32_t*)word);
+  APT_FOLLOW((k_spmm_bulk<T, OP>), (int)(want < wave ? want : wave), kBulkWarps * 32, smem, s, a, bulk_wait_polls(),
+             (volatile int32_t*)pending);
   return APT_OK;
 }
 

@@ -129,6 +129,7 @@ struct RowArgs {
   RowSplit split;
   int part_stride;         // floats per part
   const int32_t* none;     // when given and not zero: no row has edges (kRanges)
+  int32_t* status;         // flags of the call; null: the library's own word (apt_pending_flags)
 };
 
 // One slice of one edge's contribution, in two steps so that the loads of several edges are issued
@@ -504,6 +505,9 @@ int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
   }
 
 // ---- shared by spmm.cu and gat.cu -----------------------------------------------------
+constexpr int kBulkWaitPolls = 1 << 20;      // of an mbarrier, each of which may suspend for a while itself
+int bulk_wait_polls();
+int pending_word(int32_t** word);            // for flags of calls without a status word: see spmm.cu
 size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws);
 // Counted edges (ws.cnt) to places: ws.range, and the items of long rows.
 int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s);

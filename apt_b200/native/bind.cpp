@@ -268,7 +268,7 @@ int64_t read_words(const Tensor& words, const Tensor& status, const Tensor& host
   check(apt_publish_words_from(words.const_data_ptr<int64_t>(), count, status.const_data_ptr<int64_t>() + status.numel() - 1, nullptr,
                                sequence, h, s));
   check(apt_wait_published(h, count, sequence, s));
-  return h[count - 1] & 0xffffffff;
+  return (h[count - 1] & 0xffffffff) | apt_pending_flags();
 }
 
 // One captured mini-batch: launches its graph, waits for its counts, orders other streams behind its last kernel.
@@ -320,7 +320,7 @@ class Plan {
     const int64_t* const h = host_words_.const_data_ptr<int64_t>();
     py::gil_scoped_release nogil;
     check(apt_wait_published(h, count, sequence_, stream_));
-    return h[count - 1] & 0xffffffff;
+    return (h[count - 1] & 0xffffffff) | apt_pending_flags();
   }
   void finish() {
     py::gil_scoped_release nogil;
@@ -544,7 +544,7 @@ py::tuple dp_sample(const Tensor& seeds, const std::vector<int64_t>& fanouts, co
     py::gil_scoped_release nogil;
     check(apt_wait_published(h, count, sequence, s));
   }
-  const int64_t num_in = h[fanouts.size() - 1], flags = h[count - 1] & 0xffffffff;
+  const int64_t num_in = h[fanouts.size() - 1], flags = (h[count - 1] & 0xffffffff) | apt_pending_flags();
   py::object rows = py::none(), pending = py::none();
   if (look_up && num_in * dev_feats.size(1) * (int64_t)dev_feats.element_size() <= row_limit_bytes) {
     if (num_in > cur.size(0)) fail("sampler: more input nodes than were drawn");

@@ -251,6 +251,7 @@ def _flag_text(flags):
                                 "exchange refuses further use: call init() again on every rank, behind a barrier",
         _lib.FLAG_NOT_GROUPED: "edges of a block are not grouped by destination",
         _lib.FLAG_SIZE_MISMATCH: "a peer sent another number of rows than the reduction expects",
+        _lib.FLAG_COPY_TIMEOUT: "input rows of a sum did not reach shared memory in time; some of its rows are zero",
     }
     return ", ".join(v for k, v in names.items() if flags & k)
 

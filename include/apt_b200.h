@@ -54,6 +54,7 @@ typedef enum apt_dtype { APT_F32 = 0, APT_BF16 = 1, APT_F16 = 2 } apt_dtype;
 #define APT_FLAG_PEER_TIMEOUT    16 /* a peer's flag did not arrive in time */
 #define APT_FLAG_NOT_GROUPED     32 /* a block operator got edges not grouped by destination */
 #define APT_FLAG_SIZE_MISMATCH   64 /* a peer sent another number of rows than the reduction expects */
+#define APT_FLAG_COPY_TIMEOUT    128 /* input rows did not reach shared memory in time: the sums of the warp that waited are zero */
 
 const char* apt_last_error(void);
 int apt_version(void);
@@ -82,6 +83,9 @@ int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_d
 int apt_publish_words_from(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev,
                            int64_t sequence, int64_t* host, void* stream);
 int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream);
+/* Flags of kernels whose entry point has no status word (apt_spmm_*), of all devices: returns them and forgets them. A
+ * kernel's flags are there when it is done; apt_spmm_probe and apt_spmm_sum refuse with APT_ERR_TIMEOUT while one waits. */
+int32_t apt_pending_flags(void);
 /* The inputs of a captured mini-batch in one kernel: copies the seeds (device memory) into the buffer
  * the graph reads and writes words[0] = call_base, words[1] = sequence. */
 int apt_stage_replay(const int64_t* seeds, int64_t num_seeds, int64_t* seeds_buf, int64_t call_base,
@@ -98,6 +102,7 @@ int apt_profile_read(const char* tag, double* total_ms, int64_t* launches);
 /* Tuning knobs for measurements; the defaults are what the benchmark uses.
  *   gather_miss_mode, gather_miss_blocks, gather_miss_kb_per_block, gather_hit_mode, gather_hit_waves
  *                      accepted and without effect (they chose between forms of the gather that are gone)
+ *   bulk_wait_polls    polls after which a wait for rows on their way to shared memory is given up, 0 to 1048576 (default)
  *   relabel_small      1 (default): layers of up to 8192 items are relabelled by one block with
  *                      the hash table in shared memory; 0: always the multi-block path */
 int apt_set_tunable(const char* name, int64_t value);
