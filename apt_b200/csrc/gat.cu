@@ -29,6 +29,8 @@
 //                   their own the first and the last pass took 23 + 16 us.
 //   k_gat_source    grad_el in T
 //
+// k_gat_alone and k_gat_alone_backward serve the two entry points that have no buffer for weights.
+//
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
 // kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 44 + 112 + 5 us,
@@ -139,7 +141,7 @@ template <typename T, int VE>
 __global__ void __launch_bounds__(256, 3)
 k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ grad_out, int num_heads, int head_dim,
            int64_t num_dst_, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ dots, int lph,
-           int hpp, uint32_t num_src, int32_t* __restrict__ src_count /* null: not wanted */, uint32_t* __restrict__ rank) {
+           int hpp, uint32_t num_src, int32_t* __restrict__ src_count, uint32_t* __restrict__ rank) {
   wait_for_previous();
   if (*none != 0) return;
   const int lane = threadIdx.x & 31, G = gridDim.x * 8, num_dst = (int)num_dst_;
@@ -180,7 +182,7 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
         const int cnt = min(32, r.y - base);
         uint32_t my_src = src;
         if (base != r.x) my_src = (uint32_t)row[min(base + lane, r.y - 1)];
-        const bool ranked = src_count && h0 == 0 && lane < cnt;
+        const bool ranked = h0 == 0 && lane < cnt;
         uint32_t place = kNoRank;
         if (ranked && my_src < num_src) place = (uint32_t)atomicAdd(src_count + my_src, 1);
 #pragma unroll 1
@@ -232,26 +234,18 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
   }
 }
 
-// Score gradients: added to sums[source][head] (if sums), or written with the weights, both in T, for callers of the
-// edge part alone.
+// Score gradients, added to sums[source][head].
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
              int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
              float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort,
-             T* __restrict__ attn, T* __restrict__ grad_score, T* __restrict__ grad_er) {
+             T* __restrict__ grad_er) {
   wait_for_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const bool empty = *none != 0;
   if (empty)   // no edge belongs to anybody
-    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += stride) {
-      if (sums) {
-        weight[o] = 0.f;
-      } else {
-        attn[o] = Elem<T>::from_f(0.f);
-        grad_score[o] = Elem<T>::from_f(0.f);
-      }
-    }
+    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += stride) weight[o] = 0.f;
   const int64_t total = num_dst * num_heads;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
@@ -283,19 +277,12 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
 #pragma unroll
       for (int k = 0; k < C; ++k) {
         if (e0 + k >= r.y) break;
-        const int64_t o = (int64_t)(e0 + k) * num_heads + h;
         const float gs = w[k] * (dot[k] - t) * (x[k] + bias > 0.f ? 1.f : slope);
         ger += gs;
-        if (sums) {
-          if ((uint64_t)src[k] < (uint64_t)num_src) atomicAdd(sums + src[k] * num_heads + h, gs);
-        } else {
-          attn[o] = Elem<T>::from_f(w[k]);
-          grad_score[o] = Elem<T>::from_f(gs);
-        }
+        if ((uint64_t)src[k] < (uint64_t)num_src) atomicAdd(sums + src[k] * num_heads + h, gs);
       }
     }
     grad_er[i] = Elem<T>::from_f(ger);
-    if (!sums) continue;
     // the destination's edges to their places in the order by source, a share for every head's thread
 #pragma unroll 4
     for (int e = r.x + (int)h; e < r.y; e += num_heads) {
@@ -369,14 +356,18 @@ static int gat_check(const char* who, int dtype, int64_t num_edges, int num_head
   return APT_OK;
 }
 
+static int gat_ranges(const GatProblem& q, const GatEdges& g, cudaStream_t s) {
+  APT_CUDA(cudaMemsetAsync(g.none, 0, 4, s));
+  ProfScope prof("spmm_ranges", s);
+  APT_FOLLOW(k_gat_ranges, wave_grid(ceil_div(q.E, 256), 8), 256, 0, s, q.col, q.E, q.num_dst, g.range, g.none, q.status);
+  return APT_OK;
+}
+
 // Ranges and attention weights.
 template <typename T>
 static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaStream_t s) {
-  APT_CUDA(cudaMemsetAsync(g.none, 0, 4, s));
-  {
-    ProfScope prof("spmm_ranges", s);
-    APT_FOLLOW(k_gat_ranges, wave_grid(ceil_div(q.E, 256), 8), 256, 0, s, q.col, q.E, q.num_dst, g.range, g.none, q.status);
-  }
+  const int rc = gat_ranges(q, g, s);
+  if (rc != APT_OK) return rc;
   ProfScope prof("gat_rows", s);
   APT_FOLLOW(k_gat_weights<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
              q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn);
@@ -411,11 +402,11 @@ static int launch_dots(const GatProblem& q, const GatEdges& g, int64_t num_src, 
   return APT_OK;
 }
 
-// The edge part of the backward: weights are there already. With `sums` also the source side's sums of the score gradients
-// and the order of its edges (`sort`, all of it zero where it has to be).
+// The edge part of the backward: weights are there already. Leaves the source side's sums of the score gradients and the order
+// of its edges (`sort`, all of it zero where it has to be).
 template <typename T>
 static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num_src, float* dots, float* sums, const SpmmWs& sort,
-                             int long_edges, void* attn, void* grad_score, void* grad_er, cudaStream_t s) {
+                             int long_edges, void* grad_er, cudaStream_t s) {
   ProfScope prof("gat_bwd_rows", s);
   int rc;
   switch (slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T)) {
@@ -424,10 +415,10 @@ static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num
     case 4: rc = launch_dots<T, 4 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
     default: rc = launch_dots<T, 1>(q, g, num_src, dots, sort, s); break;
   }
-  if (rc == APT_OK && sums) rc = launch_slots(num_src, sort, kOrder, long_edges, (int)(q.H * q.Dh), s);
+  if (rc == APT_OK) rc = launch_slots(num_src, sort, kOrder, long_edges, (int)(q.H * q.Dh), s);
   if (rc != APT_OK) return rc;
   APT_FOLLOW(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-             q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, sort, (T*)attn, (T*)grad_score, (T*)grad_er);
+             q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, sort, (T*)grad_er);
   return APT_OK;
 }
 
@@ -439,7 +430,7 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
   const RowSplit split = row_split(dim, ve, q.E, num_src);
   const SegTable st{nullptr, nullptr, nullptr, 1};
   APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
-  int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, ws.sort, split.long_edges, nullptr, nullptr, grad_er, s);
+  int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, ws.sort, split.long_edges, grad_er, s);
   if (rc != APT_OK) return rc;
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, st, num_src, q.E, ws.sort,
                      (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr, q.status};
@@ -450,19 +441,269 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
   return APT_OK;
 }
 
-// Stream-ordered memory for the duration of a call, for the two entry points without a buffer for weights.
-struct StreamBuffer {
-  void* p = nullptr;
-  cudaStream_t s;
-  explicit StreamBuffer(cudaStream_t stream) : s(stream) {}
-  int take(size_t bytes) {
-    APT_CUDA(cudaMallocAsync(&p, bytes, s));
-    return APT_OK;
+// ---- without a buffer for weights -----------------------------------------------------
+// apt_gat_edge_softmax_sum and apt_gat_edge_backward have a few words a destination of workspace and allocate nothing: a warp
+// to a destination keeps the weights of 32 edges and 4 heads in shared memory and works them out again for further edges
+// and column blocks. They are for callers that do not hold E x heads fp32 values: 67 584 x 15 edges, bf16, 4 x 64, take 142 us
+// forward and 245 for the edge part of the backward, with such a buffer 114 and 164.
+constexpr int kAloneHeads = 4;
+
+// The weights of one destination's edges, for the heads from h0 on, a lane to an edge. What outlives a step is in shared memory:
+// as registers it took half the warps.
+struct GatAloneWarp {
+  float w[32][kAloneHeads];                                  // of the edges of the current chunk
+  float bias[kAloneHeads], most[kAloneHeads], inv[kAloneHeads];      // needed again with more than 32 edges
+};
+template <typename T>
+struct GatScores {
+  GatAloneWarp& sh;
+  const int64_t* row;
+  const T* el;
+  int H, h0, nh;
+  float slope;
+  bool few;
+  unsigned positive;       // bit h: this lane's score before the leaky part
+
+  __device__ __forceinline__ float score(int64_t src, int h, float bias) const { return Elem<T>::to_f(el[src * H + h0 + h]) + bias; }
+  __device__ __forceinline__ void start(const T* er, int d, int2 r, int lane) {
+    few = r.y - r.x <= 32;
+    positive = 0u;
+    const bool mine = few && r.x + lane < r.y;
+    const int64_t src = mine ? row[r.x + lane] : 0;
+    float bias[kAloneHeads], x[kAloneHeads];
+#pragma unroll
+    for (int h = 0; h < kAloneHeads; ++h) {
+      if (h >= nh) break;
+      bias[h] = Elem<T>::to_f(er[(int64_t)d * H + h0 + h]);
+      x[h] = mine ? score(src, h, bias[h]) : -INFINITY;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < kAloneHeads; ++h) {
+      if (h >= nh) break;
+      float most = mine ? leaky(x[h], slope) : -INFINITY, sum = 0.f;
+      if (!few)
+        for (int e = r.x + lane; e < r.y; e += 32) most = fmaxf(most, leaky(score(row[e], h, bias[h]), slope));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+      if (mine) sum = expf(leaky(x[h], slope) - most);
+      if (!few)
+        for (int e = r.x + lane; e < r.y; e += 32) sum += expf(leaky(score(row[e], h, bias[h]), slope) - most);
+      const float own = sum;
+      sum = group_sum(sum, 32);
+      const float inv = sum > 0.f ? 1.f / sum : 0.f;
+      if (mine) sh.w[lane][h] = own * inv;
+      if (mine && x[h] > 0.f) positive |= 1u << h;
+      if (!few && lane == 0) sh.bias[h] = bias[h], sh.most[h] = most, sh.inv[h] = inv;
+    }
+    __syncwarp();
   }
-  ~StreamBuffer() {
-    if (p) cudaFreeAsync(p, s);
+  // The weights of a chunk of edges.
+  __device__ __forceinline__ void chunk(int64_t src, bool mine, int lane) {
+    if (few) return;
+    __syncwarp();
+    positive = 0u;
+#pragma unroll
+    for (int h = 0; h < kAloneHeads; ++h) {
+      if (h >= nh || !mine) break;
+      const float x = score(src, h, sh.bias[h]);
+      sh.w[lane][h] = expf(leaky(x, slope) - sh.most[h]) * sh.inv[h];
+      if (x > 0.f) positive |= 1u << h;
+    }
+    __syncwarp();
   }
 };
+
+template <typename T, int VE>
+__global__ void __launch_bounds__(256, 4)
+k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er, int num_heads,
+            int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none,
+            T* __restrict__ out, T* __restrict__ attn, int lpe) {
+  wait_for_previous();
+  constexpr int U = 4;
+  __shared__ GatAloneWarp shared[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & (lpe - 1), epi = lane / lpe, ep = 32 / lpe;
+  const int nvh = head_dim / VE;
+  const int64_t dim = (int64_t)num_heads * head_dim;
+  const uint32_t row_bytes = (uint32_t)(dim * sizeof(T));
+  const bool empty = *none != 0;
+  for (int64_t d = (int64_t)blockIdx.x * 8 + warp; d < num_dst; d += (int64_t)gridDim.x * 8) {
+    const int2 r = empty ? make_int2(0, 0) : range[d];
+    const int deg = r.y - r.x;
+    for (int h0 = 0; h0 < num_heads; h0 += kAloneHeads) {
+      GatScores<T> sc{shared[warp], row, el, num_heads, h0, min(kAloneHeads, num_heads - h0), slope};
+      if (deg > 0) sc.start(er, (int)d, r, lane);
+      const int slices = sc.nh * nvh;
+      for (int c0 = 0; c0 < slices; c0 += lpe) {
+        const int c = c0 + sub, h = c < slices ? c / nvh : 0;
+        const int64_t col = (int64_t)h0 * head_dim + (int64_t)c * VE;
+        const T* const lane_ft = ft + col;
+        Acc<VE> acc;
+        acc.zero();
+        for (int base = r.x; base < r.y; base += 32) {
+          const int cnt = min(32, r.y - base);
+          const uint32_t src = lane < cnt ? (uint32_t)row[base + lane] : 0u;
+          if (c0 == 0 || deg > 32) {
+            sc.chunk(src, lane < cnt, lane);
+            if (attn && c0 == 0 && lane < cnt)
+              for (int k = 0; k < sc.nh; ++k) attn[(int64_t)(base + lane) * num_heads + h0 + k] = Elem<T>::from_f(sc.sh.w[lane][k]);
+          }
+          for (int j0 = epi; j0 - epi < cnt; j0 += ep * U) {
+            Raw<T, VE> v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const uint32_t from = __shfl_sync(0xffffffffu, src, (j0 + u * ep) & 31);
+              if (j0 + u * ep < cnt && c < slices) v[u] = load_raw<T, VE>(at_row(lane_ft, from, row_bytes));
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (j0 + u * ep < cnt && c < slices) acc.fma(v[u], sc.sh.w[j0 + u * ep][h]);
+          }
+        }
+        for (int o = lpe; o < 32; o <<= 1) acc.join(0xffffffffu, o);
+        if (epi == 0 && c < slices) store_pack<T, VE>(out + d * dim + col, acc.template rounded<T>());
+      }
+      __syncwarp();
+    }
+  }
+}
+
+template <typename T, int VE>
+__global__ void __launch_bounds__(256, 4)
+k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er,
+                     const T* __restrict__ grad_out, int num_heads, int head_dim, float slope, int64_t num_dst, int64_t E,
+                     const int2* __restrict__ range, const int32_t* __restrict__ none, T* __restrict__ attn,
+                     T* __restrict__ grad_score, T* __restrict__ grad_er, int lph, int hpp) {
+  wait_for_previous();
+  constexpr int U = 4;
+  __shared__ GatAloneWarp shared[8];
+  __shared__ float dot_sh[8][32][kAloneHeads];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p = lane & (lph - 1), rh = (lane & (lph * hpp - 1)) / lph, epi = lane / (lph * hpp), ep = 32 / (lph * hpp);
+  const int nvh = head_dim / VE;
+  const int64_t dim = (int64_t)num_heads * head_dim;
+  const uint32_t row_bytes = (uint32_t)(dim * sizeof(T));
+  const bool empty = *none != 0;
+  if (empty)   // no edge belongs to anybody
+    for (int64_t o = (int64_t)blockIdx.x * 256 + threadIdx.x; o < E * num_heads; o += (int64_t)gridDim.x * 256)
+      attn[o] = grad_score[o] = Elem<T>::from_f(0.f);
+  for (int64_t d = (int64_t)blockIdx.x * 8 + warp; d < num_dst; d += (int64_t)gridDim.x * 8) {
+    const int2 r = empty ? make_int2(0, 0) : range[d];
+    const int deg = r.y - r.x;
+    for (int h0 = 0; h0 < num_heads; h0 += kAloneHeads) {
+      GatScores<T> sc{shared[warp], row, el, num_heads, h0, min(kAloneHeads, num_heads - h0), slope};
+      if (deg > 0) sc.start(er, (int)d, r, lane);
+      float t[kAloneHeads], ger[kAloneHeads];
+#pragma unroll
+      for (int k = 0; k < kAloneHeads; ++k) t[k] = ger[k] = 0.f;
+      // up to 32 edges: t first, then the results, from the same dots; more: two walks
+      const int passes = deg > 32 ? 2 : 1;
+      for (int pass = 0; pass < passes; ++pass) {
+        for (int base = r.x; base < r.y; base += 32) {
+          const int cnt = min(32, r.y - base);
+          const uint32_t src = lane < cnt ? (uint32_t)row[base + lane] : 0u;
+          __syncwarp();
+          for (int hb = 0; hb < sc.nh; hb += hpp) {
+            const int h = hb + rh;
+            const T *const g_head = grad_out + d * dim + (int64_t)(h0 + h) * head_dim, *const ft_head = ft + (int64_t)(h0 + h) * head_dim;
+            for (int j0 = epi; j0 - epi < cnt; j0 += ep * U) {
+              uint32_t from[U];
+              float dot[U];
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                from[u] = __shfl_sync(0xffffffffu, src, (j0 + u * ep) & 31);
+                dot[u] = 0.f;
+              }
+              if (h < sc.nh)
+                for (int c = p; c < nvh; c += lph) {
+                  const Raw<T, VE> g = load_raw<T, VE>(g_head + c * VE);
+                  Raw<T, VE> v[U];
+#pragma unroll
+                  for (int u = 0; u < U; ++u)
+                    if (j0 + u * ep < cnt) v[u] = load_raw<T, VE>(at_row(ft_head + c * VE, from[u], row_bytes));
+#pragma unroll
+                  for (int u = 0; u < U; ++u) {
+                    if (j0 + u * ep >= cnt) break;
+#pragma unroll
+                    for (int q = 0; q < VE; ++q) dot[u] = fmaf(g.get(q), v[u].get(q), dot[u]);
+                  }
+                }
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                dot[u] = group_sum(dot[u], lph);
+                if (p == 0 && j0 + u * ep < cnt && h < sc.nh) dot_sh[warp][j0 + u * ep][h] = dot[u];
+              }
+            }
+          }
+          sc.chunk(src, lane < cnt, lane);
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < kAloneHeads; ++k) {
+            if (k >= sc.nh) break;
+            const float w = lane < cnt ? sc.sh.w[lane][k] : 0.f, dot = lane < cnt ? dot_sh[warp][lane][k] : 0.f;
+            if (pass == 0) t[k] += group_sum(lane < cnt ? w * dot : 0.f, 32);
+            if (pass < passes - 1) continue;
+            const float gs = w * (dot - t[k]) * (sc.positive >> k & 1u ? 1.f : slope);
+            if (lane < cnt) {
+              attn[(int64_t)(base + lane) * num_heads + h0 + k] = Elem<T>::from_f(w);
+              grad_score[(int64_t)(base + lane) * num_heads + h0 + k] = Elem<T>::from_f(gs);
+            }
+            ger[k] += group_sum(lane < cnt ? gs : 0.f, 32);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kAloneHeads; ++k)
+        if (k < sc.nh && lane == 0) grad_er[d * num_heads + h0 + k] = Elem<T>::from_f(ger[k]);
+    }
+  }
+}
+
+template <typename T, int VE>
+static int launch_alone(const GatProblem& q, const GatEdges& g, void* out, void* attn, void* grad_score, void* grad_er, cudaStream_t s) {
+  const int nvh = (int)(q.Dh / VE), grid = wave_grid(ceil_div(q.num_dst, 8), 8);
+  if (grad_er) {
+    const int lph = pow2_ge(nvh), hpp = pow2_ge(std::min(q.H, kAloneHeads), 32 / lph);
+    APT_FOLLOW((k_gat_alone_backward<T, VE>), grid, 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el, (const T*)q.er,
+               (const T*)q.grad_out, q.H, (int)q.Dh, q.slope, q.num_dst, q.E, g.range, g.none, (T*)attn, (T*)grad_score, (T*)grad_er,
+               lph, hpp);
+  } else {
+    APT_FOLLOW((k_gat_alone<T, VE>), grid, 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el, (const T*)q.er, q.H, (int)q.Dh, q.slope,
+               q.num_dst, g.range, g.none, (T*)out, (T*)attn, pow2_ge((int64_t)std::min(q.H, kAloneHeads) * nvh));
+  }
+  return APT_OK;
+}
+
+// The ranges are in the front of a workspace of apt_spmm_workspace_bytes(num_dst, 0) bytes. Backward with grad_er, else forward.
+template <typename T>
+static int gat_alone(const GatProblem& q, void* workspace, void* out, void* attn, void* grad_score, void* grad_er, cudaStream_t s) {
+  const GatEdges g{(int32_t*)workspace, (int2*)((char*)workspace + 256), nullptr};
+  const int rc = gat_ranges(q, g, s);
+  if (rc != APT_OK) return rc;
+  ProfScope prof(grad_er ? "gat_bwd_rows" : "gat_rows", s);
+  const uintptr_t other = (uintptr_t)(grad_er ? q.grad_out : out);
+  switch (slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | other, sizeof(T)) * (int)sizeof(T)) {
+    case 16: return launch_alone<T, 16 / sizeof(T)>(q, g, out, attn, grad_score, grad_er, s);
+    case 8: return launch_alone<T, 8 / sizeof(T)>(q, g, out, attn, grad_score, grad_er, s);
+    case 4: return launch_alone<T, 4 / sizeof(T)>(q, g, out, attn, grad_score, grad_er, s);
+    default: return launch_alone<T, 1>(q, g, out, attn, grad_score, grad_er, s);
+  }
+}
+
+static int gat_alone(const char* who, int dtype, const GatProblem& q, void* workspace, size_t workspace_bytes, void* out, void* attn,
+                     void* grad_score, void* grad_er, cudaStream_t s) {
+  APT_CHECK_ARG(((uintptr_t)workspace & 255) == 0, "%s: workspace must be 256-byte aligned", who);
+  const size_t need = spmm_layout(q.num_dst, 0, nullptr, nullptr);
+  if (workspace_bytes < need) {
+    set_error("%s: workspace %zu < %zu bytes", who, workspace_bytes, need);
+    return APT_ERR_CAPACITY;
+  }
+  switch (dtype) {
+    case APT_F32: return gat_alone<float>(q, workspace, out, attn, grad_score, grad_er, s);
+    case APT_BF16: return gat_alone<__nv_bfloat16>(q, workspace, out, attn, grad_score, grad_er, s);
+    default: return gat_alone<__half>(q, workspace, out, attn, grad_score, grad_er, s);
+  }
+}
 
 }  // namespace apt
 
@@ -558,14 +799,15 @@ extern "C" int apt_gat_edge_softmax_sum(int dtype, const int64_t* coo_row, const
   using namespace apt;
   const int rc = gat_check("apt_gat_edge_softmax_sum", dtype, num_edges, num_heads, head_dim, num_dst);
   if (rc != APT_OK || num_dst == 0) return rc;
-  StreamBuffer edges((cudaStream_t)stream);
-  const size_t bytes = gat_edges_layout(num_dst, num_edges, num_heads, nullptr, nullptr);
-  if (num_edges > 0) {
-    const int taken = edges.take(bytes);
-    if (taken != APT_OK) return taken;
+  cudaStream_t s = (cudaStream_t)stream;
+  APT_CHECK_ARG(out && status_word, "apt_gat_edge_softmax_sum: null output");
+  if (num_edges == 0) {
+    APT_CUDA(cudaMemsetAsync(out, 0, (size_t)num_dst * num_heads * head_dim * elem_size(dtype), s));
+    return APT_OK;
   }
-  return apt_gat_forward(dtype, coo_row, coo_col, num_edges, ft, el, er, num_heads, head_dim, negative_slope, num_dst, out,
-                         out_attn, edges.p, bytes, status_word, stream);
+  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && workspace, "apt_gat_edge_softmax_sum: null pointer");
+  const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, nullptr, num_heads, head_dim, negative_slope, num_dst, status_word};
+  return gat_alone("apt_gat_edge_softmax_sum", dtype, q, workspace, workspace_bytes, out, out_attn, nullptr, nullptr, s);
 }
 
 extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges,
@@ -574,7 +816,7 @@ extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const in
                                      void* out_attn, void* out_grad_score, void* out_grad_er, void* workspace,
                                      size_t workspace_bytes, int32_t* status_word, void* stream) {
   using namespace apt;
-  int rc = gat_check("apt_gat_edge_backward", dtype, num_edges, num_heads, head_dim, num_dst);
+  const int rc = gat_check("apt_gat_edge_backward", dtype, num_edges, num_heads, head_dim, num_dst);
   if (rc != APT_OK || num_dst == 0) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   APT_CHECK_ARG(out_grad_er && status_word, "apt_gat_edge_backward: null output");
@@ -582,25 +824,8 @@ extern "C" int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const in
     APT_CUDA(cudaMemsetAsync(out_grad_er, 0, (size_t)num_dst * num_heads * elem_size(dtype), s));
     return APT_OK;
   }
-  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && grad_out && out_attn && out_grad_score,
+  APT_CHECK_ARG(coo_row && coo_col && ft && el && er && grad_out && out_attn && out_grad_score && workspace,
                 "apt_gat_edge_backward: null pointer");
-  StreamBuffer buffer(s);
-  const size_t edges_bytes = gat_edges_layout(num_dst, num_edges, num_heads, nullptr, nullptr);
-  rc = buffer.take(edges_bytes + (size_t)num_edges * num_heads * 4);
-  if (rc != APT_OK) return rc;
-  GatEdges g;
-  gat_edges_layout(num_dst, num_edges, num_heads, (char*)buffer.p, &g);
-  float* dots = (float*)((char*)buffer.p + edges_bytes);
   const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, grad_out, num_heads, head_dim, negative_slope, num_dst, status_word};
-#define APT_RUN(T)                                                                                         \
-  do {                                                                                                     \
-    if ((rc = gat_weights<T>(q, g, nullptr, s)) != APT_OK) return rc;                                      \
-    return gat_edge_backward<T>(q, g, 0, dots, nullptr, SpmmWs{}, 0, out_attn, out_grad_score, out_grad_er, s);    \
-  } while (0)
-  switch (dtype) {
-    case APT_F32: APT_RUN(float);
-    case APT_BF16: APT_RUN(__nv_bfloat16);
-    default: APT_RUN(__half);
-  }
-#undef APT_RUN
+  return gat_alone("apt_gat_edge_backward", dtype, q, workspace, workspace_bytes, nullptr, out_attn, out_grad_score, out_grad_er, s);
 }

@@ -429,8 +429,8 @@ int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const int64_t* coo_
  * [num_src, num_heads*head_dim], grad_el [num_src, num_heads] and grad_er [num_dst,
  * num_heads]: the edges are grouped by source once and one walk sums both source-side
  * gradients. workspace: apt_gat_backward_workspace_bytes(...) bytes.
- * apt_gat_edge_softmax_sum and apt_gat_edge_backward above take the room for weights
- * from the stream's memory pool (cudaMallocAsync) and use no workspace. */
+ * apt_gat_edge_softmax_sum and apt_gat_edge_backward above do with a few words a
+ * destination and work the weights out as often as they need them. */
 size_t apt_gat_edges_bytes(int64_t num_dst, int64_t num_edges, int num_heads);
 int apt_gat_forward(int dtype, const int64_t* coo_row, const int64_t* coo_col,
                     int64_t num_edges, const void* ft, const void* el,

@@ -3,6 +3,8 @@ warp reads at once, more heads than lanes, head widths of every slice size and b
 empty destinations), the edge-part entry points of the C ABI and the backward that starts from what the forward saved,
 against the fp64 oracle. Bounds as in test_gpu_gat.py: the sums of at most a few hundred fp32 terms within 1e-5 of the
 largest value, 16-bit results within 1e-2."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -62,26 +64,79 @@ def test_forward_and_backward(dtype, H, Dh, lengths):
     ops.check_status()
 
 
-def test_edge_part_entry_points():
-    dtype, H, Dh = torch.float32, 4, 16
+def _pool_reserved():
+    """Most bytes the device's stream-ordered memory pool has held so far."""
+    rt = ctypes.CDLL("libcudart.so.12")            # the one PyTorch has loaded
+    pool, most = ctypes.c_void_p(), ctypes.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert rt.cudaMemPoolGetAttribute(pool, 6, ctypes.byref(most)) == 0      # cudaMemPoolAttrReservedMemHigh
+    return most.value
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,Dh", [(1, 1), (4, 16), (4, 64), (3, 5), (9, 8), (33, 4), (1, 300), (2, 1030)])
+@pytest.mark.parametrize("captured", [False, True], ids=["direct", "captured"])
+def test_edge_part_entry_points(dtype, H, Dh, captured):
+    # they work in a few words a destination, allocate nothing and may be captured
     row, col, ft, el, er, go = _inputs(RAGGED, H, Dh, dtype, 1)
     S, E = len(RAGGED), len(row)
+    t = [dev(row), dev(col)] + [dev(x, dtype) for x in (ft, el, er, go)]
+    p = [x.data_ptr() for x in t]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, attn, attn_b, gs, ger = (torch.full(shape, 9.0, device="cuda", dtype=dtype)
+                                  for shape in ((S, H, Dh), (E, H), (E, H), (E, H), (S, H)))
+    nbytes = lib.apt_spmm_workspace_bytes(S, 0)
+    room = torch.full((nbytes + 512,), 77, dtype=torch.uint8, device="cuda")
+    ws = room[:nbytes]
+    before = _pool_reserved()
+
+    def call():
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        check(lib.apt_gat_edge_softmax_sum(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], H, Dh, 0.2, S, out.data_ptr(),
+                                           attn.data_ptr(), ws.data_ptr(), nbytes, status.data_ptr(), stream))
+        check(lib.apt_gat_edge_backward(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], p[5], H, Dh, 0.2, S, attn_b.data_ptr(),
+                                        gs.data_ptr(), ger.data_ptr(), ws.data_ptr(), nbytes, status.data_ptr(), stream))
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call()
+        for _ in range(2):
+            graph.replay()
+    else:
+        call()
+    torch.cuda.synchronize()
+    assert _pool_reserved() == before and bool((room[nbytes:] == 77).all())
+    want, _ = orc.gat_edge_softmax_sum(row, col, ft, el, er, S, 0.2)
+    _, _, w_er, w_attn, w_gs = orc.gat_edge_softmax_sum_backward(row, col, ft, el, er, go, S, 0.2)
+    for got, w, name in ((out, want, "out"), (attn, w_attn, "attention"), (attn_b, w_attn, "attention of the backward"),
+                         (gs, w_gs, "score gradient"), (ger, w_er, "grad_er")):
+        _near(got, np.asarray(w).reshape(got.shape), dtype, name)
+    assert int(status[0]) == 0
+    st = lib.apt_gat_edge_softmax_sum(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], H, Dh, 0.2, S, out.data_ptr(), None, None, 0,
+                                      status.data_ptr(), None)
+    assert st == _lib.APT_ERR_BAD_ARG
+    st = lib.apt_gat_edge_backward(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], p[5], H, Dh, 0.2, S, attn.data_ptr(), gs.data_ptr(),
+                                   ger.data_ptr(), ws.data_ptr(), nbytes - 1, status.data_ptr(), None)
+    assert st == _lib.APT_ERR_CAPACITY
+
+
+def test_edge_part_of_ungrouped_edges():
+    dtype, H, Dh = torch.float32, 2, 8
+    row, col, ft, el, er, go = _inputs([3, 0, 4], H, Dh, dtype, 1)
+    col = col[::-1].copy()
     t = [dev(x) for x in (row, col, ft, el, er, go)]
     p = [x.data_ptr() for x in t]
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    out, attn, gs, ger = (torch.full(shape, 9.0, device="cuda") for shape in ((S, H, Dh), (E, H), (E, H), (S, H)))
-    nbytes = lib.apt_spmm_workspace_bytes(S, 0)
+    out, attn, gs, ger = (torch.full(shape, 9.0, device="cuda") for shape in ((3, H, Dh), (7, H), (7, H), (3, H)))
+    nbytes = lib.apt_spmm_workspace_bytes(3, 0)
     ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
-    check(lib.apt_gat_edge_softmax_sum(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], H, Dh, 0.2, S, out.data_ptr(), None,
-                                       ws.data_ptr(), nbytes, status.data_ptr(), None))
-    check(lib.apt_gat_edge_backward(CODE[dtype], p[0], p[1], E, p[2], p[3], p[4], p[5], H, Dh, 0.2, S, attn.data_ptr(),
-                                    gs.data_ptr(), ger.data_ptr(), ws.data_ptr(), nbytes, status.data_ptr(), None))
+    check(lib.apt_gat_edge_softmax_sum(_lib.F32, p[0], p[1], 7, p[2], p[3], p[4], H, Dh, 0.2, 3, out.data_ptr(), None, ws.data_ptr(),
+                                       nbytes, status.data_ptr(), None))
+    check(lib.apt_gat_edge_backward(_lib.F32, p[0], p[1], 7, p[2], p[3], p[4], p[5], H, Dh, 0.2, 3, attn.data_ptr(), gs.data_ptr(),
+                                    ger.data_ptr(), ws.data_ptr(), nbytes, status.data_ptr(), None))
     torch.cuda.synchronize()
-    want, _ = orc.gat_edge_softmax_sum(row, col, ft, el, er, S, 0.2)
-    _, _, w_er, w_attn, w_gs = orc.gat_edge_softmax_sum_backward(row, col, ft, el, er, go, S, 0.2)
-    for got, w, name in ((out, want, "out"), (attn, w_attn, "attention"), (gs, w_gs, "score gradient"), (ger, w_er, "grad_er")):
-        _near(got, np.asarray(w).reshape(got.shape), dtype, name)
-    assert int(status[0]) == 0
+    assert not any(bool(x.any()) for x in (out, attn, gs, ger)) and int(status[0]) == _lib.FLAG_NOT_GROUPED
 
 
 def test_ungrouped_backward_is_zero_and_flagged():
