@@ -82,6 +82,14 @@ struct ProfScope {
 void set_relabel_small(bool on);   // relabel.cu: one-block shared-memory path for small layers
 void set_bulk_wait_polls(int polls);   // spmm.cu: bound of k_spmm_bulk's waits
 
+// While another thread captures a stream, or this one does, calls that might synchronise are refused and end the capture. For
+// those that do not touch the captured work (page-locked memory of the library's own, asking a stream how it stands).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 constexpr int kNumSMs = 148;  // B200: 2 dies x 74 SMs
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }

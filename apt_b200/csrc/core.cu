@@ -123,6 +123,7 @@ int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* s
   for (int64_t spin = 1; *word != sequence; ++spin) {
     if ((spin & 0x3fff) == 0) {
       // now and then the stream is asked, so that an error on it ends the wait
+      apt::RelaxedCapture relaxed;
       const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
       if (e == cudaErrorNotReady) continue;
       APT_CUDA(e);

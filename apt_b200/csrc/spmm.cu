@@ -73,17 +73,20 @@ __device__ __forceinline__ int64_t out_row(const int64_t* coo, const int64_t* oo
 
 // One 64-bit word collects the blocks' answers: blocks done, and how many of them saw each of the three. The add that
 // counts a block also returns what the others saw, so the last block has the answer without a fence or a second
-// read (fence, counter and read in turn: 5.6 -> 4.5 us for 10 240 edges). `agg` is zero before and after; `result` may
-// be mapped host memory.
+// read (fence, counter and read in turn: 5.6 -> 4.5 us for 10 240 edges). The word, `agg` or the slot's own, is zero before
+// and after; `result` may be mapped host memory.
+constexpr int kProbeSlots = 64;
+__device__ unsigned long long g_probe_votes[kProbeSlots];
 __device__ __forceinline__ unsigned long long probe_votes(uint32_t bits) {
   return 1ull | (bits & kNotGrouped ? 1ull << 16 : 0ull) | (bits & kNotFixed ? 1ull << 32 : 0ull) |
          (bits & kHasLong ? 1ull << 48 : 0ull);
 }
 
 __global__ void __launch_bounds__(256)
-k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned long long* agg, volatile int64_t* result,
+k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned long long* agg, int slot, volatile int64_t* result,
              int64_t sequence) {
   wait_for_previous();
+  if (!agg) agg = g_probe_votes + slot;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   __shared__ uint32_t s_bits;
   constexpr int K = 4;
@@ -139,46 +142,34 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned l
   *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, sequence);
 }
 
-static int launch_probe(const int64_t* col, int64_t E, SegTable st, unsigned long long* agg, int64_t* result, int64_t sequence,
-                        cudaStream_t s) {
+static int launch_probe(const int64_t* col, int64_t E, SegTable st, unsigned long long* agg, int slot, int64_t* result,
+                        int64_t sequence, cudaStream_t s) {
   // a thousand edges a block and one wave at most: small blocks of edges are looked over by one thread block
   const int grid = wave_grid(ceil_div(E, 1024), 4, 1);
   ProfScope prof("spmm_ranges", s);
-  APT_FOLLOW(k_spmm_probe, grid, 256, 0, s, col, E, st, agg, (volatile int64_t*)result, sequence);
+  APT_FOLLOW(k_spmm_probe, grid, 256, 0, s, col, E, st, agg, slot, (volatile int64_t*)result, sequence);
   return APT_OK;
 }
 
 // Where probes leave their answers for the host: a fixed number of slots, each taken by one call and given
 // back before it returns, so that calls of several threads and streams do not meet.
 struct ProbeSlots {
-  static constexpr int kCount = 64;
   std::mutex mu;
   std::condition_variable cv;
   int64_t* host = nullptr;            // mapped: 8 words a slot
-  unsigned long long* agg[64] = {};   // device words of each device: one a slot, zero between calls
   uint64_t taken = 0;
   int64_t sequence = 0;
 };
 static ProbeSlots g_probe;
 
-static int take_slot(int dev, int* slot, int64_t* sequence) {
+static int take_slot(int* slot, int64_t* sequence) {
   std::unique_lock<std::mutex> lk(g_probe.mu);
   if (!g_probe.host) {
     void* p = nullptr;
-    APT_CUDA(cudaHostAlloc(&p, ProbeSlots::kCount * 64, cudaHostAllocMapped | cudaHostAllocPortable));
+    RelaxedCapture relaxed;
+    APT_CUDA(cudaHostAlloc(&p, kProbeSlots * 64, cudaHostAllocMapped | cudaHostAllocPortable));
     g_probe.host = (int64_t*)p;
-    for (int k = 0; k < ProbeSlots::kCount * 8; ++k) g_probe.host[k] = 0;
-  }
-  if (!g_probe.agg[dev]) {
-    void* p = nullptr;
-    APT_CUDA(cudaMalloc(&p, ProbeSlots::kCount * 8));
-    cudaError_t e = cudaMemset(p, 0, ProbeSlots::kCount * 8);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();   // once per device: the words are zero for every stream
-    if (e != cudaSuccess) {
-      cudaFree(p);
-      APT_CUDA(e);
-    }
-    g_probe.agg[dev] = (unsigned long long*)p;
+    for (int k = 0; k < kProbeSlots * 8; ++k) g_probe.host[k] = 0;
   }
   g_probe.cv.wait(lk, [] { return g_probe.taken != ~0ull; });
   *slot = __builtin_ctzll(~g_probe.taken);
@@ -205,6 +196,7 @@ int pending_word(int32_t** word) {
   std::lock_guard<std::mutex> lk(mu);
   if (!g_pending.load()) {
     void* p = nullptr;
+    RelaxedCapture relaxed;
     APT_CUDA(cudaHostAlloc(&p, 64, cudaHostAllocMapped | cudaHostAllocPortable));
     *(int32_t*)p = 0;
     g_pending.store((int32_t*)p, std::memory_order_release);
@@ -234,6 +226,7 @@ static int wait_for(const volatile int64_t* word, int64_t sequence, cudaStream_t
   for (int64_t spin = 1;; ++spin) {
     if (probe_sequence(*word) == sequence) break;
     if ((spin & 0x3fff) == 0) {
+      RelaxedCapture relaxed;
       const cudaError_t e = cudaStreamQuery(s);
       if (e == cudaErrorNotReady) continue;
       APT_CUDA(e);
@@ -518,7 +511,7 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
   const RowSplit split = row_split(feat_dim, slice_elems(bits, (int)esz), E, num_rows);
   if (mode == kDevice || mode == kOrder) APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
   if (mode == kDevice) {
-    const int rc = launch_probe(coo_col, E, st, ws.probe, ws.result, 1, s);
+    const int rc = launch_probe(coo_col, E, st, ws.probe, 0, ws.result, 1, s);
     if (rc != APT_OK) return rc;
   }
   if (mode == kDevice || mode == kRanges) {
@@ -575,15 +568,13 @@ extern "C" int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges, const i
                 "apt_spmm_probe: the number of output rows is read on the host, which a stream capture does not allow");
   int rc = check_pending("apt_spmm_probe");
   if (rc != APT_OK) return rc;
-  int dev = 0, slot = -1;
-  APT_CUDA(cudaGetDevice(&dev));
-  APT_CHECK_ARG(dev < 64, "apt_spmm_probe: device %d", dev);
+  int slot = -1;
   int64_t sequence = 0;
-  rc = take_slot(dev, &slot, &sequence);
+  rc = take_slot(&slot, &sequence);
   if (rc != APT_OK) return rc;
   int64_t* host = g_probe.host + slot * 8;
   SegTable st{coo_offset, nullptr, output_offset, num_segments};
-  rc = launch_probe(coo_col, num_edges, st, g_probe.agg[dev] + slot, host, sequence, s);
+  rc = launch_probe(coo_col, num_edges, st, nullptr, slot, host, sequence, s);
   if (rc == APT_OK) rc = wait_for(host, sequence, s);
   if (rc == APT_OK) {
     const int64_t w = *(volatile int64_t*)host, rows = probe_rows(w);

@@ -324,7 +324,10 @@ class Plan {
   }
   void finish() {
     py::gil_scoped_release nogil;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // a plan may go while some stream is being captured
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (stream_) cudaEventSynchronize(done_);
+    cudaThreadExchangeStreamCaptureMode(&mode);
   }
   // The current stream runs on behind everything the last launch enqueued (the gathered rows among it).
   void order_current_stream() {
