@@ -238,21 +238,21 @@ std::tuple<Tensor, Tensor, Tensor> gat_backward(const Tensor& coo_row, const Ten
   return {grad_ft, grad_el, grad_er};
 }
 
-// The forward's ranges and weights are saved with its inputs: the backward of a training step starts from them.
+// The forward's ranges and weights are saved with its inputs: the backward of a training step starts from them, and they
+// go when the inputs go.
 struct GatFunction : public torch::autograd::Function<GatFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& row, const Tensor& col, const Tensor& ft,
                         const Tensor& el, const Tensor& er, int64_t num_dst, double slope, const Tensor& words) {
     auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, false, words);
-    ctx->save_for_backward({row, col, ft, el, er});
+    ctx->save_for_backward({row, col, ft, el, er, edges});
     ctx->saved_data["slope"] = slope;
     ctx->saved_data["words"] = words;
-    ctx->saved_data["edges"] = edges;
     return out;
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto v = ctx->get_saved_variables();
     auto [g_ft, g_el, g_er] = gat_backward(v[0], v[1], v[2], v[3], v[4], grads[0], ctx->saved_data["slope"].toDouble(),
-                                           ctx->saved_data["words"].toTensor(), ctx->saved_data["edges"].toTensor());
+                                           ctx->saved_data["words"].toTensor(), v[5]);
     return {Tensor(), Tensor(), g_ft, g_el, g_er, Tensor(), Tensor(), Tensor()};
   }
 };

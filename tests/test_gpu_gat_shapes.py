@@ -168,3 +168,27 @@ def test_source_rows_of_many_edges(dtype, H, Dh):
     want.index_add_(0, row, attn.double() * go.double()[col])
     assert col.numel() >= 200_000
     _near(got, host(want), dtype, "grad_ft")
+
+
+def test_what_the_forward_saved_goes_with_the_backward():
+    S, f, H, Dh = 20_000, 10, 8, 16
+    row = torch.randint(0, S, (S * f,), device="cuda")
+    col = torch.arange(S, device="cuda").repeat_interleave(f)
+    leaves = [torch.randn(shape, device="cuda", requires_grad=True) for shape in ((S, H, Dh), (S, H, 1), (S, H, 1))]
+    go = torch.randn((S, H, Dh), device="cuda")
+    want = torch.autograd.grad(apt_b200.GATEdgeSoftmaxSum.apply(row, col, *leaves, S, 0.2), leaves, go)
+    saved = S * f * H * 4
+    out = apt_b200.GATEdgeSoftmaxSum.apply(row, col, *leaves, S, 0.2)
+    before = torch.cuda.memory_allocated()
+    grads = torch.autograd.grad(out, leaves, go)
+    held = sum(g.numel() * 4 for g in grads)
+    assert torch.cuda.memory_allocated() <= before + held - saved + (1 << 20)        # `out` and its graph are still there
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, leaves, go)
+    # and to wherever a caller's hooks put what is saved
+    with torch.autograd.graph.save_on_cpu():
+        base = torch.cuda.memory_allocated()
+        out = apt_b200.GATEdgeSoftmaxSum.apply(row, col, *leaves, S, 0.2)
+        assert torch.cuda.memory_allocated() <= base + out.numel() * 4 + (1 << 20)
+    for a, b in zip(torch.autograd.grad(out, leaves, go), want):
+        assert (a - b).abs().max() <= 1e-5 * b.abs().max()
