@@ -59,17 +59,6 @@ def _layer(dst_buf, rel, uniq, fanout, slot):
     return rel, uniq, _coo_col(dst_buf.numel(), dst_buf.numel(), fanout, rel.device), fanout, slot
 
 
-_ARANGE = {}
-
-
-def _arange(n, device):
-    """arange(n) as a prefix of a cached longer one."""
-    t = _ARANGE.get(device)
-    if t is None or t.numel() < n:
-        t = _ARANGE[device] = torch.arange(max(2 * n, 1 << 14), device=device)
-    return t[:n]
-
-
 def create_block(seeds: torch.Tensor, neighbors: torch.Tensor, fanout: int) -> Block:
     unique_frontier, indices = ops.relabel_csc(seeds, neighbors)
     coo_col = torch.arange(0, seeds.numel(), device=indices.device).repeat_interleave(fanout)
@@ -753,6 +742,9 @@ class SPVirtualSampler(_GraphReplay):
         beside = ws == 1 and not with_dst and not st.profiling
         with st.beside(0) if beside else contextlib.nullcontext():
             unique_frontier, _ = ops._unique_enqueue(sorted_vir, n_word, 0, ws * max(s_max, 1), uf_word, "unique_vir")
+            # the two sides of block1's edges: tensors of their own, which a caller may change
+            arange_src = torch.arange(unique_frontier.numel(), device=dev)
+            arange_dst = unique_frontier.clone() if ws == 1 and not with_dst else None   # owner 0: its destination's index
         dst_sorted = None
         if with_dst:
             dst_sorted, dst_pos, _, _ = ops._bucket(cur, cur_n)
@@ -806,9 +798,7 @@ class SPVirtualSampler(_GraphReplay):
         if beside:
             st.join(0)
             st.join(1)
-        if ws == 1 and not with_dst:
-            arange_dst = unique_frontier        # owner 0: a virtual node is its destination's index
-        else:
+        if arange_dst is None:
             arange_dst = torch.remainder(unique_frontier, cur_n if cur_n is not None else max(s_max, 1))
         # the input nodes (the reference's torch.cat of destinations and received neighbours)
         us_word = st.word(self._US)
@@ -826,16 +816,16 @@ class SPVirtualSampler(_GraphReplay):
             publish()
         rows = self._late_rows(input_nodes, in_word, cur_n, rows) if prefetch else None
         return dict(layers=layers, cur=cur, nbr=nbr, sorted_all=sorted_all, packed=packed,
-                    unique_frontier=unique_frontier, arange_dst=arange_dst, vir_src=vir_src, ori_src=ori_src,
+                    unique_frontier=unique_frontier, arange_src=arange_src, arange_dst=arange_dst, vir_src=vir_src, ori_src=ori_src,
                     unique_src=unique_src, a_src=a_src, unique_dst=unique_dst, a_dst=a_dst, dst_sorted=dst_sorted,
                     recv_dst=recv_dst, input_nodes=input_nodes, rows=rows)
 
     _CUT = ("unique_frontier", "unique_src", "arange_dst", "a_src", "a_dst", "input_nodes", "nbr", "sorted_all", "packed", "vir_src",
-            "ori_src", "unique_dst")
+            "ori_src", "unique_dst", "arange_src")
 
     def _outline(self, seeds, b):
         hops = _native.Hops(b["layers"], Block)
-        views = _native.wholes([b[name] for name in self._CUT] + [_arange(b["unique_frontier"].numel(), seeds.device)])
+        views = _native.wholes([b[name] for name in self._CUT])
         uf, us, arange_dst, a_src, a_dst = views[:5]
         outer = Block(a_src, a_dst, 0, 0, us, self.fanouts[0]), Block(views[12], arange_dst, 0, 0, uf, self.fanouts[0])
         rows = None if b["rows"] is None else _native.wholes([b["rows"]])[0]

@@ -278,3 +278,24 @@ def test_committed_strategy_fixture_one_rank():
         assert np.array_equal(host(v), want[f"ws1/0/nfp/{name}"]), name
     ops.check_status()
     reset_world()
+
+
+@pytest.mark.parametrize("model,with_dst", [("SAGE", False), ("GCN", False), ("SAGE", True)])
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_block_columns_may_be_changed_in_place(model, with_dst, use_graph):
+    n, indptr, indices = small_graph(scale=12, edge_factor=8)
+    install_graph(indptr, indices)
+    reset_world(1, 0)
+    ops.register_min_vids(torch.tensor([0, n]))
+    smp = SPVirtualSampler(0, [5, 3], model=model, shuffle_with_dst=with_dst, use_graph=use_graph)
+    seeds = dev(np.arange(0, 400, 2, dtype=I64))
+    for k in range(5):
+        ops.set_sampling(key=3, call_id=0)
+        block1 = smp.sample(None, seeds)[2][1]
+        assert torch.equal(block1.coo_row, torch.arange(block1.num_src, device="cuda"))
+        assert torch.equal(block1.coo_col, block1.src_ids % block1.num_dst)
+        ids = block1.src_ids.clone()
+        block1.coo_row.add_(1000)
+        block1.coo_col.fill_(-1)
+        assert torch.equal(block1.src_ids, ids) and torch.equal(smp.last["unique_frontier"], ids)
+    ops.check_status()
