@@ -162,18 +162,19 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
     for (int h0 = 0; h0 < num_heads; h0 += hpp) {
       const int h = h0 + rh;
       const bool rows = h < num_heads;
-      // lanes without a slice read one that exists and contribute zero
+      // lanes without a slice read one that exists and contribute nothing (no zero times what may be infinite)
       const int64_t col = (int64_t)(rows ? h : h0) * head_dim;
       const T* const grad = grad_out + (int64_t)d * num_heads * head_dim + col;
       F2 g[Acc<VE>::P];      // the gradient's slice, unpacked
       int at = 0;
+      bool mine = false;
       auto block = [&](int c0) {
         at = min(c0 + p, nvh - 1) * VE;
+        mine = c0 + p < nvh;
         const Raw<T, VE> raw = load_raw<T, VE>(grad + at);
 #pragma unroll
         for (int q = 0; q < Acc<VE>::P; ++q) {
           if constexpr (VE > 1) g[q] = pair_of(raw, q); else g[q] = f2_pack(raw.get(0), 0.f);
-          if (c0 + p >= nvh) g[q] = 0ull;
         }
       };
       block(0);
@@ -206,7 +207,7 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
               }
               float lo, hi;
               f2_unpack(pair, lo, hi);
-              dt[u] += lo + hi;
+              dt[u] += mine ? lo + hi : 0.f;
             }
           }
           float* const out = dots + (int64_t)(base + j0 + epi) * num_heads + h;

@@ -192,3 +192,29 @@ def test_what_the_forward_saved_goes_with_the_backward():
         assert torch.cuda.memory_allocated() <= base + out.numel() * 4 + (1 << 20)
     for a, b in zip(torch.autograd.grad(out, leaves, go), want):
         assert (a - b).abs().max() <= 1e-5 * b.abs().max()
+
+
+@pytest.mark.parametrize("H,Dh", [(1, 47), (3, 5), (2, 40), (1, 300)])
+def test_infinite_rows_stay_where_they_belong(H, Dh):
+    # one source's last column is infinite: its edge's gradient is not a number, the other edges' are infinite or, at other
+    # destinations, what they are without it, in every head width (lanes beyond a head's last slice read that slice)
+    row, col, ft, el, er, go = _inputs([4, 3, 5], H, Dh, torch.float32, 3)
+    row[:] = np.arange(len(row))
+    ft[1, :, -1] = np.inf
+    go[:, :, -1] = 1.0
+    args = [dev(x) for x in (row, col, ft, el, er)]
+    g_ft, g_el, g_er = ops.gat_edge_softmax_sum_backward(*args, dev(go), 0.2)
+    f, l, r, g = (torch.from_numpy(x).double() for x in (ft, el, er, go))
+    rows, cols = torch.from_numpy(row), torch.from_numpy(col)
+    raw = l[rows] + r[cols]
+    s = torch.nn.functional.leaky_relu(raw, 0.2)
+    a = torch.cat([torch.softmax(s[cols == d], 0) for d in range(3)])
+    dot = (g[cols] * f[rows]).sum(-1)
+    t = torch.stack([(a * dot)[cols == d].sum(0) for d in range(3)])
+    gs = a * (dot - t[cols]) * torch.where(raw > 0, 1.0, 0.2)
+    want = torch.zeros(l.shape, dtype=torch.float64).index_add_(0, rows, gs)
+    got = g_el.cpu().double()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and int(want.isinf().sum()) == 3 * H
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    assert bool(((got - want)[fine].abs() <= 1e-5 * want[fine].abs().max()).all()) and bool(g_ft.isfinite().all())
