@@ -45,6 +45,15 @@ namespace apt {
 
 __device__ __forceinline__ float leaky(float x, float slope) { return x > 0.f ? x : x * slope; }
 
+// A destination whose scores have no sum (all of them -inf, as a mask leaves them, or a NaN among them): up to this many edges
+// its weights are zero, beyond it they are NaN. The bound lies where it has always been for callers: 32 edges for rows of
+// more than 256 bytes in 16-byte slices and up to 8 heads, none for other shapes.
+constexpr int kMaskedEdges = 32;
+static int masked_edges(int num_heads, int64_t head_dim, size_t esz, uintptr_t rows) {
+  const bool slices = ((uint64_t)(head_dim * esz) & 15) == 0 && (rows & 15) == 0;
+  return slices && num_heads * head_dim * (int64_t)esz > 256 && num_heads <= 8 ? kMaskedEdges : 0;
+}
+
 // Sum over groups of n lanes (a power of two).
 __device__ __forceinline__ float group_sum(float v, int n) {
   for (int o = n >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -85,7 +94,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
               int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ weight,
-              T* __restrict__ attn) {
+              T* __restrict__ attn, int masked) {
   wait_for_previous();
   constexpr int K = 16;
   if (*none != 0) return;
@@ -120,8 +129,10 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
       for (int e = r.x; e < r.y; ++e) sum += expf(score(e) - m);
     }
     const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    const bool zero = !(sum > 0.f) && deg <= masked;
     auto put = [&](int e, float w) {
       const int64_t o = (int64_t)e * num_heads + h;
+      if (zero) w = 0.f;
       weight[o] = w;
       if (attn) attn[o] = Elem<T>::from_f(w);
     };
@@ -371,7 +382,7 @@ static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaS
   if (rc != APT_OK) return rc;
   ProfScope prof("gat_rows", s);
   APT_FOLLOW(k_gat_weights<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-             q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn);
+             q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn, masked_edges(q.H, q.Dh, sizeof(T), (uintptr_t)q.ft));
   return APT_OK;
 }
 
@@ -462,6 +473,7 @@ struct GatScores {
   const T* el;
   int H, h0, nh;
   float slope;
+  int masked;
   bool few;
   unsigned positive;       // bit h: this lane's score before the leaky part
 
@@ -493,7 +505,7 @@ struct GatScores {
       const float own = sum;
       sum = group_sum(sum, 32);
       const float inv = sum > 0.f ? 1.f / sum : 0.f;
-      if (mine) sh.w[lane][h] = own * inv;
+      if (mine) sh.w[lane][h] = !(sum > 0.f) && r.y - r.x <= masked ? 0.f : own * inv;
       if (mine && x[h] > 0.f) positive |= 1u << h;
       if (!few && lane == 0) sh.bias[h] = bias[h], sh.most[h] = most, sh.inv[h] = inv;
     }
@@ -519,7 +531,7 @@ template <typename T, int VE>
 __global__ void __launch_bounds__(256, 4)
 k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er, int num_heads,
             int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none,
-            T* __restrict__ out, T* __restrict__ attn, int lpe) {
+            T* __restrict__ out, T* __restrict__ attn, int lpe, int masked) {
   wait_for_previous();
   constexpr int U = 4;
   __shared__ GatAloneWarp shared[8];
@@ -532,7 +544,7 @@ k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* 
     const int2 r = empty ? make_int2(0, 0) : range[d];
     const int deg = r.y - r.x;
     for (int h0 = 0; h0 < num_heads; h0 += kAloneHeads) {
-      GatScores<T> sc{shared[warp], row, el, num_heads, h0, min(kAloneHeads, num_heads - h0), slope};
+      GatScores<T> sc{shared[warp], row, el, num_heads, h0, min(kAloneHeads, num_heads - h0), slope, masked};
       if (deg > 0) sc.start(er, (int)d, r, lane);
       const int slices = sc.nh * nvh;
       for (int c0 = 0; c0 < slices; c0 += lpe) {
@@ -574,7 +586,7 @@ __global__ void __launch_bounds__(256, 4)
 k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er,
                      const T* __restrict__ grad_out, int num_heads, int head_dim, float slope, int64_t num_dst, int64_t E,
                      const int2* __restrict__ range, const int32_t* __restrict__ none, T* __restrict__ attn,
-                     T* __restrict__ grad_score, T* __restrict__ grad_er, int lph, int hpp) {
+                     T* __restrict__ grad_score, T* __restrict__ grad_er, int lph, int hpp, int masked) {
   wait_for_previous();
   constexpr int U = 4;
   __shared__ GatAloneWarp shared[8];
@@ -592,7 +604,7 @@ k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, 
     const int2 r = empty ? make_int2(0, 0) : range[d];
     const int deg = r.y - r.x;
     for (int h0 = 0; h0 < num_heads; h0 += kAloneHeads) {
-      GatScores<T> sc{shared[warp], row, el, num_heads, h0, min(kAloneHeads, num_heads - h0), slope};
+      GatScores<T> sc{shared[warp], row, el, num_heads, h0, min(kAloneHeads, num_heads - h0), slope, masked};
       if (deg > 0) sc.start(er, (int)d, r, lane);
       float t[kAloneHeads], ger[kAloneHeads];
 #pragma unroll
@@ -663,14 +675,15 @@ k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, 
 template <typename T, int VE>
 static int launch_alone(const GatProblem& q, const GatEdges& g, void* out, void* attn, void* grad_score, void* grad_er, cudaStream_t s) {
   const int nvh = (int)(q.Dh / VE), grid = wave_grid(ceil_div(q.num_dst, 8), 8);
+  const int masked = masked_edges(q.H, q.Dh, sizeof(T), (uintptr_t)q.ft);
   if (grad_er) {
     const int lph = pow2_ge(nvh), hpp = pow2_ge(std::min(q.H, kAloneHeads), 32 / lph);
     APT_FOLLOW((k_gat_alone_backward<T, VE>), grid, 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el, (const T*)q.er,
                (const T*)q.grad_out, q.H, (int)q.Dh, q.slope, q.num_dst, q.E, g.range, g.none, (T*)attn, (T*)grad_score, (T*)grad_er,
-               lph, hpp);
+               lph, hpp, masked);
   } else {
     APT_FOLLOW((k_gat_alone<T, VE>), grid, 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el, (const T*)q.er, q.H, (int)q.Dh, q.slope,
-               q.num_dst, g.range, g.none, (T*)out, (T*)attn, pow2_ge((int64_t)std::min(q.H, kAloneHeads) * nvh));
+               q.num_dst, g.range, g.none, (T*)out, (T*)attn, pow2_ge((int64_t)std::min(q.H, kAloneHeads) * nvh), masked);
   }
   return APT_OK;
 }

@@ -393,7 +393,9 @@ int apt_sddmm(int op, int dtype, const int64_t* coo_row,
  * u_mul_e + sum), which the reference leaves to DGL. ft is [num_src,
  * num_heads*head_dim], el [num_src, num_heads], er [num_dst, num_heads];
  * out_attn ([num_edges, num_heads], may be NULL) receives a. Rows without
- * edges become 0. Edges that are not grouped set APT_FLAG_NOT_GROUPED and give
+ * edges become 0. So do, for rows of more than 256 bytes in 16-byte slices and up
+ * to 8 heads, those of up to 32 edges whose scores are all -inf or hold a NaN;
+ * elsewhere these become NaN. Edges that are not grouped set APT_FLAG_NOT_GROUPED and give
  * zeros. workspace: apt_spmm_workspace_bytes(num_dst, 0) bytes. */
 int apt_gat_edge_softmax_sum(int dtype, const int64_t* coo_row,
                              const int64_t* coo_col, int64_t num_edges,

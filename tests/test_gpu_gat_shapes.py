@@ -218,3 +218,34 @@ def test_infinite_rows_stay_where_they_belong(H, Dh):
     assert torch.equal(got[got.isinf()], want[want.isinf()])
     fine = want.isfinite()
     assert bool(((got - want)[fine].abs() <= 1e-5 * want[fine].abs().max()).all()) and bool(g_ft.isfinite().all())
+
+
+@pytest.mark.parametrize("dtype,H,Dh,zero", [(torch.bfloat16, 4, 64, True), (torch.float32, 8, 16, True), (torch.float32, 2, 64, True),
+                                             (torch.float32, 1, 8, False), (torch.float32, 16, 16, False), (torch.bfloat16, 2, 64, False)])
+@pytest.mark.parametrize("edges", [1, 15, 16, 17, 32, 33])
+def test_masked_destinations(dtype, H, Dh, zero, edges):
+    # every score of destination 1 is -inf: zeros up to 32 edges of wide rows, NaN elsewhere, and nothing for its neighbours
+    row, col, ft, el, er, go = _inputs([5, edges, 4], H, Dh, dtype, 5)
+    row[:] = np.arange(len(row)) % 9
+    row[5:5 + edges] = 9 + np.arange(edges) % 31
+    el[9:] = -np.inf
+    leaves = [dev(x, dtype).requires_grad_() for x in (ft, el, er)]
+    out = apt_b200.GATEdgeSoftmaxSum.apply(dev(row), dev(col), *leaves, 3, 0.2)
+    grads = torch.autograd.grad(out, leaves, dev(go, dtype))
+    zero = zero and edges <= 32
+    masked = out[1].float()
+    assert not bool(masked.any()) if zero else bool(masked.isnan().all())
+    assert bool(out[0::2].isfinite().all()) and bool(out[0::2].any())
+    assert bool(grads[0][:9].isfinite().all()) and bool(grads[1][:9].isfinite().all()) and bool(grads[2][0::2].isfinite().all())
+    if zero:
+        assert not bool(grads[0][9:].any()) and not bool(grads[2][1].any())
+    # the entry points without a buffer agree
+    t = [x.detach() for x in (dev(row), dev(col), *leaves)]
+    alone = torch.full((3, H, Dh), 9.0, device="cuda", dtype=dtype)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nbytes = lib.apt_spmm_workspace_bytes(3, 0)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    check(lib.apt_gat_edge_softmax_sum(CODE[dtype], *(x.data_ptr() for x in t[:2]), len(row), *(x.data_ptr() for x in t[2:]), H, Dh, 0.2, 3,
+                                       alone.data_ptr(), None, ws.data_ptr(), nbytes, status.data_ptr(), None))
+    torch.cuda.synchronize()
+    assert bool((alone[1].isnan() == out[1].isnan()).all()) and bool(((alone - out).float().nan_to_num().abs() <= 2e-2).all())
