@@ -297,6 +297,8 @@ class Plan {
     int64_t* const to = seeds_buf_.mutable_data_ptr<int64_t>();
     int64_t count = from != to ? seeds.numel() : 0;
     py::gil_scoped_release nogil;
+    // a launch nobody waited for (its iterator was given up): its seeds, which go below, may still be read
+    if (!waited_) cuda_ok(cudaEventSynchronize(done_), "cudaEventSynchronize");
     if (own_) {
       // behind everything the caller's stream holds so far: the seeds' producer, the consumer of the last results
       cuda_ok(cudaEventRecord(ready_, cur), "cudaEventRecord");
@@ -311,8 +313,9 @@ class Plan {
     check(apt_stage_replay(from, count, to, call_base, ++sequence_, replay_in_.mutable_data_ptr<int64_t>(), s));
     cuda_ok(cudaGraphLaunch(exec_, s), "cudaGraphLaunch");
     cuda_ok(cudaEventRecord(done_, s), "cudaEventRecord");
-    seeds_ = seeds;       // the copy reads it when the stream gets there
     stream_ = s;
+    waited_ = false;
+    seeds_ = seeds;       // the copy reads it when the stream gets there
   }
   // Until the counts of the last launch are in host_words; returns the status flags.
   int64_t wait() {
@@ -320,6 +323,7 @@ class Plan {
     const int64_t* const h = host_words_.const_data_ptr<int64_t>();
     py::gil_scoped_release nogil;
     check(apt_wait_published(h, count, sequence_, stream_));
+    waited_ = true;
     return (h[count - 1] & 0xffffffff) | apt_pending_flags();
   }
   void finish() {
@@ -341,6 +345,7 @@ class Plan {
   cudaStream_t own_, stream_ = nullptr;
   cudaEvent_t done_, ready_;
   int64_t sequence_ = 0;
+  bool waited_ = true;
 };
 
 // The first n rows. Below autograd: a sampler's buffers have no history to carry on, and the view costs half as much.

@@ -159,3 +159,36 @@ def test_a_batch_keeps_its_counts_to_itself(kind):
     with pytest.raises(RuntimeError, match="not grouped"):
         smp.sample(None, _seeds(n, 3))
     ops.check_status()
+
+
+def test_an_iterator_given_up_leaves_nothing_behind():
+    # its batches may not have begun when the next iterator launches on the same buffer sets; their seeds' memory is not
+    # handed out before they have
+    n = _install()
+    table, _ = _table(n, 1.0)
+    smp = apt_b200.MixedNeighborSampler(0, [4, 3], lanes=2)
+    batches = [_seeds(n, k, 200) for k in range(8)]
+    for got in smp.sample_iter(None, batches):
+        ops.load_subtensor(got[0])
+    torch.cuda.synchronize()
+
+    junk = []
+
+    def broken():
+        for k in range(2):
+            yield batches[k].clone()
+        raise KeyError("no more")
+
+    def fresh():
+        for b in batches:
+            yield b.clone()
+            junk.append(torch.full((200,), -5, device="cuda"))         # takes whatever memory has been given back
+
+    for lane in (1, 2):
+        with torch.cuda.stream(ops.STATE.lane_stream(lane)):
+            torch.cuda._sleep(400_000_000)
+    with pytest.raises(KeyError):
+        list(smp.sample_iter(None, broken()))
+    for got in smp.sample_iter(None, fresh()):
+        assert torch.equal(ops.load_subtensor(got[0]), table[got[0]])
+    ops.check_status()
