@@ -258,6 +258,21 @@ struct GatFunction : public torch::autograd::Function<GatFunction> {
 };
 
 // ------------------------------------------------------------------------------------------------ samplers
+// Page-locked words, also while some stream is being captured.
+Tensor pinned_words(int64_t count) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cuda_ok(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+  Tensor words;
+  try {
+    words = at::zeros({count}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  } catch (...) {
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    throw;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return words;
+}
+
 // Copies a word block to the host (one kernel, polled for), the last word, the status flags, from the end of `status`, and
 // returns the flags.
 int64_t read_words(const Tensor& words, const Tensor& status, const Tensor& host, int64_t sequence) {
@@ -587,6 +602,7 @@ PYBIND11_MODULE(_native, m) {
       .def("wait", &Plan::wait)
       .def("finish", &Plan::finish)
       .def("order_current_stream", &Plan::order_current_stream);
+  m.def("pinned_words", &pinned_words);
   m.def("read_words", &read_words);
   py::class_<Hops>(m, "Hops")
       .def(py::init<const py::list&, const py::object&>())

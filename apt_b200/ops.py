@@ -203,12 +203,18 @@ class NPCState:
 
     def lane_words(self) -> torch.Tensor:
         """The word block of the calling thread's lane, its status flags among them."""
-        pair = self._lane_words.get(self.lane)
-        if pair is None or pair[0].device != self.device():
-            pair = (torch.zeros(self.NUM_WORDS, dtype=torch.int64, device=self.device()),
-                    torch.zeros(self.NUM_WORDS + 1, dtype=torch.int64).pin_memory())
-            self._lane_words[self.lane] = pair
-        return pair[0]
+        words = self._lane_words.get(self.lane)
+        if words is None or words.device != self.device():
+            words = self._lane_words[self.lane] = torch.zeros(self.NUM_WORDS, dtype=torch.int64, device=self.device())
+        return words
+
+    def host_words(self) -> torch.Tensor:
+        """The calling thread's page-locked copy of a word block, with a sequence number behind it. Threads that read at the
+        same time have one each: a reader polls its copy for its own number."""
+        host = getattr(self._tls, "host", None)
+        if host is None:
+            host = self._tls.host = _native.pinned_words(self.NUM_WORDS + 1)
+        return host
 
     def word(self, k: int) -> torch.Tensor:
         """One-element view of device word k (a device-side count)."""
@@ -220,8 +226,7 @@ class NPCState:
     def read_words(self) -> torch.Tensor:
         """Copies the device words to the host (one stream sync) and raises on
         any status flag except zero-degree, which is only a notice."""
-        status = self.lane_words()
-        host = self._lane_words[self.lane][1]
+        status, host = self.lane_words(), self.host_words()
         self.check_flags(_native.read_words(self.words(), status, host, self.next_sequence()))
         return host
 

@@ -1113,7 +1113,7 @@ class DPNeighborSampler:
         key = ops._tables_key() if features is not None else None
         blocks, rows, pending, flags = _native.dp_sample(
             ids, order, g.adj_pos_map, g.num_total_nodes, g.dev_indptr, g.dev_indices, g.uva_indptr, g.uva_indices, st.sample_key,
-            call, ops._relabel_workspace(bound), words, st._lane_words[st.lane][1], st.next_sequence(), features,
+            call, ops._relabel_workspace(bound), words, st.host_words(), st.next_sequence(), features,
             _PREFETCH_LIMIT_BYTES, Block)
         if flags:
             st.check_flags(flags)
