@@ -29,7 +29,8 @@
 //                   their own the first and the last pass took 23 + 16 us.
 //   k_gat_source    grad_el in T
 //
-// k_gat_alone and k_gat_alone_backward serve the two entry points that have no buffer for weights.
+// k_gat_alone and k_gat_alone_backward serve the two entry points that have no buffer for weights, k_gat_narrow forwards of
+// narrow rows that nobody will ask for a backward.
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
@@ -581,6 +582,50 @@ k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* 
   }
 }
 
+// Narrow rows (up to APT_GAT_NARROW_BYTES in 16-byte slices), forward: a lane to a slice, as many lanes to a destination, and every lane works
+// its head's scores out itself. There are few lanes to share them, and what it saves is the weights' way through memory and a
+// launch. 30 000 destinations of 3 / 10 / 25 edges, with the weights apart -> here, us: fp32 x 32 16 / 33 / 47 -> 12 / 18 / 33,
+// bf16 8 x 8 22 / 37 / 59 -> 12 / 20 / 37, fp32 4 x 16 23 / 36 / 57 -> 16 / 27 / 49. Wider rows and other slices gain by the weights
+// apart, against one such kernel: bf16 4 x 64 35 / 45 / 67 -> 27 / 37 / 72, fp16 2 x 10 27 / 41 / 79 -> 18 / 27 / 45.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_gat_narrow(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er, int num_heads,
+             int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none,
+             T* __restrict__ out, T* __restrict__ attn, int lpe) {
+  wait_for_previous();
+  constexpr int VE = 16 / sizeof(T);
+  const int c = threadIdx.x & (lpe - 1), dim = num_heads * head_dim;
+  if (c * VE >= dim) return;
+  const int h = c * VE / head_dim;
+  const uint32_t row_bytes = (uint32_t)(dim * sizeof(T));
+  const bool empty = *none != 0, writes_attn = attn && c * VE % head_dim == 0;
+  const T* const lane_ft = ft + c * VE;
+  const T* const lane_el = el + h;
+  const int per_block = 256 / lpe;
+  for (int64_t d = (int64_t)blockIdx.x * per_block + threadIdx.x / lpe; d < num_dst; d += (int64_t)gridDim.x * per_block) {
+    const int2 r = empty ? make_int2(0, 0) : range[d];
+    const float bias = Elem<T>::to_f(er[d * num_heads + h]);
+    auto score = [&](int64_t src) { return leaky(Elem<T>::to_f(lane_el[src * num_heads]) + bias, slope); };
+    float most = -INFINITY, sum = 0.f;
+#pragma unroll 4
+    for (int e = r.x; e < r.y; ++e) most = fmaxf(most, score(row[e]));
+#pragma unroll 4
+    for (int e = r.x; e < r.y; ++e) sum += expf(score(row[e]) - most);
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    Acc<VE> acc;
+    acc.zero();
+#pragma unroll 4
+    for (int e = r.x; e < r.y; ++e) {
+      const int64_t src = row[e];
+      const Raw<T, VE> v = load_raw<T, VE>(at_row(lane_ft, (uint32_t)src, row_bytes));
+      const float w = expf(score(src) - most) * inv;
+      if (writes_attn) attn[(int64_t)e * num_heads + h] = Elem<T>::from_f(w);
+      acc.fma(v, w);
+    }
+    store_pack<T, VE>(out + d * dim + c * VE, acc.template rounded<T>());
+  }
+}
+
 template <typename T, int VE>
 __global__ void __launch_bounds__(256, 4)
 k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er,
@@ -681,6 +726,10 @@ static int launch_alone(const GatProblem& q, const GatEdges& g, void* out, void*
     APT_FOLLOW((k_gat_alone_backward<T, VE>), grid, 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el, (const T*)q.er,
                (const T*)q.grad_out, q.H, (int)q.Dh, q.slope, q.num_dst, q.E, g.range, g.none, (T*)attn, (T*)grad_score, (T*)grad_er,
                lph, hpp, masked);
+  } else if (VE * sizeof(T) == 16 && q.H * q.Dh * (int64_t)sizeof(T) <= APT_GAT_NARROW_BYTES) {
+    const int lpe = pow2_ge(q.H * nvh);
+    APT_FOLLOW((k_gat_narrow<T>), wave_grid(ceil_div(q.num_dst, 256 / lpe), 8), 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el,
+               (const T*)q.er, q.H, (int)q.Dh, q.slope, q.num_dst, g.range, g.none, (T*)out, (T*)attn, lpe);
   } else {
     APT_FOLLOW((k_gat_alone<T, VE>), grid, 256, 0, s, q.row, (const T*)q.ft, (const T*)q.el, (const T*)q.er, q.H, (int)q.Dh, q.slope,
                q.num_dst, g.range, g.none, (T*)out, (T*)attn, pow2_ge((int64_t)std::min(q.H, kAloneHeads) * nvh), masked);

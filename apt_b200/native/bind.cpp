@@ -202,15 +202,25 @@ GatShape gat_shape(const char* who, const Tensor& row, const Tensor& ft, const T
   return {code, row.numel(), num_src, num_dst, heads, ft.numel() / std::max<int64_t>(num_src * heads, 1)};
 }
 
-// Results of the forward: sums, attention (when asked for) and the edge buffer that a backward of the same block can use.
+// Results of the forward: sums, attention (when asked for) and, for a backward of the same block, the edge buffer. Without one
+// to come, narrow rows are summed in one kernel that leaves no weights.
 std::tuple<Tensor, Tensor, Tensor> gat_forward(const Tensor& coo_row, const Tensor& coo_col, const Tensor& ft_in, const Tensor& el_in,
                                                const Tensor& er_in, int64_t num_dst, double slope, bool want_attention,
-                                               const Tensor& words) {
+                                               const Tensor& words, bool want_edges) {
   const Tensor row = ids(coo_row, "coo_row"), col = ids(coo_col, "coo_col");
   const Tensor ft = cuda(ft_in, "ft"), el = cuda(el_in, "el"), er = cuda(er_in, "er");
   const GatShape g = gat_shape("gat_edge_softmax_sum", row, ft, el, er, num_dst);
   Tensor out = at::empty({num_dst, g.heads, g.head_dim}, ft.options()), attn;
   if (want_attention) attn = at::empty({g.edges, g.heads, 1}, ft.options());
+  const int64_t size = ft.element_size(), row_bytes = g.heads * g.head_dim * size;
+  if (!want_edges && row_bytes <= APT_GAT_NARROW_BYTES && g.head_dim * size % 16 == 0 && (uintptr_t)data(ft) % 16 == 0) {
+    const size_t bytes = apt_spmm_workspace_bytes(num_dst, 0);
+    const Tensor ws = scratch(ft, bytes);
+    check(apt_gat_edge_softmax_sum(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), (int)g.heads, g.head_dim,
+                                   (float)slope, num_dst, mut(out), want_attention ? mut(attn) : nullptr, ws.mutable_data_ptr(),
+                                   bytes, status_word(words), stream()));
+    return {out, attn, Tensor()};
+  }
   const size_t bytes = apt_gat_edges_bytes(num_dst, g.edges, (int)g.heads);
   const Tensor edges = scratch(ft, bytes);
   check(apt_gat_forward(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), (int)g.heads, g.head_dim, (float)slope,
@@ -242,8 +252,8 @@ std::tuple<Tensor, Tensor, Tensor> gat_backward(const Tensor& coo_row, const Ten
 // go when the inputs go.
 struct GatFunction : public torch::autograd::Function<GatFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& row, const Tensor& col, const Tensor& ft,
-                        const Tensor& el, const Tensor& er, int64_t num_dst, double slope, const Tensor& words) {
-    auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, false, words);
+                        const Tensor& el, const Tensor& er, int64_t num_dst, double slope, const Tensor& words, bool backward) {
+    auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, false, words, backward);
     ctx->save_for_backward({row, col, ft, el, er, edges});
     ctx->saved_data["slope"] = slope;
     ctx->saved_data["words"] = words;
@@ -252,8 +262,8 @@ struct GatFunction : public torch::autograd::Function<GatFunction> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto v = ctx->get_saved_variables();
     auto [g_ft, g_el, g_er] = gat_backward(v[0], v[1], v[2], v[3], v[4], grads[0], ctx->saved_data["slope"].toDouble(),
-                                           ctx->saved_data["words"].toTensor(), v[5]);
-    return {Tensor(), Tensor(), g_ft, g_el, g_er, Tensor(), Tensor(), Tensor()};
+                                           ctx->saved_data["words"].toTensor(), v[5].defined() ? OptTensor(v[5]) : std::nullopt);
+    return {Tensor(), Tensor(), g_ft, g_el, g_er, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -635,7 +645,7 @@ PYBIND11_MODULE(_native, m) {
   m.def("rows_scatter", &rows_scatter);
   m.def("gat_forward", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
                           int64_t num_dst, double slope, bool want_attention, const Tensor& words) {
-    auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, want_attention, words);
+    auto [out, attn, edges] = gat_forward(row, col, ft, el, er, num_dst, slope, want_attention, words, false);
     return std::make_tuple(out, attn);
   });
   m.def("gat_backward", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
@@ -644,6 +654,7 @@ PYBIND11_MODULE(_native, m) {
   });
   m.def("gat_apply", [](const Tensor& row, const Tensor& col, const Tensor& ft, const Tensor& el, const Tensor& er,
                         int64_t num_dst, double slope, const Tensor& words) {
-    return GatFunction::apply(row, col, ft, el, er, num_dst, slope, words);
+    const bool backward = at::GradMode::is_enabled() && (ft.requires_grad() || el.requires_grad() || er.requires_grad());
+    return GatFunction::apply(row, col, ft, el, er, num_dst, slope, words, backward);
   });
 }

@@ -397,6 +397,7 @@ int apt_sddmm(int op, int dtype, const int64_t* coo_row,
  * to 8 heads, those of up to 32 edges whose scores are all -inf or hold a NaN;
  * elsewhere these become NaN. Edges that are not grouped set APT_FLAG_NOT_GROUPED and give
  * zeros. workspace: apt_spmm_workspace_bytes(num_dst, 0) bytes. */
+#define APT_GAT_NARROW_BYTES 256 /* rows up to here, in 16-byte slices: no faster with a buffer for weights (apt_gat_forward) */
 int apt_gat_edge_softmax_sum(int dtype, const int64_t* coo_row,
                              const int64_t* coo_col, int64_t num_edges,
                              const void* ft, const void* el, const void* er,

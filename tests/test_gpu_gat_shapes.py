@@ -249,3 +249,38 @@ def test_masked_destinations(dtype, H, Dh, zero, edges):
                                        alone.data_ptr(), None, ws.data_ptr(), nbytes, status.data_ptr(), None))
     torch.cuda.synchronize()
     assert bool((alone[1].isnan() == out[1].isnan()).all()) and bool(((alone - out).float().nan_to_num().abs() <= 2e-2).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,Dh", [(1, 8), (2, 8), (3, 16), (8, 8), (1, 64), (16, 4), (1, 128), (2, 40)])
+@pytest.mark.parametrize("lengths", [[7] * 40, RAGGED], ids=["fixed", "ragged"])
+def test_forward_without_a_backward(dtype, H, Dh, lengths):
+    # rows of up to 256 bytes are summed by a kernel of their own, on both sides of that bound
+    row, col, ft, el, er, _ = _inputs(lengths, H, Dh, dtype, H + Dh)
+    S = len(lengths)
+    args = dev(row), dev(col), dev(ft, dtype), dev(el, dtype), dev(er, dtype)
+    want, want_a = orc.gat_edge_softmax_sum(row, col, ft, el, er, S, 0.2)
+    out, attn = ops.gat_edge_softmax_sum(*args, S, 0.2, return_attention=True)
+    _near(out, want, dtype, "out")
+    _near(attn, want_a, dtype, "attention")
+    plain = apt_b200.GATEdgeSoftmaxSum.apply(*args, S, 0.2)
+    assert torch.equal(plain, out) and not plain.requires_grad
+    leaf = args[2].clone().requires_grad_()
+    with torch.no_grad():
+        assert torch.equal(apt_b200.GATEdgeSoftmaxSum.apply(args[0], args[1], leaf, *args[3:], S, 0.2), out)
+    kept = apt_b200.GATEdgeSoftmaxSum.apply(args[0], args[1], leaf, *args[3:], S, 0.2)
+    assert kept.requires_grad
+    _near(kept.detach(), want, dtype, "out of a training step")
+    shifted = torch.empty(args[2].numel() + 1, device="cuda", dtype=dtype)[1:].view_as(args[2])        # no 16-byte alignment
+    shifted.copy_(args[2])
+    _near(ops.gat_edge_softmax_sum(args[0], args[1], shifted, *args[3:], S, 0.2), want, dtype, "out of unaligned rows")
+    ops.check_status()
+
+
+def test_forward_mode_is_refused():
+    row, col, ft, el, er, _ = _inputs([3, 4], 2, 8, torch.float32, 1)
+    args = [dev(x) for x in (row, col, ft, el, er)]
+    with torch.autograd.forward_ad.dual_level():
+        args[2] = torch.autograd.forward_ad.make_dual(args[2], torch.ones_like(args[2]))
+        with pytest.raises(Exception, match="jvp|forward"):
+            apt_b200.GATEdgeSoftmaxSum.apply(*args, 2, 0.2)
