@@ -328,7 +328,7 @@ class Plan {
       // behind everything the caller's stream holds so far: the seeds' producer, the consumer of the last results
       cuda_ok(cudaEventRecord(ready_, cur), "cudaEventRecord");
       cuda_ok(cudaStreamWaitEvent(own_, ready_, 0), "cudaStreamWaitEvent");
-    } else if (stream_ && stream_ != cur) {
+    } else if (launched_ && stream_ != cur) {
       cuda_ok(cudaStreamWaitEvent(cur, done_, 0), "cudaStreamWaitEvent");
     }
     if (count && !(seeds.is_cuda() && seeds.device() == seeds_buf_.device())) {
@@ -339,6 +339,7 @@ class Plan {
     cuda_ok(cudaGraphLaunch(exec_, s), "cudaGraphLaunch");
     cuda_ok(cudaEventRecord(done_, s), "cudaEventRecord");
     stream_ = s;
+    launched_ = true;
     waited_ = false;
     seeds_ = seeds;       // the copy reads it when the stream gets there
   }
@@ -355,22 +356,22 @@ class Plan {
     py::gil_scoped_release nogil;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // a plan may go while some stream is being captured
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (stream_) cudaEventSynchronize(done_);
+    if (launched_) cudaEventSynchronize(done_);
     cudaThreadExchangeStreamCaptureMode(&mode);
   }
   // The current stream runs on behind everything the last launch enqueued (the gathered rows among it).
   void order_current_stream() {
     const cudaStream_t cur = (cudaStream_t)stream();
-    if (stream_ && stream_ != cur) cuda_ok(cudaStreamWaitEvent(cur, done_, 0), "cudaStreamWaitEvent");
+    if (launched_ && stream_ != cur) cuda_ok(cudaStreamWaitEvent(cur, done_, 0), "cudaStreamWaitEvent");
   }
 
  private:
   cudaGraphExec_t exec_;
   Tensor seeds_buf_, replay_in_, host_words_, seeds_;
-  cudaStream_t own_, stream_ = nullptr;
+  cudaStream_t own_, stream_ = nullptr;      // the default stream is a null handle too: launched_ says whether there is one
   cudaEvent_t done_, ready_;
   int64_t sequence_ = 0;
-  bool waited_ = true;
+  bool launched_ = false, waited_ = true;
 };
 
 // The first n rows. Below autograd: a sampler's buffers have no history to carry on, and the view costs half as much.
