@@ -90,8 +90,11 @@ k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* 
   }
 }
 
-// Attention weights. K edges' loads are in flight; a destination of at most K edges keeps its scores in registers.
-template <typename T>
+// Attention weights, W lanes to a destination and head. K edges' loads of a lane are in flight; a destination of at most K * W
+// edges keeps its scores in registers. W is 2 above a mean of 16 edges, where one lane would walk its edges three times, two
+// dependent loads each: forward of 30 000 destinations of 20 / 25 / 32 edges, bf16 4 x 64, 58 / 72 / 90 -> 56 / 68 / 76 us,
+// fp16 2 x 10 39 / 45 / 57 -> 34 / 39 / 39. (One lane with 32 scores takes half the warps' registers: 59 / 76 / 82 and 37 / 43 / 45.)
+template <typename T, int W>
 __global__ void __launch_bounds__(256)
 k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
               int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ weight,
@@ -99,36 +102,45 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
   wait_for_previous();
   constexpr int K = 16;
   if (*none != 0) return;
-  const int64_t total = num_dst * num_heads, stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+  const int64_t total = num_dst * num_heads, stride = (int64_t)gridDim.x * blockDim.x / W;
+  const int part = threadIdx.x & (W - 1);
+  const unsigned mask = W == 1 ? 0u : ((1u << W) - 1u) << (threadIdx.x & 31 & ~(W - 1));
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / W; i < total; i += stride) {
     const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
     const int2 r = range[d];
     const float bias = Elem<T>::to_f(er[i]);
-    const int deg = r.y - r.x;
+    const int deg = r.y - r.x, mine = (deg - part + W - 1) / W;      // this lane's edges: r.x + part, every W-th
     float s[K], m = -INFINITY, sum = 0.f;
     auto score = [&](int e) { return leaky(Elem<T>::to_f(el[row[e] * num_heads + h]) + bias, slope); };
-    if (deg <= K) {
+    if (deg <= K * W) {
       uint32_t src[K];
 #pragma unroll
-      for (int k = 0; k < K; ++k) src[k] = k < deg ? (uint32_t)row[r.x + k] : 0u;
+      for (int k = 0; k < K; ++k) src[k] = k < mine ? (uint32_t)row[r.x + part + k * W] : 0u;
 #pragma unroll
-      for (int k = 0; k < K; ++k) s[k] = k < deg ? Elem<T>::to_f(el[(int64_t)src[k] * num_heads + h]) : 0.f;
+      for (int k = 0; k < K; ++k) s[k] = k < mine ? Elem<T>::to_f(el[(int64_t)src[k] * num_heads + h]) : 0.f;
 #pragma unroll
       for (int k = 0; k < K; ++k)
-        if (k < deg) {
+        if (k < mine) {
           s[k] = leaky(s[k] + bias, slope);
           m = fmaxf(m, s[k]);
         }
+    } else {
+      for (int e = r.x + part; e < r.y; e += W) m = fmaxf(m, score(e));
+    }
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) m = fmaxf(m, __shfl_xor_sync(mask, m, o));
+    if (deg <= K * W) {
 #pragma unroll
       for (int k = 0; k < K; ++k)
-        if (k < deg) {
+        if (k < mine) {
           s[k] = expf(s[k] - m);
           sum += s[k];
         }
     } else {
-      for (int e = r.x; e < r.y; ++e) m = fmaxf(m, score(e));
-      for (int e = r.x; e < r.y; ++e) sum += expf(score(e) - m);
+      for (int e = r.x + part; e < r.y; e += W) sum += expf(score(e) - m);
     }
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) sum += __shfl_xor_sync(mask, sum, o);
     const float inv = sum > 0.f ? 1.f / sum : 0.f;
     const bool zero = !(sum > 0.f) && deg <= masked;
     auto put = [&](int e, float w) {
@@ -137,12 +149,12 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
       weight[o] = w;
       if (attn) attn[o] = Elem<T>::from_f(w);
     };
-    if (deg <= K) {
+    if (deg <= K * W) {
 #pragma unroll
       for (int k = 0; k < K; ++k)
-        if (k < deg) put(r.x + k, s[k] * inv);
+        if (k < mine) put(r.x + part + k * W, s[k] * inv);
     } else {
-      for (int e = r.x; e < r.y; ++e) put(e, expf(score(e) - m) * inv);
+      for (int e = r.x + part; e < r.y; e += W) put(e, expf(score(e) - m) * inv);
     }
   }
 }
@@ -382,8 +394,13 @@ static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaS
   const int rc = gat_ranges(q, g, s);
   if (rc != APT_OK) return rc;
   ProfScope prof("gat_rows", s);
-  APT_FOLLOW(k_gat_weights<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-             q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn, masked_edges(q.H, q.Dh, sizeof(T), (uintptr_t)q.ft));
+  const int masked = masked_edges(q.H, q.Dh, sizeof(T), (uintptr_t)q.ft);
+#define APT_WEIGHTS(W)                                                                                                       \
+  APT_FOLLOW((k_gat_weights<T, W>), wave_grid(ceil_div(q.num_dst * q.H * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
+             q.H, q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn, masked)
+  if (q.E > 16 * q.num_dst) APT_WEIGHTS(2);
+  else APT_WEIGHTS(1);
+#undef APT_WEIGHTS
   return APT_OK;
 }
 
