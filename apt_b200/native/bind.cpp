@@ -123,6 +123,11 @@ Tensor gather(const Tensor& node_id, const Tensor& pos_map, const Tensor& dev_fe
   const int64_t n = id.numel(), size = dev_feats.element_size(), dim = dev_feats.size(1);
   Tensor out = at::empty({n, dim}, dev_feats.options());
   if (n == 0) return out;
+  if (n <= apt_gather_static_max_rows()) {      // the same launch without a workspace, which it does not use
+    check(apt_gather_rows_static(ptr(id), n, ptr(pos_map), num_nodes, data(dev_feats), dev_feats.size(0), dim * size, data(uva_feats),
+                                 uva_feats.size(0), uva_feats.size(1) * size, column * size, mut(out), status_word(words), stream()));
+    return out;
+  }
   const size_t bytes = apt_gather_workspace_bytes(n);
   const Tensor ws = scratch(out, bytes);
   check(apt_gather_rows(ptr(id), n, nullptr, ptr(pos_map), num_nodes, data(dev_feats), dev_feats.size(0), dim * size,

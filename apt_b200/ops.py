@@ -188,8 +188,12 @@ class NPCState:
         """int64[256] device words: [0..254] small results (counts a kernel leaves for
         the next kernel and, later, for the host), [255] status flags. Inside own_words() the small results are in
         a block of the caller's."""
-        own = getattr(self._tls, "words", None)
-        return self.lane_words() if own is None else own
+        tls = self._tls
+        own = getattr(tls, "words", None)
+        if own is not None:
+            return own
+        words = self._lane_words.get(getattr(tls, "lane", 0))
+        return words if words is not None and words.get_device() == torch.cuda.current_device() else self.lane_words()
 
     @contextlib.contextmanager
     def own_words(self, words: torch.Tensor):
@@ -928,8 +932,7 @@ def sddmm_u_mul_v(coo_row, coo_col, lhs, rhs, coo_offset, lhs_offset, rhs_offset
 
 def gat_edge_softmax_sum(coo_row, coo_col, ft, el, er, num_dst: int, negative_slope: float = 0.2,
                          return_attention: bool = False):
-    """One sampled block of a GAT layer in one kernel: u_add_v(el, er) -> leaky_relu ->
-    edge_softmax -> u_mul_e(ft, a) summed per destination (the DGL calls of
+    """One sampled block of a GAT layer: u_add_v(el, er) -> leaky_relu -> edge_softmax -> u_mul_e(ft, a) summed per destination (the DGL calls of
     python/npc/model/gatconv.py:113-124). ft [num_src, H, Dh] or [num_src, H*Dh],
     el [num_src, H(,1)], er [num_dst, H(,1)]; edges grouped by destination.
     Returns out [num_dst, H, Dh] (and the attention [E, H, 1])."""
@@ -941,9 +944,11 @@ def gat_edge_softmax_sum(coo_row, coo_col, ft, el, er, num_dst: int, negative_sl
 def gat_edge_softmax_sum_backward(coo_row, coo_col, ft, el, er, grad_out, negative_slope: float = 0.2):
     """Gradients of gat_edge_softmax_sum with respect to ft, el and er for
     grad_out [num_dst, H, Dh]: the edge part over the destinations (softmax and
-    leaky_relu backward per edge, grad_er), then one walk over the edges grouped
-    by source for both sums over the source side. Returns (grad_ft, grad_el,
-    grad_er) shaped like ft, el, er."""
+    leaky_relu backward per edge, grad_er, and grad_el added up in fp32 by
+    reductions), then one walk over the edges grouped by source for grad_ft. Both
+    source-side sums run in an order that the GPU's scheduling decides, so they
+    repeat themselves within rounding and not bit for bit. Returns (grad_ft,
+    grad_el, grad_er) shaped like ft, el, er."""
     return _native.gat_backward(coo_row, coo_col, ft, el, er, grad_out, float(negative_slope), STATE.words())
 
 
