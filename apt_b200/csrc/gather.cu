@@ -234,12 +234,15 @@ static int gather_check(const char* who, const GatherArgs& a) {
 extern "C" int apt_set_tunable(const char* name, int64_t value) {
   using namespace apt;
   APT_CHECK_ARG(name, "apt_set_tunable: null name");
-  // knobs of forms of the gather that are gone: taken and without effect
+  // knobs of forms of the gather that are gone: taken, without effect, and said so, since a measurement would show nothing
   static const struct { const char* name; int64_t lo, hi; } retired[] = {
       {"gather_miss_mode", 0, 1}, {"gather_miss_blocks", 1, 65535}, {"gather_miss_kb_per_block", 0, 1 << 20},
       {"gather_hit_mode", 0, 2}, {"gather_hit_waves", 1, 64}};
   for (const auto& r : retired)
-    if (!strcmp(name, r.name) && value >= r.lo && value <= r.hi) return APT_OK;
+    if (!strcmp(name, r.name) && value >= r.lo && value <= r.hi) {
+      fprintf(stderr, "apt_set_tunable: %s has no effect any more\n", name);
+      return APT_OK;
+    }
   if (!strcmp(name, "relabel_small") && value >= 0 && value <= 1) {
     set_relabel_small(value != 0);
     return APT_OK;
@@ -330,8 +333,8 @@ extern "C" int apt_gather_rows_static(const int64_t* index, int64_t num_rows,
   using namespace apt;
   APT_CHECK_ARG(num_rows >= 0, "apt_gather_rows_static: negative num_rows");
   if (num_rows > kStaticGatherMaxRows) {
-    set_error("apt_gather_rows_static: %lld rows exceed the built-in scratch of %lld rows per call; "
-              "split the request or use apt_gather_rows with a caller workspace",
+    set_error("apt_gather_rows_static: %lld rows exceed the built-in scratch's limit of %lld rows per call (kept although the "
+              "scratch is gone); split the request or use apt_gather_rows",
               (long long)num_rows, (long long)kStaticGatherMaxRows);
     return APT_ERR_CAPACITY;
   }

@@ -221,8 +221,9 @@ static bool g_relabel_small = true;   // apt_set_tunable("relabel_small", 0) for
 void set_relabel_small(bool on) { g_relabel_small = on; }
 
 constexpr int kSmallItems = 8192;
-// behind a sampling kernel, which fills the table on its way, the one-block form only saves launches: 1536 items 8.8 us
-// against 12.0, 6144 items 16.1 against 12.9
+// behind a sampling kernel, which fills the table on its way, the one-block form only saves launches. Sampling and relabelling
+// together, one block against the grid, fanout 5: 500 items 6.2 us against 9.8, 1536 8.0 / 11.0, 2048 8.5 / 12.2, 3072
+// 10.0 / 12.1; fanout 15: 6.2 / 9.0, 8.2 / 9.8, 8.2 / 10.6, 9.8 / 10.8; relabelling of 6144 items 16.1 / 12.9
 constexpr int kSmallSampled = 3072;
 constexpr uint32_t kSmallCap = 12288;
 constexpr uint16_t kSmallNoSlot = 0xffffu;

@@ -208,8 +208,8 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[V
 
 // Blocks an SM is to hold. The gather is bound by loads in flight, and the 64 (80) registers a thread of four (three)
 // blocks hold the slices of plain sums without spilling; edge values and 8 elements a slice need more.
-// 67 584 x 15 edges, fp32 x 256 (1.04 GB gathered, mostly out of L2): 152 us at one or two blocks, 114 at three, 109 at
-// four; bf16 x 256: 89 / 65 / 63 us; the reverse direction 186 / 149 / 158 and 104 / 82 / 90 us.
+// 67 584 x 15 edges, bf16 x 256 (0.52 GB gathered, mostly out of L2): 89 us at one or two blocks, 65 at three, 63 at four;
+// reverse 104 / 82 / 90 us. (fp32 x 256 behaved the same; rows above 512 bytes of that many edges are k_spmm_bulk's now.)
 constexpr int rows_min_blocks(int op, int elems) {
   if (op == kCopyU || op == kCopyE || op == kUMulW) return elems <= 4 ? 4 : elems <= 8 ? 3 : 2;
   return elems <= 2 ? 3 : elems <= 8 ? 2 : 1;

@@ -101,7 +101,8 @@ int apt_profile_read(const char* tag, double* total_ms, int64_t* launches);
 
 /* Tuning knobs for measurements; the defaults are what the benchmark uses.
  *   gather_miss_mode, gather_miss_blocks, gather_miss_kb_per_block, gather_hit_mode, gather_hit_waves
- *                      accepted and without effect (they chose between forms of the gather that are gone)
+ *                      accepted, without effect and reported on stderr (they chose between forms of the gather that
+ *                      are gone)
  *   bulk_wait_polls    polls after which a wait for rows on their way to shared memory is given up, 0 to 1048576 (default)
  *   relabel_small      1 (default): layers of up to 8192 items are relabelled by one block with
  *                      the hash table in shared memory; 0: always the multi-block path */
@@ -430,8 +431,10 @@ int apt_gat_edge_backward(int dtype, const int64_t* coo_row, const int64_t* coo_
  * backward with edges_valid = 1 (same block, el, er and slope) it saves working them
  * out again, with edges_valid = 0 it is scratch there. The backward gives grad_ft
  * [num_src, num_heads*head_dim], grad_el [num_src, num_heads] and grad_er [num_dst,
- * num_heads]: the edges are grouped by source once and one walk sums both source-side
- * gradients. workspace: apt_gat_backward_workspace_bytes(...) bytes.
+ * num_heads]: the edges are grouped by source once and one walk sums grad_ft; grad_el is
+ * added up in fp32 by reductions, an edge and head at a time. Both orders depend on how the
+ * blocks are scheduled: results repeat themselves within rounding, not bit for bit (the
+ * same holds for apt_spmm_sum over edges that are not grouped). workspace: apt_gat_backward_workspace_bytes(...) bytes.
  * apt_gat_edge_softmax_sum and apt_gat_edge_backward above do with a few words a
  * destination and work the weights out as often as they need them. */
 size_t apt_gat_edges_bytes(int64_t num_dst, int64_t num_edges, int num_heads);

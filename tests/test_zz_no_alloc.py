@@ -3,12 +3,12 @@ workspace-taking one (apt_gather_rows), through the C ABI.
 
 Some callers may not call cudaMalloc at all — a server that planned all of its
 device memory up front, a latency-critical loop, a process whose allocator is
-locked after start-up. For them the library keeps the gather's scratch in a
-fixed device array. This test checks that the two entry points return the
-same bytes on two calls in a row (the second one smaller, so that what the
-first call left in the shared scratch would show if it were not cleared), and
-that an oversized request is refused. The file name makes pytest collect it
-last.
+locked after start-up. The gather keeps no scratch; its limit on the rows of a
+call dates from a form that kept some in a fixed device array and is part of the
+interface. This test checks that the two entry points return the same bytes on
+two calls in a row (the second one smaller, so that whatever the first call left
+behind would show), and that an oversized request is refused. The file name makes
+pytest collect it last.
 """
 import ctypes
 
@@ -55,7 +55,7 @@ def test_static_gather_matches_workspace_gather_twice():
     n, dim = 20000, 128
     uva_t, dev_t, pos = _tables(n, dim, rng)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    for rows in (50000, 777):   # the second call reuses the scratch the first one filled
+    for rows in (50000, 777):
         ids = torch.from_numpy(rng.integers(0, n, rows).astype(np.int64)).cuda()
         want = _with_workspace(ids, pos, dev_t, uva_t, status)
         got = _static(ids, pos, dev_t, uva_t, status)
