@@ -82,9 +82,10 @@ __device__ __forceinline__ unsigned long long probe_votes(uint32_t bits) {
          (bits & kHasLong ? 1ull << 48 : 0ull);
 }
 
+// num_rows: the output rows there are (the caller's result may have more, or fewer, than the offsets end at); -1: as the offsets say.
 __global__ void __launch_bounds__(256)
-k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned long long* agg, int slot, volatile int64_t* result,
-             int64_t sequence) {
+k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_rows, unsigned long long* agg, int slot,
+             volatile int64_t* result, int64_t sequence) {
   wait_for_previous();
   if (!agg) agg = g_probe_votes + slot;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
@@ -103,7 +104,7 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned l
   }
   if (threadIdx.x == 0) s_bits = 0u;
   __syncthreads();
-  const int64_t rows = ooff[st.nseg];
+  const int64_t rows = num_rows >= 0 ? num_rows : ooff[st.nseg];
   // the one fanout that fits the sizes
   const uint32_t f = rows > 0 && E % rows == 0 ? (uint32_t)(E / rows) : 0u;
   uint32_t bits = f ? 0u : kNotFixed;
@@ -142,12 +143,12 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, unsigned l
   *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, sequence);
 }
 
-static int launch_probe(const int64_t* col, int64_t E, SegTable st, unsigned long long* agg, int slot, int64_t* result,
-                        int64_t sequence, cudaStream_t s) {
+static int launch_probe(const int64_t* col, int64_t E, SegTable st, int64_t num_rows, unsigned long long* agg, int slot,
+                        int64_t* result, int64_t sequence, cudaStream_t s) {
   // a thousand edges a block and one wave at most: small blocks of edges are looked over by one thread block
   const int grid = wave_grid(ceil_div(E, 1024), 4, 1);
   ProfScope prof("spmm_ranges", s);
-  APT_FOLLOW(k_spmm_probe, grid, 256, 0, s, col, E, st, agg, slot, (volatile int64_t*)result, sequence);
+  APT_FOLLOW(k_spmm_probe, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence);
   return APT_OK;
 }
 
@@ -511,7 +512,7 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
   const RowSplit split = row_split(feat_dim, slice_elems(bits, (int)esz), E, num_rows);
   if (mode == kDevice || mode == kOrder) APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
   if (mode == kDevice) {
-    const int rc = launch_probe(coo_col, E, st, ws.probe, 0, ws.result, 1, s);
+    const int rc = launch_probe(coo_col, E, st, num_rows, ws.probe, 0, ws.result, 1, s);
     if (rc != APT_OK) return rc;
   }
   if (mode == kDevice || mode == kRanges) {
@@ -574,7 +575,7 @@ extern "C" int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges, const i
   if (rc != APT_OK) return rc;
   int64_t* host = g_probe.host + slot * 8;
   SegTable st{coo_offset, nullptr, output_offset, num_segments};
-  rc = launch_probe(coo_col, num_edges, st, nullptr, slot, host, sequence, s);
+  rc = launch_probe(coo_col, num_edges, st, -1, nullptr, slot, host, sequence, s);
   if (rc == APT_OK) rc = wait_for(host, sequence, s);
   if (rc == APT_OK) {
     const int64_t w = *(volatile int64_t*)host, rows = probe_rows(w);

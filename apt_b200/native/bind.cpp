@@ -83,8 +83,10 @@ Tensor spmm(int op, const Tensor& coo_row, const Tensor& coo_col, const OptTenso
   const int64_t per_edge = edata ? ed.numel() / std::max<int64_t>(edges, 1) : 0;
   const int64_t dim = input ? in.size(1) : per_edge;
   const int64_t edim = edata && edges ? per_edge : dim;
-  int64_t shape[3];
-  {
+  int64_t shape[3] = {0, -1, 0};
+  if (ooff.numel() > eoff.numel()) {
+    shape[0] = ooff[-1].item<int64_t>();        // further rows behind the last segment's: the block is looked over with them
+  } else {
     py::gil_scoped_release nogil;   // other threads run while this one waits for the stream
     check(apt_spmm_probe(ptr(col), edges, ptr(eoff), ptr(ooff), (int)eoff.numel() - 1, shape, stream()));
   }

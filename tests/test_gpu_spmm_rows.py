@@ -188,3 +188,31 @@ def test_sddmm_widths(dtype, D):
         got = fn(dev(row), dev(col), dev(lhs, dtype), dev(rhs, dtype), *(dev(o) for o in off))
         # one rounding of an exact sum or product
         assert np.all(np.abs(host(got).astype(np.float64) - want) <= TOL[dtype] * np.abs(want) + 1e-38)
+
+
+@pytest.mark.parametrize("num_rows", [4, 10, 11, 25, 50, 60])
+@pytest.mark.parametrize("order", ["fixed", "ragged", "mixed"])
+def test_more_or_fewer_rows_than_the_offsets_end_at(num_rows, order):
+    # 50 edges over 10 rows, offsets that end at 10, a result of another length: rows behind are zero, edges of rows beyond it
+    # are left out, also where the edges divide evenly among the rows there are
+    rng = np.random.default_rng(num_rows)
+    E, S, n_src, D = 50, 10, 17, 12
+    col = np.repeat(np.arange(S), 5) if order == "fixed" else np.sort(rng.integers(0, S, E))
+    if order == "mixed":
+        rng.shuffle(col)
+    row, col = rng.integers(0, n_src, E).astype(I64), col.astype(I64)
+    x = rng.integers(-8, 9, (n_src, D)).astype(np.float32)          # whole numbers: sums are exact
+    want = np.zeros((max(num_rows, S), D), np.float32)
+    np.add.at(want, col, x[row])
+    t = [dev(row), dev(col), dev(x)] + [dev(np.array([0, n], dtype=I64)) for n in (E, n_src, S)]
+    out = torch.full((num_rows, D), 9.0, device="cuda")
+    nbytes = lib.apt_spmm_workspace_bytes(num_rows, E)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    p = [ctypes.c_void_p(v.data_ptr()) for v in t]
+    check(lib.apt_spmm_sum(0, _lib.F32, p[0], p[1], E, p[2], None, D, D, p[3], p[4], p[5], 1, num_rows, ctypes.c_void_p(out.data_ptr()),
+                           ctypes.c_void_p(ws.data_ptr()), nbytes, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert np.array_equal(host(out), want[:num_rows])
+    if num_rows >= S:
+        longer = dev(np.array([0, S, num_rows], dtype=I64))         # the operator takes the number of rows from the last entry
+        assert np.array_equal(host(ops.spmm_copy_u_sum(*t[:5], longer)), want)
+    ops.check_status()
