@@ -474,8 +474,9 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
 // ---- without a buffer for weights -----------------------------------------------------
 // apt_gat_edge_softmax_sum and apt_gat_edge_backward have a few words a destination of workspace and allocate nothing: a warp
 // to a destination keeps the weights of 32 edges and 4 heads in shared memory and works them out again for further edges
-// and column blocks. They are for callers that do not hold E x heads fp32 values: 67 584 x 15 edges, bf16, 4 x 64, take 142 us
-// forward and 245 for the edge part of the backward, with such a buffer 114 and 164.
+// and column blocks. They are for callers that do not hold E x heads fp32 values: 67 584 x 15 edges, bf16, 4 x 64, take 144 us
+// forward and 203 for the edge part of the backward, with such a buffer 114 and 164. Three blocks an SM for the backward (four:
+// 216, spills), four for the forward (three: 154); eight heads at a time 151 and 233.
 constexpr int kAloneHeads = 4;
 
 // The weights of one destination's edges, for the heads from h0 on, a lane to an edge. What outlives a step is in shared memory:
@@ -644,7 +645,7 @@ k_gat_narrow(const int64_t* __restrict__ row, const T* __restrict__ ft, const T*
 }
 
 template <typename T, int VE>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 3)
 k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er,
                      const T* __restrict__ grad_out, int num_heads, int head_dim, float slope, int64_t num_dst, int64_t E,
                      const int2* __restrict__ range, const int32_t* __restrict__ none, T* __restrict__ attn,
@@ -703,10 +704,19 @@ k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, 
                     for (int q = 0; q < VE; ++q) dot[u] = fmaf(g.get(q), v[u].get(q), dot[u]);
                   }
                 }
+              if (lph >= 4) {      // each step halves the edges a lane sums for (k_gat_dots)
+                const bool hi = p & (lph >> 1), lo = p & (lph >> 2);
+                const float b0 = (hi ? dot[2] : dot[0]) + __shfl_xor_sync(0xffffffffu, hi ? dot[0] : dot[2], lph >> 1);
+                const float b1 = (hi ? dot[3] : dot[1]) + __shfl_xor_sync(0xffffffffu, hi ? dot[1] : dot[3], lph >> 1);
+                const float v = group_sum((lo ? b1 : b0) + __shfl_xor_sync(0xffffffffu, lo ? b0 : b1, lph >> 2), lph >> 2);
+                const int j = j0 + ((hi ? 2 : 0) + (lo ? 1 : 0)) * ep;
+                if ((p & ((lph >> 2) - 1)) == 0 && j < cnt && h < sc.nh) dot_sh[warp][j][h] = v;
+              } else {
 #pragma unroll
-              for (int u = 0; u < U; ++u) {
-                dot[u] = group_sum(dot[u], lph);
-                if (p == 0 && j0 + u * ep < cnt && h < sc.nh) dot_sh[warp][j0 + u * ep][h] = dot[u];
+                for (int u = 0; u < U; ++u) {
+                  dot[u] = group_sum(dot[u], lph);
+                  if (p == 0 && j0 + u * ep < cnt && h < sc.nh) dot_sh[warp][j0 + u * ep][h] = dot[u];
+                }
               }
             }
           }
