@@ -80,7 +80,7 @@ struct ProfScope {
   } while (0)
 
 void set_relabel_small(bool on);   // relabel.cu: one-block shared-memory path for small layers
-void set_bulk_wait_polls(int polls);   // spmm.cu: bound of k_spmm_bulk's waits
+void set_bulk_wait_polls(int polls);   // spmm.cu: bound of k_spmm_stream's waits
 
 // While another thread captures a stream, or this one does, calls that might synchronise are refused and end the capture. For
 // those that do not touch the captured work (page-locked memory of the library's own, asking a stream how it stands).

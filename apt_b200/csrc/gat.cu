@@ -15,16 +15,16 @@
 //   k_gat_weights   one thread per destination and head: scores and softmax. Full occupancy hides the two dependent
 //                   loads of a score; any number of edges and heads.
 //   row kernel      the weighted sum is the SpMM's row kernel (kUMulW), any head width
-//   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination. The four partial dots of a
-//                   lane are reduced together: each step halves the values a lane keeps, log2(lph) + 1 shuffles
-//                   for four edges instead of 4 log2(lph).
+//   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination (wide rows of many edges:
+//                   k_spmm_stream's kDots). The four partial dots of a lane are reduced together: each step halves the values
+//                   a lane keeps, log2(lph) + 1 shuffles for four edges instead of 4 log2(lph).
 //   k_gat_scores    backward: t, grad_s and grad_er, one thread per destination and head; grad_el is added up in fp32 with
 //                   one reduction per edge and head (the heads of an edge are neighbours: one sector)
 //   row kernel      grad_ft: the weighted sum of the forward with the sides swapped. With grad_el as a second accumulator
 //                   of the same walk it held two blocks an SM instead of three: 150 us against 116, and the scores had to
 //                   be written out for it.
-//   The counting sort by source that grad_ft needs rides along: k_gat_dots has every edge's source in a register and waits
-//                   for rows most of the time, so it also counts the edges (the add returns an edge's place in its
+//   The counting sort by source that grad_ft needs rides along: the dots have every edge's source in a register and wait
+//                   for rows most of the time, so they also count the edges (the add returns an edge's place in its
 //                   row); k_dst_slots gives the rows their places; k_gat_scores writes the order. As launches of
 //                   their own the first and the last pass took 23 + 16 us.
 //   k_gat_source    grad_el in T
@@ -34,7 +34,7 @@
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 18 + 78 us. Backward of that block: 18 (saved after a forward) + 101 + 7 + 44 + 112 + 5 us,
+// kernels take 18 + 61 us. Backward of that block: 18 (saved after a forward) + 80 + 7 + 44 + 63 + 5 us,
 // where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 
@@ -264,7 +264,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
              int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
-             float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort,
+             float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort, OrderKind kind,
              T* __restrict__ grad_er) {
   wait_for_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -312,7 +312,10 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
 #pragma unroll 4
     for (int e = r.x + (int)h; e < r.y; e += num_heads) {
       const uint32_t place = sort.rank[e];
-      if (place != kNoRank) sort.order[(uint32_t)sort.range[row[e]].x + place] = make_uint2(d, (uint32_t)e);
+      if (place == kNoRank) continue;
+      const uint32_t at = (uint32_t)sort.range[row[e]].x + place;
+      if (kind == kByBoth) ((uint4*)sort.order)[at] = make_uint4(d, (uint32_t)row[e], (uint32_t)e, 0u);
+      else sort.order[at] = make_uint2(d, (uint32_t)e);
     }
   }
 }
@@ -347,19 +350,21 @@ static size_t gat_edges_layout(int64_t num_dst, int64_t E, int H, char* base, Ga
 
 struct GatBwdWs {
   float* sums;      // [num_src][heads], cleared with the front of the sort
-  SpmmWs sort;
+  SpmmWs sort;      // its order: slots of 16 bytes (kByBoth)
   float* dots;      // [E][heads]
   size_t zero_bytes;
 };
 static size_t gat_bwd_layout(int64_t num_src, int64_t E, int H, char* base, GatBwdWs* ws) {
   const size_t o_sort = align_up((size_t)(num_src > 0 ? num_src : 1) * H * 4, 256);
   const size_t o_dots = o_sort + spmm_layout(num_src, E, base + o_sort, ws ? &ws->sort : nullptr);
+  const size_t o_order = o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
   if (ws) {
     ws->sums = (float*)base;
     ws->dots = (float*)(base + o_dots);
     ws->zero_bytes = o_sort + ws->sort.zero_bytes;
+    ws->sort.order = (uint2*)(base + o_order);
   }
-  return o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
+  return o_order + align_up((size_t)(E > 0 ? E : 1) * 16, 256);
 }
 
 struct GatProblem {
@@ -414,7 +419,7 @@ static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* 
   SpmmWs ws{};
   ws.range = g.range;
   const RowArgs<T> a{q.row, (const T*)q.ft, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, ws,
-                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status};
+                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u};
   ProfScope prof("gat_rows", s);
   return launch_spmm_rows<T>(kUMulW, a, s);
 }
@@ -432,40 +437,50 @@ static int launch_dots(const GatProblem& q, const GatEdges& g, int64_t num_src, 
   return APT_OK;
 }
 
-// The edge part of the backward: weights are there already. Leaves the source side's sums of the score gradients and the order
-// of its edges (`sort`, all of it zero where it has to be).
+// Dots of the edges, whose source rows are counted on the way.
 template <typename T>
-static int gat_edge_backward(const GatProblem& q, const GatEdges& g, int64_t num_src, float* dots, float* sums, const SpmmWs& sort,
-                             int long_edges, void* grad_er, cudaStream_t s) {
-  ProfScope prof("gat_bwd_rows", s);
-  int rc;
-  switch (slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T)) {
-    case 16: rc = launch_dots<T, 16 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
-    case 8: rc = launch_dots<T, 8 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
-    case 4: rc = launch_dots<T, 4 / sizeof(T)>(q, g, num_src, dots, sort, s); break;
-    default: rc = launch_dots<T, 1>(q, g, num_src, dots, sort, s); break;
+static int gat_dots(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, int64_t num_src, cudaStream_t s) {
+  const int64_t dim = q.H * q.Dh;
+  const int slice = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T);
+  if (stream_fits(kDots, slice, dim, sizeof(T), q.H, q.E, true)) {
+    SpmmWs counts = ws.sort;
+    counts.range = g.range;
+    const RowArgs<T> a{q.row, (const T*)q.ft, nullptr, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, counts,
+                       nullptr, kRanges, 0, RowSplit{}, 0, g.none, q.status, q.col, (const T*)q.grad_out, ws.dots, (uint32_t)num_src};
+    return launch_spmm_rows<T>(kDots, a, s);
   }
-  if (rc == APT_OK) rc = launch_slots(num_src, sort, kOrder, long_edges, (int)(q.H * q.Dh), s);
-  if (rc != APT_OK) return rc;
-  APT_FOLLOW(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-             q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, dots, sums, sort, (T*)grad_er);
-  return APT_OK;
+  switch (slice) {
+    case 16: return launch_dots<T, 16 / sizeof(T)>(q, g, num_src, ws.dots, ws.sort, s);
+    case 8: return launch_dots<T, 8 / sizeof(T)>(q, g, num_src, ws.dots, ws.sort, s);
+    case 4: return launch_dots<T, 4 / sizeof(T)>(q, g, num_src, ws.dots, ws.sort, s);
+    default: return launch_dots<T, 1>(q, g, num_src, ws.dots, ws.sort, s);
+  }
 }
 
+// The weights are there already.
 template <typename T>
 static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, char* workspace, int64_t num_src, void* grad_ft,
                         void* grad_el, void* grad_er, cudaStream_t s) {
   const int64_t dim = q.H * q.Dh;
   const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
   const RowSplit split = row_split(dim, ve, q.E, num_src);
-  const SegTable st{nullptr, nullptr, nullptr, 1};
+  const OrderKind kind = order_kind(kUMulW, ve * (int)sizeof(T), dim, sizeof(T), q.H, q.E);
   APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
-  int rc = gat_edge_backward<T>(q, g, num_src, ws.dots, ws.sums, ws.sort, split.long_edges, grad_er, s);
-  if (rc != APT_OK) return rc;
-  const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, st, num_src, q.E, ws.sort,
-                     (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr, q.status};
-  ProfScope prof("spmm_rows", s);
-  rc = launch_spmm_rows<T>(kUMulW, a, s);
+  int rc;
+  {
+    ProfScope prof("gat_bwd_rows", s);
+    rc = gat_dots<T>(q, g, ws, num_src, s);
+    if (rc == APT_OK) rc = launch_slots(num_src, ws.sort, kOrder, kind, split.long_edges, (int)dim, s);
+    if (rc != APT_OK) return rc;
+    APT_FOLLOW(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
+               q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, ws.dots, ws.sums, ws.sort, kind, (T*)grad_er);
+  }
+  const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, num_src, q.E, ws.sort,
+                     (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr, q.status, nullptr, nullptr, nullptr, 0u};
+  {
+    ProfScope prof("spmm_rows", s);
+    rc = launch_spmm_rows<T>(kUMulW, a, s);
+  }
   if (rc != APT_OK) return rc;
   APT_FOLLOW(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (T*)grad_el);
   return APT_OK;

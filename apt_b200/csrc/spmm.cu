@@ -218,7 +218,7 @@ static int check_pending(const char* who) {
   return APT_ERR_TIMEOUT;
 }
 
-static std::atomic<int> g_bulk_wait_polls{kBulkWaitPolls};
+static std::atomic<int> g_bulk_wait_polls{kStreamWaitPolls};
 void set_bulk_wait_polls(int polls) { g_bulk_wait_polls = polls; }
 int bulk_wait_polls() { return g_bulk_wait_polls; }
 
@@ -309,7 +309,7 @@ k_dst_rank(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_
 // rows with one add and no block waits for another. Long rows leave their items.
 constexpr int kScanRows = 4;
 __global__ void __launch_bounds__(256)
-k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, int long_edges, int part_stride) {
+k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, OrderKind kind, int long_edges, int part_stride) {
   wait_for_previous();
   if (resolve_mode(mode, ws) != kOrder) return;
   __shared__ int scratch[33];
@@ -331,7 +331,7 @@ k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, int long_edges, int part_stri
     const int64_t d = first + k;
     if (d >= num_rows) break;
     ws.range[d] = make_int2(at, at + v[k]);
-    if (v[k] > long_edges) {
+    if (kind == kByEdge && v[k] > long_edges) {
       int size = item_edges(v[k]), parts = (v[k] + size - 1) / size, part = -1;
       if (parts > 1) {
         part = atomicAdd(ws.num_parts, parts);
@@ -350,7 +350,7 @@ k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, int long_edges, int part_stri
 }
 
 __global__ void __launch_bounds__(256)
-k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E, SegTable st, SpmmWs ws, int mode) {
+k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E, SegTable st, SpmmWs ws, int mode, OrderKind kind) {
   wait_for_previous();
   if (resolve_mode(mode, ws) != kOrder) return;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1], ioff[kMaxSegments + 1];
@@ -373,7 +373,7 @@ k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int
       if (r[k] == kNoRank) continue;
       const int seg = st.nseg > 1 ? seg_of(coo, st.nseg, e) : 0;
       d[k] = ooff[seg] + col[e];
-      o[k] = make_uint2((uint32_t)(ioff[seg] + row[e]), (uint32_t)e);
+      o[k] = make_uint2((uint32_t)(ioff[seg] + row[e]), (uint32_t)(kind == kByRow ? d[k] : e));
     }
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -384,19 +384,19 @@ k_dst_fill(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int
   }
 }
 
-int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s) {
-  APT_FOLLOW(k_dst_slots, (int)ceil_div(num_rows, 256 * kScanRows), 256, 0, s, num_rows, ws, mode, long_edges, part_stride);
+int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, OrderKind kind, int long_edges, int part_stride, cudaStream_t s) {
+  APT_FOLLOW(k_dst_slots, (int)ceil_div(num_rows, 256 * kScanRows), 256, 0, s, num_rows, ws, mode, kind, long_edges, part_stride);
   return APT_OK;
 }
 
-static int launch_group(const int64_t* row, const int64_t* col, int64_t num_edges, SegTable st, int64_t num_rows,
-                 const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s) {
+static int launch_group(const int64_t* row, const int64_t* col, int64_t num_edges, SegTable st, int64_t num_rows, const SpmmWs& ws, int mode,
+                        OrderKind kind, int long_edges, int part_stride, cudaStream_t s) {
   ProfScope prof("spmm_group", s);
   const int ge = wave_grid(ceil_div(num_edges, 256 * 4), 8, 1);
   APT_FOLLOW(k_dst_rank, ge, 256, 0, s, col, num_edges, st, num_rows, ws, mode);
-  const int rc = launch_slots(num_rows, ws, mode, long_edges, part_stride, s);
+  const int rc = launch_slots(num_rows, ws, mode, kind, long_edges, part_stride, s);
   if (rc != APT_OK) return rc;
-  APT_FOLLOW(k_dst_fill, ge, 256, 0, s, row, col, num_edges, st, ws, mode);
+  APT_FOLLOW(k_dst_fill, ge, 256, 0, s, row, col, num_edges, st, ws, mode, kind);
   return APT_OK;
 }
 
@@ -482,11 +482,11 @@ static int dispatch_sddmm(int op, int ve, const int64_t* row, const int64_t* col
 static size_t elem_size(int dtype) { return dtype == APT_F32 ? 4 : 2; }
 
 template <typename T>
-static int run_rows(int op, const RowSplit& split, const int64_t* row, int64_t E, const void* in, const void* edata,
+static int run_rows(int op, const RowSplit& split, const int64_t* row, const int64_t* col, int64_t E, const void* in, const void* edata,
                     int64_t edata_dim, int64_t feat_dim, SegTable st, int64_t num_rows, const SpmmWs& ws, int mode, int fixed,
                     void* out, cudaStream_t s) {
   const RowArgs<T> a{row, (const T*)in, (const T*)edata, edata_dim, feat_dim, st, num_rows, E, ws, (T*)out,
-                     mode, fixed, split, (int)feat_dim, nullptr, nullptr};
+                     mode, fixed, split, (int)feat_dim, nullptr, nullptr, col, nullptr, nullptr, 0u};
   ProfScope prof("spmm_rows", s);
   return launch_spmm_rows<T>(op, a, s);
 }
@@ -520,13 +520,14 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
     APT_FOLLOW(k_edge_ranges, wave_grid(ceil_div(E, 256), 8), 256, 0, s, coo_col, E, st, num_rows, ws, mode);
   }
   if (mode == kDevice || mode == kOrder) {
-    const int rc = launch_group(coo_row, coo_col, E, st, num_rows, ws, mode, split.long_edges, (int)feat_dim, s);
+    const OrderKind kind = order_kind(op, split.ve * (int)esz, feat_dim, esz, 1, E);
+    const int rc = launch_group(coo_row, coo_col, E, st, num_rows, ws, mode, kind, split.long_edges, (int)feat_dim, s);
     if (rc != APT_OK) return rc;
   }
   switch (dtype) {
-    case APT_F32: return run_rows<float>(op, split, coo_row, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
-    case APT_BF16: return run_rows<__nv_bfloat16>(op, split, coo_row, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
-    default: return run_rows<__half>(op, split, coo_row, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
+    case APT_F32: return run_rows<float>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
+    case APT_BF16: return run_rows<__nv_bfloat16>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
+    default: return run_rows<__half>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
   }
 }
 

@@ -1,5 +1,5 @@
 // Row kernels of the SpMM for __half rows.
-#include "spmm_bulk.cuh"
+#include "spmm_stream.cuh"
 
 namespace apt {
 APT_DEFINE_SPMM_ROWS(__half)

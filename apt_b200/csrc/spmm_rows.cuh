@@ -18,7 +18,7 @@
 //                block of 1024 threads per long row, the form before this, kept 26 of 148 SMs busy for
 //                62 us behind the row kernel.
 //
-// Wide rows of many edges have a kernel of their own (spmm_bulk.cuh).
+// Wide rows of many edges have a kernel of their own (spmm_stream.cuh).
 //
 // Where a row's edges are (`mode`):
 //   kFixed    every row has `fixed` consecutive edges: what a fanout sampler produces. No table.
@@ -29,13 +29,15 @@
 // What it measured is at rows_min_blocks.
 #pragma once
 
+#include <algorithm>
+
 #include "rows.cuh"
 
 namespace apt {
 
 constexpr int kMaxSegments = 64;
-// kUMulW: one fp32 weight per edge and head.
-enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kUMulW = 4 };
+// kUMulW: one fp32 weight per edge and head. kDots: no sums, but every edge's dots of its input row with the output row's own.
+enum { kCopyU = 0, kCopyE = 1, kUMulE = 2, kUAddE = 3, kUMulW = 4, kDots = 5 };
 enum { kDevice = -1, kFixed = 0, kRanges = 1, kOrder = 2 };
 
 // Rows of more edges are left to whole warps. A group narrower than a warp hands over earlier: its own pace is
@@ -74,13 +76,20 @@ struct SpmmWs {
   // written before they are read
   int2* range;          // [rows] first and last slot (edge) of every row
   uint32_t* rank;       // [edges] position inside its row
-  uint2* order;         // [edges] (source row, edge id), grouped by output row
+  uint2* order;         // grouped by output row, see OrderKind
   int4* items;          // [max_items] row, first, last slot, part (-1: the row's only item)
   float* part;          // [part_floats] partial sums
   int64_t max_items, max_parts, part_floats;
 };
 
 constexpr uint32_t kNoRank = 0xffffffffu;     // rank of an edge that belongs to no row
+
+// What the counting sort leaves in order[], a slot to an edge.
+enum OrderKind {
+  kByEdge = 0,      // uint2 (input row, edge), and items for long rows: k_spmm_rows
+  kByRow = 1,       // uint2 (input row, output row): k_spmm_stream
+  kByBoth = 2,      // uint4 (input row, output row, edge): k_spmm_stream with weights
+};
 
 __device__ __forceinline__ int seg_of(const int64_t* coo, int nseg, int64_t e) {
   int k = 0;
@@ -130,7 +139,55 @@ struct RowArgs {
   int part_stride;         // floats per part
   const int32_t* none;     // when given and not zero: no row has edges (kRanges)
   int32_t* status;         // flags of the call; null: the library's own word (apt_pending_flags)
+  const int64_t* col;      // output row of an edge, inside its segment
+  // kDots
+  const T* own;            // the output rows' own
+  float* dots;             // [E][heads]
+  uint32_t num_in;         // input rows; ws.cnt and ws.rank count their edges on the way
 };
+
+// ---- which rows k_spmm_stream takes (the figures are there) ------------------------------------
+constexpr int kStreamBlocks = 2;
+constexpr int stream_warps(bool one_slice) { return one_slice ? 12 : 10; }
+constexpr int kStreamShared = 112 * 1024 - 2560;      // a block's, beside its barriers and segment tables
+constexpr int kStreamHeads = 8;                       // weights an edge can bring along
+constexpr int kStreamMinSlices = 17, kStreamStretch = 32;
+constexpr int kStreamMinOrdered = 3 << 15, kStreamMinWide = 3 << 16, kStreamMinWeighted = 3 << 17, kStreamMinSums = 5 << 17;
+// Rows to a group; a warp has two groups on their way.
+constexpr int stream_group(bool one_slice) { return one_slice ? 8 : 4; }
+
+struct StreamPlan {
+  int row_bytes, warp_bytes;
+  int warps, shared;         // a block's
+  int lph;                   // kDots: lanes to a head
+};
+inline int stream_lph(int64_t feat_dim, size_t esz, int heads) { return pow2_ge(ceil_div((int64_t)(feat_dim / heads * esz), 16), 64); }
+inline bool stream_one_slice(int op, int64_t feat_dim, size_t esz, int heads) {
+  return op == kDots ? heads * stream_lph(feat_dim, esz, heads) <= 32 : feat_dim * (int64_t)esz <= 512;
+}
+inline StreamPlan stream_plan(int op, int64_t feat_dim, size_t esz, int heads) {
+  StreamPlan p{};
+  p.row_bytes = (int)(feat_dim * esz);
+  p.lph = op == kDots ? stream_lph(feat_dim, esz, heads) : 32;
+  p.warp_bytes = 2 * 8 * 512 + (op == kUMulW ? 64 * heads * 4 : 0);      // rows (two groups of eight of a slice a lane, four of two), weights
+  p.warps = std::min(stream_warps(stream_one_slice(op, feat_dim, esz, heads)), kStreamShared / p.warp_bytes);
+  p.shared = p.warps * p.warp_bytes;
+  return p;
+}
+// `slice`: bytes of the widest access to rows and results. `grouped`: the edges are (kFixed, kRanges).
+inline bool stream_fits(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges, bool grouped) {
+  const int64_t row = feat_dim * (int64_t)esz;
+  if (slice != 16 || row < kStreamMinSlices * 16 || row > 64 * 16 || heads > kStreamHeads) return false;
+  const int64_t least = !grouped ? kStreamMinOrdered : row > 512 ? kStreamMinWide : op == kCopyU ? kStreamMinSums : kStreamMinWeighted;
+  if (num_edges < least) return false;
+  if (op != kDots) return op == kCopyU || op == kUMulW;
+  const int lph = stream_lph(feat_dim, esz, heads);
+  return lph >= 4 && lph * heads <= 64;
+}
+inline OrderKind order_kind(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges) {
+  if (!stream_fits(op, slice, feat_dim, esz, heads, num_edges, false)) return kByEdge;
+  return op == kCopyU ? kByRow : kByBoth;
+}
 
 // One slice of one edge's contribution, in two steps so that the loads of several edges are issued
 // before any of them is used.
@@ -209,7 +266,7 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[V
 // Blocks an SM is to hold. The gather is bound by loads in flight, and the 64 (80) registers a thread of four (three)
 // blocks hold the slices of plain sums without spilling; edge values and 8 elements a slice need more.
 // 67 584 x 15 edges, bf16 x 256 (0.52 GB gathered, mostly out of L2): 89 us at one or two blocks, 65 at three, 63 at four;
-// reverse 104 / 82 / 90 us. (fp32 x 256 behaved the same; rows above 512 bytes of that many edges are k_spmm_bulk's now.)
+// reverse 104 / 82 / 90 us. (fp32 x 256 behaved the same; rows of that many edges are k_spmm_stream's now.)
 constexpr int rows_min_blocks(int op, int elems) {
   if (op == kCopyU || op == kCopyE || op == kUMulW) return elems <= 4 ? 4 : elems <= 8 ? 3 : 2;
   return elems <= 2 ? 3 : elems <= 8 ? 2 : 1;
@@ -471,14 +528,12 @@ static int launch_rows_vpl(const RowArgs<T>& a, cudaStream_t s) {
 }
 
 template <typename T, int OP>
-static int launch_bulk(const RowArgs<T>& a, cudaStream_t s, bool* taken);     // spmm_bulk.cuh
+static int launch_stream(const RowArgs<T>& a, cudaStream_t s);     // spmm_stream.cuh
 
 template <typename T, int OP>
 static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
   if constexpr (OP == kCopyU || OP == kUMulW) {
-    bool taken = false;
-    const int rc = launch_bulk<T, OP>(a, s, &taken);
-    if (taken || rc != APT_OK) return rc;
+    if (stream_fits(OP, a.split.ve * (int)sizeof(T), a.feat_dim, sizeof(T), OP == kCopyU ? 1 : (int)a.edata_dim, a.num_edges, a.mode == kFixed || a.mode == kRanges)) return launch_stream<T, OP>(a, s);
   }
   switch (a.split.ve * (int)sizeof(T)) {
     case 16: return launch_rows_vpl<T, 16 / sizeof(T), OP>(a, s);
@@ -500,16 +555,17 @@ int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
       case kCopyE: return launch_rows_ve<T, kCopyE>(a, s);                                \
       case kUMulE: return launch_rows_ve<T, kUMulE>(a, s);                                \
       case kUAddE: return launch_rows_ve<T, kUAddE>(a, s);                                \
+      case kDots: return launch_stream<T, kDots>(a, s);                                \
       default: return launch_rows_ve<T, kUMulW>(a, s);                                   \
     }                                                                                                    \
   }
 
 // ---- shared by spmm.cu and gat.cu -----------------------------------------------------
-constexpr int kBulkWaitPolls = 1 << 20;      // of an mbarrier, each of which may suspend for a while itself
+constexpr int kStreamWaitPolls = 1 << 20;      // of an mbarrier, each of which may suspend for a while itself
 int bulk_wait_polls();
 int pending_word(int32_t** word);            // for flags of calls without a status word: see spmm.cu
 size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws);
 // Counted edges (ws.cnt) to places: ws.range, and the items of long rows.
-int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, int long_edges, int part_stride, cudaStream_t s);
+int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, OrderKind kind, int long_edges, int part_stride, cudaStream_t s);
 
 }  // namespace apt

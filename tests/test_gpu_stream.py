@@ -1,0 +1,96 @@
+"""Sums and dots of wide rows of many edges, which a warp takes from a stretch of the edges: row ends, rows without edges
+and rows of many stretches, and the lanes that a row does not fill.
+
+Bounds: sums of small whole numbers are exact in fp32, and a 16-bit result is one rounding of them. The attention layer is
+held to the 2-norm of the fp64 results: about 15 fp32 terms a sum (2e-6), and 2^-9 or 2^-12 for a rounding to 16 bits. The
+gradient of el is added up in fp32 one edge after another: n edges of a source are off by about root(n) 2^-25 of it, and the
+first source here has 393 000 / 9001^(1/4) = 40 400, which is 6e-6."""
+import pytest
+import torch
+
+from apt_b200 import ops
+
+pytestmark = pytest.mark.gpu
+N_IN = 5003
+
+
+def _lengths(shape, edges, gen):
+    """Edges of every output row: a fanout; 0 to 60; one row of almost half of all edges (thousands of stretches) among short ones."""
+    if shape == "fixed":
+        return torch.full((edges // 13 + 1,), 13, device="cuda")
+    n = torch.randint(0, 61 if shape == "ragged" else 9, (edges // (30 if shape == "ragged" else 8),), device="cuda", generator=gen)
+    if shape == "hub":
+        n[n.numel() // 3] = edges // 2
+        n[-1] = n[0] = 0
+    else:
+        n[n.numel() // 2] = 0
+        n[n.numel() // 2] = max(0, edges + 5 - int(n.sum()))
+    return n
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 68), (torch.float32, 128), (torch.float32, 260 - 4), (torch.bfloat16, 136),
+                                     (torch.bfloat16, 256), (torch.float16, 264)])
+@pytest.mark.parametrize("shape,edges", [("fixed", 655_360), ("ragged", 655_360), ("hub", 98_304), ("hub", 400_000)])
+def test_sums(dtype, D, shape, edges):
+    gen = torch.Generator(device="cuda").manual_seed(D + edges)
+    n = _lengths(shape, edges, gen)
+    col = torch.arange(n.numel(), device="cuda").repeat_interleave(n)
+    if shape == "hub":
+        col = col[torch.randperm(col.numel(), device="cuda", generator=gen)]
+        pad = edges - col.numel() + 3
+        col = torch.cat([col, torch.full((max(0, pad),), n.numel() // 2, device="cuda")])
+    row = torch.randint(0, N_IN, (col.numel(),), device="cuda", generator=gen)
+    x = torch.randint(-3, 4, (N_IN, D), device="cuda", generator=gen).to(dtype)
+    off = [torch.tensor([0, k], device="cuda") for k in (col.numel(), N_IN, n.numel())]
+    assert col.numel() >= edges
+    want = torch.zeros((n.numel(), D), device="cuda", dtype=torch.float64).index_add_(0, col, x.double()[row]).to(dtype)
+    assert torch.equal(ops.spmm_copy_u_sum(row, col, x, *off), want)
+
+
+def _layer(row, col, ft, el, er, g, n_dst):
+    """The attention layer and its gradients in fp64."""
+    ft, el, er = (t.double().requires_grad_() for t in (ft, el, er))
+    s = torch.nn.functional.leaky_relu(el[row] + er[col], 0.2)
+    at = col[:, None, None].expand_as(s)
+    most = torch.full((n_dst, *s.shape[1:]), -torch.inf, device="cuda", dtype=torch.float64).scatter_reduce(0, at, s.detach(), "amax")
+    p = (s - most[col]).exp()
+    a = p / torch.zeros_like(most).index_add(0, col, p)[col]
+    out = torch.zeros((n_dst, *ft.shape[1:]), device="cuda", dtype=torch.float64).index_add(0, col, a * ft[row])
+    return (out.detach(),) + torch.autograd.grad(out, (ft, el, er), g.double())
+
+
+@pytest.mark.parametrize("dtype,H,D", [(torch.float32, 4, 32), (torch.float32, 1, 256), (torch.float32, 8, 32), (torch.float32, 4, 48),
+                                       (torch.float32, 2, 44), (torch.bfloat16, 4, 64), (torch.bfloat16, 8, 24), (torch.float16, 5, 40),
+                                       (torch.float16, 2, 256)])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_attention(dtype, H, D, ragged):
+    gen = torch.Generator(device="cuda").manual_seed(H * D)
+    n = torch.randint(0, 29, (30_001,), device="cuda", generator=gen) if ragged else torch.full((28_101,), 14, device="cuda")
+    n[7] += 500
+    col = torch.arange(n.numel(), device="cuda").repeat_interleave(n)
+    n_dst, n_src, E = n.numel(), 9001, col.numel()
+    assert E >= 393_216
+    row = (torch.rand(E, device="cuda", generator=gen) ** 4 * n_src).long().clamp_(max=n_src - 1)
+    make = lambda *shape: torch.randn(shape, device="cuda", generator=gen).to(dtype)
+    ft, el, er, g = make(n_src, H, D), make(n_src, H, 1), make(n_dst, H, 1), make(n_dst, H, D)
+    want = _layer(row, col, ft, el, er, g, n_dst)
+    leaves = [t.clone().requires_grad_() for t in (ft, el, er)]
+    out = ops.GATEdgeSoftmaxSum.apply(row, col, *leaves, n_dst, 0.2)
+    bound = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dtype]
+    for k, (got, ref) in enumerate(zip((out,) + torch.autograd.grad(out, leaves, g), want)):
+        assert float((got.double() - ref).norm() / ref.norm()) <= (max(bound, 6e-6) if k == 2 else bound)
+
+
+def test_dots_beside_infinite_features():
+    # heads of 12 slices on 16 lanes: the lanes without a slice add nothing, and a head's infinities stay in it
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    n_dst, n_src, H, D = 28_101, 9001, 4, 48
+    col = torch.arange(n_dst, device="cuda").repeat_interleave(14)
+    row = torch.randint(0, n_src, (col.numel(),), device="cuda", generator=gen)
+    make = lambda *shape: torch.randn(shape, device="cuda", generator=gen)
+    ft, el, er, g = make(n_src, H, D), make(n_src, H, 1), make(n_dst, H, 1), make(n_dst, H, D)
+    plain = ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, g)
+    ft[:, 0] = torch.inf
+    _, g_el, g_er = ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, g)
+    assert torch.equal(g_er[:, 1:], plain[2][:, 1:]) and not bool(g_er[:, 0].isfinite().any())
+    assert float((g_el[:, 1:] - plain[1][:, 1:]).norm() / plain[1][:, 1:].norm()) <= 2e-6      # (44 edges a source, added up in the order of arrival)
