@@ -209,7 +209,7 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
         if (base != r.x) my_src = (uint32_t)row[min(base + lane, r.y - 1)];
         const bool ranked = h0 == 0 && lane < cnt;
         uint32_t place = kNoRank;
-        if (ranked && my_src < num_src) place = (uint32_t)atomicAdd(src_count + my_src, 1);
+        if (ranked && my_src < num_src) place = (uint32_t)atomicAdd(src_count + spread(my_src), 1);
 #pragma unroll 1
         for (int j0 = 0; j0 < cnt; j0 += ep * 4) {
           float dt[4] = {0.f, 0.f, 0.f, 0.f};
@@ -259,7 +259,7 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
   }
 }
 
-// Score gradients, added to sums[source][head].
+// Score gradients, added to sums[spread(source)][head].
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
@@ -304,7 +304,7 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
         if (e0 + k >= r.y) break;
         const float gs = w[k] * (dot[k] - t) * (x[k] + bias > 0.f ? 1.f : slope);
         ger += gs;
-        if ((uint64_t)src[k] < (uint64_t)num_src) atomicAdd(sums + src[k] * num_heads + h, gs);
+        if ((uint64_t)src[k] < (uint64_t)num_src) atomicAdd(sums + (int64_t)spread((uint32_t)src[k]) * num_heads + h, gs);
       }
     }
     grad_er[i] = Elem<T>::from_f(ger);
@@ -322,10 +322,12 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_gat_source(const float* __restrict__ sums, int64_t n, T* __restrict__ grad_el) {
+k_gat_source(const float* __restrict__ sums, int64_t n, uint32_t num_heads, T* __restrict__ grad_el) {
   wait_for_previous();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    grad_el[i] = Elem<T>::from_f(sums[i]);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t row = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)row * num_heads);
+    grad_el[i] = Elem<T>::from_f(sums[(int64_t)spread(row) * num_heads + h]);
+  }
 }
 
 // ---- host side ----------------------------------------------------------------------
@@ -349,13 +351,13 @@ static size_t gat_edges_layout(int64_t num_dst, int64_t E, int H, char* base, Ga
 }
 
 struct GatBwdWs {
-  float* sums;      // [num_src][heads], cleared with the front of the sort
+  float* sums;      // [spread_rows(num_src)][heads], cleared with the front of the sort
   SpmmWs sort;      // its order: slots of 16 bytes (kByBoth)
   float* dots;      // [E][heads]
   size_t zero_bytes;
 };
 static size_t gat_bwd_layout(int64_t num_src, int64_t E, int H, char* base, GatBwdWs* ws) {
-  const size_t o_sort = align_up((size_t)(num_src > 0 ? num_src : 1) * H * 4, 256);
+  const size_t o_sort = align_up((size_t)spread_rows(num_src > 0 ? num_src : 1) * H * 4, 256);
   const size_t o_dots = o_sort + spmm_layout(num_src, E, base + o_sort, ws ? &ws->sort : nullptr);
   const size_t o_order = o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
   if (ws) {
@@ -482,7 +484,7 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
     rc = launch_spmm_rows<T>(kUMulW, a, s);
   }
   if (rc != APT_OK) return rc;
-  APT_FOLLOW(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (T*)grad_el);
+  APT_FOLLOW(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (uint32_t)q.H, (T*)grad_el);
   return APT_OK;
 }
 

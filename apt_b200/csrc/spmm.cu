@@ -35,7 +35,7 @@ size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) 
     return o;
   };
   const size_t o_words = take(64);
-  const size_t o_cnt = take((size_t)rows * 4);
+  const size_t o_cnt = take((size_t)spread_rows(rows) * 4);
   const size_t o_done = take((size_t)max_parts * 4);
   const size_t zero = at;
   const size_t o_range = take((size_t)(rows + 1) * 8);
@@ -298,7 +298,7 @@ k_dst_rank(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_
       d[k] = e < E ? out_row(coo, ooff, st.nseg, col, e) : (int64_t)-1;
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) r[k] = d[k] >= 0 && d[k] < num_rows ? (uint32_t)atomicAdd(ws.cnt + d[k], 1) : kNoRank;
+    for (int k = 0; k < K; ++k) r[k] = d[k] >= 0 && d[k] < num_rows ? (uint32_t)atomicAdd(ws.cnt + spread((uint32_t)d[k]), 1) : kNoRank;
 #pragma unroll
     for (int k = 0; k < K; ++k)
       if (e0 + k * stride < E) ws.rank[e0 + k * stride] = r[k];
@@ -318,7 +318,7 @@ k_dst_slots(int64_t num_rows, SpmmWs ws, int mode, OrderKind kind, int long_edge
   int v[kScanRows], mine = 0;
 #pragma unroll
   for (int k = 0; k < kScanRows; ++k) {
-    v[k] = first + k < num_rows ? ws.cnt[first + k] : 0;
+    v[k] = first + k < num_rows ? ws.cnt[spread((uint32_t)(first + k))] : 0;
     mine += v[k];
   }
   int total;

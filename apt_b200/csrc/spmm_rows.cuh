@@ -70,7 +70,7 @@ struct SpmmWs {
   int32_t* num_items;   // [1]
   int32_t* num_slots;   // [1] slots of order[] given out
   int32_t* num_parts;   // [1] rows of part[] given out
-  int32_t* cnt;         // [rows] edges per row
+  int32_t* cnt;         // [spread_rows(rows)] edges per row, at spread(row)
   int32_t* part_done;   // [max_parts] items of a row that have finished, at the row's first part
   size_t zero_bytes;
   // written before they are read
@@ -83,6 +83,13 @@ struct SpmmWs {
 };
 
 constexpr uint32_t kNoRank = 0xffffffffu;     // rank of an edge that belongs to no row
+
+// Where a row's counter is. Ids go by first occurrence, so the first rows are the ones that many edges share, and atomics on
+// one line queue up in one slice of L2: with 32 neighbours to a line, the first line of a block of a million edges over 151 552
+// sources gets 15 000 of them, one after another, which is what counting them took (27 us; sources at random 14). 32 rows
+// that are 32 apart share a line instead (a tile of 1024 rows is transposed), the first one 4800: 27 -> 17 us.
+__host__ __device__ inline uint32_t spread(uint32_t row) { return (row & ~1023u) | (row & 31u) << 5 | (row >> 5 & 31u); }
+inline int64_t spread_rows(int64_t rows) { return (rows + 1023) / 1024 * 1024; }
 
 // What the counting sort leaves in order[], a slot to an edge.
 enum OrderKind {

@@ -160,7 +160,7 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
       r.row = mode == kFixed ? (uint32_t)k / (uint32_t)fixed : out_row(k);
       if (k < hi) r.src = (uint32_t)(ioff[a.st.nseg > 1 ? seg_of(coo, a.st.nseg, k) : 0] + a.row[k]);
     }
-    if constexpr (kIsDots) r.e = k < hi && r.src < a.num_in ? (uint32_t)atomicAdd(a.ws.cnt + r.src, 1) : kNoRank;
+    if constexpr (kIsDots) r.e = k < hi && r.src < a.num_in ? (uint32_t)atomicAdd(a.ws.cnt + spread(r.src), 1) : kNoRank;
     return r;
   };
   // what was under way when the batch was loaded has arrived
