@@ -12,14 +12,14 @@
 // heads, which stay in L2):
 //
 //   k_gat_ranges    where each destination's edges are
-//   k_gat_weights   one thread per destination and head: scores and softmax. Full occupancy hides the two dependent
-//                   loads of a score; any number of edges and heads.
+//   k_gat_weights   scores and softmax, a few lanes per destination, two edges a lane, four heads at a time; any number of
+//                   edges and heads.
 //   row kernel      the weighted sum is the SpMM's row kernel (kUMulW), any head width
 //   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination (wide rows of many edges:
 //                   k_spmm_stream's kDots). The four partial dots of a lane are reduced together: each step halves the values
 //                   a lane keeps, log2(lph) + 1 shuffles for four edges instead of 4 log2(lph).
-//   k_gat_scores    backward: t, grad_s and grad_er, one thread per destination and head; grad_el is added up in fp32 with
-//                   one reduction per edge and head (the heads of an edge are neighbours: one sector)
+//   k_gat_scores    backward: t, grad_s and grad_er, the same lanes; grad_el is added up in fp32 with one reduction per edge
+//                   of all its heads
 //   row kernel      grad_ft: the weighted sum of the forward with the sides swapped. With grad_el as a second accumulator
 //                   of the same walk it held two blocks an SM instead of three: 150 us against 116, and the scores had to
 //                   be written out for it.
@@ -34,7 +34,7 @@
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 18 + 61 us. Backward of that block: 18 (saved after a forward) + 80 + 7 + 44 + 63 + 5 us,
+// kernels take 17 + 61 us. Backward of that block: 17 (saved after a forward) + 80 + 5 + 30 + 63 + 5 us,
 // where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 
@@ -90,71 +90,139 @@ k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* 
   }
 }
 
-// Attention weights, W lanes to a destination and head. K edges' loads of a lane are in flight; a destination of at most K * W
-// edges keeps its scores in registers. W is 2 above a mean of 16 edges, where one lane would walk its edges three times, two
-// dependent loads each: forward of 30 000 destinations of 20 / 25 / 32 edges, bf16 4 x 64, 58 / 72 / 90 -> 56 / 68 / 76 us,
-// fp16 2 x 10 39 / 45 / 57 -> 34 / 39 / 39. (One lane with 32 scores takes half the warps' registers: 59 / 76 / 82 and 37 / 43 / 45.)
-template <typename T, int W>
+// W lanes to a destination, kGatEdges edges a lane, the edges of a round side by side: loads and stores of a value per edge are
+// coalesced, a destination of up to W * kGatEdges edges is one round of latency, and the reductions to sums carry NH heads each.
+// A thread per destination and head before: weights 19 -> 17.5 us, scores 43 -> 30 (67 584 x 15 edges, bf16, 4 heads); forward
+// and backward of 30 000 destinations, bf16 4 x 64, 3 to 32 edges 114 - 290 -> 96 - 232 with the streams, fp32 1 x 32 x 25 170 -> 136.
+constexpr int kGatEdges = 2;
+template <int NH>
+struct Heads {
+  float v[NH];
+};
+template <int NH>
+__device__ __forceinline__ Heads<NH> load_heads(const float* p) {      // aligned to all of them
+  const Pack<float, NH> w = load_pack<float, NH>(p);
+  Heads<NH> r;
+#pragma unroll
+  for (int h = 0; h < NH; ++h) r.v[h] = w.v[h];
+  return r;
+}
+template <typename T, int NH>
+__device__ __forceinline__ Heads<NH> load_scores(const T* p) {         // the same
+  const Pack<T, NH> w = load_pack<T, NH>(p);
+  Heads<NH> r;
+#pragma unroll
+  for (int h = 0; h < NH; ++h) r.v[h] = Elem<T>::to_f(w.v[h]);
+  return r;
+}
+template <int W>
+__device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+  for (int o = 1; o < W; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Attention weights.
+template <typename T, int W, int NH>
 __global__ void __launch_bounds__(256)
 k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
               int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ weight,
               T* __restrict__ attn, int masked) {
   wait_for_previous();
-  constexpr int K = 16;
+  constexpr int K = kGatEdges;
   if (*none != 0) return;
-  const int64_t total = num_dst * num_heads, stride = (int64_t)gridDim.x * blockDim.x / W;
+  const int64_t stride = (int64_t)gridDim.x * (256 / W);
   const int part = threadIdx.x & (W - 1);
-  const unsigned mask = W == 1 ? 0u : ((1u << W) - 1u) << (threadIdx.x & 31 & ~(W - 1));
-  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / W; i < total; i += stride) {
-    const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
-    const int2 r = range[d];
-    const float bias = Elem<T>::to_f(er[i]);
-    const int deg = r.y - r.x, mine = (deg - part + W - 1) / W;      // this lane's edges: r.x + part, every W-th
-    float s[K], m = -INFINITY, sum = 0.f;
-    auto score = [&](int e) { return leaky(Elem<T>::to_f(el[row[e] * num_heads + h]) + bias, slope); };
-    if (deg <= K * W) {
-      uint32_t src[K];
+  // (all lanes of a warp stay: groups behind the last destination have no edges)
+  for (int64_t d0 = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; d0 < num_dst; d0 += stride) {
+    const int64_t d = d0 + (threadIdx.x & 31) / W;
+    const bool there = d < num_dst;
+    const int2 r = there ? range[d] : make_int2(0, 0);
+    const int deg = r.y - r.x;
+    const bool few = deg <= K * W;
+    uint32_t src[K];
 #pragma unroll
-      for (int k = 0; k < K; ++k) src[k] = k < mine ? (uint32_t)row[r.x + part + k * W] : 0u;
+    for (int k = 0; k < K; ++k) src[k] = few && r.x + part + k * W < r.y ? (uint32_t)row[r.x + part + k * W] : 0u;
+#pragma unroll 1
+    for (int h0 = 0; h0 < num_heads; h0 += NH) {
+      Heads<NH> bias, s[K];
+      float most[NH], sum[NH], inv[NH];
+      bool zero[NH];
 #pragma unroll
-      for (int k = 0; k < K; ++k) s[k] = k < mine ? Elem<T>::to_f(el[(int64_t)src[k] * num_heads + h]) : 0.f;
+      for (int h = 0; h < NH; ++h) {
+        bias.v[h] = there ? Elem<T>::to_f(er[d * num_heads + h0 + h]) : 0.f;
+        most[h] = -INFINITY;
+        sum[h] = 0.f;
+      }
+      auto scores = [&](int64_t from) {
+        Heads<NH> x = load_scores<T, NH>(el + from * num_heads + h0);
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (k < mine) {
-          s[k] = leaky(s[k] + bias, slope);
-          m = fmaxf(m, s[k]);
+        for (int h = 0; h < NH; ++h) x.v[h] = leaky(x.v[h] + bias.v[h], slope);
+        return x;
+      };
+      if (few) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (r.x + part + k * W < r.y) {
+            s[k] = scores(src[k]);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], s[k].v[h]);
+          }
+      } else {
+        for (int e = r.x + part; e < r.y; e += W) {
+          const Heads<NH> x = scores(row[e]);
+#pragma unroll
+          for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], x.v[h]);
         }
-    } else {
-      for (int e = r.x + part; e < r.y; e += W) m = fmaxf(m, score(e));
-    }
+      }
 #pragma unroll
-    for (int o = 1; o < W; o <<= 1) m = fmaxf(m, __shfl_xor_sync(mask, m, o));
-    if (deg <= K * W) {
+      for (int h = 0; h < NH; ++h)
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (k < mine) {
-          s[k] = expf(s[k] - m);
-          sum += s[k];
+        for (int o = 1; o < W; o <<= 1) most[h] = fmaxf(most[h], __shfl_xor_sync(0xffffffffu, most[h], o));
+      if (few) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (r.x + part + k * W < r.y)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+              s[k].v[h] = expf(s[k].v[h] - most[h]);
+              sum[h] += s[k].v[h];
+            }
+      } else {
+        for (int e = r.x + part; e < r.y; e += W) {
+          const Heads<NH> x = scores(row[e]);
+#pragma unroll
+          for (int h = 0; h < NH; ++h) sum[h] += expf(x.v[h] - most[h]);
         }
-    } else {
-      for (int e = r.x + part; e < r.y; e += W) sum += expf(score(e) - m);
-    }
+      }
 #pragma unroll
-    for (int o = 1; o < W; o <<= 1) sum += __shfl_xor_sync(mask, sum, o);
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
-    const bool zero = !(sum > 0.f) && deg <= masked;
-    auto put = [&](int e, float w) {
-      const int64_t o = (int64_t)e * num_heads + h;
-      if (zero) w = 0.f;
-      weight[o] = w;
-      if (attn) attn[o] = Elem<T>::from_f(w);
-    };
-    if (deg <= K * W) {
+      for (int h = 0; h < NH; ++h) {
+        sum[h] = lanes_sum<W>(sum[h]);
+        inv[h] = sum[h] > 0.f ? 1.f / sum[h] : 0.f;
+        zero[h] = !(sum[h] > 0.f) && deg <= masked;
+      }
+      auto put = [&](int e, const Heads<NH>& p) {
+        const int64_t o = (int64_t)e * num_heads + h0;
+        Pack<float, NH> w;
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (k < mine) put(r.x + part + k * W, s[k] * inv);
-    } else {
-      for (int e = r.x + part; e < r.y; e += W) put(e, expf(score(e) - m) * inv);
+        for (int h = 0; h < NH; ++h) w.v[h] = zero[h] ? 0.f : p.v[h] * inv[h];
+        store_pack<float, NH>(weight + o, w);
+        if (attn)
+#pragma unroll
+          for (int h = 0; h < NH; ++h) attn[o + h] = Elem<T>::from_f(w.v[h]);
+      };
+      if (few) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (r.x + part + k * W < r.y) put(r.x + part + k * W, s[k]);
+      } else {
+        for (int e = r.x + part; e < r.y; e += W) {
+          Heads<NH> x = scores(row[e]);
+#pragma unroll
+          for (int h = 0; h < NH; ++h) x.v[h] = expf(x.v[h] - most[h]);
+          put(e, x);
+        }
+      }
     }
   }
 }
@@ -259,63 +327,114 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
   }
 }
 
-// Score gradients, added to sums[spread(source)][head].
-template <typename T>
+// sums[] += v, for NH heads at once.
+template <int NH>
+__device__ __forceinline__ void add_heads(float* p, const Heads<NH>& v) {
+  if constexpr (NH == 4) atomicAdd((float4*)p, make_float4(v.v[0], v.v[1], v.v[2], v.v[3]));
+  else if constexpr (NH == 2) atomicAdd((float2*)p, make_float2(v.v[0], v.v[1]));
+  else atomicAdd(p, v.v[0]);
+}
+
+// Score gradients, added to sums[spread(source)][head], and the destination's edges to their places in the order by source.
+template <typename T, int W, int NH>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
              int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
              float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort, OrderKind kind,
              T* __restrict__ grad_er) {
   wait_for_previous();
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int K = kGatEdges;
   const bool empty = *none != 0;
   if (empty)   // no edge belongs to anybody
-    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += stride) weight[o] = 0.f;
-  const int64_t total = num_dst * num_heads;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const uint32_t d = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)d * num_heads);
-    const int2 r = empty ? make_int2(0, 0) : range[d];
-    const float bias = Elem<T>::to_f(er[i]);
-    float t = 0.f, ger = 0.f;
-    // two short walks rather than one that keeps everything in registers: the second finds its values in L1 and L2
-#pragma unroll 8
-    for (int e = r.x; e < r.y; ++e) {
-      const int64_t o = (int64_t)e * num_heads + h;
-      t += weight[o] * dots[o];
+    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += (int64_t)gridDim.x * blockDim.x) weight[o] = 0.f;
+  const int64_t stride = (int64_t)gridDim.x * (256 / W);
+  const int part = threadIdx.x & (W - 1);
+  for (int64_t d0 = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; d0 < num_dst; d0 += stride) {
+    const int64_t d = d0 + (threadIdx.x & 31) / W;
+    const bool there = d < num_dst;
+    const int2 r = there && !empty ? range[d] : make_int2(0, 0);
+    const int deg = r.y - r.x;
+    const bool few = deg <= K * W;
+    // an edge to its place
+    auto place_of = [&](int e) { return sort.rank[e]; };
+    auto put = [&](int e, int64_t src, uint32_t place) {
+      if (place == kNoRank) return;
+      const uint32_t at = (uint32_t)sort.range[src].x + place;
+      if (kind == kByBoth) ((uint4*)sort.order)[at] = make_uint4((uint32_t)d, (uint32_t)src, (uint32_t)e, 0u);
+      else sort.order[at] = make_uint2((uint32_t)d, (uint32_t)e);
+    };
+    int64_t src[K];
+    uint32_t place[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = r.x + part + k * W;
+      src[k] = few && e < r.y ? row[e] : 0;
+      place[k] = few && e < r.y ? place_of(e) : kNoRank;
     }
-    // four edges' loads ahead of their adds (44 us; eight or sixteen take the registers of half the warps: 51, 81)
-    constexpr int C = 4;
 #pragma unroll 1
-    for (int e0 = r.x; e0 < r.y; e0 += C) {
-      int64_t src[C];
-      float w[C], dot[C], x[C];
+    for (int h0 = 0; h0 < num_heads; h0 += NH) {
+      Heads<NH> bias, w[K], dot[K], x[K];
+      float t[NH], ger[NH];
 #pragma unroll
-      for (int k = 0; k < C; ++k) src[k] = row[min(e0 + k, r.y - 1)];
+      for (int h = 0; h < NH; ++h) {
+        bias.v[h] = there ? Elem<T>::to_f(er[d * num_heads + h0 + h]) : 0.f;
+        t[h] = ger[h] = 0.f;
+      }
+      auto fetch = [&](int e, Heads<NH>& a, Heads<NH>& b) {
+        a = load_heads<NH>(weight + (int64_t)e * num_heads + h0);
+        b = load_heads<NH>(dots + (int64_t)e * num_heads + h0);
+      };
+      if (few) {
 #pragma unroll
-      for (int k = 0; k < C; ++k) {
-        const int64_t o = (int64_t)min(e0 + k, r.y - 1) * num_heads + h;
-        w[k] = weight[o];
-        dot[k] = dots[o];
+        for (int k = 0; k < K; ++k)
+          if (r.x + part + k * W < r.y) {
+            fetch(r.x + part + k * W, w[k], dot[k]);
+            x[k] = load_scores<T, NH>(el + src[k] * num_heads + h0);
+          }
+        if (h0 == 0)
+#pragma unroll
+          for (int k = 0; k < K; ++k) put(r.x + part + k * W, src[k], place[k]);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (r.x + part + k * W < r.y)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) t[h] += w[k].v[h] * dot[k].v[h];
+      } else {
+        for (int e = r.x + part; e < r.y; e += W) {
+          fetch(e, w[0], dot[0]);
+#pragma unroll
+          for (int h = 0; h < NH; ++h) t[h] += w[0].v[h] * dot[0].v[h];
+        }
       }
 #pragma unroll
-      for (int k = 0; k < C; ++k) x[k] = Elem<T>::to_f(el[src[k] * num_heads + h]);
+      for (int h = 0; h < NH; ++h) t[h] = lanes_sum<W>(t[h]);
+      auto grad = [&](int64_t from, const Heads<NH>& a, const Heads<NH>& b, const Heads<NH>& c) {
+        Heads<NH> gs;
 #pragma unroll
-      for (int k = 0; k < C; ++k) {
-        if (e0 + k >= r.y) break;
-        const float gs = w[k] * (dot[k] - t) * (x[k] + bias > 0.f ? 1.f : slope);
-        ger += gs;
-        if ((uint64_t)src[k] < (uint64_t)num_src) atomicAdd(sums + (int64_t)spread((uint32_t)src[k]) * num_heads + h, gs);
+        for (int h = 0; h < NH; ++h) {
+          gs.v[h] = a.v[h] * (b.v[h] - t[h]) * (c.v[h] + bias.v[h] > 0.f ? 1.f : slope);
+          ger[h] += gs.v[h];
+        }
+        if ((uint64_t)from < (uint64_t)num_src) add_heads<NH>(sums + (int64_t)spread((uint32_t)from) * num_heads + h0, gs);
+      };
+      if (few) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (r.x + part + k * W < r.y) grad(src[k], w[k], dot[k], x[k]);
+      } else {
+        for (int e = r.x + part; e < r.y; e += W) {
+          const int64_t from = row[e];
+          fetch(e, w[0], dot[0]);
+          x[0] = load_scores<T, NH>(el + from * num_heads + h0);
+          if (h0 == 0) put(e, from, place_of(e));
+          grad(from, w[0], dot[0], x[0]);
+        }
       }
-    }
-    grad_er[i] = Elem<T>::from_f(ger);
-    // the destination's edges to their places in the order by source, a share for every head's thread
-#pragma unroll 4
-    for (int e = r.x + (int)h; e < r.y; e += num_heads) {
-      const uint32_t place = sort.rank[e];
-      if (place == kNoRank) continue;
-      const uint32_t at = (uint32_t)sort.range[row[e]].x + place;
-      if (kind == kByBoth) ((uint4*)sort.order)[at] = make_uint4(d, (uint32_t)row[e], (uint32_t)e, 0u);
-      else sort.order[at] = make_uint2(d, (uint32_t)e);
+#pragma unroll
+      for (int h = 0; h < NH; ++h) {
+        ger[h] = lanes_sum<W>(ger[h]);
+        if (there && part == 0) grad_er[d * num_heads + h0 + h] = Elem<T>::from_f(ger[h]);
+      }
     }
   }
 }
@@ -395,6 +514,34 @@ static int gat_ranges(const GatProblem& q, const GatEdges& g, cudaStream_t s) {
   return APT_OK;
 }
 
+// Lanes to a destination: as many as hold a mean one's edges. Heads at a time: as many as there are, if el can be read so.
+#define APT_GAT_LANES(q, RUN)                                                             \
+  do {                                                                                    \
+    const int lanes__ = pow2_ge(ceil_div(ceil_div(q.E, q.num_dst), kGatEdges)), nh__ = gat_heads(q, sizeof(T)); \
+    if (lanes__ <= 4) {                                                                   \
+      if (nh__ == 4) RUN(4, 4);                                                           \
+      else if (nh__ == 2) RUN(4, 2);                                                      \
+      else RUN(4, 1);                                                                     \
+    } else if (lanes__ <= 8) {                                                            \
+      if (nh__ == 4) RUN(8, 4);                                                           \
+      else if (nh__ == 2) RUN(8, 2);                                                      \
+      else RUN(8, 1);                                                                     \
+    } else if (lanes__ <= 16) {                                                           \
+      if (nh__ == 4) RUN(16, 4);                                                          \
+      else if (nh__ == 2) RUN(16, 2);                                                     \
+      else RUN(16, 1);                                                                    \
+    } else {                                                                              \
+      if (nh__ == 4) RUN(32, 4);                                                          \
+      else if (nh__ == 2) RUN(32, 2);                                                     \
+      else RUN(32, 1);                                                                    \
+    }                                                                                     \
+  } while (0);
+static int gat_heads(const GatProblem& q, size_t esz) {
+  for (int nh = 4; nh > 1; nh >>= 1)
+    if (q.H % nh == 0 && (uintptr_t)q.el % (nh * esz) == 0) return nh;
+  return 1;
+}
+
 // Ranges and attention weights.
 template <typename T>
 static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaStream_t s) {
@@ -402,11 +549,10 @@ static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaS
   if (rc != APT_OK) return rc;
   ProfScope prof("gat_rows", s);
   const int masked = masked_edges(q.H, q.Dh, sizeof(T), (uintptr_t)q.ft);
-#define APT_WEIGHTS(W)                                                                                                       \
-  APT_FOLLOW((k_gat_weights<T, W>), wave_grid(ceil_div(q.num_dst * q.H * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
+#define APT_WEIGHTS(W, NH)                                                                                                   \
+  APT_FOLLOW((k_gat_weights<T, W, NH>), wave_grid(ceil_div(q.num_dst * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
              q.H, q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn, masked)
-  if (q.E > 16 * q.num_dst) APT_WEIGHTS(2);
-  else APT_WEIGHTS(1);
+  APT_GAT_LANES(q, APT_WEIGHTS)
 #undef APT_WEIGHTS
   return APT_OK;
 }
@@ -474,8 +620,11 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
     rc = gat_dots<T>(q, g, ws, num_src, s);
     if (rc == APT_OK) rc = launch_slots(num_src, ws.sort, kOrder, kind, split.long_edges, (int)dim, s);
     if (rc != APT_OK) return rc;
-    APT_FOLLOW(k_gat_scores<T>, wave_grid(ceil_div(q.num_dst * q.H, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, q.H,
-               q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, ws.dots, ws.sums, ws.sort, kind, (T*)grad_er);
+#define APT_SCORES(W, NH)                                                                                                    \
+  APT_FOLLOW((k_gat_scores<T, W, NH>), wave_grid(ceil_div(q.num_dst * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
+             q.H, q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, ws.dots, ws.sums, ws.sort, kind, (T*)grad_er)
+    APT_GAT_LANES(q, APT_SCORES)
+#undef APT_SCORES
   }
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, num_src, q.E, ws.sort,
                      (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr, q.status, nullptr, nullptr, nullptr, 0u};
