@@ -480,7 +480,7 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
     return APT_ERR_CAPACITY;
   }
   ProfScope prof("unique_sorted", s);
-  const int g = wave_grid(ceil_div(num_ids, 256), 8);
+  const int g = wave_grid(ceil_div(num_ids, 256), 8, 1);
   APT_FOLLOW(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, ws.counts, status_word);
   APT_FOLLOW(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.counts, ws.info,
              out_unique, out_num_unique);

@@ -72,7 +72,7 @@ struct SampleInsert {
 };
 
 template <int G, bool INSERT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
 sample_replace_kernel(const int64_t* __restrict__ seeds, int64_t num_seeds,
                       const int64_t* __restrict__ num_seeds_dev, int fanout, CscView g, uint32_t k0,
                       uint32_t k1, uint32_t call_id, const int64_t* __restrict__ call_base_dev,

@@ -151,7 +151,7 @@ extern "C" int apt_src_to_vir(const int64_t* src, int64_t num_src, int64_t fanou
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("src_to_vir", s);
   OwnerParams p{world_size, shuffle_id_offset, rank, node_beg, node_end};
-  APT_FOLLOW(k_src_to_vir, wave_grid(ceil_div(num_src, 256), 8), 256, 0, s, nullptr, num_dst, src, num_src,
+  APT_FOLLOW(k_src_to_vir, wave_grid(ceil_div(num_src, 256), 8, 1), 256, 0, s, nullptr, num_dst, src, num_src,
              fanout, min_vids, p, 0, out_vir);
   return APT_OK;
 }
@@ -170,7 +170,7 @@ extern "C" int apt_srcdst_to_vir(const int64_t* dst, int64_t num_dst, const int6
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("src_to_vir", s);
   OwnerParams p{world_size, shuffle_id_offset, rank, node_beg, node_end};
-  APT_FOLLOW(k_src_to_vir, wave_grid(ceil_div(num_src + num_dst, 256), 8), 256, 0, s, dst, num_dst, src,
+  APT_FOLLOW(k_src_to_vir, wave_grid(ceil_div(num_src + num_dst, 256), 8, 1), 256, 0, s, dst, num_dst, src,
              num_src, fanout, min_vids, p, 1, out_vir);
   return APT_OK;
 }
@@ -208,7 +208,7 @@ extern "C" int apt_sp_pack_frontier(const int64_t* sorted_vir, const int64_t* so
   APT_CHECK_ARG(sorted_vir && sorted_ids && out && num_dst > 0, "apt_sp_pack_frontier: null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("sp_pack", s);
-  APT_FOLLOW(k_sp_pack, wave_grid(ceil_div(n, 256), 8), 256, 0, s, sorted_vir, sorted_ids, n, num_dst,
+  APT_FOLLOW(k_sp_pack, wave_grid(ceil_div(n, 256), 8, 1), 256, 0, s, sorted_vir, sorted_ids, n, num_dst,
              (int64_t)rank * sp_base * num_total_nodes, num_total_nodes, out);
   return APT_OK;
 }
@@ -222,7 +222,7 @@ extern "C" int apt_sp_unpack_frontier(const int64_t* packed, int64_t n, const in
   APT_CHECK_ARG(packed && out_vir && out_ori, "apt_sp_unpack_frontier: null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope prof("sp_unpack", s);
-  APT_FOLLOW(k_sp_unpack, wave_grid(ceil_div(n, 256), 8), 256, 0, s, packed, n, n_dev, num_total_nodes, out_vir,
+  APT_FOLLOW(k_sp_unpack, wave_grid(ceil_div(n, 256), 8, 1), 256, 0, s, packed, n, n_dev, num_total_nodes, out_vir,
              out_ori);
   return APT_OK;
 }
@@ -249,7 +249,7 @@ extern "C" int apt_sp_map_place_pack(const int64_t* neighbors, const int64_t* po
                 "apt_sp_map_place_pack: null pointer");
   ProfScope prof("sp_map_place_pack", s);
   OwnerParams p{world_size, shuffle_id_offset, rank, node_beg, node_end};
-  APT_FOLLOW(k_sp_map_place_pack, wave_grid(ceil_div(num_dst * fanout, 256), 8), 256, 0, s, neighbors, positions,
+  APT_FOLLOW(k_sp_map_place_pack, wave_grid(ceil_div(num_dst * fanout, 256), 8, 1), 256, 0, s, neighbors, positions,
              num_dst, num_dst_dev, fanout, min_vids, p, (int64_t)rank * sp_base * num_total_nodes, num_total_nodes,
              out_sorted_vir, out_packed, out_count);
   return APT_OK;
