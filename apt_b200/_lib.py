@@ -37,6 +37,8 @@ PROTOTYPES = {
     "apt_publish_words": (c_int, [P, c_int, P, c_int64, P, P]),
     "apt_publish_words_from": (c_int, [P, c_int, P, P, c_int64, P, P]),
     "apt_stage_replay": (c_int, [P, c_int64, P, c_int64, c_int64, P, P]),
+    "apt_publish_tagged": (c_int, [P, c_int, P, P, c_int64, P, P]),
+    "apt_wait_tagged": (c_int, [P, c_int, c_int64, P]),
     "apt_wait_published": (c_int, [P, c_int, c_int64, P]),
     "apt_pending_flags": (c_int, []),
     "apt_set_tunable": (c_int, [c_char_p, c_int64]),
@@ -62,6 +64,8 @@ PROTOTYPES = {
     "apt_gather_rows_beside": (c_int, [P, c_int64, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P, c_size_t, P, P]),
     "apt_gather_rows_from": (c_int, [P, c_int64, P, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P,
                                      c_size_t, P, P]),
+    "apt_gather_rows_publish": (c_int, [P, c_int64, P, P, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P,
+                                        P, c_int, P, P, c_int64, P, P]),
     "apt_gather_static_max_rows": (c_int64, []),
     "apt_gather_rows_static": (c_int, [P, c_int64, P, c_int64, P, c_int64, c_int64, P, c_int64, c_int64, c_int64, P, P, P]),
     "apt_spmm_workspace_bytes": (c_size_t, [c_int64, c_int64]),

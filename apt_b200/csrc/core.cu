@@ -80,6 +80,12 @@ k_publish_words(const int64_t* __restrict__ words, int count, const int64_t* __r
   if (threadIdx.x == 0) host[count] = sequence;
 }
 
+__global__ void __launch_bounds__(256)
+k_publish_tagged(const Tagged p) {
+  wait_for_previous();
+  publish_tagged(p);
+}
+
 // What a replay starts from, in one kernel in front of it: the seeds, the call-id base and the sequence number of its
 // counts. (A copy of the seeds, and one of the two words inside the graph, cost a launch more on the host and put a copy
 // engine between kernels twice.)
@@ -117,23 +123,44 @@ int apt_stage_replay(const int64_t* seeds, int64_t num_seeds, int64_t* seeds_buf
   return APT_OK;
 }
 
-int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream) {
-  APT_CHECK_ARG(host && count >= 0, "apt_wait_published: bad argument");
-  const volatile int64_t* word = host + count;
-  for (int64_t spin = 1; *word != sequence; ++spin) {
+int apt_publish_tagged(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev, int64_t sequence, int64_t* host,
+                       void* stream) {
+  using namespace apt;
+  APT_CHECK_ARG(words && last && host && count >= 1 && count <= 4096, "apt_publish_tagged: bad argument");
+  APT_FOLLOW(k_publish_tagged, 1, 256, 0, (cudaStream_t)stream, (Tagged{words, count, last, sequence_dev, sequence, host}));
+  return APT_OK;
+}
+
+static int wait_for_word(const volatile int64_t* word, int shift, int64_t sequence, void* stream) {
+  for (int64_t spin = 1; (int64_t)((uint64_t)*word >> shift) != sequence; ++spin) {
     if ((spin & 0x3fff) == 0) {
       // now and then the stream is asked, so that an error on it ends the wait
       apt::RelaxedCapture relaxed;
       const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
       if (e == cudaErrorNotReady) continue;
       APT_CUDA(e);
-      if (*word == sequence) break;
+      if ((int64_t)((uint64_t)*word >> shift) == sequence) break;
       apt::set_error("apt_wait_published: the stream is idle and the words have not arrived");
       return APT_ERR_TIMEOUT;
     }
 #if defined(__x86_64__)
     __builtin_ia32_pause();
 #endif
+  }
+  return APT_OK;
+}
+
+int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream) {
+  APT_CHECK_ARG(host && count >= 0, "apt_wait_published: bad argument");
+  return wait_for_word(host + count, 0, sequence, stream);
+}
+
+int apt_wait_tagged(int64_t* host, int count, int64_t sequence, void* stream) {
+  APT_CHECK_ARG(host && count >= 1, "apt_wait_tagged: bad argument");
+  for (int t = count - 1; t >= 0; --t) {
+    const int rc = wait_for_word(host + t, 32, sequence & 0xffffffffll, stream);
+    if (rc != APT_OK) return rc;
+    host[t] = (int32_t)host[t];
   }
   return APT_OK;
 }

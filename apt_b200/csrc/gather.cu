@@ -113,8 +113,10 @@ __global__ void __launch_bounds__(kGatherBlock)
 k_gather(const int64_t* __restrict__ index, int64_t n, const int64_t* __restrict__ n_dev, const int64_t* __restrict__ first_dev,
          const int64_t* __restrict__ pos_map, int64_t num_nodes, const char* __restrict__ dev_feats, int64_t num_dev_rows,
          const char* __restrict__ uva_feats, int64_t num_uva_rows, int64_t uva_row_bytes, int64_t col_offset_bytes,
-         int64_t row_bytes, int rows_per_chunk, int lpr, char* __restrict__ out, int32_t* status) {
+         int64_t row_bytes, int rows_per_chunk, int lpr, char* __restrict__ out, int32_t* status, const Tagged counts) {
   wait_for_previous();
+  // the counts of a mini-batch leave with its rows: as a kernel in front they held the rows up for 4 us
+  if (counts.host && blockIdx.x == 0) publish_tagged(counts);
   n = effective_n(n, n_dev);
   const int64_t first = first_row(first_dev, n);
   const int lane = threadIdx.x & 31;
@@ -177,6 +179,7 @@ struct GatherArgs {
   int64_t num_uva_rows, uva_row_bytes, uva_col_offset_bytes;
   char* out;
   int32_t* status_word;
+  Tagged counts;
 };
 
 // Blocks an SM for a gather that runs beside other kernels: enough reads over the host link for its full rate (one block's
@@ -202,7 +205,7 @@ static int gather_launch(const GatherArgs& a, cudaStream_t s, bool narrow = fals
 #define APT_GATHER(V)                                                                                                     \
   APT_FOLLOW(k_gather<V>, grid, kGatherBlock, 0, s, a.index, a.num_rows, a.num_rows_dev, a.first_row_dev, a.feat_pos_map, \
              a.num_nodes, a.dev_feats, a.num_dev_rows, a.uva_feats, a.num_uva_rows, a.uva_row_bytes,                      \
-             a.uva_col_offset_bytes, a.dev_row_bytes, per, lpr, a.out, a.status_word)
+             a.uva_col_offset_bytes, a.dev_row_bytes, per, lpr, a.out, a.status_word, a.counts)
   switch (width) {
     case 16: APT_GATHER(uint4); break;
     case 8: APT_GATHER(uint2); break;
@@ -281,7 +284,7 @@ extern "C" int apt_gather_rows_from(const int64_t* index, int64_t num_rows,
   using namespace apt;
   const GatherArgs a{index, num_rows, num_rows_dev, first_row_dev, feat_pos_map, num_nodes, (const char*)dev_feats,
                      num_dev_rows, dev_row_bytes, (const char*)uva_feats, num_uva_rows, uva_row_bytes,
-                     uva_col_offset_bytes, (char*)out, status_word};
+                     uva_col_offset_bytes, (char*)out, status_word, Tagged{}};
   const int rc = gather_check("apt_gather_rows", a);
   if (rc != APT_OK || num_rows == 0) return rc;
   APT_CHECK_ARG(workspace && ((uintptr_t)workspace & 255) == 0,
@@ -290,6 +293,22 @@ extern "C" int apt_gather_rows_from(const int64_t* index, int64_t num_rows,
     set_error("apt_gather_rows: workspace %zu < %zu bytes", workspace_bytes, apt_gather_workspace_bytes(num_rows));
     return APT_ERR_CAPACITY;
   }
+  return gather_launch(a, (cudaStream_t)stream);
+}
+
+extern "C" int apt_gather_rows_publish(const int64_t* index, int64_t num_rows, const int64_t* num_rows_dev, const int64_t* first_row_dev,
+                                       const int64_t* feat_pos_map, int64_t num_nodes, const void* dev_feats, int64_t num_dev_rows,
+                                       int64_t dev_row_bytes, const void* uva_feats, int64_t num_uva_rows, int64_t uva_row_bytes,
+                                       int64_t uva_col_offset_bytes, void* out, int32_t* status_word, const int64_t* words, int count,
+                                       const int64_t* last, const int64_t* sequence_dev, int64_t sequence, int64_t* host, void* stream) {
+  using namespace apt;
+  APT_CHECK_ARG(words && last && host && count >= 1 && count <= 4096, "apt_gather_rows_publish: bad argument");
+  const GatherArgs a{index, num_rows, num_rows_dev, first_row_dev, feat_pos_map, num_nodes, (const char*)dev_feats,
+                     num_dev_rows, dev_row_bytes, (const char*)uva_feats, num_uva_rows, uva_row_bytes,
+                     uva_col_offset_bytes, (char*)out, status_word, Tagged{words, count, last, sequence_dev, sequence, host}};
+  const int rc = gather_check("apt_gather_rows_publish", a);
+  if (rc != APT_OK) return rc;
+  if (num_rows == 0) return apt_publish_tagged(words, count, last, sequence_dev, sequence, host, stream);
   return gather_launch(a, (cudaStream_t)stream);
 }
 
@@ -303,7 +322,7 @@ extern "C" int apt_gather_rows_beside(const int64_t* index, int64_t num_rows,
   using namespace apt;
   const GatherArgs a{index, num_rows, num_rows_dev, nullptr, feat_pos_map, num_nodes, (const char*)dev_feats,
                      num_dev_rows, dev_row_bytes, (const char*)uva_feats, num_uva_rows, uva_row_bytes,
-                     uva_col_offset_bytes, (char*)out, status_word};
+                     uva_col_offset_bytes, (char*)out, status_word, Tagged{}};
   const int rc = gather_check("apt_gather_rows", a);
   if (rc != APT_OK || num_rows == 0) return rc;
   APT_CHECK_ARG(workspace && ((uintptr_t)workspace & 255) == 0,
@@ -340,7 +359,7 @@ extern "C" int apt_gather_rows_static(const int64_t* index, int64_t num_rows,
   }
   const GatherArgs a{index, num_rows, nullptr, nullptr, feat_pos_map, num_nodes, (const char*)dev_feats,
                      num_dev_rows, dev_row_bytes, (const char*)uva_feats, num_uva_rows, uva_row_bytes,
-                     uva_col_offset_bytes, (char*)out, status_word};
+                     uva_col_offset_bytes, (char*)out, status_word, Tagged{}};
   const int rc = gather_check("apt_gather_rows_static", a);
   if (rc != APT_OK || num_rows == 0) return rc;
   return gather_launch(a, (cudaStream_t)stream);

@@ -297,16 +297,16 @@ int64_t read_words(const Tensor& words, const Tensor& status, const Tensor& host
   void* const s = stream();
   int64_t* const h = host.mutable_data_ptr<int64_t>();
   py::gil_scoped_release nogil;
-  check(apt_publish_words_from(words.const_data_ptr<int64_t>(), count, status.const_data_ptr<int64_t>() + status.numel() - 1, nullptr,
-                               sequence, h, s));
-  check(apt_wait_published(h, count, sequence, s));
+  check(apt_publish_tagged(words.const_data_ptr<int64_t>(), count, status.const_data_ptr<int64_t>() + status.numel() - 1, nullptr, sequence,
+                           h, s));
+  check(apt_wait_tagged(h, count, sequence, s));
   return (h[count - 1] & 0xffffffff) | apt_pending_flags();
 }
 
 // One captured mini-batch: launches its graph, waits for its counts, orders other streams behind its last kernel.
 class Plan {
  public:
-  // replay_in: device words [call-id base, sequence]; host_words: page-locked, count words and the sequence; own_stream:
+  // replay_in: device words [call-id base, sequence]; host_words: page-locked, count words (apt_publish_tagged); own_stream:
   // 0 for the caller's current stream.
   Plan(uintptr_t exec, Tensor seeds_buf, Tensor replay_in, Tensor host_words, uintptr_t own_stream)
       : exec_((cudaGraphExec_t)exec), seeds_buf_(std::move(seeds_buf)), replay_in_(std::move(replay_in)),
@@ -352,10 +352,10 @@ class Plan {
   }
   // Until the counts of the last launch are in host_words; returns the status flags.
   int64_t wait() {
-    const int count = (int)host_words_.numel() - 1;
-    const int64_t* const h = host_words_.const_data_ptr<int64_t>();
+    const int count = (int)host_words_.numel();
+    int64_t* const h = host_words_.mutable_data_ptr<int64_t>();
     py::gil_scoped_release nogil;
-    check(apt_wait_published(h, count, sequence_, stream_));
+    if (!waited_) check(apt_wait_tagged(h, count, sequence_, stream_));      // (which takes the tags off)
     waited_ = true;
     return (h[count - 1] & 0xffffffff) | apt_pending_flags();
   }
@@ -579,11 +579,11 @@ py::tuple dp_sample(const Tensor& seeds, const std::vector<int64_t>& fanouts, co
     cur = uniq;
     layers.append(py::make_tuple(rel, uniq, col, f, (int64_t)k));
   }
-  check(apt_publish_words(word, count, nullptr, sequence, h, s));
+  check(apt_publish_tagged(word, count, word + count - 1, nullptr, sequence, h, s));
   Hops hops(layers, block);
   {
     py::gil_scoped_release nogil;
-    check(apt_wait_published(h, count, sequence, s));
+    check(apt_wait_tagged(h, count, sequence, s));
   }
   const int64_t num_in = h[fanouts.size() - 1], flags = (h[count - 1] & 0xffffffff) | apt_pending_flags();
   py::object rows = py::none(), pending = py::none();

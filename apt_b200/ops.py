@@ -213,11 +213,11 @@ class NPCState:
         return words
 
     def host_words(self) -> torch.Tensor:
-        """The calling thread's page-locked copy of a word block, with a sequence number behind it. Threads that read at the
+        """The calling thread's page-locked copy of a word block, with a sequence number in its words. Threads that read at the
         same time have one each: a reader polls its copy for its own number."""
         host = getattr(self._tls, "host", None)
         if host is None:
-            host = self._tls.host = _native.pinned_words(self.NUM_WORDS + 1)
+            host = self._tls.host = _native.pinned_words(self.NUM_WORDS)
         return host
 
     def word(self, k: int) -> torch.Tensor:
@@ -843,15 +843,24 @@ def load_subtensor(node_id: torch.Tensor) -> torch.Tensor:
 
 
 def _gather_enqueue(node_id: torch.Tensor, n_dev: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
-                    first_dev: Optional[torch.Tensor] = None, ws_name: str = "gather", beside: bool = False) -> torch.Tensor:
+                    first_dev: Optional[torch.Tensor] = None, ws_name: str = "gather", beside: bool = False,
+                    publish=None) -> torch.Tensor:
     """Enqueues the gather of rows [first_dev, n_dev) of node_id (device words; None: 0 and
     node_id.numel()) into `out` (allocated here when None). Calls that may overlap on the GPU
-    need workspaces of their own (`ws_name`). `beside`: on a few blocks, beside other kernels."""
+    need workspaces of their own (`ws_name`). `beside`: on a few blocks, beside other kernels. `publish`: the
+    arguments of apt_publish_tagged but for the stream; the words leave beside the rows."""
     f = STATE.feat
     n = node_id.numel()
     esz = f.dev_feats.element_size()
     if out is None:
         out = torch.empty((n, f.rank_feat_dim), dtype=f.dev_feats.dtype, device=node_id.device)
+    if publish is not None:
+        check(lib.apt_gather_rows_publish(
+            _ptr(node_id), n, _ptr(n_dev), _ptr(first_dev), _ptr(f.feat_pos_map), f.num_total_nodes,
+            _ptr(f.dev_feats), f.dev_feats.shape[0], f.rank_feat_dim * esz,
+            _ptr(f.uva_feats), f.uva_feats.shape[0], f.feat_dim * esz, f.feat_dim_offset * esz,
+            _ptr(out), STATE.status_ptr(), *publish, _stream()))
+        return out
     nbytes = lib.apt_gather_workspace_bytes(n)
     ws = STATE.workspace(ws_name, nbytes)
     launch, counts = (lib.apt_gather_rows_beside, (_ptr(n_dev),)) if beside else \

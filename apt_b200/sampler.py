@@ -93,7 +93,7 @@ class _Plan:
         self.graph = None
         self.generation = -1
         self.keepalive = None
-        # The batch's own counts, on the device and, a sequence number behind them, on the host: the gather of its rows still
+        # The batch's own counts, on the device and, the sequence number of the replay in them until it is waited for, on the host: the gather of its rows still
         # reads them when the mini-batch has been handed out and another one, on another stream, writes its own.
         self.words = None
         self.host_words = None
@@ -107,6 +107,22 @@ class _Plan:
     def __del__(self):
         if self.handle is not None:
             self.handle.finish()     # the last launch may still be running: its graph and buffers go only then
+
+
+class _Publish:
+    """Sends a plan's word block to the host once: as a kernel of its own (called), or with the gather of the rows, which then
+    do not wait for it (`taken()`: the arguments for that)."""
+
+    def __init__(self, *args):
+        self.args = args
+        self.done = False
+
+    def taken(self):
+        self.done = True
+        return self.args
+
+    def __call__(self):
+        check(lib.apt_publish_tagged(*self.taken(), ops._stream()))
 
 
 _CALL_BASE_SLOT = 100  # device words holding the call-id base and the sequence number of a graph replay
@@ -124,8 +140,8 @@ class _Ring:
 class _GraphReplay:
     """What the chained samplers share: the whole mini-batch is enqueued by `_enqueue(seeds, base_dev, publish)`
     without a host read, its result outlined by `_outline(seeds, bufs)` and narrowed by `_finish(seeds, bufs, host)` after one look at the device word
-    block, which `publish()` sends to the host as soon as it is complete (a gather of the rows goes behind it
-    and runs on while the host narrows); the enqueue is captured once per batch shape as a CUDA graph and replayed, from
+    block, which `publish` sends to the host as soon as it is complete (in front of the rows of the gather, which
+    runs on while the host narrows); the enqueue is captured once per batch shape as a CUDA graph and replayed, from
     `graph_buffers` buffer sets in turn. `sample_iter` launches mini-batch k + 1 before it reads
     mini-batch k back. Subclasses set `num_calls` (sampling calls per mini-batch).
 
@@ -182,11 +198,12 @@ class _GraphReplay:
             ops._gather_enqueue(cur, cur_n, out=rows, ws_name="gather_frontier", beside=True)
         return rows
 
-    def _late_rows(self, input_nodes, in_word, cur_n, rows):
+    def _late_rows(self, input_nodes, in_word, cur_n, rows, publish):
         """The rows of the input nodes, those behind the first cur_n when `rows` holds these already."""
+        publish = publish and publish.taken()
         if rows is None:
-            return ops._gather_enqueue(input_nodes, in_word)
-        ops._gather_enqueue(input_nodes, in_word, out=rows, first_dev=cur_n)
+            return ops._gather_enqueue(input_nodes, in_word, publish=publish)
+        ops._gather_enqueue(input_nodes, in_word, out=rows, first_dev=cur_n, publish=publish)
         ops.STATE.join(2)
         return rows
 
@@ -225,7 +242,7 @@ class _GraphReplay:
         plan.seeds_buf = torch.empty(seeds.numel(), dtype=torch.int64, device=dev)
         plan.seeds_buf.copy_(seeds)
         plan.words = torch.zeros(st.NUM_WORDS, dtype=torch.int64, device=dev)
-        plan.host_words = torch.zeros(st.NUM_WORDS + 1, dtype=torch.int64).pin_memory()
+        plan.host_words = torch.zeros(st.NUM_WORDS, dtype=torch.int64).pin_memory()
         if on_lanes:
             # lane 0 stays with the caller: its exchange context also carries the feature shuffles
             # the model side runs on its own stream while the samplers' lanes are in flight
@@ -266,16 +283,10 @@ class _GraphReplay:
         del bufs
         plan.graph = torch.cuda.CUDAGraph()
         replay_in = plan.words[_CALL_BASE_SLOT:_CALL_BASE_SLOT + 2]
-        published = []
-
-        def publish():
-            published.append(True)
-            check(lib.apt_publish_words_from(ops._ptr(plan.words), st.NUM_WORDS, st.status_ptr(), ops._ptr(replay_in[1:2]), 0,
-                                             ops._ptr(plan.host_words), ops._stream()))
-
+        publish = _Publish(ops._ptr(plan.words), st.NUM_WORDS, st.status_ptr(), ops._ptr(replay_in[1:2]), 0, ops._ptr(plan.host_words))
         with torch.cuda.graph(plan.graph):
             plan.bufs = self._enqueue(plan.seeds_buf, base_dev, publish)
-            if not published:
+            if not publish.done:
                 publish()
         plan.handle = _native.Plan(plan.graph.raw_cuda_graph_exec(), plan.seeds_buf, replay_in, plan.host_words,
                                    plan.stream.cuda_stream if on_lanes else 0)
@@ -515,12 +526,13 @@ class MixedNeighborSampler(_GraphReplay):
                 ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier", beside=True)
         uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
                                                      call if explicit else None, call_base_dev, look_up=prefetch)
-        if publish is not None:
-            publish()
         if split == 1:
+            if publish is not None:
+                publish()
             st.join(2)
         if prefetch:
-            ops._gather_enqueue(uniq3, st.word(in_slot), out=rows, first_dev=st.word(u_slot) if split else None)
+            ops._gather_enqueue(uniq3, st.word(in_slot), out=rows, first_dev=st.word(u_slot) if split else None,
+                                publish=publish.taken() if publish is not None and not publish.done else None)
         if split == 2:
             st.join(2)
         return dict(layers=layers, perm=perm, inv=inv, rows=rows, u_slot=u_slot,
@@ -610,9 +622,7 @@ class SPGATSampler(_GraphReplay):
         in_word = st.word(self._IN)
         prefetch = self.prefetch_features and _fits_prefetch(cur.numel() + recv.numel())
         input_nodes = ops.concat_ids(cur, cur_n, recv, recv_counts[ws:ws + 1], in_word, look_up=prefetch)
-        if publish is not None:
-            publish()
-        rows = self._late_rows(input_nodes, in_word, cur_n, rows) if prefetch else None
+        rows = self._late_rows(input_nodes, in_word, cur_n, rows, publish) if prefetch else None
         return dict(layers=layers, outer=_layer(cur, arange_src, unique_neigh, f, self._U), perm=perm,
                     input_nodes=input_nodes, rows=rows)
 
@@ -812,9 +822,7 @@ class SPVirtualSampler(_GraphReplay):
         in_word = st.word(self._IN)
         prefetch = self.prefetch_features and _fits_prefetch(head.numel() + unique_src.numel())
         input_nodes = ops.concat_ids(head, head_n, unique_src, us_word, in_word, look_up=prefetch)
-        if publish is not None:
-            publish()
-        rows = self._late_rows(input_nodes, in_word, cur_n, rows) if prefetch else None
+        rows = self._late_rows(input_nodes, in_word, cur_n, rows, publish) if prefetch else None
         return dict(layers=layers, cur=cur, nbr=nbr, sorted_all=sorted_all, packed=packed,
                     unique_frontier=unique_frontier, arange_src=arange_src, arange_dst=arange_dst, vir_src=vir_src, ori_src=ori_src,
                     unique_src=unique_src, a_src=a_src, unique_dst=unique_dst, a_dst=a_dst, dst_sorted=dst_sorted,

@@ -82,6 +82,12 @@ int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_d
 /* The same with the last word taken from *last instead (counts of one block, status flags of another); NULL: from words. */
 int apt_publish_words_from(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev,
                            int64_t sequence, int64_t* host, void* stream);
+/* Words of 32-bit values, each with the lower half of the sequence number in its upper half, so that nothing has to be ordered
+ * behind anything on the way: apt_wait_tagged polls every one of the count words and leaves the plain values (signed; the
+ * sequence numbers of one host buffer differ and are not 0 or -1 in that half). The last word comes from *last. */
+int apt_publish_tagged(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev,
+                       int64_t sequence, int64_t* host, void* stream);
+int apt_wait_tagged(int64_t* host, int count, int64_t sequence, void* stream);
 int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream);
 /* Flags of kernels whose entry point has no status word (apt_spmm_*), of all devices: returns them and forgets them. A
  * kernel's flags are there when it is done; apt_spmm_probe and apt_spmm_sum refuse with APT_ERR_TIMEOUT while one waits. */
@@ -289,6 +295,16 @@ int apt_gather_rows(const int64_t* index, int64_t num_rows,
                     int64_t num_uva_rows, int64_t uva_row_bytes,
                     int64_t uva_col_offset_bytes, void* out, void* workspace,
                     size_t workspace_bytes, int32_t* status_word, void* stream);
+/* apt_gather_rows_from and apt_publish_tagged in one kernel: for counts that the host may have while the rows still travel. */
+int apt_gather_rows_publish(const int64_t* index, int64_t num_rows,
+                            const int64_t* num_rows_dev, const int64_t* first_row_dev,
+                            const int64_t* feat_pos_map, int64_t num_nodes,
+                            const void* dev_feats, int64_t num_dev_rows,
+                            int64_t dev_row_bytes, const void* uva_feats,
+                            int64_t num_uva_rows, int64_t uva_row_bytes,
+                            int64_t uva_col_offset_bytes, void* out, int32_t* status_word,
+                            const int64_t* words, int count, const int64_t* last,
+                            const int64_t* sequence_dev, int64_t sequence, int64_t* host, void* stream);
 /* The same on a few blocks, to run beside other kernels on another stream. */
 int apt_gather_rows_beside(const int64_t* index, int64_t num_rows,
                     const int64_t* num_rows_dev,

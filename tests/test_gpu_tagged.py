@@ -1,0 +1,57 @@
+"""Word blocks that reach the host with a sequence number in every word, by themselves and beside the rows of a gather."""
+import ctypes
+
+import pytest
+import torch
+
+from apt_b200 import _lib
+from apt_b200._lib import check, lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _blocks(count):
+    words = torch.arange(count, dtype=torch.int64, device="cuda") * 7
+    words[0], words[count // 2] = -1, 2 ** 31 - 1
+    last = torch.tensor([0x11], device="cuda")
+    want = words.tolist()
+    want[-1] = 0x11
+    return words, last, want, torch.zeros(count, dtype=torch.int64).pin_memory()
+
+
+@pytest.mark.parametrize("count", [1, 31, 256, 300])
+def test_words_arrive_with_their_sequence(count):
+    words, last, want, host = _blocks(count)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for seq in (1, 2, 2 ** 32 + 3):      # the lower half counts
+        check(lib.apt_publish_tagged(_ptr(words), count, _ptr(last), None, seq, _ptr(host), stream))
+        check(lib.apt_wait_tagged(_ptr(host), count, seq, stream))
+        assert host.tolist() == want
+    seq_dev = torch.tensor([9], device="cuda")
+    check(lib.apt_publish_tagged(_ptr(words), count, _ptr(last), _ptr(seq_dev), 0, _ptr(host), stream))
+    check(lib.apt_wait_tagged(_ptr(host), count, 9, stream))
+    assert host.tolist() == want
+    # an idle stream without an answer ends the wait
+    assert lib.apt_wait_tagged(_ptr(host), count, 10, stream) == _lib.APT_ERR_TIMEOUT
+
+
+@pytest.mark.parametrize("rows,first", [(0, 0), (1, 0), (1203, 0), (1203, 1000), (40_000, 7)])
+def test_words_beside_the_rows_of_a_gather(rows, first):
+    count = 256
+    words, last, want, host = _blocks(count)
+    nodes, dim = 50_000, 36
+    feats = torch.arange(nodes * dim, dtype=torch.float32, device="cuda").view(nodes, dim)
+    pos = torch.arange(nodes, device="cuda")
+    ids = torch.randperm(nodes, device="cuda")[:max(rows, 1)]
+    out = torch.full((max(rows, 1), dim), -5.0, device="cuda")
+    first_dev, status = torch.tensor([first], device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    check(lib.apt_gather_rows_publish(_ptr(ids), rows, None, _ptr(first_dev), _ptr(pos), nodes, _ptr(feats), nodes, dim * 4, None, 0, dim * 4, 0,
+                                      _ptr(out), _ptr(status), _ptr(words), count, _ptr(last), None, 5, _ptr(host), stream))
+    check(lib.apt_wait_tagged(_ptr(host), count, 5, stream))
+    assert host.tolist() == want and int(status) == 0
+    assert torch.equal(out[first:rows], feats[ids[first:rows]]) and bool((out[:min(first, rows)] == -5).all())
