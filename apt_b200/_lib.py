@@ -37,6 +37,7 @@ PROTOTYPES = {
     "apt_publish_words": (c_int, [P, c_int, P, c_int64, P, P]),
     "apt_publish_words_from": (c_int, [P, c_int, P, P, c_int64, P, P]),
     "apt_stage_replay": (c_int, [P, c_int64, P, c_int64, c_int64, P, P]),
+    "apt_copy_words": (c_int, [P, P, P, c_int, P]),
     "apt_publish_tagged": (c_int, [P, c_int, P, P, c_int64, P, P]),
     "apt_wait_tagged": (c_int, [P, c_int, c_int64, P]),
     "apt_wait_published": (c_int, [P, c_int, c_int64, P]),

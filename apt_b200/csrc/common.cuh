@@ -55,6 +55,9 @@ struct ProfScope {
     }                                                                         \
   } while (0)
 
+inline dim3 as_grid(int64_t blocks) { return dim3((unsigned)blocks); }
+inline dim3 as_grid(dim3 grid) { return grid; }
+
 // The same for a kernel that opens with wait_for_previous(): its launch overlaps the end of the kernel before it on the
 // stream (programmatic dependent launch), in captured graphs too. Chains of kernels of a few microseconds are what this
 // framework's mini-batches consist of: three edge operators over 61 310 edges 38 -> 31 us, a data-parallel batch 151 -> 135.
@@ -64,7 +67,7 @@ struct ProfScope {
     attr__.id = cudaLaunchAttributeProgrammaticStreamSerialization;           \
     attr__.val.programmaticStreamSerializationAllowed = 1;                    \
     cudaLaunchConfig_t cfg__ = {};                                            \
-    cfg__.gridDim = dim3((unsigned)(grid_));                                  \
+    cfg__.gridDim = as_grid(grid_);                                  \
     cfg__.blockDim = dim3((unsigned)(block_));                                \
     cfg__.dynamicSmemBytes = (smem_);                                         \
     cfg__.stream = (stream_);                                                 \

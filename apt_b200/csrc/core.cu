@@ -86,6 +86,31 @@ k_publish_tagged(const Tagged p) {
   publish_tagged(p);
 }
 
+// Several arrays of words to places of their own: the tensors of a mini-batch that leave buffers much longer than they are, in
+// one launch (a clone each is an operator call and a copy).
+constexpr int kCopyParts = 24;
+struct WordCopies {
+  const int64_t* src[kCopyParts];
+  int64_t* dst[kCopyParts];
+  int64_t count[kCopyParts];
+};
+__global__ void __launch_bounds__(256)
+k_copy_words(const __grid_constant__ WordCopies c) {
+  wait_for_previous();
+  constexpr int K = 4;
+  const int64_t* const src = c.src[blockIdx.y];
+  int64_t* const dst = c.dst[blockIdx.y];
+  const int64_t n = c.count[blockIdx.y], stride = (int64_t)gridDim.x * 256;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += K * stride) {
+    int64_t v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = i + k * stride < n ? src[i + k * stride] : 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (i + k * stride < n) dst[i + k * stride] = v[k];
+  }
+}
+
 // What a replay starts from, in one kernel in front of it: the seeds, the call-id base and the sequence number of its
 // counts. (A copy of the seeds, and one of the two words inside the graph, cost a launch more on the host and put a copy
 // engine between kernels twice.)
@@ -111,6 +136,25 @@ int apt_publish_words_from(const int64_t* words, int count, const int64_t* last,
   using namespace apt;
   APT_CHECK_ARG(words && host && count >= 0 && count <= 4096, "apt_publish_words: bad argument");
   APT_FOLLOW(k_publish_words, 1, 256, 0, (cudaStream_t)stream, words, count, last, sequence_dev, sequence, host);
+  return APT_OK;
+}
+
+int apt_copy_words(const int64_t* const* src, int64_t* const* dst, const int64_t* counts, int num, void* stream) {
+  using namespace apt;
+  APT_CHECK_ARG(num >= 0 && (num == 0 || (src && dst && counts)), "apt_copy_words: bad argument");
+  for (int k0 = 0; k0 < num; k0 += kCopyParts) {
+    WordCopies c{};
+    const int parts = num - k0 < kCopyParts ? num - k0 : kCopyParts;
+    int64_t most = 0;
+    for (int k = 0; k < parts; ++k) {
+      c.src[k] = src[k0 + k], c.dst[k] = dst[k0 + k], c.count[k] = counts[k0 + k];
+      APT_CHECK_ARG(c.count[k] >= 0 && (c.count[k] == 0 || (c.src[k] && c.dst[k])), "apt_copy_words: bad part");
+      if (c.count[k] > most) most = c.count[k];
+    }
+    if (most == 0) continue;
+    const int64_t want = ceil_div(most, 1024), fit = (int64_t)kNumSMs * 8 / parts;
+    APT_FOLLOW(k_copy_words, dim3((unsigned)(want < fit ? want : fit), (unsigned)parts), 256, 0, (cudaStream_t)stream, c);
+  }
   return APT_OK;
 }
 

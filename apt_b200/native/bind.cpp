@@ -435,12 +435,22 @@ class Hops {
   // Tensors much longer than their views (hops that meet the same nodes again and again) are replaced by copies of the views:
   // a caller that keeps its mini-batches keeps what they consist of, within a factor of two.
   void compact() {
+    std::vector<const int64_t*> src;
+    std::vector<int64_t*> dst;
+    std::vector<int64_t> counts;
     for (Hop& h : hops_)
       for (const auto& [name, t] : {std::pair<const char*, Tensor*>{"coo_row", &h.rows}, {"coo_col", &h.cols}, {"src_ids", &h.ids}}) {
         if ((int64_t)t->storage().nbytes() <= 2 * (int64_t)t->nbytes() + kSlackBytes) continue;
-        *t = t->clone();
+        Tensor own = at::empty(t->sizes(), t->options());
+        src.push_back(t->const_data_ptr<int64_t>());
+        dst.push_back(own.mutable_data_ptr<int64_t>());
+        counts.push_back(own.numel());
+        left_.push_back(std::move(*t));      // until the copy is enqueued
+        *t = std::move(own);
         h.block.attr(name) = *t;
       }
+    check(apt_copy_words(src.data(), dst.data(), counts.data(), (int)src.size(), stream()));
+    left_.clear();
   }
   py::list blocks;
 
@@ -452,6 +462,7 @@ class Hops {
     int64_t fanout, slot;
   };
   std::vector<Hop> hops_;
+  std::vector<Tensor> left_;
 };
 
 // What sample() of a chained sampler returns, (input nodes, seeds, blocks, permutation, ids received per peer, bucket

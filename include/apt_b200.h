@@ -72,6 +72,9 @@ void apt_launch_count_reset(void);
  * its sizes with blocking copies (src/sampling.cc:176-185). */
 int apt_memcpy_async(void* dst, const void* src, size_t nbytes, void* stream);
 
+/* num arrays of 8-byte words, counts[k] of them from src[k] to dst[k], in one kernel (a few, beyond 24 arrays). */
+int apt_copy_words(const int64_t* const* src, int64_t* const* dst, const int64_t* counts, int num, void* stream);
+
 /* Small results for the host without a copy and an event: a kernel on `stream` stores
  * count words into page-locked host memory and then, behind them, a sequence number
  * (*sequence_dev when given: a word that a captured graph's replay brings along);

@@ -1,4 +1,5 @@
-"""Word blocks that reach the host with a sequence number in every word, by themselves and beside the rows of a gather."""
+"""Word blocks that reach the host with a sequence number in every word, by themselves and beside the rows of a gather, and
+arrays of words copied together."""
 import ctypes
 
 import pytest
@@ -55,3 +56,15 @@ def test_words_beside_the_rows_of_a_gather(rows, first):
     check(lib.apt_wait_tagged(_ptr(host), count, 5, stream))
     assert host.tolist() == want and int(status) == 0
     assert torch.equal(out[first:rows], feats[ids[first:rows]]) and bool((out[:min(first, rows)] == -5).all())
+
+
+@pytest.mark.parametrize("counts", [[0], [1], [0, 5, 1023, 1024, 1025], [70_001] * 3, list(range(30))])
+def test_arrays_copied_in_one_call(counts):
+    src = [torch.arange(n + 1, dtype=torch.int64, device="cuda") * 3 + k for k, n in enumerate(counts)]
+    dst = [torch.full((n + 1,), -9, dtype=torch.int64, device="cuda") for n in counts]
+    pointers = ctypes.c_void_p * len(counts)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    check(lib.apt_copy_words(pointers(*(t.data_ptr() for t in src)), pointers(*(t.data_ptr() for t in dst)),
+                             (ctypes.c_int64 * len(counts))(*counts), len(counts), stream))
+    for n, a, b in zip(counts, src, dst):
+        assert torch.equal(a[:n], b[:n]) and int(b[n]) == -9
