@@ -11,7 +11,8 @@
 // kernels and are kept apart, with fp32 weights per edge and head between them (16 MB for a million edges of four
 // heads, which stay in L2):
 //
-//   k_gat_ranges    where each destination's edges are
+//   k_gat_ranges    where each destination's edges are (6.5 us with one edge a thread; a word that every kernel looks at had
+//                   to be cleared in front, a launch more: attention of 30 000 x 15 edges, bf16 4 x 64, 41.5 -> 38.3 us forward)
 //   k_gat_weights   scores and softmax, a few lanes per destination, two edges a lane, four heads at a time; any number of
 //                   edges and heads.
 //   row kernel      the weighted sum is the SpMM's row kernel (kUMulW), any head width
@@ -61,33 +62,46 @@ __device__ __forceinline__ float group_sum(float v, int n) {
   return v;
 }
 
-// First and last edge of every destination; *none when the edges are not grouped (nothing then belongs to anybody).
+// First and last edge of every destination; a block's verdict is set when its edges are not grouped (nothing then belongs to
+// anybody). Four edges a thread are in flight, on four blocks an SM at most.
 __global__ void __launch_bounds__(256)
-k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* __restrict__ range, int32_t* none, int32_t* status) {
+k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* __restrict__ range, uint32_t* __restrict__ verdict,
+             int32_t* status) {
   wait_for_previous();
+  constexpr int K = 4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   bool bad = false;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
-    const int64_t d = col[e];
-    const int64_t prev = e > 0 ? col[e - 1] : (int64_t)-1;
-    if (d < prev || d < 0 || d >= num_dst) {
-      bad = true;
-      continue;
+  for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e0 < E; e0 += K * stride) {
+    int64_t at[K], before[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int64_t e = e0 + k * stride;
+      at[k] = e < E ? col[e] : 0;
+      before[k] = e < E && e > 0 ? col[e - 1] : (int64_t)-1;
     }
-    if (d != prev) {
-      if (prev >= 0) range[prev].y = (int)e;
-      for (int64_t t = prev + 1; t < d; ++t) range[t] = make_int2(0, 0);
-      range[d].x = (int)e;
-    }
-    if (e == E - 1) {
-      range[d].y = (int)E;
-      for (int64_t t = d + 1; t < num_dst; ++t) range[t] = make_int2(0, 0);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int64_t e = e0 + k * stride, d = at[k], prev = before[k];
+      if (e >= E) break;
+      if (d < prev || d < 0 || d >= num_dst) {
+        bad = true;
+        continue;
+      }
+      if (d != prev) {
+        if (prev >= 0) range[prev].y = (int)e;
+        for (int64_t t = prev + 1; t < d; ++t) range[t] = make_int2(0, 0);
+        range[d].x = (int)e;
+      }
+      if (e == E - 1) {
+        range[d].y = (int)E;
+        for (int64_t t = d + 1; t < num_dst; ++t) range[t] = make_int2(0, 0);
+      }
     }
   }
-  if (bad) {
-    atomicOr(none, 1);
-    atomicOr(status, APT_FLAG_NOT_GROUPED);
-  }
+  const int any = __syncthreads_or(bad);
+  if (threadIdx.x != 0) return;
+  verdict[blockIdx.x] = (uint32_t)any;
+  if (any) atomicOr(status, APT_FLAG_NOT_GROUPED);
 }
 
 // W lanes to a destination, kGatEdges edges a lane, the edges of a round side by side: loads and stores of a value per edge are
@@ -126,11 +140,11 @@ __device__ __forceinline__ float lanes_sum(float v) {
 template <typename T, int W, int NH>
 __global__ void __launch_bounds__(256)
 k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
-              int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ weight,
+              int64_t num_dst, const int2* __restrict__ range, const Verdict none, float* __restrict__ weight,
               T* __restrict__ attn, int masked) {
   wait_for_previous();
   constexpr int K = kGatEdges;
-  if (*none != 0) return;
+  if (any_found(none)) return;
   const int64_t stride = (int64_t)gridDim.x * (256 / W);
   const int part = threadIdx.x & (W - 1);
   // (all lanes of a warp stay: groups behind the last destination have no edges)
@@ -232,10 +246,10 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
 template <typename T, int VE>
 __global__ void __launch_bounds__(256, 3)
 k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ grad_out, int num_heads, int head_dim,
-           int64_t num_dst_, const int2* __restrict__ range, const int32_t* __restrict__ none, float* __restrict__ dots, int lph,
+           int64_t num_dst_, const int2* __restrict__ range, const Verdict none, float* __restrict__ dots, int lph,
            int hpp, uint32_t num_src, int32_t* __restrict__ src_count, uint32_t* __restrict__ rank) {
   wait_for_previous();
-  if (*none != 0) return;
+  if (any_found(none)) return;
   const int lane = threadIdx.x & 31, G = gridDim.x * 8, num_dst = (int)num_dst_;
   const int lpe = lph * hpp, ep = 32 / lpe;
   const int epi = lane / lpe, rh = (lane & (lpe - 1)) / lph, p = lane & (lph - 1);
@@ -339,12 +353,12 @@ __device__ __forceinline__ void add_heads(float* p, const Heads<NH>& v) {
 template <typename T, int W, int NH>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
-             int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const int32_t* __restrict__ none,
+             int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const Verdict none,
              float* __restrict__ weight, const float* __restrict__ dots, float* __restrict__ sums, const SpmmWs sort, OrderKind kind,
              T* __restrict__ grad_er) {
   wait_for_previous();
   constexpr int K = kGatEdges;
-  const bool empty = *none != 0;
+  const bool empty = any_found(none);
   if (empty)   // no edge belongs to anybody
     for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += (int64_t)gridDim.x * blockDim.x) weight[o] = 0.f;
   const int64_t stride = (int64_t)gridDim.x * (256 / W);
@@ -443,9 +457,19 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_source(const float* __restrict__ sums, int64_t n, uint32_t num_heads, T* __restrict__ grad_el) {
   wait_for_previous();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t row = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)row * num_heads);
-    grad_el[i] = Elem<T>::from_f(sums[(int64_t)spread(row) * num_heads + h]);
+  constexpr int K = 4;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += K * stride) {
+    float v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int64_t i = i0 + k * stride;
+      const uint32_t row = (uint32_t)(i / num_heads), h = (uint32_t)(i - (int64_t)row * num_heads);
+      v[k] = i < n ? sums[(int64_t)spread(row) * num_heads + h] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (i0 + k * stride < n) grad_el[i0 + k * stride] = Elem<T>::from_f(v[k]);
   }
 }
 
@@ -454,15 +478,18 @@ static size_t elem_size(int dtype) { return dtype == APT_F32 ? 4 : 2; }
 
 // What the forward leaves for the backward: the ranges and the weights.
 struct GatEdges {
-  int32_t* none;    // [1]
+  Verdict none;     // [kVerdicts] words
   int2* range;      // [num_dst]
   float* weight;    // [E][heads]
 };
+constexpr size_t kGatFront = (kVerdicts * 4 + 255) / 256 * 256;
+// The blocks of k_gat_ranges.
+static int gat_range_blocks(int64_t E) { return (int)std::min<int64_t>(kVerdicts, ceil_div(E, 1024)); }
 static size_t gat_edges_layout(int64_t num_dst, int64_t E, int H, char* base, GatEdges* g) {
-  const size_t o_range = 256;
+  const size_t o_range = kGatFront;
   const size_t o_weight = o_range + align_up((size_t)(num_dst > 0 ? num_dst : 1) * 8, 256);
   if (g) {
-    g->none = (int32_t*)base;
+    g->none = Verdict{(const uint32_t*)base, gat_range_blocks(E)};
     g->range = (int2*)(base + o_range);
     g->weight = (float*)(base + o_weight);
   }
@@ -508,9 +535,8 @@ static int gat_check(const char* who, int dtype, int64_t num_edges, int num_head
 }
 
 static int gat_ranges(const GatProblem& q, const GatEdges& g, cudaStream_t s) {
-  APT_CUDA(cudaMemsetAsync(g.none, 0, 4, s));
   ProfScope prof("spmm_ranges", s);
-  APT_FOLLOW(k_gat_ranges, wave_grid(ceil_div(q.E, 256), 8), 256, 0, s, q.col, q.E, q.num_dst, g.range, g.none, q.status);
+  APT_FOLLOW(k_gat_ranges, gat_range_blocks(q.E), 256, 0, s, q.col, q.E, q.num_dst, g.range, (uint32_t*)g.none.word, q.status);
   return APT_OK;
 }
 
@@ -627,13 +653,13 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
 #undef APT_SCORES
   }
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, num_src, q.E, ws.sort,
-                     (T*)grad_ft, kOrder, 0, split, (int)dim, nullptr, q.status, nullptr, nullptr, nullptr, 0u};
+                     (T*)grad_ft, kOrder, 0, split, (int)dim, Verdict{}, q.status, nullptr, nullptr, nullptr, 0u};
   {
     ProfScope prof("spmm_rows", s);
     rc = launch_spmm_rows<T>(kUMulW, a, s);
   }
   if (rc != APT_OK) return rc;
-  APT_FOLLOW(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 256), 8), 256, 0, s, ws.sums, num_src * q.H, (uint32_t)q.H, (T*)grad_el);
+  APT_FOLLOW(k_gat_source<T>, wave_grid(ceil_div(num_src * q.H, 1024), 8, 1), 256, 0, s, ws.sums, num_src * q.H, (uint32_t)q.H, (T*)grad_el);
   return APT_OK;
 }
 
@@ -715,7 +741,7 @@ struct GatScores {
 template <typename T, int VE>
 __global__ void __launch_bounds__(256, 4)
 k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er, int num_heads,
-            int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none,
+            int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const Verdict none,
             T* __restrict__ out, T* __restrict__ attn, int lpe, int masked) {
   wait_for_previous();
   constexpr int U = 4;
@@ -724,7 +750,7 @@ k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* 
   const int nvh = head_dim / VE;
   const int64_t dim = (int64_t)num_heads * head_dim;
   const uint32_t row_bytes = (uint32_t)(dim * sizeof(T));
-  const bool empty = *none != 0;
+  const bool empty = any_found(none);
   for (int64_t d = (int64_t)blockIdx.x * 8 + warp; d < num_dst; d += (int64_t)gridDim.x * 8) {
     const int2 r = empty ? make_int2(0, 0) : range[d];
     const int deg = r.y - r.x;
@@ -774,15 +800,16 @@ k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* 
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_gat_narrow(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er, int num_heads,
-             int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const int32_t* __restrict__ none,
+             int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const Verdict none,
              T* __restrict__ out, T* __restrict__ attn, int lpe) {
   wait_for_previous();
   constexpr int VE = 16 / sizeof(T);
+  const bool empty = any_found(none);
   const int c = threadIdx.x & (lpe - 1), dim = num_heads * head_dim;
   if (c * VE >= dim) return;
   const int h = c * VE / head_dim;
   const uint32_t row_bytes = (uint32_t)(dim * sizeof(T));
-  const bool empty = *none != 0, writes_attn = attn && c * VE % head_dim == 0;
+  const bool writes_attn = attn && c * VE % head_dim == 0;
   const T* const lane_ft = ft + c * VE;
   const T* const lane_el = el + h;
   const int per_block = 256 / lpe;
@@ -814,7 +841,7 @@ template <typename T, int VE>
 __global__ void __launch_bounds__(256, 3)
 k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er,
                      const T* __restrict__ grad_out, int num_heads, int head_dim, float slope, int64_t num_dst, int64_t E,
-                     const int2* __restrict__ range, const int32_t* __restrict__ none, T* __restrict__ attn,
+                     const int2* __restrict__ range, const Verdict none, T* __restrict__ attn,
                      T* __restrict__ grad_score, T* __restrict__ grad_er, int lph, int hpp, int masked) {
   wait_for_previous();
   constexpr int U = 4;
@@ -825,7 +852,7 @@ k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, 
   const int nvh = head_dim / VE;
   const int64_t dim = (int64_t)num_heads * head_dim;
   const uint32_t row_bytes = (uint32_t)(dim * sizeof(T));
-  const bool empty = *none != 0;
+  const bool empty = any_found(none);
   if (empty)   // no edge belongs to anybody
     for (int64_t o = (int64_t)blockIdx.x * 256 + threadIdx.x; o < E * num_heads; o += (int64_t)gridDim.x * 256)
       attn[o] = grad_score[o] = Elem<T>::from_f(0.f);
@@ -933,7 +960,7 @@ static int launch_alone(const GatProblem& q, const GatEdges& g, void* out, void*
 // The ranges are in the front of a workspace of apt_spmm_workspace_bytes(num_dst, 0) bytes. Backward with grad_er, else forward.
 template <typename T>
 static int gat_alone(const GatProblem& q, void* workspace, void* out, void* attn, void* grad_score, void* grad_er, cudaStream_t s) {
-  const GatEdges g{(int32_t*)workspace, (int2*)((char*)workspace + 256), nullptr};
+  const GatEdges g{Verdict{(const uint32_t*)workspace, gat_range_blocks(q.E)}, (int2*)((char*)workspace + kGatFront), nullptr};
   const int rc = gat_ranges(q, g, s);
   if (rc != APT_OK) return rc;
   ProfScope prof(grad_er ? "gat_bwd_rows" : "gat_rows", s);

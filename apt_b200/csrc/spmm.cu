@@ -90,7 +90,7 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
   if (!agg) agg = g_probe_votes + slot;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   __shared__ uint32_t s_bits;
-  constexpr int K = 4;
+  constexpr int K = 8;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, c[K];
   auto fetch = [&]() {
@@ -486,7 +486,7 @@ static int run_rows(int op, const RowSplit& split, const int64_t* row, const int
                     int64_t edata_dim, int64_t feat_dim, SegTable st, int64_t num_rows, const SpmmWs& ws, int mode, int fixed,
                     void* out, cudaStream_t s) {
   const RowArgs<T> a{row, (const T*)in, (const T*)edata, edata_dim, feat_dim, st, num_rows, E, ws, (T*)out,
-                     mode, fixed, split, (int)feat_dim, nullptr, nullptr, col, nullptr, nullptr, 0u};
+                     mode, fixed, split, (int)feat_dim, Verdict{}, nullptr, col, nullptr, nullptr, 0u};
   ProfScope prof("spmm_rows", s);
   return launch_spmm_rows<T>(op, a, s);
 }

@@ -131,6 +131,21 @@ inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t n
   return r;
 }
 
+// What the blocks of a kernel that looks edges over found, a word each (k_gat_ranges). A word per block is written whatever it
+// is, so that nothing has to be cleared in front; who needs the answer reads them all.
+struct Verdict {
+  const uint32_t* word;      // null: nothing was found
+  int count;
+};
+constexpr int kVerdicts = 592;
+// By all threads of a block.
+__device__ __forceinline__ bool any_found(const Verdict& v) {
+  if (!v.word) return false;
+  uint32_t found = 0u;
+  for (int t = threadIdx.x; t < v.count; t += blockDim.x) found |= v.word[t];
+  return __syncthreads_or((int)found) != 0;
+}
+
 template <typename T>
 struct RowArgs {
   const int64_t* row;
@@ -144,7 +159,7 @@ struct RowArgs {
   int mode, fixed;
   RowSplit split;
   int part_stride;         // floats per part
-  const int32_t* none;     // when given and not zero: no row has edges (kRanges)
+  Verdict none;            // found: no row has edges (kRanges)
   int32_t* status;         // flags of the call; null: the library's own word (apt_pending_flags)
   const int64_t* col;      // output row of an edge, inside its segment
   // kDots
@@ -306,7 +321,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   const int per = (int)(a.feat_dim / a.edata_dim);
   const uint32_t row_bytes = (uint32_t)(a.feat_dim * sizeof(T));
   const uint32_t ed_bytes = (uint32_t)(a.edata_dim * (OP == kUMulW ? sizeof(float) : sizeof(T)));
-  const bool none = a.none && *a.none != 0;
+  const bool none = any_found(a.none);
   // rows and edges fit 31 bits, and so does everything that counts them
   const int num_rows = (int)a.num_rows;
   const int warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

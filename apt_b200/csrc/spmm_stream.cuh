@@ -130,7 +130,7 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   }
 
   // this warp's slots, [lo, hi) of `total`; a stretch ends inside a group only where the last row ends
-  const bool none = a.none && *a.none != 0;
+  const bool none = any_found(a.none);
   const int total = mode == kOrder ? *a.ws.num_slots : none ? 0 : (int)a.num_edges;
   const int chunk = max(GE, (int)(((int64_t)total + warps - 1) / warps + GE - 1) & ~(GE - 1));
   auto out_row = [&](int k) -> uint32_t { return (uint32_t)(ooff[a.st.nseg > 1 ? seg_of(coo, a.st.nseg, k) : 0] + a.col[k]); };

@@ -94,3 +94,19 @@ def test_dots_beside_infinite_features():
     _, g_el, g_er = ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, g)
     assert torch.equal(g_er[:, 1:], plain[2][:, 1:]) and not bool(g_er[:, 0].isfinite().any())
     assert float((g_el[:, 1:] - plain[1][:, 1:]).norm() / plain[1][:, 1:].norm()) <= 2e-6      # (44 edges a source, added up in the order of arrival)
+
+
+@pytest.mark.parametrize("at", [1, 350_000, 699_999])
+def test_edges_out_of_order_belong_to_nobody(at):
+    # one edge out of its destination's turn, wherever it is: zeros everywhere, and the flag
+    gen = torch.Generator(device="cuda").manual_seed(at)
+    E, n_dst, n_src = 700_000, 50_000, 9001
+    col = torch.arange(n_dst, device="cuda").repeat_interleave(14)
+    col[at - 1], col[at] = n_dst - 1 if at < E // 2 else col[at - 1], 0
+    row = torch.randint(0, n_src, (E,), device="cuda", generator=gen)
+    make = lambda *shape: torch.randn(shape, device="cuda", generator=gen)
+    ft, el, er, g = make(n_src, 4, 32), make(n_src, 4, 1), make(n_dst, 4, 1), make(n_dst, 4, 32)
+    got = (ops.gat_edge_softmax_sum(row, col, ft, el, er, n_dst),) + tuple(ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, g))
+    with pytest.raises(RuntimeError, match="grouped"):
+        ops.check_status()
+    assert not any(bool(t.any()) for t in got)
