@@ -172,7 +172,7 @@ struct RowArgs {
 constexpr int kStreamBlocks = 2;
 constexpr int stream_warps(bool one_slice) { return one_slice ? 12 : 10; }
 constexpr int kStreamShared = 112 * 1024 - 2560;      // a block's, beside its barriers and segment tables
-constexpr int kStreamHeads = 8;                       // weights an edge can bring along
+constexpr int kStreamHeads = 8, kStreamHeadsWide = 16;      // weights an edge can bring along; of wide rows behind the sort
 constexpr int kStreamMinSlices = 17, kStreamStretch = 32;
 constexpr int kStreamMinOrdered = 3 << 15, kStreamMinWide = 3 << 16, kStreamMinWeighted = 3 << 17, kStreamMinSums = 5 << 17;
 // Rows to a group; a warp has two groups on their way.
@@ -199,7 +199,8 @@ inline StreamPlan stream_plan(int op, int64_t feat_dim, size_t esz, int heads) {
 // `slice`: bytes of the widest access to rows and results. `grouped`: the edges are (kFixed, kRanges).
 inline bool stream_fits(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges, bool grouped) {
   const int64_t row = feat_dim * (int64_t)esz;
-  if (slice != 16 || row < kStreamMinSlices * 16 || row > 64 * 16 || heads > kStreamHeads) return false;
+  if (slice != 16 || row < kStreamMinSlices * 16 || row > 64 * 16) return false;
+  if (heads > (!grouped && row > 512 && num_edges >= kStreamMinWide ? kStreamHeadsWide : kStreamHeads)) return false;
   const int64_t least = !grouped ? kStreamMinOrdered : row > 512 ? kStreamMinWide : op == kCopyU ? kStreamMinSums : kStreamMinWeighted;
   if (num_edges < least) return false;
   if (op != kDots) return op == kCopyU || op == kUMulW;

@@ -60,7 +60,7 @@ def _layer(row, col, ft, el, er, g, n_dst):
 
 
 @pytest.mark.parametrize("dtype,H,D", [(torch.float32, 4, 32), (torch.float32, 1, 256), (torch.float32, 8, 32), (torch.float32, 4, 48),
-                                       (torch.float32, 2, 44), (torch.bfloat16, 4, 64), (torch.bfloat16, 8, 24), (torch.float16, 5, 40),
+                                       (torch.float32, 2, 44), (torch.float32, 16, 16), (torch.bfloat16, 4, 64), (torch.bfloat16, 8, 24), (torch.float16, 5, 40),
                                        (torch.float16, 2, 256)])
 @pytest.mark.parametrize("ragged", [False, True])
 def test_attention(dtype, H, D, ragged):
