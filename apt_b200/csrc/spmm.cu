@@ -83,6 +83,8 @@ __device__ __forceinline__ unsigned long long probe_votes(uint32_t bits) {
 }
 
 // num_rows: the output rows there are (the caller's result may have more, or fewer, than the offsets end at); -1: as the offsets say.
+// K edges a thread at a time: four, eight where more than one wave of four would be needed (1.01 M edges 8.1 -> 7 us).
+template <int K>
 __global__ void __launch_bounds__(256)
 k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_rows, unsigned long long* agg, int slot,
              volatile int64_t* result, int64_t sequence) {
@@ -90,7 +92,6 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
   if (!agg) agg = g_probe_votes + slot;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
   __shared__ uint32_t s_bits;
-  constexpr int K = 8;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, c[K];
   auto fetch = [&]() {
@@ -148,7 +149,10 @@ static int launch_probe(const int64_t* col, int64_t E, SegTable st, int64_t num_
   // a thousand edges a block and one wave at most: small blocks of edges are looked over by one thread block
   const int grid = wave_grid(ceil_div(E, 1024), 4, 1);
   ProfScope prof("spmm_ranges", s);
-  APT_FOLLOW(k_spmm_probe, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence);
+  if (E > (int64_t)grid * 256 * 4)
+    APT_FOLLOW(k_spmm_probe<8>, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence);
+  else
+    APT_FOLLOW(k_spmm_probe<4>, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence);
   return APT_OK;
 }
 
