@@ -77,7 +77,8 @@ k_gat_ranges(const int64_t* __restrict__ col, int64_t E, int64_t num_dst, int2* 
     for (int k = 0; k < K; ++k) {
       const int64_t e = e0 + k * stride;
       at[k] = e < E ? col[e] : 0;
-      before[k] = e < E && e > 0 ? col[e - 1] : (int64_t)-1;
+      // (a negative one opens no gap in front of the table: its own edge is the bad one)
+      before[k] = e < E && e > 0 ? max(col[e - 1], (int64_t)-1) : (int64_t)-1;
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {

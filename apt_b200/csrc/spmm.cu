@@ -265,8 +265,9 @@ k_edge_ranges(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t n
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
     const int64_t d = out_row(coo, ooff, st.nseg, col, e);
-    const int64_t prev = e > 0 ? out_row(coo, ooff, st.nseg, col, e - 1) : (int64_t)-1;
-    if (d < prev || d < 0 || d >= num_rows) continue;   // the probe has seen that there is none
+    // the probe has seen that no edge is out of order or of no row; where it has not been asked, nothing is written outside the table
+    const int64_t prev = e > 0 ? max(out_row(coo, ooff, st.nseg, col, e - 1), (int64_t)-1) : (int64_t)-1;
+    if (d < prev || d < 0 || d >= num_rows) continue;
     if (d != prev) {
       if (prev >= 0) ws.range[prev].y = (int)e;
       for (int64_t t = prev + 1; t < d; ++t) ws.range[t] = make_int2(0, 0);
