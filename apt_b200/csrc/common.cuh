@@ -85,6 +85,10 @@ inline dim3 as_grid(dim3 grid) { return grid; }
 void set_relabel_small(bool on);   // relabel.cu: one-block shared-memory path for small layers
 void set_bulk_wait_polls(int polls);   // spmm.cu: bound of k_spmm_stream's waits
 
+// The tag of a sequence number (Tagged). A plain value's upper half is all zeros or all ones: no tag is, whatever the number, so that
+// words which were read already are never taken for an answer. Numbers 2^30 apart share one.
+__host__ __device__ inline uint32_t tag_of(int64_t sequence) { return ((uint32_t)sequence & 0x3fffffffu) | 0x40000000u; }
+
 // While another thread captures a stream, or this one does, calls that might synchronise are refused and end the capture. For
 // those that do not touch the captured work (page-locked memory of the library's own, asking a stream how it stands).
 struct RelaxedCapture {
@@ -200,8 +204,8 @@ __device__ __forceinline__ int owner_of(int64_t v, const int64_t* mv, const Owne
   return d;
 }
 
-// A word block (of 32-bit values) on its way to page-locked host memory, a sequence number in the upper half of every word:
-// the host polls for that, and nothing has to be ordered on the way. (A fence for a sequence number behind them all waits for
+// A word block (of 32-bit values) on its way to page-locked host memory, the tag of a sequence number in the upper half of every
+// word: the host polls for that, and nothing has to be ordered on the way. (A fence for a sequence number behind them all waits for
 // the host link, 2 us when it is idle and up to 50 beside a gather's reads.) By all threads of a block.
 struct Tagged {
   const int64_t* words;
@@ -212,7 +216,7 @@ struct Tagged {
   int64_t* host;                  // null: nothing is published
 };
 __device__ __forceinline__ void publish_tagged(const Tagged& p) {
-  const int64_t tag = (p.sequence_dev ? *p.sequence_dev : p.sequence) << 32;
+  const int64_t tag = (int64_t)tag_of(p.sequence_dev ? *p.sequence_dev : p.sequence) << 32;
   volatile int64_t* const host = p.host;
   for (int t = threadIdx.x; t < p.count; t += blockDim.x)
     host[t] = tag | ((t == p.count - 1 ? *(const volatile int64_t*)p.last : p.words[t]) & 0xffffffffll);

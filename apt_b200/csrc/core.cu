@@ -202,7 +202,7 @@ int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* s
 int apt_wait_tagged(int64_t* host, int count, int64_t sequence, void* stream) {
   APT_CHECK_ARG(host && count >= 1, "apt_wait_tagged: bad argument");
   for (int t = count - 1; t >= 0; --t) {
-    const int rc = wait_for_word(host + t, 32, sequence & 0xffffffffll, stream);
+    const int rc = wait_for_word(host + t, 32, apt::tag_of(sequence), stream);
     if (rc != APT_OK) return rc;
     host[t] = (int32_t)host[t];
   }

@@ -85,9 +85,9 @@ int apt_publish_words(const int64_t* words, int count, const int64_t* sequence_d
 /* The same with the last word taken from *last instead (counts of one block, status flags of another); NULL: from words. */
 int apt_publish_words_from(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev,
                            int64_t sequence, int64_t* host, void* stream);
-/* Words of 32-bit values, each with the lower half of the sequence number in its upper half, so that nothing has to be ordered
- * behind anything on the way: apt_wait_tagged polls every one of the count words and leaves the plain values (signed; the
- * sequence numbers of one host buffer differ and are not 0 or -1 in that half). The last word comes from *last. */
+/* Words of 32-bit values, each with 30 bits of the sequence number in its upper half, so that nothing has to be ordered
+ * behind anything on the way: apt_wait_tagged polls every one of the count words and leaves the plain values (signed;
+ * publications of one host buffer that nobody waited for differ in those bits). The last word comes from *last. */
 int apt_publish_tagged(const int64_t* words, int count, const int64_t* last, const int64_t* sequence_dev,
                        int64_t sequence, int64_t* host, void* stream);
 int apt_wait_tagged(int64_t* host, int count, int64_t sequence, void* stream);

@@ -68,3 +68,18 @@ def test_arrays_copied_in_one_call(counts):
                              (ctypes.c_int64 * len(counts))(*counts), len(counts), stream))
     for n, a, b in zip(counts, src, dst):
         assert torch.equal(a[:n], b[:n]) and int(b[n]) == -9
+
+
+@pytest.mark.parametrize("seq", [0, 2 ** 32 - 1, 2 ** 32, -1])
+def test_words_that_were_read_answer_no_later_wait(seq):
+    # a plain value's upper half is 0 or all ones, and so is that of a sequence number now and then
+    words, last, want, host = _blocks(40)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    check(lib.apt_publish_tagged(_ptr(words), 40, _ptr(last), None, 7, _ptr(host), stream))
+    check(lib.apt_wait_tagged(_ptr(host), 40, 7, stream))
+    torch.cuda.synchronize()
+    host[:] = 5 if seq in (0, 2 ** 32) else -5
+    assert lib.apt_wait_tagged(_ptr(host), 40, seq, stream) == _lib.APT_ERR_TIMEOUT
+    check(lib.apt_publish_tagged(_ptr(words), 40, _ptr(last), None, seq, _ptr(host), stream))
+    check(lib.apt_wait_tagged(_ptr(host), 40, seq, stream))
+    assert host.tolist() == want
