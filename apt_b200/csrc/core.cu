@@ -175,7 +175,7 @@ int apt_publish_tagged(const int64_t* words, int count, const int64_t* last, con
   return APT_OK;
 }
 
-static int wait_for_word(const volatile int64_t* word, int shift, int64_t sequence, void* stream) {
+static int wait_for_word(const char* who, const volatile int64_t* word, int shift, int64_t sequence, void* stream) {
   for (int64_t spin = 1; (int64_t)((uint64_t)*word >> shift) != sequence; ++spin) {
     if ((spin & 0x3fff) == 0) {
       // now and then the stream is asked, so that an error on it ends the wait
@@ -184,7 +184,7 @@ static int wait_for_word(const volatile int64_t* word, int shift, int64_t sequen
       if (e == cudaErrorNotReady) continue;
       APT_CUDA(e);
       if ((int64_t)((uint64_t)*word >> shift) == sequence) break;
-      apt::set_error("apt_wait_published: the stream is idle and the words have not arrived");
+      apt::set_error("%s: the stream is idle and the words have not arrived", who);
       return APT_ERR_TIMEOUT;
     }
 #if defined(__x86_64__)
@@ -196,13 +196,13 @@ static int wait_for_word(const volatile int64_t* word, int shift, int64_t sequen
 
 int apt_wait_published(const int64_t* host, int count, int64_t sequence, void* stream) {
   APT_CHECK_ARG(host && count >= 0, "apt_wait_published: bad argument");
-  return wait_for_word(host + count, 0, sequence, stream);
+  return wait_for_word("apt_wait_published", host + count, 0, sequence, stream);
 }
 
 int apt_wait_tagged(int64_t* host, int count, int64_t sequence, void* stream) {
   APT_CHECK_ARG(host && count >= 1, "apt_wait_tagged: bad argument");
   for (int t = count - 1; t >= 0; --t) {
-    const int rc = wait_for_word(host + t, 32, apt::tag_of(sequence), stream);
+    const int rc = wait_for_word("apt_wait_tagged", host + t, 32, apt::tag_of(sequence), stream);
     if (rc != APT_OK) return rc;
     host[t] = (int32_t)host[t];
   }

@@ -83,3 +83,12 @@ def test_words_that_were_read_answer_no_later_wait(seq):
     check(lib.apt_publish_tagged(_ptr(words), 40, _ptr(last), None, seq, _ptr(host), stream))
     check(lib.apt_wait_tagged(_ptr(host), 40, seq, stream))
     assert host.tolist() == want
+
+
+def test_a_wait_in_vain_names_itself():
+    host = torch.zeros(3, dtype=torch.int64).pin_memory()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for wait in ("apt_wait_tagged", "apt_wait_published"):
+        assert getattr(lib, wait)(_ptr(host), 2, 4, stream) == _lib.APT_ERR_TIMEOUT
+        with pytest.raises(RuntimeError, match=wait + ": the stream is idle"):
+            check(_lib.APT_ERR_TIMEOUT)
