@@ -157,7 +157,7 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
     const bool few = deg <= K * W;
     uint32_t src[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) src[k] = few && r.x + part + k * W < r.y ? (uint32_t)row[r.x + part + k * W] : 0u;
+    for (int k = 0; k < K; ++k) src[k] = few && part + k * W < deg ? (uint32_t)row[r.x + part + k * W] : 0u;
 #pragma unroll 1
     for (int h0 = 0; h0 < num_heads; h0 += NH) {
       Heads<NH> bias, s[K];
@@ -178,14 +178,14 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
       if (few) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (r.x + part + k * W < r.y) {
+          if (part + k * W < deg) {
             s[k] = scores(src[k]);
 #pragma unroll
             for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], s[k].v[h]);
           }
       } else {
-        for (int e = r.x + part; e < r.y; e += W) {
-          const Heads<NH> x = scores(row[e]);
+        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+          const Heads<NH> x = scores(row[r.x + j]);
 #pragma unroll
           for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], x.v[h]);
         }
@@ -197,15 +197,15 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
       if (few) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (r.x + part + k * W < r.y)
+          if (part + k * W < deg)
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
               s[k].v[h] = expf(s[k].v[h] - most[h]);
               sum[h] += s[k].v[h];
             }
       } else {
-        for (int e = r.x + part; e < r.y; e += W) {
-          const Heads<NH> x = scores(row[e]);
+        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+          const Heads<NH> x = scores(row[r.x + j]);
 #pragma unroll
           for (int h = 0; h < NH; ++h) sum[h] += expf(x.v[h] - most[h]);
         }
@@ -229,13 +229,13 @@ k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T
       if (few) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (r.x + part + k * W < r.y) put(r.x + part + k * W, s[k]);
+          if (part + k * W < deg) put(r.x + part + k * W, s[k]);
       } else {
-        for (int e = r.x + part; e < r.y; e += W) {
-          Heads<NH> x = scores(row[e]);
+        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+          Heads<NH> x = scores(row[r.x + j]);
 #pragma unroll
           for (int h = 0; h < NH; ++h) x.v[h] = expf(x.v[h] - most[h]);
-          put(e, x);
+          put(r.x + j, x);
         }
       }
     }
@@ -251,20 +251,21 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
            int hpp, uint32_t num_src, int32_t* __restrict__ src_count, uint32_t* __restrict__ rank) {
   wait_for_previous();
   if (any_found(none)) return;
-  const int lane = threadIdx.x & 31, G = gridDim.x * 8, num_dst = (int)num_dst_;
+  const int lane = threadIdx.x & 31;
+  const uint32_t G = gridDim.x * 8, num_dst = (uint32_t)num_dst_;
   const int lpe = lph * hpp, ep = 32 / lpe;
   const int epi = lane / lpe, rh = (lane & (lpe - 1)) / lph, p = lane & (lph - 1);
   const int nvh = head_dim / VE;
   const uint32_t row_bytes = (uint32_t)((int64_t)num_heads * head_dim * sizeof(T));
-  int d = blockIdx.x * 8 + (threadIdx.x >> 5);
+  uint32_t d = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (d >= num_dst) return;
   int2 r = range[d], nr = make_int2(0, 0);
   // lanes past the last edge hold its source too, so that a round may load past the end
-  uint32_t src = r.x < r.y ? (uint32_t)row[min(r.x + lane, r.y - 1)] : 0u, nsrc = 0;
+  uint32_t src = r.x < r.y ? (uint32_t)row[r.x + min(lane, r.y - r.x - 1)] : 0u, nsrc = 0;
   if (d + G < num_dst) nr = range[d + G];
   for (; d < num_dst; d += G) {
     int2 nnr = make_int2(0, 0);
-    if (nr.x < nr.y) nsrc = (uint32_t)row[min(nr.x + lane, nr.y - 1)];
+    if (nr.x < nr.y) nsrc = (uint32_t)row[nr.x + min(lane, nr.y - nr.x - 1)];
     if (d + 2 * G < num_dst) nnr = range[d + 2 * G];
     for (int h0 = 0; h0 < num_heads; h0 += hpp) {
       const int h = h0 + rh;
@@ -286,10 +287,10 @@ k_gat_dots(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* _
       };
       block(0);
 #pragma unroll 1
-      for (int base = r.x; base < r.y; base += 32) {
-        const int cnt = min(32, r.y - base);
+      for (int rest = r.y - r.x; rest > 0; rest -= 32) {
+        const int base = r.y - rest, cnt = min(32, rest);
         uint32_t my_src = src;
-        if (base != r.x) my_src = (uint32_t)row[min(base + lane, r.y - 1)];
+        if (base != r.x) my_src = (uint32_t)row[base + min(lane, rest - 1)];
         const bool ranked = h0 == 0 && lane < cnt;
         uint32_t place = kNoRank;
         if (ranked && my_src < num_src) place = (uint32_t)atomicAdd(src_count + spread(my_src), 1);
@@ -382,9 +383,9 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
     uint32_t place[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const int e = r.x + part + k * W;
-      src[k] = few && e < r.y ? row[e] : 0;
-      place[k] = few && e < r.y ? place_of(e) : kNoRank;
+      const bool mine = few && part + k * W < deg;
+      src[k] = mine ? row[r.x + part + k * W] : 0;
+      place[k] = mine ? place_of(r.x + part + k * W) : kNoRank;
     }
 #pragma unroll 1
     for (int h0 = 0; h0 < num_heads; h0 += NH) {
@@ -402,7 +403,7 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
       if (few) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (r.x + part + k * W < r.y) {
+          if (part + k * W < deg) {
             fetch(r.x + part + k * W, w[k], dot[k]);
             x[k] = load_scores<T, NH>(el + src[k] * num_heads + h0);
           }
@@ -411,11 +412,12 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
           for (int k = 0; k < K; ++k) put(r.x + part + k * W, src[k], place[k]);
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (r.x + part + k * W < r.y)
+          if (part + k * W < deg)
 #pragma unroll
             for (int h = 0; h < NH; ++h) t[h] += w[k].v[h] * dot[k].v[h];
       } else {
-        for (int e = r.x + part; e < r.y; e += W) {
+        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+          const int e = r.x + j;
           fetch(e, w[0], dot[0]);
 #pragma unroll
           for (int h = 0; h < NH; ++h) t[h] += w[0].v[h] * dot[0].v[h];
@@ -435,9 +437,10 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
       if (few) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (r.x + part + k * W < r.y) grad(src[k], w[k], dot[k], x[k]);
+          if (part + k * W < deg) grad(src[k], w[k], dot[k], x[k]);
       } else {
-        for (int e = r.x + part; e < r.y; e += W) {
+        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+          const int e = r.x + j;
           const int64_t from = row[e];
           fetch(e, w[0], dot[0]);
           x[0] = load_scores<T, NH>(el + from * num_heads + h0);
@@ -691,9 +694,10 @@ struct GatScores {
 
   __device__ __forceinline__ float score(int64_t src, int h, float bias) const { return Elem<T>::to_f(el[src * H + h0 + h]) + bias; }
   __device__ __forceinline__ void start(const T* er, int d, int2 r, int lane) {
-    few = r.y - r.x <= 32;
+    const uint32_t deg = r.y - r.x;
+    few = deg <= 32;
     positive = 0u;
-    const bool mine = few && r.x + lane < r.y;
+    const bool mine = few && lane < (int)deg;
     const int64_t src = mine ? row[r.x + lane] : 0;
     float bias[kAloneHeads], x[kAloneHeads];
 #pragma unroll
@@ -708,16 +712,16 @@ struct GatScores {
       if (h >= nh) break;
       float most = mine ? leaky(x[h], slope) : -INFINITY, sum = 0.f;
       if (!few)
-        for (int e = r.x + lane; e < r.y; e += 32) most = fmaxf(most, leaky(score(row[e], h, bias[h]), slope));
+        for (uint32_t k = lane; k < deg; k += 32) most = fmaxf(most, leaky(score(row[r.x + k], h, bias[h]), slope));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
       if (mine) sum = expf(leaky(x[h], slope) - most);
       if (!few)
-        for (int e = r.x + lane; e < r.y; e += 32) sum += expf(leaky(score(row[e], h, bias[h]), slope) - most);
+        for (uint32_t k = lane; k < deg; k += 32) sum += expf(leaky(score(row[r.x + k], h, bias[h]), slope) - most);
       const float own = sum;
       sum = group_sum(sum, 32);
       const float inv = sum > 0.f ? 1.f / sum : 0.f;
-      if (mine) sh.w[lane][h] = !(sum > 0.f) && r.y - r.x <= masked ? 0.f : own * inv;
+      if (mine) sh.w[lane][h] = !(sum > 0.f) && (int)deg <= masked ? 0.f : own * inv;
       if (mine && x[h] > 0.f) positive |= 1u << h;
       if (!few && lane == 0) sh.bias[h] = bias[h], sh.most[h] = most, sh.inv[h] = inv;
     }
@@ -765,8 +769,8 @@ k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* 
         const T* const lane_ft = ft + col;
         Acc<VE> acc;
         acc.zero();
-        for (int base = r.x; base < r.y; base += 32) {
-          const int cnt = min(32, r.y - base);
+        for (int rest = deg; rest > 0; rest -= 32) {
+          const int base = r.y - rest, cnt = min(32, rest);
           const uint32_t src = lane < cnt ? (uint32_t)row[base + lane] : 0u;
           if (c0 == 0 || deg > 32) {
             sc.chunk(src, lane < cnt, lane);
@@ -869,8 +873,8 @@ k_gat_alone_backward(const int64_t* __restrict__ row, const T* __restrict__ ft, 
       // up to 32 edges: t first, then the results, from the same dots; more: two walks
       const int passes = deg > 32 ? 2 : 1;
       for (int pass = 0; pass < passes; ++pass) {
-        for (int base = r.x; base < r.y; base += 32) {
-          const int cnt = min(32, r.y - base);
+        for (int rest = deg; rest > 0; rest -= 32) {
+          const int base = r.y - rest, cnt = min(32, rest);
           const uint32_t src = lane < cnt ? (uint32_t)row[base + lane] : 0u;
           __syncwarp();
           for (int hb = 0; hb < sc.nh; hb += hpp) {

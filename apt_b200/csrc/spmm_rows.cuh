@@ -175,6 +175,7 @@ constexpr int kStreamShared = 112 * 1024 - 2560;      // a block's, beside its b
 constexpr int kStreamHeads = 8, kStreamHeadsWide = 16;      // weights an edge can bring along; of wide rows behind the sort
 constexpr int kStreamMinSlices = 17, kStreamStretch = 32;
 constexpr int kStreamMinOrdered = 3 << 15, kStreamMinWide = 3 << 16, kStreamMinWeighted = 3 << 17, kStreamMinSums = 5 << 17;
+constexpr int64_t kStreamMaxEdges = 0x7fffffff - 4096;      // a warp looks up to 159 slots ahead of the last one, in 31 bits
 // Rows to a group; a warp has two groups on their way.
 constexpr int stream_group(bool one_slice) { return one_slice ? 8 : 4; }
 
@@ -199,7 +200,7 @@ inline StreamPlan stream_plan(int op, int64_t feat_dim, size_t esz, int heads) {
 // `slice`: bytes of the widest access to rows and results. `grouped`: the edges are (kFixed, kRanges).
 inline bool stream_fits(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges, bool grouped) {
   const int64_t row = feat_dim * (int64_t)esz;
-  if (slice != 16 || row < kStreamMinSlices * 16 || row > 64 * 16) return false;
+  if (slice != 16 || row < kStreamMinSlices * 16 || row > 64 * 16 || num_edges > kStreamMaxEdges) return false;
   if (heads > (!grouped && row > 512 && num_edges >= kStreamMinWide ? kStreamHeadsWide : kStreamHeads)) return false;
   const int64_t least = !grouped ? kStreamMinOrdered : row > 512 ? kStreamMinWide : op == kCopyU ? kStreamMinSums : kStreamMinWeighted;
   if (num_edges < least) return false;
@@ -323,8 +324,8 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   const uint32_t row_bytes = (uint32_t)(a.feat_dim * sizeof(T));
   const uint32_t ed_bytes = (uint32_t)(a.edata_dim * (OP == kUMulW ? sizeof(float) : sizeof(T)));
   const bool none = any_found(a.none);
-  // rows and edges fit 31 bits, and so does everything that counts them
-  const int num_rows = (int)a.num_rows;
+  // rows and edges fit 31 bits; what is added to them is compared with what is left, or unsigned
+  const uint32_t num_rows = (uint32_t)a.num_rows;
   const int warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int num_items = mode == kOrder ? min(*a.ws.num_items, (int)a.ws.max_items) : 0;
   // whole warps first take items, dealt from the last warp on (the first rows, often the longest, are the first warps': rows
@@ -350,9 +351,9 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
       src = OP == kCopyE ? 0u : (uint32_t)(ioff[a.st.nseg > 1 ? seg_of(coo, a.st.nseg, k) : 0] + a.row[k]);
     }
   };
-  auto bounds = [&](int d, int& b, int& e) {
+  auto bounds = [&](uint32_t d, int& b, int& e) {
     if (mode == kFixed) {
-      b = d * fixed;
+      b = (int)d * fixed;
       e = b + fixed;
     } else {
       const int2 r = none ? make_int2(0, 0) : a.ws.range[d];
@@ -361,16 +362,16 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     }
   };
 
-  int d = 0, G = 0;
+  uint32_t d = 0, G = 0;
   int b = 0, e = 0, nb = 0, ne = 0, part = -1;
   uint32_t src = 0, eid = 0, nsrc = 0, neid = 0;
   auto start_item = [&]() {
     const int4 m = a.ws.items[it];
-    d = m.x;
+    d = (uint32_t)m.x;
     b = m.y;
     e = m.z;
     part = m.w;
-    if (b + lane < e) resolve(b + lane, src, eid);
+    if (lane < e - b) resolve(b + lane, src, eid);
   };
   auto start_rows = [&]() {
     items = false;
@@ -381,7 +382,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     part = -1;
     if (d < num_rows) {
       bounds(d, b, e);
-      if (b + SUB < e) resolve(b + SUB, src, eid);
+      if (SUB < e - b) resolve(b + SUB, src, eid);
     }
     if (d + G < num_rows) bounds(d + G, nb, ne);
   };
@@ -409,7 +410,7 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     int nnb = 0, nne = 0;
     if (!items) {
       // the next row's indexes and the bounds of the one after it are on their way while this one is summed
-      if (d + G < num_rows && nb + SUB < ne) resolve(nb + SUB, nsrc, neid);
+      if (d + G < num_rows && SUB < ne - nb) resolve(nb + SUB, nsrc, neid);
       if (d + 2 * G < num_rows) bounds(d + 2 * G, nnb, nne);
     }
     const bool skip = !items && mode == kOrder && e - b > a.split.long_edges;
@@ -421,9 +422,10 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
       for (int i = 0; i < VPL; ++i) acc[i].zero();
       uint32_t my_src = src, my_e = eid;
 #pragma unroll 1
-      for (int k0 = b; k0 < e; k0 += LPR) {
-        if (k0 != b && k0 + SUB < e) resolve(k0 + SUB, my_src, my_e);
-        const int cnt = min(LPR, e - k0);
+      for (int left = e - b; left > 0; left -= LPR) {
+        const int k0 = e - left;
+        if (k0 != b && SUB < left) resolve(k0 + SUB, my_src, my_e);
+        const int cnt = min(LPR, left);
         int j = EPI;
         const int full = cnt & ~(EP * U - 1);
 #pragma unroll 1

@@ -104,7 +104,8 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
 
-  const int num_rows = (int)a.num_rows, heads = OP != kCopyU ? (int)a.edata_dim : 1;
+  const uint32_t num_rows = (uint32_t)a.num_rows;
+  const int heads = OP != kCopyU ? (int)a.edata_dim : 1;
   const int warps = gridDim.x * plan.warps, warp = blockIdx.x * plan.warps + w;
   const uint32_t row_bytes = plan.row_bytes;
   unsigned char* const ring = shared + w * plan.warp_bytes;
@@ -236,13 +237,13 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
 
   if (!kIsDots && mode != kFixed) {
     // rows without edges, while the first copies are on their way
-    for (int first = warp * 32; first < num_rows; first += warps * 32) {
+    for (uint32_t first = warp * 32; first < num_rows; first += warps * 32) {
       bool empty = false;
       if (first + lane < num_rows) {
         const int2 r = none ? make_int2(0, 0) : a.ws.range[first + lane];
         empty = r.x == r.y;
       }
-      for (unsigned m = __ballot_sync(0xffffffffu, empty); m; m &= m - 1) write((uint32_t)(first + __ffs(m) - 1));
+      for (unsigned m = __ballot_sync(0xffffffffu, empty); m; m &= m - 1) write(first + __ffs(m) - 1);
     }
   }
   if (lo >= hi) return;
@@ -255,7 +256,7 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   Raw<T, VE> ahead[VPL];
   uint32_t ahead_row = kNoRow;
   auto look_ahead = [&](uint32_t d) {
-    ahead_row = min(d, (uint32_t)(num_rows - 1));
+    ahead_row = min(d, num_rows - 1);
 #pragma unroll
     for (int i = 0; i < VPL; ++i) ahead[i] = load_raw<T, VE>(a.own + (uint64_t)ahead_row * a.feat_dim + col[i]);
   };
