@@ -174,6 +174,7 @@ constexpr int stream_warps(bool one_slice) { return one_slice ? 12 : 10; }
 constexpr int kStreamShared = 112 * 1024 - 2560;      // a block's, beside its barriers and segment tables
 constexpr int kStreamHeads = 8, kStreamHeadsWide = 16;      // weights an edge can bring along; of wide rows behind the sort
 constexpr int kStreamMinSlices = 17, kStreamStretch = 32;
+constexpr int kStreamParts = 32;      // parts of a row that one warp adds up
 constexpr int kStreamMinOrdered = 3 << 15, kStreamMinWide = 3 << 16, kStreamMinWeighted = 3 << 17, kStreamMinSums = 5 << 17;
 constexpr int64_t kStreamMaxEdges = 0x7fffffff - 4096;      // a warp looks up to 159 slots ahead of the last one, in 31 bits
 // Rows to a group; a warp has two groups on their way.

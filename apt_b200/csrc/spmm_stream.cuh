@@ -9,7 +9,7 @@
 //
 //   stretch     every warp has the same number of slots. Edges that come grouped are cut at row ends; behind the counting sort
 //               they are cut anywhere, sums of a row of several stretches are left in scratch and the warp that comes last adds
-//               them up in order: long rows need no items of their own and no warp has more to do than another.
+//               them up in order, above 32 stretches in two steps: long rows need no items of their own.
 //   copies      rows of up to 512 bytes by 16-byte cp.async, an instruction a row; wider ones by one cp.async.bulk each, from a lane
 //               each (that instruction is issued lane by lane, 13 instructions a row, and two cp.async with their addresses are
 //               as many: fp32 x 256 142 against 146 us in reverse, x 132 134 against 142, dots of 4 x 64 faster too).
@@ -424,6 +424,14 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   if (goes_on) leave(open ? 2 * warp : 2 * warp + 1);
   __threadfence();
   __syncwarp();
+  // whether this warp is the last of `of` that come by `counter`; what the others left can then be read
+  auto comes_last = [&](int counter, int of) {
+    int done = 0;
+    if (lane == 0 && of > 1) done = atomicAdd(a.ws.part_done + counter, 1);
+    if (__shfl_sync(0xffffffffu, done, 0) != of - 1) return false;
+    __threadfence();
+    return true;
+  };
 #pragma unroll 1
   for (int k = 0; k < 2; ++k) {
     // the first row; the last one, unless it is the first and began before this stretch
@@ -431,22 +439,33 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
     const uint32_t d = k == 0 ? first_row : last_row;
     const int2 r = a.ws.range[d];
     const int first = r.x / chunk, parts = (r.y - 1) / chunk - first + 1;
-    int done = 0;
-    if (lane == 0) done = atomicAdd(a.ws.part_done + first, 1);
-    if (__shfl_sync(0xffffffffu, done, 0) != parts - 1) continue;
-    __threadfence();
-    clear();
+    auto slot = [&](int q) { return 2 * (first + q) + (q == 0 ? 1 : 0); };
+    auto sum = [&](int from, int count, int step) {
+      clear();
 #pragma unroll 2
-    for (int q = 0; q < parts; ++q) {
-      const float* const p = part_of(2 * (first + q) + (q == 0 ? 1 : 0));
+      for (int q = 0; q < count; ++q) {
+        const float* const p = part_of(slot(from + q * step));
 #pragma unroll
-      for (int i = 0; i < VPL; ++i)
+        for (int i = 0; i < VPL; ++i)
 #pragma unroll
-        for (int t = 0; t < VE; t += 4) {
-          const float4 x = __ldcg((const float4*)(p + col[i] + t));
-          acc[i].p[t / 2] = f2_add(acc[i].p[t / 2], f2_pack(x.x, x.y));
-          acc[i].p[t / 2 + 1] = f2_add(acc[i].p[t / 2 + 1], f2_pack(x.z, x.w));
-        }
+          for (int t = 0; t < VE; t += 4) {
+            const float4 x = __ldcg((const float4*)(p + col[i] + t));
+            acc[i].p[t / 2] = f2_add(acc[i].p[t / 2], f2_pack(x.x, x.y));
+            acc[i].p[t / 2 + 1] = f2_add(acc[i].p[t / 2 + 1], f2_pack(x.z, x.w));
+          }
+      }
+    };
+    // The last of every kStreamParts stretches adds up theirs, the last of these the row. Counters: the group's first stretch, and the
+    // row's second one, in neither of which another row begins (a group of one needs none).
+    const int group = (warp - first) / kStreamParts * kStreamParts, size = min(kStreamParts, parts - group);
+    if (!comes_last(first + group, size)) continue;
+    sum(group, size, 1);
+    if (parts > kStreamParts) {
+      leave(slot(group));
+      __threadfence();
+      __syncwarp();
+      if (!comes_last(first + 1, (parts + kStreamParts - 1) / kStreamParts)) continue;
+      sum(0, (parts + kStreamParts - 1) / kStreamParts, kStreamParts);
     }
     write(d);
   }

@@ -110,3 +110,21 @@ def test_edges_out_of_order_belong_to_nobody(at):
     with pytest.raises(RuntimeError, match="grouped"):
         ops.check_status()
     assert not any(bool(t.any()) for t in got)
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 128), (torch.bfloat16, 512)])
+def test_rows_of_any_number_of_stretches(dtype, D):
+    # one row among short ones, from one stretch of 32 to 88 edges to a hundred: parts are added up by 32s, a group of one among them
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    E, n_out = 100_000, 9001
+    x = torch.randint(-3, 4, (N_IN, D), device="cuda", generator=gen).to(dtype)
+    row = torch.randint(0, N_IN, (E,), device="cuda", generator=gen)
+    others = torch.randint(0, n_out, (E,), device="cuda", generator=gen)
+    turn = torch.randperm(E, device="cuda", generator=gen)
+    off = [torch.tensor([0, k], device="cuda") for k in (E, N_IN, n_out)]
+    rest = torch.zeros((n_out, D), device="cuda", dtype=torch.float64)
+    for n in range(40, 3400, 40):
+        col = others.clone()
+        col[turn[:n]] = 4000
+        want = rest.zero_().index_add_(0, col, x.double()[row])
+        assert torch.equal(ops.spmm_copy_u_sum(row, col, x, *off), want.to(dtype)), n
