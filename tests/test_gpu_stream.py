@@ -128,3 +128,34 @@ def test_rows_of_any_number_of_stretches(dtype, D):
         col[turn[:n]] = 4000
         want = rest.zero_().index_add_(0, col, x.double()[row])
         assert torch.equal(ops.spmm_copy_u_sum(row, col, x, *off), want.to(dtype)), n
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 72), (torch.float32, 256), (torch.bfloat16, 256), (torch.float16, 512)])
+@pytest.mark.parametrize("edges", [100_000, 210_000, 700_000])
+@pytest.mark.parametrize("shape", ["fixed", "ragged", "none"])
+@pytest.mark.parametrize("further", [0, 7])
+def test_segments_in_any_order(dtype, D, edges, shape, further):
+    """Three segments; edges of the same number each, of 0 to 60, or in no order. With further output rows behind the last segment's
+    nothing about the edges is known to the host, and the kernels decide."""
+    gen = torch.Generator(device="cuda").manual_seed(D + edges)
+    fanout = 13
+    parts, dst, src = [0], [0], [0]
+    rows, cols = [], []
+    for share in (0.5, 0.03, 0.47):
+        n_dst, n_src = int(edges * share / fanout) + 1, int(3001 * share)
+        n = torch.full((n_dst,), fanout, device="cuda") if shape == "fixed" else torch.randint(0, 61, (n_dst * fanout // 30 + 1,), device="cuda", generator=gen)
+        col = torch.arange(n.numel(), device="cuda").repeat_interleave(n)
+        if shape == "none":
+            col = col[torch.randperm(col.numel(), device="cuda", generator=gen)]
+        row = torch.randint(0, n_src, (col.numel(),), device="cuda", generator=gen)
+        rows.append(row), cols.append(col)
+        parts.append(parts[-1] + col.numel()), dst.append(dst[-1] + n.numel()), src.append(src[-1] + n_src)
+    row, col = torch.cat(rows), torch.cat(cols)
+    x = torch.randint(-3, 4, (src[-1], D), device="cuda", generator=gen).to(dtype)
+    at = torch.cat([c + o for c, o in zip(cols, dst)])
+    of = torch.cat([r + o for r, o in zip(rows, src)])
+    total = dst[-1] + further
+    want = torch.zeros((total, D), device="cuda", dtype=torch.float64).index_add_(0, at, x.double()[of]).to(dtype)
+    dev = lambda v: torch.tensor(v, device="cuda")
+    got = ops.spmm_copy_u_sum(row, col, x, dev(parts), dev(src), dev(dst + [total] if further else dst))
+    assert torch.equal(got, want)

@@ -11,13 +11,17 @@ PROGRAM = r"""
 #include <cstdio>
 #include "spmm_rows.cuh"
 int main() {
-  int op, slice, dim, esz, heads, grouped;
+  int op, slice, dim, esz, heads, mode;
   long long edges;
-  while (scanf("%d %d %d %d %d %lld %d", &op, &slice, &dim, &esz, &heads, &edges, &grouped) == 7)
-    printf("%d\n", (int)apt::stream_fits(op, slice, dim, esz, heads, edges, grouped != 0));
+  while (scanf("%d %d %d %d %d %lld %d", &op, &slice, &dim, &esz, &heads, &edges, &mode) == 7)
+    printf("%d\n", mode >= 10 ? (int)apt::stream_fits(op, slice, dim, esz, heads, edges, mode > 10)
+                              : apt::row_kernels(op, slice, dim, esz, heads, edges, mode));
 }
 """
 COPY_U, MUL_W, DOTS = 0, 4, 5
+DEVICE, FIXED, RANGES, ORDER = -1, 0, 1, 2
+SORTED, GROUPED = 10, 11          # the rule by itself
+ROWS, STREAM = 1, 2
 
 
 @pytest.fixture(scope="module")
@@ -39,7 +43,15 @@ def fits(tmp_path_factory):
 def test_slots_stay_within_31_bits(fits, op, heads):
     # a warp looks at slots behind the last one: the number of the last of these has to fit an int
     ahead = 159
-    got = fits(*[(op, 16, 128, 4, heads, e, g) for e in (1 << 30, 2 ** 31 - 2 - ahead, 2 ** 31 - 2) for g in (0, 1)])
+    got = fits(*[(op, 16, 128, 4, heads, e, g) for e in (1 << 30, 2 ** 31 - 2 - ahead, 2 ** 31 - 2) for g in (SORTED, GROUPED)])
     assert got[:2] == [1, 1] and got[4:] == [0, 0]
     # not further up than that, where it still fits
-    assert fits((op, 16, 128, 4, heads, 2 ** 31 - 8192, 0)) == [1]
+    assert fits((op, 16, 128, 4, heads, 2 ** 31 - 8192, SORTED)) == [1]
+
+
+@pytest.mark.parametrize("esz,dim", [(4, 72), (4, 128), (4, 256), (2, 256), (2, 512)])
+def test_sums_that_are_looked_over_on_the_device_go_where_the_others_go(fits, esz, dim):
+    for edges in (40_000, 98_303, 98_304, 135_000, 196_608, 450_000, 655_360, 1_013_760):
+        ask = lambda mode: fits((COPY_U, 16, dim, esz, 1, edges, mode))[0]
+        assert ask(FIXED) == ask(RANGES) in (ROWS, STREAM) and ask(ORDER) in (ROWS, STREAM)
+        assert ask(DEVICE) == ask(FIXED) | ask(ORDER), edges
