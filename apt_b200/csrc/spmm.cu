@@ -26,8 +26,7 @@ size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) 
   // rows of several items have more than kItemEdges
   const int64_t max_items = num_edges / kItemEdges + num_edges / kLongRowNarrow + 1;
   const int64_t max_parts = 2 * (num_edges / kItemEdges) + 1;
-  // partial sums: room for the longest rows of a power-law block at 256 columns; a row that finds none is one item
-  const int64_t part_floats = num_edges > kItemEdges ? std::min<int64_t>(6 * num_edges + 1024, (int64_t)16 << 20) : 1;
+  const int64_t part_floats = part_room(num_edges);
   size_t at = 0;
   auto take = [&](size_t bytes) {
     const size_t o = at;

@@ -199,6 +199,22 @@ inline StreamPlan stream_plan(int op, int64_t feat_dim, size_t esz, int heads) {
   p.shared = p.warps * p.warp_bytes;
   return p;
 }
+// Floats of scratch for partial sums. k_spmm_rows: room for the longest rows of a power-law block at 256 columns; a row that finds
+// none is one item. k_spmm_stream leaves up to two rows a warp, of up to 512 columns (12 to 15 MB): with six floats an edge as
+// its only room 135 000 edges of bf16 x 512 had 79 of 296 blocks.
+constexpr int kStreamMaxColumns = 512;
+inline int64_t part_room(int64_t num_edges) {
+  if (num_edges <= kItemEdges) return 1;
+  const int64_t room = std::min<int64_t>(6 * num_edges + 1024, (int64_t)16 << 20);
+  if (num_edges < kStreamMinOrdered) return room;
+  return std::max(room, 2 * kStreamMaxColumns * std::min<int64_t>(num_edges / kStreamStretch, kNumSMs * kStreamBlocks * stream_warps(true)));
+}
+// Blocks of `warps` warps: a stretch is at least kStreamStretch edges, and behind the sort long enough for the partial sums to find room.
+inline int stream_blocks(int64_t feat_dim, int64_t num_edges, int64_t part_floats, int warps, bool grouped) {
+  int64_t least = kStreamStretch;
+  if (!grouped) least = std::max(least, ceil_div((int64_t)2 * feat_dim * num_edges, part_floats));
+  return (int)std::min<int64_t>(std::max<int64_t>(1, num_edges / (least * warps)), kNumSMs * kStreamBlocks);
+}
 // `slice`: bytes of the widest access to rows and results. `grouped`: the edges are (kFixed, kRanges).
 inline bool stream_fits(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges, bool grouped) {
   const int64_t row = feat_dim * (int64_t)esz;

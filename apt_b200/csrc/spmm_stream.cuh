@@ -488,11 +488,8 @@ static int launch_stream(const RowArgs<T>& a, cudaStream_t s) {
     const int rc = pending_word(&pending);
     if (rc != APT_OK) return rc;
   }
-  // a warp's stretch: partial sums of split rows have to find room
-  int64_t least = kStreamStretch;
-  if (a.mode != kFixed && a.mode != kRanges) least = std::max(least, ceil_div((int64_t)2 * a.feat_dim * a.num_edges, a.ws.part_floats));
-  const int64_t want = std::max<int64_t>(1, a.num_edges / (least * plan.warps));
-  APT_FOLLOW((k_spmm_stream<T, OP, VPL>), (int)std::min<int64_t>(want, kNumSMs * kStreamBlocks), plan.warps * 32, plan.shared, s, a, plan,
+  const int blocks = stream_blocks(a.feat_dim, a.num_edges, a.ws.part_floats, plan.warps, a.mode == kFixed || a.mode == kRanges);
+  APT_FOLLOW((k_spmm_stream<T, OP, VPL>), blocks, plan.warps * 32, plan.shared, s, a, plan,
              bulk_wait_polls(), (volatile int32_t*)pending);
   return APT_OK;
 }

@@ -14,13 +14,14 @@ int main() {
   int op, slice, dim, esz, heads, mode;
   long long edges;
   while (scanf("%d %d %d %d %d %lld %d", &op, &slice, &dim, &esz, &heads, &edges, &mode) == 7)
-    printf("%d\n", mode >= 10 ? (int)apt::stream_fits(op, slice, dim, esz, heads, edges, mode > 10)
+    printf("%d\n", mode == 20 ? apt::stream_blocks(dim, edges, apt::part_room(edges), apt::stream_plan(op, dim, esz, heads).warps, false) : mode >= 10 ? (int)apt::stream_fits(op, slice, dim, esz, heads, edges, mode > 10)
                               : apt::row_kernels(op, slice, dim, esz, heads, edges, mode));
 }
 """
 COPY_U, MUL_W, DOTS = 0, 4, 5
 DEVICE, FIXED, RANGES, ORDER = -1, 0, 1, 2
 SORTED, GROUPED = 10, 11          # the rule by itself
+BLOCKS = 20
 ROWS, STREAM = 1, 2
 
 
@@ -55,3 +56,10 @@ def test_sums_that_are_looked_over_on_the_device_go_where_the_others_go(fits, es
         ask = lambda mode: fits((COPY_U, 16, dim, esz, 1, edges, mode))[0]
         assert ask(FIXED) == ask(RANGES) in (ROWS, STREAM) and ask(ORDER) in (ROWS, STREAM)
         assert ask(DEVICE) == ask(FIXED) | ask(ORDER), edges
+
+
+@pytest.mark.parametrize("esz,dim,warps", [(4, 128, 12), (4, 256, 10), (2, 256, 12), (2, 512, 10)])
+def test_partial_sums_find_room(fits, esz, dim, warps):
+    # stretches of 32 edges, on up to two blocks an SM, whatever the width
+    for edges in (98_304, 135_000, 196_608, 1_013_760):
+        assert fits((COPY_U, 16, dim, esz, 1, edges, BLOCKS)) == [min(296, edges // (32 * warps))]
