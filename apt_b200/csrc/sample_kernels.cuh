@@ -71,8 +71,13 @@ struct SampleInsert {
   int32_t* slot_of;   // [S + S * fanout] slot of every item
 };
 
+// Blocks an SM holds (36 registers), and up to four waves of them: draws and insertions take very different times, and where blocks
+// are launched for a bound of the seeds the empty ones cost little. Sampling and relabelling with eight blocks an SM in one wave
+// (which is one and a third) -> so, us: 200 000 x 10 184 -> 140, 100 000 x 25 150 -> 117, 43 000 x 20 64 -> 53, 12 342 (of 61 710) x 15 29.8 -> 28.3;
+// one wave of six 156, 131, 59, 28.8; eight waves 135, 114, 55, 28.7.
+constexpr int kSampleBlocks = 6, kSampleWaves = 4;
 template <int G, bool INSERT>
-__global__ void __launch_bounds__(256, 6)
+__global__ void __launch_bounds__(256, kSampleBlocks)
 sample_replace_kernel(const int64_t* __restrict__ seeds, int64_t num_seeds,
                       const int64_t* __restrict__ num_seeds_dev, int fanout, CscView g, uint32_t k0,
                       uint32_t k1, uint32_t call_id, const int64_t* __restrict__ call_base_dev,
