@@ -597,7 +597,7 @@ static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* 
   SpmmWs ws{};
   ws.range = g.range;
   const RowArgs<T> a{q.row, (const T*)q.ft, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, ws,
-                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u, false};
+                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u};
   ProfScope prof("gat_rows", s);
   return launch_spmm_rows<T>(kUMulW, a, s);
 }
@@ -624,7 +624,7 @@ static int gat_dots(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, 
     SpmmWs counts = ws.sort;
     counts.range = g.range;
     const RowArgs<T> a{q.row, (const T*)q.ft, nullptr, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, counts,
-                       nullptr, kRanges, 0, RowSplit{}, 0, g.none, q.status, q.col, (const T*)q.grad_out, ws.dots, (uint32_t)num_src, false};
+                       nullptr, kRanges, 0, RowSplit{}, 0, g.none, q.status, q.col, (const T*)q.grad_out, ws.dots, (uint32_t)num_src};
     return launch_spmm_rows<T>(kDots, a, s);
   }
   switch (slice) {
@@ -657,7 +657,7 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
 #undef APT_SCORES
   }
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, num_src, q.E, ws.sort,
-                     (T*)grad_ft, kOrder, 0, split, (int)dim, Verdict{}, q.status, nullptr, nullptr, nullptr, 0u, false};
+                     (T*)grad_ft, kOrder, 0, split, (int)dim, Verdict{}, q.status, nullptr, nullptr, nullptr, 0u};
   {
     ProfScope prof("spmm_rows", s);
     rc = launch_spmm_rows<T>(kUMulW, a, s);

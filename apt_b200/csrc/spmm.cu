@@ -490,7 +490,7 @@ static int run_rows(int op, const RowSplit& split, const int64_t* row, const int
                     int64_t edata_dim, int64_t feat_dim, SegTable st, int64_t num_rows, const SpmmWs& ws, int mode, int fixed,
                     void* out, cudaStream_t s) {
   const RowArgs<T> a{row, (const T*)in, (const T*)edata, edata_dim, feat_dim, st, num_rows, E, ws, (T*)out,
-                     mode, fixed, split, (int)feat_dim, Verdict{}, nullptr, col, nullptr, nullptr, 0u, false};
+                     mode, fixed, split, (int)feat_dim, Verdict{}, nullptr, col, nullptr, nullptr, 0u};
   ProfScope prof("spmm_rows", s);
   return launch_spmm_rows<T>(op, a, s);
 }

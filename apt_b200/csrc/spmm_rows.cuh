@@ -166,7 +166,6 @@ struct RowArgs {
   const T* own;            // the output rows' own
   float* dots;             // [E][heads]
   uint32_t num_in;         // input rows; ws.cnt and ws.rank count their edges on the way
-  bool shared;             // k_spmm_stream and k_spmm_rows are both launched, for sorted edges and for grouped ones
 };
 
 // ---- which rows k_spmm_stream takes (the figures are there) ------------------------------------
@@ -216,6 +215,8 @@ inline int stream_blocks(int64_t feat_dim, int64_t num_edges, int64_t part_float
   return (int)std::min<int64_t>(std::max<int64_t>(1, num_edges / (least * warps)), kNumSMs * kStreamBlocks);
 }
 // `slice`: bytes of the widest access to rows and results. `grouped`: the edges are (kFixed, kRanges).
+// Where nobody knows (kDevice) the lines of edges in no order hold for grouped ones as well: with a launch of either kernel, of which one
+// returns at once, every such call paid 2 us and 30 000 x 15 grouped edges of fp32 x 128 took 57 us instead of 50 (row kernel alone 54).
 inline bool stream_fits(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges, bool grouped) {
   const int64_t row = feat_dim * (int64_t)esz;
   if (slice != 16 || row < kStreamMinSlices * 16 || row > 64 * 16 || num_edges > kStreamMaxEdges) return false;
@@ -225,16 +226,6 @@ inline bool stream_fits(int op, int slice, int64_t feat_dim, size_t esz, int hea
   if (op != kDots) return op == kCopyU || op == kUMulW;
   const int lph = stream_lph(feat_dim, esz, heads);
   return lph >= 4 && lph * heads <= 64;
-}
-// The kernels that sums are launched with. kDevice: where the lines of sorted and of grouped edges differ both are, and the one
-// that the edges are not for returns at once. (Grouped edges by the stream alone, from the line of sorted ones on: fp32 x 256, 9000 x 15
-// edges, 46 -> 54 us, bf16 x 512 49 -> 61.)
-enum { kByRows = 1, kByStream = 2 };
-inline int row_kernels(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges, int mode) {
-  const bool grouped = stream_fits(op, slice, feat_dim, esz, heads, num_edges, true);
-  const bool sorted = stream_fits(op, slice, feat_dim, esz, heads, num_edges, false);
-  if (mode == kDevice && grouped != sorted) return kByRows | kByStream;
-  return (mode == kFixed || mode == kRanges ? grouped : sorted) ? kByStream : kByRows;
 }
 inline OrderKind order_kind(int op, int slice, int64_t feat_dim, size_t esz, int heads, int64_t num_edges) {
   if (!stream_fits(op, slice, feat_dim, esz, heads, num_edges, false)) return kByEdge;
@@ -337,7 +328,6 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
     mode = probe_mode(w);
     fixed = mode == kFixed ? (int)(a.num_edges / a.num_rows) : 0;
   }
-  if (a.shared && mode == kOrder) return;
   if (mode != kOrder) {
     for (int t = threadIdx.x; t <= a.st.nseg; t += blockDim.x) {
       // no table: one segment whose rows start at 0
@@ -582,31 +572,19 @@ static int launch_rows_vpl(const RowArgs<T>& a, cudaStream_t s) {
 }
 
 template <typename T, int OP>
-static int launch_rows_slice(const RowArgs<T>& a, cudaStream_t s) {
+static int launch_stream(const RowArgs<T>& a, cudaStream_t s);     // spmm_stream.cuh
+
+template <typename T, int OP>
+static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
+  if constexpr (OP == kCopyU || OP == kUMulW) {
+    if (stream_fits(OP, a.split.ve * (int)sizeof(T), a.feat_dim, sizeof(T), OP == kCopyU ? 1 : (int)a.edata_dim, a.num_edges, a.mode == kFixed || a.mode == kRanges)) return launch_stream<T, OP>(a, s);
+  }
   switch (a.split.ve * (int)sizeof(T)) {
     case 16: return launch_rows_vpl<T, 16 / sizeof(T), OP>(a, s);
     case 8: return launch_rows_vpl<T, 8 / sizeof(T), OP>(a, s);
     case 4: return launch_rows_vpl<T, 4 / sizeof(T), OP>(a, s);
     default: return launch_rows_vpl<T, 1, OP>(a, s);
   }
-}
-
-template <typename T, int OP>
-static int launch_stream(const RowArgs<T>& a, cudaStream_t s);     // spmm_stream.cuh
-
-template <typename T, int OP>
-static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
-  if constexpr (OP == kCopyU || OP == kUMulW) {
-    const int kernels = row_kernels(OP, a.split.ve * (int)sizeof(T), a.feat_dim, sizeof(T), OP == kCopyU ? 1 : (int)a.edata_dim, a.num_edges, a.mode);
-    if (kernels & kByStream) {
-      RowArgs<T> b = a;
-      b.shared = (kernels & kByRows) != 0;
-      const int rc = launch_stream<T, OP>(b, s);
-      if (rc != APT_OK || !b.shared) return rc;
-      return launch_rows_slice<T, OP>(b, s);
-    }
-  }
-  return launch_rows_slice<T, OP>(a, s);
 }
 
 // One translation unit per element type (spmm_f32.cu, spmm_bf16.cu, spmm_f16.cu) holds these.

@@ -92,7 +92,6 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
     mode = probe_mode(w);
     fixed = mode == kFixed ? (int)(a.num_edges / a.num_rows) : 0;
   }
-  if (a.shared && mode != kOrder) return;
   for (int t = threadIdx.x; t <= a.st.nseg; t += blockDim.x) {
     // no table: one segment whose rows start at 0
     coo[t] = a.st.coo_off ? a.st.coo_off[t] : 0;

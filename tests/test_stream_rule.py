@@ -11,18 +11,15 @@ PROGRAM = r"""
 #include <cstdio>
 #include "spmm_rows.cuh"
 int main() {
-  int op, slice, dim, esz, heads, mode;
+  int op, slice, dim, esz, heads, what;
   long long edges;
-  while (scanf("%d %d %d %d %d %lld %d", &op, &slice, &dim, &esz, &heads, &edges, &mode) == 7)
-    printf("%d\n", mode == 20 ? apt::stream_blocks(dim, edges, apt::part_room(edges), apt::stream_plan(op, dim, esz, heads).warps, false) : mode >= 10 ? (int)apt::stream_fits(op, slice, dim, esz, heads, edges, mode > 10)
-                              : apt::row_kernels(op, slice, dim, esz, heads, edges, mode));
+  while (scanf("%d %d %d %d %d %lld %d", &op, &slice, &dim, &esz, &heads, &edges, &what) == 7)
+    printf("%d\n", what == 20 ? apt::stream_blocks(dim, edges, apt::part_room(edges), apt::stream_plan(op, dim, esz, heads).warps, false)
+                              : (int)apt::stream_fits(op, slice, dim, esz, heads, edges, what != 0));
 }
 """
 COPY_U, MUL_W, DOTS = 0, 4, 5
-DEVICE, FIXED, RANGES, ORDER = -1, 0, 1, 2
-SORTED, GROUPED = 10, 11          # the rule by itself
-BLOCKS = 20
-ROWS, STREAM = 1, 2
+SORTED, GROUPED, BLOCKS = 0, 1, 20
 
 
 @pytest.fixture(scope="module")
@@ -48,14 +45,6 @@ def test_slots_stay_within_31_bits(fits, op, heads):
     assert got[:2] == [1, 1] and got[4:] == [0, 0]
     # not further up than that, where it still fits
     assert fits((op, 16, 128, 4, heads, 2 ** 31 - 8192, SORTED)) == [1]
-
-
-@pytest.mark.parametrize("esz,dim", [(4, 72), (4, 128), (4, 256), (2, 256), (2, 512)])
-def test_sums_that_are_looked_over_on_the_device_go_where_the_others_go(fits, esz, dim):
-    for edges in (40_000, 98_303, 98_304, 135_000, 196_608, 450_000, 655_360, 1_013_760):
-        ask = lambda mode: fits((COPY_U, 16, dim, esz, 1, edges, mode))[0]
-        assert ask(FIXED) == ask(RANGES) in (ROWS, STREAM) and ask(ORDER) in (ROWS, STREAM)
-        assert ask(DEVICE) == ask(FIXED) | ask(ORDER), edges
 
 
 @pytest.mark.parametrize("esz,dim,warps", [(4, 128, 12), (4, 256, 10), (2, 256, 12), (2, 512, 10)])
