@@ -802,10 +802,11 @@ k_gat_alone(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* 
 // launch. 30 000 destinations of 3 / 10 / 25 edges, with the weights apart -> here, us: fp32 x 32 16 / 33 / 47 -> 12 / 18 / 33,
 // bf16 8 x 8 22 / 37 / 59 -> 12 / 20 / 37, fp32 4 x 16 23 / 36 / 57 -> 16 / 27 / 49. Wider rows and other slices gain by the weights
 // apart, against one such kernel: bf16 4 x 64 35 / 45 / 67 -> 27 / 37 / 72, fp16 2 x 10 27 / 41 / 79 -> 18 / 27 / 45.
-// (Five blocks an SM keep the compiler at 48 registers; left alone it takes 40 for fp32 and has fewer loads in flight: fp32 8 x 8, 30 000
-// destinations of 0 to 30 edges 51 -> 45 us, 1 x 32 36.4 -> 31.8, one of 20 000 edges 10.0 -> 7.5 ms.)
+// (For fp32 the compiler takes 40 registers when left alone and has fewer loads in flight; five blocks an SM keep it at 48: 8 x 8, 30 000
+// destinations of 0 to 30 edges 51 -> 45 us, 1 x 32 36.4 -> 31.7, one of 20 000 edges 10.0 -> 7.5 ms. 16-bit types have 47 registers either way, but
+// lose by the bound: bf16 1 x 16 20.4 -> 23.9, 12 x 8 50.6 -> 54.2.)
 template <typename T>
-__global__ void __launch_bounds__(256, 5)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 0)
 k_gat_narrow(const int64_t* __restrict__ row, const T* __restrict__ ft, const T* __restrict__ el, const T* __restrict__ er, int num_heads,
              int head_dim, float slope, int64_t num_dst, const int2* __restrict__ range, const Verdict none,
              T* __restrict__ out, T* __restrict__ attn, int lpe) {
