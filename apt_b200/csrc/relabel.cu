@@ -429,7 +429,7 @@ extern "C" int apt_sample_relabel_block(const int64_t* seeds, int64_t num_seeds,
     ProfScope prof("sample", s);
 #define APT_SAMPLE_INSERT(G)                                                                         \
   do {                                                                                               \
-    const int grid = wave_grid(ceil_div(num_seeds, 256 / G), kSampleBlocks, kSampleWaves);                    \
+    const int grid = wave_grid(ceil_div(num_seeds, 256 / G), kSampleBlocks, num_seeds_dev ? 1 : kSampleWaves);                    \
     if (small)                                                                                       \
       APT_FOLLOW((sample_replace_kernel<G, false>), grid, 256, 0, s, seeds, num_seeds,               \
                  num_seeds_dev, fanout, g, k0, k1, call_id, call_id_base_dev, nbr_buf, status_word,  \

@@ -105,7 +105,7 @@ extern "C" int apt_sample_csc_fanout(
   }
 #define APT_SAMPLE_G(G)                                                        \
   do {                                                                         \
-    const int grid = wave_grid(ceil_div(num_seeds, 256 / G), kSampleBlocks, kSampleWaves); \
+    const int grid = wave_grid(ceil_div(num_seeds, 256 / G), kSampleBlocks, num_seeds_dev ? 1 : kSampleWaves); \
     APT_FOLLOW((sample_replace_kernel<G, false>), grid, 256, 0, s, seeds, num_seeds,    \
                num_seeds_dev, fanout, g, k0, k1, call_id, call_id_base_dev,    \
                out_neighbors, status_word, SampleInsert{nullptr, nullptr});    \

@@ -71,10 +71,11 @@ struct SampleInsert {
   int32_t* slot_of;   // [S + S * fanout] slot of every item
 };
 
-// Blocks an SM holds (36 registers), and up to four waves of them: draws and insertions take very different times, and where blocks
-// are launched for a bound of the seeds the empty ones cost little. Sampling and relabelling with eight blocks an SM in one wave
-// (which is one and a third) -> so, us: 200 000 x 10 184 -> 140, 100 000 x 25 150 -> 117, 43 000 x 20 64 -> 53, 12 342 (of 61 710) x 15 29.8 -> 28.3;
-// one wave of six 156, 131, 59, 28.8; eight waves 135, 114, 55, 28.7.
+// Blocks an SM holds (36 registers), and waves of them where the number of seeds is known: draws and insertions take very different
+// times, and with a share of a whole wave each the slowest block decides. Where the seeds are counted on the device their number is
+// a bound, most blocks of which may be empty, and other kernels run beside: one wave (an epoch's mini-batch 128.5 us against 130). Sampling and
+// relabelling with eight blocks an SM, which is one wave and a third -> four waves of six | one of six, us: 200 000 x 10 184 -> 140 | 156,
+// 100 000 x 25 150 -> 117 | 131, 43 000 x 20 64 -> 53 | 59, 1 000 000 x 10 1033 -> 815 | 930, 12 342 (of 61 710) x 15 29.8 -> 28.3 | 28.8.
 constexpr int kSampleBlocks = 6, kSampleWaves = 4;
 template <int G, bool INSERT>
 __global__ void __launch_bounds__(256, kSampleBlocks)
