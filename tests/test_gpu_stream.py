@@ -3,8 +3,9 @@ and rows of many stretches, and the lanes that a row does not fill.
 
 Bounds: sums of small whole numbers are exact in fp32, and a 16-bit result is one rounding of them. The attention layer is
 held to the 2-norm of the fp64 results: about 15 fp32 terms a sum (2e-6), and 2^-9 or 2^-12 for a rounding to 16 bits. The
-gradient of el is added up in fp32 one edge after another: n edges of a source are off by about root(n) 2^-25 of it, and the
-first source here has 393 000 / 9001^(1/4) = 40 400, which is 6e-6."""
+gradient of el is added up in fp32 one edge after another, in the order of arrival: n additions, each off by up to 2^-24 of the sum
+so far (1 / sqrt(3) of that as a standard deviation), are off by sqrt(n / 3) 2^-24 of the largest sum on the way. The first source here
+has 393 000 / 9001^(1/4) = 40 400 edges, which is 6.9e-6; three standard deviations are 2.1e-5 (seen: up to 7.2e-6 in 250 runs)."""
 import pytest
 import torch
 
@@ -78,7 +79,7 @@ def test_attention(dtype, H, D, ragged):
     out = ops.GATEdgeSoftmaxSum.apply(row, col, *leaves, n_dst, 0.2)
     bound = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dtype]
     for k, (got, ref) in enumerate(zip((out,) + torch.autograd.grad(out, leaves, g), want)):
-        assert float((got.double() - ref).norm() / ref.norm()) <= (max(bound, 6e-6) if k == 2 else bound)
+        assert float((got.double() - ref).norm() / ref.norm()) <= (max(bound, 2.1e-5) if k == 2 else bound)
 
 
 def test_dots_beside_infinite_features():
