@@ -130,6 +130,22 @@ __device__ __forceinline__ Heads<NH> load_scores(const T* p) {         // the sa
   for (int h = 0; h < NH; ++h) r.v[h] = Elem<T>::to_f(w.v[h]);
   return r;
 }
+// What a group of lanes works on: destination i with its NH heads, or, where there are more heads (SIDE), the i-th block of NH of them,
+// those of a destination one after another.
+template <int NH, bool SIDE>
+struct HeadBlocks {
+  int64_t count;
+  int per_row;
+  __device__ __forceinline__ HeadBlocks(int64_t num_dst, int num_heads) : count(num_dst), per_row(1) {
+    if (SIDE) per_row = num_heads / NH, count *= per_row;
+  }
+  __device__ __forceinline__ void at(int64_t i, int64_t& d, int& h0) const {
+    d = i, h0 = 0;
+    if (!SIDE) return;
+    d = count >> 32 ? i / per_row : (int64_t)((uint32_t)i / (uint32_t)per_row);
+    h0 = (int)(i - d * per_row) * NH;
+  }
+};
 template <int W>
 __device__ __forceinline__ float lanes_sum(float v) {
 #pragma unroll
@@ -138,106 +154,125 @@ __device__ __forceinline__ float lanes_sum(float v) {
 }
 
 // Attention weights.
-template <typename T, int W, int NH>
+template <typename T, int W, int NH, bool SIDE>
 __global__ void __launch_bounds__(256)
 k_gat_weights(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
-              int64_t num_dst, const int2* __restrict__ range, const Verdict none, float* __restrict__ weight,
+              int64_t num_dst, const int2* __restrict__ range, const Verdict none, float* weight,
               T* __restrict__ attn, int masked) {
   wait_for_previous();
   constexpr int K = kGatEdges;
   if (any_found(none)) return;
   const int64_t stride = (int64_t)gridDim.x * (256 / W);
   const int part = threadIdx.x & (W - 1);
-  // (all lanes of a warp stay: groups behind the last destination have no edges)
-  for (int64_t d0 = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; d0 < num_dst; d0 += stride) {
-    const int64_t d = d0 + (threadIdx.x & 31) / W;
-    const bool there = d < num_dst;
+  // (all lanes of a warp stay: groups behind the last one have no edges)
+  const HeadBlocks<NH, SIDE> blocks(num_dst, num_heads);
+  for (int64_t i0 = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; i0 < blocks.count; i0 += stride) {
+    const int64_t i = i0 + (threadIdx.x & 31) / W;
+    const bool there = i < blocks.count;
+    int64_t d;
+    int h0;
+    blocks.at(i, d, h0);
     const int2 r = there ? range[d] : make_int2(0, 0);
     const int deg = r.y - r.x;
     const bool few = deg <= K * W;
     uint32_t src[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) src[k] = few && part + k * W < deg ? (uint32_t)row[r.x + part + k * W] : 0u;
-#pragma unroll 1
-    for (int h0 = 0; h0 < num_heads; h0 += NH) {
-      Heads<NH> bias, s[K];
-      float most[NH], sum[NH], inv[NH];
-      bool zero[NH];
+    Heads<NH> bias, s[K];
+    float most[NH], sum[NH], inv[NH];
+    bool zero[NH];
 #pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        bias.v[h] = there ? Elem<T>::to_f(er[d * num_heads + h0 + h]) : 0.f;
-        most[h] = -INFINITY;
-        sum[h] = 0.f;
+    for (int h = 0; h < NH; ++h) {
+      bias.v[h] = there ? Elem<T>::to_f(er[d * num_heads + h0 + h]) : 0.f;
+      most[h] = -INFINITY;
+      sum[h] = 0.f;
+    }
+    auto scores = [&](int64_t from) {
+      Heads<NH> x = load_scores<T, NH>(el + from * num_heads + h0);
+#pragma unroll
+      for (int h = 0; h < NH; ++h) x.v[h] = leaky(x.v[h] + bias.v[h], slope);
+      return x;
+    };
+    // (plain accesses: what a lane reads here it has written itself)
+    auto keep = [&](int e, const Heads<NH>& x) {
+      Pack<float, NH> w;
+#pragma unroll
+      for (int h = 0; h < NH; ++h) w.v[h] = x.v[h];
+      store_pack<float, NH>(weight + (int64_t)e * num_heads + h0, w);
+    };
+    auto kept = [&](int e) {
+      const Pack<float, NH> w = *(const Pack<float, NH>*)(weight + (int64_t)e * num_heads + h0);
+      Heads<NH> x;
+#pragma unroll
+      for (int h = 0; h < NH; ++h) x.v[h] = w.v[h];
+      return x;
+    };
+    if (few) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (part + k * W < deg) {
+          s[k] = scores(src[k]);
+#pragma unroll
+          for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], s[k].v[h]);
+        }
+    } else {
+      // the scores wait where the weights will be: a source's is fetched once
+#pragma unroll 2
+      for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+        const Heads<NH> x = scores(row[r.x + j]);
+#pragma unroll
+        for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], x.v[h]);
+        keep(r.x + j, x);
       }
-      auto scores = [&](int64_t from) {
-        Heads<NH> x = load_scores<T, NH>(el + from * num_heads + h0);
+    }
 #pragma unroll
-        for (int h = 0; h < NH; ++h) x.v[h] = leaky(x.v[h] + bias.v[h], slope);
-        return x;
-      };
-      if (few) {
+    for (int h = 0; h < NH; ++h)
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-          if (part + k * W < deg) {
-            s[k] = scores(src[k]);
+      for (int o = 1; o < W; o <<= 1) most[h] = fmaxf(most[h], __shfl_xor_sync(0xffffffffu, most[h], o));
+    if (few) {
 #pragma unroll
-            for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], s[k].v[h]);
+      for (int k = 0; k < K; ++k)
+        if (part + k * W < deg)
+#pragma unroll
+          for (int h = 0; h < NH; ++h) {
+            s[k].v[h] = expf(s[k].v[h] - most[h]);
+            sum[h] += s[k].v[h];
           }
-      } else {
-        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
-          const Heads<NH> x = scores(row[r.x + j]);
+    } else {
+#pragma unroll 2
+      for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+        Heads<NH> x = kept(r.x + j);
 #pragma unroll
-          for (int h = 0; h < NH; ++h) most[h] = fmaxf(most[h], x.v[h]);
+        for (int h = 0; h < NH; ++h) {
+          x.v[h] = expf(x.v[h] - most[h]);
+          sum[h] += x.v[h];
         }
+        keep(r.x + j, x);
       }
+    }
 #pragma unroll
-      for (int h = 0; h < NH; ++h)
+    for (int h = 0; h < NH; ++h) {
+      sum[h] = lanes_sum<W>(sum[h]);
+      inv[h] = sum[h] > 0.f ? 1.f / sum[h] : 0.f;
+      zero[h] = !(sum[h] > 0.f) && deg <= masked;
+    }
+    auto put = [&](int e, const Heads<NH>& p) {
+      const int64_t o = (int64_t)e * num_heads + h0;
+      Pack<float, NH> w;
 #pragma unroll
-        for (int o = 1; o < W; o <<= 1) most[h] = fmaxf(most[h], __shfl_xor_sync(0xffffffffu, most[h], o));
-      if (few) {
+      for (int h = 0; h < NH; ++h) w.v[h] = zero[h] ? 0.f : p.v[h] * inv[h];
+      store_pack<float, NH>(weight + o, w);
+      if (attn)
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-          if (part + k * W < deg)
+        for (int h = 0; h < NH; ++h) attn[o + h] = Elem<T>::from_f(w.v[h]);
+    };
+    if (few) {
 #pragma unroll
-            for (int h = 0; h < NH; ++h) {
-              s[k].v[h] = expf(s[k].v[h] - most[h]);
-              sum[h] += s[k].v[h];
-            }
-      } else {
-        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
-          const Heads<NH> x = scores(row[r.x + j]);
-#pragma unroll
-          for (int h = 0; h < NH; ++h) sum[h] += expf(x.v[h] - most[h]);
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        sum[h] = lanes_sum<W>(sum[h]);
-        inv[h] = sum[h] > 0.f ? 1.f / sum[h] : 0.f;
-        zero[h] = !(sum[h] > 0.f) && deg <= masked;
-      }
-      auto put = [&](int e, const Heads<NH>& p) {
-        const int64_t o = (int64_t)e * num_heads + h0;
-        Pack<float, NH> w;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) w.v[h] = zero[h] ? 0.f : p.v[h] * inv[h];
-        store_pack<float, NH>(weight + o, w);
-        if (attn)
-#pragma unroll
-          for (int h = 0; h < NH; ++h) attn[o + h] = Elem<T>::from_f(w.v[h]);
-      };
-      if (few) {
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-          if (part + k * W < deg) put(r.x + part + k * W, s[k]);
-      } else {
-        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
-          Heads<NH> x = scores(row[r.x + j]);
-#pragma unroll
-          for (int h = 0; h < NH; ++h) x.v[h] = expf(x.v[h] - most[h]);
-          put(r.x + j, x);
-        }
-      }
+      for (int k = 0; k < K; ++k)
+        if (part + k * W < deg) put(r.x + part + k * W, s[k]);
+    } else {
+#pragma unroll 2
+      for (uint32_t j = part; j < (uint32_t)deg; j += W) put(r.x + j, kept(r.x + j));
     }
   }
 }
@@ -352,7 +387,7 @@ __device__ __forceinline__ void add_heads(float* p, const Heads<NH>& v) {
 }
 
 // Score gradients, added to sums[spread(source)][head], and the destination's edges to their places in the order by source.
-template <typename T, int W, int NH>
+template <typename T, int W, int NH, bool SIDE>
 __global__ void __launch_bounds__(256)
 k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T* __restrict__ er, int num_heads, float slope,
              int64_t num_src, int64_t num_dst, int64_t E, const int2* __restrict__ range, const Verdict none,
@@ -365,9 +400,13 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
     for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < E * num_heads; o += (int64_t)gridDim.x * blockDim.x) weight[o] = 0.f;
   const int64_t stride = (int64_t)gridDim.x * (256 / W);
   const int part = threadIdx.x & (W - 1);
-  for (int64_t d0 = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; d0 < num_dst; d0 += stride) {
-    const int64_t d = d0 + (threadIdx.x & 31) / W;
-    const bool there = d < num_dst;
+  const HeadBlocks<NH, SIDE> blocks(num_dst, num_heads);
+  for (int64_t i0 = ((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) / W; i0 < blocks.count; i0 += stride) {
+    const int64_t i = i0 + (threadIdx.x & 31) / W;
+    const bool there = i < blocks.count;
+    int64_t d;
+    int h0;
+    blocks.at(i, d, h0);
     const int2 r = there && !empty ? range[d] : make_int2(0, 0);
     const int deg = r.y - r.x;
     const bool few = deg <= K * W;
@@ -385,74 +424,72 @@ k_gat_scores(const int64_t* __restrict__ row, const T* __restrict__ el, const T*
     for (int k = 0; k < K; ++k) {
       const bool mine = few && part + k * W < deg;
       src[k] = mine ? row[r.x + part + k * W] : 0;
-      place[k] = mine ? place_of(r.x + part + k * W) : kNoRank;
+      place[k] = mine && h0 == 0 ? place_of(r.x + part + k * W) : kNoRank;
     }
-#pragma unroll 1
-    for (int h0 = 0; h0 < num_heads; h0 += NH) {
-      Heads<NH> bias, w[K], dot[K], x[K];
-      float t[NH], ger[NH];
+    Heads<NH> bias, w[K], dot[K], x[K];
+    float t[NH], ger[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      bias.v[h] = there ? Elem<T>::to_f(er[d * num_heads + h0 + h]) : 0.f;
+      t[h] = ger[h] = 0.f;
+    }
+    auto fetch = [&](int e, Heads<NH>& a, Heads<NH>& b) {
+      a = load_heads<NH>(weight + (int64_t)e * num_heads + h0);
+      b = load_heads<NH>(dots + (int64_t)e * num_heads + h0);
+    };
+    if (few) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (part + k * W < deg) {
+          fetch(r.x + part + k * W, w[k], dot[k]);
+          x[k] = load_scores<T, NH>(el + src[k] * num_heads + h0);
+        }
+      // (the lanes of the first heads have the places)
+#pragma unroll
+      for (int k = 0; k < K; ++k) put(r.x + part + k * W, src[k], place[k]);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (part + k * W < deg)
+#pragma unroll
+          for (int h = 0; h < NH; ++h) t[h] += w[k].v[h] * dot[k].v[h];
+    } else {
+#pragma unroll 2
+      for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+        Heads<NH> a, b;
+        fetch(r.x + j, a, b);
+#pragma unroll
+        for (int h = 0; h < NH; ++h) t[h] += a.v[h] * b.v[h];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h) t[h] = lanes_sum<W>(t[h]);
+    auto grad = [&](int64_t from, const Heads<NH>& a, const Heads<NH>& b, const Heads<NH>& c) {
+      Heads<NH> gs;
 #pragma unroll
       for (int h = 0; h < NH; ++h) {
-        bias.v[h] = there ? Elem<T>::to_f(er[d * num_heads + h0 + h]) : 0.f;
-        t[h] = ger[h] = 0.f;
+        gs.v[h] = a.v[h] * (b.v[h] - t[h]) * (c.v[h] + bias.v[h] > 0.f ? 1.f : slope);
+        ger[h] += gs.v[h];
       }
-      auto fetch = [&](int e, Heads<NH>& a, Heads<NH>& b) {
-        a = load_heads<NH>(weight + (int64_t)e * num_heads + h0);
-        b = load_heads<NH>(dots + (int64_t)e * num_heads + h0);
-      };
-      if (few) {
+      if ((uint64_t)from < (uint64_t)num_src) add_heads<NH>(sums + (int64_t)spread((uint32_t)from) * num_heads + h0, gs);
+    };
+    if (few) {
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-          if (part + k * W < deg) {
-            fetch(r.x + part + k * W, w[k], dot[k]);
-            x[k] = load_scores<T, NH>(el + src[k] * num_heads + h0);
-          }
-        if (h0 == 0)
-#pragma unroll
-          for (int k = 0; k < K; ++k) put(r.x + part + k * W, src[k], place[k]);
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-          if (part + k * W < deg)
-#pragma unroll
-            for (int h = 0; h < NH; ++h) t[h] += w[k].v[h] * dot[k].v[h];
-      } else {
-        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
-          const int e = r.x + j;
-          fetch(e, w[0], dot[0]);
-#pragma unroll
-          for (int h = 0; h < NH; ++h) t[h] += w[0].v[h] * dot[0].v[h];
-        }
+      for (int k = 0; k < K; ++k)
+        if (part + k * W < deg) grad(src[k], w[k], dot[k], x[k]);
+    } else {
+      for (uint32_t j = part; j < (uint32_t)deg; j += W) {
+        const int e = r.x + j;
+        const int64_t from = row[e];
+        fetch(e, w[0], dot[0]);
+        x[0] = load_scores<T, NH>(el + from * num_heads + h0);
+        if (h0 == 0) put(e, from, place_of(e));
+        grad(from, w[0], dot[0], x[0]);
       }
+    }
 #pragma unroll
-      for (int h = 0; h < NH; ++h) t[h] = lanes_sum<W>(t[h]);
-      auto grad = [&](int64_t from, const Heads<NH>& a, const Heads<NH>& b, const Heads<NH>& c) {
-        Heads<NH> gs;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {
-          gs.v[h] = a.v[h] * (b.v[h] - t[h]) * (c.v[h] + bias.v[h] > 0.f ? 1.f : slope);
-          ger[h] += gs.v[h];
-        }
-        if ((uint64_t)from < (uint64_t)num_src) add_heads<NH>(sums + (int64_t)spread((uint32_t)from) * num_heads + h0, gs);
-      };
-      if (few) {
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-          if (part + k * W < deg) grad(src[k], w[k], dot[k], x[k]);
-      } else {
-        for (uint32_t j = part; j < (uint32_t)deg; j += W) {
-          const int e = r.x + j;
-          const int64_t from = row[e];
-          fetch(e, w[0], dot[0]);
-          x[0] = load_scores<T, NH>(el + from * num_heads + h0);
-          if (h0 == 0) put(e, from, place_of(e));
-          grad(from, w[0], dot[0], x[0]);
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        ger[h] = lanes_sum<W>(ger[h]);
-        if (there && part == 0) grad_er[d * num_heads + h0 + h] = Elem<T>::from_f(ger[h]);
-      }
+    for (int h = 0; h < NH; ++h) {
+      ger[h] = lanes_sum<W>(ger[h]);
+      if (there && part == 0) grad_er[d * num_heads + h0 + h] = Elem<T>::from_f(ger[h]);
     }
   }
 }
@@ -544,26 +581,34 @@ static int gat_ranges(const GatProblem& q, const GatEdges& g, cudaStream_t s) {
   return APT_OK;
 }
 
-// Lanes to a destination: as many as hold a mean one's edges. Heads at a time: as many as there are, if el can be read so.
+// Lanes to a destination: as many as hold a mean one's edges. Heads at a time: as many as there are, if el can be read so; where that leaves
+// several blocks of them these are worked on side by side. One after another, which waits for as many rounds of latency, against
+// that, us: forward of bf16 16 x 16, 30 000 destinations of 0 to 30 edges 105 -> 83, backward of fp32 5 x 4 152 -> 118, 3 x 16 142 -> 131;
+// 67 584 x 15 edges 143 -> 149, 215 -> 183, 228 -> 221.
+#define APT_GAT_SIDE(W, NH, H, RUN)  \
+  do {                               \
+    if ((H) == (NH)) RUN(W, NH, false); \
+    else RUN(W, NH, true);           \
+  } while (0)
 #define APT_GAT_LANES(q, RUN)                                                             \
   do {                                                                                    \
     const int lanes__ = pow2_ge(ceil_div(ceil_div(q.E, q.num_dst), kGatEdges)), nh__ = gat_heads(q, sizeof(T)); \
     if (lanes__ <= 4) {                                                                   \
-      if (nh__ == 4) RUN(4, 4);                                                           \
-      else if (nh__ == 2) RUN(4, 2);                                                      \
-      else RUN(4, 1);                                                                     \
+      if (nh__ == 4) APT_GAT_SIDE(4, 4, q.H, RUN);                                        \
+      else if (nh__ == 2) APT_GAT_SIDE(4, 2, q.H, RUN);                                   \
+      else APT_GAT_SIDE(4, 1, q.H, RUN);                                                  \
     } else if (lanes__ <= 8) {                                                            \
-      if (nh__ == 4) RUN(8, 4);                                                           \
-      else if (nh__ == 2) RUN(8, 2);                                                      \
-      else RUN(8, 1);                                                                     \
+      if (nh__ == 4) APT_GAT_SIDE(8, 4, q.H, RUN);                                        \
+      else if (nh__ == 2) APT_GAT_SIDE(8, 2, q.H, RUN);                                   \
+      else APT_GAT_SIDE(8, 1, q.H, RUN);                                                  \
     } else if (lanes__ <= 16) {                                                           \
-      if (nh__ == 4) RUN(16, 4);                                                          \
-      else if (nh__ == 2) RUN(16, 2);                                                     \
-      else RUN(16, 1);                                                                    \
+      if (nh__ == 4) APT_GAT_SIDE(16, 4, q.H, RUN);                                       \
+      else if (nh__ == 2) APT_GAT_SIDE(16, 2, q.H, RUN);                                  \
+      else APT_GAT_SIDE(16, 1, q.H, RUN);                                                 \
     } else {                                                                              \
-      if (nh__ == 4) RUN(32, 4);                                                          \
-      else if (nh__ == 2) RUN(32, 2);                                                     \
-      else RUN(32, 1);                                                                    \
+      if (nh__ == 4) APT_GAT_SIDE(32, 4, q.H, RUN);                                       \
+      else if (nh__ == 2) APT_GAT_SIDE(32, 2, q.H, RUN);                                  \
+      else APT_GAT_SIDE(32, 1, q.H, RUN);                                                 \
     }                                                                                     \
   } while (0);
 static int gat_heads(const GatProblem& q, size_t esz) {
@@ -579,8 +624,8 @@ static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaS
   if (rc != APT_OK) return rc;
   ProfScope prof("gat_rows", s);
   const int masked = masked_edges(q.H, q.Dh, sizeof(T), (uintptr_t)q.ft);
-#define APT_WEIGHTS(W, NH)                                                                                                   \
-  APT_FOLLOW((k_gat_weights<T, W, NH>), wave_grid(ceil_div(q.num_dst * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
+#define APT_WEIGHTS(W, NH, SIDE)                                                                                                   \
+  APT_FOLLOW((k_gat_weights<T, W, NH, SIDE>), wave_grid(ceil_div(q.num_dst * (SIDE ? q.H / NH : 1) * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
              q.H, q.slope, q.num_dst, g.range, g.none, g.weight, (T*)attn, masked)
   APT_GAT_LANES(q, APT_WEIGHTS)
 #undef APT_WEIGHTS
@@ -650,8 +695,8 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
     rc = gat_dots<T>(q, g, ws, num_src, s);
     if (rc == APT_OK) rc = launch_slots(num_src, ws.sort, kOrder, kind, split.long_edges, (int)dim, s);
     if (rc != APT_OK) return rc;
-#define APT_SCORES(W, NH)                                                                                                    \
-  APT_FOLLOW((k_gat_scores<T, W, NH>), wave_grid(ceil_div(q.num_dst * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
+#define APT_SCORES(W, NH, SIDE)                                                                                                    \
+  APT_FOLLOW((k_gat_scores<T, W, NH, SIDE>), wave_grid(ceil_div(q.num_dst * (SIDE ? q.H / NH : 1) * W, 256), 8), 256, 0, s, q.row, (const T*)q.el, (const T*)q.er, \
              q.H, q.slope, num_src, q.num_dst, q.E, g.range, g.none, g.weight, ws.dots, ws.sums, ws.sort, kind, (T*)grad_er)
     APT_GAT_LANES(q, APT_SCORES)
 #undef APT_SCORES
