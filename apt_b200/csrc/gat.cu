@@ -539,21 +539,21 @@ static size_t gat_edges_layout(int64_t num_dst, int64_t E, int H, char* base, Ga
 
 struct GatBwdWs {
   float* sums;      // [spread_rows(num_src)][heads], cleared with the front of the sort
-  SpmmWs sort;      // its order: slots of 16 bytes (kByBoth)
+  SpmmWs sort;
   float* dots;      // [E][heads]
   size_t zero_bytes;
 };
 static size_t gat_bwd_layout(int64_t num_src, int64_t E, int H, char* base, GatBwdWs* ws) {
+  // slots of 16 bytes where k_spmm_stream may take the sums behind the sort, whatever the rows' width (kByBoth)
+  const int slot = E >= kStreamMinOrdered && H <= kStreamHeadsWide ? 16 : 8;
   const size_t o_sort = align_up((size_t)spread_rows(num_src > 0 ? num_src : 1) * H * 4, 256);
-  const size_t o_dots = o_sort + spmm_layout(num_src, E, base + o_sort, ws ? &ws->sort : nullptr);
-  const size_t o_order = o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
+  const size_t o_dots = o_sort + spmm_layout(num_src, E, base + o_sort, ws ? &ws->sort : nullptr, slot);
   if (ws) {
     ws->sums = (float*)base;
     ws->dots = (float*)(base + o_dots);
     ws->zero_bytes = o_sort + ws->sort.zero_bytes;
-    ws->sort.order = (uint2*)(base + o_order);
   }
-  return o_order + align_up((size_t)(E > 0 ? E : 1) * 16, 256);
+  return o_dots + align_up((size_t)(E > 0 ? E : 1) * H * 4, 256);
 }
 
 struct GatProblem {

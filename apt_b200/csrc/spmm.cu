@@ -20,7 +20,7 @@
 
 namespace apt {
 
-size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) {
+size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws, int slot_bytes) {
   const int64_t rows = num_rows > 0 ? num_rows : 1, edges = num_edges > 0 ? num_edges : 1;
   // a row handed to whole warps has more than kLongRowNarrow edges and becomes at most edges / kItemEdges + 1 items;
   // rows of several items have more than kItemEdges
@@ -39,7 +39,7 @@ size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws) 
   const size_t zero = at;
   const size_t o_range = take((size_t)(rows + 1) * 8);
   const size_t o_rank = take((size_t)edges * 4);
-  const size_t o_order = take((size_t)edges * 8);
+  const size_t o_order = take((size_t)edges * slot_bytes);
   const size_t o_items = take((size_t)max_items * 16);
   const size_t o_part = take((size_t)part_floats * 4);
   if (ws) {

@@ -608,7 +608,8 @@ int launch_spmm_rows(int op, const RowArgs<T>& a, cudaStream_t s);
 constexpr int kStreamWaitPolls = 1 << 20;      // of an mbarrier, each of which may suspend for a while itself
 int bulk_wait_polls();
 int pending_word(int32_t** word);            // for flags of calls without a status word: see spmm.cu
-size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws);
+// slot_bytes: of order[] (OrderKind).
+size_t spmm_layout(int64_t num_rows, int64_t num_edges, char* base, SpmmWs* ws, int slot_bytes = 8);
 // Counted edges (ws.cnt) to places: ws.range, and the items of long rows.
 int launch_slots(int64_t num_rows, const SpmmWs& ws, int mode, OrderKind kind, int long_edges, int part_stride, cudaStream_t s);
 

@@ -5,6 +5,8 @@ import subprocess
 
 import pytest
 
+from apt_b200._lib import lib
+
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "apt_b200", "csrc")
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 PROGRAM = r"""
@@ -52,3 +54,14 @@ def test_partial_sums_find_room(fits, esz, dim, warps):
     # stretches of 32 edges, on up to two blocks an SM, whatever the width
     for edges in (98_304, 135_000, 196_608, 1_013_760):
         assert fits((COPY_U, 16, dim, esz, 1, edges, BLOCKS)) == [min(296, edges // (32 * warps))]
+
+
+@pytest.mark.parametrize("edges,heads", [(1, 1), (50_000, 4), (98_303, 16), (98_304, 16), (98_304, 17), (1_013_760, 4)])
+def test_the_attention_backward_holds_one_order(edges, heads):
+    # beside what the sums behind a sort take: fp32 sums of the score gradients, the dots, and 16 bytes a slot where the stream may
+    # take the walk instead of 8
+    sources = 20_000
+    sums, dots = -(-sources // 1024) * 1024 * heads * 4, edges * heads * 4
+    more = 8 * edges if edges >= 98_304 and heads <= 16 else 0
+    extra = lib.apt_gat_backward_workspace_bytes(sources, edges, heads) - lib.apt_spmm_workspace_bytes(sources, edges)
+    assert sums + dots + more <= extra <= sums + dots + more + 3 * 256
