@@ -6,27 +6,40 @@ held to the 2-norm of the fp64 results: about 15 fp32 terms a sum (2e-6), and 2^
 gradient of el is added up in fp32 one edge after another, in the order of arrival: n additions, each off by up to 2^-24 of the sum
 so far (1 / sqrt(3) of that as a standard deviation), are off by sqrt(n / 3) 2^-24 of the largest sum on the way. The first source here
 has 393 000 / 9001^(1/4) = 40 400 edges, which is 6.9e-6; three standard deviations are 2.1e-5 (seen: up to 7.2e-6 in 250 runs)."""
+import ctypes
+
 import pytest
 import torch
 
 from apt_b200 import ops
+from apt_b200._lib import check, lib
 
 pytestmark = pytest.mark.gpu
 N_IN = 5003
 
 
 def _lengths(shape, edges, gen):
-    """Edges of every output row: a fanout; 0 to 60; one row of almost half of all edges (thousands of stretches) among short ones."""
+    """Edges of every output row: a fanout; 0 to 32; one row of almost half of all edges (thousands of stretches) among short ones."""
     if shape == "fixed":
         return torch.full((edges // 13 + 1,), 13, device="cuda")
-    n = torch.randint(0, 61 if shape == "ragged" else 9, (edges // (30 if shape == "ragged" else 8),), device="cuda", generator=gen)
+    # (16 edges a row, some more rows than that takes: none makes up for a small draw by a length of its own, and none of more than 32
+    # edges makes the probe ask for the counting sort)
+    n = torch.randint(0, 33 if shape == "ragged" else 9, (edges // (15 if shape == "ragged" else 8),), device="cuda", generator=gen)
     if shape == "hub":
         n[n.numel() // 3] = edges // 2
         n[-1] = n[0] = 0
     else:
         n[n.numel() // 2] = 0
-        n[n.numel() // 2] = max(0, edges + 5 - int(n.sum()))
     return n
+
+
+def _mode(col, *off):
+    """Where the probe says a row's edges are."""
+    answer = (ctypes.c_int64 * 3)()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    check(lib.apt_spmm_probe(p(col), col.numel(), p(off[0]), p(off[2]), off[0].numel() - 1, answer,
+                             ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return answer[1]
 
 
 @pytest.mark.parametrize("dtype,D", [(torch.float32, 68), (torch.float32, 128), (torch.float32, 260 - 4), (torch.bfloat16, 136),
@@ -43,7 +56,7 @@ def test_sums(dtype, D, shape, edges):
     row = torch.randint(0, N_IN, (col.numel(),), device="cuda", generator=gen)
     x = torch.randint(-3, 4, (N_IN, D), device="cuda", generator=gen).to(dtype)
     off = [torch.tensor([0, k], device="cuda") for k in (col.numel(), N_IN, n.numel())]
-    assert col.numel() >= edges
+    assert col.numel() >= edges and _mode(col, *off) == {"fixed": 0, "ragged": 1, "hub": 2}[shape]
     want = torch.zeros((n.numel(), D), device="cuda", dtype=torch.float64).index_add_(0, col, x.double()[row]).to(dtype)
     assert torch.equal(ops.spmm_copy_u_sum(row, col, x, *off), want)
 
@@ -136,7 +149,7 @@ def test_rows_of_any_number_of_stretches(dtype, D):
 @pytest.mark.parametrize("shape", ["fixed", "ragged", "none"])
 @pytest.mark.parametrize("further", [0, 7])
 def test_segments_in_any_order(dtype, D, edges, shape, further):
-    """Three segments; edges of the same number each, of 0 to 60, or in no order. With further output rows behind the last segment's
+    """Three segments; edges of the same number each, of 0 to 32, or in no order. With further output rows behind the last segment's
     nothing about the edges is known to the host, and the kernels decide."""
     gen = torch.Generator(device="cuda").manual_seed(D + edges)
     fanout = 13
@@ -144,7 +157,7 @@ def test_segments_in_any_order(dtype, D, edges, shape, further):
     rows, cols = [], []
     for share in (0.5, 0.03, 0.47):
         n_dst, n_src = int(edges * share / fanout) + 1, int(3001 * share)
-        n = torch.full((n_dst,), fanout, device="cuda") if shape == "fixed" else torch.randint(0, 61, (n_dst * fanout // 30 + 1,), device="cuda", generator=gen)
+        n = torch.full((n_dst,), fanout, device="cuda") if shape == "fixed" else torch.randint(0, 33, (n_dst * fanout // 15 + 1,), device="cuda", generator=gen)
         col = torch.arange(n.numel(), device="cuda").repeat_interleave(n)
         if shape == "none":
             col = col[torch.randperm(col.numel(), device="cuda", generator=gen)]
@@ -156,7 +169,37 @@ def test_segments_in_any_order(dtype, D, edges, shape, further):
     at = torch.cat([c + o for c, o in zip(cols, dst)])
     of = torch.cat([r + o for r, o in zip(rows, src)])
     total = dst[-1] + further
+    mode = _mode(col, *(torch.tensor(v, device="cuda") for v in (parts, src, dst)))
+    assert col.numel() >= edges and mode == {"fixed": 0, "ragged": 1, "none": 2}[shape]
     want = torch.zeros((total, D), device="cuda", dtype=torch.float64).index_add_(0, at, x.double()[of]).to(dtype)
     dev = lambda v: torch.tensor(v, device="cuda")
     got = ops.spmm_copy_u_sum(row, col, x, dev(parts), dev(src), dev(dst + [total] if further else dst))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 72), (torch.bfloat16, 256), (torch.float32, 256)])
+@pytest.mark.parametrize("shape,edges", [("fixed", 700_000), ("ragged", 700_000), ("hub", 100_000)])
+def test_waits_that_run_out_leave_zeros(dtype, D, shape, edges):
+    # 16-byte copies and bulk copies; in the counting sort's order a row of thousands of stretches, all of which have to be done
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    n = _lengths(shape, edges, gen)
+    if shape == "hub":
+        n[1] += max(0, edges - int(n.sum()))
+    col = torch.arange(n.numel(), device="cuda").repeat_interleave(n)
+    if shape == "hub":
+        col = col[torch.randperm(col.numel(), device="cuda", generator=gen)]
+    row = torch.randint(0, N_IN, (col.numel(),), device="cuda", generator=gen)
+    x = torch.ones((N_IN, D), device="cuda", dtype=dtype)
+    off = [torch.tensor([0, k], device="cuda") for k in (col.numel(), N_IN, n.numel())]
+    check(lib.apt_set_tunable(b"bulk_wait_polls", 0))
+    try:
+        y = ops.spmm_copy_u_sum(row, col, x, *off)
+        torch.cuda.synchronize()
+        assert not bool(y.any())
+        with pytest.raises(RuntimeError, match="did not reach shared memory"):
+            ops.check_status()
+    finally:
+        check(lib.apt_set_tunable(b"bulk_wait_polls", 1 << 20))
+    y = ops.spmm_copy_u_sum(row, col, x, *off)
+    assert torch.equal(y[:, 0], n.to(dtype))
+    ops.check_status()
