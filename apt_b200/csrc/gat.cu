@@ -13,17 +13,16 @@
 //
 //   k_gat_ranges    where each destination's edges are (6.5 us with one edge a thread; a word that every kernel looks at had
 //                   to be cleared in front, a launch more: attention of 30 000 x 15 edges, bf16 4 x 64, 41.5 -> 38.3 us forward)
-//   k_gat_weights   scores and softmax, a few lanes per destination, two edges a lane, four heads at a time; any number of
+//   k_gat_weights   scores and softmax, a few lanes per destination and up to four of its heads, two edges a lane; any number of
 //                   edges and heads.
-//   row kernel      the weighted sum is the SpMM's row kernel (kUMulW), any head width
+//   sums            the weighted sum is the SpMM's (kUMulW), any head width: k_spmm_stream for wide rows of many edges, else k_spmm_rows
 //   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination (wide rows of many edges:
 //                   k_spmm_stream's kDots). The four partial dots of a lane are reduced together: each step halves the values
 //                   a lane keeps, log2(lph) + 1 shuffles for four edges instead of 4 log2(lph).
 //   k_gat_scores    backward: t, grad_s and grad_er, the same lanes; grad_el is added up in fp32 with one reduction per edge
-//                   of all its heads
-//   row kernel      grad_ft: the weighted sum of the forward with the sides swapped. With grad_el as a second accumulator
-//                   of the same walk it held two blocks an SM instead of three: 150 us against 116, and the scores had to
-//                   be written out for it.
+//                   of up to four of its heads
+//   sums            grad_ft: the weighted sum of the forward with the sides swapped. (grad_el as a second accumulator of the same
+//                   walk cost k_spmm_rows a block an SM and the scores had to be written out for it: 150 us against 116.)
 //   The counting sort by source that grad_ft needs rides along: the dots have every edge's source in a register and wait
 //                   for rows most of the time, so they also count the edges (the add returns an edge's place in its
 //                   row); k_dst_slots gives the rows their places; k_gat_scores writes the order. As launches of
@@ -35,8 +34,8 @@
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 17 + 61 us. Backward of that block: 17 (saved after a forward) + 80 + 5 + 30 + 63 + 5 us,
-// where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
+// kernels take 16 + 61 us. Backward of that block: 16 (saved after a forward) + 79 + 5 + 31 + 75 + 4 us (each kernel by itself, caches
+// cold), where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 
 #include <algorithm>

@@ -168,7 +168,15 @@ struct RowArgs {
   uint32_t num_in;         // input rows; ws.cnt and ws.rank count their edges on the way
 };
 
-// ---- which rows k_spmm_stream takes (the figures are there) ------------------------------------
+// ---- which rows k_spmm_stream takes --------------------------------------------------------------
+// The lines, us of the call by k_spmm_rows -> by k_spmm_stream on either side (15 edges a row, or 0 to 30 where it says so):
+//   sorted edges, 98 304: gains from all sizes tried on: fp32 x 128, 65 535 edges 49 -> 37, 98 310 54 -> 42; x 256 50 -> 41, 54 -> 42
+//   weighted, up to 512 bytes, 393 216: 300 000 edges bf16 4 x 64 30.5 -> 30.9, fp32 4 x 32 31.9 -> 30.4; 393 210 37.1 -> 35.2, 39.2 -> 33.9
+//   above 512 bytes, 196 608: 135 000 edges fp32 4 x 64 22.0 -> 23.2, sums of fp32 x 256 23.9 -> 27.1; 196 605 27.4 -> 27.3, 27.7 -> 29.1 (0 to 30:
+//     36.3 -> 35.6), bf16 x 512 33.0 -> 31.0; 300 000 39.2 -> 37.2, 35.4 -> 35.4, 45.7 -> 39.1
+//   sums, up to 512 bytes, 655 360: 450 000 edges fp32 x 128 32.0 -> 30.8 (0 to 30: 43.5 -> 39.4), bf16 x 256 37.8 -> 34.2, fp32 x 72 30.8 -> 30.3; 655 365
+//     44.6 -> 44.0 (60 -> 53), 50.5 -> 45.0, 38.5 -> 40.6 (54 -> 46); 1 013 760 70 -> 55 (96 -> 67), 77 -> 60, 58 -> 50. Rows that half fill the warp and have
+//     the same number of edges each lose 5 to 8 % from there to about 800 000.
 constexpr int kStreamBlocks = 2;
 constexpr int stream_warps(bool one_slice) { return one_slice ? 12 : 10; }
 constexpr int kStreamShared = 112 * 1024 - 2560;      // a block's, beside its barriers and segment tables

@@ -20,13 +20,15 @@
 //
 // us of the whole call, k_spmm_rows or a bulk-copy kernel for rows above 512 bytes (rows dealt to the warps one by one) -> here,
 // 67 584 x 15 edges:
-//   sums         fp32 x 256 forward 100 -> 101, reverse 187 -> 142; x 128 71 -> 54, 134 -> 107; bf16 x 256 77 -> 59, 144 -> 121
-//   attention    forward, both directions: bf16 4 x 64 103 -> 81, 369 -> 282; fp32 4 x 64 156 -> 118, 548 -> 392; 4 x 32 99 -> 73, 356 -> 260
-// Against it: sums of grouped rows of up to 512 bytes, 30 000 x 15 31 -> 33, 16 000 x 15 23 -> 26 (the start of a stream is three
-// dependent fetches). Behind the sort it gains from a hundred thousand edges on: 9000 x 15, x 128 55 -> 45, x 256 61 -> 53.
-// Hence the lines of stream_fits.
+//   sums         fp32 x 256 forward 98 -> 101, reverse 190 -> 129; x 128 71 -> 52, 134 -> 97; bf16 x 256 79 -> 59, 143 -> 111
+//   attention    forward, both directions: bf16 4 x 64 104 -> 75, 375 -> 261; fp32 4 x 64 158 -> 116, 556 -> 380; 4 x 32 100 -> 67, 357 -> 236
+// Against it: the start of a stream is three dependent fetches, which few edges a warp do not make up for. Hence the lines of stream_fits.
+// 16-bit rows of two slices a lane spill 92 bytes with weights and 20 in kDots at ten warps (bf16 2 x 256, 67 584 x 15 edges,
+// both directions 676 -> 456 all the same).
+// Hub rows: 100 000 edges in no order, half of them in one row, fp32 x 128: 135 -> 77, 400 000 330 -> 192 (218 and 400 with one warp to add up
+// all parts of a row).
 // Both gradients of the attention in one walk (a source's features in registers, dots and sums of its edges) saved a walk and lost
-// it again: 70 instructions an edge, 147 us against 82 + 62, with the dots on mma.sync 181.
+// it again: 70 instructions an edge, 147 us, which the two walks take as well; with the dots on mma.sync 181.
 #pragma once
 
 #include "spmm_rows.cuh"
