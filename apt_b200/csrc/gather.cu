@@ -1,20 +1,26 @@
 // Cache-aware feature-row gather: one launch, no scratch.
 //
-// A warp takes a chunk of rows. One lane to a row looks the id up (p = feat_pos_map[id]: p >= 0 cache row, p < -1 host row
-// -p - 2, p == -1 no such row: zeros and a flag); the rows that live in page-locked host memory are copied first, then
-// those of the cache, with four vectors (and, narrow rows, several rows) a lane in flight. The reads over the host
-// link of all warps are outstanding together and beside the other warps' copies from HBM.
+// A warp takes a chunk of rows. One lane to a row looks the id up (p = feat_pos_map[id]: p >= 0 cache row, p < -1 row -p - 2 of the
+// table in page-locked host memory, p == -1 no such row: zeros and a flag) and leaves the row's address in shared memory. In
+// the result the chunk is one run of elements, which the warp copies from end to end, 8 of 32 lanes each in flight:
+// rows of any width fill all lanes, and what is in flight does not depend on it. The division that finds an element's row is a
+// multiplication.
 //
-// Against the three kernels it replaces (decode ids and compact a miss list, copy the hits, copy the misses), B200:
-//   495 616 rows x 2 KiB      357 -> 327 us (6.2 TB/s, 0.95 of the measured copy rate)
-//   143 000 rows x 512 B      31 -> 28 us; with 2.7 % from host memory 72 -> 50 us
-//   1 203 rows x 400 B, a tenth from host memory    15.5 -> 5.0 us
-//   6 158 rows x 390 B (2-byte vectors)             26 -> 4.7 us
-// and, in mini-batches that run beside one another on lanes, 7 470 -> 7 830 papers-shaped mini-batches a second. Bound
-// by HBM, by the host link (64 bytes to a few KiB a request, about 50 M rows/s) and, small requests, by three dependent
-// loads.
+// Rows one after another, the form before this, had a row of more than 32 elements as one load of 32 in flight, and a row of
+// 33 took the steps of 64. us, that form -> this one (distinct rows, all cached unless it says so):
+//   495 616 x 2 KiB     331 -> 320 (6.36 TB/s, 0.97 of the measured copy rate)
+//   243 961 x 880 B     145 -> 76           243 961 x 882 B (2-byte elements)   172 -> 113
+//   200 000 x 1 KiB     104 -> 68           200 000 x 1200 B                    144 -> 84
+//   318 250 x 288 B      49 -> 40           318 250 x 292 B (4-byte elements)    66 -> 47
+//   400 000 x 200 B (8-byte elements) 48 -> 41      400 000 x 66 B (2-byte elements)  70 -> 23
+//   143 000 x 512 B, 2.7 % of them from host memory 50.7 -> 46.7
+// Bound by HBM, by the host link (64 bytes to a few KiB a request, about 50 M rows/s) and, small requests, by three dependent
+// loads; rows of 2-byte elements by their loads and stores (copying 882-byte rows through shared memory in 16-byte vectors, shifted on the way
+// out, took 93 instead of 113 us and rows below 512 bytes longer; two elements to a lane 135). The host rows by themselves, in
+// front of the others, two at a time through shared memory: 143 000 x 512 B 90. Chunks of 16 KiB instead of kChunkBytes: 880 B 80, 1 KiB 71;
+// of 2 KiB 89, 75.
 //
-// Rows are opaque bytes. The vector width V is the widest of 16/8/4/2/1 bytes that divides every row size, column offset
+// Rows are opaque bytes. An element V is the widest of 16/8/4/2/1 bytes that divides every row size, column offset
 // and base address involved.
 #include <string.h>
 
@@ -22,9 +28,11 @@
 
 namespace apt {
 
-constexpr int kRowsPerGroup = 4;   // rows (or vectors of a long row) whose loads are in flight together
 constexpr int kGatherBlock = 256;
 constexpr int kGatherWaves = 4;    // cap on the grid, in units of 148 x 8 blocks
+constexpr int kGatherVectors = 8;  // elements a lane has in flight
+constexpr int kChunkBytes = 4096;
+constexpr int kGatherBlocks = 5;   // an SM (48 registers)
 
 template <typename V>
 __device__ __forceinline__ V ld_vec(const V* p) { return __ldg(p); }
@@ -47,125 +55,6 @@ __device__ __forceinline__ int64_t first_row(const int64_t* first_dev, int64_t n
   return f < 0 ? 0 : (f > n ? n : f);
 }
 
-// A group of kRowsPerGroup rows a lane from those whose flag is set in `mask`: lpr lanes to a row of up to 32 vectors,
-// 32 / lpr rows side by side. `p` is the lane's own row's position in the table, src_of finds the row there.
-template <typename V>
-struct RowGroup {
-  V v[kRowsPerGroup];
-  int row[kRowsPerGroup];     // row of the chunk, -1: none
-
-  template <typename SRC>
-  __device__ __forceinline__ void load(unsigned& mask, int64_t p, int chunks, int lpr, SRC src_of, int lane) {
-    const int side = 32 / lpr, which = lane / lpr, c = lane & (lpr - 1);
-#pragma unroll
-    for (int k = 0; k < kRowsPerGroup; ++k) {
-      // this lane's row is the `which`-th of the next `side` rows of the mask
-      int mine = -1;
-      for (int q = 0; q < side && mask; ++q) {
-        const int l = __ffs(mask) - 1;
-        mask &= mask - 1;
-        if (q == which) mine = l;
-      }
-      const int64_t pk = __shfl_sync(0xffffffffu, p, mine < 0 ? 0 : mine);
-      row[k] = c < chunks ? mine : -1;
-      if (row[k] >= 0) v[k] = ld_vec<V>((const V*)src_of(pk) + c);
-    }
-  }
-  __device__ __forceinline__ void store(char* out, int64_t first_row, int64_t row_bytes, int lpr, int lane) const {
-    const int c = lane & (lpr - 1);
-#pragma unroll
-    for (int k = 0; k < kRowsPerGroup; ++k)
-      if (row[k] >= 0) st_vec<V>((V*)(out + (first_row + row[k]) * row_bytes) + c, v[k]);
-  }
-};
-
-// All rows of the mask; rows of more than 32 vectors one at a time, four vectors a lane in flight.
-template <typename V, typename SRC>
-__device__ __forceinline__ void copy_rows(unsigned mask, int64_t p, int64_t first_row, int chunks, int lpr, SRC src_of, char* out,
-                                          int64_t row_bytes, int lane) {
-  if (chunks <= 32) {
-    while (mask) {
-      RowGroup<V> g;
-      g.load(mask, p, chunks, lpr, src_of, lane);
-      g.store(out, first_row, row_bytes, lpr, lane);
-    }
-    return;
-  }
-  while (mask) {
-    const int l = __ffs(mask) - 1;
-    mask &= mask - 1;
-    const V* const src = (const V*)src_of(__shfl_sync(0xffffffffu, p, l));
-    V* const dst = (V*)(out + (first_row + l) * row_bytes);
-    int c = lane;
-    for (; c + 96 < chunks; c += 128) {
-      V v[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = ld_vec<V>(src + c + 32 * k);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) st_vec<V>(dst + c + 32 * k, v[k]);
-    }
-    for (; c < chunks; c += 32) st_vec<V>(dst + c, ld_vec<V>(src + c));
-  }
-}
-
-template <typename V>
-__global__ void __launch_bounds__(kGatherBlock)
-k_gather(const int64_t* __restrict__ index, int64_t n, const int64_t* __restrict__ n_dev, const int64_t* __restrict__ first_dev,
-         const int64_t* __restrict__ pos_map, int64_t num_nodes, const char* __restrict__ dev_feats, int64_t num_dev_rows,
-         const char* __restrict__ uva_feats, int64_t num_uva_rows, int64_t uva_row_bytes, int64_t col_offset_bytes,
-         int64_t row_bytes, int rows_per_chunk, int lpr, char* __restrict__ out, int32_t* status, const Tagged counts) {
-  wait_for_previous();
-  // the counts of a mini-batch leave with its rows: as a kernel in front they held the rows up for 4 us
-  if (counts.host && blockIdx.x == 0) publish_tagged(counts);
-  n = effective_n(n, n_dev);
-  const int64_t first = first_row(first_dev, n);
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (kGatherBlock / 32);
-  const int64_t warp = (int64_t)blockIdx.x * (kGatherBlock / 32) + (threadIdx.x >> 5);
-  const int chunks = (int)(row_bytes / (int64_t)sizeof(V));
-  int flags = 0;
-  for (int64_t r0 = first + warp * rows_per_chunk; r0 < n; r0 += warps * rows_per_chunk) {
-    int64_t p = -2;
-    const bool live = lane < rows_per_chunk && r0 + lane < n;
-    if (live) {
-      const int64_t id = index[r0 + lane];
-      p = -1;
-      if (id < 0 || id >= num_nodes) {
-        flags |= APT_FLAG_ID_OUT_OF_RANGE;
-      } else {
-        p = pos_map[id];
-        if (p == -1) {
-          flags |= APT_FLAG_FEAT_NOT_EXIST;
-        } else if (p >= num_dev_rows || (-p - 2) >= num_uva_rows) {
-          flags |= APT_FLAG_ID_OUT_OF_RANGE;
-          p = -1;
-        }
-      }
-    }
-    const unsigned hits = __ballot_sync(0xffffffffu, live && p >= 0);
-    const unsigned misses = __ballot_sync(0xffffffffu, live && p < -1);
-    unsigned none = __ballot_sync(0xffffffffu, live && p == -1);
-    auto cached = [&](int64_t q) { return dev_feats + q * row_bytes; };
-    auto hosted = [&](int64_t q) { return uva_feats + (-q - 2) * uva_row_bytes + col_offset_bytes; };
-    // the reads over the host link first: they take longest, and the other warps' copies run meanwhile (holding them in
-    // registers over this warp's own copies cost every request without misses a fifth)
-    copy_rows<V>(misses, p, r0, chunks, lpr, hosted, out, row_bytes, lane);
-    copy_rows<V>(hits, p, r0, chunks, lpr, cached, out, row_bytes, lane);
-    while (none) {                 // no such row: zeros
-      const int l = __ffs(none) - 1;
-      none &= none - 1;
-      for (int c = lane; c < chunks; c += 32) st_vec<V>((V*)(out + (r0 + l) * row_bytes) + c, zero_vec<V>());
-    }
-  }
-  if (flags) atomicOr(status, flags);
-}
-
-static int vec_width(uint64_t bits) {
-  for (int w = 16; w > 1; w >>= 1)
-    if ((bits & (uint64_t)(w - 1)) == 0) return w;
-  return 1;
-}
-
 struct GatherArgs {
   const int64_t* index;
   int64_t num_rows;
@@ -182,6 +71,72 @@ struct GatherArgs {
   Tagged counts;
 };
 
+// A warp's rows, one after another in the result: where each of them is. By all lanes; null: there is no such row, zeros.
+__device__ __forceinline__ void find_rows(const GatherArgs& a, int64_t r0, int rows, const char** place, int lane, int& flags) {
+  const char* row = nullptr;
+  if (lane < rows) {
+    const int64_t id = a.index[r0 + lane];
+    if (id < 0 || id >= a.num_nodes) {
+      flags |= APT_FLAG_ID_OUT_OF_RANGE;
+    } else {
+      const int64_t p = a.feat_pos_map[id];
+      if (p == -1) {
+        flags |= APT_FLAG_FEAT_NOT_EXIST;
+      } else if (p >= a.num_dev_rows || (-p - 2) >= a.num_uva_rows) {
+        flags |= APT_FLAG_ID_OUT_OF_RANGE;
+      } else {
+        row = p >= 0 ? a.dev_feats + p * a.dev_row_bytes : a.uva_feats + (-p - 2) * a.uva_row_bytes + a.uva_col_offset_bytes;
+      }
+    }
+  }
+  __syncwarp();      // (the rows before have been read)
+  place[lane] = row;
+  __syncwarp();
+}
+
+template <typename V>
+__global__ void __launch_bounds__(kGatherBlock, kGatherBlocks)
+k_gather(const __grid_constant__ GatherArgs a, uint32_t elems, uint32_t inverse, int rows_per_chunk) {
+  wait_for_previous();
+  // the counts of a mini-batch leave with its rows: as a kernel in front they held the rows up for 4 us
+  if (a.counts.host && blockIdx.x == 0) publish_tagged(a.counts);
+  __shared__ const char* places[kGatherBlock / 32][32];
+  const int64_t n = effective_n(a.num_rows, a.num_rows_dev), first = first_row(a.first_row_dev, n);
+  const int lane = threadIdx.x & 31;
+  const char** const place = places[threadIdx.x >> 5];
+  const int64_t warps = (int64_t)gridDim.x * (kGatherBlock / 32);
+  const int64_t warp = (int64_t)blockIdx.x * (kGatherBlock / 32) + (threadIdx.x >> 5);
+  int flags = 0;
+  for (int64_t r0 = first + warp * rows_per_chunk; r0 < n; r0 += warps * rows_per_chunk) {
+    const int rows = (int)min((int64_t)rows_per_chunk, n - r0);
+    find_rows(a, r0, rows, place, lane, flags);
+    const uint32_t total = (uint32_t)rows * elems;
+    V* const dst = (V*)(a.out + r0 * a.dev_row_bytes) + lane;
+    for (uint32_t e0 = 0; e0 < total; e0 += 32 * kGatherVectors) {
+      V v[kGatherVectors];
+#pragma unroll
+      for (int u = 0; u < kGatherVectors; ++u) {
+        const uint32_t e = e0 + u * 32 + lane, r = __umulhi(2 * e + 1, inverse);
+        v[u] = zero_vec<V>();
+        if (e < total) {
+          const char* const from = place[r];
+          if (from) v[u] = ld_vec<V>((const V*)from + (e - r * elems));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kGatherVectors; ++u)
+        if (e0 + u * 32 + lane < total) st_vec<V>(dst + e0 + u * 32, v[u]);
+    }
+  }
+  if (flags) atomicOr(a.status_word, flags);
+}
+
+static int vec_width(uint64_t bits) {
+  for (int w = 16; w > 1; w >>= 1)
+    if ((bits & (uint64_t)(w - 1)) == 0) return w;
+  return 1;
+}
+
 // Blocks an SM for a gather that runs beside other kernels: enough reads over the host link for its full rate (one block's
 // warps have 16 KiB each in flight, of the 80 KB that rate times latency asks of the whole chip), and room for the others,
 // which at the full grid wait until it ends.
@@ -192,28 +147,25 @@ static int gather_launch(const GatherArgs& a, cudaStream_t s, bool narrow = fals
   if (a.num_dev_rows > 0) bits |= (uintptr_t)a.dev_feats;
   if (a.num_uva_rows > 0) bits |= (uint64_t)a.uva_row_bytes | (uint64_t)a.uva_col_offset_bytes | (uintptr_t)a.uva_feats;
   const int width = vec_width(bits);
-  const int64_t vectors = a.dev_row_bytes / width;
-  int lpr = 1;
-  while (lpr < vectors && lpr < 32) lpr <<= 1;
-  // chunks as large as leave every warp of the chip one: a small request wants all SMs, a large one few lookups
-  const int64_t all_warps = (int64_t)kNumSMs * 8 * (kGatherBlock / 32);
-  int per = 32 / lpr;
-  while (per < 32 && (int64_t)per * all_warps < a.num_rows) per <<= 1;
-  int grid = wave_grid(ceil_div(a.num_rows, (int64_t)per * (kGatherBlock / 32)), 8, kGatherWaves);
+  const int64_t elems = a.dev_row_bytes / width;
+  // One row where every warp of the chip can have its own (a pass over several waits for the slowest, a row from the host); else as many
+  // as fill the lanes or take up to kChunkBytes, while every warp of the chip has that many (and 32, a lane to look each up).
+  int rows = 1;
+  while (rows < 32 && (int64_t)rows * kNumSMs * 64 < a.num_rows && (rows * a.dev_row_bytes < 512 || 2 * rows * a.dev_row_bytes <= kChunkBytes))
+    rows <<= 1;
+  // (2 e + 1) / (2 elems) in 32 bits is the row of element e: exact while e < 2^18 and elems < 2^12, and rows that share a chunk have
+  // 4096 bytes or fewer together
+  const uint32_t inverse = rows > 1 ? (uint32_t)(((1ull << 31) + elems - 1) / elems) : 0u;
+  int grid = wave_grid(ceil_div(a.num_rows, (int64_t)rows * (kGatherBlock / 32)), 8, kGatherWaves);
   if (narrow && grid > kNumSMs * kNarrowBlocks) grid = kNumSMs * kNarrowBlocks;
   ProfScope prof("gather_hit", s);
-#define APT_GATHER(V)                                                                                                     \
-  APT_FOLLOW(k_gather<V>, grid, kGatherBlock, 0, s, a.index, a.num_rows, a.num_rows_dev, a.first_row_dev, a.feat_pos_map, \
-             a.num_nodes, a.dev_feats, a.num_dev_rows, a.uva_feats, a.num_uva_rows, a.uva_row_bytes,                      \
-             a.uva_col_offset_bytes, a.dev_row_bytes, per, lpr, a.out, a.status_word, a.counts)
   switch (width) {
-    case 16: APT_GATHER(uint4); break;
-    case 8: APT_GATHER(uint2); break;
-    case 4: APT_GATHER(uint32_t); break;
-    case 2: APT_GATHER(uint16_t); break;
-    default: APT_GATHER(uint8_t); break;
+    case 16: APT_FOLLOW(k_gather<uint4>, grid, kGatherBlock, 0, s, a, (uint32_t)elems, inverse, rows); break;
+    case 8: APT_FOLLOW(k_gather<uint2>, grid, kGatherBlock, 0, s, a, (uint32_t)elems, inverse, rows); break;
+    case 4: APT_FOLLOW(k_gather<uint32_t>, grid, kGatherBlock, 0, s, a, (uint32_t)elems, inverse, rows); break;
+    case 2: APT_FOLLOW(k_gather<uint16_t>, grid, kGatherBlock, 0, s, a, (uint32_t)elems, inverse, rows); break;
+    default: APT_FOLLOW(k_gather<uint8_t>, grid, kGatherBlock, 0, s, a, (uint32_t)elems, inverse, rows); break;
   }
-#undef APT_GATHER
   return APT_OK;
 }
 
