@@ -58,6 +58,9 @@ PROTOTYPES = {
     "apt_unique_workspace_bytes": (c_size_t, [c_int64]),
     "apt_unique_workspace_init": (c_int, [P, c_size_t, P]),
     "apt_unique_sorted": (c_int, [P, c_int64, P, c_int64, c_int64, P, c_size_t, P, P, P, P, P]),
+    "apt_unique_ids": (c_int, [P, c_int64, P, c_int64, c_int64, c_int64, P, c_size_t, P, P, P, P]),
+    "apt_unique_inverse": (c_int, [P, c_int64, P, c_int64, c_int64, c_int64, P, c_size_t, P, P, c_int64, P, P, P, P, P, c_int64, P, P, P,
+                                   P, c_int64, c_int64, c_int64, P, P]),
     "apt_concat_ids": (c_int, [P, c_int64, P, P, c_int64, P, P, P, P]),
     "apt_concat_row_ids": (c_int, [P, c_int64, P, P, c_int64, P, P, P, P, c_int64, c_int64, c_int64, P, P]),
     "apt_gather_workspace_bytes": (c_size_t, [c_int64]),
@@ -86,6 +89,7 @@ PROTOTYPES = {
     "apt_srcdst_to_vir": (c_int, [P, c_int64, P, c_int64, c_int64, P, c_int, c_int, c_int, c_int, c_int, P, P]),
     "apt_vir_send_sizes": (c_int, [P, c_int64, P, P, c_int64, P, c_int, c_int64, P, c_int, P, P, P]),
     "apt_sp_map_place_pack": (c_int, [P, P, c_int64, P, c_int64, P, c_int, c_int, c_int, c_int, c_int, c_int64, c_int64, P, P, P, P]),
+    "apt_sp_one_rank": (c_int, [P, c_int64, P, c_int64, c_int64, c_int64] + [P] * 13),
     "apt_sp_pack_frontier": (c_int, [P, P, c_int64, c_int64, c_int, c_int64, c_int64, P, P]),
     "apt_sp_unpack_frontier": (c_int, [P, c_int64, P, c_int64, P, P, P]),
     "apt_hotness_add": (c_int, [P, c_int64, P, P, c_int64, P, P]),

@@ -1,5 +1,7 @@
 // Owner bucketing (stable partition of ids by owning rank) and the sorted
 // unique + inverse over a bounded id range.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace apt {
@@ -152,7 +154,9 @@ k_concat_ids(const int64_t* __restrict__ a, int64_t na, const int64_t* __restric
 // ranking and emitting walk level 1 only (range/1024 words), so the cost of a
 // call follows the number of ids, not the width of the range. Both levels are
 // all-zero between calls: the pass that emits the ids also clears what it read.
-// Three launches: mark (and count per tile of words), emit (ranks, ids, clear), inverse.
+// Three launches: mark (and count per tile of words), emit (ranks, ids, clear), inverse. The last can be enqueued beside what is made of the
+// distinct ids, and leaves other things that take the same ids (OneRank, ListOf): us of a mini-batch, papers-shaped 218 -> 216, with
+// source-split sampling for attention 231 -> 224. (The list written by the emit, whose lanes have several ids one after another to look up: 242.)
 constexpr int kUniqBlock = 256;
 constexpr int kSharedTiles = 1024;    // up to here a block adds its counts up in shared memory first
 constexpr int kGroup = 256;           // tiles whose counts are added up once more where there are many
@@ -166,10 +170,17 @@ struct TileCounts {
   int shift;           // level-0 word -> tile
 };
 
+// The number of ids: `n`, or the device's count of groups of `per`.
+__device__ __forceinline__ int64_t ids_of(int64_t n, const int64_t* n_dev, int64_t per) {
+  if (!n_dev) return n;
+  const int64_t v = *n_dev * per;
+  return v < 0 ? 0 : min(v, n);
+}
+
 // Runs of lanes whose ids share a word (the virtual ids of a sampled hop come in runs of its fanout) are joined
 // first: one atomic a run. 23 000 ids in runs of 25: 24 us with one an id.
 __global__ void __launch_bounds__(256)
-k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
+k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev, int64_t per,
             int64_t lo, int64_t hi, uint32_t* __restrict__ l0, uint32_t* __restrict__ l1,
             TileCounts counts, int32_t* status) {
   wait_for_previous();
@@ -179,7 +190,7 @@ k_uniq_mark(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restric
     for (int t = threadIdx.x; t < counts.tiles; t += 256) here[t] = 0;
     __syncthreads();
   }
-  n = effective_n(n, n_dev);
+  n = ids_of(n, n_dev, per);
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int flags = 0;
@@ -326,16 +337,55 @@ k_uniq_emit(uint32_t* __restrict__ l0, uint32_t* __restrict__ l1, int64_t nwords
   if (lane < per_warp && mine) l1[w1] = 0u;
 }
 
+// The distinct ids behind `head`'s, in a list of their own (as the inverse's launch makes it, a launch for the list alone, 4 us of a
+// source-split mini-batch's chain, is not needed). all null: no such list.
+struct ListOf {
+  const int64_t* head;
+  int64_t num_head;
+  const int64_t* num_head_dev;
+  const int64_t* unique;
+  int64_t num_unique;
+  const int64_t* num_unique_dev;
+  int64_t* all;
+  int64_t* num_all;
+  RowTables tables;      // of a gather of the list's rows
+};
+
+// What a bucketing by owner leaves in a world of one rank: ids [0, count) where they are. all null: nothing.
+struct OneRank {
+  int64_t* perm;
+  int64_t num;
+  const int64_t* num_dev;      // null: as many as there are ids
+  int64_t *sizes, *offsets;
+};
+
 __global__ void __launch_bounds__(256)
-k_uniq_inverse(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev,
-               int64_t lo, int64_t hi, const uint2* __restrict__ info, TileCounts counts, int64_t* __restrict__ out_inverse) {
+k_uniq_inverse(const int64_t* __restrict__ ids, int64_t n, const int64_t* __restrict__ n_dev, int64_t per,
+               int64_t lo, int64_t hi, const uint2* __restrict__ info, TileCounts counts, int64_t* __restrict__ out_inverse, const OneRank one,
+               const ListOf list, int32_t* status) {
   wait_for_previous();
-  n = effective_n(n, n_dev);
+  n = ids_of(n, n_dev, per);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = i; t < counts.tiles; t += stride) {      // the emit is done with them
     counts.tile[t] = 0;
     if (t % kGroup == 0) counts.group[t / kGroup] = 0;
+  }
+  if (one.perm) {
+    const int64_t count = one.num_dev ? effective_n(one.num, one.num_dev) : n;
+    for (int64_t t = i; t < count; t += stride) one.perm[t] = t;
+    if (i == 0) one.sizes[0] = one.sizes[1] = one.offsets[0] = count;
+  }
+  if (list.all) {
+    const int64_t heads = effective_n(list.num_head, list.num_head_dev), total = heads + effective_n(list.num_unique, list.num_unique_dev);
+    if (i == 0 && list.num_all) *list.num_all = total;
+    int flags = 0;
+    for (int64_t t = i; t < total; t += stride) {
+      const int64_t v = t < heads ? list.head[t] : list.unique[t - heads];
+      list.all[t] = v;
+      flags |= check_row(list.tables, v);
+    }
+    if (flags) atomicOr(status, flags);
   }
   for (; i < n; i += stride) {
     const int64_t v = ids[i];
@@ -453,6 +503,39 @@ extern "C" int apt_unique_workspace_init(void* workspace, size_t workspace_bytes
   return APT_OK;
 }
 
+namespace apt {
+static int uniq_check(const char* who, const int64_t* ids, int64_t num_ids, int64_t lo, int64_t hi, void* workspace, size_t workspace_bytes,
+                      const void* out, UniqWs* ws) {
+  APT_CHECK_ARG(ids && workspace && out, "%s: null pointer", who);
+  const size_t need = uniq_layout(hi - lo, (char*)workspace, ws);
+  if (workspace_bytes < need) {
+    set_error("%s: workspace %zu < %zu bytes", who, workspace_bytes, need);
+    return APT_ERR_CAPACITY;
+  }
+  return APT_OK;
+}
+static int uniq_sizes(const char* who, int64_t num_ids, int64_t lo, int64_t hi) {
+  APT_CHECK_ARG(num_ids >= 0 && hi >= lo, "%s: bad sizes", who);
+  APT_CHECK_ARG(hi - lo < ((int64_t)1 << 36), "%s: id range too wide for a bitmap", who);
+  return APT_OK;
+}
+static int uniq_ids(const int64_t* ids, int64_t num_ids, const int64_t* num_ids_dev, int64_t per, int64_t lo, int64_t hi, const UniqWs& ws,
+                    int64_t* out_unique, int64_t* out_num_unique, int32_t* status_word, cudaStream_t s) {
+  APT_FOLLOW(k_uniq_mark, wave_grid(ceil_div(num_ids, 256), 8, 1), 256, 0, s, ids, num_ids, num_ids_dev, per, lo, hi, ws.l0, ws.l1, ws.counts,
+             status_word);
+  APT_FOLLOW(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, lo, ws.counts, ws.info, out_unique,
+             out_num_unique);
+  return APT_OK;
+}
+static int uniq_inverse(const int64_t* ids, int64_t num_ids, const int64_t* num_ids_dev, int64_t per, int64_t lo, int64_t hi, const UniqWs& ws,
+                        int64_t* out_inverse, const OneRank& one, const ListOf& list, int32_t* status_word, cudaStream_t s) {
+  const int64_t most = std::max(num_ids, list.all ? list.num_head + list.num_unique : 0);
+  APT_FOLLOW(k_uniq_inverse, wave_grid(ceil_div(most, 256), 8, 1), 256, 0, s, ids, num_ids, num_ids_dev, per, lo, hi, ws.info, ws.counts,
+             out_inverse, one, list, status_word);
+  return APT_OK;
+}
+}  // namespace apt
+
 extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
                                  const int64_t* num_ids_dev, int64_t id_lo,
                                  int64_t id_hi, void* workspace, size_t workspace_bytes,
@@ -460,8 +543,8 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
                                  int64_t* out_num_unique, int32_t* status_word,
                                  void* stream) {
   using namespace apt;
-  APT_CHECK_ARG(num_ids >= 0 && id_hi >= id_lo, "apt_unique_sorted: bad sizes");
-  APT_CHECK_ARG(id_hi - id_lo < ((int64_t)1 << 36), "apt_unique_sorted: id range too wide for a bitmap");
+  int rc = uniq_sizes("apt_unique_sorted", num_ids, id_lo, id_hi);
+  if (rc != APT_OK) return rc;
   APT_CHECK_ARG(out_num_unique && status_word, "apt_unique_sorted: null output word");
   cudaStream_t s = (cudaStream_t)stream;
   if (num_ids == 0 || id_hi == id_lo) {
@@ -472,20 +555,62 @@ extern "C" int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
     }
     return APT_OK;
   }
-  APT_CHECK_ARG(ids && workspace && out_unique && out_inverse, "apt_unique_sorted: null pointer");
   UniqWs ws;
-  const size_t need = uniq_layout(id_hi - id_lo, (char*)workspace, &ws);
-  if (workspace_bytes < need) {
-    set_error("apt_unique_sorted: workspace %zu < %zu bytes", workspace_bytes, need);
-    return APT_ERR_CAPACITY;
-  }
+  rc = uniq_check("apt_unique_sorted", ids, num_ids, id_lo, id_hi, workspace, workspace_bytes, out_unique && out_inverse ? out_unique : nullptr, &ws);
+  if (rc != APT_OK) return rc;
   ProfScope prof("unique_sorted", s);
-  const int g = wave_grid(ceil_div(num_ids, 256), 8, 1);
-  APT_FOLLOW(k_uniq_mark, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.l0, ws.l1, ws.counts, status_word);
-  APT_FOLLOW(k_uniq_emit, ws.nblocks, kUniqBlock, 0, s, ws.l0, ws.l1, ws.nwords1, ws.per_warp, id_lo, ws.counts, ws.info,
-             out_unique, out_num_unique);
-  APT_FOLLOW(k_uniq_inverse, g, 256, 0, s, ids, num_ids, num_ids_dev, id_lo, id_hi, ws.info, ws.counts, out_inverse);
-  return APT_OK;
+  rc = uniq_ids(ids, num_ids, num_ids_dev, 1, id_lo, id_hi, ws, out_unique, out_num_unique, status_word, s);
+  return rc != APT_OK ? rc : uniq_inverse(ids, num_ids, num_ids_dev, 1, id_lo, id_hi, ws, out_inverse, OneRank{}, ListOf{}, status_word, s);
+}
+
+extern "C" int apt_unique_ids(const int64_t* ids, int64_t num_ids, const int64_t* num_ids_dev, int64_t ids_per, int64_t id_lo, int64_t id_hi,
+                              void* workspace, size_t workspace_bytes, int64_t* out_unique, int64_t* out_num_unique, int32_t* status_word,
+                              void* stream) {
+  using namespace apt;
+  int rc = uniq_sizes("apt_unique_ids", num_ids, id_lo, id_hi);
+  if (rc != APT_OK) return rc;
+  APT_CHECK_ARG(out_num_unique && status_word && ids_per >= 1, "apt_unique_ids: bad argument");
+  cudaStream_t s = (cudaStream_t)stream;
+  if (num_ids == 0 || id_hi == id_lo) {
+    APT_CUDA(cudaMemsetAsync(out_num_unique, 0, sizeof(int64_t), s));
+    return APT_OK;
+  }
+  UniqWs ws;
+  rc = uniq_check("apt_unique_ids", ids, num_ids, id_lo, id_hi, workspace, workspace_bytes, out_unique, &ws);
+  if (rc != APT_OK) return rc;
+  ProfScope prof("unique_sorted", s);
+  return uniq_ids(ids, num_ids, num_ids_dev, ids_per, id_lo, id_hi, ws, out_unique, out_num_unique, status_word, s);
+}
+
+extern "C" int apt_unique_inverse(const int64_t* ids, int64_t num_ids, const int64_t* num_ids_dev, int64_t ids_per, int64_t id_lo, int64_t id_hi,
+                                  void* workspace, size_t workspace_bytes, int64_t* out_inverse, const int64_t* unique, int64_t num_unique,
+                                  const int64_t* num_unique_dev, int64_t* out_perm, int64_t* out_bucket_sizes, int64_t* out_bucket_offsets,
+                                  const int64_t* head, int64_t num_head, const int64_t* num_head_dev, int64_t* out_all, int64_t* out_num_all,
+                                  const int64_t* feat_pos_map, int64_t feat_num_nodes, int64_t num_dev_rows, int64_t num_uva_rows,
+                                  int32_t* status_word, void* stream) {
+  using namespace apt;
+  int rc = uniq_sizes("apt_unique_inverse", num_ids, id_lo, id_hi);
+  if (rc != APT_OK) return rc;
+  APT_CHECK_ARG(ids_per >= 1 && (num_ids == 0 || out_inverse) && num_unique >= 0 && (num_unique == 0 || unique), "apt_unique_inverse: bad argument");
+  APT_CHECK_ARG(!out_bucket_sizes == !out_bucket_offsets && !out_bucket_sizes == !out_perm, "apt_unique_inverse: null pointer");
+  APT_CHECK_ARG(!out_all || (num_head >= 0 && (num_head == 0 || head) && num_unique_dev && status_word), "apt_unique_inverse: bad list");
+  cudaStream_t s = (cudaStream_t)stream;
+  if (num_ids == 0 || id_hi == id_lo) {
+    if (num_ids > 0) APT_CUDA(cudaMemsetAsync(out_inverse, 0xff, sizeof(int64_t) * num_ids, s));
+    if (out_bucket_sizes)      // (of distinct ids: there are none; of the ids themselves, if there are any)
+      APT_FOLLOW(k_bucket_one_rank, 1, 256, 0, s, ids, num_unique_dev ? 0 : num_ids, num_unique_dev ? nullptr : num_ids_dev, out_perm, out_perm,
+                 out_bucket_sizes, out_bucket_offsets);
+    return out_all ? apt_concat_row_ids(head, num_head, num_head_dev, nullptr, 0, nullptr, out_all, out_num_all, feat_pos_map, feat_num_nodes,
+                                        num_dev_rows, num_uva_rows, status_word, stream) : APT_OK;
+  }
+  UniqWs ws;
+  rc = uniq_check("apt_unique_inverse", ids, num_ids, id_lo, id_hi, workspace, workspace_bytes, out_inverse, &ws);
+  if (rc != APT_OK) return rc;
+  ProfScope prof("unique_sorted", s);
+  const OneRank one{out_perm, num_unique, num_unique_dev, out_bucket_sizes, out_bucket_offsets};
+  const ListOf list{head, num_head, num_head_dev, unique, num_unique, num_unique_dev, out_all, out_num_all,
+                    RowTables{feat_pos_map, feat_num_nodes, num_dev_rows, num_uva_rows}};
+  return uniq_inverse(ids, num_ids, num_ids_dev, ids_per, id_lo, id_hi, ws, out_inverse, one, list, status_word, s);
 }
 
 extern "C" int apt_concat_ids(const int64_t* a, int64_t num_a, const int64_t* num_a_dev, const int64_t* b,

@@ -128,6 +128,42 @@ k_sp_map_place_pack(const int64_t* __restrict__ nbr, const int64_t* __restrict__
   }
 }
 
+// Both sides of the hop in a world of one rank, which owns every node and sends to itself: neighbour i is of destination i / fanout, which is its
+// virtual node as well (owner 0), and every destination has neighbours, so the distinct virtual nodes are the
+// destinations in order. What bucketing, packing, unpacking and two sorted uniques over the virtual ids leave is written
+// as it is: 12 launches on three streams before (a mini-batch of 931 seeds x (25, 10), 128 columns: 187 -> 173 us with the list of the inverse).
+struct SpOneRank {
+  int64_t *sorted_vir, *packed, *vir_src, *ori_src, *dst_of;                       // [num_dst * fanout]
+  int64_t *unique_vir, *arange_src, *arange_dst, *unique_dst;                      // [num_dst]
+  int64_t *num_neighbors, *num_unique_vir, *num_unique_dst;
+};
+__global__ void __launch_bounds__(256)
+k_sp_one_rank(const int64_t* __restrict__ nbr, int64_t num_dst, const int64_t* __restrict__ num_dst_dev, int64_t fanout, int64_t num_total_nodes,
+              const SpOneRank o) {
+  wait_for_previous();
+  num_dst = effective_n(num_dst, num_dst_dev);
+  const int64_t n = num_dst * fanout, stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (first == 0) {
+    if (o.num_neighbors) *o.num_neighbors = n;
+    *o.num_unique_vir = *o.num_unique_dst = num_dst;
+  }
+  for (int64_t i = first; i < n; i += stride) {
+    const int64_t v = nbr[i], d = n >> 32 ? i / fanout : (int64_t)((uint32_t)i / (uint32_t)fanout);
+    const int64_t packed = d * num_total_nodes + v;
+    int64_t vir = d, ori = v;
+    if (v < 0 || v >= num_total_nodes) {      // no node (flagged by the sampling): as it would be unpacked
+      vir = packed / num_total_nodes;
+      ori = packed - vir * num_total_nodes;
+    }
+    o.sorted_vir[i] = d;
+    o.packed[i] = packed;
+    o.vir_src[i] = vir;
+    o.ori_src[i] = ori;
+    o.dst_of[i] = d;
+  }
+  for (int64_t i = first; i < num_dst; i += stride) o.unique_vir[i] = o.arange_src[i] = o.arange_dst[i] = o.unique_dst[i] = i;
+}
+
 static int check_owner_args(const char* who, int world_size, int shuffle_id_offset, int rank,
                             int node_beg, int node_end) {
   APT_CHECK_ARG(world_size >= 1 && world_size <= kMaxRanks, "%s: world_size %d outside [1,%d]", who,
@@ -252,5 +288,31 @@ extern "C" int apt_sp_map_place_pack(const int64_t* neighbors, const int64_t* po
   APT_FOLLOW(k_sp_map_place_pack, wave_grid(ceil_div(num_dst * fanout, 256), 8, 1), 256, 0, s, neighbors, positions,
              num_dst, num_dst_dev, fanout, min_vids, p, (int64_t)rank * sp_base * num_total_nodes, num_total_nodes,
              out_sorted_vir, out_packed, out_count);
+  return APT_OK;
+}
+
+extern "C" int apt_sp_one_rank(const int64_t* neighbors, int64_t num_dst, const int64_t* num_dst_dev, int64_t fanout, int64_t sp_base,
+                               int64_t num_total_nodes, int64_t* out_sorted_vir, int64_t* out_packed, int64_t* out_vir_src, int64_t* out_ori_src,
+                               int64_t* out_dst_of, int64_t* out_unique_vir, int64_t* out_arange_src, int64_t* out_arange_dst,
+                               int64_t* out_unique_dst, int64_t* out_num_neighbors, int64_t* out_num_unique_vir, int64_t* out_num_unique_dst,
+                               void* stream) {
+  using namespace apt;
+  APT_CHECK_ARG(num_dst >= 0 && fanout >= 1 && sp_base > 0 && num_total_nodes > 0, "apt_sp_one_rank: bad sizes");
+  APT_CHECK_ARG(num_dst <= sp_base, "apt_sp_one_rank: %lld destinations exceed sp_base %lld", (long long)num_dst, (long long)sp_base);
+  APT_CHECK_ARG((double)sp_base * (double)num_total_nodes < 9.2e18, "apt_sp_one_rank: packed id overflows 63 bits");
+  APT_CHECK_ARG(out_num_unique_vir && out_num_unique_dst, "apt_sp_one_rank: null output word");
+  cudaStream_t s = (cudaStream_t)stream;
+  if (num_dst == 0) {
+    if (out_num_neighbors) APT_CUDA(cudaMemsetAsync(out_num_neighbors, 0, 8, s));
+    APT_CUDA(cudaMemsetAsync(out_num_unique_vir, 0, 8, s));
+    APT_CUDA(cudaMemsetAsync(out_num_unique_dst, 0, 8, s));
+    return APT_OK;
+  }
+  APT_CHECK_ARG(neighbors && out_sorted_vir && out_packed && out_vir_src && out_ori_src && out_dst_of && out_unique_vir && out_arange_src &&
+                    out_arange_dst && out_unique_dst, "apt_sp_one_rank: null pointer");
+  ProfScope prof("sp_map_place_pack", s);
+  const SpOneRank o{out_sorted_vir, out_packed, out_vir_src, out_ori_src, out_dst_of, out_unique_vir, out_arange_src, out_arange_dst, out_unique_dst,
+                    out_num_neighbors, out_num_unique_vir, out_num_unique_dst};
+  APT_FOLLOW(k_sp_one_rank, wave_grid(ceil_div(num_dst * fanout, 256), 8, 1), 256, 0, s, neighbors, num_dst, num_dst_dev, fanout, num_total_nodes, o);
   return APT_OK;
 }

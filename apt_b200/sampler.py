@@ -12,7 +12,6 @@ buffers are narrowed to their real lengths. The results are identical to
 calling the operators one by one (``chained=False``), which reads a count
 after every relabelling like the reference does (src/cuda/relabel.cu:119).
 """
-import contextlib
 import os
 import queue
 import threading
@@ -206,6 +205,11 @@ class _GraphReplay:
         ops._gather_enqueue(input_nodes, in_word, out=rows, first_dev=cur_n, publish=publish)
         ops.STATE.join(2)
         return rows
+
+    @staticmethod
+    def _alone():
+        """Whether this rank exchanges nothing and side streams may be used."""
+        return ops._exchange().name == "local" and not ops.STATE.profiling
 
     @staticmethod
     def _leave_rows(input_nodes, rows, plan):
@@ -504,12 +508,18 @@ class MixedNeighborSampler(_GraphReplay):
         words = st.words()
         recv_view = words[16:16 + ws + 1]
         sizes_view = recv_view if ws == 1 else words[128:128 + ws + 1]
-        sorted_ids, perm, sizes, offsets = ops._bucket(cur, cur_n, sizes_view, words[64:64 + ws])
-        recv, recv_counts = ops._exchange().exchange_ids_enqueue(sorted_ids, sizes, offsets, recv_view)
-        total = recv_counts[ws:ws + 1]
         lo, hi = ops._owned_range()
         u_slot, in_slot = slot, slot + 1
-        uniq2, inv = ops._unique_enqueue(recv, total, lo, hi, st.word(u_slot), "unique_np")
+        alone = self._alone()
+        if alone:
+            # one rank receives what it has; what only the caller wants (the permutation, the sizes, the inverse) is made beside the outermost
+            # hop, of whose chain it was 5 us
+            uniq2 = ops._unique_ids(cur, cur_n, 1, lo, hi, st.word(u_slot), "unique_np")
+            inv, perm, _ = ops._unique_inverse(cur, cur_n, 1, lo, hi, "unique_np", sizes=sizes_view, offsets=words[64:64 + ws], side=3)
+        else:
+            sorted_ids, perm, sizes, offsets = ops._bucket(cur, cur_n, sizes_view, words[64:64 + ws])
+            recv, recv_counts = ops._exchange().exchange_ids_enqueue(sorted_ids, sizes, offsets, recv_view)
+            uniq2, inv = ops._unique_enqueue(recv, recv_counts[ws:ws + 1], lo, hi, st.word(u_slot), "unique_np")
         # The block of the outermost hop lists its destination nodes (the frontier uniq2, sorted and
         # distinct) first, so input row j is the row of uniq2[j] for j below the frontier's size: those
         # rows are fetched on a second stream while the hop is still being sampled and relabelled,
@@ -526,6 +536,8 @@ class MixedNeighborSampler(_GraphReplay):
                 ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier", beside=True)
         uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
                                                      call if explicit else None, call_base_dev, look_up=prefetch)
+        if alone:
+            st.join(3)      # the sizes leave with the counts
         if split == 1:
             if publish is not None:
                 publish()
@@ -606,22 +618,29 @@ class SPGATSampler(_GraphReplay):
         f = self.fanouts[0]
         rows = self._early_rows(cur, cur_n, min(cur.numel() * f, int(st.graph.num_total_nodes)))
         nbr = ops._sample(cur, f, cur_n, call if explicit else None, call_base_dev)
-        n_word = None
-        if cur_n is not None:
-            n_word = st.word(self._N)
-            torch.mul(cur_n, f, out=n_word)
         # sorted unique of the neighbours + the position of every neighbour in it (torch.unique with
         # return_inverse, python/npc/sampler.py:224-226)
-        u_word = st.word(self._U)
-        unique_neigh, arange_src = ops._unique_enqueue(nbr, n_word, 0, int(st.graph.num_total_nodes), u_word,
-                                                       "unique_gat")
+        u_word, in_word = st.word(self._U), st.word(self._IN)
+        n_total = int(st.graph.num_total_nodes)
         recv_view = words[16:16 + ws + 1]
         sizes_view = recv_view if ws == 1 else words[128:128 + ws + 1]
-        sorted_ids, perm, sizes, offsets = ops._bucket(unique_neigh, u_word, sizes_view, words[64:64 + ws])
-        recv, recv_counts = ops._exchange().exchange_ids_enqueue(sorted_ids, sizes, offsets, recv_view)
-        in_word = st.word(self._IN)
-        prefetch = self.prefetch_features and _fits_prefetch(cur.numel() + recv.numel())
-        input_nodes = ops.concat_ids(cur, cur_n, recv, recv_counts[ws:ws + 1], in_word, look_up=prefetch)
+        alone = self._alone()
+        if alone:
+            # one rank receives what it has: the permutation, the sizes and the input nodes are made with the inverse
+            prefetch = self.prefetch_features and _fits_prefetch(cur.numel() + min(nbr.numel(), n_total))
+            unique_neigh = ops._unique_ids(nbr, cur_n, f, 0, n_total, u_word, "unique_gat")
+            arange_src, perm, input_nodes = ops._unique_inverse(nbr, cur_n, f, 0, n_total, "unique_gat", unique_neigh, u_word, sizes_view,
+                                                                words[64:64 + ws], None, cur, cur_n, in_word, prefetch)
+        else:
+            n_word = None
+            if cur_n is not None:
+                n_word = st.word(self._N)
+                torch.mul(cur_n, f, out=n_word)
+            unique_neigh, arange_src = ops._unique_enqueue(nbr, n_word, 0, n_total, u_word, "unique_gat")
+            sorted_ids, perm, sizes, offsets = ops._bucket(unique_neigh, u_word, sizes_view, words[64:64 + ws])
+            recv, recv_counts = ops._exchange().exchange_ids_enqueue(sorted_ids, sizes, offsets, recv_view)
+            prefetch = self.prefetch_features and _fits_prefetch(cur.numel() + recv.numel())
+            input_nodes = ops.concat_ids(cur, cur_n, recv, recv_counts[ws:ws + 1], in_word, look_up=prefetch)
         rows = self._late_rows(input_nodes, in_word, cur_n, rows, publish) if prefetch else None
         return dict(layers=layers, outer=_layer(cur, arange_src, unique_neigh, f, self._U), perm=perm,
                     input_nodes=input_nodes, rows=rows)
@@ -733,84 +752,83 @@ class SPVirtualSampler(_GraphReplay):
         if self.model != "GCN" and not with_dst:
             rows = self._early_rows(cur, cur_n, min(n_max, max(hi - lo, 0)))
         nbr = ops._sample(cur, f, cur_n, call if explicit else None, call_base_dev)
-        n_word = None
-        if cur_n is not None:
-            n_word = st.word(self._N)
-            torch.mul(cur_n, f, out=n_word)
-        _, pos, _, _ = ops._bucket(nbr, n_word)
-        sorted_vir = torch.empty(n_max, dtype=torch.int64, device=dev)
-        packed = torch.empty(n_max, dtype=torch.int64, device=dev)
-        owner = ops._owner_args()
         n_total = int(st.graph.num_total_nodes)
-        check(lib.apt_sp_map_place_pack(ops._ptr(nbr), ops._ptr(pos), s_max, ops._ptr(cur_n), f, *owner, ops.SP_BASE,
-                                        n_total, ops._ptr(sorted_vir), ops._ptr(packed), None, ops._stream()))
-        uf_word = st.word(self._UF)
-        # the unique virtual nodes come from the ids as they stand (owner x num_dst + destination); with
-        # destinations every neighbour's id is shifted by world_size x num_dst afterwards, which keeps the order
-        # the three uniques of this sampler are small and wait mostly for memory: where they do not need one another's
-        # results they run side by side
-        beside = ws == 1 and not with_dst and not st.profiling
-        with st.beside(0) if beside else contextlib.nullcontext():
+        uf_word, n_word = st.word(self._UF), None
+        alone = not with_dst and self._alone()
+        if alone:
+            ops._owner_args()
+            vir_src, ori_src, a_dst, sorted_all, packed = (torch.empty(n_max, dtype=torch.int64, device=dev) for _ in range(5))
+            unique_frontier, arange_src, arange_dst, unique_dst = (torch.empty(s_max, dtype=torch.int64, device=dev) for _ in range(4))
+            check(lib.apt_sp_one_rank(ops._ptr(nbr), s_max, ops._ptr(cur_n), f, ops.SP_BASE, n_total, *map(ops._ptr, (
+                sorted_all, packed, vir_src, ori_src, a_dst, unique_frontier, arange_src, arange_dst, unique_dst)), None,
+                ops._ptr(uf_word), ops._ptr(st.word(self._UD)), ops._stream()))
+            recv_dst = dst_sorted = None
+            total, per = cur_n, f
+        else:
+            if cur_n is not None:
+                n_word = st.word(self._N)
+                torch.mul(cur_n, f, out=n_word)
+            _, pos, _, _ = ops._bucket(nbr, n_word)
+            sorted_vir = torch.empty(n_max, dtype=torch.int64, device=dev)
+            packed = torch.empty(n_max, dtype=torch.int64, device=dev)
+            owner = ops._owner_args()
+            check(lib.apt_sp_map_place_pack(ops._ptr(nbr), ops._ptr(pos), s_max, ops._ptr(cur_n), f, *owner, ops.SP_BASE,
+                                            n_total, ops._ptr(sorted_vir), ops._ptr(packed), None, ops._stream()))
+            # the unique virtual nodes come from the ids as they stand (owner x num_dst + destination); with
+            # destinations every neighbour's id is shifted by world_size x num_dst afterwards, which keeps the order
             unique_frontier, _ = ops._unique_enqueue(sorted_vir, n_word, 0, ws * max(s_max, 1), uf_word, "unique_vir")
-            # the two sides of block1's edges: tensors of their own, which a caller may change
-            arange_src = torch.arange(unique_frontier.numel(), device=dev)
-            arange_dst = unique_frontier.clone() if ws == 1 and not with_dst else None   # owner 0: its destination's index
-        dst_sorted = None
-        if with_dst:
-            dst_sorted, dst_pos, _, _ = ops._bucket(cur, cur_n)
-            dst_vir = torch.empty(s_max, dtype=torch.int64, device=dev)
-            scratch = torch.empty(s_max, dtype=torch.int64, device=dev)
-            # a destination is a neighbour list of length one: owner(destination) x num_dst + its index,
-            # placed by the bucket's positions (MapSrcDsttoVir, src/cuda/npc_kernel.cu:15-70)
-            check(lib.apt_sp_map_place_pack(ops._ptr(cur), ops._ptr(dst_pos), s_max, ops._ptr(cur_n), 1, *owner,
-                                            ops.SP_BASE, n_total, ops._ptr(dst_vir), ops._ptr(scratch), None,
-                                            ops._stream()))
-            shift = cur_n * ws if cur_n is not None else ws * s_max
-            sorted_src = sorted_vir + shift
-            unique_frontier = unique_frontier + shift
-            sorted_all = ops.concat_ids(dst_vir, cur_n, sorted_src, n_word, st.word(self._ALL))
-            all_word = st.word(self._ALL)
-        else:
-            sorted_all, all_word = sorted_vir, n_word
-        counts = words[16:16 + ws + 1]
-        dst_counts = words[self._RDST:self._RDST + ws + 1]
-        recv_dst = None
-        if ws == 1 and not with_dst:
-            recv, total = packed, n_word
-        else:
-            send_sizes = words[self._SEND:self._SEND + k * ws]
-            recv_sizes = words[self._RECV:self._RECV + k * ws]
-            check(lib.apt_vir_send_sizes(ops._ptr(sorted_all), sorted_all.numel(), ops._ptr(all_word),
-                                         ops._ptr(unique_frontier), unique_frontier.numel(), ops._ptr(uf_word), ws, s_max,
-                                         ops._ptr(cur_n), int(with_dst), None, ops._ptr(send_sizes), ops._stream()))
-            ex = ops._exchange()
-            ex.exchange_fixed(send_sizes.view(ws, k), recv_sizes.view(ws, k))
-            ids_at = 1 if with_dst else 0
-            if ws == 1:
-                recv = packed
-                counts[0:1].copy_(send_sizes[ids_at:ids_at + 1])
-                counts[1:2].copy_(send_sizes[ids_at:ids_at + 1])
-                recv_dst = dst_sorted
-                dst_counts[0:1].copy_(send_sizes[0:1])
-                dst_counts[1:2].copy_(send_sizes[0:1])
+            arange_src = torch.arange(unique_frontier.numel(), device=dev)      # a tensor of its own, which a caller may change
+            dst_sorted = None
+            if with_dst:
+                dst_sorted, dst_pos, _, _ = ops._bucket(cur, cur_n)
+                dst_vir = torch.empty(s_max, dtype=torch.int64, device=dev)
+                scratch = torch.empty(s_max, dtype=torch.int64, device=dev)
+                # a destination is a neighbour list of length one: owner(destination) x num_dst + its index,
+                # placed by the bucket's positions (MapSrcDsttoVir, src/cuda/npc_kernel.cu:15-70)
+                check(lib.apt_sp_map_place_pack(ops._ptr(cur), ops._ptr(dst_pos), s_max, ops._ptr(cur_n), 1, *owner,
+                                                ops.SP_BASE, n_total, ops._ptr(dst_vir), ops._ptr(scratch), None,
+                                                ops._stream()))
+                shift = cur_n * ws if cur_n is not None else ws * s_max
+                sorted_src = sorted_vir + shift
+                unique_frontier = unique_frontier + shift
+                sorted_all = ops.concat_ids(dst_vir, cur_n, sorted_src, n_word, st.word(self._ALL))
+                all_word = st.word(self._ALL)
             else:
-                if with_dst:
-                    recv_dst, _ = ex.exchange_ids_enqueue(dst_sorted, None, torch.cumsum(send_sizes[0::k], 0), dst_counts)
-                recv, _ = ex.exchange_ids_enqueue(packed, None, torch.cumsum(send_sizes[ids_at::k], 0), counts)
-            total = counts[ws:ws + 1]
-        vir_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
-        ori_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
-        check(lib.apt_sp_unpack_frontier(ops._ptr(recv), recv.numel(), ops._ptr(total), n_total,
-                                         ops._ptr(vir_src), ops._ptr(ori_src), ops._stream()))
-        with st.beside(1) if beside else contextlib.nullcontext():
+                sorted_all, all_word = sorted_vir, n_word
+            counts = words[16:16 + ws + 1]
+            dst_counts = words[self._RDST:self._RDST + ws + 1]
+            recv_dst = None
+            if ws == 1 and not with_dst:
+                recv, total = packed, n_word
+            else:
+                send_sizes = words[self._SEND:self._SEND + k * ws]
+                recv_sizes = words[self._RECV:self._RECV + k * ws]
+                check(lib.apt_vir_send_sizes(ops._ptr(sorted_all), sorted_all.numel(), ops._ptr(all_word),
+                                             ops._ptr(unique_frontier), unique_frontier.numel(), ops._ptr(uf_word), ws, s_max,
+                                             ops._ptr(cur_n), int(with_dst), None, ops._ptr(send_sizes), ops._stream()))
+                ex = ops._exchange()
+                ex.exchange_fixed(send_sizes.view(ws, k), recv_sizes.view(ws, k))
+                ids_at = 1 if with_dst else 0
+                if ws == 1:
+                    recv = packed
+                    counts[0:1].copy_(send_sizes[ids_at:ids_at + 1])
+                    counts[1:2].copy_(send_sizes[ids_at:ids_at + 1])
+                    recv_dst = dst_sorted
+                    dst_counts[0:1].copy_(send_sizes[0:1])
+                    dst_counts[1:2].copy_(send_sizes[0:1])
+                else:
+                    if with_dst:
+                        recv_dst, _ = ex.exchange_ids_enqueue(dst_sorted, None, torch.cumsum(send_sizes[0::k], 0), dst_counts)
+                    recv, _ = ex.exchange_ids_enqueue(packed, None, torch.cumsum(send_sizes[ids_at::k], 0), counts)
+                total = counts[ws:ws + 1]
+            vir_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
+            ori_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
+            check(lib.apt_sp_unpack_frontier(ops._ptr(recv), recv.numel(), ops._ptr(total), n_total,
+                                             ops._ptr(vir_src), ops._ptr(ori_src), ops._stream()))
+            per = 1
             unique_dst, a_dst = ops._unique_enqueue(vir_src, total, 0, ws * ops.SP_BASE, st.word(self._UD), "unique_vdst")
-        unique_src, a_src = ops._unique_enqueue(ori_src, total, lo, hi, st.word(self._US), "unique_sp_src")
-        if beside:
-            st.join(0)
-            st.join(1)
-        if arange_dst is None:
             arange_dst = torch.remainder(unique_frontier, cur_n if cur_n is not None else max(s_max, 1))
-        # the input nodes (the reference's torch.cat of destinations and received neighbours)
+        # the input nodes (the reference's torch.cat of destinations and received neighbours), made with the latter's inverse
         us_word = st.word(self._US)
         none = torch.empty(0, dtype=torch.int64, device=dev)
         if with_dst:
@@ -820,8 +838,10 @@ class SPVirtualSampler(_GraphReplay):
         else:
             head, head_n = cur, cur_n
         in_word = st.word(self._IN)
-        prefetch = self.prefetch_features and _fits_prefetch(head.numel() + unique_src.numel())
-        input_nodes = ops.concat_ids(head, head_n, unique_src, us_word, in_word, look_up=prefetch)
+        prefetch = self.prefetch_features and _fits_prefetch(head.numel() + min(ori_src.numel(), max(hi - lo, 0)))
+        unique_src = ops._unique_ids(ori_src, total, per, lo, hi, us_word, "unique_sp_src")
+        a_src, _, input_nodes = ops._unique_inverse(ori_src, total, per, lo, hi, "unique_sp_src", unique_src, us_word, head=head,
+                                                    head_n=head_n, all_out=in_word, look_up=prefetch)
         rows = self._late_rows(input_nodes, in_word, cur_n, rows, publish) if prefetch else None
         return dict(layers=layers, cur=cur, nbr=nbr, sorted_all=sorted_all, packed=packed,
                     unique_frontier=unique_frontier, arange_src=arange_src, arange_dst=arange_dst, vir_src=vir_src, ori_src=ori_src,

@@ -261,6 +261,26 @@ int apt_unique_sorted(const int64_t* ids, int64_t num_ids,
                       int64_t* out_unique, int64_t* out_inverse,
                       int64_t* out_num_unique, int32_t* status_word,
                       void* stream);
+/* The same in two calls, so that what is made of the distinct ids need not wait for the inverse (which may be enqueued on a stream that
+ * waits for the first): apt_unique_inverse has to follow apt_unique_ids, with the same ids and workspace, before that is used again. With
+ * num_ids_dev the number of ids is *num_ids_dev * ids_per (at most num_ids).
+ * The second call also leaves, where it is asked to (each may be NULL):
+ *   out_perm, out_bucket_sizes, out_bucket_offsets   what apt_bucket_by_owner leaves in a world of one rank, of the ids or, with num_unique_dev
+ *                        (unique: the first call's result, num_unique its bound, num_unique_dev its count), of the distinct ones
+ *   out_all              head[0 .. num_head) (num_head_dev: a device count, at most num_head), then unique; their number in *out_num_all
+ *                        (may be NULL). With feat_pos_map the list's ids are those of a gather, flag what it would flag
+ *                        (as apt_concat_row_ids). */
+int apt_unique_ids(const int64_t* ids, int64_t num_ids, const int64_t* num_ids_dev, int64_t ids_per, int64_t id_lo, int64_t id_hi,
+                   void* workspace, size_t workspace_bytes, int64_t* out_unique, int64_t* out_num_unique,
+                   int32_t* status_word, void* stream);
+int apt_unique_inverse(const int64_t* ids, int64_t num_ids, const int64_t* num_ids_dev, int64_t ids_per, int64_t id_lo, int64_t id_hi,
+                       void* workspace, size_t workspace_bytes, int64_t* out_inverse,
+                       const int64_t* unique, int64_t num_unique, const int64_t* num_unique_dev,
+                       int64_t* out_perm, int64_t* out_bucket_sizes, int64_t* out_bucket_offsets,
+                       const int64_t* head, int64_t num_head, const int64_t* num_head_dev, int64_t* out_all, int64_t* out_num_all,
+                       const int64_t* feat_pos_map, int64_t feat_num_nodes, int64_t num_dev_rows, int64_t num_uva_rows,
+                       int32_t* status_word, void* stream);
+
 
 /* ---------------------------------------------------------------- gather
  * Cache-aware feature-row gather. Takes the role of IndexSelectAll /
@@ -529,6 +549,13 @@ int apt_sp_map_place_pack(const int64_t* neighbors, const int64_t* positions,
                           int node_end, int64_t sp_base, int64_t num_total_nodes,
                           int64_t* out_sorted_vir, int64_t* out_packed,
                           int64_t* out_count, void* stream);
+/* The whole hop where one rank owns every node (nothing is sent): what apt_bucket_by_owner, apt_sp_map_place_pack, apt_sp_unpack_frontier and
+ * apt_unique_sorted over both sides' virtual ids leave there. out_dst_of: the inverse of the received virtual ids; the distinct
+ * virtual ids of both sides and the two sides of their block's edges (out_arange_*) are 0 .. num_dst - 1. */
+int apt_sp_one_rank(const int64_t* neighbors, int64_t num_dst, const int64_t* num_dst_dev, int64_t fanout, int64_t sp_base,
+                    int64_t num_total_nodes, int64_t* out_sorted_vir, int64_t* out_packed, int64_t* out_vir_src, int64_t* out_ori_src,
+                    int64_t* out_dst_of, int64_t* out_unique_vir, int64_t* out_arange_src, int64_t* out_arange_dst, int64_t* out_unique_dst,
+                    int64_t* out_num_neighbors /* may be NULL */, int64_t* out_num_unique_vir, int64_t* out_num_unique_dst, void* stream);
 int apt_sp_pack_frontier(const int64_t* sorted_vir, const int64_t* sorted_ids,
                          int64_t n, int64_t num_dst, int rank, int64_t sp_base,
                          int64_t num_total_nodes, int64_t* out, void* stream);

@@ -9,6 +9,16 @@ from apt_b200 import _lib
 from tests.gpu_util import dev
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _own_tables():
+    """The tables installed before come back."""
+    saved, ops.STATE.feat = ops.STATE.feat, ops.FeatStorage()
+    yield
+    ops.STATE.feat = saved
+    ops.STATE.generation += 1
+
 TYPES = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}
 
 
