@@ -16,8 +16,8 @@
 //   k_gat_weights   scores and softmax, a few lanes per destination and up to four of its heads, two edges a lane; any number of
 //                   edges and heads.
 //   sums            the weighted sum is the SpMM's (kUMulW), any head width: k_spmm_stream for wide rows of many edges, else k_spmm_rows
-//   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination (wide rows of many edges:
-//                   k_spmm_stream's kDots). The four partial dots of a lane are reduced together: each step halves the values
+//   k_gat_dots      backward: <g, ft> of every edge and head, one warp per destination (16-bit heads of 32 to 256 columns: k_gat_dots_mma,
+//                   gat_dots.cuh; other wide rows of many edges: k_spmm_stream's kDots). The four partial dots of a lane are reduced together: each step halves the values
 //                   a lane keeps, log2(lph) + 1 shuffles for four edges instead of 4 log2(lph).
 //   k_gat_scores    backward: t, grad_s and grad_er, the same lanes; grad_el is added up in fp32 with one reduction per edge
 //                   of up to four of its heads
@@ -34,12 +34,13 @@
 //
 // One kernel that did scores and rows in turn (a warp per destination) was bound by the registers of the one
 // and the latency of the other: 133 - 149 us forward on 67 584 x 15 edges, bf16, 4 x 64, in three forms; the two
-// kernels take 16 + 61 us. Backward of that block: 16 (saved after a forward) + 79 + 5 + 31 + 75 + 4 us (each kernel by itself, caches
+// kernels take 16 + 61 us. Backward of that block: 16 (saved after a forward) + 56 + 5 + 31 + 75 + 4 us (each kernel by itself, caches
 // cold), where the edge kernel and two reverse SpMM calls with a sort each took 803 us.
 #include <math.h>
 
 #include <algorithm>
 
+#include "gat_dots.cuh"
 #include "spmm_rows.cuh"
 
 namespace apt {
@@ -664,6 +665,9 @@ template <typename T>
 static int gat_dots(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, int64_t num_src, cudaStream_t s) {
   const int64_t dim = q.H * q.Dh;
   const int slice = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T);
+  if constexpr (sizeof(T) == 2)
+    if (dots_mma_fits(q.H, q.Dh, slice, q.E))
+      return launch_dots_mma<T>(q.H, q.Dh, q.row, q.col, (const T*)q.ft, (const T*)q.grad_out, q.E, q.num_dst, g.none, ws.dots, (uint32_t)num_src, ws.sort, s);
   if (stream_fits(kDots, slice, dim, sizeof(T), q.H, q.E, true)) {
     SpmmWs counts = ws.sort;
     counts.range = g.range;

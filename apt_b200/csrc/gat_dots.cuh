@@ -1,0 +1,206 @@
+// The attention backward's dots <grad_out[dst], ft[src]> of every edge and head on the tensor cores, for 16-bit rows whose heads are 32, 64,
+// 128 or 256 columns wide.
+//
+// A warp takes a stretch of the edges, 16 of them (M) against 8 destinations (N) a step: the edges' rows come to shared memory by cp.async, two
+// groups on their way, the destinations' stay in registers while the edges, which are grouped, walk over them. Of the 16 x 8
+// products of a head one in eight is an edge's own; what the others cost is 32 instructions a group of 256 columns, where multiplying and
+// reducing across lanes took 46 an edge. The k of a product may be in any order, so a lane's share of two steps is 16 bytes side by
+// side in both operands: one load each. Sums are fp32 as they were: the gradients' distance from 64 bits is the same to seven digits.
+//
+// Bound by rows out of L2 (43 us for a million rows of 512 bytes however they are fetched) and the atomics that count the
+// edges of every source for the sort behind. us of the dots, multiplied out -> here: bf16 4 x 64, 67 584 x 15 edges 75 -> 56, x 3 edges 40 -> 22,
+// 30 000 x 10 35 -> 21, 5 000 x 10 8.6 -> 6.0; f16 4 x 32, 40 000 x 15 32 -> 21, 2 x 32 20 -> 18, 2 x 32 x 3 edges 18.6 -> 6.3, bf16 1 x 32,
+// 55 721 x 17 28 -> 18; 1 000 x 10 of 8 x 32 4.9 -> 4.1. So they take every shape they can be built for. (Shared addresses worked out for
+// every access and a predicate for every row, 27 instructions an edge: 62 instead of 56.)
+#pragma once
+
+#include "spmm_rows.cuh"
+
+namespace apt {
+
+constexpr int kDotsBlocks = 2, kDotsEdges = 16, kDotsTile = 8;
+// Warps a block: as many as shared memory (rows of 512 bytes) or registers hold.
+constexpr int dots_warps(int chunks) { return chunks == 8 ? 6 : chunks == 4 ? 10 : 14; }
+
+template <typename T>
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, bool first) {
+  const float c0 = first ? 0.f : d[0], c1 = first ? 0.f : d[1], c2 = first ? 0.f : d[2], c3 = first ? 0.f : d[3];
+  if constexpr (Elem<T>::kIsBf16)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// NC chunks of 32 columns to a row, CPH of them to a head.
+template <typename T, int NC, int CPH>
+__global__ void __launch_bounds__(dots_warps(NC) * 32, kDotsBlocks)
+k_gat_dots_mma(const int64_t* __restrict__ row, const int64_t* __restrict__ col, const T* __restrict__ ft, const T* __restrict__ grad, int64_t E,
+               int64_t num_dst, int chunk, const Verdict none, float* __restrict__ dots, uint32_t num_src, int32_t* __restrict__ src_count,
+               uint32_t* __restrict__ rank) {
+  wait_for_previous();
+  constexpr int H = NC / CPH, kRow = NC * 64, kVectors = NC * 4, kSide = 32 / kVectors;      // vectors of 16 bytes to a row, rows a copy instruction
+  extern __shared__ __align__(128) unsigned char shared[];
+  if (any_found(none)) return;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warp = blockIdx.x * dots_warps(NC) + (threadIdx.x >> 5);
+  unsigned char* const ring = shared + (threadIdx.x >> 5) * 2 * kDotsEdges * kRow;
+  const int lo = (int)min((int64_t)warp * chunk, E), hi = (int)min((int64_t)(warp + 1) * chunk, E);
+  if (lo >= hi) return;
+
+  struct Batch {      // 32 edges, a lane to each
+    uint32_t src, dst, place;
+  };
+  auto load = [&](int base) {
+    Batch b{0u, 0xffffffffu, kNoRank};
+    const int e = base + lane;
+    if (e < hi) {
+      b.src = (uint32_t)row[e], b.dst = (uint32_t)col[e];
+      if (b.src < num_src) b.place = (uint32_t)atomicAdd(src_count + spread(b.src), 1);
+    }
+    return b;
+  };
+  // Vector v of row q of a stage. Neighbouring rows' halves of a line change places, so that eight lanes read eight different vectors: the
+  // address of an even chunk and that of an odd one, beside which all others are constants.
+  const int vec = lane % kVectors, side = lane / kVectors;
+  const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
+  const uint32_t put_even = ring_at + side * kRow + (NC > 1 ? vec ^ ((side & 1) << 2) : vec) * 16;
+  const uint32_t put_odd = ring_at + side * kRow + (NC > 1 ? vec ^ ((~side & 1) << 2) : vec) * 16;
+  const unsigned char* const get_even = ring + g * kRow + ((NC > 1 ? (g & 1) * 4 : 0) + t) * 16;
+  const unsigned char* const get_odd = ring + g * kRow + (NC > 1 ? (~g & 1) * 4 + t : t) * 16;
+  const char* const lane_ft = (const char*)ft + vec * 16;
+  auto copy = [&](int stage, int q, uint32_t src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((kSide & 1 && q & 1 ? put_odd : put_even) + (stage * kDotsEdges + q) * kRow),
+                 "l"(lane_ft + (uint64_t)src * kRow) : "memory");
+  };
+  auto issue = [&](uint32_t batch_src, int first, int count, int stage) {
+    if (count >= kDotsEdges) {
+#pragma unroll
+      for (int q = 0; q < kDotsEdges; q += kSide) copy(stage, q, __shfl_sync(0xffffffffu, batch_src, first + q + side));
+    } else {
+#pragma unroll 1
+      for (int q = 0; q < count; q += kSide) {      // (rows behind the last edge's: row 0)
+        const uint32_t src = __shfl_sync(0xffffffffu, batch_src, first + q + side);
+        copy(stage, q, src);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  Batch now = load(lo), next = load(lo + 32);
+  issue(now.src, 0, hi - lo, 0);
+  issue(now.src, kDotsEdges, hi - lo - kDotsEdges, 1);
+
+  uint32_t tile = 0xfffffff0u;      // destinations in registers: tile ... tile + 7
+  uint4 b[NC];
+  const T* const lane_grad = grad + t * 8;
+#pragma unroll 1
+  for (int base = lo; base < hi; base += 32) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int pos = half * kDotsEdges, count = min(kDotsEdges, hi - base - pos);
+      if (count <= 0) break;
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      const uint32_t d0 = __shfl_sync(0xffffffffu, now.dst, pos + g), d1 = __shfl_sync(0xffffffffu, now.dst, pos + g + 8);
+      uint32_t first = __shfl_sync(0xffffffffu, now.dst, pos);
+      const uint32_t last = __shfl_sync(0xffffffffu, now.dst, pos + count - 1);
+#pragma unroll 1
+      for (;;) {
+        if (first - tile >= kDotsTile) {
+          tile = first;
+          const T* const own = lane_grad + min((uint64_t)tile + g, (uint64_t)num_dst - 1) * (NC * 32);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) b[c] = __ldg((const uint4*)(own + c * 32));
+        }
+        float acc[H][4];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const unsigned char* const p = (c & 1 ? get_odd : get_even) + half * kDotsEdges * kRow + (c & ~1) * 64;
+          const uint4 x = *(const uint4*)p, y = *(const uint4*)(p + 8 * kRow);
+          mma_16x8x16<T>(acc[c / CPH], x.x, y.x, x.y, y.y, b[c].x, b[c].y, c % CPH == 0);
+          mma_16x8x16<T>(acc[c / CPH], x.z, y.z, x.w, y.w, b[c].z, b[c].w, false);
+        }
+        // an edge's own product is with the lane that has its destination's column
+        float* const out = dots + (int64_t)(base + pos + g) * H;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t s = (i ? d1 : d0) - tile;
+          if ((s >> 1) == (uint32_t)t) {
+            float v[H];
+#pragma unroll
+            for (int h = 0; h < H; ++h) v[h] = s & 1u ? acc[h][2 * i + 1] : acc[h][2 * i];
+            if constexpr (H % 4 == 0) {
+#pragma unroll
+              for (int h = 0; h < H; h += 4) *(float4*)(out + 8 * i * H + h) = make_float4(v[h], v[h + 1], v[h + 2], v[h + 3]);
+            } else if constexpr (H == 2) {
+              *(float2*)(out + 8 * i * H) = make_float2(v[0], v[1]);
+            } else {
+              out[8 * i * H] = v[0];
+            }
+          }
+        }
+        if (last - tile < kDotsTile) break;
+        // the first edge of the group whose destination lies behind these
+        const unsigned behind = __ballot_sync(0xffffffffu, lane >= pos && lane < pos + count && now.dst >= tile + kDotsTile);
+        if (!behind) break;      // (not of edges that rise)
+        first = __shfl_sync(0xffffffffu, now.dst, __ffs(behind) - 1);
+      }
+      __syncwarp();      // read by all lanes: the next copies may overwrite it
+      issue(next.src, pos, hi - base - 32 - pos, half);
+    }
+    if (base + lane < hi) rank[base + lane] = now.place;
+    now = next;
+    next = load(base + 64);
+  }
+}
+
+// slice: bytes of the widest access to both sides' rows.
+inline bool dots_mma_fits(int heads, int64_t head_dim, int slice, int64_t num_edges) {
+  const int64_t dim = heads * head_dim;
+  auto pow2 = [](int64_t x) { return x > 0 && (x & (x - 1)) == 0; };
+  return slice == 16 && num_edges <= kStreamMaxEdges && head_dim >= 32 && dim <= 256 && pow2(head_dim) && pow2(heads);
+}
+
+template <typename T, int NC, int CPH>
+static int launch_dots_mma(const int64_t* row, const int64_t* col, const T* ft, const T* grad, int64_t E, int64_t num_dst, const Verdict& none,
+                           float* dots, uint32_t num_src, const SpmmWs& sort, cudaStream_t s) {
+  constexpr int kWarps = dots_warps(NC), kShared = kWarps * 2 * kDotsEdges * NC * 64;
+  static bool sized[64] = {};
+  int dev = 0;
+  APT_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !sized[dev]) {
+    APT_CUDA(cudaFuncSetAttribute(k_gat_dots_mma<T, NC, CPH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShared));
+    if (dev < 64) sized[dev] = true;
+  }
+  // stretches of whole groups, as many as there are warps; of 32 edges at least
+  const int64_t warps = (int64_t)kNumSMs * kDotsBlocks * kWarps;
+  const int64_t chunk = std::max<int64_t>(32, ceil_div(ceil_div(E, warps), kDotsEdges) * kDotsEdges);
+  APT_FOLLOW((k_gat_dots_mma<T, NC, CPH>), (int)ceil_div(ceil_div(E, chunk), kWarps), kWarps * 32, kShared, s, row, col, ft, grad, E, num_dst,
+             (int)chunk, none, dots, num_src, sort.cnt, sort.rank);
+  return APT_OK;
+}
+
+template <typename T>
+static int launch_dots_mma(int heads, int64_t head_dim, const int64_t* row, const int64_t* col, const T* ft, const T* grad, int64_t E, int64_t num_dst,
+                           const Verdict& none, float* dots, uint32_t num_src, const SpmmWs& sort, cudaStream_t s) {
+#define APT_DOTS(NC, CPH) \
+  if (heads * head_dim == (NC) * 32 && head_dim == (CPH) * 32) return launch_dots_mma<T, NC, CPH>(row, col, ft, grad, E, num_dst, none, dots, num_src, sort, s)
+  APT_DOTS(1, 1);
+  APT_DOTS(2, 1);
+  APT_DOTS(4, 1);
+  APT_DOTS(8, 1);
+  APT_DOTS(2, 2);
+  APT_DOTS(4, 2);
+  APT_DOTS(8, 2);
+  APT_DOTS(4, 4);
+  APT_DOTS(8, 4);
+  APT_DOTS(8, 8);
+#undef APT_DOTS
+  set_error("apt_gat_backward: %d heads of %lld columns have no product kernel", heads, (long long)head_dim);
+  return APT_ERR_BAD_ARG;
+}
+
+}  // namespace apt

@@ -1,0 +1,59 @@
+"""The attention backward's dots by tensor-core products of 16 edges with 8 destinations: every split of a row into heads that they take, groups of
+edges whose destinations fill one tile of them, several, or lie far apart, stretches that end inside a group, and infinite rows, which are
+nobody else's business. Against the fp64 oracle, bounds as in test_gpu_gat.py."""
+import numpy as np
+import pytest
+import torch
+
+from apt_b200 import ops
+from oracle import oracle as orc
+from tests.gpu_util import dev, host
+
+pytestmark = pytest.mark.gpu
+SPLITS = [(1, 32), (2, 32), (4, 32), (8, 32), (1, 64), (2, 64), (4, 64), (1, 128), (2, 128), (1, 256)]
+LENGTHS = {
+    "one each": [1] * 75, "three each": [3] * 331, "fifteen each": [15] * 70, "long": [500, 1, 700, 0, 90],
+    "gaps": [2, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 5, 1, 0, 0, 0, 0, 0, 0, 0, 0, 30, 0, 7] * 3, "one": [1], "sixteen": [16], "seventeen": [17],
+    "a warp's": [31, 1], "and one more": [31, 2],
+}
+
+
+def _round(x, dtype):
+    return torch.from_numpy(x).to(dtype).float().numpy()
+
+
+def _inputs(lengths, H, D, dtype, n_src=90):
+    rng = np.random.default_rng(H * 1000 + D + len(lengths))
+    col = np.repeat(np.arange(len(lengths)), lengths).astype(np.int64)
+    row = rng.integers(0, n_src, len(col)).astype(np.int64)
+    make = lambda *shape: _round(rng.standard_normal(shape).astype(np.float32), dtype)      # noqa: E731
+    return row, col, make(n_src, H, D), make(n_src, H), make(len(lengths), H), make(len(lengths), H, D)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,D", SPLITS)
+@pytest.mark.parametrize("lengths", sorted(LENGTHS))
+def test_gradients(dtype, H, D, lengths):
+    n = LENGTHS[lengths]
+    row, col, ft, el, er, go = _inputs(n, H, D, dtype)
+    want = orc.gat_edge_softmax_sum_backward(row, col, ft, el, er, go, len(n), 0.2)[:3]
+    got = ops.gat_edge_softmax_sum_backward(dev(row), dev(col), *(dev(x, dtype) for x in (ft, el, er, go)), 0.2)
+    for a, b, name in zip(got, want, ("ft", "el", "er")):
+        err = np.abs(host(a).astype(np.float64).reshape(b.shape) - b).max() / max(np.abs(b).max(), 1.0)
+        assert err <= 1e-2, f"grad_{name}: {err:.2e}"
+    ops.check_status()
+
+
+def test_infinite_rows_stay_with_their_edges():
+    H, D, n = 4, 64, [3] * 40
+    row, col, ft, el, er, go = _inputs(n, H, D, torch.bfloat16)
+    row[:] = np.arange(len(row)) % 80
+    clean = [host(x) for x in ops.gat_edge_softmax_sum_backward(dev(row), dev(col), *(dev(x, torch.bfloat16) for x in (ft, el, er, go)), 0.2)]
+    ft[85] = np.inf      # of no edge
+    ft[7, 1] = np.inf
+    got = [host(x) for x in ops.gat_edge_softmax_sum_backward(dev(row), dev(col), *(dev(x, torch.bfloat16) for x in (ft, el, er, go)), 0.2)]
+    hit = np.unique(col[row == 7])
+    others = np.setdiff1d(np.arange(len(n)), hit)
+    er_got, er_clean = (x.reshape(len(n), H) for x in (got[2], clean[2]))
+    assert np.array_equal(er_got[others], er_clean[others]) and np.array_equal(er_got[:, [0, 2, 3]], er_clean[:, [0, 2, 3]])
+    assert not np.isfinite(er_got[hit, 1]).any()
