@@ -125,8 +125,15 @@ inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t n
   // 64 -> 98 us for bf16 x 256.
   r.vpl = nvec <= 32 ? 1 : nvec <= 64 ? 2 : 4;
   r.lpe = pow2_ge(ceil_div(nvec, r.vpl));
-  // edges side by side: never more than half the mean row, whose second half would idle those lanes
-  r.ep = pow2_le(num_edges / (num_rows * 2), 32 / r.lpe);
+  // Edges side by side: as many as fill the chip's lanes, never more than half the mean row, whose second half would idle those lanes. Where
+  // the rows fill the chip by themselves they go side by side instead: no sums to join, and rows of 15 edges are walked in as many
+  // steps by half the warps. us, as many edges as go -> rows first (42 727 x 15 edges unless it says so; forward | reverse):
+  // bf16 x 128 32 -> 24.5 | 48 -> 36, x 64 22 -> 13 | 29.5 -> 24, fp32 x 64 30 -> 24 | 48 -> 36, x 32 21 -> 13.7 | 29 -> 23, 60 000 x 8 of bf16 x 10
+  // 20.5 -> 8.1, 5 000 x 15 of fp32 x 64 6.7 -> 5.6; 1 000 x 15, which do not fill it, stay as they are (one by one 4.5 -> 5.1). Four
+  // lanes to a row at least: with two, rows of very different lengths wait for one another (67 000 x 15 of bf16 x 4 11 -> 17 | 19 -> 27).
+  const int most = pow2_le(num_edges / (num_rows * 2), 32 / r.lpe);
+  r.ep = 1;
+  while (r.ep < most && (r.lpe * r.ep < 4 || num_rows * r.lpe * r.ep * 2 <= (int64_t)kNumSMs * 24 * 32)) r.ep <<= 1;
   r.long_edges = r.lpe * r.ep == 32 ? kLongRow : kLongRowNarrow;
   return r;
 }
