@@ -77,6 +77,9 @@ PROTOTYPES = {
     "apt_spmm_probe": (c_int, [P, c_int64, P, P, c_int, P, P]),
     "apt_spmm_sum_known": (c_int, [c_int, c_int, P, P, c_int64, P, P, c_int64, c_int64, P, P, P, c_int, c_int64, c_int, c_int,
                                    P, P, c_size_t, P]),
+    "apt_spmm_widened_bytes": (c_size_t, [c_int, c_int64, c_int64, c_int64, c_int]),
+    "apt_spmm_copy_u_widened": (c_int, [c_int, P, P, c_int64, P, c_int64, c_int64, P, P, P, c_int, c_int64, c_int, c_int, P, P, c_size_t,
+                                        P, c_size_t, P]),
     "apt_sddmm": (c_int, [c_int, c_int, P, P, c_int64, P, P, c_int64, P, P, P, c_int, P, P]),
     "apt_gat_edge_softmax_sum": (c_int, [c_int, P, P, c_int64, P, P, P, c_int, c_int64, c_float, c_int64, P, P, P, c_size_t, P, P]),
     "apt_gat_edge_backward": (c_int, [c_int, P, P, c_int64, P, P, P, P, c_int, c_int64, c_float, c_int64, P, P, P, P, c_size_t, P, P]),

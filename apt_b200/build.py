@@ -16,7 +16,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libapt_b200.so")
 NATIVE = os.path.join(PKG_DIR, "native")
 NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
-SOURCES = ["core.cu", "sample.cu", "relabel.cu", "bucket.cu", "gather.cu", "spmm.cu", "spmm_f32.cu", "spmm_bf16.cu",
+SOURCES = ["core.cu", "sample.cu", "relabel.cu", "bucket.cu", "gather.cu", "spmm.cu", "widen.cu", "spmm_f32.cu", "spmm_bf16.cu",
            "spmm_f16.cu", "gat.cu", "virt.cu", "hotness.cu", "p2p.cu", "util.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -621,17 +621,18 @@ static size_t elem_size(int dtype) { return dtype == APT_F32 ? 4 : 2; }
 template <typename T>
 static int run_rows(int op, const RowSplit& split, const int64_t* row, const int64_t* col, int64_t E, const void* in, const void* edata,
                     int64_t edata_dim, int64_t feat_dim, SegTable st, int64_t num_rows, const SpmmWs& ws, int mode, int fixed,
-                    void* out, cudaStream_t s) {
+                    void* out, int64_t width, cudaStream_t s) {
   const RowArgs<T> a{row, (const T*)in, (const T*)edata, edata_dim, feat_dim, st, num_rows, E, ws, (T*)out,
-                     mode, fixed, split, (int)feat_dim, Verdict{}, nullptr, col, nullptr, nullptr, 0u};
+                     mode, fixed, split, (int)feat_dim, Verdict{}, nullptr, col, nullptr, nullptr, 0u, width};
   ProfScope prof("spmm_rows", s);
   return launch_spmm_rows<T>(op, a, s);
 }
 
-// Everything behind the argument checks; mode kDevice: nothing is known about the block yet.
+// Everything behind the argument checks; mode kDevice: nothing is known about the block yet. `width`: RowArgs (no slice of the result is
+// aligned then, and the input is).
 static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t E, const void* input,
                     const void* edata, int64_t edata_dim, int64_t feat_dim, SegTable st, int64_t num_rows, void* out,
-                    void* workspace, size_t workspace_bytes, int mode, int fixed, cudaStream_t s) {
+                    void* workspace, size_t workspace_bytes, int mode, int fixed, int64_t width, cudaStream_t s) {
   const size_t esz = elem_size(dtype);
   SpmmWs ws{};
   if (mode != kFixed) {
@@ -643,7 +644,7 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
     }
   }
   // edge values are read in slices only when there is one per column
-  uint64_t bits = (uint64_t)(feat_dim * esz) | (uintptr_t)out;
+  uint64_t bits = (uint64_t)(feat_dim * esz) | (width ? 0 : (uintptr_t)out);
   if (op != kCopyE) bits |= (uintptr_t)input;
   if (op != kCopyU && edata_dim == feat_dim) bits |= (uintptr_t)edata;
   const RowSplit split = row_split(feat_dim, slice_elems(bits, (int)esz), E, num_rows);
@@ -664,9 +665,9 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
     if (rc != APT_OK) return rc;
   }
   switch (dtype) {
-    case APT_F32: return run_rows<float>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
-    case APT_BF16: return run_rows<__nv_bfloat16>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
-    default: return run_rows<__half>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, s);
+    case APT_F32: return run_rows<float>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, width, s);
+    case APT_BF16: return run_rows<__nv_bfloat16>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, width, s);
+    default: return run_rows<__half>(op, split, coo_row, coo_col, E, input, edata, edata_dim, feat_dim, st, num_rows, ws, mode, fixed, out, width, s);
   }
 }
 
@@ -757,7 +758,45 @@ extern "C" int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row, con
                 "apt_spmm_sum: null pointer");
   const SegTable st{coo_offset, input_offset, output_offset, num_segments};
   return spmm_run(op, dtype, coo_row, coo_col, num_edges, input, edata, edata_dim, feat_dim, st, num_out_rows, out,
-                  workspace, workspace_bytes, mode, fixed, s);
+                  workspace, workspace_bytes, mode, fixed, 0, s);
+}
+
+extern "C" size_t apt_spmm_widened_bytes(int dtype, int64_t num_edges, int64_t num_input_rows, int64_t feat_dim, int mode) {
+  using namespace apt;
+  if (dtype < APT_F32 || dtype > APT_F16 || num_edges < 0 || feat_dim <= 0 || mode < kFixed || mode > kOrder) return 0;
+  const size_t esz = elem_size(dtype);
+  return widen_pays(feat_dim, esz, num_input_rows, num_edges, mode != kOrder) ? (size_t)num_input_rows * widened_dim(feat_dim, esz) * esz : 0;
+}
+
+extern "C" int apt_spmm_copy_u_widened(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges, const void* input,
+                                       int64_t num_input_rows, int64_t feat_dim, const int64_t* coo_offset,
+                                       const int64_t* input_offset, const int64_t* output_offset, int num_segments,
+                                       int64_t num_out_rows, int mode, int fixed, void* out, void* widened, size_t widened_bytes,
+                                       void* workspace, size_t workspace_bytes, void* stream) {
+  using namespace apt;
+  const size_t need = apt_spmm_widened_bytes(dtype, num_edges, num_input_rows, feat_dim, mode);
+  if (need == 0 || num_out_rows <= 0 || !input)
+    return apt_spmm_sum_known(kCopyU, dtype, coo_row, coo_col, num_edges, input, nullptr, feat_dim, feat_dim, coo_offset, input_offset,
+                              output_offset, num_segments, num_out_rows, mode, fixed, out, workspace, workspace_bytes, stream);
+  int64_t edata_dim = 0;
+  int rc = spmm_check("apt_spmm_copy_u_widened", kCopyU, dtype, num_edges, &edata_dim, feat_dim, num_segments, num_out_rows);
+  if (rc != APT_OK) return rc;
+  APT_CHECK_ARG(mode != kFixed || (fixed >= 0 && (int64_t)fixed * num_out_rows == num_edges),
+                "apt_spmm_copy_u_widened: %lld rows of %d edges are not %lld edges", (long long)num_out_rows, fixed, (long long)num_edges);
+  APT_CHECK_ARG(coo_row && coo_col && coo_offset && input_offset && output_offset && out && widened, "apt_spmm_copy_u_widened: null pointer");
+  APT_CHECK_ARG(((uintptr_t)widened & 15) == 0, "apt_spmm_copy_u_widened: the buffer of widened rows must be 16-byte aligned");
+  if (widened_bytes < need) {
+    set_error("apt_spmm_copy_u_widened: %zu < %zu bytes for widened rows", widened_bytes, need);
+    return APT_ERR_CAPACITY;
+  }
+  const size_t esz = elem_size(dtype);
+  cudaStream_t s = (cudaStream_t)stream;
+  rc = widen_rows(input, num_input_rows, feat_dim * (int64_t)esz, widened, s);
+  if (rc != APT_OK) return rc;
+  const SegTable st{coo_offset, input_offset, output_offset, num_segments};
+  const int64_t dim = widened_dim(feat_dim, esz);
+  return spmm_run(kCopyU, dtype, coo_row, coo_col, num_edges, widened, nullptr, dim, dim, st, num_out_rows, out, workspace, workspace_bytes,
+                  mode, fixed, feat_dim, s);
 }
 
 extern "C" int apt_spmm_sum(int op, int dtype, const int64_t* coo_row, const int64_t* coo_col,

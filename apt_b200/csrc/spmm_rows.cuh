@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "rows.cuh"
+#include "widen.cuh"
 
 namespace apt {
 
@@ -173,6 +174,7 @@ struct RowArgs {
   const T* own;            // the output rows' own
   float* dots;             // [E][heads]
   uint32_t num_in;         // input rows; ws.cnt and ws.rank count their edges on the way
+  int64_t width;           // columns of an output row where input rows were widened to feat_dim; 0: feat_dim
 };
 
 // ---- which rows k_spmm_stream takes --------------------------------------------------------------
@@ -204,11 +206,12 @@ inline int stream_lph(int64_t feat_dim, size_t esz, int heads) { return pow2_ge(
 inline bool stream_one_slice(int op, int64_t feat_dim, size_t esz, int heads) {
   return op == kDots ? heads * stream_lph(feat_dim, esz, heads) <= 32 : feat_dim * (int64_t)esz <= 512;
 }
-inline StreamPlan stream_plan(int op, int64_t feat_dim, size_t esz, int heads) {
+inline StreamPlan stream_plan(int op, int64_t feat_dim, size_t esz, int heads, bool widened = false) {
   StreamPlan p{};
   p.row_bytes = (int)(feat_dim * esz);
   p.lph = op == kDots ? stream_lph(feat_dim, esz, heads) : 32;
   p.warp_bytes = 2 * 8 * 512 + (op == kUMulW ? 64 * heads * 4 : 0);      // rows (two groups of eight of a slice a lane, four of two), weights
+  if (widened) p.warp_bytes += stream_one_slice(op, feat_dim, esz, heads) ? 512 : 1024;      // the row that is written
   p.warps = std::min(stream_warps(stream_one_slice(op, feat_dim, esz, heads)), kStreamShared / p.warp_bytes);
   p.shared = p.warps * p.warp_bytes;
   return p;
@@ -306,7 +309,7 @@ __device__ __forceinline__ void slice_add(Acc<VE>& acc, const EdgeSlice<T, VE, O
 }
 
 // The sums of the edges read side by side meet, and the lanes of the first of them write the row's column block.
-template <typename T, int VE, int VPL>
+template <typename T, int VE, int VPL, bool WIDENED>
 __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], const int (&col)[VPL], int d, int c0, int nvec, int lpe, int lpr, int vl,
                                            int epi, unsigned gmask) {
 #pragma unroll 1
@@ -317,7 +320,8 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[V
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     if (c0 + vl + i * lpe >= nvec) continue;
-    store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
+    if constexpr (WIDENED) store_some<T, VE>(a.out + (int64_t)d * a.width + col[i], acc[i].template rounded<T>(), (int)a.width - col[i]);
+    else store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
   }
 }
 
@@ -331,7 +335,8 @@ constexpr int rows_min_blocks(int op, int elems) {
 }
 
 // WIDE: a warp to an edge (lpe 32, ep 1), which leaves the geometry to the compiler and its registers to more warps.
-template <typename T, int VE, int VPL, int OP, bool WIDE>
+// WIDENED: the input's rows are (widen.cuh), the result's are not.
+template <typename T, int VE, int VPL, int OP, bool WIDE, bool WIDENED>
 __global__ void __launch_bounds__(256, rows_min_blocks(OP, VE * VPL))
 k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
   wait_for_previous();
@@ -540,11 +545,11 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
           }
           c0 = cc;
           if (cc + lpe * VPL < nvec) {
-            rows_write<T, VE, VPL>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
+            rows_write<T, VE, VPL, WIDENED>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
           }
         }
       }
-      rows_write<T, VE, VPL>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
+      rows_write<T, VE, VPL, WIDENED>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
     }
     if (items) {
       it += warps;
@@ -563,26 +568,26 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
 }
 
 // ---- launch -----------------------------------------------------------------------
-template <typename T, int VE, int VPL, int OP, bool WIDE>
+template <typename T, int VE, int VPL, int OP, bool WIDE, bool WIDENED>
 static int launch_rows_kernel(const RowArgs<T>& a, cudaStream_t s) {
   static int occupancy[64] = {};
   int per_sm = 0;
-  const int rc = blocks_per_sm(k_spmm_rows<T, VE, VPL, OP, WIDE>, 256, occupancy, &per_sm);
+  const int rc = blocks_per_sm(k_spmm_rows<T, VE, VPL, OP, WIDE, WIDENED>, 256, occupancy, &per_sm);
   if (rc != APT_OK) return rc;
   const int64_t want = ceil_div(a.num_rows, 256 / (a.split.lpe * a.split.ep));
   const int64_t wave = (int64_t)kNumSMs * per_sm;
-  APT_FOLLOW((k_spmm_rows<T, VE, VPL, OP, WIDE>), (int)(want < wave ? want : wave), 256, 0, s, a);
+  APT_FOLLOW((k_spmm_rows<T, VE, VPL, OP, WIDE, WIDENED>), (int)(want < wave ? want : wave), 256, 0, s, a);
   return APT_OK;
 }
 
-template <typename T, int VE, int OP>
+template <typename T, int VE, int OP, bool WIDENED = false>
 static int launch_rows_vpl(const RowArgs<T>& a, cudaStream_t s) {
   // rows of two and four slices a lane are wide ones
   switch (a.split.vpl) {
     case 1:
-      return a.split.lpe == 32 ? launch_rows_kernel<T, VE, 1, OP, true>(a, s) : launch_rows_kernel<T, VE, 1, OP, false>(a, s);
-    case 2: return launch_rows_kernel<T, VE, 2, OP, true>(a, s);
-    default: return launch_rows_kernel<T, VE, 4, OP, true>(a, s);
+      return a.split.lpe == 32 ? launch_rows_kernel<T, VE, 1, OP, true, WIDENED>(a, s) : launch_rows_kernel<T, VE, 1, OP, false, WIDENED>(a, s);
+    case 2: return launch_rows_kernel<T, VE, 2, OP, true, WIDENED>(a, s);
+    default: return launch_rows_kernel<T, VE, 4, OP, true, WIDENED>(a, s);
   }
 }
 
@@ -594,6 +599,8 @@ static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
   if constexpr (OP == kCopyU || OP == kUMulW) {
     if (stream_fits(OP, a.split.ve * (int)sizeof(T), a.feat_dim, sizeof(T), OP == kCopyU ? 1 : (int)a.edata_dim, a.num_edges, a.mode == kFixed || a.mode == kRanges)) return launch_stream<T, OP>(a, s);
   }
+  if constexpr (OP == kCopyU)
+    if (a.width) return launch_rows_vpl<T, 16 / sizeof(T), OP, true>(a, s);
   switch (a.split.ve * (int)sizeof(T)) {
     case 16: return launch_rows_vpl<T, 16 / sizeof(T), OP>(a, s);
     case 8: return launch_rows_vpl<T, 8 / sizeof(T), OP>(a, s);

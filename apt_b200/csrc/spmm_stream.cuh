@@ -79,7 +79,7 @@ struct SlotBatch {
   uint32_t e;          // edge; kDots: its place among those of its input row
 };
 
-template <typename T, int OP, int VPL>
+template <typename T, int OP, int VPL, bool WIDENED>
 __global__ void __launch_bounds__(stream_warps(VPL == 1) * 32, kStreamBlocks)
 k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ StreamPlan plan, int polls, volatile int32_t* pending) {
   wait_for_previous();
@@ -111,7 +111,7 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   const int warps = gridDim.x * plan.warps, warp = blockIdx.x * plan.warps + w;
   const uint32_t row_bytes = plan.row_bytes;
   unsigned char* const ring = shared + w * plan.warp_bytes;
-  float* const weights = (float*)(ring + 2 * GE * kSlot);      // [2][32][heads]
+  float* const weights = (float*)(ring + 2 * GE * kSlot);      // [2][32][heads]; WIDENED: the row that is written
 
   // the lane's slices of 16 bytes, 32 apart; in kDots a head's slices have a power of two of lanes (plan.lph)
   int col[VPL], head[VPL];
@@ -192,6 +192,16 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   };
   clear();
   auto write = [&](uint32_t d) {
+    if constexpr (WIDENED) {
+      T* const row = (T*)weights;
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < VPL; ++i)
+        if (valid[i]) store_pack<T, VE>(row + col[i], acc[i].template rounded<T>());
+      __syncwarp();
+      store_row(a.out + (uint64_t)d * a.width, row, (int)a.width, lane);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
       if (valid[i]) store_pack<T, VE>(a.out + (uint64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
@@ -474,14 +484,14 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
 }
 
 // Wide rows of many edges: see the top of the file.
-template <typename T, int OP, int VPL>
+template <typename T, int OP, int VPL, bool WIDENED>
 static int launch_stream(const RowArgs<T>& a, cudaStream_t s) {
-  const StreamPlan plan = stream_plan(OP, a.feat_dim, sizeof(T), (int)a.edata_dim);
+  const StreamPlan plan = stream_plan(OP, a.feat_dim, sizeof(T), (int)a.edata_dim, WIDENED);
   static bool sized[64] = {};
   int dev = 0;
   APT_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !sized[dev]) {
-    APT_CUDA(cudaFuncSetAttribute(k_spmm_stream<T, OP, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared));
+    APT_CUDA(cudaFuncSetAttribute(k_spmm_stream<T, OP, VPL, WIDENED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared));
     if (dev < 64) sized[dev] = true;
   }
   int32_t* pending = nullptr;
@@ -490,14 +500,17 @@ static int launch_stream(const RowArgs<T>& a, cudaStream_t s) {
     if (rc != APT_OK) return rc;
   }
   const int blocks = stream_blocks(a.feat_dim, a.num_edges, a.ws.part_floats, plan.warps, a.mode == kFixed || a.mode == kRanges);
-  APT_FOLLOW((k_spmm_stream<T, OP, VPL>), blocks, plan.warps * 32, plan.shared, s, a, plan,
+  APT_FOLLOW((k_spmm_stream<T, OP, VPL, WIDENED>), blocks, plan.warps * 32, plan.shared, s, a, plan,
              bulk_wait_polls(), (volatile int32_t*)pending);
   return APT_OK;
 }
 
 template <typename T, int OP>
 static int launch_stream(const RowArgs<T>& a, cudaStream_t s) {
-  return stream_one_slice(OP, a.feat_dim, sizeof(T), (int)a.edata_dim) ? launch_stream<T, OP, 1>(a, s) : launch_stream<T, OP, 2>(a, s);
+  const bool one_slice = stream_one_slice(OP, a.feat_dim, sizeof(T), (int)a.edata_dim);
+  if constexpr (OP == kCopyU)
+    if (a.width) return one_slice ? launch_stream<T, OP, 1, true>(a, s) : launch_stream<T, OP, 2, true>(a, s);
+  return one_slice ? launch_stream<T, OP, 1, false>(a, s) : launch_stream<T, OP, 2, false>(a, s);
 }
 
 }  // namespace apt

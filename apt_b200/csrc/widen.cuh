@@ -1,0 +1,84 @@
+// Input rows of any width laid out in whole 16-byte slices (widen.cu), and when a sum has that done.
+#pragma once
+
+#include <algorithm>
+
+#include "rows.cuh"
+
+namespace apt {
+
+// When a sum has its input widened. The copy reads and writes every input row once (5.6 TB/s: 67 000 x 404 B 11 us, 469 000 x 404 B 69) and a call with
+// one more buffer and launch takes the host 3 us longer; the gain is per edge, the larger the narrower the accesses are otherwise, and larger
+// behind the sort, where a row's edges are walked from a list. us of a call, rows as they are -> widened:
+//   in no order, 1 005 000 edges from 67 000 rows into 168 000   bf16 x 17 103 -> 86, x 61 122 -> 99, x 101 154 -> 119, x 251 292 -> 170; x 34 107 -> 95, x 198
+//     179 -> 169; fp32 x 31 108 -> 95, x 101 161 -> 133, x 251 368 -> 183, x 198 245 -> 170
+//   240 000 edges from 20 000 into 44 000   bf16 x 31 55 -> 51, x 101 78 -> 61, x 251 121 -> 70, x 198 78 -> 71; fp32 x 31 55 -> 53, x 101 78 -> 59, x 198 82 -> 70
+//   where it does not pay: bf16 x 9 87 -> 85 and 47 -> 48; accesses of 8 bytes, bf16 x 140 138 -> 155, x 36 91 -> 94; of 4, fp32 x 34 106 -> 112, bf16 x 102
+//     67 -> 68; 96 000 edges, fp32 x 101 into 94 000 rows 61 -> 68 (k_spmm_stream takes no less than 98 304)
+//   grouped, 1 005 000 edges from 168 000 rows   bf16 x 17 40 -> 32, x 61 51 -> 41, x 251 139 -> 97; x 140 69 -> 83, fp32 x 101 76 -> 83; from 368 000
+//     bf16 x 61 51 -> 54, x 101 79 -> 86; 240 000 edges from 44 000 bf16 x 61 22 -> 23, x 251 37 -> 35
+constexpr int kWidenLeast = 34, kWidenMost = 4096;      // bytes of a row
+constexpr int64_t kWidenEdges = 3 << 15, kWidenGrouped = 3 << 17;
+
+// Elements of a row of `dim` in whole slices.
+inline int64_t widened_dim(int64_t dim, size_t esz) { return (dim * (int64_t)esz + 15) / 16 * (16 / (int64_t)esz); }
+
+inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num_edges, bool grouped) {
+  const int64_t row = dim * (int64_t)esz;
+  const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
+  if (slice == 16 || row < kWidenLeast || row > kWidenMost || num_in_rows <= 0) return false;
+  if (grouped) return slice == 2 && num_edges >= kWidenGrouped && num_edges / 4 >= num_in_rows;
+  if (num_edges < kWidenEdges || num_edges / 3 < num_in_rows) return false;
+  return slice == 2 || row >= (slice == 4 ? 384 : 768) || (slice == 4 && row >= 64 && row <= 128 && num_edges >= 2 * kWidenEdges);
+}
+
+// `out`: num_rows * ceil(row_bytes / 16) slices, 16-byte aligned. `in` is aligned to its elements of 2 or 4 bytes.
+int widen_rows(const void* in, int64_t num_rows, int64_t row_bytes, void* out, cudaStream_t s);
+
+// The first n elements of a slice, at any element's address: pairs of 16-bit ones where they are aligned. (k_spmm_rows, whose rows are several
+// to a warp; bf16 x 101 114 us against 94 for 104 columns.)
+template <typename T, int VE>
+__device__ __forceinline__ void store_some(T* p, const Pack<T, VE>& r, int n) {
+  if constexpr (sizeof(T) == 2) {
+    const unsigned int* const w = (const unsigned int*)&r;
+    if (((uintptr_t)p & 2) == 0) {
+#pragma unroll
+      for (int t = 0; t < VE; t += 2) {
+        if (t + 1 < n) *(unsigned int*)(p + t) = w[t / 2];
+        else if (t < n) p[t] = r.v[t];
+      }
+    } else {
+      if (n > 0) p[0] = r.v[0];
+#pragma unroll
+      for (int t = 1; t < VE; t += 2) {
+        if (t + 1 < VE && t + 1 < n) *(unsigned int*)(p + t) = __funnelshift_r(w[t / 2], w[(t + 1) / 2 < VE / 2 ? (t + 1) / 2 : 0], 16);
+        else if (t < n) p[t] = r.v[t];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < VE; ++t)
+      if (t < n) p[t] = r.v[t];
+  }
+}
+
+// A row of n elements that a warp has in shared memory, to any element's address: side by side lanes write side by side words. (k_spmm_stream, whose
+// stores are in its loop many times over: lanes that write their slices themselves 244 us instead of 161 for bf16 x 251, four words a lane at a
+// time 235. As a run time branch beside aligned stores they had cost rows of 256 bf16 81 -> 110.)
+template <typename T>
+__device__ __forceinline__ void store_row(T* out, const T* row, int n, int lane) {
+  if constexpr (sizeof(T) == 2) {
+    const unsigned short* const h = (const unsigned short*)row;
+    const int odd = (int)((uintptr_t)out >> 1 & 1), words = (n - odd) >> 1;
+    unsigned int* const w = (unsigned int*)(out + odd);
+#pragma unroll 1
+    for (int t = lane; t < words; t += 32) w[t] = (unsigned int)h[odd + 2 * t] | (unsigned int)h[odd + 2 * t + 1] << 16;
+    if (odd && lane == 0) out[0] = row[0];
+    if ((n - odd & 1) && lane == 31) out[n - 1] = row[n - 1];
+  } else {
+#pragma unroll 2
+    for (int t = lane; t < n; t += 32) out[t] = row[t];
+  }
+}
+
+}  // namespace apt

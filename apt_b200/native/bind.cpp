@@ -97,6 +97,22 @@ Tensor spmm(int op, const Tensor& coo_row, const Tensor& coo_col, const OptTenso
     bytes = apt_spmm_workspace_bytes(shape[0], edges);
     ws = scratch(out, bytes);
   }
+  // room for widened input rows; without it the sum does without
+  size_t wide_bytes = op == 0 && input && shape[0] > 0 ? apt_spmm_widened_bytes(code, edges, in.size(0), dim, (int)shape[1]) : 0;
+  Tensor wide;
+  if (wide_bytes) {
+    try {
+      wide = scratch(out, wide_bytes);
+    } catch (const c10::OutOfMemoryError&) {
+      wide_bytes = 0;
+    }
+  }
+  if (wide_bytes) {
+    check(apt_spmm_copy_u_widened(code, ptr(row), ptr(col), edges, data(in), in.size(0), dim, ptr(eoff), ptr(ioff), ptr(ooff),
+                                  (int)eoff.numel() - 1, shape[0], (int)shape[1], (int)shape[2], mut(out), wide.mutable_data_ptr(),
+                                  wide_bytes, bytes ? ws.mutable_data_ptr() : nullptr, bytes, stream()));
+    return out;
+  }
   check(apt_spmm_sum_known(op, code, ptr(row), ptr(col), edges, input ? data(in) : nullptr, edata ? data(ed) : nullptr, edim,
                            dim, ptr(eoff), input_offset ? ptr(ioff) : nullptr, ptr(ooff), (int)eoff.numel() - 1, shape[0],
                            (int)shape[1], (int)shape[2], mut(out), bytes ? ws.mutable_data_ptr() : nullptr, bytes, stream()));

@@ -417,6 +417,25 @@ int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row,
                        int fixed, void* out, void* workspace,
                        size_t workspace_bytes, void* stream);
 
+/* apt_spmm_sum_known of op 0 for rows that are no whole number of 16-byte slices,
+ * whose input is copied to such a pitch first and then read a slice at a time:
+ * results are the same. apt_spmm_widened_bytes is what the copy takes, or 0
+ * where the sum does better without (no buffer is used then). num_input_rows:
+ * rows of `input`, all segments together. */
+size_t apt_spmm_widened_bytes(int dtype, int64_t num_edges,
+                              int64_t num_input_rows, int64_t feat_dim,
+                              int mode);
+int apt_spmm_copy_u_widened(int dtype, const int64_t* coo_row,
+                            const int64_t* coo_col, int64_t num_edges,
+                            const void* input, int64_t num_input_rows,
+                            int64_t feat_dim, const int64_t* coo_offset,
+                            const int64_t* input_offset,
+                            const int64_t* output_offset, int num_segments,
+                            int64_t num_out_rows, int mode, int fixed, void* out,
+                            void* widened, size_t widened_bytes,
+                            void* workspace, size_t workspace_bytes,
+                            void* stream);
+
 /* op: 0 u_add_v, 1 u_mul_v; out has num_edges rows of feat_dim columns. */
 int apt_sddmm(int op, int dtype, const int64_t* coo_row,
               const int64_t* coo_col, int64_t num_edges, const void* lhs,

@@ -1,0 +1,97 @@
+"""Sums over rows that are no whole number of 16-byte slices, whose input is laid out anew first (csrc/widen.cuh): the lines of
+the rule, the ends of rows and of tiles, and an input that starts and ends anywhere."""
+import pytest
+import torch
+
+from apt_b200 import ops
+from apt_b200._lib import check, lib
+
+pytestmark = pytest.mark.gpu
+_EPS = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+def _block(dst, src, per, ordered, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    row = torch.randint(0, src, (dst * per,), generator=g, device="cuda")
+    col = torch.arange(dst, device="cuda").repeat_interleave(per)
+    if not ordered:
+        p = torch.randperm(dst * per, generator=g, device="cuda")
+        row, col = row[p], col[p]
+        col[0], col[-1] = dst - 1, 0      # (in no order, whatever the permutation)
+    return row, col, g
+
+
+def _expect(got, row, col, x, dst, most):
+    want = torch.zeros(dst, x.shape[1], dtype=torch.float64, device="cuda").index_add_(0, col, x[row].double())
+    size = torch.zeros(dst, x.shape[1], dtype=torch.float64, device="cuda").index_add_(0, col, x[row].double().abs())
+    # fp32 sums of up to `most` terms in some order, and one rounding to the result's type
+    bound = size * most * 2.0 ** -24 + want.abs() * _EPS[x.dtype] * 1.01 + 1e-7
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dim", [9, 17, 18, 31, 61, 101, 119, 137, 197, 198, 251, 255, 301, 511])
+@pytest.mark.parametrize("segments", [1, 3])
+def test_sums_in_no_order(dtype, dim, segments):
+    # 100 000 edges and more go the widened way where the width does (kWidenEdges, twice that)
+    dst, src, per = 19_997, 9_001, 11
+    parts = [_block(dst, src, per, False, 7 * dim + k) for k in range(segments)]
+    x = torch.randn(segments * src, dim, generator=parts[0][2], device="cuda").to(dtype)
+    off = lambda n: torch.arange(segments + 1, device="cuda") * n
+    row, col = torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts])
+    got = ops.spmm_copy_u_sum(row, col, x, off(dst * per), off(src), off(dst))
+    for k, (r, c, _) in enumerate(parts):
+        most = int(torch.bincount(c).max()) + 40
+        _expect(got[k * dst:(k + 1) * dst], r, c, x[k * src:(k + 1) * src], dst, most)
+
+
+@pytest.mark.parametrize("dim", [17, 31, 61, 119, 251, 257])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_sums_of_grouped_edges(dim, ragged):
+    dst, src, per = 40_001, 90_000, 10
+    row, col, g = _block(dst, src, per, True, dim)
+    if ragged:
+        keep = torch.rand(dst * per, generator=g, device="cuda") < 0.99
+        row, col = row[keep], col[keep]
+    x = torch.randn(src, dim, generator=g, device="cuda").to(torch.bfloat16)
+    off = lambda n: torch.tensor([0, n], device="cuda")
+    got = ops.spmm_copy_u_sum(row, col, x, off(row.numel()), off(src), off(dst))
+    _expect(got, row, col, x, dst, 2 * per)
+
+
+@pytest.mark.parametrize("dtype,dim", [(torch.float32, 101), (torch.bfloat16, 61), (torch.float16, 251), (torch.bfloat16, 255)])
+@pytest.mark.parametrize("first", [0, 1, 2, 3, 5, 7])
+def test_input_anywhere_is_read_within_its_ends(dtype, dim, first):
+    """What lies around the input (NaN) is not part of any sum, and the result ends where it ends."""
+    dst, src, per = 10_007, 1_003, 10
+    row, col, g = _block(dst, src, per, False, first)
+    room = torch.full((first + src * dim + 64,), float("nan"), dtype=dtype, device="cuda")
+    x = room[first:first + src * dim].view(src, dim)
+    x.copy_(torch.randn(src, dim, generator=g, device="cuda"))
+    off = lambda n: torch.tensor([0, n], device="cuda")
+    e, d, s = off(dst * per), off(dst), off(src)
+    code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
+    wide = lib.apt_spmm_widened_bytes(code, dst * per, src, dim, 2)
+    assert wide >= src * dim * x.element_size()
+    ws_bytes = lib.apt_spmm_workspace_bytes(dst, dst * per)
+    buf, ws = torch.empty(wide, dtype=torch.uint8, device="cuda"), torch.empty(ws_bytes, dtype=torch.uint8, device="cuda")
+    out = torch.full((first + dst * dim + 64,), 7.0, dtype=dtype, device="cuda")
+    at = out.data_ptr() + first * x.element_size()
+    run = lambda size: lib.apt_spmm_copy_u_widened(code, row.data_ptr(), col.data_ptr(), dst * per, x.data_ptr(), src, dim, e.data_ptr(), s.data_ptr(),
+                                                   d.data_ptr(), 1, dst, 2, 0, at, buf.data_ptr(), size, ws.data_ptr(), ws_bytes,
+                                                   torch.cuda.current_stream().cuda_stream)
+    check(run(wide))
+    got = out[first:first + dst * dim].view(dst, dim)
+    _expect(got, row, col, x, dst, int(torch.bincount(col).max()) + 40)
+    assert (out[:first] == 7.0).all() and (out[first + dst * dim:] == 7.0).all()
+    assert run(wide - 1) != 0      # a buffer that is too small is refused
+
+
+def test_rows_that_stay_as_they_are():
+    bytes_of = lib.apt_spmm_widened_bytes
+    assert bytes_of(1, 1_000_000, 67_000, 256, 2) == 0          # whole slices
+    assert bytes_of(1, 90_000, 8_000, 101, 2) == 0              # few edges
+    assert bytes_of(1, 1_000_000, 400_000, 101, 2) == 0         # input rows that few edges read
+    assert bytes_of(1, 1_000_000, 150_000, 102, 1) == 0         # grouped, read four bytes a lane
+    assert bytes_of(1, 1_000_000, 67_000, 101, -1) == 0         # unknown block
+    assert bytes_of(1, 1_000_000, 67_000, 101, 2) == 67_000 * 208
