@@ -88,6 +88,11 @@ PROTOTYPES = {
     "apt_gat_backward_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int]),
     "apt_gat_backward": (c_int, [c_int, P, P, c_int64, P, P, P, P, c_int, c_int64, c_float, c_int64, c_int64, P, P, P, P,
                                  c_size_t, c_int, P, c_size_t, P, P]),
+    "apt_gat_widened_bytes": (c_size_t, [c_int, c_int64, c_int64, c_int64, c_int, c_int64]),
+    "apt_gat_forward_widened": (c_int, [c_int, P, P, c_int64, P, P, P, c_int, c_int64, c_float, c_int64, c_int64, P, P, P, c_size_t, P, c_size_t,
+                                        P, P]),
+    "apt_gat_backward_widened": (c_int, [c_int, P, P, c_int64, P, P, P, P, c_int, c_int64, c_float, c_int64, c_int64, P, P, P, P, c_size_t,
+                                         c_int, P, c_size_t, P, c_size_t, P, P]),
     "apt_src_to_vir": (c_int, [P, c_int64, c_int64, c_int64, P, c_int, c_int, c_int, c_int, c_int, P, P]),
     "apt_srcdst_to_vir": (c_int, [P, c_int64, P, c_int64, c_int64, P, c_int, c_int, c_int, c_int, c_int, P, P]),
     "apt_vir_send_sizes": (c_int, [P, c_int64, P, P, c_int64, P, c_int, c_int64, P, c_int, P, P, P]),

@@ -632,17 +632,34 @@ static int gat_weights(const GatProblem& q, const GatEdges& g, void* attn, cudaS
   return APT_OK;
 }
 
+// Rows of heads that are no whole slices, widened head by head (widen.cuh); without a buffer, or where that does not pay, `dim` is 0.
+struct GatWide {
+  void *ft, *grad;
+  int64_t dim;      // of a head
+};
+// num_dst 0: the sources only.
+static size_t gat_wide_layout(int dtype, int64_t E, int64_t num_src, int64_t num_dst, int H, int64_t Dh, char* base, GatWide* w) {
+  const size_t esz = elem_size(dtype);
+  if (!widen_gat_pays(Dh, H, esz, num_src, E, num_dst > 0)) return 0;
+  const int64_t dim = widened_dim(Dh, esz);
+  const size_t o_grad = align_up((size_t)num_src * H * dim * esz, 256);
+  if (w) *w = GatWide{base, base + o_grad, dim};
+  return o_grad + (size_t)num_dst * H * dim * esz;
+}
+
 template <typename T>
-static int gat_forward(const GatProblem& q, const GatEdges& g, void* out, void* attn, cudaStream_t s) {
-  const int rc = gat_weights<T>(q, g, attn, s);
+static int gat_forward(const GatProblem& q, const GatEdges& g, const GatWide& wide, int64_t num_src, void* out, void* attn, cudaStream_t s) {
+  int rc = gat_weights<T>(q, g, attn, s);
+  if (rc == APT_OK && wide.dim) rc = widen_rows(q.ft, num_src * q.H, q.Dh * sizeof(T), wide.ft, s);
   if (rc != APT_OK) return rc;
-  const int64_t dim = q.H * q.Dh;
+  const int64_t dim = q.H * (wide.dim ? wide.dim : q.Dh);
   // a slice stays inside a head, so that one weight serves it
-  const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)out, sizeof(T));
+  const int ve = wide.dim ? 16 / sizeof(T) : slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)out, sizeof(T));
   SpmmWs ws{};
   ws.range = g.range;
-  const RowArgs<T> a{q.row, (const T*)q.ft, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst, q.E, ws,
-                     (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u};
+  const RowArgs<T> a{q.row, (const T*)(wide.dim ? wide.ft : q.ft), (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst,
+                     q.E, ws, (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u,
+                     wide.dim ? q.H * q.Dh : 0};
   ProfScope prof("gat_rows", s);
   return launch_spmm_rows<T>(kUMulW, a, s);
 }
@@ -685,14 +702,22 @@ static int gat_dots(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, 
 
 // The weights are there already.
 template <typename T>
-static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, char* workspace, int64_t num_src, void* grad_ft,
-                        void* grad_el, void* grad_er, cudaStream_t s) {
+static int gat_backward(const GatProblem& as_given, const GatEdges& g, const GatWide& wide, const GatBwdWs& ws, char* workspace, int64_t num_src,
+                        void* grad_ft, void* grad_el, void* grad_er, cudaStream_t s) {
+  GatProblem q = as_given;
+  if (wide.dim) q.ft = wide.ft, q.grad_out = wide.grad, q.Dh = wide.dim;
   const int64_t dim = q.H * q.Dh;
-  const int ve = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
+  const int ve = wide.dim ? 16 / sizeof(T) : slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
   const RowSplit split = row_split(dim, ve, q.E, num_src);
   const OrderKind kind = order_kind(kUMulW, ve * (int)sizeof(T), dim, sizeof(T), q.H, q.E);
   APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
   int rc;
+  if (wide.dim) {
+    ProfScope prof("gat_widen", s);
+    rc = widen_rows(as_given.ft, num_src * q.H, as_given.Dh * sizeof(T), wide.ft, s);
+    if (rc == APT_OK) rc = widen_rows(as_given.grad_out, q.num_dst * q.H, as_given.Dh * sizeof(T), wide.grad, s);
+    if (rc != APT_OK) return rc;
+  }
   {
     ProfScope prof("gat_bwd_rows", s);
     rc = gat_dots<T>(q, g, ws, num_src, s);
@@ -705,7 +730,7 @@ static int gat_backward(const GatProblem& q, const GatEdges& g, const GatBwdWs& 
 #undef APT_SCORES
   }
   const RowArgs<T> a{nullptr, (const T*)q.grad_out, (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, num_src, q.E, ws.sort,
-                     (T*)grad_ft, kOrder, 0, split, (int)dim, Verdict{}, q.status, nullptr, nullptr, nullptr, 0u};
+                     (T*)grad_ft, kOrder, 0, split, (int)dim, Verdict{}, q.status, nullptr, nullptr, nullptr, 0u, wide.dim ? q.H * as_given.Dh : 0};
   {
     ProfScope prof("spmm_rows", s);
     rc = launch_spmm_rows<T>(kUMulW, a, s);
@@ -1051,12 +1076,41 @@ extern "C" size_t apt_gat_edges_bytes(int64_t num_dst, int64_t num_edges, int nu
   return apt::gat_edges_layout(num_dst, num_edges, num_heads, nullptr, nullptr);
 }
 
+extern "C" size_t apt_gat_widened_bytes(int dtype, int64_t num_edges, int64_t num_src, int64_t num_dst, int num_heads, int64_t head_dim) {
+  using namespace apt;
+  if (dtype < APT_F32 || dtype > APT_F16 || num_edges < 0 || num_src < 0 || num_dst < 0 || num_heads < 1 || head_dim < 1) return 0;
+  return gat_wide_layout(dtype, num_edges, num_src, num_dst, num_heads, head_dim, nullptr, nullptr);
+}
+
+// The buffer of widened rows as the caller gives it, or none.
+static int gat_wide(const char* who, int dtype, int64_t E, int64_t num_src, int64_t num_dst, int H, int64_t Dh, void* widened, size_t bytes,
+                    apt::GatWide* w) {
+  using namespace apt;
+  *w = GatWide{};
+  if (!widened) return APT_OK;
+  APT_CHECK_ARG(((uintptr_t)widened & 255) == 0, "%s: the buffer of widened rows must be 256-byte aligned", who);
+  const size_t need = gat_wide_layout(dtype, E, num_src, num_dst, H, Dh, (char*)widened, w);
+  if (bytes < need) {
+    set_error("%s: %zu < %zu bytes for widened rows", who, bytes, need);
+    return APT_ERR_CAPACITY;
+  }
+  return APT_OK;
+}
+
 extern "C" int apt_gat_forward(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges, const void* ft,
                                const void* el, const void* er, int num_heads, int64_t head_dim, float negative_slope,
                                int64_t num_dst, void* out, void* out_attn, void* edges, size_t edges_bytes,
                                int32_t* status_word, void* stream) {
+  return apt_gat_forward_widened(dtype, coo_row, coo_col, num_edges, ft, el, er, num_heads, head_dim, negative_slope, 0, num_dst, out, out_attn,
+                                 edges, edges_bytes, nullptr, 0, status_word, stream);
+}
+
+extern "C" int apt_gat_forward_widened(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges, const void* ft,
+                                       const void* el, const void* er, int num_heads, int64_t head_dim, float negative_slope,
+                                       int64_t num_src, int64_t num_dst, void* out, void* out_attn, void* edges, size_t edges_bytes,
+                                       void* widened, size_t widened_bytes, int32_t* status_word, void* stream) {
   using namespace apt;
-  const int rc = gat_check("apt_gat_forward", dtype, num_edges, num_heads, head_dim, num_dst);
+  int rc = gat_check("apt_gat_forward", dtype, num_edges, num_heads, head_dim, num_dst);
   if (rc != APT_OK || num_dst == 0) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   APT_CHECK_ARG(out && status_word, "apt_gat_forward: null output");
@@ -1072,11 +1126,14 @@ extern "C" int apt_gat_forward(int dtype, const int64_t* coo_row, const int64_t*
     set_error("apt_gat_forward: edge buffer %zu < %zu bytes", edges_bytes, need);
     return APT_ERR_CAPACITY;
   }
+  GatWide wide;
+  rc = gat_wide("apt_gat_forward", dtype, num_edges, num_src, 0, num_heads, head_dim, widened, widened_bytes, &wide);
+  if (rc != APT_OK) return rc;
   const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, nullptr, num_heads, head_dim, negative_slope, num_dst, status_word};
   switch (dtype) {
-    case APT_F32: return gat_forward<float>(q, g, out, out_attn, s);
-    case APT_BF16: return gat_forward<__nv_bfloat16>(q, g, out, out_attn, s);
-    default: return gat_forward<__half>(q, g, out, out_attn, s);
+    case APT_F32: return gat_forward<float>(q, g, wide, num_src, out, out_attn, s);
+    case APT_BF16: return gat_forward<__nv_bfloat16>(q, g, wide, num_src, out, out_attn, s);
+    default: return gat_forward<__half>(q, g, wide, num_src, out, out_attn, s);
   }
 }
 
@@ -1090,6 +1147,17 @@ extern "C" int apt_gat_backward(int dtype, const int64_t* coo_row, const int64_t
                                 int64_t head_dim, float negative_slope, int64_t num_src, int64_t num_dst, void* grad_ft,
                                 void* grad_el, void* grad_er, void* edges, size_t edges_bytes, int edges_valid,
                                 void* workspace, size_t workspace_bytes, int32_t* status_word, void* stream) {
+  return apt_gat_backward_widened(dtype, coo_row, coo_col, num_edges, ft, el, er, grad_out, num_heads, head_dim, negative_slope, num_src,
+                                  num_dst, grad_ft, grad_el, grad_er, edges, edges_bytes, edges_valid, workspace, workspace_bytes, nullptr, 0,
+                                  status_word, stream);
+}
+
+extern "C" int apt_gat_backward_widened(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges,
+                                        const void* ft, const void* el, const void* er, const void* grad_out, int num_heads,
+                                        int64_t head_dim, float negative_slope, int64_t num_src, int64_t num_dst, void* grad_ft,
+                                        void* grad_el, void* grad_er, void* edges, size_t edges_bytes, int edges_valid,
+                                        void* workspace, size_t workspace_bytes, void* widened, size_t widened_bytes,
+                                        int32_t* status_word, void* stream) {
   using namespace apt;
   int rc = gat_check("apt_gat_backward", dtype, num_edges, num_heads, head_dim, num_dst);
   if (rc != APT_OK) return rc;
@@ -1116,11 +1184,14 @@ extern "C" int apt_gat_backward(int dtype, const int64_t* coo_row, const int64_t
     set_error("apt_gat_backward: buffers of %zu and %zu bytes, %zu and %zu needed", edges_bytes, workspace_bytes, need_e, need_w);
     return APT_ERR_CAPACITY;
   }
+  GatWide wide;
+  rc = gat_wide("apt_gat_backward", dtype, num_edges, num_src, num_dst, num_heads, head_dim, widened, widened_bytes, &wide);
+  if (rc != APT_OK) return rc;
   const GatProblem q{coo_row, coo_col, num_edges, ft, el, er, grad_out, num_heads, head_dim, negative_slope, num_dst, status_word};
 #define APT_RUN(T)                                                                                          \
   do {                                                                                                      \
     if (!edges_valid && (rc = gat_weights<T>(q, g, nullptr, s)) != APT_OK) return rc;                       \
-    return gat_backward<T>(q, g, ws, (char*)workspace, num_src, grad_ft, grad_el, grad_er, s);              \
+    return gat_backward<T>(q, g, wide, ws, (char*)workspace, num_src, grad_ft, grad_el, grad_er, s);              \
   } while (0)
   switch (dtype) {
     case APT_F32: APT_RUN(float);

@@ -309,9 +309,9 @@ __device__ __forceinline__ void slice_add(Acc<VE>& acc, const EdgeSlice<T, VE, O
 }
 
 // The sums of the edges read side by side meet, and the lanes of the first of them write the row's column block.
-template <typename T, int VE, int VPL, bool WIDENED>
-__device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], const int (&col)[VPL], int d, int c0, int nvec, int lpe, int lpr, int vl,
-                                           int epi, unsigned gmask) {
+template <typename T, int VE, int VPL, int OP, bool WIDENED>
+__device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[VPL], const int (&col)[VPL], const int (&head)[VPL], int d, int c0, int nvec, int lpe,
+                                           int lpr, int vl, int epi, unsigned gmask) {
 #pragma unroll 1
   for (int o = lpe; o < lpr; o <<= 1)
 #pragma unroll
@@ -320,8 +320,12 @@ __device__ __forceinline__ void rows_write(const RowArgs<T>& a, Acc<VE> (&acc)[V
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     if (c0 + vl + i * lpe >= nvec) continue;
-    if constexpr (WIDENED) store_some<T, VE>(a.out + (int64_t)d * a.width + col[i], acc[i].template rounded<T>(), (int)a.width - col[i]);
-    else store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
+    if constexpr (WIDENED) {
+      // weighted rows are widened head by head
+      const int heads = OP == kUMulW ? (int)a.edata_dim : 1, h = OP == kUMulW ? head[i] : 0;
+      const int from = OP == kUMulW ? (int)a.feat_dim / heads : 0, to = (int)a.width / heads;
+      store_some<T, VE>(a.out + (int64_t)d * a.width + col[i] - h * (from - to), acc[i].template rounded<T>(), to - (col[i] - h * from));
+    } else store_pack<T, VE>(a.out + (int64_t)d * a.feat_dim + col[i], acc[i].template rounded<T>());
   }
 }
 
@@ -545,11 +549,11 @@ k_spmm_rows(const __grid_constant__ RowArgs<T> a) {
           }
           c0 = cc;
           if (cc + lpe * VPL < nvec) {
-            rows_write<T, VE, VPL, WIDENED>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
+            rows_write<T, VE, VPL, OP, WIDENED>(a, acc, col, head, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
           }
         }
       }
-      rows_write<T, VE, VPL, WIDENED>(a, acc, col, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
+      rows_write<T, VE, VPL, OP, WIDENED>(a, acc, col, head, d, c0, nvec, lpe, LPR, vl, EPI, GMASK);
     }
     if (items) {
       it += warps;
@@ -599,7 +603,7 @@ static int launch_rows_ve(const RowArgs<T>& a, cudaStream_t s) {
   if constexpr (OP == kCopyU || OP == kUMulW) {
     if (stream_fits(OP, a.split.ve * (int)sizeof(T), a.feat_dim, sizeof(T), OP == kCopyU ? 1 : (int)a.edata_dim, a.num_edges, a.mode == kFixed || a.mode == kRanges)) return launch_stream<T, OP>(a, s);
   }
-  if constexpr (OP == kCopyU)
+  if constexpr (OP == kCopyU || OP == kUMulW)
     if (a.width) return launch_rows_vpl<T, 16 / sizeof(T), OP, true>(a, s);
   switch (a.split.ve * (int)sizeof(T)) {
     case 16: return launch_rows_vpl<T, 16 / sizeof(T), OP>(a, s);

@@ -111,7 +111,7 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
   const int warps = gridDim.x * plan.warps, warp = blockIdx.x * plan.warps + w;
   const uint32_t row_bytes = plan.row_bytes;
   unsigned char* const ring = shared + w * plan.warp_bytes;
-  float* const weights = (float*)(ring + 2 * GE * kSlot);      // [2][32][heads]; WIDENED: the row that is written
+  float* const weights = (float*)(ring + 2 * GE * kSlot);      // [2][32][heads]; WIDENED: the row that is written behind them
 
   // the lane's slices of 16 bytes, 32 apart; in kDots a head's slices have a power of two of lanes (plan.lph)
   int col[VPL], head[VPL];
@@ -191,15 +191,17 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
     for (int i = 0; i < VPL; ++i) acc[i].zero();
   };
   clear();
+  const int part = WIDENED ? (int)a.width / heads : 0, part_more = WIDENED ? (int)a.feat_dim / heads - part : 0;
+  const uint32_t part_inverse = WIDENED && kWeights ? (uint32_t)(((1ull << 31) + part - 1) / part) : 0u;
   auto write = [&](uint32_t d) {
     if constexpr (WIDENED) {
-      T* const row = (T*)weights;
+      T* const row = (T*)(weights + (kWeights ? 64 * heads : 0));
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < VPL; ++i)
         if (valid[i]) store_pack<T, VE>(row + col[i], acc[i].template rounded<T>());
       __syncwarp();
-      store_row(a.out + (uint64_t)d * a.width, row, (int)a.width, lane);
+      store_row(a.out + (uint64_t)d * a.width, row, (int)a.width, lane, kWeights ? part_inverse : 0u, part_more);
       return;
     }
 #pragma unroll
@@ -508,7 +510,7 @@ static int launch_stream(const RowArgs<T>& a, cudaStream_t s) {
 template <typename T, int OP>
 static int launch_stream(const RowArgs<T>& a, cudaStream_t s) {
   const bool one_slice = stream_one_slice(OP, a.feat_dim, sizeof(T), (int)a.edata_dim);
-  if constexpr (OP == kCopyU)
+  if constexpr (OP == kCopyU || OP == kUMulW)
     if (a.width) return one_slice ? launch_stream<T, OP, 1, true>(a, s) : launch_stream<T, OP, 2, true>(a, s);
   return one_slice ? launch_stream<T, OP, 1, false>(a, s) : launch_stream<T, OP, 2, false>(a, s);
 }

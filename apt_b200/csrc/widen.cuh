@@ -32,6 +32,23 @@ inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num
   return slice == 2 || row >= (slice == 4 ? 384 : 768) || (slice == 4 && row >= 64 && row <= 128 && num_edges >= 2 * kWidenEdges);
 }
 
+// The same for the attention layer, whose rows are widened head by head: in the forward the sources' (num_dst 0), in the backward both sides', for
+// the dots as well as for the walk. us of forward and backward, rows as they are -> widened, 15 edges a destination:
+//   900 000 edges, 150 000 sources   bf16 4 x 47 886 -> 383, 1 x 47 275 -> 175, 4 x 18 320 -> 263, 4 x 10 210 -> 192; fp32 4 x 47 1004 -> 460, 1 x 47 275 -> 222
+//   900 000, 600 000 sources         bf16 4 x 47 1258 -> 610, 1 x 47 377 -> 304; fp32 4 x 47 1349 -> 781; there fp32 1 x 47 (walk and dots 272 -> 277) and
+//     bf16 4 x 18 (305 -> 315) stay as they are, and the forwards of 4-byte accesses (fp32 4 x 47 223 -> 235)
+//   150 000, 25 000 sources          bf16 4 x 47 205 -> 103, fp32 4 x 47 194 -> 112; 300 000, 50 000 fp32 1 x 47 120 -> 103. Below kWidenGatBytes the host's
+//     90 us are what such a layer takes.
+//   Accesses of 8 bytes, backward alone: bf16 4 x 12 87 -> 97, fp32 8 x 10 219 -> 217
+constexpr int64_t kWidenGatBytes = 32 << 20;      // that the edges read
+inline bool widen_gat_pays(int64_t head_dim, int heads, size_t esz, int64_t num_src, int64_t num_edges, bool backward) {
+  const int64_t row = head_dim * (int64_t)esz;
+  const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
+  if (slice > 4 || row < 16 || row * heads > kWidenMost || num_src <= 0 || num_edges < kWidenEdges || num_edges * row * heads < kWidenGatBytes) return false;
+  if (slice == 2) return num_edges >= num_src;
+  return backward ? num_edges / (row * heads >= 384 ? 1 : 2) >= num_src : row * heads >= 128 && num_edges / 4 >= num_src;
+}
+
 // `out`: num_rows * ceil(row_bytes / 16) slices, 16-byte aligned. `in` is aligned to its elements of 2 or 4 bytes.
 int widen_rows(const void* in, int64_t num_rows, int64_t row_bytes, void* out, cudaStream_t s);
 
@@ -64,20 +81,23 @@ __device__ __forceinline__ void store_some(T* p, const Pack<T, VE>& r, int n) {
 
 // A row of n elements that a warp has in shared memory, to any element's address: side by side lanes write side by side words. (k_spmm_stream, whose
 // stores are in its loop many times over: lanes that write their slices themselves 244 us instead of 161 for bf16 x 251, four words a lane at a
-// time 235. As a run time branch beside aligned stores they had cost rows of 256 bf16 81 -> 110.)
+// time 235, slices of 4 x 47 weighted ones put together in shared memory 450 instead of 145. As a run time branch beside aligned stores they had
+// cost rows of 256 bf16 81 -> 110.)
+// Weighted rows are in parts of `part` elements with `more` behind each; inverse: ceil(2^31 / part), else 0.
 template <typename T>
-__device__ __forceinline__ void store_row(T* out, const T* row, int n, int lane) {
+__device__ __forceinline__ void store_row(T* out, const T* row, int n, int lane, uint32_t inverse, int more) {
+  auto at = [&](int t) { return inverse ? t + (int)__umulhi(2u * t + 1u, inverse) * more : t; };
   if constexpr (sizeof(T) == 2) {
     const unsigned short* const h = (const unsigned short*)row;
     const int odd = (int)((uintptr_t)out >> 1 & 1), words = (n - odd) >> 1;
     unsigned int* const w = (unsigned int*)(out + odd);
 #pragma unroll 1
-    for (int t = lane; t < words; t += 32) w[t] = (unsigned int)h[odd + 2 * t] | (unsigned int)h[odd + 2 * t + 1] << 16;
+    for (int t = lane; t < words; t += 32) w[t] = (unsigned int)h[at(odd + 2 * t)] | (unsigned int)h[at(odd + 2 * t + 1)] << 16;
     if (odd && lane == 0) out[0] = row[0];
-    if ((n - odd & 1) && lane == 31) out[n - 1] = row[n - 1];
+    if ((n - odd & 1) && lane == 31) out[n - 1] = row[at(n - 1)];
   } else {
 #pragma unroll 2
-    for (int t = lane; t < n; t += 32) out[t] = row[t];
+    for (int t = lane; t < n; t += 32) out[t] = row[at(t)];
   }
 }
 

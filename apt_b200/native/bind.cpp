@@ -65,6 +65,15 @@ void* mut(const Tensor& t) { return t.numel() ? t.mutable_data_ptr() : nullptr; 
 int32_t* status_word(const Tensor& words) { return (int32_t*)(words.mutable_data_ptr<int64_t>() + words.numel() - 1); }
 
 Tensor scratch(const Tensor& like, size_t bytes) { return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)); }
+// Scratch that a call does without where there is none: undefined then.
+Tensor room_for(const Tensor& like, size_t bytes) {
+  if (!bytes) return Tensor();
+  try {
+    return scratch(like, bytes);
+  } catch (const c10::OutOfMemoryError&) {
+    return Tensor();
+  }
+}
 
 // ------------------------------------------------------------------------------------------ SpMM / SDDMM
 Tensor spmm(int op, const Tensor& coo_row, const Tensor& coo_col, const OptTensor& input, const OptTensor& edata,
@@ -97,17 +106,9 @@ Tensor spmm(int op, const Tensor& coo_row, const Tensor& coo_col, const OptTenso
     bytes = apt_spmm_workspace_bytes(shape[0], edges);
     ws = scratch(out, bytes);
   }
-  // room for widened input rows; without it the sum does without
-  size_t wide_bytes = op == 0 && input && shape[0] > 0 ? apt_spmm_widened_bytes(code, edges, in.size(0), dim, (int)shape[1]) : 0;
-  Tensor wide;
-  if (wide_bytes) {
-    try {
-      wide = scratch(out, wide_bytes);
-    } catch (const c10::OutOfMemoryError&) {
-      wide_bytes = 0;
-    }
-  }
-  if (wide_bytes) {
+  const size_t wide_bytes = op == 0 && input && shape[0] > 0 ? apt_spmm_widened_bytes(code, edges, in.size(0), dim, (int)shape[1]) : 0;
+  const Tensor wide = room_for(out, wide_bytes);
+  if (wide.defined()) {
     check(apt_spmm_copy_u_widened(code, ptr(row), ptr(col), edges, data(in), in.size(0), dim, ptr(eoff), ptr(ioff), ptr(ooff),
                                   (int)eoff.numel() - 1, shape[0], (int)shape[1], (int)shape[2], mut(out), wide.mutable_data_ptr(),
                                   wide_bytes, bytes ? ws.mutable_data_ptr() : nullptr, bytes, stream()));
@@ -246,9 +247,11 @@ std::tuple<Tensor, Tensor, Tensor> gat_forward(const Tensor& coo_row, const Tens
   }
   const size_t bytes = apt_gat_edges_bytes(num_dst, g.edges, (int)g.heads);
   const Tensor edges = scratch(ft, bytes);
-  check(apt_gat_forward(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), (int)g.heads, g.head_dim, (float)slope,
-                        num_dst, mut(out), want_attention ? mut(attn) : nullptr, edges.mutable_data_ptr(), bytes,
-                        status_word(words), stream()));
+  const size_t wide_bytes = apt_gat_widened_bytes(g.code, g.edges, g.num_src, 0, (int)g.heads, g.head_dim);
+  const Tensor wide = room_for(ft, wide_bytes);
+  check(apt_gat_forward_widened(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), (int)g.heads, g.head_dim, (float)slope,
+                                g.num_src, num_dst, mut(out), want_attention ? mut(attn) : nullptr, edges.mutable_data_ptr(), bytes,
+                                wide.defined() ? wide.mutable_data_ptr() : nullptr, wide_bytes, status_word(words), stream()));
   return {out, attn, edges};
 }
 
@@ -265,9 +268,12 @@ std::tuple<Tensor, Tensor, Tensor> gat_backward(const Tensor& coo_row, const Ten
   const Tensor edges = edges_of_forward ? *edges_of_forward : scratch(ft, edges_bytes);
   const size_t bytes = apt_gat_backward_workspace_bytes(g.num_src, g.edges, (int)g.heads);
   const Tensor ws = scratch(ft, bytes);
-  check(apt_gat_backward(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), data(grad), (int)g.heads, g.head_dim,
-                         (float)slope, g.num_src, g.num_dst, mut(grad_ft), mut(grad_el), mut(grad_er), edges.mutable_data_ptr(),
-                         edges_bytes, edges_of_forward ? 1 : 0, ws.mutable_data_ptr(), bytes, status_word(words), stream()));
+  const size_t wide_bytes = g.num_dst ? apt_gat_widened_bytes(g.code, g.edges, g.num_src, g.num_dst, (int)g.heads, g.head_dim) : 0;
+  const Tensor wide = room_for(ft, wide_bytes);
+  check(apt_gat_backward_widened(g.code, ptr(row), ptr(col), g.edges, data(ft), data(el), data(er), data(grad), (int)g.heads, g.head_dim,
+                                 (float)slope, g.num_src, g.num_dst, mut(grad_ft), mut(grad_el), mut(grad_er), edges.mutable_data_ptr(),
+                                 edges_bytes, edges_of_forward ? 1 : 0, ws.mutable_data_ptr(), bytes,
+                                 wide.defined() ? wide.mutable_data_ptr() : nullptr, wide_bytes, status_word(words), stream()));
   return {grad_ft, grad_el, grad_er};
 }
 

@@ -513,6 +513,33 @@ int apt_gat_backward(int dtype, const int64_t* coo_row, const int64_t* coo_col,
                      void* workspace, size_t workspace_bytes,
                      int32_t* status_word, void* stream);
 
+/* The two for heads that are no whole number of 16-byte slices, whose rows are
+ * copied to such a pitch first (apt_spmm_copy_u_widened). apt_gat_widened_bytes is
+ * what that takes, or 0 where it does not pay: of a forward with num_dst 0, else
+ * of a backward. Without a buffer they are the two above. */
+size_t apt_gat_widened_bytes(int dtype, int64_t num_edges, int64_t num_src,
+                             int64_t num_dst, int num_heads, int64_t head_dim);
+int apt_gat_forward_widened(int dtype, const int64_t* coo_row,
+                            const int64_t* coo_col, int64_t num_edges,
+                            const void* ft, const void* el, const void* er,
+                            int num_heads, int64_t head_dim,
+                            float negative_slope, int64_t num_src,
+                            int64_t num_dst, void* out, void* out_attn,
+                            void* edges, size_t edges_bytes, void* widened,
+                            size_t widened_bytes, int32_t* status_word,
+                            void* stream);
+int apt_gat_backward_widened(int dtype, const int64_t* coo_row,
+                             const int64_t* coo_col, int64_t num_edges,
+                             const void* ft, const void* el, const void* er,
+                             const void* grad_out, int num_heads,
+                             int64_t head_dim, float negative_slope,
+                             int64_t num_src, int64_t num_dst, void* grad_ft,
+                             void* grad_el, void* grad_er, void* edges,
+                             size_t edges_bytes, int edges_valid,
+                             void* workspace, size_t workspace_bytes,
+                             void* widened, size_t widened_bytes,
+                             int32_t* status_word, void* stream);
+
 /* ------------------------------------------- SNP virtual nodes (SAGE / GCN)
  * The id arithmetic of the SNP strategy with virtual nodes: neighbour i of
  * local destination i / fanout, owned by rank o, becomes the virtual node

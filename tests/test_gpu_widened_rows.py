@@ -95,3 +95,35 @@ def test_rows_that_stay_as_they_are():
     assert bytes_of(1, 1_000_000, 150_000, 102, 1) == 0         # grouped, read four bytes a lane
     assert bytes_of(1, 1_000_000, 67_000, 101, -1) == 0         # unknown block
     assert bytes_of(1, 1_000_000, 67_000, 101, 2) == 67_000 * 208
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,head_dim", [(4, 47), (1, 47), (8, 10), (4, 10), (3, 33), (2, 255), (1, 601), (9, 18), (17, 9)])
+def test_attention_of_heads_that_are_no_whole_slices(dtype, heads, head_dim):
+    """Against the same heads with columns of zeros behind them, which are read as they are."""
+    dst, src, per = 20_003, 60_001, 14
+    row, col, g = _block(dst, src, per, True, head_dim)
+    keep = torch.rand(dst * per, generator=g, device="cuda") < 0.95
+    row, col = row[keep], col[keep]
+    code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
+    size = heads * head_dim * dtype.itemsize
+    if head_dim % 2:
+        assert (lib.apt_gat_widened_bytes(code, row.numel(), src, dst, heads, head_dim) > 0) == (row.numel() * size >= 32 << 20 and size <= 4096)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(dtype)
+    ft, el, er, grad = normal(src, heads, head_dim), normal(src, heads, 1), normal(dst, heads, 1), normal(dst, heads, head_dim)
+    per_slice = 16 // dtype.itemsize
+    more = -head_dim % per_slice
+    pad = lambda x: torch.nn.functional.pad(x, (0, more)).contiguous()
+
+    def layer(ft, grad):
+        leaves = [ft.detach().requires_grad_(), el.detach().requires_grad_(), er.detach().requires_grad_()]
+        out = ops.GATEdgeSoftmaxSum.apply(row, col, *leaves, dst, 0.2)
+        return (out.detach(),) + torch.autograd.grad(out, leaves, grad)
+
+    got, want = layer(ft, grad), layer(pad(ft), pad(grad))
+    want = (want[0][..., :head_dim], want[1][..., :head_dim], want[2], want[3])
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and torch.isfinite(a).all()
+        # the same terms in another order: fp32 sums a few 2^-24 of their terms apart, and then at most one rounding further
+        a, b = a.double(), b.double()
+        assert ((a - b).abs() <= 2 * _EPS[dtype] * b.abs() + 2e-5 * b.abs().max()).all()
