@@ -28,6 +28,7 @@
 //                   row); k_dst_slots gives the rows their places; k_gat_scores writes the order. As launches of
 //                   their own the first and the last pass took 23 + 16 us.
 //   k_gat_source    grad_el in T
+//   k_widen         heads that are no whole slices, laid out so first (widen.cuh)
 //
 // k_gat_alone and k_gat_alone_backward serve the two entry points that have no buffer for weights, k_gat_narrow forwards of
 // narrow rows that nobody will ask for a backward.

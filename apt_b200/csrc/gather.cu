@@ -138,7 +138,7 @@ static int vec_width(uint64_t bits) {
 }
 
 // Blocks an SM for a gather that runs beside other kernels: enough reads over the host link for its full rate (one block's
-// warps have 16 KiB each in flight, of the 80 KB that rate times latency asks of the whole chip), and room for the others,
+// warps have 4 KiB each in flight, of the 80 KB that rate times latency asks of the whole chip), and room for the others,
 // which at the full grid wait until it ends.
 constexpr int kNarrowBlocks = 1;
 

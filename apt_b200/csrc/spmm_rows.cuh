@@ -5,8 +5,7 @@
 //
 //   lane split   `lpe` lanes cover one input row (VPL slices of up to 16 bytes each), `ep` edges of the
 //                row are read side by side, and their partial sums meet in a shuffle butterfly at the
-//                end. Narrow rows need the second factor: with 4 lanes to a 64-byte row and one edge at a
-//                time a row of 100 edges is 100 / 4 rounds of load latency.
+//                end. The second factor is for narrow rows that are too few to fill the chip side by side (row_split).
 //   in flight    the loads of U edges (U * VPL slices a lane) are issued before any of them is added;
 //                the next row's bounds and source indexes are fetched while this row's slices are
 //                on their way, so that a short row costs one round of latency and not three. Full rounds carry
@@ -18,7 +17,7 @@
 //                block of 1024 threads per long row, the form before this, kept 26 of 148 SMs busy for
 //                62 us behind the row kernel.
 //
-// Wide rows of many edges have a kernel of their own (spmm_stream.cuh).
+// Wide rows of many edges have a kernel of their own (spmm_stream.cuh). Rows that are no whole slices may have been laid out anew (widen.cuh).
 //
 // Where a row's edges are (`mode`):
 //   kFixed    every row has `fixed` consecutive edges: what a fanout sampler produces. No table.
