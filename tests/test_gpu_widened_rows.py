@@ -30,7 +30,7 @@ def _expect(got, row, col, x, dst, most):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("dim", [9, 17, 18, 31, 61, 101, 119, 137, 197, 198, 251, 255, 301, 511])
+@pytest.mark.parametrize("dim", [9, 17, 18, 31, 61, 101, 119, 137, 197, 198, 251, 255, 301, 511, 1001])
 @pytest.mark.parametrize("segments", [1, 3])
 def test_sums_in_no_order(dtype, dim, segments):
     # 100 000 edges and more go the widened way where the width does (kWidenEdges, twice that)
@@ -43,6 +43,42 @@ def test_sums_in_no_order(dtype, dim, segments):
     for k, (r, c, _) in enumerate(parts):
         most = int(torch.bincount(c).max()) + 40
         _expect(got[k * dst:(k + 1) * dst], r, c, x[k * src:(k + 1) * src], dst, most)
+
+
+@pytest.mark.parametrize("dtype,dim", [(torch.float32, 31), (torch.float32, 101), (torch.bfloat16, 17), (torch.bfloat16, 61), (torch.bfloat16, 119),
+                                       (torch.float16, 251), (torch.float32, 251), (torch.float16, 601)])
+def test_rows_that_many_edges_share(dtype, dim):
+    """Rows cut into items, or into stretches of several warps: their parts meet in scratch."""
+    dst, src, per = 30_011, 9_001, 8
+    row, col, g = _block(dst, src, per, False, dim)
+    hub = torch.rand(dst * per, generator=g, device="cuda")
+    col[hub < 0.2], col[(hub > 0.2) & (hub < 0.21)] = 5, 29_000
+    x = torch.randn(src, dim, generator=g, device="cuda").to(dtype)
+    off = lambda n: torch.tensor([0, n], device="cuda")
+    got = ops.spmm_copy_u_sum(row, col, x, off(dst * per), off(src), off(dst))
+    _expect(got, row, col, x, dst, 4096)      # sums of sums: no term goes through more additions than that
+
+
+@pytest.mark.parametrize("heads,head_dim", [(4, 47), (1, 33), (8, 17)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_gradients_of_sources_that_many_edges_share(dtype, heads, head_dim):
+    dst, src, per = 30_011, 20_001, 15
+    row, col, g = _block(dst, src, per, True, head_dim)
+    hub = torch.rand(dst * per, generator=g, device="cuda")
+    row[hub < 0.2], row[(hub > 0.2) & (hub < 0.21)] = 7, 19_000
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(dtype)
+    ft, el, er, grad = normal(src, heads, head_dim), normal(src, heads, 1), normal(dst, heads, 1), normal(dst, heads, head_dim)
+    leaves = [t.requires_grad_() for t in (ft, el, er)]
+    out = ops.GATEdgeSoftmaxSum.apply(row, col, *leaves, dst, 0.2)
+    got = torch.autograd.grad(out, leaves, grad)[0].double()
+    score = torch.nn.functional.leaky_relu(el.detach().double()[row, :, 0] + er.detach().double()[col, :, 0], 0.2).view(dst, per, heads)
+    weight = torch.softmax(score, 1).view(-1, heads, 1)
+    zeros = torch.zeros(src, heads, head_dim, dtype=torch.float64, device="cuda")
+    want = zeros.index_add(0, row, weight * grad.double()[col])
+    size = zeros.index_add(0, row, weight * grad.double()[col].abs())
+    # weights within a few 2^-24 of themselves (an exponential, a sum of 15 and a quotient, from fp32 scores of up to 8), fp32 sums of up to 4096
+    # additions a term, one rounding
+    assert ((got - want).abs() <= size * (4096 + 64) * 2.0 ** -24 + want.abs() * _EPS[dtype] * 1.01 + 1e-7).all()
 
 
 @pytest.mark.parametrize("dim", [17, 31, 61, 119, 251, 257])
