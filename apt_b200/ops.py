@@ -574,14 +574,19 @@ def unique_sorted(ids: torch.Tensor, id_lo: int, id_hi: int):
     return uniq[:num_unique], inv
 
 
-def _unique_workspace(rng, ws_name):
-    """The cached bitmap over a range of ids, zero."""
+def _unique_bitmap(rng, ws_name):
+    """The cached bitmap over a range of ids, as it was left."""
     nbytes = lib.apt_unique_workspace_bytes(rng)
     if ws_name != "unique":
         # a bitmap of its own per id range: a captured graph that replays this call must find
         # the layout it was captured with, whatever ran on the shared bitmap in between
         ws_name = f"{ws_name}:{rng}"
-    ws = STATE.workspace(ws_name, nbytes)
+    return STATE.workspace(ws_name, nbytes)
+
+
+def _unique_workspace(rng, ws_name):
+    """The same, zero."""
+    ws = _unique_bitmap(rng, ws_name)
     if getattr(ws, "_apt_clean_range", None) != rng:
         # the bitmap has to be zero once per id range (the layout follows the range);
         # every call then leaves it zero again
@@ -609,6 +614,7 @@ def _unique_ids(ids, n_dev, per, id_lo, id_hi, count_out, ws_name):
     rng = int(id_hi) - int(id_lo)
     uniq = torch.empty(min(n, max(rng, 0)), dtype=torch.int64, device=ids.device)
     ws = _unique_workspace(rng, ws_name)
+    ws._apt_clean_range = None      # until the inverse has it zero again
     check(lib.apt_unique_ids(_ptr(ids), n, _ptr(n_dev), int(per), int(id_lo), int(id_hi), _ptr(ws), ws.numel(), _ptr(uniq), _ptr(count_out),
                              STATE.status_ptr(), _stream()))
     return uniq
@@ -619,24 +625,32 @@ def _unique_inverse(ids, n_dev, per, id_lo, id_hi, ws_name, uniq=None, uniq_n=No
     """The inverse of _unique_ids, on side stream `side` (which the caller joins) or the current one. From the same launch:
     with `sizes` and `offsets` what _bucket leaves in a world of one rank, of the ids or of the distinct ones (`uniq`, whose count is uniq_n);
     with `head` the list concat_ids(head, head_n, uniq, uniq_n, all_out, look_up). Returns (inverse, permutation or None, list or None)."""
-    if sizes is not None and STATE.shuffle_min_vids is None:
-        raise RuntimeError("register_min_vids has not been called")
-    n, dev = ids.numel(), ids.device
-    inv = torch.empty(n, dtype=torch.int64, device=dev)
-    n_uniq = 0 if uniq is None else uniq.numel()
-    perm = None if sizes is None else torch.empty(n if uniq is None else n_uniq, dtype=torch.int64, device=dev)
-    listed = None if head is None else torch.empty(head.numel() + n_uniq, dtype=torch.int64, device=dev)
-    if perm is not None and perm.numel() == 0:
-        sizes.zero_()
-        offsets.zero_()
-        sizes = offsets = None
-    ws = _unique_workspace(int(id_hi) - int(id_lo), ws_name)
-    with contextlib.nullcontext() if side is None else STATE.beside(side):
-        check(lib.apt_unique_inverse(
-            _ptr(ids), n, _ptr(n_dev), int(per), int(id_lo), int(id_hi), _ptr(ws), ws.numel(), _ptr(inv), _ptr(uniq), n_uniq, _ptr(uniq_n),
-            _ptr(perm), _ptr(sizes), _ptr(offsets),
-            _ptr(head), 0 if head is None else head.numel(), _ptr(head_n), _ptr(listed), _ptr(all_out),
-            *(_row_tables() if look_up else (None, 0, 0, 0)), STATE.status_ptr(), _stream()))
+    rng = int(id_hi) - int(id_lo)
+    ws = _unique_bitmap(rng, ws_name)
+    try:
+        if sizes is not None and STATE.shuffle_min_vids is None:
+            raise RuntimeError("register_min_vids has not been called")
+        n, dev = ids.numel(), ids.device
+        inv = torch.empty(n, dtype=torch.int64, device=dev)
+        n_uniq = 0 if uniq is None else uniq.numel()
+        perm = None if sizes is None else torch.empty(n if uniq is None else n_uniq, dtype=torch.int64, device=dev)
+        listed = None if head is None else torch.empty(head.numel() + n_uniq, dtype=torch.int64, device=dev)
+        if perm is not None and perm.numel() == 0:
+            sizes.zero_()
+            offsets.zero_()
+            sizes = offsets = None
+        with contextlib.nullcontext() if side is None else STATE.beside(side):
+            check(lib.apt_unique_inverse(
+                _ptr(ids), n, _ptr(n_dev), int(per), int(id_lo), int(id_hi), _ptr(ws), ws.numel(), _ptr(inv), _ptr(uniq), n_uniq, _ptr(uniq_n),
+                _ptr(perm), _ptr(sizes), _ptr(offsets),
+                _ptr(head), 0 if head is None else head.numel(), _ptr(head_n), _ptr(listed), _ptr(all_out),
+                *(_row_tables() if look_up else (None, 0, 0, 0)), STATE.status_ptr(), _stream()))
+    except BaseException:
+        # the distinct ids' counts are still in the bitmap, which a captured graph may take next without looking
+        if not torch.cuda.is_current_stream_capturing():
+            lib.apt_unique_workspace_init(_ptr(ws), ws.numel(), _stream())
+        raise
+    ws._apt_clean_range = rng
     return inv, perm, listed
 
 

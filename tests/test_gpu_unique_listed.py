@@ -74,3 +74,45 @@ def test_ids_outside_and_rows_that_do_not_exist():
         ops.check_status()
     _, _, all_ids = both(torch.empty(0, dtype=torch.int64, device="cuda"), 6, False)
     assert word.tolist() == [0, 2] and host(all_ids).tolist() == [1, 2]
+
+
+def test_a_second_half_that_fails():
+    """The distinct ids by themselves: what they leave in the bitmap is gone before anybody else's, a captured graph's too."""
+    reset_world()
+    lo, hi = 7, 300_000
+    ids = np.random.default_rng(3).integers(lo, hi, 20_000).astype(np.int64)
+    ids_dev, word = dev(ids), torch.zeros(4, dtype=torch.int64, device="cuda")
+    want, want_inv = np.unique(ids, return_inverse=True)
+
+    def both():
+        uniq = ops._unique_ids(ids_dev, None, 1, lo, hi, word[0:1], "unique_half")
+        return uniq, ops._unique_inverse(ids_dev, None, 1, lo, hi, "unique_half")[0]
+
+    def right(uniq, inv):
+        torch.cuda.synchronize()
+        return int(word[0]) == len(want) and np.array_equal(host(uniq)[:len(want)], want) and np.array_equal(host(inv), want_inv)
+
+    assert right(*both())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        of_graph = both()
+    saved, ops.STATE.shuffle_min_vids = ops.STATE.shuffle_min_vids, None
+    try:
+        for then in ("call", "graph"):
+            ops._unique_ids(ids_dev, None, 1, lo, hi, word[0:1], "unique_half")
+            with pytest.raises(RuntimeError, match="register_min_vids"):
+                ops._unique_inverse(ids_dev, None, 1, lo, hi, "unique_half", sizes=word[1:3], offsets=word[3:4])
+            # (the bitmap is looked at before it is used: counts left in it would send the next call beyond its buffers)
+            torch.cuda.synchronize()
+            assert int(ops._unique_bitmap(hi - lo, "unique_half").count_nonzero()) == 0
+            if then == "graph":
+                graph.replay()
+                assert right(*of_graph)
+            else:
+                assert right(*both())
+        # a first half whose second never came: the next call starts from an empty bitmap
+        ops._unique_ids(ids_dev, None, 1, lo, hi, word[0:1], "unique_half")
+        assert right(*both())
+    finally:
+        ops.STATE.shuffle_min_vids = saved
+    ops.check_status()
