@@ -659,7 +659,7 @@ static int gat_forward(const GatProblem& q, const GatEdges& g, const GatWide& wi
   SpmmWs ws{};
   ws.range = g.range;
   const RowArgs<T> a{q.row, (const T*)(wide.dim ? wide.ft : q.ft), (const T*)g.weight, q.H, dim, SegTable{nullptr, nullptr, nullptr, 1}, q.num_dst,
-                     q.E, ws, (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u,
+                     q.E, ws, (T*)out, kRanges, 0, row_split(dim, ve, q.E, q.num_dst, false), (int)dim, g.none, q.status, q.col, nullptr, nullptr, 0u,
                      wide.dim ? q.H * q.Dh : 0};
   ProfScope prof("gat_rows", s);
   return launch_spmm_rows<T>(kUMulW, a, s);
@@ -709,7 +709,7 @@ static int gat_backward(const GatProblem& as_given, const GatEdges& g, const Gat
   if (wide.dim) q.ft = wide.ft, q.grad_out = wide.grad, q.Dh = wide.dim;
   const int64_t dim = q.H * q.Dh;
   const int ve = wide.dim ? 16 / sizeof(T) : slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.grad_out | (uintptr_t)grad_ft, sizeof(T));
-  const RowSplit split = row_split(dim, ve, q.E, num_src);
+  const RowSplit split = row_split(dim, ve, q.E, num_src, true);
   const OrderKind kind = order_kind(kUMulW, ve * (int)sizeof(T), dim, sizeof(T), q.H, q.E);
   APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
   int rc;

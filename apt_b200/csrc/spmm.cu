@@ -647,7 +647,7 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
   uint64_t bits = (uint64_t)(feat_dim * esz) | (width ? 0 : (uintptr_t)out);
   if (op != kCopyE) bits |= (uintptr_t)input;
   if (op != kCopyU && edata_dim == feat_dim) bits |= (uintptr_t)edata;
-  const RowSplit split = row_split(feat_dim, slice_elems(bits, (int)esz), E, num_rows);
+  const RowSplit split = row_split(feat_dim, slice_elems(bits, (int)esz), E, num_rows, mode == kOrder || mode == kDevice);
   if (mode == kDevice || mode == kOrder) APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
   if (mode == kDevice) {
     const int rc = launch_probe(coo_col, E, st, num_rows, ws.probe, 0, ws.result, 1, s);

@@ -110,13 +110,16 @@ __host__ __device__ inline int item_edges(int deg) {
   return per;
 }
 
+constexpr int64_t kRowsManyOrdered = 3 << 13;
+
 // How rows are divided among lanes: slices of `ve` elements, `vpl` of them a lane.
 struct RowSplit {
   int ve, vpl;
   int lpe, ep;       // lanes to an edge, edges side by side: powers of two, lpe * ep <= 32
   int long_edges;    // longer rows are whole warps' work (kOrder)
 };
-inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t num_rows) {
+// ordered: the rows' edges come by a sort's list (kOrder), or may (kDevice).
+inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t num_rows, bool ordered) {
   RowSplit r;
   const int64_t nvec = feat_dim / ve;
   r.ve = ve;
@@ -131,9 +134,14 @@ inline RowSplit row_split(int64_t feat_dim, int ve, int64_t num_edges, int64_t n
   // bf16 x 128 32 -> 24.5 | 48 -> 36, x 64 22 -> 13 | 29.5 -> 24, fp32 x 64 30 -> 24 | 48 -> 36, x 32 21 -> 13.7 | 29 -> 23, 60 000 x 8 of bf16 x 10
   // 20.5 -> 8.1, 5 000 x 15 of fp32 x 64 6.7 -> 5.6; 1 000 x 15, which do not fill it, stay as they are (one by one 4.5 -> 5.1). Four
   // lanes to a row at least: with two, rows of very different lengths wait for one another (67 000 x 15 of bf16 x 4 11 -> 17 | 19 -> 27).
+  // The edges of long rows stay side by side: in a list, rows of more than kLongRowNarrow edges would all become items, and many edges one
+  // after another make the last wave of rows long. As many edges as go -> rows first, us: in a list fp32 x 32, 7 000 x 16 33 -> 33, x 20 34 -> 36; 15 000 x 16
+  // 38 -> 37, x 20 40 -> 42, x 32 48 -> 54; 60 000 x 24 86 -> 82, x 28 92 -> 97, x 40 115 -> 161; one after another fp32 x 16, 15 000 x 30 21 -> 20.4, x 50
+  // 24 -> 25, x 200 45 -> 59; 60 000 x 30 43 -> 32, x 50 54 -> 44.
+  const int64_t longest = !ordered ? 40 : num_rows >= kRowsManyOrdered ? 24 : 16;
   const int most = pow2_le(num_edges / (num_rows * 2), 32 / r.lpe);
   r.ep = 1;
-  while (r.ep < most && (r.lpe * r.ep < 4 || num_rows * r.lpe * r.ep * 2 <= (int64_t)kNumSMs * 24 * 32)) r.ep <<= 1;
+  while (r.ep < most && (num_edges > longest * num_rows || r.lpe * r.ep < 4 || num_rows * r.lpe * r.ep * 2 <= (int64_t)kNumSMs * 24 * 32)) r.ep <<= 1;
   r.long_edges = r.lpe * r.ep == 32 ? kLongRow : kLongRowNarrow;
   return r;
 }
