@@ -51,14 +51,16 @@ k_gat_dots_mma(const int64_t* __restrict__ row, const int64_t* __restrict__ col,
   const int lo = (int)min((int64_t)warp * chunk, E), hi = (int)min((int64_t)(warp + 1) * chunk, E);
   if (lo >= hi) return;
 
-  struct Batch {      // 32 edges, a lane to each
+  // 32 edges, a lane to each. Destinations stay below 2^31, whatever the ids are by now (they were looked at when the ranges were made, maybe a forward
+  // pass ago): tiles then rise until a group is done, and no edge's is that of the lanes behind the last one.
+  struct Batch {
     uint32_t src, dst, place;
   };
   auto load = [&](int base) {
     Batch b{0u, 0xffffffffu, kNoRank};
     const int e = base + lane;
     if (e < hi) {
-      b.src = (uint32_t)row[e], b.dst = (uint32_t)col[e];
+      b.src = (uint32_t)row[e], b.dst = min((uint32_t)col[e], 0x7fffffffu);
       if (b.src < num_src) b.place = (uint32_t)atomicAdd(src_count + spread(b.src), 1);
     }
     return b;

@@ -57,3 +57,22 @@ def test_infinite_rows_stay_with_their_edges():
     er_got, er_clean = (x.reshape(len(n), H) for x in (got[2], clean[2]))
     assert np.array_equal(er_got[others], er_clean[others]) and np.array_equal(er_got[:, [0, 2, 3]], er_clean[:, [0, 2, 3]])
     assert not np.isfinite(er_got[hit, 1]).any()
+
+
+def test_ids_that_have_changed_since_the_forward():
+    """The ranges are the forward's; what the destinations' ids have become since is read within its ends, and the pass comes to its end."""
+    H, D, n = 2, 64, [15] * 40
+    row, col, ft, el, er, go = _inputs(n, H, D, torch.bfloat16)
+    row, ids = dev(row), dev(col)
+    leaves = [dev(x, torch.bfloat16).view(-1, H, x.size // H // len(x)).requires_grad_() for x in (ft, el, er)]
+    layer = lambda: ops.GATEdgeSoftmaxSum.apply(row, ids, *leaves, len(n), 0.2)      # noqa: E731
+    out, grad = layer(), dev(go, torch.bfloat16)
+    want = torch.autograd.grad(out, leaves, grad, retain_graph=True)
+    kept = ids.clone()
+    for bad in (-1, -9, 2 ** 31 - 1, 2 ** 31, 2 ** 32 - 4, 2 ** 40 + 3, 39):
+        ids.data[5::16] = bad
+        torch.autograd.grad(out, leaves, grad, retain_graph=True)
+        torch.cuda.synchronize()
+        ids.data.copy_(kept)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(layer(), leaves, grad), want))
+    ops.check_status()
