@@ -3,15 +3,18 @@
 //
 // A warp takes a stretch of the edges, 16 of them (M) against 8 destinations (N) a step: the edges' rows come to shared memory by cp.async, two
 // groups on their way, the destinations' stay in registers while the edges, which are grouped, walk over them. Of the 16 x 8
-// products of a head one in eight is an edge's own; what the others cost is 32 instructions a group of 256 columns, where multiplying and
-// reducing across lanes took 46 an edge. The k of a product may be in any order, so a lane's share of two steps is 16 bytes side by
-// side in both operands: one load each. Sums are fp32 as they were: the gradients' distance from 64 bits is the same to seven digits.
+// products of a head one in eight is an edge's own; what the others cost is 16 instructions a group of 256 columns (bf16 32) and their additions, where
+// multiplying and reducing across lanes took 46 an edge. The k of a product may be in any order, so a lane's share of two steps is 16 bytes side by
+// side in both operands: one load each.
 //
-// Bound by rows out of L2 (43 us for a million rows of 512 bytes however they are fetched) and the atomics that count the
-// edges of every source for the sort behind. us of the dots, multiplied out -> here: bf16 4 x 64, 67 584 x 15 edges 75 -> 56, x 3 edges 40 -> 22,
-// 30 000 x 10 35 -> 21, 5 000 x 10 8.6 -> 6.0; f16 4 x 32, 40 000 x 15 32 -> 21, 2 x 32 20 -> 18, 2 x 32 x 3 edges 18.6 -> 6.3, bf16 1 x 32,
-// 55 721 x 17 28 -> 18; 1 000 x 10 of 8 x 32 4.9 -> 4.1. So they take every shape they can be built for. (Shared addresses worked out for
-// every access and a predicate for every row, 27 instructions an edge: 62 instead of 56.)
+// Sums are fp32 and no further from 64 bits than multiplied out (products()). 2-norm of the dots' error over theirs, multiplied out | here, normal values: bf16
+// 1 x 32 2.94e-8 | 2.82e-8, 4 x 64 3.93e-8 | 3.84e-8, 2 x 128 4.80e-8 | 4.70e-8, 1 x 256 5.50e-8 | 5.46e-8; f16 4 x 32 5.59e-8 | 5.44e-8, 4 x 64 6.21e-8 | 6.14e-8, 2 x 128
+// 6.77e-8 | 6.75e-8, 1 x 256 7.29e-8 | 7.23e-8. Accumulated in the tensor cores from step to step: bf16 1 x 32 3.9e-8, 4 x 64 6.5e-8, 1 x 256 2.3e-7, f16 1 x 256 3.4e-7.
+//
+// us of a backward pass, multiplied out -> here: bf16 4 x 64, 67 584 x 15 edges 190 -> 185, x 3 edges 87 -> 74, 30 000 x 10 86 -> 77; 4 x 32, 67 584 x 15 200 -> 160; 1 x 128
+// 193 -> 148; 1 x 32 111 -> 98; f16 8 x 32 213 -> 200, 30 000 x 10 97 -> 85; 2 x 64, 67 584 x 15 199 -> 150. (Accumulated in the tensor cores bf16 4 x 64 170, 4 x 32 150: the
+// products that make the cut good take 14 us of a million edges of 256 columns.) So they take every shape they can be built for. Shared addresses worked out for every
+// access and a predicate for every row, 27 instructions an edge, took the dots from 56 to 62.
 #pragma once
 
 #include "spmm_rows.cuh"
@@ -23,8 +26,8 @@ constexpr int kDotsBlocks = 2, kDotsEdges = 16, kDotsTile = 8;
 constexpr int dots_warps(int chunks) { return chunks == 8 ? 6 : chunks == 4 ? 10 : 14; }
 
 template <typename T>
-__device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, bool first) {
-  const float c0 = first ? 0.f : d[0], c1 = first ? 0.f : d[1], c2 = first ? 0.f : d[2], c3 = first ? 0.f : d[3];
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
+                                             float c0 = 0.f, float c1 = 0.f, float c2 = 0.f, float c3 = 0.f) {
   if constexpr (Elem<T>::kIsBf16)
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
@@ -33,6 +36,26 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// The products of 32 columns, two steps of 16. The tensor cores cut sums off where fp32 additions round, so that nothing is added up in them beyond a step, and
+// of 16-bit values whose own products are exact, which leaves the cut as the larger error, it is made good: what the same products leave of the sum.
+template <typename T>
+__device__ __forceinline__ void products(F2 (&sum)[2], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, uint32_t a4, uint32_t a5,
+                                         uint32_t a6, uint32_t a7, uint32_t b2, uint32_t b3) {
+  float p[4], q[4];
+  mma_16x8x16<T>(p, a0, a1, a2, a3, b0, b1);
+  mma_16x8x16<T>(q, a4, a5, a6, a7, b2, b3);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) sum[i] = f2_add(f2_pack(p[2 * i], p[2 * i + 1]), f2_pack(q[2 * i], q[2 * i + 1]));
+  if constexpr (Elem<T>::kIsBf16) {
+    float p_rest[4], q_rest[4];
+    mma_16x8x16<T>(p_rest, a0, a1, a2, a3, b0, b1, -p[0], -p[1], -p[2], -p[3]);
+    mma_16x8x16<T>(q_rest, a4, a5, a6, a7, b2, b3, -q[0], -q[1], -q[2], -q[3]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      sum[i] = f2_add(sum[i], f2_add(f2_pack(p_rest[2 * i], p_rest[2 * i + 1]), f2_pack(q_rest[2 * i], q_rest[2 * i + 1])));
+  }
 }
 
 // NC chunks of 32 columns to a row, CPH of them to a head.
@@ -117,13 +140,25 @@ k_gat_dots_mma(const int64_t* __restrict__ row, const int64_t* __restrict__ col,
 #pragma unroll
           for (int c = 0; c < NC; ++c) b[c] = __ldg((const uint4*)(own + c * 32));
         }
-        float acc[H][4];
+        F2 acc[H][2], part[4][2];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           const unsigned char* const p = (c & 1 ? get_odd : get_even) + half * kDotsEdges * kRow + (c & ~1) * 64;
           const uint4 x = *(const uint4*)p, y = *(const uint4*)(p + 8 * kRow);
-          mma_16x8x16<T>(acc[c / CPH], x.x, y.x, x.y, y.y, b[c].x, b[c].y, c % CPH == 0);
-          mma_16x8x16<T>(acc[c / CPH], x.z, y.z, x.w, y.w, b[c].z, b[c].w, false);
+          F2 sum[2];
+          products<T>(sum, x.x, y.x, x.y, y.y, b[c].x, b[c].y, x.z, y.z, x.w, y.w, b[c].z, b[c].w);
+          // in pairs, pairs of pairs, ...
+#pragma unroll
+          for (int level = 0; level < 4; ++level) {
+            const bool pair = (c % CPH + 1) % (2 << level) == 0 && (1 << level) < CPH;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (pair) sum[i] = f2_add(part[level][i], sum[i]);
+              else part[level][i] = sum[i];
+            }
+            if (!pair) break;
+          }
+          if (c % CPH == CPH - 1) acc[c / CPH][0] = sum[0], acc[c / CPH][1] = sum[1];
         }
         // an edge's own product is with the lane that has its destination's column
         float* const out = dots + (int64_t)(base + pos + g) * H;
@@ -133,7 +168,11 @@ k_gat_dots_mma(const int64_t* __restrict__ row, const int64_t* __restrict__ col,
           if ((s >> 1) == (uint32_t)t) {
             float v[H];
 #pragma unroll
-            for (int h = 0; h < H; ++h) v[h] = s & 1u ? acc[h][2 * i + 1] : acc[h][2 * i];
+            for (int h = 0; h < H; ++h) {
+              float even, odd;
+              f2_unpack(acc[h][i], even, odd);
+              v[h] = s & 1u ? odd : even;
+            }
             if constexpr (H % 4 == 0) {
 #pragma unroll
               for (int h = 0; h < H; h += 4) *(float4*)(out + 8 * i * H + h) = make_float4(v[h], v[h + 1], v[h + 2], v[h + 3]);

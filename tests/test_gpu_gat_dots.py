@@ -76,3 +76,29 @@ def test_ids_that_have_changed_since_the_forward():
         ids.data.copy_(kept)
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(layer(), leaves, grad), want))
     ops.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,D", [(2, 128), (1, 256)])
+def test_dots_are_rounded_sums(dtype, H, D):
+    """Two sources of a destination whose rows have the same dot with its gradient, the same products in another order, and the same score: half of each
+    weight, and gradients of the scores that are a quarter of what the two computed dots differ by."""
+    dst = 3000
+    g = torch.Generator(device="cuda").manual_seed(D)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(dtype)      # noqa: E731
+    pairs = torch.randperm(D, generator=g, device="cuda").view(2, D // 2)
+    swap = torch.empty(D, dtype=torch.int64, device="cuda")
+    swap[pairs[0]], swap[pairs[1]] = pairs[1], pairs[0]
+    grad = normal(dst, H, D)
+    grad[..., pairs[1]] = grad[..., pairs[0]]
+    ft = torch.empty(2 * dst, H, D, dtype=dtype, device="cuda")
+    ft[::2] = normal(dst, H, D)
+    ft[1::2] = ft[::2][..., swap]
+    col = torch.arange(dst, device="cuda").repeat_interleave(2)
+    el, er = torch.ones(2 * dst, H, 1, dtype=dtype, device="cuda"), torch.ones(dst, H, 1, dtype=dtype, device="cuda")
+    got = ops.gat_edge_softmax_sum_backward(torch.arange(2 * dst, device="cuda"), col, ft, el, er, grad, 0.2)[1].double()
+    dots = (ft[::2].double() * grad.double()).sum(-1)
+    # An fp32 value is off by 2^-24 / sqrt(3) of the largest it may be, at 0.7 of that in the mean, wherever it is rounded: eight times from product to
+    # sum, down a tree, by less every time, less than three such steps together, and once more for the mean of the two.
+    error = 4 * got.norm() / 2 ** 0.5 / 2 ** 0.5 / dots.norm()
+    assert error <= 2.0 ** -23, float(error)
