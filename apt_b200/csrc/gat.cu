@@ -684,7 +684,7 @@ static int gat_dots(const GatProblem& q, const GatEdges& g, const GatBwdWs& ws, 
   const int64_t dim = q.H * q.Dh;
   const int slice = slice_elems((uint64_t)(q.Dh * sizeof(T)) | (uintptr_t)q.ft | (uintptr_t)q.grad_out, sizeof(T)) * (int)sizeof(T);
   if constexpr (sizeof(T) == 2)
-    if (dots_mma_fits(q.H, q.Dh, slice, q.E))
+    if (dots_mma_fits<T>(q.H, q.Dh, slice, q.E, q.num_dst))
       return launch_dots_mma<T>(q.H, q.Dh, q.row, q.col, (const T*)q.ft, (const T*)q.grad_out, q.E, q.num_dst, g.none, ws.dots, (uint32_t)num_src, ws.sort, s);
   if (stream_fits(kDots, slice, dim, sizeof(T), q.H, q.E, true)) {
     SpmmWs counts = ws.sort;

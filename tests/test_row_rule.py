@@ -55,3 +55,31 @@ def test_long_rows_keep_their_edges_side_by_side(split, dim, ve):
 
 def test_few_rows_take_as_many_edges_as_go(split):
     assert split((16, 4, 500 * 15, 500, 1), (16, 4, 500 * 15, 500, 0), (16, 4, 500 * 100, 500, 1)) == [(4, 4), (4, 4), (4, 8)]
+
+
+DOTS = r"""
+#include <cstdio>
+#include "gat_dots.cuh"
+int main() {
+  int bf16, heads, dim, slice;
+  long long edges, dst;
+  while (scanf("%d %d %d %d %lld %lld", &bf16, &heads, &dim, &slice, &edges, &dst) == 6)
+    printf("%d\n", (int)(bf16 ? apt::dots_mma_fits<__nv_bfloat16>(heads, dim, slice, edges, dst) : apt::dots_mma_fits<__half>(heads, dim, slice, edges, dst)));
+}
+"""
+
+
+def test_dots_of_blocks_whose_destinations_are_sparse(tmp_path):
+    """Wide rows of many edges with few edges to a destination go to the kernel that fetches the gradient's rows in use alone."""
+    if not os.path.exists(NVCC):
+        pytest.skip("needs nvcc")
+    (tmp_path / "dots.cu").write_text(DOTS)
+    subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "--expt-relaxed-constexpr", "-I", CSRC, str(tmp_path / "dots.cu"),
+                    "-o", str(tmp_path / "dots"), "-cudart", "shared", "-Xlinker", "--unresolved-symbols=ignore-all"], check=True)
+    ask = lambda *q: [int(v) for v in subprocess.run([str(tmp_path / "dots")], input="\n".join(" ".join(map(str, x)) for x in q), capture_output=True,      # noqa: E731
+                                                     text=True, check=True).stdout.split()]
+    wide = [(b, h, d, 16, e, n) for b, h, d in ((1, 4, 64), (1, 1, 256), (0, 8, 32)) for e, n in
+            ((1_000_000, 66_666), (1_000_000, 200_000), (1_000_000, 200_001), (1_000_000, 500_000), (1_000_000, 500_001), (393_215, 400_000))]
+    assert ask(*wide) == [1, 1, 0, 0, 0, 1] * 2 + [1, 1, 1, 1, 0, 1]
+    # narrow rows, heads that are no power of two, rows that are no whole slices
+    assert ask((1, 4, 32, 16, 1_000_000, 900_000), (1, 3, 64, 16, 1_000_000, 60_000), (1, 4, 48, 16, 1_000_000, 60_000), (1, 4, 64, 8, 1_000_000, 60_000)) == [1, 0, 0, 0]
