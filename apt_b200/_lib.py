@@ -75,6 +75,7 @@ PROTOTYPES = {
     "apt_spmm_workspace_bytes": (c_size_t, [c_int64, c_int64]),
     "apt_spmm_sum": (c_int, [c_int, c_int, P, P, c_int64, P, P, c_int64, c_int64, P, P, P, c_int, c_int64, P, P, c_size_t, P]),
     "apt_spmm_probe": (c_int, [P, c_int64, P, P, c_int, P, P]),
+    "apt_spmm_probe_rows": (c_int, [P, c_int64, P, P, c_int, c_int, P, P]),
     "apt_spmm_sum_known": (c_int, [c_int, c_int, P, P, c_int64, P, P, c_int64, c_int64, P, P, P, c_int, c_int64, c_int, c_int,
                                    P, P, c_size_t, P]),
     "apt_spmm_widened_bytes": (c_size_t, [c_int, c_int64, c_int64, c_int64, c_int]),

@@ -70,27 +70,33 @@ __device__ __forceinline__ int64_t out_row(const int64_t* coo, const int64_t* oo
   return ooff[nseg > 1 ? seg_of(coo, nseg, e) : 0] + col[e];
 }
 
-// One 64-bit word collects the blocks' answers: blocks done, and how many of them saw each of the three. The add that
+// One 64-bit word collects the blocks' answers: blocks done, how many of them saw each of the three (10 bits each), and pairs of one row (24). The add that
 // counts a block also returns what the others saw, so the last block has the answer without a fence or a second
 // read (fence, counter and read in turn: 5.6 -> 4.5 us for 10 240 edges). The word, `agg` or the slot's own, is zero before
 // and after; `result` may be mapped host memory.
 constexpr int kProbeSlots = 64;
+constexpr unsigned long long kVoteMask = 1023, kMostPairs = 16383;      // pairs a block adds at most
+static_assert(kNumSMs * 4 < (int)kVoteMask && (unsigned long long)kNumSMs * 4 * kMostPairs < 1ull << 24, "votes of a wave of four blocks an SM");
 __device__ unsigned long long g_probe_votes[kProbeSlots];
-__device__ __forceinline__ unsigned long long probe_votes(uint32_t bits) {
-  return 1ull | (bits & kNotGrouped ? 1ull << 16 : 0ull) | (bits & kNotFixed ? 1ull << 32 : 0ull) |
-         (bits & kHasLong ? 1ull << 48 : 0ull);
+__device__ __forceinline__ unsigned long long probe_votes(uint32_t bits, uint32_t pairs) {
+  return 1ull | (bits & kNotGrouped ? 1ull << 10 : 0ull) | (bits & kNotFixed ? 1ull << 20 : 0ull) | (bits & kHasLong ? 1ull << 30 : 0ull) |
+         min((unsigned long long)pairs, kMostPairs) << 40;
 }
 
+// Rows with many of the edges (`count_pairs`): of edges in no order, how many of the pairs that a warp's 32 edges make are of one row, in a quarter
+// of those it holds first. All rows alike, that is one pair in as many as there are rows; kHubs times as many, and rows of far more edges than
+// the mean take part (the source of a draw at u^1.5 of the range 1.4 times, at u^2 3.2, at u^3 25 and more). A million edges are 4.7 million pairs.
+constexpr int kHubs = 2, kPairShare = 4;      // of the rounds that a thread has on their way
 // num_rows: the output rows there are (the caller's result may have more, or fewer, than the offsets end at); -1: as the offsets say.
 // K edges a thread at a time: four, eight where more than one wave of four would be needed (1.01 M edges 8.1 -> 7 us).
 template <int K>
 __global__ void __launch_bounds__(256)
 k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t num_rows, unsigned long long* agg, int slot,
-             volatile int64_t* result, int64_t sequence) {
+             volatile int64_t* result, int64_t sequence, int count_pairs) {
   wait_for_previous();
   if (!agg) agg = g_probe_votes + slot;
   __shared__ int64_t coo[kMaxSegments + 1], ooff[kMaxSegments + 1];
-  __shared__ uint32_t s_bits;
+  __shared__ uint32_t s_bits, s_pairs;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, c[K];
   auto fetch = [&]() {
@@ -102,8 +108,21 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
     coo[t] = st.coo_off[t];
     ooff[t] = st.out_off[t];
   }
-  if (threadIdx.x == 0) s_bits = 0u;
+  if (threadIdx.x == 0) s_bits = s_pairs = 0u;
   __syncthreads();
+  if (count_pairs) {
+    uint32_t pairs = 0u;      // each of them twice
+#pragma unroll
+    for (int k = 0; k < K / kPairShare; ++k) {
+      const bool there = e0 + k * stride < E;
+      const unsigned all = __ballot_sync(0xffffffffu, there);
+      // (edges that do not fall are likely to be grouped, which asks for no pairs)
+      const int64_t before = __shfl_up_sync(0xffffffffu, c[k], 1);
+      if (__any_sync(0xffffffffu, there && (threadIdx.x & 31) && c[k] < before) && there) pairs += __popc(__match_any_sync(all, (unsigned)c[k])) - 1;
+    }
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&s_pairs, pairs / 2);
+  }
   const int64_t rows = num_rows >= 0 ? num_rows : ooff[st.nseg];
   // the one fanout that fits the sizes
   const uint32_t f = rows > 0 && E % rows == 0 ? (uint32_t)(E / rows) : 0u;
@@ -132,26 +151,29 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
   if ((threadIdx.x & 31) == 0 && bits) atomicOr(&s_bits, bits);
   __syncthreads();
   if (threadIdx.x != 0) return;
-  unsigned long long all = probe_votes(s_bits);
+  unsigned long long all = probe_votes(s_bits, s_pairs);
   if (gridDim.x > 1) {
     all += atomicAdd(agg, all);
-    if ((all & 0xffffu) != gridDim.x) return;
+    if ((all & kVoteMask) != gridDim.x) return;
     atomicExch(agg, 0ull);
   }
-  const bool fixed = !(all >> 32 & 0xffffu), grouped = !(all >> 16 & 0xffffu), has_long = (all >> 48) != 0;
+  const bool fixed = !(all >> 20 & kVoteMask), grouped = !(all >> 10 & kVoteMask), has_long = (all >> 30 & kVoteMask) != 0;
   const bool fits = rows >= 0 && rows < 0x7fffffff;
-  *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, sequence);
+  // 32 edges make 496 pairs; a warp's are of one segment, whose rows are taken to be as many as the others'
+  const int64_t looked_at = min(E, (int64_t)gridDim.x * 256 * (K / kPairShare));
+  const bool hubs = fits && (int64_t)(all >> 40) * 2 * (rows / st.nseg) >= looked_at * 31 * kHubs;
+  *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, hubs, sequence);
 }
 
 static int launch_probe(const int64_t* col, int64_t E, SegTable st, int64_t num_rows, unsigned long long* agg, int slot,
-                        int64_t* result, int64_t sequence, cudaStream_t s) {
+                        int64_t* result, int64_t sequence, bool count_pairs, cudaStream_t s) {
   // a thousand edges a block and one wave at most: small blocks of edges are looked over by one thread block
   const int grid = wave_grid(ceil_div(E, 1024), 4, 1);
   ProfScope prof("spmm_ranges", s);
   if (E > (int64_t)grid * 256 * 4)
-    APT_FOLLOW(k_spmm_probe<8>, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence);
+    APT_FOLLOW(k_spmm_probe<8>, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence, (int)count_pairs);
   else
-    APT_FOLLOW(k_spmm_probe<4>, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence);
+    APT_FOLLOW(k_spmm_probe<4>, grid, 256, 0, s, col, E, st, num_rows, agg, slot, (volatile int64_t*)result, sequence, (int)count_pairs);
   return APT_OK;
 }
 
@@ -178,7 +200,7 @@ static int take_slot(int* slot, int64_t* sequence) {
   g_probe.cv.wait(lk, [] { return g_probe.taken != ~0ull; });
   *slot = __builtin_ctzll(~g_probe.taken);
   g_probe.taken |= 1ull << *slot;
-  *sequence = ++g_probe.sequence & 0x7fffffff;
+  *sequence = ++g_probe.sequence & kProbeSequences;
   return APT_OK;
 }
 
@@ -650,7 +672,7 @@ static int spmm_run(int op, int dtype, const int64_t* coo_row, const int64_t* co
   const RowSplit split = row_split(feat_dim, slice_elems(bits, (int)esz), E, num_rows, mode == kOrder || mode == kDevice);
   if (mode == kDevice || mode == kOrder) APT_CUDA(cudaMemsetAsync(workspace, 0, ws.zero_bytes, s));
   if (mode == kDevice) {
-    const int rc = launch_probe(coo_col, E, st, num_rows, ws.probe, 0, ws.result, 1, s);
+    const int rc = launch_probe(coo_col, E, st, num_rows, ws.probe, 0, ws.result, 1, false, s);
     if (rc != APT_OK) return rc;
   }
   if (mode == kDevice || mode == kRanges) {
@@ -697,7 +719,18 @@ extern "C" size_t apt_spmm_workspace_bytes(int64_t num_out_rows, int64_t num_edg
 extern "C" int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges, const int64_t* coo_offset,
                               const int64_t* output_offset, int num_segments, int64_t* out_rows_mode_fixed,
                               void* stream) {
+  int64_t answer[4];
+  const int rc = apt_spmm_probe_rows(coo_col, num_edges, coo_offset, output_offset, num_segments, 0, out_rows_mode_fixed ? answer : nullptr, stream);
+  if (rc == APT_OK)
+    for (int k = 0; k < 3; ++k) out_rows_mode_fixed[k] = answer[k];
+  return rc;
+}
+
+extern "C" int apt_spmm_probe_rows(const int64_t* coo_col, int64_t num_edges, const int64_t* coo_offset,
+                                   const int64_t* output_offset, int num_segments, int want_hubs, int64_t* out_rows_mode_fixed_hubs,
+                                   void* stream) {
   using namespace apt;
+  int64_t* const out_rows_mode_fixed = out_rows_mode_fixed_hubs;
   APT_CHECK_ARG(num_segments >= 1 && num_segments <= kMaxSegments, "apt_spmm_probe: %d segments outside [1,%d]",
                 num_segments, kMaxSegments);
   APT_CHECK_ARG(num_edges >= 0 && num_edges < (int64_t)0x7fffffff, "apt_spmm_probe: bad num_edges");
@@ -716,13 +749,14 @@ extern "C" int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges, const i
   if (rc != APT_OK) return rc;
   int64_t* host = g_probe.host + slot * 8;
   SegTable st{coo_offset, nullptr, output_offset, num_segments};
-  rc = launch_probe(coo_col, num_edges, st, -1, nullptr, slot, host, sequence, s);
+  rc = launch_probe(coo_col, num_edges, st, -1, nullptr, slot, host, sequence, want_hubs != 0, s);
   if (rc == APT_OK) rc = wait_for(host, sequence, s);
   if (rc == APT_OK) {
     const int64_t w = *(volatile int64_t*)host, rows = probe_rows(w);
     out_rows_mode_fixed[0] = rows;
     out_rows_mode_fixed[1] = probe_mode(w);
     out_rows_mode_fixed[2] = probe_mode(w) == kFixed && rows > 0 ? num_edges / rows : 0;
+    out_rows_mode_fixed[3] = probe_mode(w) == kOrder && (probe_hubs(w) || (want_hubs && num_edges / kHubMean >= rows));
     if (probe_mode(w) == 3) {
       set_error("apt_spmm_probe: the number of output rows is negative or above 2^31");
       rc = APT_ERR_BAD_ARG;
@@ -763,9 +797,9 @@ extern "C" int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row, con
 
 extern "C" size_t apt_spmm_widened_bytes(int dtype, int64_t num_edges, int64_t num_input_rows, int64_t feat_dim, int mode) {
   using namespace apt;
-  if (dtype < APT_F32 || dtype > APT_F16 || num_edges < 0 || feat_dim <= 0 || mode < kFixed || mode > kOrder) return 0;
+  if (dtype < APT_F32 || dtype > APT_F16 || num_edges < 0 || feat_dim <= 0 || mode < kFixed || mode > kOrderEven) return 0;
   const size_t esz = elem_size(dtype);
-  return widen_pays(feat_dim, esz, num_input_rows, num_edges, mode != kOrder) ? (size_t)num_input_rows * widened_dim(feat_dim, esz) * esz : 0;
+  return widen_pays(feat_dim, esz, num_input_rows, num_edges, mode) ? (size_t)num_input_rows * widened_dim(feat_dim, esz) * esz : 0;
 }
 
 extern "C" int apt_spmm_copy_u_widened(int dtype, const int64_t* coo_row, const int64_t* coo_col, int64_t num_edges, const void* input,
@@ -775,6 +809,7 @@ extern "C" int apt_spmm_copy_u_widened(int dtype, const int64_t* coo_row, const 
                                        void* workspace, size_t workspace_bytes, void* stream) {
   using namespace apt;
   const size_t need = apt_spmm_widened_bytes(dtype, num_edges, num_input_rows, feat_dim, mode);
+  if (mode == kOrderEven) mode = kOrder;
   if (need == 0 || num_out_rows <= 0 || !input)
     return apt_spmm_sum_known(kCopyU, dtype, coo_row, coo_col, num_edges, input, nullptr, feat_dim, feat_dim, coo_offset, input_offset,
                               output_offset, num_segments, num_out_rows, mode, fixed, out, workspace, workspace_bytes, stream);

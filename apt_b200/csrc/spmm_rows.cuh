@@ -54,14 +54,16 @@ struct SegTable {
   int nseg;
 };
 
-// The probe's answer in one word, so that a single store delivers it to the host: rows (31 bits), mode (2), sequence (31).
-// Rows that do not fit (or are negative) answer mode 3.
-__host__ __device__ inline int64_t probe_pack(int64_t rows, int mode, int64_t sequence) {
-  return (sequence << 33) | ((int64_t)mode << 31) | rows;
+// The probe's answer in one word, so that a single store delivers it to the host: rows (31 bits), mode (2), whether a few rows have many of the edges (1),
+// sequence (30). Rows that do not fit (or are negative) answer mode 3.
+__host__ __device__ inline int64_t probe_pack(int64_t rows, int mode, bool hubs, int64_t sequence) {
+  return (sequence << 34) | ((int64_t)hubs << 33) | ((int64_t)mode << 31) | rows;
 }
 __host__ __device__ inline int64_t probe_rows(int64_t w) { return w & 0x7fffffff; }
 __host__ __device__ inline int probe_mode(int64_t w) { return (int)(w >> 31) & 3; }
-__host__ __device__ inline int64_t probe_sequence(int64_t w) { return (int64_t)((uint64_t)w >> 33); }
+__host__ __device__ inline bool probe_hubs(int64_t w) { return w >> 33 & 1; }
+__host__ __device__ inline int64_t probe_sequence(int64_t w) { return (int64_t)((uint64_t)w >> 34); }
+constexpr int64_t kProbeSequences = (1 << 30) - 1;
 
 struct SpmmWs {
   // zero when a call starts that groups edges or asks the device for the mode

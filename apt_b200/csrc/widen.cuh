@@ -8,28 +8,33 @@
 namespace apt {
 
 // When a sum has its input widened. The copy reads and writes every input row once (5.6 TB/s: 67 000 x 404 B 11 us, 469 000 x 404 B 69) and a call with
-// one more buffer and launch takes the host 3 us longer; the gain is per edge, the larger the narrower the accesses are otherwise, and larger
-// behind the sort, where a row's edges are walked from a list. us of a call, rows as they are -> widened:
-//   in no order, 1 005 000 edges from 67 000 rows into 168 000   bf16 x 17 103 -> 86, x 61 122 -> 99, x 101 154 -> 119, x 251 292 -> 170; x 34 107 -> 95, x 198
-//     179 -> 169; fp32 x 31 108 -> 95, x 101 161 -> 133, x 251 368 -> 183, x 198 245 -> 170
-//   240 000 edges from 20 000 into 44 000   bf16 x 31 55 -> 51, x 101 78 -> 61, x 251 121 -> 70, x 198 78 -> 71; fp32 x 31 55 -> 53, x 101 78 -> 59, x 198 82 -> 70
-//   where it does not pay: bf16 x 9 87 -> 85 and 47 -> 48; accesses of 8 bytes, bf16 x 140 138 -> 155, x 36 91 -> 94; of 4, fp32 x 34 106 -> 112, bf16 x 102
-//     67 -> 68; 96 000 edges, fp32 x 101 into 94 000 rows 61 -> 68 (k_spmm_stream takes no less than 98 304)
+// one more buffer and launch takes the host 3 us longer; the gain is per edge, and in no order it lies with the rows of very many edges, whose items
+// are walked by single warps at the pace of the narrow accesses, where k_spmm_stream cuts them anywhere. us of a call, rows as they are -> widened:
+//   in no order, some rows with many of the edges (sources drawn at u^2 of the range, 10 edges a row)   1 000 000 edges from 125 000 rows bf16 x 17 .91 of the
+//     time, x 61 .83, x 251 .45, x 198 .81; fp32 x 101 .76, x 137 .51; 99 000 from 12 000 bf16 x 61 .88, x 251 .55, fp32 x 101 .73, x 251 .56
+//     where it does not pay   99 000 edges bf16 x 17 1.09, x 34 1.07, fp32 x 31 1.08 (400 000 .99; from 133 000 rows 1 000 000 1.09); rows beyond the 1024 bytes of
+//     k_spmm_stream, fp32 x 602 from 8 edges a row 1.06, from 60 .94; accesses of 8 bytes, bf16 x 140 1.12, x 36 1.03; 70 000 edges, fp32 x 251 1.1
+//   in no order, all rows alike   99 000 edges bf16 x 251 1.10, fp32 x 101 1.24, bf16 x 198 1.32; 1 000 000 bf16 x 251 .78, fp32 x 137 .82, x 251 .88, but bf16 x 101 .94 -
+//     1.04, x 198 1.12, fp32 x 101 1.03, and from three edges a row fp32 x 251 1.13
 //   grouped, 1 005 000 edges from 168 000 rows   bf16 x 17 40 -> 32, x 61 51 -> 41, x 251 139 -> 97; x 140 69 -> 83, fp32 x 101 76 -> 83; from 368 000
 //     bf16 x 61 51 -> 54, x 101 79 -> 86; 240 000 edges from 44 000 bf16 x 61 22 -> 23, x 251 37 -> 35
 constexpr int kWidenLeast = 34, kWidenMost = 4096;      // bytes of a row
-constexpr int64_t kWidenEdges = 3 << 15, kWidenGrouped = 3 << 17;
+constexpr int64_t kWidenEdges = 3 << 15, kWidenGrouped = 3 << 17, kWidenEven = 15 << 16;
+constexpr int64_t kHubMean = 256;      // a mean row that is as good as some of very many edges
+constexpr int kOrderEven = 3;          // kOrder without such rows
 
 // Elements of a row of `dim` in whole slices.
 inline int64_t widened_dim(int64_t dim, size_t esz) { return (dim * (int64_t)esz + 15) / 16 * (16 / (int64_t)esz); }
 
-inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num_edges, bool grouped) {
-  const int64_t row = dim * (int64_t)esz;
+inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num_edges, int mode) {
+  const int64_t row = dim * (int64_t)esz, wide = widened_dim(dim, esz) * (int64_t)esz;
   const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
   if (slice == 16 || row < kWidenLeast || row > kWidenMost || num_in_rows <= 0) return false;
-  if (grouped) return slice == 2 && num_edges >= kWidenGrouped && num_edges / 4 >= num_in_rows;
-  if (num_edges < kWidenEdges || num_edges / 3 < num_in_rows) return false;
-  return slice == 2 || row >= (slice == 4 ? 384 : 768) || (slice == 4 && row >= 64 && row <= 128 && num_edges >= 2 * kWidenEdges);
+  if (mode < 2) return slice == 2 && num_edges >= kWidenGrouped && num_edges / 4 >= num_in_rows;      // (grouped)
+  if (mode == kOrderEven) return slice == (int)esz && row >= 480 && wide <= 1024 && num_edges >= kWidenEven && num_edges / 8 >= num_in_rows;
+  if (num_edges < kWidenEdges || num_edges / (wide > 1024 ? 16 : slice == (int)esz ? 3 : 4) < num_in_rows) return false;
+  if (row <= 128 && (slice == 4 || row <= 64)) return slice <= 4 && num_edges >= 2 * kWidenEdges && (slice == 2 || (row >= 64 && num_edges / 6 >= num_in_rows));
+  return slice == 2 || row >= (slice == 4 ? 384 : 768);
 }
 
 // The same for the attention layer, whose rows are widened head by head: in the forward the sources' (num_dst 0), in the backward both sides', for

@@ -92,12 +92,13 @@ Tensor spmm(int op, const Tensor& coo_row, const Tensor& coo_col, const OptTenso
   const int64_t per_edge = edata ? ed.numel() / std::max<int64_t>(edges, 1) : 0;
   const int64_t dim = input ? in.size(1) : per_edge;
   const int64_t edim = edata && edges ? per_edge : dim;
-  int64_t shape[3] = {0, -1, 0};
+  int64_t shape[4] = {0, -1, 0, 0};
   if (ooff.numel() > eoff.numel()) {
     shape[0] = ooff[-1].item<int64_t>();        // further rows behind the last segment's: the block is looked over with them
   } else {
     py::gil_scoped_release nogil;   // other threads run while this one waits for the stream
-    check(apt_spmm_probe(ptr(col), edges, ptr(eoff), ptr(ooff), (int)eoff.numel() - 1, shape, stream()));
+    const bool may_widen = op == 0 && input && apt_spmm_widened_bytes(code, edges, in.size(0), dim, 2) > 0;
+    check(apt_spmm_probe_rows(ptr(col), edges, ptr(eoff), ptr(ooff), (int)eoff.numel() - 1, may_widen, shape, stream()));
   }
   Tensor out = at::empty({shape[0], dim}, given.options());
   Tensor ws;
@@ -106,11 +107,12 @@ Tensor spmm(int op, const Tensor& coo_row, const Tensor& coo_col, const OptTenso
     bytes = apt_spmm_workspace_bytes(shape[0], edges);
     ws = scratch(out, bytes);
   }
-  const size_t wide_bytes = op == 0 && input && shape[0] > 0 ? apt_spmm_widened_bytes(code, edges, in.size(0), dim, (int)shape[1]) : 0;
+  const int mode = shape[1] == 2 && !shape[3] ? 3 : (int)shape[1];      // 3: in no order, and no row with very many of the edges
+  const size_t wide_bytes = op == 0 && input && shape[0] > 0 ? apt_spmm_widened_bytes(code, edges, in.size(0), dim, mode) : 0;
   const Tensor wide = room_for(out, wide_bytes);
   if (wide.defined()) {
     check(apt_spmm_copy_u_widened(code, ptr(row), ptr(col), edges, data(in), in.size(0), dim, ptr(eoff), ptr(ioff), ptr(ooff),
-                                  (int)eoff.numel() - 1, shape[0], (int)shape[1], (int)shape[2], mut(out), wide.mutable_data_ptr(),
+                                  (int)eoff.numel() - 1, shape[0], mode, (int)shape[2], mut(out), wide.mutable_data_ptr(),
                                   wide_bytes, bytes ? ws.mutable_data_ptr() : nullptr, bytes, stream()));
     return out;
   }

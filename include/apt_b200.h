@@ -408,6 +408,14 @@ int apt_spmm_probe(const int64_t* coo_col, int64_t num_edges,
                    const int64_t* coo_offset, const int64_t* output_offset,
                    int num_segments, int64_t* out_rows_mode_fixed /* host[3] */,
                    void* stream);
+/* The same; out[3] = 1 for a block of mode 2 some of whose output rows have very many of the
+ * edges, which is looked for where want_hubs is not 0. */
+int apt_spmm_probe_rows(const int64_t* coo_col, int64_t num_edges,
+                        const int64_t* coo_offset,
+                        const int64_t* output_offset, int num_segments,
+                        int want_hubs,
+                        int64_t* out_rows_mode_fixed_hubs /* host[4] */,
+                        void* stream);
 int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row,
                        const int64_t* coo_col, int64_t num_edges,
                        const void* input, const void* edata, int64_t edata_dim,
@@ -421,7 +429,8 @@ int apt_spmm_sum_known(int op, int dtype, const int64_t* coo_row,
  * whose input is copied to such a pitch first and then read a slice at a time:
  * results are the same. apt_spmm_widened_bytes is what the copy takes, or 0
  * where the sum does better without (no buffer is used then). num_input_rows:
- * rows of `input`, all segments together. */
+ * rows of `input`, all segments together. mode: as apt_spmm_probe_rows answers it,
+ * but 3 for a block of mode 2 that was found without such rows. */
 size_t apt_spmm_widened_bytes(int dtype, int64_t num_edges,
                               int64_t num_input_rows, int64_t feat_dim,
                               int mode);

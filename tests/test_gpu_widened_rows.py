@@ -133,6 +133,47 @@ def test_rows_that_stay_as_they_are():
     assert bytes_of(1, 1_000_000, 67_000, 101, 2) == 67_000 * 208
 
 
+def test_rows_that_all_have_as_many_edges_stay_as_they_are():
+    """Mode 3: in no order, and no row with very many of the edges."""
+    bytes_of = lib.apt_spmm_widened_bytes
+    assert bytes_of(1, 900_000, 67_000, 251, 3) == 0 and bytes_of(0, 400_000, 20_000, 101, 3) == 0
+    assert bytes_of(1, 1_000_000, 67_000, 101, 3) == 0 and bytes_of(1, 1_000_000, 67_000, 198, 3) == 0
+    assert bytes_of(1, 1_000_000, 200_000, 251, 3) == 0 and bytes_of(0, 1_000_000, 67_000, 602, 3) == 0
+    assert bytes_of(1, 1_000_000, 67_000, 251, 3) == 67_000 * 512 and bytes_of(0, 1_000_000, 67_000, 137, 3) == 67_000 * 560
+    # with such rows, but a copy that takes longer than it gives
+    assert bytes_of(0, 1_000_000, 300_000, 602, 2) == 0 and bytes_of(0, 150_000, 9_000, 31, 2) == 0 and bytes_of(1, 100_000, 9_000, 17, 2) == 0
+
+
+@pytest.mark.parametrize("edges", [98_304, 100_003, 606_208, 606_241, 1_500_001])
+@pytest.mark.parametrize("rows", [40, 5_003, 20_000])
+@pytest.mark.parametrize("segments", [1, 4])
+@pytest.mark.parametrize("drawn", ["alike", "u^2", "u^3", "one row", "grouped"])
+def test_rows_with_very_many_of_the_edges_are_seen(edges, rows, segments, drawn):
+    import ctypes
+
+    g = torch.Generator(device="cuda").manual_seed(edges + rows)
+    u = torch.rand(edges, generator=g, device="cuda", dtype=torch.float64)
+    col = (u.pow({"u^2": 2, "u^3": 3}.get(drawn, 1)) * rows).long().clamp_(max=rows - 1)
+    if drawn == "one row":
+        col[torch.rand(edges, generator=g, device="cuda") < 0.1] = rows // 2
+    cut = [edges * k // segments for k in range(segments + 1)]
+    if drawn == "grouped":
+        for a, b in zip(cut, cut[1:]):
+            col[a:b] = col[a:b].sort()[0]
+    off, out = torch.tensor(cut, device="cuda"), torch.arange(segments + 1, device="cuda") * rows
+    got, old = (ctypes.c_int64 * 4)(), (ctypes.c_int64 * 3)()
+    for want_hubs in (1, 0):
+        check(lib.apt_spmm_probe_rows(col.data_ptr(), edges, off.data_ptr(), out.data_ptr(), segments, want_hubs, got, None))
+        check(lib.apt_spmm_probe(col.data_ptr(), edges, off.data_ptr(), out.data_ptr(), segments, old, None))
+        assert list(got)[:3] == list(old)
+        many = drawn != "grouped" and (edges // 256 >= rows * segments or drawn in ("u^2", "u^3") or (drawn == "one row" and rows > 200))
+        if drawn == "grouped":
+            assert got[1] in (1, 2)
+        else:
+            # (what 40 rows' drawn differences come to is left open)
+            assert got[1] == 2 and (rows == 40 and drawn != "alike" or got[3] == (many and want_hubs))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("heads,head_dim", [(4, 47), (1, 47), (8, 10), (4, 10), (3, 33), (2, 255), (1, 601), (9, 18), (17, 9)])
 def test_attention_of_heads_that_are_no_whole_slices(dtype, heads, head_dim):
