@@ -166,7 +166,7 @@ def test_rows_with_very_many_of_the_edges_are_seen(edges, rows, segments, drawn)
         check(lib.apt_spmm_probe_rows(col.data_ptr(), edges, off.data_ptr(), out.data_ptr(), segments, want_hubs, got, None))
         check(lib.apt_spmm_probe(col.data_ptr(), edges, off.data_ptr(), out.data_ptr(), segments, old, None))
         assert list(got)[:3] == list(old)
-        many = drawn != "grouped" and (edges // 256 >= rows * segments or drawn in ("u^2", "u^3") or (drawn == "one row" and rows > 200))
+        many = drawn != "grouped" and (edges // 128 >= rows * segments or drawn in ("u^2", "u^3") or (drawn == "one row" and rows > 200))
         if drawn == "grouped":
             assert got[1] in (1, 2)
         else:
