@@ -47,13 +47,18 @@ inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num
 //   150 000, 25 000 sources          bf16 4 x 47 205 -> 103, fp32 4 x 47 194 -> 112; 300 000, 50 000 fp32 1 x 47 120 -> 103. Below kWidenGatBytes the host's
 //     90 us are what such a layer takes.
 //   Accesses of 8 bytes, backward alone: bf16 4 x 12 87 -> 97, fp32 8 x 10 219 -> 217
+//   Sources that few edges read: forward of 200 000 edges, 180 000 sources bf16 2 x 127 56 -> 67, 4 x 47 55 -> 61, 60 000 sources 2 x 127 .77 of the time; backward of
+//     240 000, 72 000 sources fp32 1 x 47 76 -> 83, bf16 8 x 10 96 -> 100, of 900 000, 270 000 sources fp32 1 x 47 .87; forward of 200 000 edges,
+//     18 000 sources fp32 1 x 47 21.7 -> 22.7, of 240 000, 22 000 sources .88
 constexpr int64_t kWidenGatBytes = 32 << 20;      // that the edges read
+constexpr int64_t kWidenGatMany = 1 << 19;
 inline bool widen_gat_pays(int64_t head_dim, int heads, size_t esz, int64_t num_src, int64_t num_edges, bool backward) {
   const int64_t row = head_dim * (int64_t)esz;
   const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
   if (slice > 4 || row < 16 || row * heads > kWidenMost || num_src <= 0 || num_edges < kWidenEdges || num_edges * row * heads < kWidenGatBytes) return false;
-  if (slice == 2) return num_edges >= num_src;
-  return backward ? num_edges / (row * heads >= 384 ? 1 : 2) >= num_src : row * heads >= 128 && num_edges / 4 >= num_src;
+  if (slice == 2) return num_edges / (backward ? 1 : 2) >= num_src;
+  if (!backward) return row * heads >= 128 && num_edges / 4 >= num_src && num_edges * row * heads >= kWidenGatBytes / 4 * 5;
+  return num_edges / (row * heads >= 384 ? 1 : num_edges >= kWidenGatMany ? 2 : 4) >= num_src;
 }
 
 // `out`: num_rows * ceil(row_bytes / 16) slices, 16-byte aligned. `in` is aligned to its elements of 2 or 4 bytes.

@@ -144,6 +144,14 @@ def test_rows_that_all_have_as_many_edges_stay_as_they_are():
     assert bytes_of(0, 1_000_000, 300_000, 602, 2) == 0 and bytes_of(0, 150_000, 9_000, 31, 2) == 0 and bytes_of(1, 100_000, 9_000, 17, 2) == 0
 
 
+def test_attention_over_sources_that_few_edges_read_stays_as_it_is():
+    bytes_of = lib.apt_gat_widened_bytes
+    assert bytes_of(1, 200_000, 180_000, 0, 2, 127) == 0 and bytes_of(1, 200_000, 100_000, 0, 2, 127) > 0      # forward
+    assert bytes_of(1, 200_000, 180_000, 20_000, 2, 127) > 0                                                     # backward
+    assert bytes_of(0, 240_000, 72_000, 60_000, 1, 47) == 0 and bytes_of(0, 240_000, 60_000, 60_000, 1, 47) > 0
+    assert bytes_of(0, 900_000, 270_000, 60_000, 1, 47) > 0
+
+
 @pytest.mark.parametrize("edges", [98_304, 100_003, 606_208, 606_241, 1_500_001])
 @pytest.mark.parametrize("rows", [40, 5_003, 20_000])
 @pytest.mark.parametrize("segments", [1, 4])
