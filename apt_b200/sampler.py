@@ -208,8 +208,8 @@ class _GraphReplay:
 
     @staticmethod
     def _alone():
-        """Whether this rank exchanges nothing and side streams may be used."""
-        return ops._exchange().name == "local" and not ops.STATE.profiling
+        """Whether this rank exchanges nothing."""
+        return ops._exchange().name == "local"
 
     @staticmethod
     def _leave_rows(input_nodes, rows, plan):
@@ -514,8 +514,9 @@ class MixedNeighborSampler(_GraphReplay):
         if alone:
             # one rank receives what it has; what only the caller wants (the permutation, the sizes, the inverse) is made beside the outermost
             # hop, of whose chain it was 5 us
+            side = None if st.profiling else 3      # (timed kernels run one by one)
             uniq2 = ops._unique_ids(cur, cur_n, 1, lo, hi, st.word(u_slot), "unique_np")
-            inv, perm, _ = ops._unique_inverse(cur, cur_n, 1, lo, hi, "unique_np", sizes=sizes_view, offsets=words[64:64 + ws], side=3)
+            inv, perm, _ = ops._unique_inverse(cur, cur_n, 1, lo, hi, "unique_np", sizes=sizes_view, offsets=words[64:64 + ws], side=side)
         else:
             sorted_ids, perm, sizes, offsets = ops._bucket(cur, cur_n, sizes_view, words[64:64 + ws])
             recv, recv_counts = ops._exchange().exchange_ids_enqueue(sorted_ids, sizes, offsets, recv_view)
@@ -536,8 +537,8 @@ class MixedNeighborSampler(_GraphReplay):
                 ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier", beside=True)
         uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
                                                      call if explicit else None, call_base_dev, look_up=prefetch)
-        if alone:
-            st.join(3)      # the sizes leave with the counts
+        if alone and side is not None:
+            st.join(side)      # the sizes leave with the counts
         if split == 1:
             if publish is not None:
                 publish()
@@ -798,29 +799,26 @@ class SPVirtualSampler(_GraphReplay):
             counts = words[16:16 + ws + 1]
             dst_counts = words[self._RDST:self._RDST + ws + 1]
             recv_dst = None
-            if ws == 1 and not with_dst:
-                recv, total = packed, n_word
+            send_sizes = words[self._SEND:self._SEND + k * ws]
+            recv_sizes = words[self._RECV:self._RECV + k * ws]
+            check(lib.apt_vir_send_sizes(ops._ptr(sorted_all), sorted_all.numel(), ops._ptr(all_word),
+                                         ops._ptr(unique_frontier), unique_frontier.numel(), ops._ptr(uf_word), ws, s_max,
+                                         ops._ptr(cur_n), int(with_dst), None, ops._ptr(send_sizes), ops._stream()))
+            ex = ops._exchange()
+            ex.exchange_fixed(send_sizes.view(ws, k), recv_sizes.view(ws, k))
+            ids_at = 1 if with_dst else 0
+            if ws == 1:
+                recv = packed
+                counts[0:1].copy_(send_sizes[ids_at:ids_at + 1])
+                counts[1:2].copy_(send_sizes[ids_at:ids_at + 1])
+                recv_dst = dst_sorted
+                dst_counts[0:1].copy_(send_sizes[0:1])
+                dst_counts[1:2].copy_(send_sizes[0:1])
             else:
-                send_sizes = words[self._SEND:self._SEND + k * ws]
-                recv_sizes = words[self._RECV:self._RECV + k * ws]
-                check(lib.apt_vir_send_sizes(ops._ptr(sorted_all), sorted_all.numel(), ops._ptr(all_word),
-                                             ops._ptr(unique_frontier), unique_frontier.numel(), ops._ptr(uf_word), ws, s_max,
-                                             ops._ptr(cur_n), int(with_dst), None, ops._ptr(send_sizes), ops._stream()))
-                ex = ops._exchange()
-                ex.exchange_fixed(send_sizes.view(ws, k), recv_sizes.view(ws, k))
-                ids_at = 1 if with_dst else 0
-                if ws == 1:
-                    recv = packed
-                    counts[0:1].copy_(send_sizes[ids_at:ids_at + 1])
-                    counts[1:2].copy_(send_sizes[ids_at:ids_at + 1])
-                    recv_dst = dst_sorted
-                    dst_counts[0:1].copy_(send_sizes[0:1])
-                    dst_counts[1:2].copy_(send_sizes[0:1])
-                else:
-                    if with_dst:
-                        recv_dst, _ = ex.exchange_ids_enqueue(dst_sorted, None, torch.cumsum(send_sizes[0::k], 0), dst_counts)
-                    recv, _ = ex.exchange_ids_enqueue(packed, None, torch.cumsum(send_sizes[ids_at::k], 0), counts)
-                total = counts[ws:ws + 1]
+                if with_dst:
+                    recv_dst, _ = ex.exchange_ids_enqueue(dst_sorted, None, torch.cumsum(send_sizes[0::k], 0), dst_counts)
+                recv, _ = ex.exchange_ids_enqueue(packed, None, torch.cumsum(send_sizes[ids_at::k], 0), counts)
+            total = counts[ws:ws + 1]
             vir_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
             ori_src = torch.empty(recv.numel(), dtype=torch.int64, device=dev)
             check(lib.apt_sp_unpack_frontier(ops._ptr(recv), recv.numel(), ops._ptr(total), n_total,

@@ -299,3 +299,36 @@ def test_block_columns_may_be_changed_in_place(model, with_dst, use_graph):
         block1.coo_col.fill_(-1)
         assert torch.equal(block1.src_ids, ids) and torch.equal(smp.last["unique_frontier"], ids)
     ops.check_status()
+
+
+@pytest.mark.parametrize("kind", ["np", "snp_gat", "SAGE", "GCN"])
+def test_profiled_mini_batches_run_the_kernels_of_the_others(kind):
+    from apt_b200.sampler import MixedNeighborSampler, SPGATSampler
+
+    n, indptr, indices = small_graph(scale=12, edge_factor=8)
+    reset_world()
+    install_graph(indptr, indices)
+    _world(1, 0, n)
+    seeds = dev(np.random.default_rng(4).permutation(n)[:200].astype(I64))
+    make = {"np": MixedNeighborSampler, "snp_gat": SPGATSampler}.get(kind, lambda r, f: SPVirtualSampler(r, f, model=kind))
+    got = []
+
+    def count(tag):
+        t, k = ctypes.c_double(), ctypes.c_int64()
+        lib.apt_profile_read(tag, ctypes.byref(t), ctypes.byref(k))
+        return k.value
+
+    for profiled in (False, True):
+        ops.set_sampling(key=5, call_id=0)
+        smp = make(0, [5, 4])
+        ops.profile_enable(profiled)
+        try:
+            out = smp.sample(None, seeds)
+            torch.cuda.synchronize()
+            if profiled:
+                assert count(b"bucket") == 0 and count(b"unique_sorted") == 2 and count(b"sample") + count(b"relabel") > 0
+        finally:
+            ops.profile_enable(False)
+        got.append([out[0].clone()] + [t.clone() for b in out[2] for t in (b.coo_row, b.coo_col, b.src_ids)] + [t.clone().cpu() for t in out[3:]])
+    assert len(got[0]) == len(got[1]) and all(torch.equal(a, b) for a, b in zip(*got))
+    ops.check_status()
