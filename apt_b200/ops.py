@@ -639,6 +639,8 @@ def _unique_inverse(ids, n_dev, per, id_lo, id_hi, ws_name, uniq=None, uniq_n=No
             sizes.zero_()
             offsets.zero_()
             sizes = offsets = None
+        if listed is not None and listed.numel() == 0:
+            all_out.zero_()
         with contextlib.nullcontext() if side is None else STATE.beside(side):
             check(lib.apt_unique_inverse(
                 _ptr(ids), n, _ptr(n_dev), int(per), int(id_lo), int(id_hi), _ptr(ws), ws.numel(), _ptr(inv), _ptr(uniq), n_uniq, _ptr(uniq_n),

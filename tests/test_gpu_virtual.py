@@ -332,3 +332,23 @@ def test_profiled_mini_batches_run_the_kernels_of_the_others(kind):
         got.append([out[0].clone()] + [t.clone() for b in out[2] for t in (b.coo_row, b.coo_col, b.src_ids)] + [t.clone().cpu() for t in out[3:]])
     assert len(got[0]) == len(got[1]) and all(torch.equal(a, b) for a, b in zip(*got))
     ops.check_status()
+
+
+@pytest.mark.parametrize("kind", ["np", "snp_gat", "SAGE", "GCN", "SAGE with destinations"])
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_no_seeds_behind_a_mini_batch(kind, use_graph):
+    """A batch without seeds is one without input nodes, whatever the batch before it has left in the words."""
+    from apt_b200.sampler import MixedNeighborSampler, SPGATSampler
+
+    n, indptr, indices = small_graph(scale=10, edge_factor=8)
+    reset_world()
+    install_graph(indptr, indices)
+    _world(1, 0, n)
+    make = {"np": MixedNeighborSampler, "snp_gat": SPGATSampler}.get(
+        kind, lambda r, f, **k: SPVirtualSampler(r, f, model=kind[:4].strip(), shuffle_with_dst="with" in kind, **k))
+    smp = make(0, [5, 4], use_graph=use_graph)
+    smp.sample(None, dev(np.arange(50)))
+    out = smp.sample(None, torch.empty(0, dtype=torch.int64, device="cuda"))
+    assert out[0].numel() == 0 and out[1].numel() == 0
+    assert all(b.num_src == b.num_dst == b.coo_row.numel() == b.coo_col.numel() == 0 for b in out[2])
+    ops.check_status()
