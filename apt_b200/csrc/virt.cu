@@ -131,7 +131,7 @@ k_sp_map_place_pack(const int64_t* __restrict__ nbr, const int64_t* __restrict__
 // Both sides of the hop in a world of one rank, which owns every node and sends to itself: neighbour i is of destination i / fanout, which is its
 // virtual node as well (owner 0), and every destination has neighbours, so the distinct virtual nodes are the
 // destinations in order. What bucketing, packing, unpacking and two sorted uniques over the virtual ids leave is written
-// as it is: 12 launches on three streams before (a mini-batch of 931 seeds x (25, 10), 128 columns: 187 -> 173 us with the list of the inverse).
+// as it is (a neighbour that is no node, which the sampling has flagged, stays its destination's): 12 launches on three streams before (a mini-batch of 931 seeds x (25, 10), 128 columns: 187 -> 173 us with the list of the inverse).
 struct SpOneRank {
   int64_t *sorted_vir, *packed, *vir_src, *ori_src, *dst_of;                       // [num_dst * fanout]
   int64_t *unique_vir, *arange_src, *arange_dst, *unique_dst;                      // [num_dst]
@@ -149,16 +149,10 @@ k_sp_one_rank(const int64_t* __restrict__ nbr, int64_t num_dst, const int64_t* _
   }
   for (int64_t i = first; i < n; i += stride) {
     const int64_t v = nbr[i], d = n >> 32 ? i / fanout : (int64_t)((uint32_t)i / (uint32_t)fanout);
-    const int64_t packed = d * num_total_nodes + v;
-    int64_t vir = d, ori = v;
-    if (v < 0 || v >= num_total_nodes) {      // no node (flagged by the sampling): as it would be unpacked
-      vir = packed / num_total_nodes;
-      ori = packed - vir * num_total_nodes;
-    }
     o.sorted_vir[i] = d;
-    o.packed[i] = packed;
-    o.vir_src[i] = vir;
-    o.ori_src[i] = ori;
+    o.packed[i] = d * num_total_nodes + v;
+    o.vir_src[i] = d;
+    o.ori_src[i] = v;
     o.dst_of[i] = d;
   }
   for (int64_t i = first; i < num_dst; i += stride) o.unique_vir[i] = o.arange_src[i] = o.arange_dst[i] = o.unique_dst[i] = i;

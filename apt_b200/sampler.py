@@ -718,8 +718,8 @@ class SPVirtualSampler(_GraphReplay):
     # word slots of the chained form: [0..13] hop counts, [16..48] packed ids received per peer (+ total),
     # [50] neighbours, [51] unique virtual nodes, [52] unique received neighbours, [53] unique received
     # virtual nodes, [54] destinations + neighbours, [55] input nodes, [64..96] destinations received per peer
-    # (+ total), [128..191] send sizes, [192..253] receive sizes. With one rank and no destinations sent along, the
-    # sizes are [50] and [51] and nothing is exchanged.
+    # (+ total), [128..191] send sizes, [192..253] receive sizes. With one rank and no destinations sent along,
+    # nothing is exchanged and [50] and [54] stay unused: the neighbours are the destinations times the fanout.
     _N, _UF, _US, _UD, _ALL, _IN, _RDST, _SEND, _RECV = 50, 51, 52, 53, 54, 55, 64, 128, 192
 
     def _enqueue(self, seeds: torch.Tensor, call_base_dev, publish=None):

@@ -606,7 +606,8 @@ int apt_sp_map_place_pack(const int64_t* neighbors, const int64_t* positions,
                           int64_t* out_count, void* stream);
 /* The whole hop where one rank owns every node (nothing is sent): what apt_bucket_by_owner, apt_sp_map_place_pack, apt_sp_unpack_frontier and
  * apt_unique_sorted over both sides' virtual ids leave there. out_dst_of: the inverse of the received virtual ids; the distinct
- * virtual ids of both sides and the two sides of their block's edges (out_arange_*) are 0 .. num_dst - 1. */
+ * virtual ids of both sides and the two sides of their block's edges (out_arange_*) are 0 .. num_dst - 1. A neighbour that is no node is left
+ * with its destination's virtual id. */
 int apt_sp_one_rank(const int64_t* neighbors, int64_t num_dst, const int64_t* num_dst_dev, int64_t fanout, int64_t sp_base,
                     int64_t num_total_nodes, int64_t* out_sorted_vir, int64_t* out_packed, int64_t* out_vir_src, int64_t* out_ori_src,
                     int64_t* out_dst_of, int64_t* out_unique_vir, int64_t* out_arange_src, int64_t* out_arange_dst, int64_t* out_unique_dst,

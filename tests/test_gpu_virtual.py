@@ -352,3 +352,30 @@ def test_no_seeds_behind_a_mini_batch(kind, use_graph):
     assert out[0].numel() == 0 and out[1].numel() == 0
     assert all(b.num_src == b.num_dst == b.coo_row.numel() == b.coo_col.numel() == 0 for b in out[2])
     ops.check_status()
+
+
+@pytest.mark.parametrize("num_dst,used,fanout", [(1, None, 1), (1, None, 25), (40, 0, 3), (300, 257, 7), (70_000, 69_999, 5), (20_000, None, 32)])
+@pytest.mark.parametrize("counted", [False, True])
+def test_hop_of_one_rank_by_itself(num_dst, used, fanout, counted):
+    """apt_sp_one_rank against the ids that packing, unpacking and numpy's unique give, neighbours that are no nodes among them."""
+    n_total, count = 1000, num_dst if used is None else used
+    rng = np.random.default_rng(num_dst + fanout)
+    nbr = rng.integers(0, n_total, num_dst * fanout).astype(I64)
+    odd = rng.random(len(nbr)) < 0.01
+    nbr[odd] = rng.choice([-1, n_total, n_total + 5], odd.sum())
+    long, short = ([torch.full((size,), -7, dtype=torch.int64, device="cuda") for _ in range(k)] for size, k in ((num_dst * fanout, 5), (num_dst, 4)))
+    words = torch.full((3,), -7, dtype=torch.int64, device="cuda")
+    n_dev = None if used is None else torch.tensor([used], device="cuda")
+    at = lambda t: None if t is None else t.data_ptr()      # noqa: E731
+    nbr_dev = dev(nbr)
+    check(lib.apt_sp_one_rank(at(nbr_dev), num_dst, at(n_dev), fanout, num_dst + 3, n_total, *map(at, long), *map(at, short), at(words[0:1]) if counted else None,
+                              at(words[1:2]), at(words[2:3]), torch.cuda.current_stream().cuda_stream))
+    m, own = count * fanout, np.repeat(np.arange(count), fanout)
+    sorted_vir, packed, vir_src, ori_src, dst_of = (host(t) for t in long)
+    assert words.tolist() == [m if counted else -7, count, count]
+    assert np.array_equal(sorted_vir[:m], own) and np.array_equal(vir_src[:m], own) and np.array_equal(ori_src[:m], nbr[:m])
+    assert np.array_equal(packed[:m], own * n_total + nbr[:m])
+    distinct, inverse = np.unique(vir_src[:m], return_inverse=True)
+    assert np.array_equal(distinct, np.arange(count)) and np.array_equal(dst_of[:m], inverse)
+    assert all(np.array_equal(host(t)[:count], distinct) for t in short)
+    assert all((host(t)[k:] == -7).all() for t, k in [(t, m) for t in long] + [(t, count) for t in short])
