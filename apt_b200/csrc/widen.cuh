@@ -25,13 +25,17 @@ constexpr int64_t kWidenEdges = 3 << 15, kWidenGrouped = 3 << 17, kWidenEven = 1
 constexpr int64_t kHubMean = 128;
 constexpr int kOrderEven = 3;          // kOrder without such rows
 
+// A buffer that there is no memory for is done without, but only after PyTorch's allocator has given back all that it keeps: none larger than any that the lines
+// here were measured with would be asked for (the widest rows of 1 000 000).
+constexpr int64_t kWidenCopy = (int64_t)4 << 30;
+
 // Elements of a row of `dim` in whole slices.
 inline int64_t widened_dim(int64_t dim, size_t esz) { return (dim * (int64_t)esz + 15) / 16 * (16 / (int64_t)esz); }
 
 inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num_edges, int mode) {
   const int64_t row = dim * (int64_t)esz, wide = widened_dim(dim, esz) * (int64_t)esz;
   const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
-  if (slice == 16 || row < kWidenLeast || row > kWidenMost || num_in_rows <= 0) return false;
+  if (slice == 16 || row < kWidenLeast || row > kWidenMost || num_in_rows <= 0 || num_in_rows > kWidenCopy / wide) return false;
   if (mode < 2) return slice == 2 && num_edges >= kWidenGrouped && num_edges / 4 >= num_in_rows;      // (grouped)
   if (mode == kOrderEven) return slice == (int)esz && row >= 480 && wide <= 1024 && num_edges >= kWidenEven && num_edges / 8 >= num_in_rows;
   if (num_edges < kWidenEdges || num_edges / (wide > 1024 ? 16 : slice == (int)esz ? 3 : 4) < num_in_rows) return false;
@@ -56,6 +60,7 @@ inline bool widen_gat_pays(int64_t head_dim, int heads, size_t esz, int64_t num_
   const int64_t row = head_dim * (int64_t)esz;
   const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
   if (slice > 4 || row < 16 || row * heads > kWidenMost || num_src <= 0 || num_edges < kWidenEdges || num_edges * row * heads < kWidenGatBytes) return false;
+  if (num_src > kWidenCopy / (widened_dim(head_dim, esz) * (int64_t)esz * heads)) return false;
   if (slice == 2) return num_edges / (backward ? 1 : 2) >= num_src;
   if (!backward) return row * heads >= 128 && num_edges / 4 >= num_src && num_edges * row * heads >= kWidenGatBytes / 4 * 5;
   return num_edges / (row * heads >= 384 ? 1 : num_edges >= kWidenGatMany ? 2 : 4) >= num_src;

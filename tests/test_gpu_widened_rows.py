@@ -144,6 +144,12 @@ def test_rows_that_all_have_as_many_edges_stay_as_they_are():
     assert bytes_of(0, 1_000_000, 300_000, 602, 2) == 0 and bytes_of(0, 150_000, 9_000, 31, 2) == 0 and bytes_of(1, 100_000, 9_000, 17, 2) == 0
 
 
+def test_copies_are_of_bounded_size():
+    edges = 200_000_000
+    assert lib.apt_spmm_widened_bytes(1, edges, 8_388_608, 251, 2) == 4 << 30 and lib.apt_spmm_widened_bytes(1, edges, 8_388_609, 251, 2) == 0
+    assert lib.apt_gat_widened_bytes(1, edges, 11_184_810, 0, 4, 47) > 0 and lib.apt_gat_widened_bytes(1, edges, 11_184_811, 0, 4, 47) == 0
+
+
 def test_attention_over_sources_that_few_edges_read_stays_as_it_is():
     bytes_of = lib.apt_gat_widened_bytes
     assert bytes_of(1, 200_000, 180_000, 0, 2, 127) == 0 and bytes_of(1, 200_000, 100_000, 0, 2, 127) > 0      # forward
