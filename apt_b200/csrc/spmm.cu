@@ -161,7 +161,7 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
   const bool fits = rows >= 0 && rows < 0x7fffffff;
   // 32 edges make 496 pairs; a warp's are of one segment, whose rows are taken to be as many as the others'
   const int64_t looked_at = min(E, (int64_t)gridDim.x * 256 * (K / kPairShare));
-  const bool hubs = fits && (int64_t)(all >> 40) * 2 * (rows / st.nseg) >= looked_at * 31 * kHubs;
+  const bool hubs = count_pairs && fits && (int64_t)(all >> 40) * 2 * rows >= looked_at * 31 * kHubs * st.nseg;
   *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, hubs, sequence);
 }
 
