@@ -74,7 +74,10 @@ def test_ids_that_have_changed_since_the_forward():
         torch.autograd.grad(out, leaves, grad, retain_graph=True)
         torch.cuda.synchronize()
         ids.data.copy_(kept)
-    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(layer(), leaves, grad), want))
+    # (sums over a source's edges are in no order: two roundings to 16 bits apart, and a few 2^-24 of their terms)
+    for a, b in zip(torch.autograd.grad(layer(), leaves, grad), want):
+        a, b = a.double(), b.double()
+        assert ((a - b).abs() <= 2.0 ** -7 * b.abs() + 2e-5 * b.abs().max()).all()
     ops.check_status()
 
 

@@ -218,3 +218,114 @@ def test_attention_of_heads_that_are_no_whole_slices(dtype, heads, head_dim):
         # the same terms in another order: fp32 sums a few 2^-24 of their terms apart, and then at most one rounding further
         a, b = a.double(), b.double()
         assert ((a - b).abs() <= 2 * _EPS[dtype] * b.abs() + 2e-5 * b.abs().max()).all()
+
+
+# ---- every edge once: whole numbers whose sums are exact in fp32, so that one edge more or less shows
+def _whole(shape, dtype, g, most):
+    return torch.randint(-most, most + 1, shape, generator=g, device="cuda").to(dtype)
+
+
+@pytest.mark.parametrize("dtype,dim", [(torch.float32, 31), (torch.float32, 101), (torch.bfloat16, 17), (torch.bfloat16, 61), (torch.float16, 251), (torch.float32, 251),
+                                       (torch.float16, 601)])
+@pytest.mark.parametrize("edges", [240_088, 1_000_003])
+def test_every_edge_of_a_shared_row_counts_once(dtype, dim, edges):
+    dst, src = 30_011, 9_001
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    row, col = torch.randint(0, src, (edges,), generator=g, device="cuda"), torch.randint(0, dst, (edges,), generator=g, device="cuda")
+    hub = torch.rand(edges, generator=g, device="cuda")
+    col[hub < 0.2], col[(hub > 0.2) & (hub < 0.21)] = 5, 29_000
+    x = _whole((src, dim), dtype, g, 9)
+    off = lambda n: torch.tensor([0, n], device="cuda")      # noqa: E731
+    got = ops.spmm_copy_u_sum(row, col, x, off(edges), off(src), off(dst))
+    want = torch.zeros(dst, dim, dtype=torch.float64, device="cuda").index_add_(0, col, x[row].double())
+    assert want.abs().max() < 2 ** 24 and torch.equal(got, want.float().to(dtype))      # (one rounding to the result's type)
+
+
+@pytest.mark.parametrize("heads,head_dim", [(4, 47), (1, 33), (8, 17), (1, 31), (4, 63), (2, 127)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_every_edge_of_a_shared_source_counts_once(dtype, heads, head_dim):
+    """Equal scores and 16 edges to a destination: weights of 1/16, which whole numbers keep exact."""
+    dst, src, per = 30_011, 20_001, 16
+    row, col, g = _block(dst, src, per, True, head_dim)
+    hub = torch.rand(dst * per, generator=g, device="cuda")
+    row[hub < 0.2], row[(hub > 0.2) & (hub < 0.21)] = 7, 19_000
+    ft, grad = _whole((src, heads, head_dim), dtype, g, 9), _whole((dst, heads, head_dim), dtype, g, 9)
+    el, er = torch.ones(src, heads, 1, dtype=dtype, device="cuda"), torch.ones(dst, heads, 1, dtype=dtype, device="cuda")
+    leaves = [t.requires_grad_() for t in (ft, el, er)]
+    out = ops.GATEdgeSoftmaxSum.apply(row, col, *leaves, dst, 0.2)
+    got = torch.autograd.grad(out, leaves, grad)[0]
+    zeros = lambda n: torch.zeros(n, heads, head_dim, dtype=torch.float64, device="cuda")      # noqa: E731
+    want = zeros(src).index_add(0, row, grad.double()[col] / 16)
+    assert want.abs().max() < 2 ** 20 and torch.equal(got, want.float().to(dtype))
+    assert torch.equal(out.detach(), (zeros(dst).index_add(0, col, ft.detach().double()[row]) / 16).float().to(dtype))
+
+
+@pytest.mark.parametrize("heads,head_dim", [(1, 31), (4, 31), (2, 63), (4, 63), (2, 127)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_widened_heads_that_the_tensor_cores_take(dtype, heads, head_dim):
+    """Heads whose widened rows are those of k_gat_dots_mma, against the same with a column of zeros."""
+    per, src = 15, 30_001
+    dst = max((32 << 20) // (per * heads * head_dim * 2), 98_304 // per) + 101      # the bytes and the edges from which on rows are widened
+    row, col, g = _block(dst, src, per, True, head_dim)
+    code = {torch.bfloat16: 1, torch.float16: 2}[dtype]
+    assert lib.apt_gat_widened_bytes(code, dst * per, src, dst, heads, head_dim) > 0
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(dtype)      # noqa: E731
+    ft, el, er, grad = normal(src, heads, head_dim), normal(src, heads, 1), normal(dst, heads, 1), normal(dst, heads, head_dim)
+    pad = lambda x: torch.nn.functional.pad(x, (0, 1)).contiguous()      # noqa: E731
+
+    def gradients(ft, grad):
+        leaves = [t.detach().requires_grad_() for t in (ft, el, er)]
+        return torch.autograd.grad(ops.GATEdgeSoftmaxSum.apply(row, col, *leaves, dst, 0.2), leaves, grad)
+
+    for k, (a, b) in enumerate(zip(gradients(ft, grad), gradients(pad(ft), pad(grad)))):
+        a, b = a.double(), b[..., :head_dim].double() if k == 0 else b.double()
+        # the same products; sums in no order (sources) a few 2^-24 of their terms apart, and a rounding further
+        assert ((a - b).abs() <= 2 * _EPS[dtype] * b.abs() + 2e-5 * b.abs().max()).all(), k
+
+
+def test_widened_attention_in_a_captured_graph():
+    dst, src, per, heads, head_dim = 20_003, 30_001, 15, 4, 47
+    row, col, g = _block(dst, src, per, True, 3)
+    ft, grad = (_whole((n, heads, head_dim), torch.bfloat16, g, 3) for n in (src, dst))
+    el, er = (torch.randn(n, heads, 1, generator=g, device="cuda").bfloat16() for n in (src, dst))
+    assert lib.apt_gat_widened_bytes(1, dst * per, src, 0, heads, head_dim) > 0
+
+    def layer():
+        out = ops.gat_edge_softmax_sum(row, col, ft, el, er, dst)
+        return (out,) + tuple(ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, grad, 0.2))
+
+    want = [t.double() for t in layer()]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        layer()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = layer()
+    for fill in (0.0, float("nan")):      # what the results held before is not part of them
+        for t in got:
+            t.fill_(fill)
+        graph.replay()
+        for a, b in zip(got, want):
+            assert ((a.double() - b).abs() <= 2 * _EPS[torch.bfloat16] * b.abs() + 2e-5 * b.abs().max()).all()
+
+
+def test_sums_without_room_for_the_copy():
+    dst, src, edges, dim = 10_007, 500_003, 1_700_003, 251
+    g = torch.Generator(device="cuda").manual_seed(2)
+    row, col = torch.randint(0, src, (edges,), generator=g, device="cuda"), torch.randint(0, dst, (edges,), generator=g, device="cuda")
+    x = _whole((src, dim), torch.bfloat16, g, 3)
+    off = [torch.tensor([0, n], device="cuda") for n in (edges, src, dst)]
+    need = lib.apt_spmm_widened_bytes(1, edges, src, dim, 2)
+    assert need >= src * 512
+    want = ops.spmm_copy_u_sum(row, col, x, *off)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total, before = torch.cuda.get_device_properties(0).total_memory, torch.cuda.memory_stats().get("num_ooms", 0)
+    kept = torch.cuda.memory_reserved()
+    torch.cuda.set_per_process_memory_fraction((kept + need * 3 // 4) / total)
+    try:
+        got = ops.spmm_copy_u_sum(row, col, x, *off)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.cuda.memory_stats().get("num_ooms", 0) > before and torch.equal(got, want)      # (whole numbers: exact in any order)
