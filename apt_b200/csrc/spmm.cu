@@ -83,10 +83,12 @@ __device__ __forceinline__ unsigned long long probe_votes(uint32_t bits, uint32_
          min((unsigned long long)pairs, kMostPairs) << 40;
 }
 
-// Rows with many of the edges (`count_pairs`): of edges in no order, how many of the pairs that a warp's 32 edges make are of one row, in a quarter
-// of those it holds first. All rows alike, that is one pair in as many as there are rows; kHubs times as many, and rows of far more edges than
-// the mean take part (the source of a draw at u^1.5 of the range 1.4 times, at u^2 3.2, at u^3 25 and more). A million edges are 4.7 million pairs.
-constexpr int kHubs = 2, kPairShare = 4;      // of the rounds that a thread has on their way
+// Rows with many of the edges (`count_pairs`): of edges in no order, how many of the pairs that a warp's first 32 edges make are of one row. All rows
+// alike, that is one pair in as many as there are rows; kHubs times as many, and rows of far more edges than
+// the mean take part (the source of a draw at u^1.5 of the range 1.4 times, at u^2 3.2, at u^3 25 and more). 100 000 edges make 390 000 pairs, 600 000 and more
+// 2.3 million. It takes a call 0.3 to 1.1 us. (Two rounds of every warp, a million edges: 12.4 us for this kernel instead of 8, the match takes its unit
+// a while.)
+constexpr int kHubs = 2;
 // num_rows: the output rows there are (the caller's result may have more, or fewer, than the offsets end at); -1: as the offsets say.
 // K edges a thread at a time: four, eight where more than one wave of four would be needed (1.01 M edges 8.1 -> 7 us).
 template <int K>
@@ -111,17 +113,14 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
   if (threadIdx.x == 0) s_bits = s_pairs = 0u;
   __syncthreads();
   if (count_pairs) {
-    uint32_t pairs = 0u;      // each of them twice
-#pragma unroll
-    for (int k = 0; k < K / kPairShare; ++k) {
-      const bool there = e0 + k * stride < E;
-      const unsigned all = __ballot_sync(0xffffffffu, there);
-      // (edges that do not fall are likely to be grouped, which asks for no pairs)
-      const int64_t before = __shfl_up_sync(0xffffffffu, c[k], 1);
-      if (__any_sync(0xffffffffu, there && (threadIdx.x & 31) && c[k] < before) && there) pairs += __popc(__match_any_sync(all, (unsigned)c[k])) - 1;
+    const bool there = e0 < E;
+    const unsigned all = __ballot_sync(0xffffffffu, there);
+    // (edges that do not fall are likely to be grouped, which asks for no pairs)
+    const int64_t before = __shfl_up_sync(0xffffffffu, c[0], 1);
+    if (__any_sync(0xffffffffu, there && (threadIdx.x & 31) && c[0] < before)) {
+      const uint32_t pairs = __reduce_add_sync(0xffffffffu, there ? __popc(__match_any_sync(all, (unsigned)c[0])) - 1 : 0);      // each of them twice
+      if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&s_pairs, pairs / 2);
     }
-    pairs = __reduce_add_sync(0xffffffffu, pairs);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&s_pairs, pairs / 2);
   }
   const int64_t rows = num_rows >= 0 ? num_rows : ooff[st.nseg];
   // the one fanout that fits the sizes
@@ -160,7 +159,7 @@ k_spmm_probe(const int64_t* __restrict__ col, int64_t E, SegTable st, int64_t nu
   const bool fixed = !(all >> 20 & kVoteMask), grouped = !(all >> 10 & kVoteMask), has_long = (all >> 30 & kVoteMask) != 0;
   const bool fits = rows >= 0 && rows < 0x7fffffff;
   // 32 edges make 496 pairs; a warp's are of one segment, whose rows are taken to be as many as the others'
-  const int64_t looked_at = min(E, (int64_t)gridDim.x * 256 * (K / kPairShare));
+  const int64_t looked_at = min(E, (int64_t)gridDim.x * 256);
   const bool hubs = count_pairs && fits && (int64_t)(all >> 40) * 2 * rows >= looked_at * 31 * kHubs * st.nseg;
   *result = probe_pack(fits ? rows : 0, !fits ? 3 : fixed ? kFixed : !grouped || has_long ? kOrder : kRanges, hubs, sequence);
 }
