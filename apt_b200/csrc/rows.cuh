@@ -100,6 +100,20 @@ struct Acc {
       for (int q = 0; q < P; ++q) p[q] = f2_add(p[q], pair_of(v, q));
     }
   }
+  __device__ __forceinline__ void add(const Acc& o) {
+#pragma unroll
+    for (int q = 0; q < P; ++q) p[q] = f2_add(p[q], o.p[q]);
+  }
+  // = v + u
+  template <typename T>
+  __device__ __forceinline__ void sum_of(const Raw<T, VE>& v, const Raw<T, VE>& u) {
+    if constexpr (VE == 1) {
+      p[0] = f2_pack(v.get(0) + u.get(0), 0.f);
+    } else {
+#pragma unroll
+      for (int q = 0; q < P; ++q) p[q] = f2_add(pair_of(v, q), pair_of(u, q));
+    }
+  }
   // += w * v
   template <typename T>
   __device__ __forceinline__ void fma(const Raw<T, VE>& v, float w) {

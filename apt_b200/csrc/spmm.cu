@@ -89,6 +89,7 @@ __device__ __forceinline__ unsigned long long probe_votes(uint32_t bits, uint32_
 // 2.3 million. It takes a call 0.3 to 1.1 us. (Two rounds of every warp, a million edges: 12.4 us for this kernel instead of 8, the match takes its unit
 // a while.)
 constexpr int kHubs = 2;
+
 // num_rows: the output rows there are (the caller's result may have more, or fewer, than the offsets end at); -1: as the offsets say.
 // K edges a thread at a time: four, eight where more than one wave of four would be needed (1.01 M edges 8.1 -> 7 us).
 template <int K>
