@@ -363,8 +363,20 @@ k_spmm_stream(const __grid_constant__ RowArgs<T> a, const __grid_constant__ Stre
           }
         };
         if (marks == 0u) {
+          if constexpr (OP == kCopyU) {
+            // in pairs: a long row is no further from 64 bits than in the items of k_spmm_rows
 #pragma unroll
-          for (int q = 0; q < 4; ++q) add(q);
+            for (int i = 0; i < VPL; ++i) {
+              Acc<VE> front, back;
+              front.sum_of(v[0][i], v[1][i]);
+              back.sum_of(v[2][i], v[3][i]);
+              front.add(back);
+              acc[i].add(front);
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) add(q);
+          }
         } else {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
