@@ -14,7 +14,8 @@ namespace apt {
 //     time, x 61 .83, x 251 .45, x 198 .81; fp32 x 101 .76, x 137 .51; 99 000 from 12 000 bf16 x 61 .88, x 251 .55, fp32 x 101 .73, x 251 .56
 //     where it does not pay   99 000 edges bf16 x 17 1.09, x 34 1.07, fp32 x 31 1.08 (400 000 .99; from 133 000 rows 1 000 000 1.09); rows beyond the 1024 bytes of
 //     k_spmm_stream, fp32 x 602 from 8 edges a row 1.06, from 60 .94; accesses of 8 bytes, bf16 x 140 1.12, x 36 1.03; 70 000 edges, fp32 x 251 1.1
-//   in no order, all rows alike   99 000 edges bf16 x 251 1.10, fp32 x 101 1.24, bf16 x 198 1.32; 1 000 000 bf16 x 251 .78, fp32 x 137 .82, x 251 .88, but bf16 x 101 .94 -
+//   in no order, all rows alike   99 000 edges bf16 x 251 1.10, fp32 x 101 1.24, bf16 x 198 1.32; 400 000 bf16 x 251 .83 - .96, fp32 x 251 1.06 - 1.19; 1 000 000 bf16 x 251
+//     .78, fp32 x 137 .82, x 251 .88, but bf16 x 101 .94 -
 //     1.04, x 198 1.12, fp32 x 101 1.03, and from three edges a row fp32 x 251 1.13
 //   grouped, 1 005 000 edges from 168 000 rows   bf16 x 17 40 -> 32, x 61 51 -> 41, x 251 139 -> 97; x 140 69 -> 83, fp32 x 101 76 -> 83; from 368 000
 //     bf16 x 61 51 -> 54, x 101 79 -> 86; 240 000 edges from 44 000 bf16 x 61 22 -> 23, x 251 37 -> 35
@@ -37,7 +38,7 @@ inline bool widen_pays(int64_t dim, size_t esz, int64_t num_in_rows, int64_t num
   const int slice = slice_elems((uint64_t)row, (int)esz) * (int)esz;
   if (slice == 16 || row < kWidenLeast || row > kWidenMost || num_in_rows <= 0 || num_in_rows > kWidenCopy / wide) return false;
   if (mode < 2) return slice == 2 && num_edges >= kWidenGrouped && num_edges / 4 >= num_in_rows;      // (grouped)
-  if (mode == kOrderEven) return slice == (int)esz && row >= 480 && wide <= 1024 && num_edges >= kWidenEven && num_edges / 8 >= num_in_rows;
+  if (mode == kOrderEven) return slice == (int)esz && row >= 480 && wide <= 1024 && num_edges >= (slice == 2 ? kWidenGrouped : kWidenEven) && num_edges / 8 >= num_in_rows;
   if (num_edges < kWidenEdges || num_edges / (wide > 1024 ? 16 : slice == (int)esz ? 3 : 4) < num_in_rows) return false;
   if (row <= 128 && (slice == 4 || row <= 64)) return slice <= 4 && num_edges >= 2 * kWidenEdges && (slice == 2 || (row >= 64 && num_edges / 6 >= num_in_rows));
   return slice == 2 || row >= (slice == 4 ? 384 : 768);

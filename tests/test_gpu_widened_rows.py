@@ -136,10 +136,10 @@ def test_rows_that_stay_as_they_are():
 def test_rows_that_all_have_as_many_edges_stay_as_they_are():
     """Mode 3: in no order, and no row with very many of the edges."""
     bytes_of = lib.apt_spmm_widened_bytes
-    assert bytes_of(1, 900_000, 67_000, 251, 3) == 0 and bytes_of(0, 400_000, 20_000, 101, 3) == 0
+    assert bytes_of(1, 390_000, 20_000, 251, 3) == 0 and bytes_of(0, 900_000, 20_000, 137, 3) == 0 and bytes_of(0, 400_000, 20_000, 101, 3) == 0
     assert bytes_of(1, 1_000_000, 67_000, 101, 3) == 0 and bytes_of(1, 1_000_000, 67_000, 198, 3) == 0
     assert bytes_of(1, 1_000_000, 200_000, 251, 3) == 0 and bytes_of(0, 1_000_000, 67_000, 602, 3) == 0
-    assert bytes_of(1, 1_000_000, 67_000, 251, 3) == 67_000 * 512 and bytes_of(0, 1_000_000, 67_000, 137, 3) == 67_000 * 560
+    assert bytes_of(1, 400_000, 40_000, 251, 3) == 40_000 * 512 and bytes_of(0, 1_000_000, 67_000, 137, 3) == 67_000 * 560
     # with such rows, but a copy that takes longer than it gives
     assert bytes_of(0, 1_000_000, 300_000, 602, 2) == 0 and bytes_of(0, 150_000, 9_000, 31, 2) == 0 and bytes_of(1, 100_000, 9_000, 17, 2) == 0
 
