@@ -12,7 +12,6 @@
 namespace apt {
 
 constexpr int kWidenSlices = 4;      // a lane has on their way
-constexpr int kWidenRows = 1 << 11;  // a chunk, at most
 
 // Bytes [p, p + valid) in front of zeros; whole elements of 2 or 4 bytes.
 __device__ __forceinline__ uint4 slice_by_elements(const char* p, int valid) {
@@ -91,8 +90,9 @@ k_widen(const char* __restrict__ in, int64_t num_rows, int row_bytes, uint32_t s
 
 int widen_rows(const void* in, int64_t num_rows, int64_t row_bytes, void* out, cudaStream_t s) {
   const int64_t slices = ceil_div(row_bytes, 16);
-  // about a round of slices for every lane of a chunk's warp; the row of slice i: exact while i < 2^18 and slices < 2^12 (k_gather)
-  const int per = (int)std::max<int64_t>(1, std::min<int64_t>(kWidenRows, 32 * kWidenSlices / slices));
+  // about a round of slices for every lane of a chunk's warp, of 64 rows at most (rows of two slices and more); the row of slice i: exact while i < 2^18 and
+  // slices < 2^12 (k_gather)
+  const int per = (int)std::max<int64_t>(1, 32 * kWidenSlices / slices);
   const uint32_t inverse = (uint32_t)(((1ull << 31) + slices - 1) / slices);
   APT_FOLLOW(k_widen, wave_grid(ceil_div(num_rows, (int64_t)per * 8), 8), 256, 0, s, (const char*)in, num_rows, (int)row_bytes, (uint32_t)slices,
              inverse, per, (uint4*)out);

@@ -40,11 +40,11 @@ sys.path.insert(0, ROOT)
 STAGE_TAGS = ("sample", "relabel", "bucket", "unique_sorted", "gather_hit", "p2p_push", "p2p_wait", "p2p_pull")
 # DRAM bytes (read + written) per algorithmic byte of the gather kernel, from an ncu capture of that kernel
 # alone at the mini-batch's size: 143 000 random rows of 512 bytes out of a 2 GB cache table moved
-# 88.5 MB of DRAM reads (every row once, and a sector for each id's position) and 16.3 MB of DRAM writes (the rest of
+# 87.4 MB of DRAM reads (every row once, and a sector for each id's position) and 20.1 MB of DRAM writes (the rest of
 # the 73.2 MB written was still in the 126 MB L2 when the kernel ended) for 148.7 MB algorithmic.
-HIT_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (88.5 + 16.3) / 148.7
+HIT_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (87.4 + 20.1) / 148.7
 HIT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_gather at 143 000 rows x 512 B "
-                      "(104.8 MB per 148.7 MB algorithmic), scaled by this launch's algorithmic bytes; writes that "
+                      "(107.5 MB per 148.7 MB algorithmic), scaled by this launch's algorithmic bytes; writes that "
                       "stay in L2 past the kernel's end are not in it")
 # the pool's reference figure for a peer copy over NVLink, GB/s per direction (900 nominal); the benchmark
 # also measures a copy-engine peer copy in its own run and reports fractions of all three
