@@ -1,5 +1,5 @@
-"""The gather copies a chunk of rows as one run of elements: widths and numbers of rows around a warp's lanes, its eight elements in flight, the
-chunk's bytes and the longest row that shares a chunk, with rows of the host table and rows of neither among them. Copied bytes: exact."""
+"""The gather's widths around a warp's lanes, its eight elements in flight and the bytes of a chunk, with rows of the host table and rows of neither among
+them, in requests so small that every row has a warp to itself (rows that share a chunk: test_gpu_gather_host_rows.py). Copied bytes: exact."""
 import numpy as np
 import pytest
 import torch

@@ -29,11 +29,16 @@ def _expect(got, row, col, x, dst, most):
     assert ((got.double() - want).abs() <= bound).all()
 
 
+def _whole(shape, dtype, g, most):
+    """Whole numbers, whose sums are exact in fp32: one edge more or less shows."""
+    return torch.randint(-most, most + 1, shape, generator=g, device="cuda").to(dtype)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("dim", [9, 17, 18, 31, 61, 101, 119, 137, 197, 198, 251, 255, 301, 511, 1001])
 @pytest.mark.parametrize("segments", [1, 3])
 def test_sums_in_no_order(dtype, dim, segments):
-    # 100 000 edges and more go the widened way where the width does (kWidenEdges, twice that)
+    # (rows of about as many edges: most widths are read as they are; with some rows of very many below)
     dst, src, per = 19_997, 9_001, 11
     parts = [_block(dst, src, per, False, 7 * dim + k) for k in range(segments)]
     x = torch.randn(segments * src, dim, generator=parts[0][2], device="cuda").to(dtype)
@@ -43,6 +48,24 @@ def test_sums_in_no_order(dtype, dim, segments):
     for k, (r, c, _) in enumerate(parts):
         most = int(torch.bincount(c).max()) + 40
         _expect(got[k * dst:(k + 1) * dst], r, c, x[k * src:(k + 1) * src], dst, most)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dim", [9, 17, 18, 31, 61, 101, 119, 137, 197, 198, 251, 255, 301, 511, 1001])
+@pytest.mark.parametrize("segments", [1, 3])
+def test_sums_in_no_order_with_rows_of_many_edges(dtype, dim, segments):
+    """Whole numbers, exactly: 220 000 edges and more drawn at u^2 of the rows go the widened way where the width does."""
+    dst, src, edges = 19_997, 9_001, 219_967
+    g = torch.Generator(device="cuda").manual_seed(7 * dim)
+    off = lambda n: torch.arange(segments + 1, device="cuda") * n      # noqa: E731
+    row = torch.randint(0, src, (segments * edges,), generator=g, device="cuda")
+    u = torch.rand(segments * edges, generator=g, device="cuda", dtype=torch.float64)
+    col = (u * u * dst).long().clamp_(max=dst - 1)
+    x = _whole((segments * src, dim), dtype, g, 9)
+    got = ops.spmm_copy_u_sum(row, col, x, off(edges), off(src), off(dst))
+    part = torch.arange(segments, device="cuda").repeat_interleave(edges)
+    want = torch.zeros(segments * dst, dim, dtype=torch.float64, device="cuda").index_add_(0, col + part * dst, x.double()[row + part * src])
+    assert torch.equal(got, want.float().to(dtype))
 
 
 @pytest.mark.parametrize("dtype,dim", [(torch.float32, 31), (torch.float32, 101), (torch.bfloat16, 17), (torch.bfloat16, 61), (torch.bfloat16, 119),
@@ -220,11 +243,7 @@ def test_attention_of_heads_that_are_no_whole_slices(dtype, heads, head_dim):
         assert ((a - b).abs() <= 2 * _EPS[dtype] * b.abs() + 2e-5 * b.abs().max()).all()
 
 
-# ---- every edge once: whole numbers whose sums are exact in fp32, so that one edge more or less shows
-def _whole(shape, dtype, g, most):
-    return torch.randint(-most, most + 1, shape, generator=g, device="cuda").to(dtype)
-
-
+# ---- every edge once
 @pytest.mark.parametrize("dtype,dim", [(torch.float32, 31), (torch.float32, 101), (torch.bfloat16, 17), (torch.bfloat16, 61), (torch.float16, 251), (torch.float32, 251),
                                        (torch.float16, 601)])
 @pytest.mark.parametrize("edges", [240_088, 1_000_003])
