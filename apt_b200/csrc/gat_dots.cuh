@@ -13,7 +13,7 @@
 //
 // us of a backward pass, multiplied out -> here: bf16 4 x 64, 67 584 x 15 edges 190 -> 185, x 3 edges 87 -> 74, 30 000 x 10 86 -> 77; 4 x 32, 67 584 x 15 200 -> 160; 1 x 128
 // 193 -> 148; 1 x 32 111 -> 98; f16 8 x 32 213 -> 200, 30 000 x 10 97 -> 85; 2 x 64, 67 584 x 15 199 -> 150. (Accumulated in the tensor cores bf16 4 x 64 170, 4 x 32 150: the
-// products that make the cut good take 14 us of a million edges of 256 columns.) So they take every shape they can be built for. Shared addresses worked out for every
+// products that make the cut good take 14 us of a million edges of 256 columns, the look for sums that are none, which these figures are without, 2 - 3.) So they take every shape they can be built for. Shared addresses worked out for every
 // access and a predicate for every row, 27 instructions an edge, took the dots from 56 to 62.
 #pragma once
 
@@ -55,6 +55,19 @@ __device__ __forceinline__ void products(F2 (&sum)[2], uint32_t a0, uint32_t a1,
 #pragma unroll
     for (int i = 0; i < 2; ++i)
       sum[i] = f2_add(sum[i], f2_add(f2_pack(p_rest[2 * i], p_rest[2 * i + 1]), f2_pack(q_rest[2 * i], q_rest[2 * i + 1])));
+  }
+}
+
+// An edge's dots that came to NaN, multiplied out: nothing is left of an infinite sum, and that taken from it is no number. us of a backward of 67 584 x 15 edges
+// from 150 000 sources, without -> with: 4 x 64 196 -> 199, 1 x 256 185 -> 189, 1 x 128 138 -> 141, 1 x 32 86 -> 88, 8 x 32 235 -> 241. (What is left kept beside a
+// head's sum and added where that is finite spilled: 8 x 32 256.)
+template <typename T>
+__device__ __noinline__ void dots_again(const T* __restrict__ x, const T* __restrict__ y, int heads, int head_dim, float* dots) {
+  for (int h = 0; h < heads; ++h) {
+    if (dots[h] == dots[h]) continue;
+    float sum = 0.f;
+    for (int c = h * head_dim; c < (h + 1) * head_dim; ++c) sum = fmaf(Elem<T>::to_f(x[c]), Elem<T>::to_f(y[c]), sum);
+    dots[h] = sum;
   }
 }
 
@@ -180,6 +193,15 @@ k_gat_dots_mma(const int64_t* __restrict__ row, const int64_t* __restrict__ col,
               *(float2*)(out + 8 * i * H) = make_float2(v[0], v[1]);
             } else {
               out[8 * i * H] = v[0];
+            }
+            if constexpr (Elem<T>::kIsBf16) {
+              bool none = false;
+#pragma unroll
+              for (int h = 0; h < H; ++h) none |= v[h] != v[h];
+              if (none) {
+                const uint64_t src = min((uint32_t)row[base + pos + g + 8 * i], num_src - 1), dst = min((uint64_t)tile + s, (uint64_t)num_dst - 1);
+                dots_again(ft + src * (NC * 32), grad + dst * (NC * 32), H, CPH * 32, out + 8 * i * H);
+              }
             }
           }
         }

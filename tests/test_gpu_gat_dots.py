@@ -105,3 +105,34 @@ def test_dots_are_rounded_sums(dtype, H, D):
     # sum, down a tree, by less every time, less than three such steps together, and once more for the mean of the two.
     error = 4 * got.norm() / 2 ** 0.5 / 2 ** 0.5 / dots.norm()
     assert error <= 2.0 ** -23, float(error)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,D", [(4, 32), (2, 64), (1, 256)])
+@pytest.mark.parametrize("what", ["infinity", "a sum beyond fp32"])
+def test_infinite_dots_are_infinite(dtype, H, D, what):
+    """Four sources of a destination with the same score; the dot of one is infinite, for an infinite value or from finite ones. Its own gradient is none,
+    the other three's are minus what infinity it is. All other destinations' are what they are without it."""
+    dst, at = 40, 3 * D // 4 + 1
+    if what != "infinity" and dtype == torch.float16:
+        pytest.skip("products of 16-bit floats of this range have no such sum")
+    g = torch.Generator(device="cuda").manual_seed(D)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(dtype)      # noqa: E731
+    row, col = torch.arange(4 * dst, device="cuda"), torch.arange(dst, device="cuda").repeat_interleave(4)
+    ft, grad = normal(4 * dst, H, D), normal(dst, H, D)
+    el, er = torch.ones(4 * dst, H, 1, dtype=dtype, device="cuda"), torch.ones(dst, H, 1, dtype=dtype, device="cuda")
+    clean = ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, grad, 0.2)[1].view(dst, 4, H)
+    for d, sign in ((5, 1), (22, -1)):
+        if what == "infinity":
+            grad[d, 0, at] = 2.0
+            ft[4 * d + 1, 0, at] = sign * float("inf")
+        else:
+            grad[d, 0, at - 1:at + 1] = 2.0 ** 100
+            ft[4 * d + 1, 0, at - 1:at + 1] = sign * 2.0 ** 30
+            ft[[4 * d, 4 * d + 2, 4 * d + 3], 0, at - 1:at + 1] = 0
+    got = ops.gat_edge_softmax_sum_backward(row, col, ft, el, er, grad, 0.2)[1].view(dst, 4, H)
+    for d, sign in ((5, 1), (22, -1)):
+        assert got[d, 1, 0].isnan() and (got[d, [0, 2, 3], 0] == -sign * float("inf")).all(), got[d, :, 0]
+        got[d, :, 0] = clean[d, :, 0]
+    assert torch.equal(got, clean)
+    ops.check_status()
