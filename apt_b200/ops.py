@@ -173,6 +173,18 @@ class NPCState:
     def join(self, k: int):
         torch.cuda.current_stream().wait_stream(self.side_stream(k))
 
+    @contextlib.contextmanager
+    def joined_if_it_fails(self, *sides: Optional[int]):
+        """For what runs while side streams are at work (None: no such stream). Where it raises, the current stream waits for them all the
+        same: their buffers are given back and their scratch is the next caller's."""
+        try:
+            yield
+        except BaseException:
+            for k in sides:
+                if k is not None:
+                    self.join(k)
+            raise
+
     def lane_stream(self, lane: int) -> torch.cuda.Stream:
         """The one stream on which work that uses lane `lane`'s scratch is enqueued: everything on
         a lane runs in order, whichever sampler put it there."""

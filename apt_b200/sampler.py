@@ -510,7 +510,7 @@ class MixedNeighborSampler(_GraphReplay):
         sizes_view = recv_view if ws == 1 else words[128:128 + ws + 1]
         lo, hi = ops._owned_range()
         u_slot, in_slot = slot, slot + 1
-        alone = self._alone()
+        alone, side = self._alone(), None
         if alone:
             # one rank receives what it has; what only the caller wants (the permutation, the sizes, the inverse) is made beside the outermost
             # hop, of whose chain it was 5 us
@@ -529,15 +529,17 @@ class MixedNeighborSampler(_GraphReplay):
         prefetch = self.prefetch_features and _fits_prefetch(uniq2.numel() * (1 + self.las_fanouts))
         split = self.gather_split if prefetch and not st.profiling else 0
         rows = None
-        if prefetch:
-            rows = torch.empty((uniq2.numel() * (1 + self.las_fanouts), f.rank_feat_dim), dtype=f.dev_feats.dtype,
-                               device=uniq2.device)
-        if split:
-            with st.beside(2):
-                ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier", beside=True)
-        uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
-                                                     call if explicit else None, call_base_dev, look_up=prefetch)
-        if alone and side is not None:
+        with st.joined_if_it_fails(side):
+            if prefetch:
+                rows = torch.empty((uniq2.numel() * (1 + self.las_fanouts), f.rank_feat_dim), dtype=f.dev_feats.dtype,
+                                   device=uniq2.device)
+            if split:
+                with st.beside(2):
+                    ops._gather_enqueue(uniq2, st.word(u_slot), out=rows, ws_name="gather_frontier", beside=True)
+            with st.joined_if_it_fails(2 if split else None):
+                uniq3, rel3, _ = ops._sample_relabel_enqueue(uniq2, self.las_fanouts, st.word(u_slot), st.word(in_slot),
+                                                             call if explicit else None, call_base_dev, look_up=prefetch)
+        if side is not None:
             st.join(side)      # the sizes leave with the counts
         if split == 1:
             if publish is not None:
