@@ -224,14 +224,16 @@ k_gat_dots_mma(const int64_t* __restrict__ row, const int64_t* __restrict__ col,
 // Where most destinations have no edges, the eight rows of a tile are fetched for one or two that have, and a group of edges goes through several tiles.
 // k_gat_dots, a warp to a destination, loses there all the same; k_spmm_stream, which takes wide rows of many edges, fetches those in use alone. us of a
 // backward, k_spmm_stream -> here, 1 000 000 edges from 150 000 sources: f16 8 x 32, 66 666 destinations of 15 edges side by side 214 -> 200, 4 apart 309 -> 309, 8 apart
-// 374 -> 396; bf16 4 x 64 188 -> 184, 3 apart 212 -> 214, 4 apart 220 -> 231; 500 000 of 2 side by side 284 -> 261; 333 333 of 3, accumulated in the tensor cores, 2 apart
-// 310 -> 278, 4 apart 350 -> 382, 8 apart 426 -> 578. The lines, edges to a destination, are where none of them loses.
+// 374 -> 396; bf16, whose products are made twice, side by side, 2 and 3 apart 1 x 256 192, 220, 226 -> 188, 216, 228, 2 x 128 201, 230, 236 -> 200, 227, 240, 4 x 64
+// 198, 232, 247 -> 199, 231, 251, 8 x 32 233, 296, 345 -> 240, 305, 362; 100 000 of 10 1 x 256 197 -> 197, 2 x 128 205 -> 207, 4 x 64 208 -> 211, 8 x 32 257 -> 269. The lines, edges to a
+// destination and columns of a bf16 head, are where none of them loses more than 3 %.
 template <typename T>
 inline bool dots_mma_fits(int heads, int64_t head_dim, int slice, int64_t num_edges, int64_t num_dst) {
   const int64_t dim = heads * head_dim;
   auto pow2 = [](int64_t x) { return x > 0 && (x & (x - 1)) == 0; };
   if (sizeof(T) != 2 || slice != 16 || num_edges > kStreamMaxEdges || head_dim < 32 || dim > 256 || !pow2(head_dim) || !pow2(heads)) return false;
-  return num_edges / (Elem<T>::kIsBf16 ? 5 : 2) >= num_dst || !stream_fits(kDots, slice, dim, sizeof(T), heads, num_edges, true);
+  const bool many = Elem<T>::kIsBf16 ? head_dim >= 64 && num_edges / 5 >= num_dst : num_edges / 2 >= num_dst;
+  return many || !stream_fits(kDots, slice, dim, sizeof(T), heads, num_edges, true);
 }
 
 template <typename T, int NC, int CPH>

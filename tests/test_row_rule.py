@@ -83,3 +83,5 @@ def test_dots_of_blocks_whose_destinations_are_sparse(tmp_path):
     assert ask(*wide) == [1, 1, 0, 0, 0, 1] * 2 + [1, 1, 1, 1, 0, 1]
     # narrow rows, heads that are no power of two, rows that are no whole slices
     assert ask((1, 4, 32, 16, 1_000_000, 900_000), (1, 3, 64, 16, 1_000_000, 60_000), (1, 4, 48, 16, 1_000_000, 60_000), (1, 4, 64, 8, 1_000_000, 60_000)) == [1, 0, 0, 0]
+    # bf16 heads of 32 columns, whose products are made twice: wide rows of many edges are the stream's
+    assert ask((1, 8, 32, 16, 1_000_000, 60_000), (1, 8, 32, 16, 393_215, 60_000), (1, 4, 64, 16, 1_000_000, 60_000)) == [0, 1, 1]
